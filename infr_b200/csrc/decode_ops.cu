@@ -1040,7 +1040,11 @@ __global__ void __launch_bounds__(256) attn_combine_wide_kernel(const float *__r
         float l = 0.f;
         for (int s = lane; s < n_splits; s += 32) {
             const float ls = ml[2 * s + 1];
-            const float wgt = ls == 0.f ? 0.f : expf(ml[2 * s] - m);
+            if (ls == 0.f) {
+                s_w[warp][s] = -1.f;  // a tile past the row's causal end
+                continue;
+            }
+            const float wgt = expf(ml[2 * s] - m);
             s_w[warp][s] = wgt;
             l += wgt * ls;
         }
@@ -1056,7 +1060,9 @@ __global__ void __launch_bounds__(256) attn_combine_wide_kernel(const float *__r
 #pragma unroll 4
         for (int s = warp; s < n_splits; s += 8) {
             const float wgt = s_w[hh][s];
-            const float4 p = *reinterpret_cast<const float4 *>(po + (size_t)s * head_dim);
+            float4 p = *reinterpret_cast<const float4 *>(po + (size_t)s * head_dim);
+            // nobody wrote that tile's sums: what an earlier op left there may read as NaN, which no weight of 0 would cancel
+            if (wgt < 0.f) p = make_float4(0.f, 0.f, 0.f, 0.f);
             acc.x = fmaf(wgt, p.x, acc.x), acc.y = fmaf(wgt, p.y, acc.y), acc.z = fmaf(wgt, p.z, acc.z), acc.w = fmaf(wgt, p.w, acc.w);
         }
         *reinterpret_cast<float4 *>(&s_acc[warp][e]) = acc;
