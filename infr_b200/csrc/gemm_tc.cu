@@ -5,7 +5,8 @@
 // their f32 sums are the integers of the CPU's dot products (exact up to 2^24; a larger sum is rounded like any float):
 //   Q4_K  q * sc          <= 15 * 63 = 945       one multiply per weight; an int8 form needs two (q * (sc & 7), q * (sc >> 3))
 //   Q4_K  m_s, 64h + l    the block minimum: sum_s m_s * bsum_s as ONE K = 16 instruction (8 sub-blocks x {64h, l})
-//   Q6_K  sc * nib, sc * 16 * (hb - 2)            two multiplies into one accumulator (|sc * (q - 32)| can reach 4096)
+//   Q6_K  sl * (q - 32), sh * (q - 32)            sc = 16 sh + sl, one accumulator each (a block's |L| <= 15 * 32 * 127 * 256 and |H|
+//                                                 <= 8 * 32 * 127 * 256 stay below 2^24; sums of sc * (q - 32) reach 1.3e8); sum = 16 H + L
 //   Q2_0  code - 1                                one accumulator per 32-element activation group
 // The f32 expression of the CPU is applied per block (crates/infr-cpu/src/kernels.rs:151-184, :5641-5668):
 // C += d8 * (d * sd - dmin * sm), C += (d8 * d) * sd, C += d * (d8_0 * s_0 + d8_1 * s_1), accumulated in block order in registers.
@@ -22,10 +23,11 @@
 // TN = 32 (Q4_K) keeps to half an SM's shared and tensor memory, so that two CTAs hide each other's waits.
 // Measured (B200, us, cold weights; before = the int8 tensor-memory GEMM for Q4_K, the wide GEMV 32 rows at a time for Q6_K, the
 // 8-row GEMV walk for Q2_0):  Q4_K 4096 -> 14336, 512 rows 161 -> 108, 113 rows 53 -> 33, 64 rows 30 -> 24;  Q6_K 14336 ->
-// 4096, 113 rows 125 -> 53, 512 rows 520 -> 174;  Q2_0 14336 -> 4096, 77 rows 201 -> 78.
+// 4096, 113 rows 125 -> 57, 512 rows 520 -> 179 (54 and 171 with one accumulator, whose sums round above 2^24; 60 and 192 with
+// two accumulators drained by 8 warps);  Q2_0 14336 -> 4096, 77 rows 201 -> 78.
 // What bounds it: at 128 tokens a Q4_K job takes ~2800 cycles where its MMAs take 1100; the epilogue (D and M: 128 KB per job
 // out of tensor memory, busy 2100 of them) is the slowest role, 8 or 16 warps alike.  Q6_K: the unpack warps (~3700 cycles per
-// block and warp).  Q2_0: the epilogue, one drain per 64 elements (~1000 cycles).
+// block and warp) and, at 128 tokens, the drain between two blocks (one set of accumulators fits).  Q2_0: the epilogue, one drain per 64 elements (~1000 cycles).
 // Every wait is bounded: on expiry the role raises a CTA flag and a status word, every role leaves its loop, copies in
 // flight are drained and the tensor memory is freed.
 #include <cuda.h>
@@ -54,7 +56,8 @@ struct Cfg {
     static constexpr int kTeams = 2;                                             // of four unpack warps each
     static constexpr int kUnpack = 4 * kTeams;
     static constexpr int kTeamUnits = kUnits / kTeams;
-    static constexpr int kAcc = FMT == F_Q2 ? 2 : 1;                             // accumulators per job
+    static constexpr int kAcc = FMT == F_Q4 ? 1 : 2;                             // accumulators per job
+    static constexpr int kJobBuf = FMT == F_Q6 && TN == 128 ? 1 : 2;             // jobs that have accumulators at a time
     static constexpr int kRowBytes = FMT == F_Q6 ? 224 : 144;
     static constexpr int kRaw = kTM * kRowBytes;
     static constexpr int kUnitBytes = (FMT == F_Q4 ? 256 : 128) * TN;            // activation operand of one group
@@ -71,14 +74,14 @@ struct Cfg {
     static constexpr int kRing = FMT == F_Q2 ? 16 : 4;                           // row scales, per job
     static constexpr int kScale = FMT == F_Q4 ? 2 : 1;                           // floats per row and job (d, dmin)
     static constexpr int kSmem = kNB * kUnitBytes + kStages * kStage + kMin + kRing * kTM * kScale * 4;
-    static constexpr int kEpi = TN == 32 ? 4 : ((TN == 128 && FMT == F_Q4) || FMT == F_Q2 ? 16 : 8);
+    static constexpr int kEpi = TN == 32 ? 4 : (TN == 128 || FMT == F_Q2 ? 16 : 8);
     static constexpr int kCols = TN / (kEpi / 4);                                // output columns of an epilogue thread
-    static constexpr int kChunk = TN == 64 && FMT != F_Q2 ? 16 : 8;                              // columns per tensor-memory load (registers)
+    static constexpr int kChunk = TN == 64 && FMT == F_Q4 ? 16 : 8;                   // columns per tensor-memory load (registers)
     static constexpr int kWarps = kUnpack + kEpi + 3;
     static constexpr int kCtas = TN == 32 && FMT != F_Q6 ? 2 : 1;
-    // tensor-memory columns: accumulators of two jobs, block-minimum sums of two jobs (one where there is no room), operands
+    // tensor-memory columns: accumulators of two jobs (one where there is no room), block-minimum sums of two jobs (one where there is no room), operands
     static constexpr int kMBuf = FMT == F_Q4 ? (TN == 128 ? 1 : 2) : 0;
-    static constexpr uint32_t kColM = 2 * kAcc * TN;
+    static constexpr uint32_t kColM = kJobBuf * kAcc * TN;
     static constexpr uint32_t kColA = kColM + kMBuf * TN;
     static constexpr uint32_t kCols0 = kColA + kSlots * kGroupSlots * 32;
     static constexpr uint32_t kTmem = kCols0 <= 256 ? 256 : 512;
@@ -196,7 +199,7 @@ __device__ __forceinline__ uint32_t h2add(uint32_t a, uint32_t b) {
 __device__ __forceinline__ constexpr uint32_t dup(uint32_t h) { return h | (h << 16); }
 // f16 bit patterns of the small constants used below (integers and powers of two)
 constexpr uint32_t H_1024 = 0x6400, H_N1024 = 0xE400, H_N1152 = 0xE480, H_N64 = 0xD400, H_1_16 = 0x2C00, H_1_4 = 0x3400, H_1_64 = 0x2400,
-                   H_16 = 0x4C00, H_4 = 0x4400, H_1 = 0x3C00;
+                   H_1 = 0x3C00, H_N1032 = 0xE408, H_N1056 = 0xE420, H_N1536 = 0xE600;
 
 // Q4_K: 64 elements = two sub-blocks in 8 words, scales s0 (low nibbles) and s1 (high nibbles).  Operand values leave in
 // the order (0, 2, 1, 3) of every four elements; gemm_tc_prep_kernel lays the activations out the same way.
@@ -214,29 +217,30 @@ __device__ __forceinline__ void unpack_q4(const uint32_t *w, uint32_t s0, uint32
     }
 }
 
-// int8 scale (low byte) -> f16 in both halves
-__device__ __forceinline__ uint32_t h2_of_s8(uint32_t byte) { return h2add(dup(H_1024) | ((byte ^ 0x80u) & 0xFFu) * 0x10001u, dup(H_N1152)); }
-
 // Q6_K: 32 elements (part = 0..3 of a half block): low nibbles from ql[8 words], two high bits from qh[8 words], scales of
-// the two 16-element sub-blocks.  o[0..15] = sc * nib, o[16..31] = sc * 16 * (hb - 2), the same element order as above.
+// the two 16-element sub-blocks (low byte each).  o[0..15] = sl * (q - 32), o[16..31] = sh * (q - 32) with sc = 16 sh + sl,
+// 0 <= sl < 16, -8 <= sh < 8, the same element order as above.
 template <int PART>
 __device__ __forceinline__ void unpack_q6(const uint32_t *ql, const uint32_t *qh, uint32_t sc0, uint32_t sc1, uint32_t (&o)[32]) {
     constexpr bool HI = PART >= 2;
-    constexpr uint32_t lm = HI ? 0x00F000F0u : 0x000F000Fu, hm = 0x00030003u << (2 * PART);
-    // -(1024 + 2 * 4^PART)
-    constexpr uint32_t off = PART == 0 ? 0xE402u : (PART == 1 ? 0xE408u : (PART == 2 ? 0xE420u : 0xE480u));
-    constexpr uint32_t mul = PART == 0 ? H_16 : (PART == 1 ? H_4 : (PART == 2 ? H_1 : H_1_4));  // 16 / 4^PART
-    const uint32_t s[2] = {h2_of_s8(sc0), h2_of_s8(sc1)};
+    // the nibbles stay where they are, so q is built at bit 0 (parts 0, 1) or bit 4 (parts 2, 3), below the f16 of 1024
+    constexpr uint32_t lm = HI ? 0x00F000F0u : 0x000F000Fu, hm = HI ? 0x03000300u : 0x00300030u;
+    constexpr uint32_t off = HI ? H_N1536 : H_N1056;         // -(1024 + 16 * 32), -(1024 + 32)
+    constexpr int up = PART & 1 ? 2 : 4;                     // the high bits' way to their place (bytes 1 and 3: 8 less)
+    const uint32_t sc[2] = {sc0, sc1};
 #pragma unroll
     for (int g = 0; g < 2; g++) {
-        const uint32_t sl = HI ? h2mul(s[g], dup(H_1_16)) : s[g], sh = h2mul(s[g], dup(mul));
+        uint32_t sl = h2add(dup(H_1024) | (sc[g] & 0xFu) * 0x10001u, dup(H_N1024));
+        uint32_t sh = h2add(dup(H_1024) | (((sc[g] >> 4) & 0xFu) ^ 8u) * 0x10001u, dup(H_N1032));
+        if (HI) sl = h2mul(sl, dup(H_1_16)), sh = h2mul(sh, dup(H_1_16));
 #pragma unroll
         for (int i = 4 * g; i < 4 * g + 4; i++) {
-            const uint32_t v = ql[i], u = v >> 8, y = qh[i], z = y >> 8;
-            o[2 * i] = h2mul(h2add((v & lm) | dup(H_1024), dup(H_N1024)), sl);
-            o[2 * i + 1] = h2mul(h2add((u & lm) | dup(H_1024), dup(H_N1024)), sl);
-            o[16 + 2 * i] = h2mul(h2add((y & hm) | dup(H_1024), dup(off)), sh);
-            o[17 + 2 * i] = h2mul(h2add((z & hm) | dup(H_1024), dup(off)), sh);
+            const uint32_t v = ql[i], u = v >> 8, y = qh[i] << up, z = qh[i] >> (8 - up);
+            const uint32_t a = h2add((v & lm) | ((y & hm) | dup(H_1024)), dup(off)), b = h2add((u & lm) | ((z & hm) | dup(H_1024)), dup(off));
+            o[2 * i] = h2mul(a, sl);
+            o[2 * i + 1] = h2mul(b, sl);
+            o[16 + 2 * i] = h2mul(a, sh);
+            o[17 + 2 * i] = h2mul(b, sh);
         }
     }
 }
@@ -511,7 +515,7 @@ __global__ void __launch_bounds__(Cfg<FMT, TN>::kWarps * 32, Cfg<FMT, TN>::kCtas
                 constexpr int me = decltype(which)::value;
                 const uint32_t idesc = (1u << 4) | ((uint32_t)(TN >> 3) << 17) | ((uint32_t)(kTM >> 4) << 24);
                 const uint64_t bd0 = mk_desc(su32(bring), TN * 16);
-                const uint32_t td = tmem + (uint32_t)(me * K::kAcc * TN);
+                const uint32_t td = tmem + (uint32_t)((K::kJobBuf == 2 ? me : 0) * K::kAcc * TN);
                 int j = 0;                // jobs of this CTA, over all tiles
                 uint32_t q = 0, qp = 0;   // activation ring: next group's place and phase
                 int ls = 0;               // raw stage of the job
@@ -529,7 +533,13 @@ __global__ void __launch_bounds__(Cfg<FMT, TN>::kWarps * 32, Cfg<FMT, TN>::kCtas
                                 continue;
                             }
                             const uint32_t jp = (uint32_t)(j >> 1) & 1u;
-                            if (j >= 2 && !(ok = wait_warp(bar(K::B_ACCFREE + me), jp ^ 1u, dead))) break;
+                            // the job that had these accumulators before (with one set: the other issuer's last job; seen in order,
+                            // because job j - 2 was begun only after job j - 3 had been drained)
+                            if (K::kJobBuf == 2) {
+                                if (j >= 2 && !(ok = wait_warp(bar(K::B_ACCFREE + me), jp ^ 1u, dead))) break;
+                            } else {
+                                if (j >= 1 && !(ok = wait_warp(bar(K::B_ACCFREE + (me ^ 1)), (uint32_t)((j - 1) >> 1) & 1u, dead))) break;
+                            }
 #pragma unroll
                             for (int g = 0; g < K::kGroups; g++) {
                                 // room in tensor memory, and the barrier that says it is filled
@@ -549,10 +559,10 @@ __global__ void __launch_bounds__(Cfg<FMT, TN>::kWarps * 32, Cfg<FMT, TN>::kCtas
                                 if (lane == 0) {
 #pragma unroll
                                     for (int k = 0; k < 4 * K::kGroupSlots; k++) {
-                                        // Q6_K: the low-nibble and the high-bit operands of a slot meet the same 32 activations
+                                        // Q6_K: the sl and the sh operands of a slot meet the same 32 activations
                                         const int pl = FMT == F_Q6 ? (k >> 2) * 4 + (k & 1) * 2 : k * 2;
-                                        const uint32_t dst = td + (FMT == F_Q2 ? (uint32_t)((k >> 1) * TN) : 0u);
-                                        const uint32_t keep = FMT == F_Q2 ? (uint32_t)(k & 1) : (uint32_t)(g > 0 || k > 0);
+                                        const uint32_t dst = td + (K::kAcc == 2 ? (uint32_t)(((k >> 1) & 1) * TN) : 0u);
+                                        const uint32_t keep = (uint32_t)(g > 0 || (K::kAcc == 2 ? (k >= 4 || (k & 1)) : k > 0));
                                         mma_ta(dst, ta + (uint32_t)(k * 8), bd + (uint64_t)(pl * TN), idesc, keep);
                                     }
                                     mma_commit(bar(K::B_AFREE + sl));
@@ -752,7 +762,7 @@ __global__ void __launch_bounds__(Cfg<FMT, TN>::kWarps * 32, Cfg<FMT, TN>::kCtas
                     }
 #pragma unroll 1
                     for (int jj = 0; jj < K::kJobs; jj++, j++) {
-                        const int s = j & 1;
+                        const int s = j & 1, sa = K::kJobBuf == 2 ? s : 0;
                         if (!(ok = wait_warp(bar(K::B_ACCRDY + s), (uint32_t)((j >> 1) & 1), dead))) break;
                         tc_fence_after();
                         const float *d8 = reinterpret_cast<const float *>(ex + (FMT == F_Q4 ? 32 * TN : 0)) + (FMT == F_Q2 ? jj * 2 * TN : 0) + col0;
@@ -767,9 +777,9 @@ __global__ void __launch_bounds__(Cfg<FMT, TN>::kWarps * 32, Cfg<FMT, TN>::kCtas
                         uint32_t sd[2][K::kChunk], sm[2][K::kChunk];
                         auto fetch = [&](int c) {
                             const int f = (c / K::kChunk) & 1;
-                            tld(tlane + (uint32_t)(s * K::kAcc * TN + c), sd[f]);
+                            tld(tlane + (uint32_t)(sa * K::kAcc * TN + c), sd[f]);
                             if (FMT == F_Q4) tld(tlane + K::kColM + (uint32_t)((K::kMBuf == 2 ? s * TN : 0) + c), sm[f]);
-                            if (FMT == F_Q2) tld(tlane + (uint32_t)(s * K::kAcc * TN + TN + c), sm[f]);
+                            if (K::kAcc == 2) tld(tlane + (uint32_t)(sa * K::kAcc * TN + TN + c), sm[f]);
                         };
                         fetch(0);
 #pragma unroll
@@ -793,7 +803,7 @@ __global__ void __launch_bounds__(Cfg<FMT, TN>::kWarps * 32, Cfg<FMT, TN>::kCtas
                                     if (FMT == F_Q4) {
                                         acc[c + n] = fmaf(dv[k], fmaf(-dm, __uint_as_float(sm[fb][n]), dw * f), acc[c + n]);
                                     } else if (FMT == F_Q6) {
-                                        acc[c + n] = fmaf(dw * dv[k], f, acc[c + n]);
+                                        acc[c + n] = fmaf(dw * dv[k], fmaf(16.f, __uint_as_float(sm[fb][n]), f), acc[c + n]);
                                     } else {
                                         part_sum[c + n] = fmaf(dw, fmaf(ev[k], __uint_as_float(sm[fb][n]), dv[k] * f), part_sum[c + n]);
                                     }

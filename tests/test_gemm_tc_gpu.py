@@ -64,6 +64,29 @@ def test_gemm_tc_extreme_codes(tc, oracle, dt):
     assert fx.rel_l2(tc.run_linear(dt, w, x, m, in_f, out_f), oracle.linear(dt, w, x, m, in_f, out_f)) < TOL
 
 
+def _q6_rows(rng, out_f, in_f):
+    """Codes 60..63 under scales of +127: a weight is 3556..3937 steps, so a block of codes near 127 sums to 1.2e8."""
+    blk = rng.integers(0, 256, (out_f * in_f // 256, 210), dtype=np.uint8)
+    blk[:, :128] |= 0xCC  # both nibbles 12..15
+    blk[:, 128:192] = 0xFF
+    blk[:, 192:208] = 127
+    blk[:, 208:210] = np.array([0.01], np.float16).view(np.uint8)
+    return blk.ravel()
+
+
+@pytest.mark.parametrize("m", [20, 40, 100])  # the three token tiles
+@pytest.mark.parametrize("x_of", ["same sign", "halves cancel"])
+def test_gemm_tc_block_sums_beyond_24_bits(tc, oracle, m, x_of):
+    # |block sum|, or what it climbs to half way, is above 2^24: still the CPU's integers, so the bound stays that of f32
+    in_f, out_f, rng = 2048, 130, np.random.default_rng(m)
+    x = rng.uniform(0.9, 1.0, (m, in_f)).astype(np.float32)
+    if x_of == "halves cancel":
+        x[:, np.arange(in_f) % 256 >= 128] *= -1.0
+    for dt, w in ((Q6K, _q6_rows(rng, out_f, in_f)),):
+        got, want = tc.run_linear(dt, w, x, m, in_f, out_f), oracle.linear(dt, w, x, m, in_f, out_f)
+        assert fx.rel_l2(got, want) < TOL
+
+
 @pytest.mark.parametrize("dt", [Q4K, Q6K, Q2_0])
 def test_gemm_tc_two_weights_and_repeat(tc, dt):
     # two matrices against the same rows in one launch; op by op, captured and replayed give the same bits
