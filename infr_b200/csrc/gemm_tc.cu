@@ -1,9 +1,11 @@
 // Batched GEMM C[m, out_f] = Q8(x)[m, in_f] * W^T for Q4_K, Q6_K and Q2_0 weights on tcgen05.mma kind::f16, exact in the
 // integer block sums.
 //
-// Why f16 operands: every integer that the formats multiply is exactly representable in 11 bits, so the products and
-// their f32 sums are the integers of the CPU's dot products (exact up to 2^24; a larger sum is rounded like any float):
-//   Q4_K  q * sc          <= 15 * 63 = 945       one multiply per weight; an int8 form needs two (q * (sc & 7), q * (sc >> 3))
+// Why f16 operands: every integer that the formats multiply is exactly representable in 11 bits, so the products and,
+// while they stay below 2^24, their f32 sums are integers.  The operands are chosen so that every partial sum of a block does:
+//   Q4_K  (q - 8) * sc    <= 8 * 63 = 504        one multiply per weight; an int8 form needs two (q * (sc & 7), q * (sc >> 3)).  A block's
+//                                                 sum stays below 504 * 127 * 256 < 2^24 (q * sc: 3.1e7); the last instruction of a block
+//                                                 adds 8 * sum_s sc_s * bsum_s (K = 16, as below): one rounding, where |sum| > 2^24
 //   Q4_K  m_s, 64h + l    the block minimum: sum_s m_s * bsum_s as ONE K = 16 instruction (8 sub-blocks x {64h, l})
 //   Q6_K  sl * (q - 32), sh * (q - 32)            sc = 16 sh + sl, one accumulator each (a block's |L| <= 15 * 32 * 127 * 256 and |H|
 //                                                 <= 8 * 32 * 127 * 256 stay below 2^24; sums of sc * (q - 32) reach 1.3e8); sum = 16 H + L
@@ -22,12 +24,14 @@
 //               and two commits; per job one commit to the epilogue
 // TN = 32 (Q4_K) keeps to half an SM's shared and tensor memory, so that two CTAs hide each other's waits.
 // Measured (B200, us, cold weights; before = the int8 tensor-memory GEMM for Q4_K, the wide GEMV 32 rows at a time for Q6_K, the
-// 8-row GEMV walk for Q2_0):  Q4_K 4096 -> 14336, 512 rows 161 -> 108, 113 rows 53 -> 33, 64 rows 30 -> 24;  Q6_K 14336 ->
+// 8-row GEMV walk for Q2_0):  Q4_K 4096 -> 14336, 512 rows 161 -> 111, 113 rows 53 -> 35, 64 rows 30 -> 25
+// (108, 34 and 25 without the centred codes and their correction);  Q6_K 14336 ->
 // 4096, 113 rows 125 -> 57, 512 rows 520 -> 179 (54 and 171 with one accumulator, whose sums round above 2^24; 60 and 192 with
 // two accumulators drained by 8 warps);  Q2_0 14336 -> 4096, 77 rows 201 -> 78.
 // What bounds it: at 128 tokens a Q4_K job takes ~2800 cycles where its MMAs take 1100; the epilogue (D and M: 128 KB per job
 // out of tensor memory, busy 2100 of them) is the slowest role, 8 or 16 warps alike.  Q6_K: the unpack warps (~3700 cycles per
-// block and warp) and, at 128 tokens, the drain between two blocks (one set of accumulators fits).  Q2_0: the epilogue, one drain per 64 elements (~1000 cycles).
+// block and warp) and, at 128 tokens, the drain between two blocks (one set of accumulators fits).  Q2_0: the epilogue,
+// one drain per 64 elements (~1000 cycles).
 // Every wait is bounded: on expiry the role raises a CTA flag and a status word, every role leaves its loop, copies in
 // flight are drained and the tensor memory is freed.
 #include <cuda.h>
@@ -70,10 +74,9 @@ struct Cfg {
     static constexpr int kStages = TN == 64 || (FMT == F_Q6 && TN == 32) ? 4 : 3;
     // activation ring: whole pairs of jobs, so that a barrier of the ring always belongs to the same issuer
     static constexpr int kNB = FMT == F_Q2 ? (TN == 32 ? 8 : 12) : (FMT == F_Q6 || TN == 64 ? 8 : 4);
-    static constexpr int kMin = FMT == F_Q4 ? 2 * 2 * kTM * 16 : 0;              // two buffers of the block-minimum operand
-    static constexpr int kRing = FMT == F_Q2 ? 16 : 4;                           // row scales, per job
-    static constexpr int kScale = FMT == F_Q4 ? 2 : 1;                           // floats per row and job (d, dmin)
-    static constexpr int kSmem = kNB * kUnitBytes + kStages * kStage + kMin + kRing * kTM * kScale * 4;
+    static constexpr int kMin = FMT == F_Q4 ? 2 * 4 * kTM * 16 : 0;              // two buffers of the minimum and the scale operand
+    static constexpr int kRing = FMT == F_Q2 ? 16 : (FMT == F_Q6 ? 4 : 0);       // row scales, per job (Q4_K: read from the raw stage)
+    static constexpr int kSmem = kNB * kUnitBytes + kStages * kStage + kMin + kRing * kTM * 4;
     static constexpr int kEpi = TN == 32 ? 4 : (TN == 128 || FMT == F_Q2 ? 16 : 8);
     static constexpr int kCols = TN / (kEpi / 4);                                // output columns of an epilogue thread
     static constexpr int kChunk = TN == 64 && FMT == F_Q4 ? 16 : 8;                   // columns per tensor-memory load (registers)
@@ -198,22 +201,21 @@ __device__ __forceinline__ uint32_t h2add(uint32_t a, uint32_t b) {
 }
 __device__ __forceinline__ constexpr uint32_t dup(uint32_t h) { return h | (h << 16); }
 // f16 bit patterns of the small constants used below (integers and powers of two)
-constexpr uint32_t H_1024 = 0x6400, H_N1024 = 0xE400, H_N1152 = 0xE480, H_N64 = 0xD400, H_1_16 = 0x2C00, H_1_4 = 0x3400, H_1_64 = 0x2400,
+constexpr uint32_t H_1024 = 0x6400, H_N1024 = 0xE400, H_N1152 = 0xE480, H_64 = 0x5400, H_N72 = 0xD480, H_N8192 = 0xF000, H_1_16 = 0x2C00, H_1_4 = 0x3400, H_1_64 = 0x2400,
                    H_1 = 0x3C00, H_N1032 = 0xE408, H_N1056 = 0xE420, H_N1536 = 0xE600;
 
-// Q4_K: 64 elements = two sub-blocks in 8 words, scales s0 (low nibbles) and s1 (high nibbles).  Operand values leave in
-// the order (0, 2, 1, 3) of every four elements; gemm_tc_prep_kernel lays the activations out the same way.
+// Q4_K: 64 elements = two sub-blocks in 8 words, scales s0 (low nibbles) and s1 (high nibbles); value = (q - 8) * scale.
+// Operand values leave in the order (0, 2, 1, 3) of every four elements; gemm_tc_prep_kernel lays the activations out the same way.
 __device__ __forceinline__ void unpack_q4(const uint32_t *w, uint32_t s0, uint32_t s1, uint32_t (&o)[32]) {
     const uint32_t a0 = h2add(dup(H_1024) | s0 * 0x10001u, dup(H_N1024)), a1 = h2add(dup(H_1024) | s1 * 0x10001u, dup(H_N1024));
-    const uint32_t c0 = h2mul(a0, dup(H_N1024));                             // (1024 + q) * sc - 1024 * sc: one rounding, exact
-    const uint32_t b1 = h2mul(a1, dup(H_1_16)), c1 = h2mul(a1, dup(H_N64));  // (1024 + 16 q) * (sc / 16) - 64 * sc
+    const uint32_t c0 = h2mul(a0, dup(H_N72)), c1 = h2mul(a1, dup(H_N72));  // (64 + q) * sc - 72 * sc: one rounding, exact
 #pragma unroll
     for (int i = 0; i < 8; i++) {
-        const uint32_t v = w[i], u = v >> 8;
-        o[2 * i] = h2fma((v & 0x000F000Fu) | dup(H_1024), a0, c0);
-        o[2 * i + 1] = h2fma((u & 0x000F000Fu) | dup(H_1024), a0, c0);
-        o[16 + 2 * i] = h2fma((v & 0x00F000F0u) | dup(H_1024), b1, c1);
-        o[17 + 2 * i] = h2fma((u & 0x00F000F0u) | dup(H_1024), b1, c1);
+        const uint32_t v = w[i];  // a nibble at bit 4 under the f16 of 64 is 64 + q
+        o[2 * i] = h2fma(((v << 4) & 0x00F000F0u) | dup(H_64), a0, c0);
+        o[2 * i + 1] = h2fma(((v >> 4) & 0x00F000F0u) | dup(H_64), a0, c0);
+        o[16 + 2 * i] = h2fma((v & 0x00F000F0u) | dup(H_64), a1, c1);
+        o[17 + 2 * i] = h2fma(((v >> 8) & 0x00F000F0u) | dup(H_64), a1, c1);
     }
 }
 
@@ -396,8 +398,8 @@ __global__ void __launch_bounds__(Cfg<FMT, TN>::kWarps * 32, Cfg<FMT, TN>::kCtas
     extern __shared__ __align__(1024) uint8_t smem[];
     uint8_t *bring = smem;
     uint8_t *stage0 = bring + K::kNB * K::kUnitBytes;
-    uint8_t *amin = stage0 + K::kStages * K::kStage;                      // [2][2 planes][128][16 B]
-    float *dwring = reinterpret_cast<float *>(amin + K::kMin);            // [kRing][128][kScale]
+    uint8_t *amin = stage0 + K::kStages * K::kStage;                      // [2]{minima, 8 * scales}[2 planes][128][16 B]
+    float *dwring = reinterpret_cast<float *>(amin + K::kMin);            // [kRing][128]
     __shared__ uint64_t bars[K::B_COUNT];
     __shared__ uint32_t tmem_base_s;
     __shared__ int s_dead;
@@ -573,12 +575,15 @@ __global__ void __launch_bounds__(Cfg<FMT, TN>::kWarps * 32, Cfg<FMT, TN>::kCtas
                             }
                             if (!ok) break;
                             if (FMT == F_Q4) {
-                                // (the block-minimum operands are there: their writers arrived on the barriers above, after
+                                // (the minimum and scale operands are there: their writers arrived on the barriers above, after
                                 // the stage that holds the activation side had landed)
+                                if (lane == 0)
+                                    mma_sa(td, mk_desc(su32(amin + (me * 4 + 2) * kTM * 16), kTM * 16),
+                                           mk_desc(su32(stage0 + ls * K::kStage + K::kRaw), TN * 16), idesc, 1u);
                                 if (K::kMBuf == 1 && j >= 1 && !(ok = wait_warp(bar(K::B_MFREE), (uint32_t)((j - 1) & 1), dead))) break;
                                 tc_fence_after();
                                 if (lane == 0)
-                                    mma_sa(tmem + K::kColM + (uint32_t)(K::kMBuf == 2 ? me * TN : 0), mk_desc(su32(amin + me * 2 * kTM * 16), kTM * 16),
+                                    mma_sa(tmem + K::kColM + (uint32_t)(K::kMBuf == 2 ? me * TN : 0), mk_desc(su32(amin + me * 4 * kTM * 16), kTM * 16),
                                            mk_desc(su32(stage0 + ls * K::kStage + K::kRaw), TN * 16), idesc, 0u);
                             }
                             if (lane == 0) mma_commit(bar(K::B_ACCRDY + me));
@@ -643,16 +648,20 @@ __global__ void __launch_bounds__(Cfg<FMT, TN>::kWarps * 32, Cfg<FMT, TN>::kCtas
                         if (!(ok = room(l0))) break;
                         tst32(cols(l0, 0), o);
                         if ((js & 1) == team) {
-                            // block minimum and row scales: the teams take turns; the job before last has been multiplied
+                            // block minima and scales: the teams take turns; the job before last has been multiplied
                             const int s = js & 1;
                             if (js >= 2 && !(ok = wait_warp(bar(K::B_ACCRDY + s), (uint32_t)(((js >> 1) - 1) & 1), dead))) break;
                             const uint32_t n0 = hdr.z & 0x3F3F3F3Fu, n1 = ((hdr.w >> 4) & 0x0F0F0F0Fu) | ((hdr.z >> 2) & 0x30303030u);
+                            const uint32_t c0 = hdr.y & 0x3F3F3F3Fu, c1 = (hdr.w & 0x0F0F0F0Fu) | ((hdr.y >> 2) & 0x30303030u);
                             auto two = [](uint32_t v, uint32_t sel) { return h2add(__byte_perm(v, 0x64646464u, sel), dup(H_N1024)); };
+                            auto two8 = [](uint32_t v, uint32_t sel) { return h2add(__byte_perm(v, 0x70707070u, sel), dup(H_N8192)); };  // 8 v
                             const uint4 p = make_uint4(two(n0, 0x4140), two(n0, 0x4342), two(n1, 0x4140), two(n1, 0x4342));
-                            uint4 *mp = reinterpret_cast<uint4 *>(amin + s * 2 * kTM * 16) + row;
+                            const uint4 e = make_uint4(two8(c0, 0x4140), two8(c0, 0x4342), two8(c1, 0x4140), two8(c1, 0x4342));
+                            uint4 *mp = reinterpret_cast<uint4 *>(amin + s * 4 * kTM * 16) + row;
                             mp[0] = p;
                             mp[kTM] = p;
-                            reinterpret_cast<float2 *>(dwring)[(js % K::kRing) * kTM + row] = make_float2(h2f(hdr.x), h2f(hdr.x >> 16));
+                            mp[2 * kTM] = e;
+                            mp[3 * kTM] = e;
                             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                         }
                         unpack_q4(w + 8, (sc >> 16) & 0xFFu, sc >> 24, o);
@@ -690,7 +699,7 @@ __global__ void __launch_bounds__(Cfg<FMT, TN>::kWarps * 32, Cfg<FMT, TN>::kCtas
                             realign(v, ow, sh, u);
                             scw[0] = team ? u[2] : u[0];
                             scw[1] = team ? u[3] : u[1];
-                            if (team == 0) dwring[(js % K::kRing) * kTM + row] = h2f(u[4]);
+                            if (team == 0) dwring[(js % (K::kRing ? K::kRing : 1)) * kTM + row] = h2f(u[4]);
                         }
                         __syncwarp();
                         if (lane == 0) bar_arrive(bar(K::B_SFREE + ls));
@@ -727,7 +736,7 @@ __global__ void __launch_bounds__(Cfg<FMT, TN>::kWarps * 32, Cfg<FMT, TN>::kCtas
 #pragma unroll
                             for (int i4 = 0; i4 < 4; i4++) c[i4] = (k & 1) ? w[w0 + 1 + i4] : __funnelshift_r(w[w0 + i4], w[w0 + i4 + 1], 16);
                             unpack_q2(c, o);
-                            dwring[((js * K::kUnits + team * K::kTeamUnits + k) % K::kRing) * kTM + row] = h2f(dh);
+                            dwring[((js * K::kUnits + team * K::kTeamUnits + k) % (K::kRing ? K::kRing : 1)) * kTM + row] = h2f(dh);
                             if (!(ok = room(l0 + k))) break;
                             tst32(cols(l0 + k, 0), o);
                             publish(team * K::kTeamUnits + k);
@@ -768,10 +777,10 @@ __global__ void __launch_bounds__(Cfg<FMT, TN>::kWarps * 32, Cfg<FMT, TN>::kCtas
                         const float *d8 = reinterpret_cast<const float *>(ex + (FMT == F_Q4 ? 32 * TN : 0)) + (FMT == F_Q2 ? jj * 2 * TN : 0) + col0;
                         float dw, dm = 0.f;
                         if (FMT == F_Q4) {
-                            const float2 v = reinterpret_cast<const float2 *>(dwring)[(j % K::kRing) * kTM + row];
-                            dw = v.x, dm = v.y;
+                            const uint32_t v = *reinterpret_cast<const uint32_t *>(ex - K::kRaw + row * K::kRowBytes);
+                            dw = h2f(v), dm = h2f(v >> 16);
                         } else {
-                            dw = dwring[(j % K::kRing) * kTM + row];
+                            dw = dwring[(j % (K::kRing ? K::kRing : 1)) * kTM + row];
                         }
                         // the next columns' loads are in flight while these are folded in
                         uint32_t sd[2][K::kChunk], sm[2][K::kChunk];

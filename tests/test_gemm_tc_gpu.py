@@ -74,15 +74,25 @@ def _q6_rows(rng, out_f, in_f):
     return blk.ravel()
 
 
+def _q4_rows(rng, out_f, in_f):
+    """Every scale and minimum 63, codes 12..15: a weight is 756..945 steps, a block of codes near 127 sums to 2.7e7."""
+    blk = rng.integers(0, 256, (out_f * in_f // 256, 144), dtype=np.uint8)
+    blk[:, 0:4] = np.array([0.01, 0.02], np.float16).view(np.uint8)
+    blk[:, 4:16] = 0xFF
+    blk[:, 16:] |= 0xCC
+    return blk.ravel()
+
+
 @pytest.mark.parametrize("m", [20, 40, 100])  # the three token tiles
 @pytest.mark.parametrize("x_of", ["same sign", "halves cancel"])
 def test_gemm_tc_block_sums_beyond_24_bits(tc, oracle, m, x_of):
-    # |block sum|, or what it climbs to half way, is above 2^24: still the CPU's integers, so the bound stays that of f32
+    # |block sum|, or what it climbs to half way, is above 2^24: the CPU converts the integer, here the last addition rounds
+    # (2^-23 of the sum at most), so the bound stays that of f32
     in_f, out_f, rng = 2048, 130, np.random.default_rng(m)
     x = rng.uniform(0.9, 1.0, (m, in_f)).astype(np.float32)
     if x_of == "halves cancel":
         x[:, np.arange(in_f) % 256 >= 128] *= -1.0
-    for dt, w in ((Q6K, _q6_rows(rng, out_f, in_f)),):
+    for dt, w in ((Q4K, _q4_rows(rng, out_f, in_f)), (Q6K, _q6_rows(rng, out_f, in_f))):
         got, want = tc.run_linear(dt, w, x, m, in_f, out_f), oracle.linear(dt, w, x, m, in_f, out_f)
         assert fx.rel_l2(got, want) < TOL
 
