@@ -259,8 +259,8 @@ INFR_API int32_t infr_cuda_gemv_q8(infr_cuda_ctx *ctx, int32_t dtype, const infr
                                    const infr_cuda_buf *qs, const infr_cuda_buf *d, const infr_cuda_buf *sums,
                                    const infr_cuda_buf *sums16, infr_cuda_buf *y, uint32_t m, uint32_t in_f,
                                    uint32_t out_f);
-/* Two weights of one format against the same quantised rows (infr_cuda_gemv_q8 twice, same results): q and k, or gate
- * and up, of a decode step.  The reference gets the same effect from `w_off` slices of one fused weight
+/* Two weights of one format against the same quantised rows (infr_cuda_gemv_q8 twice; for at most 24 rows the same bits,
+ * above equal up to the order of f32 sums, see infr_cuda_linear_pair): q and k, or gate and up, of a decode step.  The reference gets the same effect from `w_off` slices of one fused weight
  * (crates/infr-llama/src/seam/runner.rs:3445-3461, :3842-3879); here the two weights may live anywhere, and Q4_K
  * pairs run as ONE launch (a decode step pays a fixed few microseconds per dependent launch). */
 INFR_API int32_t infr_cuda_gemv_q8_pair(infr_cuda_ctx *ctx, int32_t dtype, const infr_cuda_buf *w1, uint64_t w_off1, infr_cuda_buf *y1,
@@ -296,9 +296,12 @@ INFR_API int32_t infr_cuda_linear(infr_cuda_ctx *ctx, int32_t dtype, const infr_
                                   const infr_cuda_buf *x, infr_cuda_buf *y, uint32_t m, uint32_t in_f,
                                   uint32_t out_f, int32_t act);
 
-/* Two Op::Linear of one weight format on the same rows (q and k, gate and up), results as from two infr_cuda_linear
- * calls: the rows are quantised once (and laid out once for the prefill GEMM); for at most 8 rows of Q4_K the two
- * products are one launch.  infr_cuda_execute pairs neighbouring Linear ops of a graph the same way. */
+/* Two Op::Linear of one weight format on the same rows (q and k, gate and up): the rows are quantised once (and laid out
+ * once for the prefill GEMM), and where a kernel takes two weights the two products are one launch.  Results as from two
+ * infr_cuda_linear calls, up to the order of f32 sums: the batched GEMM splits K by the height of both weights together,
+ * and for 25..32 rows of Q4_K that height decides between it and the wide GEMV (up to 24 rows, and with Q2_0 up to 16, the
+ * bits are those of two calls).  infr_cuda_execute pairs neighbouring Linear ops of a graph the same way, so a plan and
+ * direct calls differ by as much. */
 INFR_API int32_t infr_cuda_linear_pair(infr_cuda_ctx *ctx, int32_t dtype, const infr_cuda_buf *w1, uint64_t w_off1, infr_cuda_buf *y1,
                                        uint32_t out_f1, const infr_cuda_buf *w2, uint64_t w_off2, infr_cuda_buf *y2, uint32_t out_f2,
                                        const infr_cuda_buf *x, uint32_t m, uint32_t in_f, int32_t act);

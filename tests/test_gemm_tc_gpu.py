@@ -124,6 +124,43 @@ def test_gemm_tc_two_weights_and_repeat(tc, dt):
     plan.close()
 
 
+@pytest.mark.parametrize("dt,in_f,n1,n2,m", [
+    (Q4K, 4096, 4096, 1024, 24), (Q2_0, 2048, 1000, 256, 16),     # below the line: the bits of two calls
+    (Q4K, 4096, 4096, 1024, 33), (Q4K, 4096, 4096, 1024, 113),    # K splits of 4 and 16 on their own, another together
+    (Q4K, 4096, 8192, 8192, 32),                                  # large together, not each
+    (Q4K, 4096, 12288, 12288, 25), (Q4K, 4096, 12288, 200, 32),   # both large; one of them
+    (Q6K, 2048, 1024, 256, 300), (Q2_0, 2048, 1000, 256, 300),
+])
+def test_a_pair_against_two_calls_and_the_cpu(backend, oracle, dt, in_f, n1, n2, m):
+    be, bb = fx.BLOCK[dt]
+    rows = [synth.weight(dt, 40, in_f, seed=s) for s in (1, 2)]  # the weights repeat with period 40 rows
+    w1, w2 = (backend.from_numpy(np.tile(r, n // 40 + 1)[:n * in_f // be * bb]) for r, n in zip(rows, (n1, n2)))
+    xh = synth.normal(5, (m, in_f))
+    x = backend.from_numpy(xh)
+    want = [oracle.linear(dt, r, xh, m, in_f, 40) for r in rows]
+    y = [backend.alloc(m * n * 4) for n in (n1, n2, n1, n2)]
+
+    def check():
+        single, pair = ([backend.download(b, np.float32).reshape(m, -1) for b in y[i:i + 2]] for i in (0, 2))
+        for s, p, cpu in zip(single, pair, want):
+            if m <= (16 if dt == Q2_0 else 24):
+                np.testing.assert_array_equal(p, s)
+            for got in (s, p):
+                last = got.shape[1] // 40 * 40 - 40
+                assert max(fx.rel_l2(got[:, r:r + 40], cpu) for r in (0, last)) < TOL
+    backend.linear(dt, w1, x, y[0], m, in_f, n1)
+    backend.linear(dt, w2, x, y[1], m, in_f, n2)
+    backend.linear_pair(dt, w1, y[2], n1, w2, y[3], n2, x, m, in_f)
+    check()
+    if dt == Q6K or (dt == Q4K and m <= 32):  # the same from quantised rows
+        q = [backend.alloc(n) for n in (m * in_f, m * in_f // 256 * 4, m * in_f // 32 * 4, m * in_f // 16 * 4)]
+        backend.quantize_q8(256, x, m, in_f, *q)
+        backend.gemv_q8(dt, w1, *q, y[0], m, in_f, n1)
+        backend.gemv_q8(dt, w2, *q, y[1], m, in_f, n2)
+        backend.gemv_q8_pair(dt, w1, y[2], n1, w2, y[3], n2, *q, m, in_f)
+        check()
+
+
 @pytest.mark.parametrize("dt", [Q4K, Q6K, Q2_0])
 @pytest.mark.parametrize("bad", [np.inf, np.nan])
 def test_gemm_tc_non_finite_activations(tc, oracle, dt, bad):
