@@ -255,7 +255,16 @@ Status CudaBackend::gemv_q8_push(infr_cuda_comm *c, int dtype, const uint8_t *w,
     p.rank = c->rank;
     cudaError_t e;
     int n_launch = 1;
-    if (wide) {
+    if (wide && tc_wins(dtype, m, in_f, out_f)) {
+        // the shapes that gemv_q8 gives to the GEMM, so that the bits are gemv_q8's: its result behind the GEMM's own scratch, then pushed
+        const size_t own = tc_scratch_bytes(dtype, m, in_f, out_f);
+        Status s = ensure_scratch(own + (size_t)m * out_f * 4);
+        if (!s.ok()) return s;
+        float *y = reinterpret_cast<float *>(scratch() + own);
+        s = tc_linear(dtype, w, y, out_f, nullptr, nullptr, 0, nullptr, &a, m, in_f);
+        if (!s.ok()) return s;
+        e = launch_push_results(y, (size_t)m * out_f, p, stream_);
+    } else if (wide) {
         // a few dozen rows: the wide GEMV; with several K chunks the kernel that adds them is the one that pushes
         const size_t pb = gemv_wide_partial_bytes((int)m, (int)in_f, (int)out_f);
         Status s = ensure_scratch(pb);

@@ -483,6 +483,20 @@ cudaError_t launch_wide_nt(const CUtensorMap &tmap, const Q8Dev &a, float *y, fl
 
 }  // namespace
 
+// Sends n finished results y to every rank's staging (a GEMV with more than one kernel's worth of partial sums pushes the same way).
+cudaError_t launch_push_results(const float *y, size_t n, const GemvPush &push, cudaStream_t st) {
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)((n + 255) / 256));
+    cfg.blockDim = dim3(256);
+    cfg.stream = st;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, wide_sum_chunks_kernel, y, (float *)nullptr, n, 1, push, (const float *)nullptr, (float *)nullptr, (size_t)0);
+}
+
 // Scratch for the partial results of launch_gemv_wide (0 when K fits one chunk of 2048 elements).
 size_t gemv_wide_partial_bytes(int m, int in_f, int out_f) {
     const int kz = (in_f / 256 + kWWarps - 1) / kWWarps;

@@ -99,6 +99,7 @@ int gemv_wide_launches(int in_f);
 cudaError_t launch_gemv_wide(int dtype, const uint8_t *w, const Q8Dev &a, float *y, float *partials, int m, int in_f, int out_f,
                              const DeviceInfo &dev, uint32_t *status, cudaStream_t st, const GemvPush *push = nullptr, const uint8_t *w2 = nullptr,
                              float *y2 = nullptr, int out_f2 = 0);
+cudaError_t launch_push_results(const float *y, size_t n, const GemvPush &push, cudaStream_t st);
 
 // Prefill GEMM C[m,out_f] = Q8(256) activations x Q4_K weights on tcgen05 (kind::i8, TMEM accumulators);
 // bit-identical to the CPU production path.

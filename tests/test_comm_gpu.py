@@ -86,7 +86,8 @@ def _q8_set(backend, rows, k):
 
 
 @pytest.mark.parametrize("dt,in_f,m", [(Q4K, 2048, 1), (Q4K, 1024, 5), (Q6K, 4096, 1), (Q6K, 2048, 8), (Q4K, 4096, 8),
-                                       (Q4K, 2048, 12), (Q4K, 4096, 32), (Q6K, 6144, 20)])  # 9..32 rows: the wide GEMV, one or several K chunks
+                                       (Q4K, 2048, 12), (Q4K, 4096, 32), (Q6K, 6144, 20),  # 9..32 rows: the wide GEMV, one or several K chunks
+                                       (Q4K, 49152, 25)])  # so many weights that gemv_q8 takes the GEMM
 def test_pushed_gemv_and_pulling_norm_match_gemv_all_reduce_norm(backend, dt, in_f, m):
     """The exchange without a kernel of its own (infr_cuda_gemv_q8_push + infr_cuda_add_rms_norm_q8_pull) on one rank:
     the same bits as gemv_q8 -> all_reduce -> add_rms_norm_q8, several pairs in a row (both parities of the staging),
