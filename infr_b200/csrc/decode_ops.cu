@@ -1026,6 +1026,7 @@ __global__ void __launch_bounds__(256) attn_combine_wide_kernel(const float *__r
                                                                 float *__restrict__ d, int32_t *__restrict__ sums, int32_t *__restrict__ sums16) {
     __shared__ float s_w[4][kCombineMaxSplits];
     __shared__ float s_l[4];
+    __shared__ int s_n[4];
     __shared__ __align__(16) float s_acc[8][256];
     pdl_go();
     pdl_wait();
@@ -1038,18 +1039,18 @@ __global__ void __launch_bounds__(256) attn_combine_wide_kernel(const float *__r
         for (int s = lane; s < n_splits; s += 32) m = fmaxf(m, ml[2 * s]);
         m = warp_max(m);
         float l = 0.f;
+        int n = 0;
         for (int s = lane; s < n_splits; s += 32) {
             const float ls = ml[2 * s + 1];
-            if (ls == 0.f) {
-                s_w[warp][s] = -1.f;  // a tile past the row's causal end
-                continue;
-            }
+            if (ls == 0.f) break;  // past the row's causal end, as all tiles after it (a tile with keys has l >= 1, or NaN)
             const float wgt = expf(ml[2 * s] - m);
             s_w[warp][s] = wgt;
             l += wgt * ls;
+            n = s + 1;
         }
         l = warp_sum(l);
-        if (lane == 0) s_l[warp] = l;
+        n = __reduce_max_sync(0xffffffffu, n);
+        if (lane == 0) s_l[warp] = l, s_n[warp] = n;
     }
     __syncthreads();
 #pragma unroll
@@ -1057,12 +1058,12 @@ __global__ void __launch_bounds__(256) attn_combine_wide_kernel(const float *__r
         const int e = h * 128 + lane * 4, hh = e / head_dim, dim0 = e % head_dim;
         const float *po = part_o + ((size_t)row * n_head + head0 + hh) * n_splits * head_dim + dim0;
         float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+        // (nobody writes the sums of the tiles past the causal end: what an earlier op left there may read as NaN)
+        const int n = s_n[hh];
 #pragma unroll 4
-        for (int s = warp; s < n_splits; s += 8) {
+        for (int s = warp; s < n; s += 8) {
             const float wgt = s_w[hh][s];
-            float4 p = *reinterpret_cast<const float4 *>(po + (size_t)s * head_dim);
-            // nobody wrote that tile's sums: what an earlier op left there may read as NaN, which no weight of 0 would cancel
-            if (wgt < 0.f) p = make_float4(0.f, 0.f, 0.f, 0.f);
+            const float4 p = *reinterpret_cast<const float4 *>(po + (size_t)s * head_dim);
             acc.x = fmaf(wgt, p.x, acc.x), acc.y = fmaf(wgt, p.y, acc.y), acc.z = fmaf(wgt, p.z, acc.z), acc.w = fmaf(wgt, p.w, acc.w);
         }
         *reinterpret_cast<float4 *>(&s_acc[warp][e]) = acc;
