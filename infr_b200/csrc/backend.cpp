@@ -284,11 +284,11 @@ Status CudaBackend::linear(int dtype, const uint8_t *w, const float *x, float *y
     if (m == 0 || out_f == 0) return Status::Ok();
     cudaSetDevice(device_);
     // More than 8 rows with int8 activations.  Q4_K and Q6_K: up to 32 rows (a decode step over that many sequences) take
-    // the wide GEMV, more the tensor-memory GEMM (tc_applies has the measured line); Q2_0: up to 16 rows walk the 8-row GEMV,
-    // more the GEMM.  Rows that the GEMM's tiled copies cannot fetch are walked.  mmq_kernel 1: the bit-identical GEMM for
+    // the wide GEMV, more the tensor-memory GEMM; Q2_0: up to 16 rows walk the 8-row GEMV, more the GEMM (gemv_rows has the
+    // measured lines).  Rows that the GEMM's tiled copies cannot fetch are walked.  mmq_kernel 1: the bit-identical GEMM for
     // Q4_K, 2: the tensor-memory GEMM for every batch above 8 rows, 3: everything through the GEMV 8 rows at a time (the
     // parity tests and the bench compare them).
-    if (wide_applies(dtype, m, in_f, act) && !tc_wins(dtype, m, in_f, out_f)) {
+    if (wide_applies(dtype, m, in_f, out_f, act) && !tc_wins(dtype, m, in_f, out_f)) {
         Q8Dev a;
         uint8_t *partials = nullptr;
         Status s = quantize_for(dtype, x, m, in_f, &a, gemv_wide_partial_bytes(m < 32 ? (int)m : 32, (int)in_f, (int)out_f), &partials);
@@ -303,7 +303,7 @@ Status CudaBackend::linear(int dtype, const uint8_t *w, const float *x, float *y
         if (s.ok()) launches_ += 2;
         return s;
     }
-    if (tc_applies(dtype, m, in_f, act) || (wide_applies(dtype, m, in_f, act) && tc_wins(dtype, m, in_f, out_f)))
+    if (tc_applies(dtype, m, in_f, out_f, act) || (wide_applies(dtype, m, in_f, out_f, act) && tc_wins(dtype, m, in_f, out_f)))
         return tc_linear(dtype, w, y, out_f, nullptr, nullptr, 0, x, nullptr, m, in_f);
     // Decode shapes (m <= 8) run the streaming GEMV; wider batches are walked 8 rows at a time, all rows quantised once.
     Q8Dev a_all{};
@@ -376,9 +376,23 @@ Status CudaBackend::linear(int dtype, const uint8_t *w, const float *x, float *y
     return Status::Ok();
 }
 
-bool CudaBackend::wide_applies(int dtype, uint32_t m, uint32_t in_f, int act) const {
+// Rows up to which a batch takes the GEMVs (Q4_K, Q6_K: the wide one; Q2_0: the 8-row one, walked) where the GEMM could run
+// too; out_f: the height of all weights of the call.  Measured, GEMV / GEMM (us): Q4_K 32 rows 4096 -> 14336 27 / 26, 4096 -> 4096
+// 13 / 17.  Q6_K 32 rows 4096 -> 14336 33 / 41, 33 rows 54 / 41; against few weights a second pass costs less than the GEMM's two
+// other launches: 2048 -> 2048 33 rows 12.1 / 13.6, 48 rows 13.9 / 15.7, 4096 -> 1024 33 rows 15.0 / 16.1, but 4096 -> 512 15.4 / 13.4
+// and 4096 -> 2048 18.8 / 17.7.  Q2_0 16 rows 4096 -> 14336 33 / 45, 17 rows 42 / 45, 24 rows 47 / 45; 8192 -> 28672 24 rows 123 / 160;
+// 14336 -> 4096 17 rows 53 / 46, 2048 -> 8192 17 rows 26 / 19.
+static uint32_t gemv_rows(int dtype, uint32_t in_f, uint64_t out_f) {
+    const uint64_t w = out_f * in_f;
+    if (dtype == DT_Q6K) return 4 * out_f >= in_f && w <= (4u << 20) ? 48 : 32;
+    if (dtype != DT_Q2_0) return 32;
+    if (out_f < 3 * (uint64_t)in_f || w < (48u << 20)) return 16;
+    return w >= (96u << 20) ? 24 : 17;
+}
+
+bool CudaBackend::wide_applies(int dtype, uint32_t m, uint32_t in_f, uint64_t out_f, int act) const {
     if (act != INFR_ACT_INT8 || m <= 8 || gemv_impl_ != 0 || mmq_impl_ != 0 || in_f == 0 || in_f % 256) return false;
-    if (m > 32) return false;  // one pass of the weights; above, the tensor-memory GEMM is faster
+    if (m > gemv_rows(dtype, in_f, out_f)) return false;
     if (dtype == DT_Q4K) return true;
     if (dtype == DT_Q6K) return in_f % 2048 == 0;  // (rows of a whole number of 16-byte units: the TMA stride rule)
     return false;
@@ -405,11 +419,9 @@ Status CudaBackend::wide_gemm(int dtype, const uint8_t *w, const Q8Dev &a, float
     return Status::Ok();
 }
 
-// Measured, 4096 x 14336 (us): Q4_K 32 rows wide GEMV 27 / GEMM 26, 4096 x 4096 13 / 17; Q6_K 32 rows 33 / 45, 64 rows 65 / 39;
-// Q2_0 16 rows walked 32 / GEMM 45, 32 rows 61 / 45.
-bool CudaBackend::tc_applies(int dtype, uint32_t m, uint32_t in_f, int act) const {
+bool CudaBackend::tc_applies(int dtype, uint32_t m, uint32_t in_f, uint64_t out_f, int act) const {
     if (act != INFR_ACT_INT8 || m <= 8 || gemv_impl_ != 0 || (mmq_impl_ != 0 && mmq_impl_ != 2) || !gemm_tc_takes(dtype, (int)in_f)) return false;
-    return mmq_impl_ == 2 || m > (dtype == DT_Q2_0 ? 16u : 32u);
+    return mmq_impl_ == 2 || m > gemv_rows(dtype, in_f, out_f);
 }
 
 // Where the wide GEMV applies too: a batch against enough Q4_K weights that the GEMM's fixed cost (the layout launch and the
@@ -446,7 +458,9 @@ Status CudaBackend::tc_linear(int dtype, const uint8_t *w, float *y, uint32_t ou
 // Two weights of one format against the same f32 rows (q and k, gate and up): the rows are quantised once.
 Status CudaBackend::linear_pair(int dtype, const uint8_t *w1, float *y1, uint32_t out_f1, const uint8_t *w2, float *y2, uint32_t out_f2,
                                 const float *x, uint32_t m, uint32_t in_f, int act) {
-    const bool wide = wide_applies(dtype, m, in_f, act), gemm = wide && tc_wins(dtype, m, in_f, (uint64_t)out_f1 + out_f2);
+    // (Q2_0 rows below the line are walked weight by weight)
+    const uint64_t both = dtype == DT_Q2_0 ? (out_f1 > out_f2 ? out_f1 : out_f2) : (uint64_t)out_f1 + out_f2;
+    const bool wide = wide_applies(dtype, m, in_f, both, act), gemm = wide && tc_wins(dtype, m, in_f, both);
     if (wide && !gemm && out_f1 && out_f2) {
         cudaSetDevice(device_);
         const int mm = m < 32 ? (int)m : 32;
@@ -455,7 +469,7 @@ Status CudaBackend::linear_pair(int dtype, const uint8_t *w1, float *y1, uint32_
         Status s = quantize_for(dtype, x, m, in_f, &a, gemv_wide_partial_bytes(mm, (int)in_f, (int)(out_f1 + out_f2)), &partials);
         return s.ok() ? wide_gemm(dtype, w1, a, y1, m, in_f, out_f1, reinterpret_cast<float *>(partials), w2, y2, out_f2) : s;
     }
-    if ((gemm || tc_applies(dtype, m, in_f, act)) && out_f1 && out_f2) {
+    if ((gemm || tc_applies(dtype, m, in_f, both, act)) && out_f1 && out_f2) {
         cudaSetDevice(device_);
         return tc_linear(dtype, w1, y1, out_f1, w2, y2, out_f2, x, nullptr, m, in_f);
     }
@@ -484,9 +498,9 @@ Status CudaBackend::linear_pair(int dtype, const uint8_t *w1, float *y1, uint32_
 Status CudaBackend::gemv_q8(int dtype, const uint8_t *w, const Q8Dev &a, float *y, uint32_t m, uint32_t in_f, uint32_t out_f) {
     if (dtype != DT_Q4K && dtype != DT_Q6K && dtype != DT_Q2_0)
         return Status::Err(INFR_E_UNSUPPORTED, fmt("gemv_q8: weight dtype code %d", dtype));
-    const bool wide = m > 8 && wide_applies(dtype, m, in_f, INFR_ACT_INT8);
-    // (Q6_K rows above what the wide GEMV takes in one pass: the tensor-memory GEMM)
-    const bool tc = dtype == DT_Q6K && mmq_impl_ == 0 && tc_applies(dtype, m, in_f, INFR_ACT_INT8);
+    const bool wide = m > 8 && wide_applies(dtype, m, in_f, out_f, INFR_ACT_INT8);
+    // (Q6_K rows above what the wide GEMV takes: the tensor-memory GEMM)
+    const bool tc = dtype == DT_Q6K && mmq_impl_ == 0 && tc_applies(dtype, m, in_f, out_f, INFR_ACT_INT8);
     if (m == 0 || (m > 8 && !wide && !tc))
         return Status::Err(INFR_E_INVALID, fmt("gemv_q8: m=%u (1..8; more rows where the wide GEMV applies: Q4_K up to 32, Q6_K with in_f a multiple of 2048)", m));
     if (in_f == 0 || in_f % (uint32_t)block_elems(dtype) || in_f % 16) return Status::Err(INFR_E_INVALID, fmt("gemv_q8: in_f=%u", in_f));
@@ -518,7 +532,7 @@ Status CudaBackend::gemv_q8_pair(int dtype, const uint8_t *w1, float *y1, uint32
         if (s.ok()) launches_++;
         return s;
     }
-    if (m > 8 && m <= 32 && out_f1 && out_f2 && wide_applies(dtype, m, in_f, INFR_ACT_INT8) && a.gran == 256 && (dtype != DT_Q6K || a.sums16)) {
+    if (m > 8 && m <= 32 && out_f1 && out_f2 && wide_applies(dtype, m, in_f, (uint64_t)out_f1 + out_f2, INFR_ACT_INT8) && a.gran == 256 && (dtype != DT_Q6K || a.sums16)) {
         if (tc_wins(dtype, m, in_f, (uint64_t)out_f1 + out_f2)) {
             cudaSetDevice(device_);
             return tc_linear(dtype, w1, y1, out_f1, w2, y2, out_f2, nullptr, &a, m, in_f);

@@ -235,7 +235,7 @@ Status CudaBackend::gemv_q8_push(infr_cuda_comm *c, int dtype, const uint8_t *w,
     if (!c) return Status::Err(INFR_E_INVALID, "gemv_q8_push: null comm");
     if (!c->connected) return Status::Err(INFR_E_INVALID, "gemv_q8_push: the peers' buffers are not connected");
     if (c->pushed) return Status::Err(INFR_E_INVALID, "gemv_q8_push: the previous pushed result has not been consumed (rms_norm_q8_pull)");
-    const bool wide = m > 8 && m <= 32 && wide_applies(dtype, m, in_f, INFR_ACT_INT8);
+    const bool wide = m > 8 && m <= 32 && wide_applies(dtype, m, in_f, out_f, INFR_ACT_INT8);
     if (m < 1 || (m > 8 && !wide))
         return Status::Err(INFR_E_INVALID, fmt("gemv_q8_push: m=%u (1..8; up to 32 where the wide GEMV applies)", m));
     if ((uint64_t)m * out_f > c->push_cap)

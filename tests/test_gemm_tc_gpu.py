@@ -161,6 +161,23 @@ def test_a_pair_against_two_calls_and_the_cpu(backend, oracle, dt, in_f, n1, n2,
         check()
 
 
+@pytest.mark.parametrize("dt,in_f,out_f,rows", [
+    (Q6K, 2048, 2048, (33, 48, 49)), (Q6K, 2048, 2080, (33,)), (Q6K, 4096, 1000, (33,)),  # two passes of the wide GEMV, or the GEMM
+    (Q2_0, 4096, 12320, (16, 17, 18)), (Q2_0, 4096, 24600, (24, 25)),                   # the 8-row GEMV walked, or the GEMM
+])
+def test_batches_at_the_lines_between_kernels(backend, oracle, dt, in_f, out_f, rows):
+    be, bb = fx.BLOCK[dt]
+    part = synth.weight(dt, 40, in_f, seed=1)  # the weights repeat with period 40 rows
+    w = backend.from_numpy(np.tile(part, out_f // 40 + 1)[:out_f * in_f // be * bb])
+    for m in rows:
+        x = synth.normal(m, (m, in_f))
+        y = backend.alloc(m * out_f * 4)
+        backend.linear(dt, w, backend.from_numpy(x), y, m, in_f, out_f)
+        got, want = backend.download(y, np.float32).reshape(m, out_f), oracle.linear(dt, part, x, m, in_f, 40)
+        for r in (0, out_f // 40 * 40 - 40):
+            assert fx.rel_l2(got[:, r:r + 40], want) < TOL
+
+
 @pytest.mark.parametrize("dt", [Q4K, Q6K, Q2_0])
 @pytest.mark.parametrize("bad", [np.inf, np.nan])
 def test_gemm_tc_non_finite_activations(tc, oracle, dt, bad):
