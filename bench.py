@@ -217,8 +217,18 @@ def _int8_peak(be):
             "how": "tcgen05.mma kind::i8 M=128 N=256 K=32 from resident shared-memory operands, 2 issuers per SM, CUDA events"}
 
 
-def _mmq_case(be, infr_b200, m, in_f, out_f, seed, steps, warmup, peak=None):
-    """Prefill MMQ (Linear with m > 8): int8 TOPS = 2*m*in_f*out_f / time; the activation quantiser is inside."""
+def _f16_peak():
+    """Dense 16-bit tensor rate (a bf16 GEMM; f16 runs at the same rate), TFLOP/s, burst."""
+    p = os.path.join(ROOT, "MEASURED_PEAKS.json")
+    try:
+        with open(p) as f:
+            return float(json.load(f)["bf16_tflops"]), "measured (cuBLAS bf16 GEMM, burst)"
+    except (OSError, KeyError, ValueError):
+        return 1590.0, "fallback"
+
+
+def _mmq_case(be, infr_b200, m, in_f, out_f, seed, steps, warmup):
+    """Prefill MMQ (Linear with m > 8): TOPS = 2*m*in_f*out_f / time; the activation quantiser is inside."""
     from infr_b200 import synth
 
     w = synth.weight(infr_b200.Q4K, out_f, in_f, seed)
@@ -234,14 +244,13 @@ def _mmq_case(be, infr_b200, m, in_f, out_f, seed, steps, warmup, peak=None):
     ms = be.timer_stop()
     ops = 2.0 * m * in_f * out_f
     tops = ops * steps / (ms * 1e-3) / 1e12
-    res = {"workload": f"prefill MMQ q4_k M={m} K={in_f} N={out_f} (quantise + tcgen05 kind::i8 GEMM)",
-           "int8_ops": ops, "us": ms * 1e3 / steps, "tops": tops, "frac_of_4500_tops_spec": tops / 4500.0}
-    if peak:
-        # algorithmic ops 2*M*K*N; the kernel issues twice that on the tensor cores (the 6-bit sub-block scale is
-        # split into two int8 operands so that the int32 block sums stay exact) plus the tf32 min term
-        res["roofline"] = {"bound": "int8", "achieved": tops, "peak": peak["burst_tops"], "unit": "TOPS", "frac": tops / peak["burst_tops"],
-                           "peak_source": "measured (infr_cuda_tensor_peak_i8, burst)", "peak_spec": 4500.0,
-                           "alg_ops_per_launch": ops, "kernel": "gemm_tc_prep_kernel + gemm_tc_kernel"}
+    res = {"workload": f"prefill MMQ q4_k M={m} K={in_f} N={out_f} (quantise + tcgen05 kind::f16 GEMM)",
+           "ops": ops, "us": ms * 1e3 / steps, "tops": tops}
+    # algorithmic ops 2*M*K*N; the kernel multiplies each weight once, as an f16 integer, and adds two K = 16 instructions per
+    # 256-element block (minima, scales)
+    peak, source = _f16_peak()
+    res["roofline"] = {"bound": "f16", "achieved": tops, "peak": peak, "unit": "TFLOP/s", "frac": tops / peak, "peak_source": source,
+                       "peak_spec": 2250.0, "alg_ops_per_launch": ops, "kernel": "gemm_tc_prep_kernel + gemm_tc_kernel"}
     for b in (wb, xb, yb):
         b.close()
     return res
@@ -845,12 +854,12 @@ def _ep_moe(be, infr_b200, dist, rank, world, local, steps, warmup):
             "us_per_layer": us, "mode": mode, "scaling": "strong", "parity": parity}
 
 
-def _mmq_sharded(be, infr_b200, dist, rank, world, steps, warmup, peak_tops=None):
+def _mmq_sharded(be, infr_b200, dist, rank, world, steps, warmup):
     """The prefill configuration (M = 512 tokens, K = 4096, N = 14336 Q4_K rows) split by output rows over the ranks
     (the column-parallel half of the reference's tensor-parallel lowering, crates/infr-llama/src/seam/mod.rs:2711-2798):
     rank r multiplies the same 512 activation rows, quantised redundantly on every rank, with rows
     [r * 14336 / N, (r + 1) * 14336 / N) of one seeded weight.  No collective: a consumer of the full result would
-    all-gather.  Reports per-GPU and aggregate int8 TOPS; rank 0 checks its shard against the unsharded product."""
+    all-gather.  Reports per-GPU and aggregate TOPS; rank 0 checks its shard against the unsharded product."""
     from infr_b200 import shard, synth
 
     m, in_f, out_f = 512, 4096, 14336
@@ -885,9 +894,8 @@ def _mmq_sharded(be, infr_b200, dist, rank, world, steps, warmup, peak_tops=None
     agg = 2.0 * m * in_f * out_f / (us * 1e-6) / 1e12
     res = {"workload": f"prefill MMQ q4_k M={m} K={in_f} N={out_f} split by output rows over {world} GPU(s) ({cnt} rows on rank 0), "
                        f"activations quantised on every rank, no collective",
-           "us": us, "aggregate_tops": agg, "per_gpu_tops": agg / world, "scaling": "strong", "parity": parity}
-    if peak_tops:
-        res["per_gpu_frac_of_measured_int8_peak"] = agg / world / peak_tops
+           "us": us, "aggregate_tops": agg, "per_gpu_tops": agg / world, "scaling": "strong", "parity": parity,
+           "per_gpu_frac_of_f16_peak": agg / world / _f16_peak()[0]}
     for b in (wb, xb, yb):
         b.close()
     return res
@@ -1044,14 +1052,13 @@ def run_b200(args):
                 sweep.append(_gemv_case(be, infr_b200, dtype, o, i_, m, seed, sw_steps, 5, caps.l2_bytes, hbm_peak))
         out["sweep"] = sweep
         out["int8_peak"] = _int8_peak(be)
-        out["mmq"] = _mmq_case(be, infr_b200, 512, 4096, 14336, 5, 20, 3, out["int8_peak"])
+        out["mmq"] = _mmq_case(be, infr_b200, 512, 4096, 14336, 5, 20, 3)
         out["moe"] = _moe_case(be, infr_b200, 20, 3, hbm_peak)
         out["decode_linears"] = [_decode_linears_case(be, infr_b200, b, 10, 3) for b in (1, 32)]
         out["decode_step"] = [_decode_step_case(be, infr_b200, b, 10, 3, hbm_peak) for b in (1, 32)]
 
     if not args.no_sweep:
-        peak_tops = out["int8_peak"]["burst_tops"] if "int8_peak" in out else _int8_peak(be)["burst_tops"]
-        mq = _mmq_sharded(be, infr_b200, dist, rank, world, 20, 3, peak_tops)
+        mq = _mmq_sharded(be, infr_b200, dist, rank, world, 20, 3)
         if rank == 0:
             out["mmq_sharded"] = mq
         tp = _tp_decode(be, infr_b200, dist, rank, world, local, 10, 3)

@@ -73,7 +73,8 @@ typedef struct infr_cuda_graph infr_cuda_graph;
  * so that the parity tests can reach every kernel of the library on every shape:
  *   gemv_kernel 1: the direct-load byte-dot GEMV for all formats and batches;
  *   mmq_kernel  1: the Q4_K prefill GEMM whose f32 output is bit-identical to the CPU's (slower),
- *               2: the grouped tensor-memory GEMM also for MoE layers with a handful of rows per expert,
+ *               2: the tensor-memory GEMM for every batch above 8 rows that it can fetch, also for MoE layers with a handful
+ *                  of rows per expert,
  *               3: no GEMM: batches of more than 8 rows are walked through the GEMV 8 rows at a time. */
 typedef struct {
     int32_t device;
@@ -114,7 +115,9 @@ INFR_API int32_t infr_cuda_alloc_uninit(infr_cuda_ctx *ctx, size_t bytes, int32_
  * never leave the backend's own padded allocations, and must not leave the caller's either). */
 INFR_API int32_t infr_cuda_wrap(infr_cuda_ctx *ctx, void *device_ptr, size_t bytes, int32_t usage, infr_cuda_buf **out);
 /* The CUDA stream (cudaStream_t as void*) the context enqueues all its work on, so that a caller can order
- * its own kernels and collectives with the context's without a device-wide synchronise. */
+ * its own kernels and collectives with the context's without a device-wide synchronise.  Activations a caller's kernel
+ * writes are waited for.  Weights are fetched before that wait (they do not change between launches): a caller's kernel
+ * that writes a weight on this stream must not release its dependents early (griddepcontrol.launch_dependents). */
 INFR_API void *infr_cuda_stream(infr_cuda_ctx *ctx);
 INFR_API void infr_cuda_free(infr_cuda_ctx *ctx, infr_cuda_buf *buf);
 
