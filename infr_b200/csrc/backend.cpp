@@ -704,14 +704,21 @@ Status CudaBackend::moe_ffn(const MoeArgs &a) {
     const size_t rows = a.rows, ne = a.ne, nff = a.n_ff, nu = a.n_used, nx = a.n_expert;
     const size_t n_pairs = rows * nu;
     const size_t max_items = n_pairs / 8 + nx + 1;
-    // Experts that see a few dozen rows each run on the tensor-memory GEMM in grouped form (one 32-row slab of an
-    // expert's rows per tile column: the expert's weights are unpacked once per slab); with only a handful of rows
-    // per expert the 8-row grouped GEMV does less padded work.  The line, measured on 128 experts, top-8, 2048 -> 768 (us a
-    // layer, items / GEMM): 10 pairs per expert 232 / 246, 11 pairs 263 / 250 (most experts then need a second item), 16 pairs
-    // 334 / 262.
+    // Experts that see a few dozen rows each run on the tensor-memory GEMM in grouped form (one slab of 32 or 64 of an expert's
+    // rows per token tile: the expert's weights are unpacked once per slab); with only a handful of rows per expert the 8-row
+    // grouped GEMV does less padded work.  An expert's load is that of the whole layer, also on a rank that holds some experts.
+    // Measured, us a layer (items / slabs of 32 / of 64), by pairs per expert:
+    //   128 experts, 2048 -> 768   8: 232 / 259 / 296, 12: 266 / 259 / 296, 24: 388 / 292 / 323, 32: 500 / 365 / 337
+    //   32 experts, 4096 -> 1792   8: 243 / 274 / 293, 16: 424 / 268 / 300, 32: 444 / 350 / 314, 64: 841 / 524 / 415
+    //   60 experts, 2048 -> 1536   26: 348 / 243 / 254, 34: 447 / 313 / 266
+    // Where a slab per expert is at most a wave of tiles, so that a tile has an SM to itself either way, 64 rows cost no more:
+    //   8 experts, 4096 -> 2048    8: 242 / 147 / 130, 32: 268 / 169 / 136, 128: 494 / 292 / 260
+    //   16 experts, 2048 -> 1024   8: 117 / 90 / 83, 32: 129 / 110 / 89;  1024 -> 256   8: 51 / 57 / 52, 16: 59 / 59 / 53
     // (a layer with a Q6_K bank takes 8-row items throughout: the GEMM's copies want rows of whole 2048-element chunks)
-    const bool grouped_gemm = !any_q6 && (mmq_impl_ == 2 || (mmq_impl_ == 0 && 2 * n_pairs >= (size_t)21 * a.n_local));
-    const size_t max_slabs = n_pairs / kGemmTcSlab + a.n_local + 1;
+    const bool one_wave = (size_t)a.n_local * ((nff + 127) / 128) <= (size_t)dev_.sm_count;
+    const bool grouped_gemm = !any_q6 && (mmq_impl_ == 2 || (mmq_impl_ == 0 && 2 * n_pairs >= (size_t)(one_wave ? 16 : 21) * nx));
+    const int slab = one_wave || n_pairs >= 28 * nx ? 64 : 32;
+    const size_t max_slabs = n_pairs / slab + a.n_local + 1;
     // scratch carve-up (all 256-byte aligned)
     size_t off = 0;
     auto take = [&](size_t bytes) {
@@ -727,8 +734,8 @@ Status CudaBackend::moe_ffn(const MoeArgs &a) {
     const size_t o_g = take(n_pairs * nff * 4), o_u = take(n_pairs * nff * 4);
     const size_t o_aq = take(n_pairs * nff), o_ad = take(n_pairs * (nff / 256) * 4), o_as = take(n_pairs * (nff / 32) * 4);
     const size_t o_y = take(n_pairs * ne * 4);
-    const size_t o_px = grouped_gemm ? take(gemm_tc_grouped_record_bytes(DT_Q4K, (int)max_slabs, (int)ne)) : 0;
-    const size_t o_pa = grouped_gemm ? take(gemm_tc_grouped_record_bytes(DT_Q4K, (int)max_slabs, (int)nff)) : 0;
+    const size_t o_px = grouped_gemm ? take(gemm_tc_grouped_record_bytes(slab, (int)max_slabs, (int)ne)) : 0;
+    const size_t o_pa = grouped_gemm ? take(gemm_tc_grouped_record_bytes(slab, (int)max_slabs, (int)nff)) : 0;
     Status s = ensure_scratch(off);
     if (!s.ok()) return s;
     uint8_t *b = scratch();
@@ -754,7 +761,7 @@ Status CudaBackend::moe_ffn(const MoeArgs &a) {
     } while (0)
     INFR_STEP(launch_moe_router(a.router, a.router_x, logits, (int)rows, (int)ne, (int)nx, stream_), "moe router");
     INFR_STEP(launch_moe_route(logits, (int)rows, (int)nx, (int)nu, a.scale, a.norm_w, ids, w, stream_), "moe route");
-    INFR_STEP(launch_moe_bucket(ids, (int)rows, (int)nu, (int)nx, (int)a.expert_lo, (int)a.n_local, grouped_gemm ? kGemmTcSlab : 8, prow, pslot, ie, ip, ic, ni,
+    INFR_STEP(launch_moe_bucket(ids, (int)rows, (int)nu, (int)nx, (int)a.expert_lo, (int)a.n_local, grouped_gemm ? slab : 8, prow, pslot, ie, ip, ic, ni,
                                 nullptr, stream_),
               "moe bucket");
     // stage A: every distinct row quantised once (lib.rs:2688-2718)
@@ -771,10 +778,10 @@ Status CudaBackend::moe_ffn(const MoeArgs &a) {
         // stage B: both banks read the same gathered activation planes (laid out once); stage C; stage D on the
         // re-quantised pairs; stage E
         auto layout = [&](const Q8Dev &acts, uint8_t *rec, uint32_t k, const int32_t *rows_of) {
-            return launch_gemm_tc_grouped_prep(DT_Q4K, acts, rec, (int)k, ie, ip, ic, ni, rows_of, (int)max_slabs, stream_);
+            return launch_gemm_tc_grouped_prep(slab, acts, rec, (int)k, ie, ip, ic, ni, rows_of, (int)max_slabs, stream_);
         };
         auto gemm = [&](const uint8_t *bank, const uint8_t *rec, float *out, uint32_t k, uint32_t o) {
-            return launch_gemm_tc_grouped(DT_Q4K, bank, (int)a.n_local, rec, out, (int)k, (int)o, ie, ip, ic, ni, (int)max_slabs, dev_, status_dev_, stream_);
+            return launch_gemm_tc_grouped(slab, bank, (int)a.n_local, rec, out, (int)k, (int)o, ie, ip, ic, ni, (int)max_slabs, dev_, status_dev_, stream_);
         };
         INFR_STEP(layout(xa, b + o_px, (uint32_t)ne, prow), "moe layout x");
         INFR_STEP(gemm(a.gate, b + o_px, g, (uint32_t)ne, (uint32_t)nff), "moe gate (grouped gemm)");

@@ -1021,32 +1021,30 @@ cudaError_t launch_gemm_tc(int dtype, const uint8_t *w, const void *records, flo
     return v4 ? launch_sum<float4>(partials, c, n1, p2, c2, n2, kz, st) : launch_sum<float>(partials, c, n1, p2, c2, n2, kz, st);
 }
 
-// Grouped form over a bank of n_experts matrices; slabs of up to kGemmTcSlab rows (work items of moe_bucket_kernel).
-size_t gemm_tc_grouped_record_bytes(int dtype, int max_slabs, int in_f) {
-    const int f = fmt_of(dtype), n = max_slabs * kGemmTcSlab;
-    return units_bytes(f, n, in_f) + extra_bytes(f, n, in_f);
+// Grouped form over a bank of n_experts Q4_K matrices; slabs of up to `slab` rows (work items of moe_bucket_kernel).
+size_t gemm_tc_grouped_record_bytes(int slab, int max_slabs, int in_f) {
+    const int n = max_slabs * slab;
+    return units_bytes(F_Q4, n, in_f) + extra_bytes(F_Q4, n, in_f);
 }
-cudaError_t launch_gemm_tc_grouped_prep(int dtype, const Q8Dev &a, void *records, int in_f, const int *slab_expert, const int *slab_p0,
+cudaError_t launch_gemm_tc_grouped_prep(int slab, const Q8Dev &a, void *records, int in_f, const int *slab_expert, const int *slab_p0,
                                         const int *slab_cnt, const int *n_slabs, const int *pair_row, int max_slabs, cudaStream_t st) {
-    if (!gemm_tc_takes(dtype, in_f) || max_slabs < 1) return cudaErrorInvalidValue;
-    const int f = fmt_of(dtype), n = max_slabs * kGemmTcSlab;
-    uint8_t *u = static_cast<uint8_t *>(records), *e = u + units_bytes(f, n, in_f);
-    return launch_prep<false>(f, nullptr, a, n, kGemmTcSlab, in_f, u, e, n, TcGroup{slab_expert, slab_p0, slab_cnt, n_slabs, pair_row}, st);
+    if (!gemm_tc_takes(DT_Q4K, in_f) || max_slabs < 1) return cudaErrorInvalidValue;
+    const int n = max_slabs * slab;
+    uint8_t *u = static_cast<uint8_t *>(records), *e = u + units_bytes(F_Q4, n, in_f);
+    return launch_prep<false>(F_Q4, nullptr, a, n, slab, in_f, u, e, n, TcGroup{slab_expert, slab_p0, slab_cnt, n_slabs, pair_row}, st);
 }
-cudaError_t launch_gemm_tc_grouped(int dtype, const uint8_t *bank, int n_experts, const void *records, float *y, int in_f, int out_f,
+cudaError_t launch_gemm_tc_grouped(int slab, const uint8_t *bank, int n_experts, const void *records, float *y, int in_f, int out_f,
                                    const int *slab_expert, const int *slab_p0, const int *slab_cnt, const int *n_slabs, int max_slabs,
                                    const DeviceInfo &dev, uint32_t *status, cudaStream_t st) {
-    if (!gemm_tc_takes(dtype, in_f) || out_f < 1 || max_slabs < 1 || n_experts < 1) return cudaErrorInvalidValue;
-    const int f = fmt_of(dtype), n = max_slabs * kGemmTcSlab;
-    const uint8_t *u = static_cast<const uint8_t *>(records), *e = u + units_bytes(f, n, in_f);
+    if (!gemm_tc_takes(DT_Q4K, in_f) || out_f < 1 || max_slabs < 1 || n_experts < 1 || (slab != 32 && slab != 64)) return cudaErrorInvalidValue;
+    const int n = max_slabs * slab;
+    const uint8_t *u = static_cast<const uint8_t *>(records), *e = u + units_bytes(F_Q4, n, in_f);
     CUtensorMap mw;
-    if (!weight_map(f, bank, (size_t)n_experts * out_f, in_f, &mw)) return cudaErrorInvalidValue;
+    if (!weight_map(F_Q4, bank, (size_t)n_experts * out_f, in_f, &mw)) return cudaErrorInvalidValue;
     TcGroup g{slab_expert, slab_p0, slab_cnt, n_slabs, nullptr};
     TcMat m1{y, out_f}, m2{nullptr, 0};
-    const int tiles = ((out_f + kTM - 1) / kTM) * max_slabs, cap = ctas_of(f, kGemmTcSlab, dev), grid = tiles < cap ? tiles : cap;
-    if (f == F_Q2) return cudaErrorInvalidValue;  // (no 32-token form; no caller has Q2_0 banks)
-    if (f == F_Q4) return launch_tn<F_Q4>(kGemmTcSlab, mw, mw, u, e, m1, m2, n, in_f, status, g, 1, grid, st);
-    return launch_tn<F_Q6>(kGemmTcSlab, mw, mw, u, e, m1, m2, n, in_f, status, g, 1, grid, st);
+    const int tiles = ((out_f + kTM - 1) / kTM) * max_slabs, cap = ctas_of(F_Q4, slab, dev), grid = tiles < cap ? tiles : cap;
+    return launch_tn<F_Q4>(slab, mw, mw, u, e, m1, m2, n, in_f, status, g, 1, grid, st);
 }
 
 }  // namespace infr

@@ -121,13 +121,12 @@ size_t gemm_tc_partial_bytes(int dtype, int m, int in_f, int out_f, const Device
 cudaError_t launch_gemm_tc_prep(int dtype, const float *x, const Q8Dev *a, void *records, int m, int in_f, cudaStream_t st);
 cudaError_t launch_gemm_tc(int dtype, const uint8_t *w, const void *records, float *c, float *partials, int m, int in_f, int out_f, const DeviceInfo &dev,
                            uint32_t *status, cudaStream_t st, const uint8_t *w2 = nullptr, float *c2 = nullptr, int out_f2 = 0);
-// The same over a bank of expert matrices, one slab of up to kGemmTcSlab routed rows per token tile; `a` quantised rows,
-// gathered through pair_row when it is non-null.
-constexpr int kGemmTcSlab = 32;
-size_t gemm_tc_grouped_record_bytes(int dtype, int max_slabs, int in_f);
-cudaError_t launch_gemm_tc_grouped_prep(int dtype, const Q8Dev &a, void *records, int in_f, const int *slab_expert, const int *slab_p0,
+// The same over a bank of Q4_K expert matrices, one slab of up to `slab` (32, 64) routed rows of an expert per token tile; `a`
+// quantised rows, gathered through pair_row when it is non-null.
+size_t gemm_tc_grouped_record_bytes(int slab, int max_slabs, int in_f);
+cudaError_t launch_gemm_tc_grouped_prep(int slab, const Q8Dev &a, void *records, int in_f, const int *slab_expert, const int *slab_p0,
                                         const int *slab_cnt, const int *n_slabs, const int *pair_row, int max_slabs, cudaStream_t st);
-cudaError_t launch_gemm_tc_grouped(int dtype, const uint8_t *bank, int n_experts, const void *records, float *y, int in_f, int out_f,
+cudaError_t launch_gemm_tc_grouped(int slab, const uint8_t *bank, int n_experts, const void *records, float *y, int in_f, int out_f,
                                    const int *slab_expert, const int *slab_p0, const int *slab_cnt, const int *n_slabs, int max_slabs,
                                    const DeviceInfo &dev, uint32_t *status, cudaStream_t st);
 // Grouped Q4_K GEMM over a bank of n_experts matrices [out_f, in_f] stored back to back: work item i

@@ -236,3 +236,32 @@ def test_expert_parallel_slices_add_up_to_the_whole_layer(backend):
     assert fx.rel_l2(thirds, whole) < 1e-5
     with pytest.raises(infr_b200.BackendError):
         run(6, 3)  # leaves [0, n_expert)
+
+
+def test_a_rank_takes_the_form_of_the_whole_layer(backend):
+    """Two pairs per expert: 8-row items for the whole layer, and for a rank that holds an eighth of the experts, although
+    all pairs divided by its own experts would be sixteen."""
+    rows, ne, nx, nu, nff = 32, 256, 128, 8, 256
+    gate, up, down = _banks(nx, nff, ne, seed=500)
+    xb, rb = backend.from_numpy(synth.normal(5, (rows, ne))), backend.from_numpy(synth.normal(6, (nx, ne), 1.0 / np.sqrt(ne)))
+    dst, launches = backend.alloc(rows * ne * 4), []
+    for n in (nx, nx // 8):
+        banks = [backend.from_numpy(b[:b.nbytes // nx * n], infr_b200.USAGE_WEIGHTS) for b in (gate, up, down)]
+        before = backend.launch_count()
+        backend.moe_ffn(xb, xb, rb, *banks, dst, rows=rows, ne=ne, n_expert=nx, n_used=nu, n_ff_exp=nff, expert_lo=0, n_local=n)
+        launches.append(backend.launch_count() - before)
+        backend.sync()
+    assert launches[0] == launches[1]
+
+
+@pytest.mark.parametrize("nx,nu,rows", [(2, 2, 63), (2, 2, 64), (2, 2, 65), (2, 2, 129), (5, 2, 200), (160, 8, 560)])
+def test_moe_slab_edges(backend, oracle, nx, nu, rows):
+    """Every expert sees every row (63..129 rows: the edges of 64-row slabs), or a ragged number; many experts: 28 pairs each."""
+    ne, nff = 512, 256
+    gate, up, down = _banks(nx, nff, ne, seed=700)
+    router, x = synth.normal(7, (nx, ne), 1.0 / np.sqrt(ne)), synth.normal(8, (rows, ne))
+    got = _run(backend, x, router, gate, up, down, rows, ne, nx, nu, nff)[0]
+    want = oracle.moe_ffn(x, router, gate, up, down, rows=rows, ne=ne, n_expert=nx, n_used=nu, n_ff_exp=nff)[0]
+    # between the GEMMs values are coded in 8 bits: an f32 rounding can move a code by one
+    assert fx.rel_l2(got, want) < 1e-3
+    assert max(fx.rel_l2(got[r], want[r]) for r in range(rows)) < 1e-2
