@@ -69,11 +69,11 @@ struct Cfg {
     static constexpr int kStage = kRaw + kExtra;
     // Tensor-memory room for groups, per team.  Each team of unpack warps owns its own: a team that shared one with another
     // could find its barrier two phases behind, which a parity wait cannot tell from "done".
-    static constexpr int kTeamSlots = FMT == F_Q2 ? (TN == 32 ? 2 : 4) : (FMT == F_Q4 && TN != 64 ? 1 : 2);
+    static constexpr int kTeamSlots = FMT == F_Q2 ? 4 : (FMT == F_Q4 && TN != 64 ? 1 : 2);
     static constexpr int kSlots = kTeams * kTeamSlots;
     static constexpr int kStages = TN == 64 || (FMT == F_Q6 && TN == 32) ? 4 : 3;
     // activation ring: whole pairs of jobs, so that a barrier of the ring always belongs to the same issuer
-    static constexpr int kNB = FMT == F_Q2 ? (TN == 32 ? 8 : 12) : (FMT == F_Q6 || TN == 64 ? 8 : 4);
+    static constexpr int kNB = FMT == F_Q2 ? 12 : (FMT == F_Q6 || TN == 64 ? 8 : 4);
     static constexpr int kMin = FMT == F_Q4 ? 2 * 4 * kTM * 16 : 0;              // two buffers of the minimum and the scale operand
     static constexpr int kRing = FMT == F_Q2 ? 16 : (FMT == F_Q6 ? 4 : 0);       // row scales, per job (Q4_K: read from the raw stage)
     static constexpr int kSmem = kNB * kUnitBytes + kStages * kStage + kMin + kRing * kTM * 4;
@@ -93,6 +93,7 @@ struct Cfg {
     static constexpr int B_SFULL = 0, B_SFREE = B_SFULL + kStages, B_BFULL = B_SFREE + kStages, B_BFREE = B_BFULL + kNB,
                          B_AREADY = B_BFREE + kNB, B_AFREE = B_AREADY + kReady, B_ACCRDY = B_AFREE + kSlots, B_ACCFREE = B_ACCRDY + 2,
                          B_MFREE = B_ACCFREE + 2, B_DRAIN = B_MFREE + 1, B_COUNT = B_DRAIN + 2;
+    static_assert(FMT != F_Q2 || TN == 64, "Q2_0 has one token tile");
     static_assert(kCols0 <= 512 && (kCtas == 1 || kCols0 <= 256), "tensor memory");
     static_assert(kSmem <= (kCtas == 2 ? 112 : 225) * 1024, "shared memory");
     static_assert(kNB % (2 * kGroups) == 0 && kWarps <= 32, "");
@@ -306,8 +307,8 @@ __global__ void __launch_bounds__(256) gemm_tc_prep_kernel(const float *__restri
                                                            uint8_t *__restrict__ extra, int n_tok, TcGroup grp) {
     pdl_go();
     pdl_wait();
-    using C32 = Cfg<FMT, 32>;
-    constexpr int UPS = C32::kUnits, UB = C32::kUnitBytes / 32, EB = C32::kExtra / 32, STK = C32::kStageK;
+    using C64 = Cfg<FMT, 64>;
+    constexpr int UPS = C64::kUnits, UB = C64::kUnitBytes / 64, EB = C64::kExtra / 64, STK = C64::kStageK;  // (per token: the same for every tile)
     const int lane = threadIdx.x & 31, nb = in_f >> 8, nst = in_f / STK;
     const long long wg = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (wg >= (long long)n_tok * nb) return;
@@ -498,7 +499,7 @@ __global__ void __launch_bounds__(Cfg<FMT, TN>::kWarps * 32, Cfg<FMT, TN>::kCtas
             }
             if (*dead) {
                 // copies in flight land before the CTA's shared memory is released
-                for (int k = js > K::kStages ? js - K::kStages : 0; k <= js; k++)
+                for (int k = js > K::kStages ? js - K::kStages : 0; k <= js || k < pre; k++)
                     for (uint32_t i = 0; i < (1u << 14) && !try_bar(bar(K::B_SFULL + k % K::kStages), (uint32_t)((k / K::kStages) & 1)); i++) {
                     }
                 for (int k = ju > K::kNB ? ju - K::kNB : 0; k < ju; k++)
