@@ -40,7 +40,8 @@ CASES = [
     (Q6K, 32, 4096, 1024),
     (Q6K, 32, 14336, 4096),  # the Q6_K FFN down of the Q4_K_M mix
     (Q6K, 31, 4096, 1000),   # odd row count of the matrix: the last tile is partial
-    (Q6K, 80, 2048, 72),     # three passes (no Q6_K GEMM exists: every batch above 8 rows comes here)
+    (Q6K, 48, 2048, 720),    # few weights: two passes
+    (Q6K, 80, 2048, 72),     # the tensor-memory GEMM
 ]
 
 
