@@ -28,7 +28,8 @@
 // (108, 34 and 25 without the centred codes and their correction);  Q6_K 14336 ->
 // 4096, 113 rows 125 -> 57, 512 rows 520 -> 179 (54 and 171 with one accumulator, whose sums round above 2^24; 60 and 192 with
 // two accumulators drained by 8 warps);  Q2_0 14336 -> 4096, 77 rows 201 -> 78.
-// What bounds it: at 128 tokens a Q4_K job takes ~2800 cycles where its MMAs take 1100; the epilogue (D and M: 128 KB per job
+// What bounds it (clock64 traces of the roles, taken before the block's second K = 16 instruction and Q6_K's second accumulator): at
+// 128 tokens a Q4_K job takes ~2800 cycles where its MMAs take 1100; the epilogue (D and M: 128 KB per job
 // out of tensor memory, busy 2100 of them) is the slowest role, 8 or 16 warps alike.  Q6_K: the unpack warps (~3700 cycles per
 // block and warp) and, at 128 tokens, the drain between two blocks (one set of accumulators fits).  Q2_0: the epilogue,
 // one drain per 64 elements (~1000 cycles).
