@@ -13,6 +13,9 @@
 // weights.  Measured (hidden 2048, 128 experts, top-8, 768 wide): seven launches of the general path 61 us (three GEMVs of 11.6 us,
 // whose lanes read activations 64 bytes apart: 16-way bank conflicts; a router on 8 CTAs 11.6 us), these three 24 us: router 4, gate
 // and up 11, down 7.
+//
+// Only the weights are const __restrict__ (pdl.cuh): the ids were, and the down kernel's load of them went above its wait.  Wherever the
+// gate / up launch left SMs idle, so that the next one was resident beside it, it took whatever the scratch held.
 #include "kernels.h"
 #include "pdl.cuh"
 
@@ -50,7 +53,7 @@ __device__ __forceinline__ float hf(uint32_t bits) { return __half2float(__ushor
 // ---- router: warp = expert, its groups of eight lanes a row each.  The rows go to shared memory in one round trip; eight lanes replay
 // the CPU's accumulators.  (Row pitch ne + 8: the four groups on disjoint banks.)
 constexpr int kRtWarps = 4, kRtRowsCta = 4;
-__global__ void __launch_bounds__(kRtWarps * 32) moe_router_row_kernel(const float *__restrict__ router, const float *__restrict__ x, float *__restrict__ logits,
+__global__ void __launch_bounds__(kRtWarps * 32) moe_router_row_kernel(const float *__restrict__ router, const float *x, float *__restrict__ logits,
                                                                        int rows, int ne, int n_expert) {
     extern __shared__ __align__(16) float s_rt[];  // [the experts' rows][rows][ne + 8]
     pdl_go();
@@ -85,7 +88,7 @@ static_assert(kRtRowsCta == kRtWarps, "a warp stages one expert row and one acti
 // ---- routing of one row by one warp: moe_route_kernel's operations in the same order.  EPL: experts of a lane (e = lane + 32 i),
 // in registers.  p: [32 EPL] floats of shared memory, for the sum in index order.
 template <int EPL>
-__device__ __forceinline__ void moe_route_row(const float *__restrict__ logits, float *p, int n_expert, int n_used, float scale, int norm_w, int lane, int &id,
+__device__ __forceinline__ void moe_route_row(const float *logits, float *p, int n_expert, int n_used, float scale, int norm_w, int lane, int &id,
                                               float &weight) {
     float v[EPL], mx = -INFINITY;
 #pragma unroll
@@ -153,7 +156,7 @@ __device__ __forceinline__ void moe_route_row(const float *__restrict__ logits, 
 // u * 4 + t holds elements 2u, 2u + 1 of both: (lo, hi, lo, hi).  Blocks are 64 bytes more than their kilobyte apart: the two blocks of
 // eight lanes' 16-byte reads lie on different banks.
 constexpr int kBlockPitch = 68;  // float4
-__device__ __forceinline__ void stage_block_pairs(const float *__restrict__ x, float4 *s, int n, int tid, int nthr) {
+__device__ __forceinline__ void stage_block_pairs(const float *x, float4 *s, int n, int tid, int nthr) {
     for (int i = tid; i < n / 4; i += nthr) {
         const int b = i >> 6, r = i & 63, u = r >> 2, t = r & 3;
         const float *src = x + b * 256 + t * 64 + 2 * u;
@@ -211,7 +214,7 @@ __device__ __forceinline__ void block_dot(const Piece (&w)[N], const float4 *s_x
 
 // Gate and up of every selected expert, SiLU.  Task = (rank, FFN row); a warp's four-lane group g takes blocks g, g + 8, ...
 constexpr int kEpl = 4;  // up to 128 experts
-__global__ void __launch_bounds__(kRowThreads, 1) moe_gate_up_row_kernel(const float *__restrict__ logits, const float *__restrict__ x, const uint8_t *__restrict__ gate,
+__global__ void __launch_bounds__(kRowThreads, 1) moe_gate_up_row_kernel(const float *logits, const float *x, const uint8_t *__restrict__ gate,
                                                                         const uint8_t *__restrict__ up, float *__restrict__ act, int32_t *__restrict__ sel_ids,
                                                                         float *__restrict__ sel_w, int ne, int nff, int n_expert, int n_used, float scale, int norm_w) {
     extern __shared__ __align__(16) float4 s_x[];  // [ne / 256][kBlockPitch]
@@ -266,8 +269,8 @@ __global__ void __launch_bounds__(kRowThreads, 1) moe_gate_up_row_kernel(const f
 // Down of every selected expert and the weighted sum in rank order.  Warp = output row; its eight groups of four lanes take 8 / P ranks
 // at a time, P groups a rank's blocks.  (CTAs of 256 threads and 64 registers find room beside the launch before, but spill: 31 us a layer
 // for 24.)
-__global__ void __launch_bounds__(kRowThreads, 1) moe_down_row_kernel(const uint8_t *__restrict__ down, const float *__restrict__ act, const int32_t *__restrict__ sel_ids,
-                                                                      const float *__restrict__ sel_w, float *__restrict__ dst, int ne, int nff, int n_used, int P) {
+__global__ void __launch_bounds__(kRowThreads, 1) moe_down_row_kernel(const uint8_t *__restrict__ down, const float *act, const int32_t *sel_ids,
+                                                                      const float *sel_w, float *__restrict__ dst, int ne, int nff, int n_used, int P) {
     extern __shared__ __align__(16) float4 s_x[];  // [n_used][nff / 256][kBlockPitch]
     __shared__ int s_id[32];
     __shared__ float s_w[32];

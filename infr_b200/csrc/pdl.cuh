@@ -3,6 +3,9 @@
 // exited), and must call pdl_wait before it touches anything the previous kernel wrote.  Every kernel launched this
 // way calls pdl_wait in all of its threads before any of them can exit, so that "the previous kernel has completed"
 // carries through a chain of such launches.
+// What an earlier kernel of the stream writes is not passed as a `const T *__restrict__` parameter: that says that nothing changes it while
+// this kernel runs, which is not so, and the compiler moves such a load above pdl_wait (the memory clobber holds ordinary loads only).
+// Weights may be const __restrict__.
 #pragma once
 #include <cuda_runtime.h>
 

@@ -54,3 +54,28 @@ def test_moe_row_ties_and_nan(be, oracle):
     _, ids, w, _ = _run(be, x, router, gate, up, down, 1, ne, n_expert, n_used, nff)
     np.testing.assert_array_equal(ids.ravel(), np.arange(n_used))
     assert np.isnan(w).all()
+
+
+def test_moe_row_takes_the_ids_of_its_own_call(be, oracle):
+    # Layers whose gate / up launch leaves SMs idle, so that the down launch is resident while the row is being routed, and ids that change
+    # from call to call: neither the ids of the call before nor what the caller's buffer held may be used.
+    ne, n_expert, n_used, nff, calls = 512, 60, 4, 256, 24
+    gate, up, down = _banks(n_expert, nff, ne, seed=4)
+    router = synth.normal(17, (n_expert, ne), 1.0 / np.sqrt(ne))
+    x = synth.normal(5, (calls, ne))
+    rb, gb, ub, db = (be.from_numpy(a) for a in (router, gate, up, down))
+    xs, ys = [be.from_numpy(x[i:i + 1]) for i in range(calls)], [be.alloc(ne * 4) for _ in range(calls)]
+    ids, w = be.from_numpy(np.zeros(n_used, np.int32)), be.from_numpy(np.zeros(n_used, np.float32))
+    args = dict(rows=1, ne=ne, n_expert=n_expert, n_used=n_used, n_ff_exp=nff)
+    for own in (False, True):
+        be.sync()
+        for xb, yb in zip(xs, ys):
+            if own:  # one call at a time
+                be.upload(ids, np.zeros(n_used, np.int32))
+                be.upload(w, np.zeros(n_used, np.float32))
+                be.sync()
+            be.moe_ffn(xb, xb, rb, gb, ub, db, yb, **args, **(dict(sel_ids=ids, sel_w=w) if own else {}))
+        for i, yb in enumerate(ys):
+            want = oracle.moe_ffn(x[i:i + 1], router, gate, up, down, **args)[0].ravel()
+            assert np.abs(be.download(yb, np.float32) - want).max() / np.abs(want).max() < 1e-5
+            be.upload(yb, np.zeros(ne, np.float32))
