@@ -94,7 +94,7 @@ __device__ __forceinline__ void rope_pair(float a, float b, float ang, float *oa
 }
 
 // thread = (row, head, pair or pass-through element)
-__global__ void __launch_bounds__(256) rope_kernel(const float *__restrict__ x, const int32_t *__restrict__ positions,
+__global__ void __launch_bounds__(256) rope_kernel(const float *x, const int32_t *positions,
                                                    float *__restrict__ dst, int rows, int n_head, int head_dim, int rope_dim,
                                                    float theta, int neox) {
     pdl_go();
@@ -126,11 +126,11 @@ __global__ void __launch_bounds__(256) rope_kernel(const float *__restrict__ x, 
 // row positions[r].  Full-head rotation only (rope_dim == head_dim).
 constexpr int kRopeTable = 128;  // frequencies a block keeps
 constexpr int kPageRows = 128;  // rows of a page of a paged KV cache = keys of an attention tile
-__global__ void __launch_bounds__(256) rope_write_kv_kernel(float *__restrict__ q, const float *__restrict__ k, const float *__restrict__ v,
-                                                            const int32_t *__restrict__ positions, __half *__restrict__ k_cache,
+__global__ void __launch_bounds__(256) rope_write_kv_kernel(float *__restrict__ q, const float *k, const float *v,
+                                                            const int32_t *positions, __half *__restrict__ k_cache,
                                                             __half *__restrict__ v_cache, int rows, int n_head, int n_kv, int head_dim,
                                                             float theta, int neox, int rows_per_seq, size_t seq_stride, int write_pos,
-                                                            const int32_t *__restrict__ block_table, int table_stride, int n_pages) {
+                                                            const int32_t *block_table, int table_stride, int n_pages) {
     // The frequencies (f64 powers) depend on nothing before: a block forms each once, before the wait.  (Longer heads: one by one.)
     __shared__ float s_freq[kRopeTable];
     pdl_go();
@@ -183,7 +183,7 @@ __global__ void __launch_bounds__(256) rope_write_kv_kernel(float *__restrict__ 
     }
 }
 
-__global__ void __launch_bounds__(256) write_kv_kernel(const float *__restrict__ src, __half *__restrict__ cache, size_t n) {
+__global__ void __launch_bounds__(256) write_kv_kernel(const float *src, __half *__restrict__ cache, size_t n) {
     pdl_go();
     pdl_wait();
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
@@ -276,11 +276,11 @@ constexpr int kAttnChunkPairs = 16;   // (query row, head) pairs of a chunk's ti
 constexpr int kAttnChunkStride = 136;  // floats between pairs of 128 values: four pairs read 8 words each from distinct banks
 
 template <int HD, int G, bool BULK>
-__global__ void __launch_bounds__(kAttnThreads) attn_split_kernel(const float *__restrict__ q, const __half *__restrict__ k_cache,
-                                                               const __half *__restrict__ v_cache, float *__restrict__ part_o,
+__global__ void __launch_bounds__(kAttnThreads) attn_split_kernel(const float *q, const __half *k_cache,
+                                                               const __half *v_cache, float *__restrict__ part_o,
                                                                float *__restrict__ part_ml, int rows, int n_head, int n_kv, int pos,
                                                                float scale, int n_splits, size_t seq_stride, uint32_t *__restrict__ status,
-                                                               const int32_t *__restrict__ seq_pos, const int32_t *__restrict__ block_table,
+                                                               const int32_t *seq_pos, const int32_t *block_table,
                                                                int table_stride, int n_pages) {
     constexpr int CPR = HD * 2 / 16;           // 16-byte pieces per row
     constexpr int NT = (2 * G + 7) / 8;        // 8-column groups of the instruction: column c = head c / 2, piece c % 2
@@ -524,11 +524,11 @@ __global__ void __launch_bounds__(kAttnThreads) attn_split_kernel(const float *_
 // Measured (113 rows at position 384, 32 heads / 8): 51 -> 45 us a layer; one CTA per row was bound by its 64 KB tile and its
 // three barriers per row.
 template <int G>
-__global__ void __launch_bounds__(kAttnThreads) attn_chunk_kernel(const float *__restrict__ q, const __half *__restrict__ k_cache,
-                                                                  const __half *__restrict__ v_cache, float *__restrict__ part_o,
+__global__ void __launch_bounds__(kAttnThreads) attn_chunk_kernel(const float *q, const __half *k_cache,
+                                                                  const __half *v_cache, float *__restrict__ part_o,
                                                                   float *__restrict__ part_ml, int rows, int n_head, int n_kv, int pos, float scale,
                                                                   int n_splits, size_t seq_stride, uint32_t *__restrict__ status,
-                                                                  const int32_t *__restrict__ seq_pos, const int32_t *__restrict__ block_table,
+                                                                  const int32_t *seq_pos, const int32_t *block_table,
                                                                   int table_stride, int n_pages) {
     constexpr int HD = 128, P = kAttnChunkPairs, SP = kAttnChunkStride, R = P / G, CPR = HD * 2 / 16, NT = 2 * P / 8, NT1 = (2 * G + 7) / 8;
     using L = AttnSmem<HD>;
@@ -706,7 +706,7 @@ __global__ void __launch_bounds__(kAttnThreads) attn_chunk_kernel(const float *_
 }
 
 // CTA = (query row, head), thread = output dim: merges the tiles' (m, l, o).
-__global__ void attn_combine_kernel(const float *__restrict__ part_o, const float *__restrict__ part_ml, float *__restrict__ dst,
+__global__ void attn_combine_kernel(const float *part_o, const float *part_ml, float *__restrict__ dst,
                                     int head_dim, int n_splits) {
     pdl_go();
     pdl_wait();
@@ -726,7 +726,7 @@ __global__ void attn_combine_kernel(const float *__restrict__ part_o, const floa
 }
 
 // ---------------------------------------------------------------------------------------------- elementwise
-__global__ void __launch_bounds__(256) gated_silu_kernel(const float *__restrict__ gate, const float *__restrict__ up,
+__global__ void __launch_bounds__(256) gated_silu_kernel(const float *gate, const float *up,
                                                          float *__restrict__ dst, size_t n) {
     pdl_go();
     pdl_wait();
@@ -736,7 +736,7 @@ __global__ void __launch_bounds__(256) gated_silu_kernel(const float *__restrict
     }
 }
 
-__global__ void __launch_bounds__(256) add_kernel(const float *__restrict__ a, const float *__restrict__ b, float *__restrict__ dst, size_t n) {
+__global__ void __launch_bounds__(256) add_kernel(const float *a, const float *b, float *__restrict__ dst, size_t n) {
     pdl_go();
     pdl_wait();
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) dst[i] = a[i] + b[i];
@@ -770,7 +770,7 @@ __device__ __forceinline__ void argmax_block(float bv, uint32_t bi, float *s_v, 
     }
 }
 
-__global__ void __launch_bounds__(256) argmax_stage1_kernel(const float *__restrict__ x, float *__restrict__ cand_v,
+__global__ void __launch_bounds__(256) argmax_stage1_kernel(const float *x, float *__restrict__ cand_v,
                                                             uint32_t *__restrict__ cand_i, uint32_t n, uint32_t chunk) {
     __shared__ float s_v[32];
     __shared__ uint32_t s_i[32];
@@ -784,7 +784,7 @@ __global__ void __launch_bounds__(256) argmax_stage1_kernel(const float *__restr
     argmax_block(bv, bi, s_v, s_i, cand_v + (size_t)blockIdx.y * gridDim.x + blockIdx.x, cand_i + (size_t)blockIdx.y * gridDim.x + blockIdx.x);
 }
 
-__global__ void __launch_bounds__(256) argmax_stage2_kernel(const float *__restrict__ cand_v, const uint32_t *__restrict__ cand_i,
+__global__ void __launch_bounds__(256) argmax_stage2_kernel(const float *cand_v, const uint32_t *cand_i,
                                                             uint32_t *__restrict__ dst, uint32_t n_chunks) {
     __shared__ float s_v[32];
     __shared__ uint32_t s_i[32];
@@ -1002,7 +1002,7 @@ __global__ void __launch_bounds__(1024) rms_norm_q8_pull_kernel(const float *a, 
 }
 
 // silu(gate) * up straight to int8: warp = (row, 256-element block); nff % 256 == 0.
-__global__ void __launch_bounds__(256) gated_silu_q8_kernel(const float *__restrict__ gate, const float *__restrict__ up, int rows, int nff,
+__global__ void __launch_bounds__(256) gated_silu_q8_kernel(const float *gate, const float *up, int rows, int nff,
                                                             int8_t *__restrict__ qs, float *__restrict__ d, int32_t *__restrict__ sums,
                                                             int32_t *__restrict__ sums16) {
     pdl_go();
@@ -1029,7 +1029,7 @@ __global__ void __launch_bounds__(256) gated_silu_q8_kernel(const float *__restr
 // With Q8 false the same sums are stored as f32 instead, so the two forms agree bit for bit.
 constexpr int kCombineMaxSplits = 512;
 template <bool Q8>
-__global__ void __launch_bounds__(256) attn_combine_wide_kernel(const float *__restrict__ part_o, const float *__restrict__ part_ml, int n_head,
+__global__ void __launch_bounds__(256) attn_combine_wide_kernel(const float *part_o, const float *part_ml, int n_head,
                                                                 int head_dim, int n_splits, float *__restrict__ dst, int8_t *__restrict__ qs,
                                                                 float *__restrict__ d, int32_t *__restrict__ sums, int32_t *__restrict__ sums16) {
     __shared__ float s_w[4][kCombineMaxSplits];

@@ -102,7 +102,7 @@ constexpr int record_bytes(int nt) { return nt * 576; }
 
 // One warp per (token, 256 elements); lane l owns elements [8l, 8l + 8) = lane t = l % 4 of group l / 4.  Quantises per 32 with
 // the operations of quantize.cu in the same order (crates/infr-cpu/src/quant.rs:97-117).  Tokens past the last one are zero.
-__global__ void __launch_bounds__(256) gemm_q2_prep_kernel(const float *__restrict__ x, int m, int nt, int in_f, uint8_t *__restrict__ act, int n_tok) {
+__global__ void __launch_bounds__(256) gemm_q2_prep_kernel(const float *x, int m, int nt, int in_f, uint8_t *__restrict__ act, int n_tok) {
     pdl_go();
     pdl_wait();
     const int lane = threadIdx.x & 31, nc = (in_f + 255) >> 8, nb = in_f >> 6;
@@ -140,7 +140,7 @@ struct Q2Mat {
 
 // NTW: groups of 8 tokens of a warp.  KH: the two halves of the warps share the blocks, else the tokens.
 template <int NTW, bool KH>
-__global__ void __launch_bounds__(kThreadsQ2, 1) gemm_q2_kernel(Q2Mat m1, Q2Mat m2, const uint8_t *__restrict__ act, int m, int nb, int kz,
+__global__ void __launch_bounds__(kThreadsQ2, 1) gemm_q2_kernel(Q2Mat m1, Q2Mat m2, const uint8_t *act, int m, int nb, int kz,
                                                                 uint32_t *__restrict__ status) {
     constexpr int NT = KH ? NTW : 2 * NTW, kRaw = kRowsCta * kRowPitch, kRec = record_bytes(NT), kAct = kHalfBlk * kRec, kSums = 4 * NTW;
     extern __shared__ __align__(128) uint8_t smem[];
@@ -337,7 +337,7 @@ __device__ __forceinline__ void add_to(float &a, float v) { a += v; }
 // y[i] = part[0][i] + part[1][i] + ... in split order (the same bits on every run), for two results.  V = float4, or float
 // where a result's size is not a multiple of four or its address not 16-byte aligned.
 template <typename V>
-__global__ void __launch_bounds__(256) gemm_q2_sum_kernel(const V *__restrict__ part, V *__restrict__ y, size_t n1, const V *__restrict__ part2,
+__global__ void __launch_bounds__(256) gemm_q2_sum_kernel(const V *part, V *__restrict__ y, size_t n1, const V *part2,
                                                           V *__restrict__ y2, size_t n2, int kz) {
     pdl_go();
     pdl_wait();

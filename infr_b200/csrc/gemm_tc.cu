@@ -323,7 +323,7 @@ namespace {
 // F32: quantises f32 rows (quantize_q8, crates/infr-cpu/src/quant.rs:27-58: the operations of quantize.cu in the same order);
 // otherwise re-lays rows that are already quantised.  Slots past the last token are zero.
 template <int FMT, bool F32>
-__global__ void __launch_bounds__(256) gemm_tc_prep_kernel(const float *__restrict__ x, Q8Dev a, int m, int tn, int in_f, uint8_t *__restrict__ units,
+__global__ void __launch_bounds__(256) gemm_tc_prep_kernel(const float *x, Q8Dev a, int m, int tn, int in_f, uint8_t *__restrict__ units,
                                                            uint8_t *__restrict__ extra, int n_tok, TcGroup grp) {
     pdl_go();
     pdl_wait();
@@ -400,8 +400,8 @@ __global__ void __launch_bounds__(256) gemm_tc_prep_kernel(const float *__restri
 
 template <int FMT, int TN>
 __global__ void __launch_bounds__(Cfg<FMT, TN>::kWarps * 32, Cfg<FMT, TN>::kCtas)
-    gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_w2, const uint8_t *__restrict__ units,
-                   const uint8_t *__restrict__ extra, TcMat m1, TcMat m2, int m, int in_f, uint32_t *__restrict__ status, TcGroup grp, TcSplit split) {
+    gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_w2, const uint8_t *units,
+                   const uint8_t *extra, TcMat m1, TcMat m2, int m, int in_f, uint32_t *__restrict__ status, TcGroup grp, TcSplit split) {
     using K = Cfg<FMT, TN>;
     extern __shared__ __align__(1024) uint8_t smem[];
     uint8_t *bring = smem;

@@ -184,7 +184,7 @@ __device__ __forceinline__ void quant_items(const float4 (&pa)[4], const float4 
 template <int M, bool FUSED, int KW, int SB, bool PUSH>
 __global__ void __launch_bounds__(KW * 32, 16 / KW)
     gemv_q4k_mma_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ MmaSecond sec, Q8Dev a,
-                        const float *__restrict__ x, float *__restrict__ y, int m, int in_f, int out_f, MmaGeom geo, MmaGroup grp,
+                        const float *x, float *__restrict__ y, int m, int in_f, int out_f, MmaGeom geo, MmaGroup grp,
                         uint32_t *__restrict__ status, const __grid_constant__ typename PushParam<PUSH>::type push) {
     constexpr int kW = KW, kThreadsMma = KW * 32, kStepBlocks = SB, kSlotBytes = kTileRows * SB * 144;
     extern __shared__ __align__(128) uint8_t smem[];

@@ -360,9 +360,9 @@ __device__ __forceinline__ void block_q6_any(const uint8_t *p0, const uint8_t *p
 
 // Shared memory: tiles [warps][2][16 rows]; staged activations [8][nb][352] and scales [nb][8] as in the kernel above; barriers [warps][2].
 __global__ void __launch_bounds__(256) gemv_q6_mma_grouped_kernel(const uint8_t *__restrict__ bank, Q8Dev a, float *__restrict__ y, int in_f, int out_f,
-                                                                  const int *__restrict__ item_expert, const int *__restrict__ item_p0,
-                                                                  const int *__restrict__ item_cnt, const int *__restrict__ n_items,
-                                                                  const int *__restrict__ pair_row, uint32_t *__restrict__ status) {
+                                                                  const int *item_expert, const int *item_p0,
+                                                                  const int *item_cnt, const int *n_items,
+                                                                  const int *pair_row, uint32_t *__restrict__ status) {
     extern __shared__ __align__(128) uint8_t smem[];
     const int nb = in_f >> 8, row_bytes = nb * 210, tile_bytes = kRows6 * row_bytes, kw = blockDim.x >> 5;
     uint8_t *s_act = smem + (size_t)kw * 2 * tile_bytes;

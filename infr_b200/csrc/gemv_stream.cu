@@ -252,7 +252,7 @@ struct StreamSecond {
 // (A token of an 8B ternary model: 161 quantiser launches of 2.1 us and 64 GEMV launches less, 3.81 -> 3.40 ms with the same bits.)
 template <int DT, int M, bool FUSED>
 __global__ void __launch_bounds__(kStreamThreads, (M <= 2 ? 2 : 1))
-    gemv_stream_kernel(const uint8_t *__restrict__ W, Q8Dev a, const float *__restrict__ x, float *__restrict__ y, int m, int in_f, int out_f,
+    gemv_stream_kernel(const uint8_t *__restrict__ W, Q8Dev a, const float *x, float *__restrict__ y, int m, int in_f, int out_f,
                        StreamGeom geo, StreamSecond sec, uint32_t *__restrict__ status) {
     using F = Fmt<DT>;
     extern __shared__ __align__(128) uint8_t smem[];

@@ -389,8 +389,8 @@ __global__ void __launch_bounds__(kWWarps * 32, 1)
 // y[i] = part[0][i] + part[1][i] + ... in chunk order (the same bits on every run).
 // With push.world != 0 the sums go to the peers' staging instead (GemvPush).
 // A second set of partial results (part2, n2 elements each) is added into y2 by the threads behind the first n.
-__global__ void wide_sum_chunks_kernel(const float *__restrict__ part, float *__restrict__ y, size_t n, int kz, const __grid_constant__ GemvPush push,
-                                       const float *__restrict__ part2, float *__restrict__ y2, size_t n2) {
+__global__ void wide_sum_chunks_kernel(const float *part, float *__restrict__ y, size_t n, int kz, const __grid_constant__ GemvPush push,
+                                       const float *part2, float *__restrict__ y2, size_t n2) {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n + n2) return;

@@ -27,7 +27,7 @@ namespace infr {
 // What bounds it: one warp a scheduler, whose chain of reads and multiply-adds nothing hides (24 reads a column of eight and block).
 // Measured (128 experts x 2048, 256 rows): 18.5 us; 256 columns at a time through registers, 2 x 2 a group: 19.7.
 constexpr int kRtRows = 8, kRtExperts = 16, kRtK = 512, kRtPitch = kRtK + 4, kRtBuf = (kRtRows + kRtExperts) * kRtPitch;
-__global__ void __launch_bounds__(128) moe_router_kernel(const float *__restrict__ router, const float *__restrict__ x,
+__global__ void __launch_bounds__(128) moe_router_kernel(const float *__restrict__ router, const float *x,
                                                          float *__restrict__ logits, int rows, int ne, int n_expert) {
     pdl_go();
     pdl_wait();
@@ -99,7 +99,7 @@ __global__ void __launch_bounds__(128) moe_router_kernel(const float *__restrict
 }
 
 // One warp per row.  n_expert <= 1024.
-__global__ void __launch_bounds__(128) moe_route_kernel(const float *__restrict__ logits, int rows, int n_expert, int n_used,
+__global__ void __launch_bounds__(128) moe_route_kernel(const float *logits, int rows, int n_expert, int n_used,
                                                         float scale, int norm_w, int32_t *__restrict__ sel_ids,
                                                         float *__restrict__ sel_w) {
     pdl_go();
@@ -179,7 +179,7 @@ __global__ void __launch_bounds__(128) moe_route_kernel(const float *__restrict_
 //   pair_row[p], pair_of_slot[r * n_used + rank] = p, item_{expert,p0,cnt}[], n_items
 // Expert parallelism: only experts [e_lo, e_lo + n_local) are listed (item_expert is the index inside this
 // rank's banks); pairs routed elsewhere get pair_of_slot = -1 and contribute nothing to this rank's output.
-__global__ void __launch_bounds__(1024) moe_bucket_kernel(const int32_t *__restrict__ sel_ids, int rows, int n_used, int n_expert,
+__global__ void __launch_bounds__(1024) moe_bucket_kernel(const int32_t *sel_ids, int rows, int n_used, int n_expert,
                                                           int e_lo, int n_local, int item_rows,
                                                           int32_t *__restrict__ pair_row, int32_t *__restrict__ pair_of_slot,
                                                           int32_t *__restrict__ item_expert, int32_t *__restrict__ item_p0,
@@ -282,7 +282,7 @@ __global__ void __launch_bounds__(1024) moe_bucket_kernel(const int32_t *__restr
 }
 
 // One warp per (pair, 256-block): act = silu(gate) * up, then quantize_q8 of that block.
-__global__ void __launch_bounds__(256) moe_swiglu_quant_kernel(const float *__restrict__ gate, const float *__restrict__ up,
+__global__ void __launch_bounds__(256) moe_swiglu_quant_kernel(const float *gate, const float *up,
                                                                int n_pairs, int nff, int8_t *__restrict__ qs, float *__restrict__ d,
                                                                int32_t *__restrict__ sums, int32_t *__restrict__ sums16,
                                                                float *__restrict__ act_out) {
@@ -334,8 +334,8 @@ __global__ void __launch_bounds__(256) moe_swiglu_quant_kernel(const float *__re
 }
 
 // out[r, i] = sum over ranks (in rank order) of w[r, rank] * y[pair_of_slot[r, rank], i].
-__global__ void __launch_bounds__(256) moe_combine_kernel(const float *__restrict__ y_pairs, const int32_t *__restrict__ pair_of_slot,
-                                                          const float *__restrict__ sel_w, int rows, int n_used, int ne,
+__global__ void __launch_bounds__(256) moe_combine_kernel(const float *y_pairs, const int32_t *pair_of_slot,
+                                                          const float *sel_w, int rows, int n_used, int ne,
                                                           float *__restrict__ out) {
     pdl_go();
     pdl_wait();

@@ -26,7 +26,7 @@ __device__ __forceinline__ float amax4(float4 v) {
 __device__ __forceinline__ int q1(float v, float id) { return q8_round_code(v, id); }
 
 template <int GRAN>
-__global__ void __launch_bounds__(256) quantize_q8_kernel(const float *__restrict__ x, int rows, int k,
+__global__ void __launch_bounds__(256) quantize_q8_kernel(const float *x, int rows, int k,
                                                           int8_t *__restrict__ qs, float *__restrict__ d,
                                                           int32_t *__restrict__ sums,
                                                           int32_t *__restrict__ sums16,
