@@ -273,6 +273,10 @@ Status CudaBackend::quantize_for(int dtype, const float *x, uint32_t rows, uint3
     return Status::Ok();
 }
 
+static bool overlap(const float *a, size_t na, const float *b, size_t nb) {
+    return (uintptr_t)a < (uintptr_t)b + nb * 4 && (uintptr_t)b < (uintptr_t)a + na * 4;
+}
+
 Status CudaBackend::linear(int dtype, const uint8_t *w, const float *x, float *y, uint32_t m, uint32_t in_f,
                            uint32_t out_f, int act) {
     if (dtype != DT_Q4K && dtype != DT_Q6K && dtype != DT_Q2_0)
@@ -306,8 +310,10 @@ Status CudaBackend::linear(int dtype, const uint8_t *w, const float *x, float *y
     if (q2_applies(dtype, m, in_f, act)) return q2_linear(w, y, out_f, nullptr, nullptr, 0, x, m, in_f);
     if (tc_applies(dtype, m, in_f, out_f, act) || (wide_applies(dtype, m, in_f, out_f, act) && tc_wins(dtype, m, in_f, out_f)))
         return tc_linear(dtype, w, y, out_f, nullptr, nullptr, 0, x, nullptr, m, in_f);
+    // Kernels that read the f32 rows in every CTA need a result apart from them: in place the rows are quantised first.
+    const bool in_place = overlap(x, (size_t)m * in_f, y, (size_t)m * out_f);
     // One Q2_0 row: quantised inside the GEMV.
-    if (dtype == DT_Q2_0 && m == 1 && act == INFR_ACT_INT8 && gemv_impl_ == 0) {
+    if (dtype == DT_Q2_0 && m == 1 && act == INFR_ACT_INT8 && gemv_impl_ == 0 && !in_place) {
         const cudaError_t e = launch_gemv_q2_row(w, y, (int)out_f, nullptr, nullptr, 0, x, (int)in_f, dev_, status_dev_, stream_);
         if (e == cudaSuccess) launches_++;
         if (e != cudaErrorInvalidValue) return cuda_status(e, "gemv_q2");
@@ -512,7 +518,10 @@ Status CudaBackend::linear_pair(int dtype, const uint8_t *w1, float *y1, uint32_
             if (e != cudaErrorInvalidValue) return cuda_status(e, "linear_pair");
             cudaGetLastError();  // rows too long to stage m of them in one CTA: quantise first, then the pair
         }
-        if (dtype == DT_Q2_0 && m == 1 && gemv_impl_ == 0) {
+        // (in place: quantise first; results that overlap each other: one launch each, in order)
+        const size_t nx = (size_t)m * in_f, n1 = (size_t)m * out_f1, n2 = (size_t)m * out_f2;
+        const bool apart = !overlap(x, nx, y1, n1) && !overlap(x, nx, y2, n2) && !overlap(y1, n1, y2, n2);
+        if (dtype == DT_Q2_0 && m == 1 && gemv_impl_ == 0 && apart) {
             const cudaError_t e = launch_gemv_q2_row(w1, y1, (int)out_f1, w2, y2, (int)out_f2, x, (int)in_f, dev_, status_dev_, stream_);
             if (e == cudaSuccess) launches_++;
             if (e != cudaErrorInvalidValue) return cuda_status(e, "linear_pair");

@@ -1,0 +1,45 @@
+"""A Linear whose result lies over its rows (the op list's contract allows it) reads them all before it writes: vs the CPU restatement,
+with the tolerance of the same call into a buffer of its own."""
+import numpy as np
+import pytest
+
+import fixtures as fx
+import infr_b200
+from infr_b200 import Q2_0, synth
+
+pytestmark = pytest.mark.gpu
+N = 4096  # enough CTAs that some store while others have not begun
+
+
+@pytest.fixture(scope="module")
+def be():
+    b = infr_b200.CudaBackend(device=0)
+    yield b
+    b.close()
+
+
+def _rows(be, m, seed):
+    x = synth.normal(seed, (m, N))
+    return x, be.from_numpy(x)
+
+
+@pytest.mark.parametrize("dt,m", [(Q2_0, 1)])
+def test_linear_in_place(be, oracle, dt, m):
+    w = synth.weight(dt, N, N, seed=1)
+    wb = be.from_numpy(w)
+    for seed in range(4):
+        x, xb = _rows(be, m, seed)
+        be.linear(dt, wb, xb, xb, m, N, N)
+        assert fx.rel_l2(be.download(xb, np.float32).reshape(m, N), oracle.linear(dt, w, x, m, N, N)) < 1e-6
+
+
+@pytest.mark.parametrize("dt,m", [(Q2_0, 1)])
+@pytest.mark.parametrize("first", [True, False])
+def test_pair_with_one_result_over_the_rows(be, oracle, dt, m, first):
+    w1, w2 = synth.weight(dt, N, N, seed=1), synth.weight(dt, N, N, seed=2)
+    b1, b2, other = be.from_numpy(w1), be.from_numpy(w2), be.alloc(m * N * 4)
+    x, xb = _rows(be, m, 9)
+    y1, y2 = (xb, other) if first else (other, xb)
+    be.linear_pair(dt, b1, y1, N, b2, y2, N, xb, m, N)
+    for w, y in ((w1, y1), (w2, y2)):  # both from the rows as they were
+        assert fx.rel_l2(be.download(y, np.float32).reshape(m, N), oracle.linear(dt, w, x, m, N, N)) < 1e-6
