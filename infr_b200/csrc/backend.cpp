@@ -322,7 +322,7 @@ Status CudaBackend::linear(int dtype, const uint8_t *w, const float *x, float *y
     // Decode shapes (m <= 8) run the streaming GEMV; wider batches are walked 8 rows at a time, all rows quantised once.
     Q8Dev a_all{};
     // (a single Q4_K chunk quantises its rows inside the GEMV; with several chunks that would repeat the work in every CTA)
-    const bool pre_quantised = act == INFR_ACT_INT8 && (!(dtype == DT_Q4K && gemv_impl_ == 0) || m > 8);
+    const bool pre_quantised = act == INFR_ACT_INT8 && (!(dtype == DT_Q4K && gemv_impl_ == 0) || m > 8 || in_place);
     if (pre_quantised) {
         Status s = quantize_for(dtype, x, m, in_f, &a_all);
         if (!s.ok()) return s;
@@ -507,7 +507,10 @@ Status CudaBackend::linear_pair(int dtype, const uint8_t *w1, float *y1, uint32_
     if (act == INFR_ACT_INT8 && m >= 1 && m <= 8 && (dtype == DT_Q4K || dtype == DT_Q6K || dtype == DT_Q2_0) && in_f &&
         in_f % (uint32_t)block_elems(dtype) == 0 && in_f % 16 == 0 && out_f1 && out_f2) {
         cudaSetDevice(device_);
-        if (dtype == DT_Q4K && gemv_impl_ == 0 && in_f % 256 == 0) {
+        // (in place: quantise first; results that overlap each other: one launch each, in order)
+        const size_t nx = (size_t)m * in_f, n1 = (size_t)m * out_f1, n2 = (size_t)m * out_f2;
+        const bool apart = !overlap(x, nx, y1, n1) && !overlap(x, nx, y2, n2) && !overlap(y1, n1, y2, n2);
+        if (dtype == DT_Q4K && gemv_impl_ == 0 && in_f % 256 == 0 && apart) {
             // one kernel: the rows are quantised inside the GEMV while the first weights stream in
             const cudaError_t e = launch_gemv_q4k_mma_pair(w1, y1, (int)out_f1, w2, y2, (int)out_f2, nullptr, x, (int)m, (int)in_f, dev_,
                                                            status_dev_, stream_);
@@ -518,9 +521,6 @@ Status CudaBackend::linear_pair(int dtype, const uint8_t *w1, float *y1, uint32_
             if (e != cudaErrorInvalidValue) return cuda_status(e, "linear_pair");
             cudaGetLastError();  // rows too long to stage m of them in one CTA: quantise first, then the pair
         }
-        // (in place: quantise first; results that overlap each other: one launch each, in order)
-        const size_t nx = (size_t)m * in_f, n1 = (size_t)m * out_f1, n2 = (size_t)m * out_f2;
-        const bool apart = !overlap(x, nx, y1, n1) && !overlap(x, nx, y2, n2) && !overlap(y1, n1, y2, n2);
         if (dtype == DT_Q2_0 && m == 1 && gemv_impl_ == 0 && apart) {
             const cudaError_t e = launch_gemv_q2_row(w1, y1, (int)out_f1, w2, y2, (int)out_f2, x, (int)in_f, dev_, status_dev_, stream_);
             if (e == cudaSuccess) launches_++;
@@ -565,7 +565,8 @@ Status CudaBackend::gemv_q8(int dtype, const uint8_t *w, const Q8Dev &a, float *
 
 Status CudaBackend::gemv_q8_pair(int dtype, const uint8_t *w1, float *y1, uint32_t out_f1, const uint8_t *w2, float *y2, uint32_t out_f2,
                                  const Q8Dev &a, uint32_t m, uint32_t in_f) {
-    if (dtype == DT_Q4K && gemv_impl_ == 0 && m >= 1 && m <= 8 && in_f && in_f % 256 == 0 && out_f1 && out_f2 && a.gran == 256) {
+    if (dtype == DT_Q4K && gemv_impl_ == 0 && m >= 1 && m <= 8 && in_f && in_f % 256 == 0 && out_f1 && out_f2 && a.gran == 256 &&
+        !overlap(y1, (size_t)m * out_f1, y2, (size_t)m * out_f2)) {
         cudaSetDevice(device_);
         Status s = cuda_status(launch_gemv_q4k_mma_pair(w1, y1, (int)out_f1, w2, y2, (int)out_f2, &a, nullptr, (int)m, (int)in_f, dev_, status_dev_, stream_),
                                "gemv_q8_pair");

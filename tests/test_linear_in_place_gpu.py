@@ -5,7 +5,7 @@ import pytest
 
 import fixtures as fx
 import infr_b200
-from infr_b200 import Q2_0, synth
+from infr_b200 import Q2_0, Q4K, synth
 
 pytestmark = pytest.mark.gpu
 N = 4096  # enough CTAs that some store while others have not begun
@@ -23,7 +23,7 @@ def _rows(be, m, seed):
     return x, be.from_numpy(x)
 
 
-@pytest.mark.parametrize("dt,m", [(Q2_0, 1)])
+@pytest.mark.parametrize("dt,m", [(Q2_0, 1), (Q4K, 1), (Q4K, 8)])
 def test_linear_in_place(be, oracle, dt, m):
     w = synth.weight(dt, N, N, seed=1)
     wb = be.from_numpy(w)
@@ -33,7 +33,7 @@ def test_linear_in_place(be, oracle, dt, m):
         assert fx.rel_l2(be.download(xb, np.float32).reshape(m, N), oracle.linear(dt, w, x, m, N, N)) < 1e-6
 
 
-@pytest.mark.parametrize("dt,m", [(Q2_0, 1)])
+@pytest.mark.parametrize("dt,m", [(Q2_0, 1), (Q4K, 1), (Q4K, 8)])
 @pytest.mark.parametrize("first", [True, False])
 def test_pair_with_one_result_over_the_rows(be, oracle, dt, m, first):
     w1, w2 = synth.weight(dt, N, N, seed=1), synth.weight(dt, N, N, seed=2)
