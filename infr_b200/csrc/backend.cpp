@@ -319,6 +319,12 @@ Status CudaBackend::linear(int dtype, const uint8_t *w, const float *x, float *y
         if (e != cudaErrorInvalidValue) return cuda_status(e, "gemv_q2");
         cudaGetLastError();
     }
+    if (act == INFR_ACT_F32 && in_place) {  // the f32 kernels read the rows while they store: from a copy
+        Status s = ensure_scratch((size_t)m * in_f * 4);
+        if (s.ok()) s = cuda_status(cudaMemcpyAsync(scratch(), x, (size_t)m * in_f * 4, cudaMemcpyDeviceToDevice, stream_), "linear: rows");
+        if (!s.ok()) return s;
+        x = reinterpret_cast<const float *>(scratch());
+    }
     // Decode shapes (m <= 8) run the streaming GEMV; wider batches are walked 8 rows at a time, all rows quantised once.
     Q8Dev a_all{};
     // (a single Q4_K chunk quantises its rows inside the GEMV; with several chunks that would repeat the work in every CTA)

@@ -5,10 +5,11 @@ import pytest
 
 import fixtures as fx
 import infr_b200
-from infr_b200 import Q2_0, Q4K, synth
+from infr_b200 import ACT_F32, ACT_INT8, Q2_0, Q4K, Q6K, synth
 
 pytestmark = pytest.mark.gpu
 N = 4096  # enough CTAs that some store while others have not begun
+TOL = {ACT_INT8: 1e-6, ACT_F32: 1e-5}
 
 
 @pytest.fixture(scope="module")
@@ -23,14 +24,14 @@ def _rows(be, m, seed):
     return x, be.from_numpy(x)
 
 
-@pytest.mark.parametrize("dt,m", [(Q2_0, 1), (Q4K, 1), (Q4K, 8)])
-def test_linear_in_place(be, oracle, dt, m):
+@pytest.mark.parametrize("dt,m,act", [(Q2_0, 1, ACT_INT8), (Q4K, 1, ACT_INT8), (Q4K, 8, ACT_INT8), (Q2_0, 3, ACT_F32), (Q4K, 9, ACT_F32), (Q6K, 1, ACT_F32)])
+def test_linear_in_place(be, oracle, dt, m, act):
     w = synth.weight(dt, N, N, seed=1)
     wb = be.from_numpy(w)
     for seed in range(4):
         x, xb = _rows(be, m, seed)
-        be.linear(dt, wb, xb, xb, m, N, N)
-        assert fx.rel_l2(be.download(xb, np.float32).reshape(m, N), oracle.linear(dt, w, x, m, N, N)) < 1e-6
+        be.linear(dt, wb, xb, xb, m, N, N, act)
+        assert fx.rel_l2(be.download(xb, np.float32).reshape(m, N), oracle.linear(dt, w, x, m, N, N, reference=act == ACT_F32)) < TOL[act]
 
 
 @pytest.mark.parametrize("dt,m", [(Q2_0, 1), (Q4K, 1), (Q4K, 8)])
