@@ -135,12 +135,12 @@ __global__ void __launch_bounds__(256) gemm_q2_prep_kernel(const float *x, int m
 struct Q2Mat {
     const uint8_t *w;
     float *c;  // [m, out_f] (K split: the first of kz partial results)
-    int out_f;
+    int out_f, kz;
 };
 
 // NTW: groups of 8 tokens of a warp.  KH: the two halves of the warps share the blocks, else the tokens.
 template <int NTW, bool KH>
-__global__ void __launch_bounds__(kThreadsQ2, 1) gemm_q2_kernel(Q2Mat m1, Q2Mat m2, const uint8_t *act, int m, int nb, int kz,
+__global__ void __launch_bounds__(kThreadsQ2, 1) gemm_q2_kernel(Q2Mat m1, Q2Mat m2, const uint8_t *act, int m, int nb, int tiles,
                                                                 uint32_t *__restrict__ status) {
     constexpr int NT = KH ? NTW : 2 * NTW, kRaw = kRowsCta * kRowPitch, kRec = record_bytes(NT), kAct = kHalfBlk * kRec, kSums = 4 * NTW;
     extern __shared__ __align__(128) uint8_t smem[];
@@ -157,12 +157,12 @@ __global__ void __launch_bounds__(kThreadsQ2, 1) gemm_q2_kernel(Q2Mat m1, Q2Mat 
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
-    // work item: K split fastest, then weight rows (neighbouring CTAs share activations), then tokens
-    const int rt1 = (m1.out_f + kRowsCta - 1) / kRowsCta, row_tiles = rt1 + (m2.out_f + kRowsCta - 1) / kRowsCta;
-    const int ks = blockIdx.x % kz, r = blockIdx.x / kz, rt = r % row_tiles, tt = r / row_tiles;
-    const bool second = rt >= rt1;
+    // work item: the first matrix, then the second; K split fastest, then weight rows (neighbouring CTAs share activations), then tokens
+    const int items1 = (m1.out_f + kRowsCta - 1) / kRowsCta * tiles * m1.kz;
+    const bool second = (int)blockIdx.x >= items1;
     const uint8_t *W = second ? m2.w : m1.w;
-    const int of = second ? m2.out_f : m1.out_f, row0 = (second ? rt - rt1 : rt) * kRowsCta;
+    const int of = second ? m2.out_f : m1.out_f, kz = second ? m2.kz : m1.kz, row_tiles = (of + kRowsCta - 1) / kRowsCta;
+    const int i0 = (int)blockIdx.x - (second ? items1 : 0), ks = i0 % kz, r = i0 / kz, tt = r / row_tiles, row0 = r % row_tiles * kRowsCta;
     const int b_begin = (int)((long long)ks * nb / kz), b_end = (int)((long long)(ks + 1) * nb / kz);
     const int n_half = (b_end - b_begin + kHalfBlk - 1) / kHalfBlk;
     const size_t row_bytes = (size_t)nb * 18;
@@ -298,13 +298,13 @@ __global__ void __launch_bounds__(kThreadsQ2, 1) gemm_q2_kernel(Q2Mat m1, Q2Mat 
 }
 
 template <int NTW, bool KH>
-cudaError_t launch_ntw(int grid, cudaStream_t st, Q2Mat m1, Q2Mat m2, const uint8_t *act, int m, int nb, int kz, uint32_t *status) {
+cudaError_t launch_ntw(int grid, cudaStream_t st, Q2Mat m1, Q2Mat m2, const uint8_t *act, int m, int nb, int tiles, uint32_t *status) {
     constexpr int NT = KH ? NTW : 2 * NTW;
     constexpr size_t smem = (size_t)2 * kRowsCta * kRowPitch + (size_t)2 * kHalfBlk * record_bytes(NT) + (size_t)16 * 4 * NTW * 32 * 8;
     static_assert(smem <= 227 * 1024 - 64, "shared memory");
     cudaError_t e = cudaFuncSetAttribute(gemm_q2_kernel<NTW, KH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    return launch_pdl(gemm_q2_kernel<NTW, KH>, dim3((unsigned)grid), dim3(kThreadsQ2), smem, st, m1, m2, act, m, nb, kz, status);
+    return launch_pdl(gemm_q2_kernel<NTW, KH>, dim3((unsigned)grid), dim3(kThreadsQ2), smem, st, m1, m2, act, m, nb, tiles, status);
 }
 
 // Tokens are cut evenly: the fewest tiles of at most 80, each of the fewest groups of 8 (pairs of groups above 40 tokens).
@@ -331,28 +331,36 @@ int q2_splits(int m, int in_f, int out_f1, int out_f2, const DeviceInfo &dev) {
     return best;
 }
 
+// Up to 16 rows a pair has the bits of two calls: each matrix is split as it would be alone.  (12 rows of 4096 -> 2 x 14336: 2 ways each,
+// 40 us; 1 way as both heights together would have it, 36; walked 8 rows at a time 68.)  More rows: by both heights together.
+constexpr int kPairBits = 16;
+void q2_pair_splits(int m, int in_f, int out_f1, int out_f2, const DeviceInfo &dev, int &kz1, int &kz2) {
+    kz1 = kz2 = q2_splits(m, in_f, out_f1, out_f2, dev);
+    if (out_f2 && m <= kPairBits) kz1 = q2_splits(m, in_f, out_f1, 0, dev), kz2 = q2_splits(m, in_f, out_f2, 0, dev);
+}
+
 __device__ __forceinline__ void add_to(float4 &a, const float4 &v) { a.x += v.x, a.y += v.y, a.z += v.z, a.w += v.w; }
 __device__ __forceinline__ void add_to(float &a, float v) { a += v; }
 
-// y[i] = part[0][i] + part[1][i] + ... in split order (the same bits on every run), for two results.  V = float4, or float
+// y[i] = part[0][i] + part[1][i] + ... in split order (the same bits on every run), for two results (n = 0: none).  V = float4, or float
 // where a result's size is not a multiple of four or its address not 16-byte aligned.
 template <typename V>
-__global__ void __launch_bounds__(256) gemm_q2_sum_kernel(const V *part, V *__restrict__ y, size_t n1, const V *part2,
-                                                          V *__restrict__ y2, size_t n2, int kz) {
+__global__ void __launch_bounds__(256) gemm_q2_sum_kernel(const V *part, V *__restrict__ y, size_t n1, int kz, const V *part2,
+                                                          V *__restrict__ y2, size_t n2, int kz2) {
     pdl_go();
     pdl_wait();
     size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n1 + n2) return;
-    if (i >= n1) i -= n1, part = part2, y = y2, n1 = n2;
+    if (i >= n1) i -= n1, part = part2, y = y2, n1 = n2, kz = kz2;
     V acc = part[i];
     for (int s = 1; s < kz; s++) add_to(acc, part[(size_t)s * n1 + i]);
     y[i] = acc;
 }
 template <typename V>
-cudaError_t launch_sum(const float *p, float *y, size_t n1, const float *p2, float *y2, size_t n2, int kz, cudaStream_t st) {
+cudaError_t launch_sum(const float *p, float *y, size_t n1, int kz, const float *p2, float *y2, size_t n2, int kz2, cudaStream_t st) {
     constexpr size_t L = sizeof(V) / 4;
     return launch_pdl(gemm_q2_sum_kernel<V>, dim3((unsigned)(((n1 + n2) / L + 255) / 256)), dim3(256), 0, st, reinterpret_cast<const V *>(p),
-                      reinterpret_cast<V *>(y), n1 / L, reinterpret_cast<const V *>(p2), reinterpret_cast<V *>(y2), n2 / L, kz);
+                      reinterpret_cast<V *>(y), n1 / L, kz, reinterpret_cast<const V *>(p2), reinterpret_cast<V *>(y2), n2 / L, kz2);
 }
 
 size_t q2_align(size_t v) { return (v + 255) / 256 * 256; }
@@ -363,8 +371,9 @@ bool gemm_q2_takes(int in_f) { return in_f > 0 && in_f % 64 == 0; }
 // Scratch: the activation records (gemm_q2_record_bytes), then the parts of a split K (gemm_q2_partial_bytes).
 size_t gemm_q2_record_bytes(int m, int in_f) { return q2_align((size_t)q2_tiles(m) * (in_f / 64) * record_bytes(q2_nt(m))); }
 size_t gemm_q2_partial_bytes(int m, int in_f, int out_f1, int out_f2, const DeviceInfo &dev) {
-    const int kz = q2_splits(m, in_f, out_f1, out_f2, dev);
-    return kz > 1 ? q2_align((size_t)kz * m * ((size_t)out_f1 + out_f2) * 4) : 0;
+    int kz1, kz2;
+    q2_pair_splits(m, in_f, out_f1, out_f2, dev, kz1, kz2);
+    return q2_align(((kz1 > 1 ? (size_t)kz1 * out_f1 : 0) + (kz2 > 1 ? (size_t)kz2 * out_f2 : 0)) * m * 4);
 }
 
 cudaError_t launch_gemm_q2_prep(const float *x, void *records, int m, int in_f, cudaStream_t st) {
@@ -378,28 +387,30 @@ cudaError_t launch_gemm_q2(const uint8_t *w, const void *records, float *c, floa
                            uint32_t *status, cudaStream_t st, const uint8_t *w2, float *c2, int out_f2) {
     if (m < 1 || out_f < 1 || !gemm_q2_takes(in_f) || (w2 && out_f2 < 1)) return cudaErrorInvalidValue;
     if (!w2) out_f2 = 0;
-    const int kz = q2_splits(m, in_f, out_f, out_f2, dev);
-    if (kz > 1 && !partials) return cudaErrorInvalidValue;
-    float *p2 = partials + (kz > 1 ? (size_t)kz * m * out_f : 0);
-    const Q2Mat m1{w, kz > 1 ? partials : c, out_f}, m2{w2, kz > 1 ? p2 : c2, out_f2};
-    const int grid = q2_row_tiles(out_f, out_f2) * q2_tiles(m) * kz;
+    int kz1, kz2;
+    q2_pair_splits(m, in_f, out_f, out_f2, dev, kz1, kz2);
+    // elements whose parts are to be added
+    const size_t n1 = kz1 > 1 ? (size_t)m * out_f : 0, n2 = kz2 > 1 ? (size_t)m * out_f2 : 0;
+    if (n1 + n2 && !partials) return cudaErrorInvalidValue;
+    float *p2 = partials + kz1 * n1;
+    const Q2Mat m1{w, n1 ? partials : c, out_f, kz1}, m2{w2, n2 ? p2 : c2, out_f2, kz2};
+    const int tiles = q2_tiles(m), grid = (q2_row_tiles(out_f, 0) * kz1 + q2_row_tiles(out_f2, 0) * kz2) * tiles;
     const uint8_t *act = static_cast<const uint8_t *>(records);
     const int nb = in_f / 64;
     cudaError_t e = cudaErrorInvalidValue;
     switch (q2_nt(m)) {
-    case 1: e = launch_ntw<1, true>(grid, st, m1, m2, act, m, nb, kz, status); break;
-    case 2: e = launch_ntw<2, true>(grid, st, m1, m2, act, m, nb, kz, status); break;
-    case 3: e = launch_ntw<3, true>(grid, st, m1, m2, act, m, nb, kz, status); break;
-    case 4: e = launch_ntw<4, true>(grid, st, m1, m2, act, m, nb, kz, status); break;
-    case 5: e = launch_ntw<5, true>(grid, st, m1, m2, act, m, nb, kz, status); break;
-    case 6: e = launch_ntw<3, false>(grid, st, m1, m2, act, m, nb, kz, status); break;
-    case 8: e = launch_ntw<4, false>(grid, st, m1, m2, act, m, nb, kz, status); break;
-    case 10: e = launch_ntw<5, false>(grid, st, m1, m2, act, m, nb, kz, status); break;
+    case 1: e = launch_ntw<1, true>(grid, st, m1, m2, act, m, nb, tiles, status); break;
+    case 2: e = launch_ntw<2, true>(grid, st, m1, m2, act, m, nb, tiles, status); break;
+    case 3: e = launch_ntw<3, true>(grid, st, m1, m2, act, m, nb, tiles, status); break;
+    case 4: e = launch_ntw<4, true>(grid, st, m1, m2, act, m, nb, tiles, status); break;
+    case 5: e = launch_ntw<5, true>(grid, st, m1, m2, act, m, nb, tiles, status); break;
+    case 6: e = launch_ntw<3, false>(grid, st, m1, m2, act, m, nb, tiles, status); break;
+    case 8: e = launch_ntw<4, false>(grid, st, m1, m2, act, m, nb, tiles, status); break;
+    case 10: e = launch_ntw<5, false>(grid, st, m1, m2, act, m, nb, tiles, status); break;
     }
-    if (e != cudaSuccess || kz == 1) return e;
-    const size_t n1 = (size_t)m * out_f, n2 = (size_t)m * out_f2;
-    const bool v4 = n1 % 4 == 0 && n2 % 4 == 0 && (uintptr_t)c % 16 == 0 && (!n2 || (uintptr_t)c2 % 16 == 0);
-    return v4 ? launch_sum<float4>(partials, c, n1, p2, c2, n2, kz, st) : launch_sum<float>(partials, c, n1, p2, c2, n2, kz, st);
+    if (e != cudaSuccess || !(n1 + n2)) return e;
+    const bool v4 = n1 % 4 == 0 && n2 % 4 == 0 && (!n1 || (uintptr_t)c % 16 == 0) && (!n2 || (uintptr_t)c2 % 16 == 0);
+    return v4 ? launch_sum<float4>(partials, c, n1, kz1, p2, c2, n2, kz2, st) : launch_sum<float>(partials, c, n1, kz1, p2, c2, n2, kz2, st);
 }
 
 }  // namespace infr

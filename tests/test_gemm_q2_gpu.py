@@ -72,3 +72,24 @@ def test_gemm_q2_extreme_codes(be, oracle):
     x[5, 40] = np.inf
     got, want = be.run_linear(Q2_0, w, x, m, in_f, out_f), oracle.linear(Q2_0, w, x, m, in_f, out_f)
     np.testing.assert_array_equal(np.isnan(got), np.isnan(want))
+
+
+@pytest.mark.parametrize("m", [9, 12, 16])
+@pytest.mark.parametrize("in_f,n1,n2", [
+    (4096, 14336, 14336),  # split 2 ways alone, not at all by both heights together
+    (4096, 4096, 1024),    # 9 and 15 ways alone, 7 together
+    (64, 300, 40),         # one block: neither is split
+    (4096, 28672, 515),    # only the second matrix, of a height that is not a multiple of four
+])
+def test_short_pair_has_the_bits_of_two_calls(be, oracle, m, in_f, n1, n2):
+    part = synth.weight(Q2_0, 40, in_f, seed=3)  # the weights repeat with period 40 rows
+    w1, w2 = (be.from_numpy(np.tile(part, n // 40 + 1)[:n * in_f // 64 * 18]) for n in (n1, n2))
+    xh = synth.normal(7, (m, in_f))
+    x, y = be.from_numpy(xh), [be.alloc(m * n * 4) for n in (n1, n2, n1, n2)]
+    be.linear(Q2_0, w1, x, y[0], m, in_f, n1)
+    be.linear(Q2_0, w2, x, y[1], m, in_f, n2)
+    be.linear_pair(Q2_0, w1, y[2], n1, w2, y[3], n2, x, m, in_f)
+    want = oracle.linear(Q2_0, part, xh, m, in_f, 40)
+    for n, a, b in ((n1, y[0], y[2]), (n2, y[1], y[3])):
+        np.testing.assert_array_equal(be.download(a, np.uint32), be.download(b, np.uint32))
+        assert fx.rel_l2(be.download(b, np.float32).reshape(m, n)[:, -n % 40 and -(n % 40) - 40 or -40:][:, :40], want) < TOL
