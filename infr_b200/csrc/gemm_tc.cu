@@ -566,6 +566,8 @@ __global__ void __launch_bounds__(Cfg<FMT, TN>::kWarps * 32, Cfg<FMT, TN>::kCtas
                             if (j >= 2 && !(ok = wait_bar(bar(K::B_ACCFREE + s), jp ^ 1u, dead))) break;
                         } else {
                             if (j >= 1 && !(ok = wait_bar(bar(K::B_ACCFREE + pass), (uint32_t)(j - 1) & 1u, dead))) break;
+                            // its reads come before this pass's multiplications (pass 0: the fence behind the operands' wait)
+                            if (pass > 0) tc_fence_after();
                         }
 #pragma unroll
                         for (int u = 0; u < K::kUnits; u++) {

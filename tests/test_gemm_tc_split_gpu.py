@@ -1,5 +1,6 @@
 """The tensor-memory GEMM over several token tiles: whole waves of tiles over all of K, the tiles past them split over K (gemm_tc.cu,
 split_of), vs the CPU restatement.  Tolerance as in test_gemm_tc_gpu.py: the block sums are the CPU's integers."""
+import numpy as np
 import pytest
 
 import fixtures as fx
@@ -31,3 +32,21 @@ def test_gemm_tc_tail_split(be, oracle, dt, m, in_f, out_f):
     got, want = be.run_linear(dt, w, x, m, in_f, out_f), oracle.linear(dt, w, x, m, in_f, out_f)
     assert fx.rel_l2(got, want) < TOL
     assert max(fx.rel_l2(got[r], want[r]) for r in range(m)) < 2 * TOL
+
+
+@pytest.mark.parametrize("m", [65, 113, 128])
+def test_gemm_tc_q6_halves_share_accumulators(be, oracle, m):
+    # 128-token tiles of Q6_K multiply a block in two halves of the tokens, whose accumulators are drained and filled in turn: many blocks
+    # through one set of them, the same bits on every run
+    in_f, out_f = 28672, 2600  # 21 row tiles: K split 7 ways, 16 blocks a CTA
+    part = synth.weight(Q6K, 40, in_f, seed=m)  # the weights repeat with period 40 rows
+    w = be.from_numpy(np.tile(part, out_f // 40))
+    xh = synth.normal(6, (m, in_f))
+    x, y = be.from_numpy(xh), be.alloc(m * out_f * 4)
+    runs = set()
+    for _ in range(20):
+        be.linear(Q6K, w, x, y, m, in_f, out_f)
+        runs.add(be.download(y, np.uint32).tobytes())
+    assert len(runs) == 1
+    got, want = be.download(y, np.float32).reshape(m, out_f // 40, 40), oracle.linear(Q6K, part, xh, m, in_f, 40)
+    assert max(fx.rel_l2(got[:, i], want) for i in range(out_f // 40)) < TOL
