@@ -92,11 +92,16 @@ _OP_RECORDS = {(nt, nu, nf): struct.Struct(f"=I{nt}I{32 - 4 * nt}x{nu}I{48 - 4 *
 assert all(r.size == C.sizeof(_OpDesc) for r in _OP_RECORDS.values())
 
 
-def _op_record(tag, tensors, u, f) -> bytes:
+def _op_record(tag, tensors, u, f, convert=True) -> bytes:
+    """convert: counts and factors go through int() and float() where they are not numbers of that kind; otherwise they are refused."""
     try:
         return _OP_RECORDS[len(tensors), len(u), len(f)].pack(tag, *tensors, *u, *f)
-    except (struct.error, OverflowError):  # what a ctypes field converts and a packed record does not (floats for counts, values out of range)
-        return bytes(_OpDesc(tag, tuple(tensors), tuple(int(v) for v in u), tuple(float(v) for v in f)))
+    except (struct.error, OverflowError):  # what a ctypes field takes and a packed record does not (values out of range), or neither does
+        op = _OpDesc(tag)
+        for field, values in (op.t, tensors), (op.u, map(int, u) if convert else u), (op.f, map(float, f) if convert else f):
+            for i, v in enumerate(values):
+                field[i] = v
+        return bytes(op)
 
 
 class _MoeDesc(C.Structure):
@@ -314,16 +319,16 @@ class Graph:
     def output(self, numel, dtype=F32):
         return self._decl(TK_OUTPUT, dtype, numel)
 
-    def _op(self, tag, tensors, u=(), f=()):
-        self.ops.append(_op_record(tag, tensors, u, f))
+    def _op(self, tag, tensors, u=(), f=(), convert=True):
+        self.ops.append(_op_record(tag, tensors, u, f, convert))
 
     def linear(self, x, weight, dst, m, in_f, out_f, w_off=0):
-        self._op(OP_LINEAR, (x, weight, dst), (m, in_f, out_f, w_off))
+        self._op(OP_LINEAR, (x, weight, dst), (m, in_f, out_f, w_off), convert=False)
 
     def moe_ffn(self, x, router_x, router, gate_exps, up_exps, down_exps, dst, *, ne, n_expert, n_used,
                 n_ff_exp, scale=1.0, norm_w=True, fused_gate_up=False, weight_before=False):
         self._op(OP_MOE_FFN, (x, router_x, router, gate_exps, up_exps, down_exps, dst),
-                 (ne, n_expert, n_used, n_ff_exp, int(norm_w), int(fused_gate_up), int(weight_before), 0, 0), (scale,))
+                 (ne, n_expert, n_used, n_ff_exp, int(norm_w), int(fused_gate_up), int(weight_before), 0, 0), (scale,), convert=False)
 
     # The remaining ops of a dense decode step, field for field with the Rust variants (graph.rs:141-896).
     def rms_norm(self, x, weight, dst, rows, dim, eps):

@@ -37,3 +37,24 @@ def test_graph_keeps_its_records():
     g.linear(a, b, c, 1, 256, 4, w_off=256)
     op = _OpDesc.from_buffer_copy(g.ops[0])
     assert (op.tag, list(op.t)[:3], list(op.u)[:4]) == (infr_b200.OP_LINEAR, [a, b, c], [1, 256, 4, 256])
+
+
+@pytest.mark.parametrize("bad", [{"m": 2.5}, {"in_f": 256.0}, {"out_f": "4"}, {"w_off": None}])
+def test_linear_refuses_what_is_no_integer(bad):
+    g = infr_b200.Graph()
+    a, b, c = g.input(256), g.weight(256 * 4, infr_b200.Q4K), g.output(4)
+    with pytest.raises(TypeError):
+        g.linear(a, b, c, **{**dict(m=1, in_f=256, out_f=4, w_off=0), **bad})
+    assert not g.ops
+    g.linear(a, b, c, np.int64(1), 256, 2**32 + 4)  # integers of any type; out of range: wraps like the field
+    assert list(_OpDesc.from_buffer_copy(g.ops[0]).u)[:3] == [1, 256, 4]
+
+
+@pytest.mark.parametrize("bad", [{"ne": 256.0}, {"n_used": 1.5}, {"scale": "1"}])
+def test_moe_ffn_refuses_what_is_no_number(bad):
+    g = infr_b200.Graph()
+    t = [g.input(256) for _ in range(7)]
+    with pytest.raises(TypeError):
+        g.moe_ffn(*t, **{**dict(ne=256, n_expert=4, n_used=2, n_ff_exp=256, scale=1.0), **bad})
+    g.moe_ffn(*t, ne=256, n_expert=4, n_used=2, n_ff_exp=256, scale=2)
+    assert _OpDesc.from_buffer_copy(g.ops[0]).f[0] == 2.0
