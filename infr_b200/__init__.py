@@ -301,7 +301,20 @@ class Graph:
 
     def __init__(self):
         self.tensors: list[tuple[int, int, int]] = []
-        self.ops: list[bytes] = []  # records of _OpDesc
+        self._ops: list = []  # packed records, or the structures that a reader of `ops` was given
+        self._shown = False
+
+    @property
+    def ops(self) -> list:
+        """The op list as structures (`_OpDesc`): entries can be read, edited, added and removed until compile."""
+        if not self._shown:
+            self._ops[:] = map(_OpDesc.from_buffer_copy, self._ops)
+            self._shown = True
+        return self._ops
+
+    @ops.setter
+    def ops(self, ops):
+        self._ops, self._shown = ops, True
 
     def _decl(self, kind, dtype, numel) -> int:
         self.tensors.append((kind, dtype, int(numel)))
@@ -320,7 +333,8 @@ class Graph:
         return self._decl(TK_OUTPUT, dtype, numel)
 
     def _op(self, tag, tensors, u=(), f=(), convert=True):
-        self.ops.append(_op_record(tag, tensors, u, f, convert))
+        record = _op_record(tag, tensors, u, f, convert)
+        self._ops.append(_OpDesc.from_buffer_copy(record) if self._shown else record)
 
     def linear(self, x, weight, dst, m, in_f, out_f, w_off=0):
         self._op(OP_LINEAR, (x, weight, dst), (m, in_f, out_f, w_off), convert=False)
@@ -513,10 +527,10 @@ class CudaBackend:
             except struct.error:  # (values that a ctypes field converts)
                 for i, t in enumerate(g.tensors):
                     tens[i] = _TensorDecl(*t)
-        ops = (_OpDesc * max(len(g.ops), 1))()
-        if g.ops:
-            ops = type(ops).from_buffer_copy(b"".join(g.ops))
-        desc = _GraphDesc(tens, len(g.tensors), ops, len(g.ops))
+        ops = (_OpDesc * max(len(g._ops), 1))()
+        if g._ops:
+            ops = type(ops).from_buffer_copy(b"".join(g._ops))
+        desc = _GraphDesc(tens, len(g.tensors), ops, len(g._ops))
         h = C.c_void_p()
         self._check(self.L.infr_cuda_compile(self.ctx, C.byref(desc), C.byref(h)))
         return Plan(self, h)

@@ -58,3 +58,30 @@ def test_moe_ffn_refuses_what_is_no_number(bad):
         g.moe_ffn(*t, **{**dict(ne=256, n_expert=4, n_used=2, n_ff_exp=256, scale=1.0), **bad})
     g.moe_ffn(*t, ne=256, n_expert=4, n_used=2, n_ff_exp=256, scale=2)
     assert _OpDesc.from_buffer_copy(g.ops[0]).f[0] == 2.0
+
+
+def test_ops_can_be_read_and_edited():
+    g = infr_b200.Graph()
+    a, b, c = g.input(256), g.input(256), g.output(256)
+    g.add(a, b, c, 256)
+    g.add(c, b, c, 128)
+    ops = g.ops
+    assert [(o.tag, list(o.t)[:3], o.u[0]) for o in ops] == [(infr_b200.OP_ADD, [a, b, c], 256), (infr_b200.OP_ADD, [c, b, c], 128)]
+    ops[1].u[0] = 64
+    g.copy(a, 0, c, 0, 8)
+    assert g.ops is ops and ops[2].tag == infr_b200.OP_COPY  # what is emitted later shows up as a structure too
+    del ops[2]
+    ops.append(_OpDesc.from_buffer_copy(ops[0]))
+    g.ops = g.ops[:2] + [ops[2]]
+    got = []
+
+    class Lib:  # the library's side of compile
+        @staticmethod
+        def infr_cuda_compile(ctx, desc, out):
+            got.extend((desc._obj.ops[i].tag, desc._obj.ops[i].u[0]) for i in range(desc._obj.n_ops))
+            return 0
+
+    be = infr_b200.CudaBackend.__new__(infr_b200.CudaBackend)
+    be.L, be.ctx = Lib, None
+    be.compile(g)
+    assert got == [(infr_b200.OP_ADD, 256), (infr_b200.OP_ADD, 64), (infr_b200.OP_ADD, 256)]
