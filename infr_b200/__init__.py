@@ -296,25 +296,30 @@ class Comm:
         self.handle = None
 
 
+class _OpList(list):
+    """Structures; what the graph appends as a record becomes one."""
+
+    def append(self, op):
+        super().append(_OpDesc.from_buffer_copy(op) if type(op) is bytes else op)
+
+
 class Graph:
     """Ordered op list over typed handles (crates/infr-core/src/graph.rs:1317-1460)."""
 
     def __init__(self):
         self.tensors: list[tuple[int, int, int]] = []
-        self._ops: list = []  # packed records, or the structures that a reader of `ops` was given
-        self._shown = False
+        self._ops: list = []  # packed records; an _OpList from the first look at `ops`
 
     @property
     def ops(self) -> list:
         """The op list as structures (`_OpDesc`): entries can be read, edited, added and removed until compile."""
-        if not self._shown:
-            self._ops[:] = map(_OpDesc.from_buffer_copy, self._ops)
-            self._shown = True
+        if type(self._ops) is not _OpList:
+            self._ops = _OpList(map(_OpDesc.from_buffer_copy, self._ops))
         return self._ops
 
     @ops.setter
     def ops(self, ops):
-        self._ops, self._shown = ops, True
+        self._ops = _OpList(ops)
 
     def _decl(self, kind, dtype, numel) -> int:
         self.tensors.append((kind, dtype, int(numel)))
@@ -333,8 +338,7 @@ class Graph:
         return self._decl(TK_OUTPUT, dtype, numel)
 
     def _op(self, tag, tensors, u=(), f=(), convert=True):
-        record = _op_record(tag, tensors, u, f, convert)
-        self._ops.append(_OpDesc.from_buffer_copy(record) if self._shown else record)
+        self._ops.append(_op_record(tag, tensors, u, f, convert))
 
     def linear(self, x, weight, dst, m, in_f, out_f, w_off=0):
         self._op(OP_LINEAR, (x, weight, dst), (m, in_f, out_f, w_off), convert=False)
