@@ -337,16 +337,16 @@ class Graph:
     def output(self, numel, dtype=F32):
         return self._decl(TK_OUTPUT, dtype, numel)
 
-    def _op(self, tag, tensors, u=(), f=(), convert=True):
-        self._ops.append(_op_record(tag, tensors, u, f, convert))
+    def _op(self, tag, tensors, u=(), f=()):
+        self._ops.append(_op_record(tag, tensors, u, f, True))
 
     def linear(self, x, weight, dst, m, in_f, out_f, w_off=0):
-        self._op(OP_LINEAR, (x, weight, dst), (m, in_f, out_f, w_off), convert=False)
+        self._ops.append(_op_record(OP_LINEAR, (x, weight, dst), (m, in_f, out_f, w_off), (), False))
 
     def moe_ffn(self, x, router_x, router, gate_exps, up_exps, down_exps, dst, *, ne, n_expert, n_used,
                 n_ff_exp, scale=1.0, norm_w=True, fused_gate_up=False, weight_before=False):
-        self._op(OP_MOE_FFN, (x, router_x, router, gate_exps, up_exps, down_exps, dst),
-                 (ne, n_expert, n_used, n_ff_exp, int(norm_w), int(fused_gate_up), int(weight_before), 0, 0), (scale,), convert=False)
+        counts = (ne, n_expert, n_used, n_ff_exp, int(norm_w), int(fused_gate_up), int(weight_before), 0, 0)
+        self._ops.append(_op_record(OP_MOE_FFN, (x, router_x, router, gate_exps, up_exps, down_exps, dst), counts, (scale,), False))
 
     # The remaining ops of a dense decode step, field for field with the Rust variants (graph.rs:141-896).
     def rms_norm(self, x, weight, dst, rows, dim, eps):
