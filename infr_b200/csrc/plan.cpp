@@ -223,6 +223,8 @@ Status CudaBackend::compile(const infr_graph_desc &g, infr_cuda_plan **out) {
             ok = ok && a.u[5] == rq.u[5] && a.f[0] == rq.f[0];                       // same pairing and base
             ok = ok && wk.t[0] == a.t[2] && wk.u[0] == a.u[0] && wv.u[0] == a.u[0];  // the rotated k is what WriteKv stores
             ok = ok && wk.u[1] == a.u[1] * a.u[2] && wv.u[1] == wk.u[1] && wk.u[2] == wv.u[2] && wk.t[1] != wv.t[1];
+            // v is neither what the group does not write nor what it rotates in place, q neither k nor the rotated k
+            ok = ok && wv.t[0] != a.t[2] && wv.t[0] != rq.t[0] && rq.t[0] != a.t[0] && rq.t[0] != a.t[2];
             ok = ok && plan->tensors[a.t[2]].kind == INFR_TK_INTERNAL;
             if (ok) {
                 const uint32_t nh = rq.u[1], nkv = a.u[1], hd = a.u[2];

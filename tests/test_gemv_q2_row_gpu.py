@@ -76,3 +76,33 @@ def test_rope_group_shares_its_rotated_keys(be):
     for a, b in zip(fused, apart):
         np.testing.assert_array_equal(a, b)
     assert np.abs(out).max() > 0
+
+
+@pytest.mark.parametrize("v_is,q_is", [("rotated k", "q"), ("q", "q"), ("v", "k"), ("v", "rotated k")])
+def test_rope_group_needs_handles_of_its_own(be, v_is, q_is):
+    # rope, rope, write_kv, write_kv where a handle stands in two places: the values of the ops one by one
+    rows, nh, hd, base = 3, 4, 64, 10000.0
+    n = rows * nh * hd
+    g = infr_b200.Graph()
+    h = {"q": g.input(n), "k": g.input(n), "v": g.input(n), "rotated k": g.internal(n)}
+    p, kc, vc = g.input(rows, infr_b200.I32), g.input(n, infr_b200.F16), g.input(n, infr_b200.F16)
+    g.rope(h["k"], p, h["rotated k"], rows, nh, hd, hd, base)
+    g.rope(h[q_is], p, h[q_is], rows, nh, hd, hd, base)
+    g.write_kv(h["rotated k"], kc, rows, nh * hd, 0)
+    g.write_kv(h[v_is], vc, rows, nh * hd, 0)
+    host = {s: synth.normal(i, (rows, nh * hd)) for i, s in enumerate(("q", "k", "v"))}
+    pos = be.from_numpy(np.arange(rows, dtype=np.int32))
+    results = []
+    for plan in (True, False):
+        b = {s: be.from_numpy(a) for s, a in host.items()}
+        b["rotated k"], ck, cv = be.alloc(n * 4), be.alloc(n * 2), be.alloc(n * 2)
+        if plan:
+            be.execute(be.compile(g), {**{h[s]: b[s] for s in host}, p: pos, kc: ck, vc: cv})
+        else:
+            be.rope(b["k"], pos, b["rotated k"], rows, nh, hd, hd, base)
+            be.rope(b[q_is], pos, b[q_is], rows, nh, hd, hd, base)
+            be.write_kv(b["rotated k"], ck, rows, nh * hd, 0)
+            be.write_kv(b[v_is], cv, rows, nh * hd, 0)
+        results.append([be.download(x, np.uint16) for x in (ck, cv, b["q"], b["k"])])
+    for x, y in zip(*results):
+        np.testing.assert_array_equal(x, y)
