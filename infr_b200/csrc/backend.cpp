@@ -720,13 +720,13 @@ Status CudaBackend::moe_ffn_f32(const MoeArgs &a) {
     } while (0)
     // one decoded token: router, gate and up, down (router_x and x: the row as the router and as the experts see it)
     if (rows == 1 && moe_row_takes((int)ne, (int)nff, (int)nx, (int)nu, a.x, a.router, a.gate, a.up, a.down)) {
-        INFR_STEP(launch_moe_router(a.router, a.router_x, logits, (int)rows, (int)ne, (int)nx, stream_), "moe router");
+        INFR_STEP(launch_moe_router(a.router, a.router_x, logits, (int)rows, (int)ne, (int)nx, dev_, stream_), "moe router");
         INFR_STEP(launch_moe_gate_up_row(logits, a.x, a.gate, a.up, act, ids, w, (int)ne, (int)nff, (int)nx, (int)nu, a.scale, a.norm_w, dev_, stream_),
                   "moe gate, up");
         INFR_STEP(launch_moe_down_row(a.down, act, ids, w, a.dst, (int)ne, (int)nff, (int)nu, dev_, stream_), "moe down");
         return Status::Ok();
     }
-    INFR_STEP(launch_moe_router(a.router, a.router_x, logits, (int)rows, (int)ne, (int)nx, stream_), "moe router");
+    INFR_STEP(launch_moe_router(a.router, a.router_x, logits, (int)rows, (int)ne, (int)nx, dev_, stream_), "moe router");
     INFR_STEP(launch_moe_route(logits, (int)rows, (int)nx, (int)nu, a.scale, a.norm_w, ids, w, stream_), "moe route");
     INFR_STEP(launch_gemv_q4k_f32_sel(a.gate, ids, gu_stride, a.x, (int)nu, g, (int)n_pairs, (int)ne, (int)nff, dev_, stream_), "moe gate f32");
     INFR_STEP(launch_gemv_q4k_f32_sel(a.up, ids, gu_stride, a.x, (int)nu, u, (int)n_pairs, (int)ne, (int)nff, dev_, stream_), "moe up f32");
@@ -814,7 +814,7 @@ Status CudaBackend::moe_ffn(const MoeArgs &a) {
         if (!s.ok()) return s;                      \
         launches_++;                                \
     } while (0)
-    INFR_STEP(launch_moe_router(a.router, a.router_x, logits, (int)rows, (int)ne, (int)nx, stream_), "moe router");
+    INFR_STEP(launch_moe_router(a.router, a.router_x, logits, (int)rows, (int)ne, (int)nx, dev_, stream_), "moe router");
     INFR_STEP(launch_moe_route(logits, (int)rows, (int)nx, (int)nu, a.scale, a.norm_w, ids, w, stream_), "moe route");
     INFR_STEP(launch_moe_bucket(ids, (int)rows, (int)nu, (int)nx, (int)a.expert_lo, (int)a.n_local, grouped_gemm ? slab : 8, prow, pslot, ie, ip, ic, ni,
                                 nullptr, stream_),

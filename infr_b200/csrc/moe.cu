@@ -352,12 +352,17 @@ __global__ void __launch_bounds__(256) moe_combine_kernel(const float *y_pairs, 
 }
 
 cudaError_t launch_moe_router(const float *router, const float *x, float *logits, int rows, int ne, int n_expert,
-                              cudaStream_t st) {
+                              const DeviceInfo &dev, cudaStream_t st) {
     if (rows < 1 || n_expert < 1) return cudaErrorInvalidValue;
     const dim3 grid((unsigned)((rows + kRtRows - 1) / kRtRows), (unsigned)((n_expert + kRtExperts - 1) / kRtExperts));
     if (grid.y > 65535) return cudaErrorInvalidValue;
-    // A few rows: a warp an expert and four rows, all columns staged at once (27 rows, 128 experts x 2048: 15 us by tiles, 7.4 so; 256 rows would be five waves of CTAs).
-    if (rows <= 64) {
+    // A few rows: a warp an expert and four rows, all columns staged at once, as long as its CTAs are four waves at most.  Measured, tiles /
+    // rows (us a layer; waves): 27 rows, 128 experts x 2048 15 / 7.4 (the router alone); 64 rows, 64 experts x 2048 (0.6) 85 / 71,
+    // 128 x 4096 (3.5) 155 / 145, 512 x 1024 (2.3) 72 / 77, 256 x 4096 (6.9) 163 / 175; 48 rows, 192 x 6144 (3.9) 205 / 195, 256 x 6144
+    // (5.2) 208 / 213; 32 rows, 512 x 2048 (2.3) 86 / 87, 512 x 4096 (6.9) 127 / 144.
+    const size_t row_smem = moe_router_row_smem(ne);
+    const size_t row_ctas = (size_t)((n_expert + 3) / 4) * ((rows + 3) / 4), fit = (size_t)dev.max_smem_optin / (row_smem + 1024);
+    if (rows <= 64 && row_ctas <= 4 * (size_t)dev.sm_count * (fit < 16 ? fit : 16)) {
         const cudaError_t e = launch_moe_router_row(router, x, logits, rows, ne, n_expert, st);
         if (e != cudaErrorInvalidValue) return e;
         cudaGetLastError();

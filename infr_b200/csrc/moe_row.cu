@@ -344,9 +344,10 @@ bool moe_row_takes(int ne, int nff, int n_expert, int n_used, const float *x, co
     return (((uintptr_t)x | (uintptr_t)router | (uintptr_t)gate | (uintptr_t)up | (uintptr_t)down) & 15) == 0;
 }
 
-// A few rows (up to 64 or so: a wave of CTAs), columns in whole groups of eight; cudaErrorInvalidValue: launch_moe_router's tiles take it.
+// A few rows (launch_moe_router draws the line), columns in whole groups of eight; cudaErrorInvalidValue: the tiles take it.
+size_t moe_router_row_smem(int ne) { return (size_t)(kRtRowsCta + kRtWarps) * (ne + 8) * 4; }
 cudaError_t launch_moe_router_row(const float *router, const float *x, float *logits, int rows, int ne, int n_expert, cudaStream_t st) {
-    const size_t smem = (size_t)(kRtRowsCta + kRtWarps) * (ne + 8) * 4;
+    const size_t smem = moe_router_row_smem(ne);
     if (rows < 1 || ne % 8 || smem > 220 * 1024 || (((uintptr_t)router | (uintptr_t)x) & 15)) return cudaErrorInvalidValue;
     cudaError_t e = cudaFuncSetAttribute(moe_router_row_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;

@@ -79,3 +79,17 @@ def test_moe_row_takes_the_ids_of_its_own_call(be, oracle):
             want = oracle.moe_ffn(x[i:i + 1], router, gate, up, down, **args)[0].ravel()
             assert np.abs(be.download(yb, np.float32) - want).max() / np.abs(want).max() < 1e-5
             be.upload(yb, np.zeros(ne, np.float32))
+
+
+@pytest.mark.parametrize("rows,ne,n_expert", [
+    (64, 6144, 148), (64, 6144, 149),  # the last whole four waves of the router for a few rows, and one expert more: its tiles
+    (5, 2048, 33),                     # rows and experts that are no multiple of four
+])
+def test_moe_router_kernels_at_the_line(be, oracle, rows, ne, n_expert):
+    nff = 256
+    gate, up, down = (np.tile(b, n_expert) for b in _banks(1, nff, ne, seed=3))  # (every expert the same)
+    router, x = synth.normal(17, (n_expert, ne), 1.0 / np.sqrt(ne)), synth.normal(3, (rows, ne))
+    got, ids, _, lg = _run(be, x, router, gate, up, down, rows, ne, n_expert, 1, nff)
+    want, o_ids, _, o_lg = oracle.moe_ffn(x, router, gate, up, down, rows=rows, ne=ne, n_expert=n_expert, n_used=1, n_ff_exp=nff)
+    np.testing.assert_array_equal(lg.view(np.uint32), o_lg.view(np.uint32))
+    np.testing.assert_array_equal(ids, o_ids)
