@@ -239,8 +239,8 @@ struct StreamGeom {
     uint32_t act_bytes;  // staged activations (codes + scales + sums), 16-byte aligned
 };
 
-// A second matrix with the same in_f against the same row in the same launch (q and k, gate and up): its rows follow the first
-// matrix's.  out_f == 0: none.
+// PAIR: a second matrix with the same in_f against the same row in the same launch (q and k, gate and up); its rows follow the first
+// matrix's.  (A template parameter: asking every row which matrix it is in cost a lone 64 -> 128256 matrix 13 %.)
 struct StreamSecond {
     const uint8_t *w;
     float *y;
@@ -249,8 +249,8 @@ struct StreamSecond {
 
 // FUSED (Q2_0, one row): the row comes as f32 and every CTA quantises it itself, per 32 elements, with the operations of quantize.cu in
 // the same order (crates/infr-cpu/src/quant.rs:97-117), while its first weights are in flight.
-// (A token of an 8B ternary model: 161 quantiser launches of 2.1 us and 64 GEMV launches less, 3.81 -> 3.40 ms with the same bits.)
-template <int DT, int M, bool FUSED>
+// (A token of an 8B ternary model, 161 quantiser launches of 2.1 us and 64 GEMV launches less: 3.02 -> 2.61 ms with the same bits.)
+template <int DT, int M, bool FUSED, bool PAIR>
 __global__ void __launch_bounds__(kStreamThreads, (M <= 2 ? 2 : 1))
     gemv_stream_kernel(const uint8_t *__restrict__ W, Q8Dev a, const float *x, float *__restrict__ y, int m, int in_f, int out_f,
                        StreamGeom geo, StreamSecond sec, uint32_t *__restrict__ status) {
@@ -272,12 +272,12 @@ __global__ void __launch_bounds__(kStreamThreads, (M <= 2 ? 2 : 1))
     pdl_launch_dependents();
 
     // balanced contiguous row range of this CTA
-    const int rows = out_f + sec.out_f;
+    const int rows = PAIR ? out_f + sec.out_f : out_f;
     const int G = gridDim.x, base = rows / G, rem = rows % G;
     const int r_begin = blockIdx.x * base + (blockIdx.x < rem ? blockIdx.x : rem);
     const int r_count = base + (blockIdx.x < rem ? 1 : 0);
     const size_t row_bytes = (size_t)nb * F::kBlockBytes;
-    auto row_start = [&](int row) { return row < out_f ? (size_t)W + (size_t)row * row_bytes : (size_t)sec.w + (size_t)(row - out_f) * row_bytes; };
+    auto row_start = [&](int row) { return !PAIR || row < out_f ? (size_t)W + (size_t)row * row_bytes : (size_t)sec.w + (size_t)(row - out_f) * row_bytes; };
     uint8_t *ring = smem + (size_t)warp * S * geo.slot_bytes;
     uint64_t *wbar = bars + warp * kMaxSlots;
     int2 *wmeta = meta + warp * kMaxSlots;
@@ -437,7 +437,7 @@ __global__ void __launch_bounds__(kStreamThreads, (M <= 2 ? 2 : 1))
             for (int i = 0; i < M; i++) {
                 const float v = warp_sum(acc[i]);
                 if (lane == 0 && i < m) {
-                    if (row < out_f)
+                    if (!PAIR || row < out_f)
                         y[(size_t)i * out_f + row] = v;
                     else
                         sec.y[(size_t)i * sec.out_f + row - out_f] = v;
@@ -452,7 +452,7 @@ __global__ void __launch_bounds__(kStreamThreads, (M <= 2 ? 2 : 1))
     }
 }
 
-template <int DT, int M, bool FUSED = false>
+template <int DT, int M, bool FUSED = false, bool PAIR = false>
 cudaError_t launch_stream_dt(const uint8_t *w, const Q8Dev &a, float *y, int m, int in_f, int out_f,
                              const DeviceInfo &dev, uint32_t *status, cudaStream_t st, const float *x = nullptr, StreamSecond sec = StreamSecond{}) {
     using F = Fmt<DT>;
@@ -478,7 +478,7 @@ cudaError_t launch_stream_dt(const uint8_t *w, const Q8Dev &a, float *y, int m, 
     const size_t smem = (size_t)slots * per_slot + fixed;
     int grid = (out_f + sec.out_f + kStreamWarps - 1) / kStreamWarps;
     if (grid > dev.sm_count * per_sm) grid = dev.sm_count * per_sm;
-    auto kernel = gemv_stream_kernel<DT, M, FUSED>;
+    auto kernel = gemv_stream_kernel<DT, M, FUSED, PAIR>;
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};
@@ -533,7 +533,8 @@ cudaError_t launch_gemv_q2_row(const uint8_t *w, float *y, int out_f, const uint
                                uint32_t *status, cudaStream_t st) {
     if (in_f < 64 || in_f % 64 || out_f < 1 || (w2 && out_f2 < 1) || (uintptr_t)x % 16) return cudaErrorInvalidValue;
     const Q8Dev none{nullptr, nullptr, nullptr, nullptr, 32};
-    return launch_stream_dt<DT_Q2_0, 1, true>(w, none, y, 1, in_f, out_f, dev, status, st, x, StreamSecond{w2, y2, w2 ? out_f2 : 0});
+    if (!w2) return launch_stream_dt<DT_Q2_0, 1, true>(w, none, y, 1, in_f, out_f, dev, status, st, x);
+    return launch_stream_dt<DT_Q2_0, 1, true, true>(w, none, y, 1, in_f, out_f, dev, status, st, x, StreamSecond{w2, y2, out_f2});
 }
 
 }  // namespace infr

@@ -17,7 +17,7 @@ def be():
     b.close()
 
 
-@pytest.mark.parametrize("in_f,n1,n2", [(64, 1, 3), (192, 37, 16), (704, 300, 41), (14336, 130, 64), (16448, 20, 300)])
+@pytest.mark.parametrize("in_f,n1,n2", [(64, 1, 3), (192, 37, 16), (704, 300, 41), (14336, 130, 64), (16384, 65, 7), (16448, 20, 300)])
 def test_q2_row_is_quantise_then_gemv(be, oracle, in_f, n1, n2):
     w1, w2 = synth.weight(Q2_0, n1, in_f, seed=1), synth.weight(Q2_0, n2, in_f, seed=2)
     x = synth.normal(3, (1, in_f))
