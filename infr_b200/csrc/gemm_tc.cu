@@ -946,8 +946,10 @@ int ctas_of(int fmt, int tn, const DeviceInfo &dev) { return dev.sm_count * (tn 
 // values are coded in 8 bits, where another order moves codes: the constants of this estimate (microseconds a block of a tile, 2 a
 // tile's start and end, 2.5 the kernel that adds the parts, 2e-6 each of their words) stay what they were, so that a decode step or a
 // prompt chunk keeps its bits.  They are high by a quarter by now; with others 113 rows of 4096 -> 14336 took the same time.
-// More tokens: whole waves of tiles are not split, the remaining ones fill the SMs (448 tiles on 148 SMs: 3 waves and 4 tiles, each of
-// them over 16 CTAs: 97 -> 81 us).
+// More tokens: whole waves of tiles (or all but one of them) are not split, the remaining ones fill the SMs (448 tiles on 148 SMs: 3 waves,
+// and 4 tiles over 8 CTAs each).  Estimate in microseconds: blk a block of a tile, tile its start and end, sum the kernel that adds the
+// parts, word each of their words; fitted to 130..1024 rows of 13 shapes with up to 23 splits each, where the choice is 1.2 % (Q4_K) and
+// 0.1 % (Q6_K) above the best of them on average, 10 % and 2 % at worst.  (Q6_K, 130 rows of 4096 -> 5120: 54 us unsplit, 46 three ways.)
 TcSplit split_of(int fmt, int tn, int m, int in_f, int row_tiles, int out_f, const DeviceInfo &dev) {
     const int cap = ctas_of(fmt, tn, dev), tt = (m + tn - 1) / tn, tiles = row_tiles * tt, nst = in_f / 256;
     if (tt == 1) {
@@ -962,14 +964,15 @@ TcSplit split_of(int fmt, int tn, int m, int in_f, int row_tiles, int out_f, con
         }
         return best == 1 ? TcSplit{tiles, 1, nullptr} : TcSplit{0, best, nullptr};
     }
-    const double blk = fmt == F_Q4 ? 1.5 : 2.0;
+    const bool q4 = fmt == F_Q4;
+    const double blk = q4 ? 1.2 : 2.7, tile = q4 ? 3.0 : 2.0, sum = q4 ? 1.5 : 2.0, word = q4 ? 1e-6 : 2e-7;
     TcSplit best{tiles, 1, nullptr};
-    double best_cost = (double)((tiles + cap - 1) / cap) * (nst * blk + 1.5);
+    double best_cost = (double)((tiles + cap - 1) / cap) * (nst * blk + tile);
     for (int full = tiles / cap * cap, k = 0; k < 2 && full >= 0; k++, full -= cap) {
         const int rest = tiles - full;
         for (int kz = 2; kz <= 16 && kz <= nst && rest > 0; kz++) {
             const int waves = (rest * kz + cap - 1) / cap, len = (nst + kz - 1) / kz;
-            const double cost = (double)(full / cap) * (nst * blk + 1.5) + waves * (len * blk + 1.5) + 2.5 + 2e-6 * rest * kz * tn * kTM;
+            const double cost = (double)(full / cap) * (nst * blk + tile) + waves * (len * blk + tile) + sum + word * rest * kz * tn * kTM;
             if (cost < best_cost * 0.98) best = TcSplit{full, kz, nullptr}, best_cost = cost;
         }
     }

@@ -50,3 +50,21 @@ def test_gemm_tc_q6_halves_share_accumulators(be, oracle, m):
     assert len(runs) == 1
     got, want = be.download(y, np.float32).reshape(m, out_f // 40, 40), oracle.linear(Q6K, part, xh, m, in_f, 40)
     assert max(fx.rel_l2(got[:, i], want) for i in range(out_f // 40)) < TOL
+
+
+@pytest.mark.parametrize("dt", [Q4K, Q6K])
+@pytest.mark.parametrize("m,in_f,n1,n2", [
+    (130, 4096, 4096, 1024),    # fewer tiles than SMs, all of them split
+    (300, 2048, 16384, 2600),   # 450 tiles: whole waves in front of the split ones, which lie in the second matrix (its last row tile partial)
+    (257, 4096, 300, 6400),     # 159 tiles, the first matrix of three
+])
+def test_gemm_tc_tail_split_of_a_pair(be, oracle, dt, m, in_f, n1, n2):
+    parts = [synth.weight(dt, 40, in_f, seed=s) for s in (1, 2)]  # the weights repeat with period 40 rows
+    w1, w2 = (be.from_numpy(np.resize(p, p.size // 40 * n)) for p, n in zip(parts, (n1, n2)))
+    xh = synth.normal(6, (m, in_f))
+    x, y1, y2 = be.from_numpy(xh), be.alloc(m * n1 * 4), be.alloc(m * n2 * 4)
+    be.linear_pair(dt, w1, y1, n1, w2, y2, n2, x, m, in_f)
+    for p, y, n in zip(parts, (y1, y2), (n1, n2)):
+        want = oracle.linear(dt, p, xh, m, in_f, 40)
+        got = be.download(y, np.float32).reshape(m, n)
+        assert fx.rel_l2(got, np.tile(want, (1, n // 40 + 1))[:, :n]) < TOL
