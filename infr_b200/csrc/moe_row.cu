@@ -283,22 +283,23 @@ __global__ void __launch_bounds__(kRowThreads, 1) moe_down_row_kernel(const uint
     const uint32_t row_bytes = (uint32_t)nb * 144u;
     __syncthreads();
     constexpr int kPre = 4;  // steps in flight
-    bool staged = false;
-    for (int row = blockIdx.x * kRowWarps + warp; row < ne; row += gridDim.x * kRowWarps) {
-        Piece w[kPre];
-        int fr = gr, fb = gb;  // the next step to fetch: its rank and block
-        auto fetch = [&](Piece &p) {
-            if (fr < n_used && fb < nb) p = fetch_piece(down + ((size_t)s_id[fr] * ne + row) * row_bytes + (size_t)fb * 144, t);
-            fb += P;
-            if (fb - gb >= per * P) fb = gb, fr += R;
-        };
+    int row = blockIdx.x * kRowWarps + warp;  // (every warp has one: ne is a multiple of 256, and a CTA has 16 of them)
+    Piece w[kPre];
+    int fr, fb;  // the next step to fetch: its rank and block
+    auto fetch = [&](Piece &p) {
+        if (fr < n_used && fb < nb) p = fetch_piece(down + ((size_t)s_id[fr] * ne + row) * row_bytes + (size_t)fb * 144, t);
+        fb += P;
+        if (fb - gb >= per * P) fb = gb, fr += R;
+    };
+    auto fetch_first = [&]() {
+        fr = gr, fb = gb;
 #pragma unroll
         for (int k = 0; k < kPre; k++) fetch(w[k]);
-        if (!staged) {  // (the first weights are on their way)
-            stage_block_pairs(act, s_x, n_used * nff, threadIdx.x, kRowThreads);
-            __syncthreads();
-            staged = true;
-        }
+    };
+    fetch_first();
+    stage_block_pairs(act, s_x, n_used * nff, threadIdx.x, kRowThreads);  // the first weights are on their way
+    __syncthreads();
+    while (true) {
         float o = 0.f;
         u64 acc[1] = {0ull};
         int rank0 = 0, i = 0;
@@ -326,10 +327,9 @@ __global__ void __launch_bounds__(kRowThreads, 1) moe_down_row_kernel(const uint
             }
         }
         if (lane == 0) dst[row] = o;
-    }
-    if (!staged) {  // a warp without a row helps to stage
-        stage_block_pairs(act, s_x, n_used * nff, threadIdx.x, kRowThreads);
-        __syncthreads();
+        row += gridDim.x * kRowWarps;
+        if (row >= ne) break;
+        fetch_first();
     }
 }
 
