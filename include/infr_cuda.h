@@ -73,8 +73,8 @@ typedef struct infr_cuda_graph infr_cuda_graph;
  * so that the parity tests can reach every kernel of the library on every shape:
  *   gemv_kernel 1: the direct-load byte-dot GEMV for all formats and batches;
  *   mmq_kernel  1: the Q4_K prefill GEMM whose f32 output is bit-identical to the CPU's (slower),
- *               2: the tensor-memory GEMM for every batch above 8 rows that it can fetch, also for MoE layers with a handful
- *                  of rows per expert,
+ *               2: the tensor-memory GEMM for every Q4_K and Q6_K batch above 8 rows that it can fetch, also for MoE layers with a
+ *                  handful of rows per expert (Q2_0 batches have one GEMM, the default),
  *               3: no GEMM: batches of more than 8 rows are walked through the GEMV 8 rows at a time. */
 typedef struct {
     int32_t device;

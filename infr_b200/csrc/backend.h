@@ -208,15 +208,16 @@ private:
     cudaEvent_t up_ev_[kUpSlots] = {};
     int up_next_ = 0;
     int gemv_impl_ = 0;                // 0 = bulk-copy ring kernel, 1 = direct-load kernel
-    int mmq_impl_ = 0;                 // 0 = by shape, 1 = bit-identical MMQ, 2 = tensor-memory GEMM above 8 rows, 3 = GEMV walk
+    int mmq_impl_ = 0;                 // 0 = by shape, 1 = bit-identical MMQ, 2 = batched GEMMs above 8 rows, 3 = GEMV walk
     Status check_device_status();
     // Batches of 9..32 rows (Q4_K, Q6_K; Q6_K up to 48 against few weights) through the wide GEMV.
     bool wide_applies(int dtype, uint32_t m, uint32_t in_f, uint64_t out_f, int act) const;
     Status wide_gemm(int dtype, const uint8_t *w, const Q8Dev &a, float *y, uint32_t m, uint32_t in_f, uint32_t out_f, float *partials,
                      const uint8_t *w2 = nullptr, float *y2 = nullptr, uint32_t out_f2 = 0);
-    // Larger batches (and Q2_0 above 16..24 rows) through the tensor-memory GEMM, from f32 rows (x) or quantised ones (a).
+    // Q2_0 batches above 8 rows through the GEMM on the warp matrix unit.
     bool q2_applies(int dtype, uint32_t m, uint32_t in_f, int act) const;
     Status q2_linear(const uint8_t *w, float *y, uint32_t out_f, const uint8_t *w2, float *y2, uint32_t out_f2, const float *x, uint32_t m, uint32_t in_f);
+    // Larger Q4_K and Q6_K batches through the tensor-memory GEMM, from f32 rows (x) or quantised ones (a).
     bool tc_applies(int dtype, uint32_t m, uint32_t in_f, uint64_t out_f, int act) const;
     bool tc_wins(int dtype, uint32_t m, uint32_t in_f, uint64_t out_f) const;
     size_t tc_scratch_bytes(int dtype, uint32_t m, uint32_t in_f, uint32_t out_f1, uint32_t out_f2 = 0) const;

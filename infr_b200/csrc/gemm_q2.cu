@@ -30,6 +30,7 @@
 // gemm_q2_prep_kernel lays them out in the order the lanes consume them, so that half a stage is one bulk copy.  Split K writes
 // partial results that a second kernel adds in split order.
 // Every wait is bounded; a CTA that gives up records a status word, waits (bounded) for its copies and returns.
+#include "f32x2.cuh"
 #include "gemv_common.cuh"
 #include "pdl.cuh"
 #include "q8_code.cuh"
@@ -46,8 +47,6 @@ constexpr int kRowPitch = 176;  // 144 bytes + up to 14 before and after, rounde
 constexpr int kMaxNtw = 5;       // groups of 8 tokens of a warp
 constexpr uint32_t kSpinQ2 = 1u << 22;
 constexpr uint32_t kMagic = 0x4B400000u;  // f32 bits of 1.5 * 2^23
-
-typedef unsigned long long u64;
 
 __device__ __forceinline__ uint32_t q2_su32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ bool q2_wait(uint32_t bar, uint32_t parity, uint32_t spins) {
@@ -72,29 +71,6 @@ __device__ __forceinline__ void q2_mma(uint32_t (&d)[4], const uint32_t (&a)[4],
         : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3])
         : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "r"(c.x), "r"(c.y), "r"(c.z), "r"(c.w));
 }
-// pairs of f32
-__device__ __forceinline__ u64 f2_pack(uint32_t lo, uint32_t hi) {
-    u64 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(lo), "r"(hi));
-    return r;
-}
-__device__ __forceinline__ u64 f2_dup(float v) { return f2_pack(__float_as_uint(v), __float_as_uint(v)); }
-__device__ __forceinline__ u64 f2_add(u64 a, u64 b) {
-    u64 r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ u64 f2_mul(u64 a, u64 b) {
-    u64 r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ u64 f2_fma(u64 a, u64 b, u64 c) {
-    u64 r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-
 // Activations: per (token tile, 64-element block) a record of NT x 512 bytes of codes, NT x 64 bytes of scales.
 //   codes  [n][lane g * 4 + t][group h][2 words]: token 8 n + g, elements 32 h + 8 t + {0, 2, 4, 6} and + {1, 3, 5, 7}
 //   scales [n][t][group h][2]: tokens 8 n + 2 t, + 1
@@ -385,7 +361,7 @@ cudaError_t launch_gemm_q2_prep(const float *x, void *records, int m, int in_f, 
 
 cudaError_t launch_gemm_q2(const uint8_t *w, const void *records, float *c, float *partials, int m, int in_f, int out_f, const DeviceInfo &dev,
                            uint32_t *status, cudaStream_t st, const uint8_t *w2, float *c2, int out_f2) {
-    if (m < 1 || out_f < 1 || !gemm_q2_takes(in_f) || (w2 && out_f2 < 1)) return cudaErrorInvalidValue;
+    if (m <= 8 || out_f < 1 || !gemm_q2_takes(in_f) || (w2 && out_f2 < 1)) return cudaErrorInvalidValue;
     if (!w2) out_f2 = 0;
     int kz1, kz2;
     q2_pair_splits(m, in_f, out_f, out_f2, dev, kz1, kz2);
@@ -399,7 +375,6 @@ cudaError_t launch_gemm_q2(const uint8_t *w, const void *records, float *c, floa
     const int nb = in_f / 64;
     cudaError_t e = cudaErrorInvalidValue;
     switch (q2_nt(m)) {
-    case 1: e = launch_ntw<1, true>(grid, st, m1, m2, act, m, nb, tiles, status); break;
     case 2: e = launch_ntw<2, true>(grid, st, m1, m2, act, m, nb, tiles, status); break;
     case 3: e = launch_ntw<3, true>(grid, st, m1, m2, act, m, nb, tiles, status); break;
     case 4: e = launch_ntw<4, true>(grid, st, m1, m2, act, m, nb, tiles, status); break;

@@ -41,6 +41,7 @@
 
 #include <type_traits>
 
+#include "f32x2.cuh"
 #include "gemv_common.cuh"
 #include "pdl.cuh"
 #include "q8_code.cuh"
@@ -146,24 +147,6 @@ __device__ __forceinline__ bool elect_one() {
     uint32_t p;
     asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
     return p != 0;
-}
-// pairs of f32
-typedef unsigned long long u64;
-__device__ __forceinline__ u64 f2_pack(uint32_t lo, uint32_t hi) {
-    u64 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(lo), "r"(hi));
-    return r;
-}
-__device__ __forceinline__ u64 f2_dup(float v) { return f2_pack(__float_as_uint(v), __float_as_uint(v)); }
-__device__ __forceinline__ u64 f2_mul(u64 a, u64 b) {
-    u64 r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ u64 f2_fma(u64 a, u64 b, u64 c) {
-    u64 r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
 }
 __device__ __forceinline__ void bar_arrive(uint32_t bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory"); }
 

@@ -567,7 +567,6 @@ cudaError_t launch_grouped_q6_mma(const uint8_t *bank, const Q8Dev &a, float *y,
     int kw = 8;
     while (kw > 2 && need(kw) > (size_t)dev.max_smem_optin / 2 - 2048) kw /= 2;
     if (need(kw) > (size_t)dev.max_smem_optin - 1024) return cudaErrorInvalidValue;
-    if (kw == 2 && need(4) <= (size_t)dev.max_smem_optin - 1024 && need(2) > (size_t)dev.max_smem_optin / 2 - 2048) kw = 4;
     cudaError_t e = cudaFuncSetAttribute(gemv_q6_mma_grouped_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)need(kw));
     if (e != cudaSuccess) return e;
     int gx = out_f / 16 / (8 * kw);  // about eight tiles a warp

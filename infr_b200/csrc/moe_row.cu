@@ -16,6 +16,7 @@
 //
 // Only the weights are const __restrict__ (pdl.cuh): the ids were, and the down kernel's load of them went above its wait.  Wherever the
 // gate / up launch left SMs idle, so that the next one was resident beside it, it took whatever the scratch held.
+#include "f32x2.cuh"
 #include "kernels.h"
 #include "pdl.cuh"
 
@@ -26,27 +27,6 @@ namespace {
 
 constexpr int kRowThreads = 512, kRowWarps = kRowThreads / 32;
 
-typedef unsigned long long u64;
-__device__ __forceinline__ u64 pk(float lo, float hi) {
-    u64 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-    return r;
-}
-__device__ __forceinline__ u64 add2(u64 a, u64 b) {
-    u64 r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ u64 mul2(u64 a, u64 b) {
-    u64 r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ u64 fma2(u64 a, u64 b, u64 c) {
-    u64 r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
 __device__ __forceinline__ float both(u64 v) { return __uint_as_float((uint32_t)v) + __uint_as_float((uint32_t)(v >> 32)); }
 __device__ __forceinline__ float hf(uint32_t bits) { return __half2float(__ushort_as_half((unsigned short)(bits & 0xffffu))); }
 
@@ -185,10 +165,10 @@ __device__ __forceinline__ void block_dot(const Piece (&w)[N], const float4 *s_x
         const int sh = 16 * (t & 1);
         s >>= sh, n >>= sh;
         const float d = hf(h.x), dm = hf(h.x >> 16);
-        sc[m] = pk(__fmul_rn(d, (float)(s & 0xFFu)), __fmul_rn(d, (float)((s >> 8) & 0xFFu)));
-        mn[m] = pk(__fmul_rn(dm, (float)(-(int)(n & 0xFFu))), __fmul_rn(dm, (float)(-(int)((n >> 8) & 0xFFu))));
+        sc[m] = f2_pack(__fmul_rn(d, (float)(s & 0xFFu)), __fmul_rn(d, (float)((s >> 8) & 0xFFu)));
+        mn[m] = f2_pack(__fmul_rn(dm, (float)(-(int)(n & 0xFFu))), __fmul_rn(dm, (float)(-(int)((n >> 8) & 0xFFu))));
     }
-    const u64 neg = pk(-8388608.0f, -8388608.0f);
+    const u64 neg = f2_pack(-8388608.0f, -8388608.0f);
     // a byte under the exponent of 2^23 is 2^23 + byte
     auto under = [](uint32_t v, int k) { return __uint_as_float(__byte_perm(v, 0x4B000000u, 0x7440u + k)); };
 #pragma unroll
@@ -207,7 +187,7 @@ __device__ __forceinline__ void block_dot(const Piece (&w)[N], const float4 *s_x
             for (int k = 0; k < 2; k++)
 #pragma unroll
                 for (int m = 0; m < N; m++)
-                    acc[m] = fma2(add2(mul2(sc[m], add2(pk(under(lo[m], 2 * h + k), under(hi[m], 2 * h + k)), neg)), mn[m]), k ? xv.y : xv.x, acc[m]);
+                    acc[m] = f2_fma(f2_add(f2_mul(sc[m], f2_add(f2_pack(under(lo[m], 2 * h + k), under(hi[m], 2 * h + k)), neg)), mn[m]), k ? xv.y : xv.x, acc[m]);
         }
     }
 }
