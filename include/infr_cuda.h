@@ -294,17 +294,19 @@ INFR_API int32_t infr_cuda_gemv_block_acc(infr_cuda_ctx *ctx, int32_t dtype, con
                                           uint32_t in_f, uint32_t out_f);
 
 /* Op::Linear of any m (crates/infr-cpu/src/lib.rs:985-1492): dispatches to the GEMV (m <= 8) or the
- * MMQ GEMM.  act as above. */
+ * batched kernels.  act as above.  y may lie over x: every row is read before the result is written. */
 INFR_API int32_t infr_cuda_linear(infr_cuda_ctx *ctx, int32_t dtype, const infr_cuda_buf *w, uint64_t w_off,
                                   const infr_cuda_buf *x, infr_cuda_buf *y, uint32_t m, uint32_t in_f,
                                   uint32_t out_f, int32_t act);
 
 /* Two Op::Linear of one weight format on the same rows (q and k, gate and up): the rows are quantised once (and laid out
  * once for the prefill GEMM), and where a kernel takes two weights the two products are one launch.  Results as from two
- * infr_cuda_linear calls, up to the order of f32 sums: the batched GEMM splits K by the height of both weights together,
- * and for 25..32 rows of Q4_K that height decides between it and the wide GEMV (up to 24 rows, and with Q2_0 up to 16, the
- * bits are those of two calls).  infr_cuda_execute pairs neighbouring Linear ops of a graph the same way, so a plan and
- * direct calls differ by as much. */
+ * infr_cuda_linear calls, up to the order of f32 sums: the height of both weights together decides over how many warps the
+ * GEMV for up to 8 rows of Q4_K splits K, how the batched GEMMs split it, and for 25..32 rows of Q4_K which of the GEMM and
+ * the wide GEMV runs.  The bits are those of two calls for 9..24 rows of Q4_K, up to 32 of Q6_K and up to 16 of Q2_0.
+ * Up to 8 rows of INFR_ACT_INT8 a result may lie over the rows (both are of the rows as they were) or the second over the
+ * first.  infr_cuda_execute pairs neighbouring Linear ops of a graph the same way, so a plan and direct calls differ by as
+ * much. */
 INFR_API int32_t infr_cuda_linear_pair(infr_cuda_ctx *ctx, int32_t dtype, const infr_cuda_buf *w1, uint64_t w_off1, infr_cuda_buf *y1,
                                        uint32_t out_f1, const infr_cuda_buf *w2, uint64_t w_off2, infr_cuda_buf *y2, uint32_t out_f2,
                                        const infr_cuda_buf *x, uint32_t m, uint32_t in_f, int32_t act);
