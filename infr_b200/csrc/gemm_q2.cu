@@ -12,10 +12,10 @@
 // the conversion to f32 is part of the instruction: the accumulator starts as the bit pattern of 1.5 * 2^23, so the int32 result
 // read as f32 is 1.5 * 2^23 + s, and one packed subtraction gives s exactly.
 //
-// What bounds it: issue and the f32 pipe.  Per 32 rows x 40 tokens x 64 elements a warp issues 308 instructions: 20 matrix
-// instructions, 100 packed f32 operations (2.5 per output and group), 40 to unpack, 31 loads, and ~80 moves that put the start value
-// into the accumulators (a conversion of the int32 sums instead costs as much); 0.53 instructions a cycle and scheduler, f32 pipe
-// 45 %, matrix unit 27 % busy.
+// What bounds it (profiles/batched_gemm_and_moe_kernels.md): issue and the f32 pipe.  Per 32 rows x 40 tokens x 64 elements a warp issues
+// 315 instructions, of them 20 matrix instructions and 100 packed f32 operations (2.5 per output and group), and moves that put the
+// start value into the accumulators (a conversion of the int32 sums instead costs as much); 0.49 instructions a cycle and scheduler, f32
+// pipe 41 %, matrix unit 25 % busy.
 // Measured (us, whole call, against the tensor-memory form for rows of whole 512-element chunks, the 8-row walk for others):
 // 14336 -> 4096, 77 rows 78 -> 41;  4096 -> 14336, 12 rows 32 -> 20, 64 rows 46 -> 38, 512 rows 282 -> 232;  4096 -> 4096, 32 rows
 // 21 -> 13;  4160 -> 1000, 40 rows 52 -> 13;  14336 -> 4096, 1024 rows 502 -> 417.

@@ -26,14 +26,12 @@
 // TN = 32 (Q4_K) keeps to half an SM's shared and tensor memory, so that two CTAs hide each other's waits.
 // Tiles: whole waves of them are multiplied over all of K; the rest of them is split over K so that it fills the SMs too, and a
 // small kernel adds the parts in split order (deterministic).
-// Measured (B200, us, cold weights, whole call; before = a warp issuing under `lane == 0`, stages held until the epilogue, whole waves
-// only):  Q4_K 4096 -> 14336, 512 rows 112 -> 81, 113 rows 35 -> 30, 4096 -> 2 x 14336, 32 rows 40 -> 35;  14336 -> 4096, 1024 rows
-// 194 -> 160;  Q6_K 14336 -> 4096, 113 rows 57 -> 54, 512 rows 183 -> 176.  Of the 512 rows' 31 us, 12 came from the operands of LOP3
-// (and_or below), the rest from the split of the last wave (448 tiles on 148 SMs) and the issuer.
-// What bounds it: instructions.  At 128 tokens a Q4_K job takes ~2400 cycles, its MMAs 1150; the warps issue 6600 instructions a job
-// (0.67 a cycle and scheduler): unpacking 1450, folding 1850 (a third of them moves out of the loads' registers), the rest waits on
-// barriers, their polls and addresses.  Without the fold, or without the unpacking, it would take 72 us.  One issuer's job of
-// seven commits and nine waits takes it ~1100 cycles.  Unpacking alone runs at 600 cycles a job and SM.
+// Measured (B200, us, whole calls over rotated cold weights, back to back, so that a call's layout launch overlaps the call before; before
+// = a warp issuing under `lane == 0`, stages held until the epilogue, whole waves only):  Q4_K 4096 -> 14336, 512 rows 113 -> 82 (a call
+// that waits for the one before it: 112 -> 89), 113 rows 35 -> 30, 1024 rows 192 -> 153;  14336 -> 4096, 1024 rows 194 -> 175;  Q6_K
+// 14336 -> 4096, 113 rows 57 -> 53, 512 rows 183 -> 177.  Some Q6_K shapes lost: 33..64 rows of 4096 -> 14336 49 -> 52.
+// What bounds it (profiles/batched_gemm_and_moe_kernels.md): issue slots and waits.  At 128 tokens a Q4_K job takes ~2550 cycles, its MMAs
+// 1150 (tensor pipe 45 % busy); the warps issue 6670 instructions a job, 0.66 a cycle and scheduler.
 // Every wait is bounded: on expiry the role raises a CTA flag and a status word, every role leaves its loop, copies in
 // flight are drained and the tensor memory is freed.
 #include <cuda.h>

@@ -303,8 +303,10 @@ __global__ void __launch_bounds__(KW * 32, 16 / KW)
 // plain bulk copy.  A warp owns whole tiles (all of K, two in flight) and stores its sums itself: no barrier between the warps of a CTA
 // after the staging of the activations.  A lane's rows start on any even address: its words are put together from two aligned loads
 // and a shift by 0 or 16 bits.
-// What bounds it: shared-memory loads (64 a block and lane) and the instructions around 18 matrix instructions a block (~300); the
-// weights of 105 experts of 2048 x 768 are 135 MB = 21 us.  Measured there (27 rows, top-8 of 128): 49 us; the byte-dot kernel, whose lanes load 2 bytes at a time, 196.
+// What bounds it (profiles/batched_gemm_and_moe_kernels.md): the chain of loads and instructions around 18 matrix instructions a block with
+// two warps a scheduler (0.46 instructions a cycle), and items of unequal size; shared memory is 44 % busy.  The weights of 105 experts
+// of 2048 x 768 are 135 MB = 21 us.  Measured there (27 rows, top-8 of 128): 51 us; the byte-dot kernel, whose lanes load 2 bytes at a
+// time, 196.
 __device__ __forceinline__ void block_q6_any(const uint8_t *p0, const uint8_t *p1, uint32_t sh, const uint8_t *st, const float *s_d8b, int t, int n0,
                                              float (&accf)[4]) {
     // p0, p1: the word boundary at or below the block; sh: 0, or 16 where the block starts two bytes past it

@@ -30,6 +30,8 @@ def be():
     (80, 1088, 130),    # a full token tile
     (81, 640, 512),     # two token tiles of 48
     (100, 14336, 64),   # K split over many CTAs
+    (250, 576, 300),    # four token tiles
+    (1024, 1024, 70),   # thirteen, the last one short
     (70, 256, 40000),   # more tiles than SMs
 ])
 def test_gemm_q2_matches_production_cpu(be, oracle, m, in_f, out_f):

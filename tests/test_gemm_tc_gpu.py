@@ -125,7 +125,8 @@ def test_gemm_tc_two_weights_and_repeat(tc, dt):
 
 
 @pytest.mark.parametrize("dt,in_f,n1,n2,m", [
-    (Q4K, 4096, 4096, 1024, 24), (Q2_0, 2048, 1000, 256, 16),     # below the line: the bits of two calls
+    (Q4K, 4096, 4096, 1024, 24),                                  # the wide GEMV: the bits of two calls
+    (Q2_0, 2048, 1000, 256, 16),                                  # its GEMM, each matrix split as it would be alone: the same
     (Q4K, 4096, 4096, 1024, 33), (Q4K, 4096, 4096, 1024, 113),    # K splits of 4 and 16 on their own, another together
     (Q4K, 4096, 8192, 8192, 32),                                  # large together, not each
     (Q4K, 4096, 12288, 12288, 25), (Q4K, 4096, 12288, 200, 32),   # both large; one of them
@@ -163,7 +164,7 @@ def test_a_pair_against_two_calls_and_the_cpu(backend, oracle, dt, in_f, n1, n2,
 
 @pytest.mark.parametrize("dt,in_f,out_f,rows", [
     (Q6K, 2048, 2048, (33, 48, 49)), (Q6K, 2048, 2080, (33,)), (Q6K, 4096, 1000, (33,)),  # two passes of the wide GEMV, or the GEMM
-    (Q2_0, 4096, 12320, (16, 17, 18)), (Q2_0, 4096, 24600, (24, 25)),                   # the 8-row GEMV walked, or the GEMM
+    (Q2_0, 4096, 12320, (8, 9, 16, 17, 18)), (Q2_0, 4096, 24600, (24, 25)),             # the GEMV, or the GEMM on the warp matrix unit
 ])
 def test_batches_at_the_lines_between_kernels(backend, oracle, dt, in_f, out_f, rows):
     be, bb = fx.BLOCK[dt]

@@ -24,8 +24,10 @@ def be():
 @pytest.mark.parametrize("rows,ne,n_expert,n_used,nff", [
     (2, 256, 2, 1, 256),     # one block a row
     (17, 768, 3, 1, 1280),   # 3 and 5 blocks; items of 8 rows and a rest
-    (40, 2304, 4, 2, 2048),  # 9 blocks: the longest rows of two warps a CTA with room for one CTA an SM; 8 blocks
-    (9, 4608, 3, 1, 256),    # 18 blocks: the byte-dot kernel
+    (40, 2304, 4, 2, 2048),  # 9 and 8 blocks: two warps a CTA, one CTA an SM
+    (9, 3584, 3, 1, 1792),   # 14 blocks: the longest rows that two warps have room for; 7: the longest with room for two CTAs
+    (9, 3840, 3, 1, 256),    # 15 blocks: the byte-dot kernel
+    (9, 4608, 3, 1, 256),    # 18 blocks
 ])
 def test_moe_q6_banks_match_cpu(be, oracle, rows, ne, n_expert, n_used, nff):
     bank = lambda o, i, s: np.concatenate([synth.weight(Q6K, o, i, s + 3 * e) for e in range(n_expert)])
