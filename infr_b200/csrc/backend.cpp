@@ -273,6 +273,33 @@ Status CudaBackend::quantize_for(int dtype, const float *x, uint32_t rows, uint3
     return Status::Ok();
 }
 
+// Up to 8 quantised rows through the GEMV of the format; rows so long that m of them staged exceed shared memory in narrower batches.
+Status CudaBackend::gemv_q8_rows(int dtype, const uint8_t *w, const Q8Dev &a, float *y, uint32_t m, uint32_t in_f, uint32_t out_f) {
+    uint32_t step = m;
+    for (uint32_t t0 = 0; t0 < m;) {
+        const uint32_t n = m - t0 < step ? m - t0 : step;
+        Q8Dev sub = a;
+        sub.qs = a.qs + (size_t)t0 * in_f;
+        sub.d = a.d + (size_t)t0 * (in_f / a.gran);
+        sub.sums = a.sums + (size_t)t0 * (in_f / 32);
+        if (a.sums16) sub.sums16 = a.sums16 + (size_t)t0 * (in_f / 16);
+        float *yt = y + (size_t)t0 * out_f;
+        const cudaError_t e = gemv_impl_ == 1   ? launch_gemv_q8(dtype, w, sub, yt, (int)n, (int)in_f, (int)out_f, nullptr, dev_, stream_)
+                              : dtype == DT_Q4K ? launch_gemv_q4k_mma(w, &sub, nullptr, yt, (int)n, (int)in_f, (int)out_f, dev_, status_dev_, stream_)
+                                                : launch_gemv_stream(dtype, w, sub, yt, (int)n, (int)in_f, (int)out_f, dev_, status_dev_, stream_);
+        if (e == cudaErrorInvalidValue && step > 1) {
+            cudaGetLastError();
+            step /= 2;
+            continue;
+        }
+        Status s = cuda_status(e, "gemv_q8");
+        if (!s.ok()) return s;
+        launches_ += 1;
+        t0 += n;
+    }
+    return Status::Ok();
+}
+
 static bool overlap(const float *a, size_t na, const float *b, size_t nb) {
     return (uintptr_t)a < (uintptr_t)b + nb * 4 && (uintptr_t)b < (uintptr_t)a + na * 4;
 }
@@ -364,35 +391,12 @@ Status CudaBackend::linear(int dtype, const uint8_t *w, const float *x, float *y
         } else {
             // this chunk's rows of the quantised batch
             Q8Dev a = a_all;
-            Status s;
-            const int gran = a.gran, ngr = (int)in_f / gran;
             a.qs = a_all.qs + (size_t)r0 * in_f;
-            a.d = a_all.d + (size_t)r0 * ngr;
+            a.d = a_all.d + (size_t)r0 * (in_f / a.gran);
             a.sums = a_all.sums + (size_t)r0 * (in_f / 32);
             if (a_all.sums16) a.sums16 = a_all.sums16 + (size_t)r0 * (in_f / 16);
-            // rows so long that `mm` staged activation rows exceed shared memory are run in narrower batches
-            uint32_t step = mm;
-            for (uint32_t t0 = 0; t0 < mm;) {
-                const uint32_t n = mm - t0 < step ? mm - t0 : step;
-                Q8Dev sub = a;
-                sub.qs = a.qs + (size_t)t0 * in_f;
-                sub.d = a.d + (size_t)t0 * ngr;
-                sub.sums = a.sums + (size_t)t0 * (in_f / 32);
-                if (a.sums16) sub.sums16 = a.sums16 + (size_t)t0 * (in_f / 16);
-                float *yt = yr + (size_t)t0 * out_f;
-                cudaError_t e = gemv_impl_ == 1   ? launch_gemv_q8(dtype, w, sub, yt, (int)n, (int)in_f, (int)out_f, nullptr, dev_, stream_)
-                                : dtype == DT_Q4K ? launch_gemv_q4k_mma(w, &sub, nullptr, yt, (int)n, (int)in_f, (int)out_f, dev_, status_dev_, stream_)
-                                                  : launch_gemv_stream(dtype, w, sub, yt, (int)n, (int)in_f, (int)out_f, dev_, status_dev_, stream_);
-                if (e == cudaErrorInvalidValue && step > 1) {
-                    cudaGetLastError();
-                    step /= 2;
-                    continue;
-                }
-                s = cuda_status(e, "gemv_q8");
-                if (!s.ok()) return s;
-                launches_ += 1;
-                t0 += n;
-            }
+            Status s = gemv_q8_rows(dtype, w, a, yr, mm, in_f, out_f);
+            if (!s.ok()) return s;
         }
     }
     return Status::Ok();
@@ -527,7 +531,7 @@ Status CudaBackend::linear_pair(int dtype, const uint8_t *w1, float *y1, uint32_
                 return Status::Ok();
             }
             if (e != cudaErrorInvalidValue) return cuda_status(e, "linear_pair");
-            cudaGetLastError();  // rows too long to stage m of them in one CTA: quantise first, then the pair
+            cudaGetLastError();  // rows too long to stage m of them in one CTA: quantise first
         }
         if (dtype == DT_Q2_0 && m == 1 && gemv_impl_ == 0 && apart) {
             const cudaError_t e = launch_gemv_q2_row(w1, y1, (int)out_f1, w2, y2, (int)out_f2, x, (int)in_f, dev_, status_dev_, stream_);
@@ -537,7 +541,8 @@ Status CudaBackend::linear_pair(int dtype, const uint8_t *w1, float *y1, uint32_
         }
         Q8Dev a;
         Status s = quantize_for(dtype, x, m, in_f, &a);
-        return s.ok() ? gemv_q8_pair(dtype, w1, y1, out_f1, w2, y2, out_f2, a, m, in_f) : s;
+        if (s.ok()) s = gemv_q8_rows(dtype, w1, a, y1, m, in_f, out_f1);
+        return s.ok() ? gemv_q8_rows(dtype, w2, a, y2, m, in_f, out_f2) : s;
     }
     Status s = linear(dtype, w1, x, y1, m, in_f, out_f1, act);
     return s.ok() ? linear(dtype, w2, x, y2, m, in_f, out_f2, act) : s;

@@ -210,6 +210,7 @@ private:
     int gemv_impl_ = 0;                // 0 = bulk-copy ring kernel, 1 = direct-load kernel
     int mmq_impl_ = 0;                 // 0 = by shape, 1 = bit-identical MMQ, 2 = batched GEMMs above 8 rows, 3 = GEMV walk
     Status check_device_status();
+    Status gemv_q8_rows(int dtype, const uint8_t *w, const Q8Dev &a, float *y, uint32_t m, uint32_t in_f, uint32_t out_f);
     // Batches of 9..32 rows (Q4_K, Q6_K; Q6_K up to 48 against few weights) through the wide GEMV.
     bool wide_applies(int dtype, uint32_t m, uint32_t in_f, uint64_t out_f, int act) const;
     Status wide_gemm(int dtype, const uint8_t *w, const Q8Dev &a, float *y, uint32_t m, uint32_t in_f, uint32_t out_f, float *partials,

@@ -44,3 +44,13 @@ def test_pair_with_one_result_over_the_rows(be, oracle, dt, m, first):
     be.linear_pair(dt, b1, y1, N, b2, y2, N, xb, m, N)
     for w, y in ((w1, y1), (w2, y2)):  # both from the rows as they were
         assert fx.rel_l2(be.download(y, np.float32).reshape(m, N), oracle.linear(dt, w, x, m, N, N)) < 1e-6
+
+
+@pytest.mark.parametrize("dt,m,in_f", [(Q6K, 5, 12544), (Q6K, 8, 14080), (Q4K, 8, 28672), (Q2_0, 8, 14080)])
+def test_pair_whose_rows_do_not_fit_a_cta_together(be, oracle, dt, m, in_f):
+    # in narrower batches, as a single call takes them
+    w1, w2 = synth.weight(dt, 40, in_f, seed=1), synth.weight(dt, 130, in_f, seed=2)
+    x, y1, y2 = synth.normal(3, (m, in_f)), be.alloc(m * 40 * 4), be.alloc(m * 130 * 4)
+    be.linear_pair(dt, be.from_numpy(w1), y1, 40, be.from_numpy(w2), y2, 130, be.from_numpy(x), m, in_f)
+    for w, y, n in ((w1, y1, 40), (w2, y2, 130)):
+        assert fx.rel_l2(be.download(y, np.float32).reshape(m, n), oracle.linear(dt, w, x, m, in_f, n)) < 1e-6
