@@ -12,7 +12,7 @@
 // the conversion to f32 is part of the instruction: the accumulator starts as the bit pattern of 1.5 * 2^23, so the int32 result
 // read as f32 is 1.5 * 2^23 + s, and one packed subtraction gives s exactly.
 //
-// What bounds it (profiles/batched_gemm_and_moe_kernels.md): issue and the f32 pipe.  Per 32 rows x 40 tokens x 64 elements a warp issues
+// What bounds it: issue and the f32 pipe.  Per 32 rows x 40 tokens x 64 elements a warp issues
 // 315 instructions, of them 20 matrix instructions and 100 packed f32 operations (2.5 per output and group), and moves that put the
 // start value into the accumulators (a conversion of the int32 sums instead costs as much); 0.49 instructions a cycle and scheduler, f32
 // pipe 41 %, matrix unit 25 % busy.

@@ -30,7 +30,7 @@
 // = a warp issuing under `lane == 0`, stages held until the epilogue, whole waves only):  Q4_K 4096 -> 14336, 512 rows 113 -> 82 (a call
 // that waits for the one before it: 112 -> 89), 113 rows 35 -> 30, 1024 rows 192 -> 153;  14336 -> 4096, 1024 rows 194 -> 175;  Q6_K
 // 14336 -> 4096, 113 rows 57 -> 53, 512 rows 183 -> 177.  Some Q6_K shapes lost: 33..64 rows of 4096 -> 14336 49 -> 52.
-// What bounds it (profiles/batched_gemm_and_moe_kernels.md): issue slots and waits.  At 128 tokens a Q4_K job takes ~2550 cycles, its MMAs
+// What bounds it: issue slots and waits.  At 128 tokens a Q4_K job takes ~2550 cycles, its MMAs
 // 1150 (tensor pipe 45 % busy); the warps issue 6670 instructions a job, 0.66 a cycle and scheduler.
 // Every wait is bounded: on expiry the role raises a CTA flag and a status word, every role leaves its loop, copies in
 // flight are drained and the tensor memory is freed.

@@ -303,7 +303,7 @@ __global__ void __launch_bounds__(KW * 32, 16 / KW)
 // plain bulk copy.  A warp owns whole tiles (all of K, two in flight) and stores its sums itself: no barrier between the warps of a CTA
 // after the staging of the activations.  A lane's rows start on any even address: its words are put together from two aligned loads
 // and a shift by 0 or 16 bits.
-// What bounds it (profiles/batched_gemm_and_moe_kernels.md): the chain of loads and instructions around 18 matrix instructions a block with
+// What bounds it: the chain of loads and instructions around 18 matrix instructions a block with
 // two warps a scheduler (0.46 instructions a cycle), and items of unequal size; shared memory is 44 % busy.  The weights of 105 experts
 // of 2048 x 768 are 135 MB = 21 us.  Measured there (27 rows, top-8 of 128): 51 us; the byte-dot kernel, whose lanes load 2 bytes at a
 // time, 196.
