@@ -348,6 +348,14 @@ Status CudaBackend::linear(int dtype, const uint8_t *w, const float *x, float *y
         if (e != cudaErrorInvalidValue) return cuda_status(e, "gemv_q2");
         cudaGetLastError();
     }
+    // One Q6_K row: quantised inside the GEMV.
+    if (dtype == DT_Q6K && m == 1 && act == INFR_ACT_INT8 && gemv_impl_ == 0 && !in_place && gemv_row_takes(dtype, (int)in_f)) {
+        const GemvRowMat mat{w, y, (int)out_f};
+        const cudaError_t e = launch_gemv_row(dtype, &mat, 1, nullptr, x, (int)in_f, dev_, status_dev_, stream_);
+        if (e == cudaSuccess) launches_++;
+        if (e != cudaErrorInvalidValue) return cuda_status(e, "gemv_row");
+        cudaGetLastError();
+    }
     if (act == INFR_ACT_F32 && in_place) {  // the f32 kernels read the rows while they store: from a copy
         Status s = ensure_scratch((size_t)m * in_f * 4);
         if (s.ok()) s = cuda_status(cudaMemcpyAsync(scratch(), x, (size_t)m * in_f * 4, cudaMemcpyDeviceToDevice, stream_), "linear: rows");
@@ -522,6 +530,13 @@ Status CudaBackend::linear_pair(int dtype, const uint8_t *w1, float *y1, uint32_
         // (in place: quantise first; results that overlap each other: one launch each, in order)
         const size_t nx = (size_t)m * in_f, n1 = (size_t)m * out_f1, n2 = (size_t)m * out_f2;
         const bool apart = !overlap(x, nx, y1, n1) && !overlap(x, nx, y2, n2) && !overlap(y1, n1, y2, n2);
+        if (m == 1 && gemv_impl_ == 0 && apart && gemv_row_takes(dtype, (int)in_f)) {
+            const GemvRowMat mats[2] = {{w1, y1, (int)out_f1}, {w2, y2, (int)out_f2}};
+            const cudaError_t e = launch_gemv_row(dtype, mats, 2, nullptr, x, (int)in_f, dev_, status_dev_, stream_);
+            if (e == cudaSuccess) launches_++;
+            if (e != cudaErrorInvalidValue) return cuda_status(e, "linear_pair");
+            cudaGetLastError();
+        }
         if (dtype == DT_Q4K && gemv_impl_ == 0 && in_f % 256 == 0 && apart) {
             // one kernel: the rows are quantised inside the GEMV while the first weights stream in
             const cudaError_t e = launch_gemv_q4k_mma_pair(w1, y1, (int)out_f1, w2, y2, (int)out_f2, nullptr, x, (int)m, (int)in_f, dev_,
@@ -585,6 +600,14 @@ Status CudaBackend::gemv_q8_pair(int dtype, const uint8_t *w1, float *y1, uint32
                                "gemv_q8_pair");
         if (s.ok()) launches_++;
         return s;
+    }
+    if (m == 1 && gemv_impl_ == 0 && out_f1 && out_f2 && a.gran == act_gran(dtype) && gemv_row_takes(dtype, (int)in_f) && !overlap(y1, out_f1, y2, out_f2)) {
+        cudaSetDevice(device_);
+        const GemvRowMat mats[2] = {{w1, y1, (int)out_f1}, {w2, y2, (int)out_f2}};
+        const cudaError_t e = launch_gemv_row(dtype, mats, 2, &a, nullptr, (int)in_f, dev_, status_dev_, stream_);
+        if (e == cudaSuccess) launches_++;
+        if (e != cudaErrorInvalidValue) return cuda_status(e, "gemv_q8_pair");
+        cudaGetLastError();
     }
     if (m > 8 && m <= 32 && out_f1 && out_f2 && wide_applies(dtype, m, in_f, (uint64_t)out_f1 + out_f2, INFR_ACT_INT8) && a.gran == 256 && (dtype != DT_Q6K || a.sums16)) {
         if (tc_wins(dtype, m, in_f, (uint64_t)out_f1 + out_f2)) {

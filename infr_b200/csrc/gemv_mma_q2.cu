@@ -187,10 +187,8 @@ __global__ void __launch_bounds__(KW * 32, 16 / KW)
                         const int2 bs = *reinterpret_cast<const int2 *>(s_bs + gi * 8 + n0);
                         accf[0] = fmaf(d0 * e.x, (float)(pr[0] - bs.x), accf[0]);
                         accf[2] = fmaf(d1 * e.x, (float)(pr[2] - bs.x), accf[2]);
-                        if (M > 1) {
-                            accf[1] = fmaf(d0 * e.y, (float)(pr[1] - bs.y), accf[1]);
-                            accf[3] = fmaf(d1 * e.y, (float)(pr[3] - bs.y), accf[3]);
-                        }
+                        accf[1] = fmaf(d0 * e.y, (float)(pr[1] - bs.y), accf[1]);
+                        accf[3] = fmaf(d1 * e.y, (float)(pr[3] - bs.y), accf[3]);
                     }
                 }
             }
@@ -302,8 +300,7 @@ cudaError_t launch_m(const uint8_t *w, const Q8Dev &a, float *y, int m, int in_f
 cudaError_t launch_gemv_q2_mma(const uint8_t *w, const Q8Dev &a, float *y, int m, int in_f, int out_f, const DeviceInfo &dev,
                                uint32_t *status, cudaStream_t st) {
     if (m < 1 || m > 8 || in_f % kChunkElems || a.gran != 32) return cudaErrorInvalidValue;
-    if (m == 1) return launch_m<1>(w, a, y, m, in_f, out_f, dev, status, st);
-    if (m == 2) return launch_m<2>(w, a, y, m, in_f, out_f, dev, status, st);
+    if (m <= 2) return launch_m<2>(w, a, y, m, in_f, out_f, dev, status, st);
     if (m <= 4) return launch_m<4>(w, a, y, m, in_f, out_f, dev, status, st);
     return launch_m<8>(w, a, y, m, in_f, out_f, dev, status, st);
 }

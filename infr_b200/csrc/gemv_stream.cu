@@ -507,6 +507,12 @@ cudaError_t launch_stream_m(int dt, const uint8_t *w, const Q8Dev &a, float *y, 
 cudaError_t launch_gemv_stream(int dt, const uint8_t *w, const Q8Dev &a, float *y, int m, int in_f, int out_f,
                                const DeviceInfo &dev, uint32_t *status, cudaStream_t st) {
     if (m < 1 || m > 8 || (dt != DT_Q4K && dt != DT_Q6K && dt != DT_Q2_0)) return cudaErrorInvalidValue;
+    if (dt == DT_Q2_0 && m == 1 && gemv_row_takes(dt, in_f) && a.gran == 32) {
+        const GemvRowMat mat{w, y, out_f};
+        const cudaError_t e = launch_gemv_row(dt, &mat, 1, &a, nullptr, in_f, dev, status, st);
+        if (e != cudaErrorInvalidValue) return e;
+        cudaGetLastError();
+    }
     if (dt == DT_Q2_0 && m > 1 && in_f % 512 == 0 && a.gran == 32) {
         // batches on rows of whole 512-element chunks take the matrix-unit kernel (1.6x faster at m = 4 and 8,
         // no gain at m = 1); it declines shapes whose staged activations do not fit, and those fall through
@@ -533,6 +539,12 @@ cudaError_t launch_gemv_q2_row(const uint8_t *w, float *y, int out_f, const uint
                                uint32_t *status, cudaStream_t st) {
     if (in_f < 64 || in_f % 64 || out_f < 1 || (w2 && out_f2 < 1) || (uintptr_t)x % 16) return cudaErrorInvalidValue;
     const Q8Dev none{nullptr, nullptr, nullptr, nullptr, 32};
+    if (gemv_row_takes(DT_Q2_0, in_f)) {
+        const GemvRowMat mats[2] = {{w, y, out_f}, {w2, y2, out_f2}};
+        const cudaError_t e = launch_gemv_row(DT_Q2_0, mats, w2 ? 2 : 1, nullptr, x, in_f, dev, status, st);
+        if (e != cudaErrorInvalidValue) return e;
+        cudaGetLastError();
+    }
     if (!w2) return launch_stream_dt<DT_Q2_0, 1, true>(w, none, y, 1, in_f, out_f, dev, status, st, x);
     return launch_stream_dt<DT_Q2_0, 1, true, true>(w, none, y, 1, in_f, out_f, dev, status, st, x, StreamSecond{w2, y2, out_f2});
 }
