@@ -1,6 +1,7 @@
 // CudaBackend: device memory, graph walking and op dispatch (host side).
 #include "backend.h"
 
+#include <algorithm>
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
@@ -351,7 +352,7 @@ Status CudaBackend::linear(int dtype, const uint8_t *w, const float *x, float *y
     // One Q6_K row: quantised inside the GEMV.
     if (dtype == DT_Q6K && m == 1 && act == INFR_ACT_INT8 && gemv_impl_ == 0 && !in_place && gemv_row_takes(dtype, (int)in_f)) {
         const GemvRowMat mat{w, y, (int)out_f};
-        const cudaError_t e = launch_gemv_row(dtype, &mat, 1, nullptr, x, (int)in_f, dev_, status_dev_, stream_);
+        const cudaError_t e = launch_gemv_row(GemvRow{dtype, (int)in_f, &mat, 1, nullptr, x}, dev_, status_dev_, stream_);
         if (e == cudaSuccess) launches_++;
         if (e != cudaErrorInvalidValue) return cuda_status(e, "gemv_row");
         cudaGetLastError();
@@ -532,7 +533,7 @@ Status CudaBackend::linear_pair(int dtype, const uint8_t *w1, float *y1, uint32_
         const bool apart = !overlap(x, nx, y1, n1) && !overlap(x, nx, y2, n2) && !overlap(y1, n1, y2, n2);
         if (m == 1 && gemv_impl_ == 0 && apart && gemv_row_takes(dtype, (int)in_f)) {
             const GemvRowMat mats[2] = {{w1, y1, (int)out_f1}, {w2, y2, (int)out_f2}};
-            const cudaError_t e = launch_gemv_row(dtype, mats, 2, nullptr, x, (int)in_f, dev_, status_dev_, stream_);
+            const cudaError_t e = launch_gemv_row(GemvRow{dtype, (int)in_f, mats, 2, nullptr, x}, dev_, status_dev_, stream_);
             if (e == cudaSuccess) launches_++;
             if (e != cudaErrorInvalidValue) return cuda_status(e, "linear_pair");
             cudaGetLastError();
@@ -561,6 +562,42 @@ Status CudaBackend::linear_pair(int dtype, const uint8_t *w1, float *y1, uint32_
     }
     Status s = linear(dtype, w1, x, y1, m, in_f, out_f1, act);
     return s.ok() ? linear(dtype, w2, x, y2, m, in_f, out_f2, act) : s;
+}
+
+Status CudaBackend::linear_row(const GemvRow &d, bool *taken) {
+    *taken = false;
+    if (reference_ || gemv_impl_ != 0 || !gemv_row_takes(d.dtype, d.in_f) || d.n < 1 || d.n > kGemvRowMats) return Status::Ok();
+    // Every CTA reads its row while others store: results lie apart from what is read and from each other.
+    struct Span {
+        uintptr_t a, b;
+        bool w;
+    } sp[2 * kGemvRowMats + 1];
+    int n = 0;
+    auto put = [&](const float *p, size_t k, bool w) {
+        if (p) sp[n++] = Span{(uintptr_t)p, (uintptr_t)p + 4 * k, w};
+    };
+    put(d.x, (size_t)d.in_f, false);
+    for (int i = 0; i < d.n; i++) {
+        put(d.mats[i].x, (size_t)d.in_f, false);
+        put(d.mats[i].y, (size_t)d.mats[i].out_f, true);
+    }
+    std::sort(sp, sp + n, [](const Span &p, const Span &q) { return p.a < q.a; });
+    uintptr_t end_any = 0, end_written = 0;
+    for (int i = 0; i < n; i++) {
+        if (sp[i].a < (sp[i].w ? end_any : end_written)) return Status::Ok();
+        if (sp[i].b > end_any) end_any = sp[i].b;
+        if (sp[i].w && sp[i].b > end_written) end_written = sp[i].b;
+    }
+    cudaSetDevice(device_);
+    const cudaError_t e = launch_gemv_row(d, dev_, status_dev_, stream_);
+    if (e == cudaErrorInvalidValue) {
+        cudaGetLastError();
+        return Status::Ok();
+    }
+    Status s = cuda_status(e, "gemv_row");
+    if (s.ok()) launches_++;
+    *taken = true;
+    return s;
 }
 
 Status CudaBackend::gemv_q8(int dtype, const uint8_t *w, const Q8Dev &a, float *y, uint32_t m, uint32_t in_f, uint32_t out_f) {
@@ -604,7 +641,7 @@ Status CudaBackend::gemv_q8_pair(int dtype, const uint8_t *w1, float *y1, uint32
     if (m == 1 && gemv_impl_ == 0 && out_f1 && out_f2 && a.gran == act_gran(dtype) && gemv_row_takes(dtype, (int)in_f) && !overlap(y1, out_f1, y2, out_f2)) {
         cudaSetDevice(device_);
         const GemvRowMat mats[2] = {{w1, y1, (int)out_f1}, {w2, y2, (int)out_f2}};
-        const cudaError_t e = launch_gemv_row(dtype, mats, 2, &a, nullptr, (int)in_f, dev_, status_dev_, stream_);
+        const cudaError_t e = launch_gemv_row(GemvRow{dtype, (int)in_f, mats, 2, &a}, dev_, status_dev_, stream_);
         if (e == cudaSuccess) launches_++;
         if (e != cudaErrorInvalidValue) return cuda_status(e, "gemv_q8_pair");
         cudaGetLastError();

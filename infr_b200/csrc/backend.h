@@ -26,7 +26,7 @@ struct infr_cuda_comm;  // comm.cu
 
 // One launch group of a compiled plan: a single op, or neighbouring ops one kernel computes.
 struct PlanStep {
-    enum Kind { kSingle = 0, kAddRmsNorm = 1, kRopeWriteKv = 2, kLinearPair = 3 };
+    enum Kind { kSingle = 0, kAddRmsNorm = 1, kRopeWriteKv = 2, kLinearPair = 3, kRow = 4, kRows = 5 };  // kRow, kRows: Linears of one row, on one row or each on its own
     int kind;
     uint32_t op0, n_ops;
 };
@@ -111,6 +111,9 @@ public:
     // out once for the tensor-memory GEMM; results are those of two `linear` calls.
     Status linear_pair(int dtype, const uint8_t *w1, float *y1, uint32_t out_f1, const uint8_t *w2, float *y2, uint32_t out_f2, const float *x,
                        uint32_t m, uint32_t in_f, int act);
+    // One-row Linears in one launch (gemv_row.cu).  *taken false: nothing was launched (the kernel does not take the call, spans overlap, or
+    // the options ask for another kernel) and the caller runs the ops one by one.
+    Status linear_row(const GemvRow &d, bool *taken);
     // Op::MoeFfn (crates/infr-cpu/src/lib.rs:2264-2984), qwen3moe configuration.  Optional debug outputs:
     // sel_ids [rows,n_used] i32, sel_w [rows,n_used] f32, logits [rows,n_expert] f32 (null = not wanted).
     struct MoeArgs {

@@ -621,7 +621,7 @@ cudaError_t launch_gemv_q4k_mma_pair(const uint8_t *w1, float *y1, int out_f1, c
     if (m < 1 || m > 8 || in_f % 256 || out_f1 < 1 || out_f2 < 1) return cudaErrorInvalidValue;
     if (m == 1) {
         const GemvRowMat mats[2] = {{w1, y1, out_f1}, {w2, y2, out_f2}};
-        return launch_gemv_row(DT_Q4K, mats, 2, a, x, in_f, dev, status, st);
+        return launch_gemv_row(GemvRow{DT_Q4K, in_f, mats, 2, a, x}, dev, status, st);
     }
     if (a) return launch_mma<false>(w1, *a, nullptr, y1, m, in_f, out_f1, dev, status, st, w2, y2, out_f2);
     Q8Dev none{nullptr, nullptr, nullptr, nullptr, 256};
@@ -633,7 +633,7 @@ cudaError_t launch_gemv_q4k_mma(const uint8_t *w, const Q8Dev *a, const float *x
     if (m < 1 || m > 8 || in_f % 256) return cudaErrorInvalidValue;
     if (m == 1) {
         const GemvRowMat mat{w, y, out_f};
-        return launch_gemv_row(DT_Q4K, &mat, 1, a, x, in_f, dev, status, st, push);
+        return launch_gemv_row(GemvRow{DT_Q4K, in_f, &mat, 1, a, x}, dev, status, st, push);
     }
     if (a) return launch_mma<false>(w, *a, nullptr, y, m, in_f, out_f, dev, status, st, nullptr, nullptr, 0, push);
     Q8Dev none{nullptr, nullptr, nullptr, nullptr, 256};

@@ -548,7 +548,7 @@ cudaError_t launch_gemv_q6_mma(const uint8_t *w, const Q8Dev &a, float *y, int m
     if (m < 1 || m > 8 || in_f % 2048 || a.gran != 256 || !a.sums16) return cudaErrorInvalidValue;
     if (m == 1) {
         const GemvRowMat mat{w, y, out_f};
-        return launch_gemv_row(DT_Q6K, &mat, 1, &a, nullptr, in_f, dev, status, st, push);
+        return launch_gemv_row(GemvRow{DT_Q6K, in_f, &mat, 1, &a}, dev, status, st, push);
     }
     if (m == 2) return launch_m6<2>(w, a, y, m, in_f, out_f, dev, status, st, push);
     if (m <= 4) return launch_m6<4>(w, a, y, m, in_f, out_f, dev, status, st, push);

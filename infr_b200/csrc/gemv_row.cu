@@ -387,13 +387,15 @@ __device__ __forceinline__ void half_q2(const uint8_t *p0, const uint8_t *p1, ui
     }
 }
 
-// Matrices with one in_f in one launch: their 16-row tiles follow each other in the CTAs' tile ranges.
+// Matrices with one in_f in one launch: their 16-row tiles follow each other in the CTAs' tile ranges.  NM > kSameRow: with a row each.
+constexpr int kSameRow = 3;
 template <int NM>
 struct RowMats {
     CUtensorMap map[NM];
     float *y[NM];
     int out_f[NM];
-    int tile_end[NM];  // tiles of matrices 0..i
+    int tile_end[NM];                       // tiles of matrices 0..i
+    const float *x[NM > kSameRow ? NM : 1];
 };
 struct RowGeom {
     int units, upw;  // K units of a row, of a warp
@@ -471,29 +473,38 @@ __global__ void __launch_bounds__(RowFmt<DT>::kWarps * 32, 2)
     if constexpr (PUSH) {
         if (threadIdx.x == 0) s_epoch = *reinterpret_cast<const volatile uint32_t *>(push.ctrl);  // read after the barrier of a batch
     }
-    [[maybe_unused]] RowAct<DT == DT_Q2_0 ? DT_Q4K : DT> act;
-    if constexpr (DT == DT_Q2_0) {
-        for (int u = 0; u < n_units; u++) put_act_q2<FUSED>(acts + (size_t)u * F::kActBytes, a, x, u0 + u, lane);
-        __syncwarp();
-    } else if constexpr (ONE) {
-        load_act<FUSED>(act, a, x, u0, lane);
-    } else {
-        int u = 0;
-        for (; u + 2 <= n_units; u += 2) {  // two units' loads in flight together
-            RowAct<DT> r0, r1;
-            load_act<FUSED>(r0, a, x, u0 + u, lane);
-            load_act<FUSED>(r1, a, x, u0 + u + 1, lane);
-            r0.put(acts + (size_t)u * F::kActBytes, lane);
-            r1.put(acts + (size_t)(u + 1) * F::kActBytes, lane);
-        }
-        if (u < n_units) {
-            load_act<FUSED>(act, a, x, u0 + u, lane);
-            act.put(acts + (size_t)u * F::kActBytes, lane);
-        }
-        __syncwarp();
+    int c_mat = 0, c_end = 0;  // the matrix whose row is in use, its last tile + 1
+    if (NM > kSameRow) {
+        while (t_begin >= mats.tile_end[c_mat]) c_mat++;
+        c_end = mats.tile_end[c_mat];
+        x = mats.x[c_mat];
     }
+    [[maybe_unused]] RowAct<DT == DT_Q2_0 ? DT_Q4K : DT> act;
     [[maybe_unused]] RowB4 b4;
-    if constexpr (DT == DT_Q4K && ONE) select_q4k(act, g, b4);
+    auto take_row = [&]() {
+        if constexpr (DT == DT_Q2_0) {
+            for (int u = 0; u < n_units; u++) put_act_q2<FUSED>(acts + (size_t)u * F::kActBytes, a, x, u0 + u, lane);
+            __syncwarp();
+        } else if constexpr (ONE) {
+            load_act<FUSED>(act, a, x, u0, lane);
+        } else {
+            int u = 0;
+            for (; u + 2 <= n_units; u += 2) {  // two units' loads in flight together
+                RowAct<DT> r0, r1;
+                load_act<FUSED>(r0, a, x, u0 + u, lane);
+                load_act<FUSED>(r1, a, x, u0 + u + 1, lane);
+                r0.put(acts + (size_t)u * F::kActBytes, lane);
+                r1.put(acts + (size_t)(u + 1) * F::kActBytes, lane);
+            }
+            if (u < n_units) {
+                load_act<FUSED>(act, a, x, u0 + u, lane);
+                act.put(acts + (size_t)u * F::kActBytes, lane);
+            }
+            __syncwarp();
+        }
+        if constexpr (DT == DT_Q4K && ONE) select_q4k(act, g, b4);
+    };
+    take_row();
 
     // ---- tiles ----
     int slot = 0;
@@ -502,6 +513,13 @@ __global__ void __launch_bounds__(RowFmt<DT>::kWarps * 32, 2)
     for (int b0 = 0; b0 < n_tiles; b0 += kPartTiles) {
         const int nb = min(kPartTiles, n_tiles - b0);
         for (int k = 0; k < nb; k++) {
+            if (NM > kSameRow && t_begin + b0 + k == c_end) {
+                c_mat++;
+                c_end = mats.tile_end[c_mat];
+                x = mats.x[c_mat];
+                __syncwarp();
+                take_row();
+            }
             float acc = 0.f;                               // of row g (t even) or g + 8 (t odd)
             [[maybe_unused]] float share[2] = {0.f, 0.f};  // Q2_0: this lane's shares of rows g, g + 8
             for (int u = 0; u < (ONE ? 1 : n_units); u++) {
@@ -548,26 +566,38 @@ __global__ void __launch_bounds__(RowFmt<DT>::kWarps * 32, 2)
             }
             if (t < 2) part0[k * kRowTile] = acc;
         }
-        __syncthreads();
-        for (int i = threadIdx.x; i < nb * kRowTile; i += blockDim.x) {
-            float v4[4] = {0.f, 0.f, 0.f, 0.f};  // (four chains: less latency, and fewer roundings of a growing sum)
-            for (int w = 0; w < kw; w += 4)
+        // a CTA has 32 threads or more, a batch 64 results
+        float *out[2];
+        int at[2] = {-1, -1};  // row of its matrix, -1: none
 #pragma unroll
-                for (int j = 0; j < 4; j++)
-                    if (w + j < kw) v4[j] += parts[(w + j) * kPartTiles * kRowTile + i];
-            const float v = (v4[0] + v4[1]) + (v4[2] + v4[3]);
+        for (int q = 0; q < 2; q++) {
+            const int i = threadIdx.x + q * blockDim.x;
+            if (i >= nb * kRowTile) break;
             int T = t_begin + b0 + i / kRowTile, mi = 0;
             if (NM > 1) {
                 while (T >= mats.tile_end[mi]) mi++;
                 if (mi) T -= mats.tile_end[mi - 1];
             }
             const int row = T * kRowTile + i % kRowTile;
-            if (row < mats.out_f[mi]) {
-                if constexpr (PUSH)
-                    push_store(push, s_epoch, (size_t)row, v);
-                else
-                    mats.y[mi][row] = v;
-            }
+            if (row >= mats.out_f[mi]) continue;
+            at[q] = row;
+            out[q] = mats.y[mi] + row;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int q = 0; q < 2; q++) {
+            const int i = threadIdx.x + q * blockDim.x;
+            if (at[q] < 0) continue;
+            float v4[4] = {0.f, 0.f, 0.f, 0.f};  // (four chains: less latency, and fewer roundings of a growing sum)
+            for (int w = 0; w < kw; w += 4)
+#pragma unroll
+                for (int j = 0; j < 4; j++)
+                    if (w + j < kw) v4[j] += parts[(w + j) * kPartTiles * kRowTile + i];
+            const float v = (v4[0] + v4[1]) + (v4[2] + v4[3]);
+            if constexpr (PUSH)
+                push_store(push, s_epoch, (size_t)at[q], v);
+            else
+                *out[q] = v;
         }
         if (b0 + kPartTiles < n_tiles) __syncthreads();
     }
@@ -656,35 +686,40 @@ cudaError_t launch_row(const RowMats<NM> &mats, const Q8Dev &a, const float *x, 
 }
 
 template <int DT, int NM>
-cudaError_t launch_row_dt(const GemvRowMat *m, const Q8Dev *a, const float *x, int in_f, const DeviceInfo &dev, uint32_t *status, cudaStream_t st,
-                          const GemvPush *push) {
+cudaError_t launch_row_dt(const GemvRow &d, const DeviceInfo &dev, uint32_t *status, cudaStream_t st, const GemvPush *push) {
     using F = RowFmt<DT>;
-    RowGeom geo{in_f / F::kUnit, 0, 0, 0};
+    RowGeom geo{d.in_f / F::kUnit, 0, 0, 0};
     geo.upw = (geo.units + F::kWarps - 1) / F::kWarps;
     const int kw = (geo.units + geo.upw - 1) / geo.upw;
     RowMats<NM> mats;
     memset(&mats, 0, sizeof mats);
-    for (int i = 0; i < NM; i++) {
-        if (!row_map<DT>(&mats.map[i], m[i].w, geo.units, m[i].out_f)) return cudaErrorInvalidValue;
-        mats.y[i] = m[i].y;
-        mats.out_f[i] = m[i].out_f;
-        geo.tiles += (m[i].out_f + kRowTile - 1) / kRowTile;
+    for (int i = 0; i < d.n; i++) {
+        if (!row_map<DT>(&mats.map[i], d.mats[i].w, geo.units, d.mats[i].out_f)) return cudaErrorInvalidValue;
+        mats.y[i] = d.mats[i].y;
+        mats.out_f[i] = d.mats[i].out_f;
+        geo.tiles += (d.mats[i].out_f + kRowTile - 1) / kRowTile;
         mats.tile_end[i] = geo.tiles;
+        if constexpr (NM > kSameRow) mats.x[i] = d.mats[i].x;
     }
+    for (int i = d.n; i < NM; i++) mats.tile_end[i] = geo.tiles;
     const Q8Dev none{nullptr, nullptr, nullptr, nullptr, 0};
-#define INFR_ROW(ONE_)                                                                                                                      \
-    do {                                                                                                                                    \
-        if (push) {                                                                                                                         \
-            if constexpr (NM == 1 && DT != DT_Q2_0) return launch_row<DT, NM, false, ONE_, true>(mats, *a, nullptr, geo, kw, dev, status, st, *push); \
-            return cudaErrorInvalidValue;                                                                                                   \
-        }                                                                                                                                   \
-        if (x) return launch_row<DT, NM, true, ONE_, false>(mats, none, x, geo, kw, dev, status, st, NoPush{});                             \
-        return launch_row<DT, NM, false, ONE_, false>(mats, *a, nullptr, geo, kw, dev, status, st, NoPush{});                               \
+    const bool one = geo.upw == 1 && DT != DT_Q2_0;
+#define INFR_ROW(FUSED_, PUSH_, A_, P_)                                                                                         \
+    do {                                                                                                                      \
+        if constexpr (DT != DT_Q2_0)                                                                                          \
+            if (one) return launch_row<DT, NM, FUSED_, true, PUSH_>(mats, A_, d.x, geo, kw, dev, status, st, P_);               \
+        return launch_row<DT, NM, FUSED_, false, PUSH_>(mats, A_, d.x, geo, kw, dev, status, st, P_);                           \
     } while (0)
-    if constexpr (DT != DT_Q2_0) {
-        if (geo.upw == 1) INFR_ROW(true);
+    if constexpr (NM > kSameRow) {
+        INFR_ROW(true, false, none, NoPush{});
+    } else {
+        if (push) {
+            if constexpr (NM == 1 && DT != DT_Q2_0) INFR_ROW(false, true, *d.codes, *push);
+            return cudaErrorInvalidValue;
+        }
+        if (d.codes) INFR_ROW(false, false, *d.codes, NoPush{});
+        INFR_ROW(true, false, none, NoPush{});
     }
-    INFR_ROW(false);
 #undef INFR_ROW
 }
 
@@ -695,23 +730,26 @@ bool gemv_row_takes(int dt, int in_f) {
     return dt == DT_Q4K ? in_f % 256 == 0 : dt == DT_Q6K ? in_f % 2048 == 0 : dt == DT_Q2_0 && in_f % 512 == 0;
 }
 
-cudaError_t launch_gemv_row(int dt, const GemvRowMat *m, int n_mats, const Q8Dev *a, const float *x, int in_f, const DeviceInfo &dev, uint32_t *status,
-                            cudaStream_t st, const GemvPush *push) {
-    if (!gemv_row_takes(dt, in_f) || (push && (x || n_mats != 1)) || (!a && !x)) return cudaErrorInvalidValue;
-    if (a && (a->gran != act_gran(dt) || (dt == DT_Q6K && !a->sums16))) return cudaErrorInvalidValue;
-    if (x && (uintptr_t)x % 16) return cudaErrorInvalidValue;
-    for (int i = 0; i < n_mats; i++)
-        if (m[i].out_f < 1) return cudaErrorInvalidValue;
-#define INFR_ROW_DT(N)                                                                                            \
-    do {                                                                                                          \
-        if (dt == DT_Q4K) return launch_row_dt<DT_Q4K, N>(m, a, x, in_f, dev, status, st, push);                  \
-        if (dt == DT_Q6K) return launch_row_dt<DT_Q6K, N>(m, a, x, in_f, dev, status, st, push);                  \
-        return launch_row_dt<DT_Q2_0, N>(m, a, x, in_f, dev, status, st, push);                                   \
+cudaError_t launch_gemv_row(const GemvRow &d, const DeviceInfo &dev, uint32_t *status, cudaStream_t st, const GemvPush *push) {
+    const int dt = d.dtype;
+    if (!gemv_row_takes(dt, d.in_f) || d.n < 1 || d.n > kGemvRowMats || (push && (!d.codes || d.n != 1))) return cudaErrorInvalidValue;
+    const bool own_rows = !d.codes && !d.x;
+    if (!own_rows && d.n > kSameRow) return cudaErrorInvalidValue;
+    if (d.codes && (d.codes->gran != act_gran(dt) || (dt == DT_Q6K && !d.codes->sums16))) return cudaErrorInvalidValue;
+    if (d.x && (uintptr_t)d.x % 16) return cudaErrorInvalidValue;
+    for (int i = 0; i < d.n; i++)
+        if (d.mats[i].out_f < 1 || (own_rows && (!d.mats[i].x || (uintptr_t)d.mats[i].x % 16))) return cudaErrorInvalidValue;
+#define INFR_ROW_DT(N)                                                                         \
+    do {                                                                                       \
+        if (dt == DT_Q4K) return launch_row_dt<DT_Q4K, N>(d, dev, status, st, push);           \
+        if (dt == DT_Q6K) return launch_row_dt<DT_Q6K, N>(d, dev, status, st, push);           \
+        return launch_row_dt<DT_Q2_0, N>(d, dev, status, st, push);                            \
     } while (0)
-    if (n_mats == 1) INFR_ROW_DT(1);
-    if (n_mats == 2) INFR_ROW_DT(2);
+    if (own_rows) INFR_ROW_DT(kGemvRowMats);
+    if (d.n == 1) INFR_ROW_DT(1);
+    if (d.n == 2) INFR_ROW_DT(2);
+    INFR_ROW_DT(3);
 #undef INFR_ROW_DT
-    return cudaErrorInvalidValue;
 }
 
 }  // namespace infr

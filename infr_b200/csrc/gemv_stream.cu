@@ -509,7 +509,7 @@ cudaError_t launch_gemv_stream(int dt, const uint8_t *w, const Q8Dev &a, float *
     if (m < 1 || m > 8 || (dt != DT_Q4K && dt != DT_Q6K && dt != DT_Q2_0)) return cudaErrorInvalidValue;
     if (dt == DT_Q2_0 && m == 1 && gemv_row_takes(dt, in_f) && a.gran == 32) {
         const GemvRowMat mat{w, y, out_f};
-        const cudaError_t e = launch_gemv_row(dt, &mat, 1, &a, nullptr, in_f, dev, status, st);
+        const cudaError_t e = launch_gemv_row(GemvRow{dt, in_f, &mat, 1, &a}, dev, status, st);
         if (e != cudaErrorInvalidValue) return e;
         cudaGetLastError();
     }
@@ -541,7 +541,7 @@ cudaError_t launch_gemv_q2_row(const uint8_t *w, float *y, int out_f, const uint
     const Q8Dev none{nullptr, nullptr, nullptr, nullptr, 32};
     if (gemv_row_takes(DT_Q2_0, in_f)) {
         const GemvRowMat mats[2] = {{w, y, out_f}, {w2, y2, out_f2}};
-        const cudaError_t e = launch_gemv_row(DT_Q2_0, mats, w2 ? 2 : 1, nullptr, x, in_f, dev, status, st);
+        const cudaError_t e = launch_gemv_row(GemvRow{DT_Q2_0, in_f, mats, w2 ? 2 : 1, nullptr, x}, dev, status, st);
         if (e != cudaErrorInvalidValue) return e;
         cudaGetLastError();
     }

@@ -89,16 +89,24 @@ cudaError_t launch_gemv_q4k_mma(const uint8_t *w, const Q8Dev *a, const float *x
 // gate and up: a decode step pays a fixed few microseconds per dependent launch).
 cudaError_t launch_gemv_q4k_mma_pair(const uint8_t *w1, float *y1, int out_f1, const uint8_t *w2, float *y2, int out_f2, const Q8Dev *a,
                                      const float *x, int m, int in_f, const DeviceInfo &dev, uint32_t *status, cudaStream_t st);
-// One row against n_mats (1, 2) matrices [out_f, in_f] of one format in one launch (gemv_row.cu): pre-quantised (`a`; Q6_K with the sums
-// per 16) or f32, quantised inside (`x`).  gemv_row_takes: formats and row lengths; cudaErrorInvalidValue: not taken.
+// One row against up to three matrices [out_f, in_f] of one format in one launch (gemv_row.cu), or up to kGemvRowMats matrices against an
+// f32 row each (mats[i].x; `x` and `codes` null).  gemv_row_takes: formats and row lengths; cudaErrorInvalidValue: not taken.
+constexpr int kGemvRowMats = 24;
 struct GemvRowMat {
     const uint8_t *w;
     float *y;
     int out_f;
+    const float *x = nullptr;
+};
+struct GemvRow {
+    int dtype, in_f;
+    const GemvRowMat *mats;
+    int n;
+    const Q8Dev *codes = nullptr;  // pre-quantised row (Q6_K: with the sums per 16), or
+    const float *x = nullptr;      // f32 row, quantised inside
 };
 bool gemv_row_takes(int dt, int in_f);
-cudaError_t launch_gemv_row(int dt, const GemvRowMat *m, int n_mats, const Q8Dev *a, const float *x, int in_f, const DeviceInfo &dev, uint32_t *status,
-                            cudaStream_t st, const GemvPush *push = nullptr);
+cudaError_t launch_gemv_row(const GemvRow &d, const DeviceInfo &dev, uint32_t *status, cudaStream_t st, const GemvPush *push = nullptr);
 // y[m,out_f] (m <= 8) from f32 activations and dequantised weights.
 cudaError_t launch_gemv_f32(int dt, const uint8_t *w, const float *x, float *y, int m, int in_f, int out_f,
                             const DeviceInfo &dev, cudaStream_t st);

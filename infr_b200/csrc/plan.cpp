@@ -8,6 +8,7 @@
 //                                        (runner.rs:3824-3838 emits exactly this pair between the two halves of a layer)
 //   Linear, Linear (same rows, same format) -> rows quantised once, one launch for a decode batch of Q4_K
 //                                        (runner.rs:3476-3523 q/k/v, :3882-3933 gate/up)
+//   one-row Linears of one format and length that do not depend on each other -> up to 24 in a launch (three on the same row)
 //   Rope(k), Rope(q), WriteKv, WriteKv -> q rotated in place, k rotated and v cast straight into the f16 caches
 //                                        (runner.rs:3611-3656), when the rotated k has no other reader
 // The grouped norm and rope launches compute the same values with the same roundings as the separate ops (the kernels
@@ -87,6 +88,31 @@ bool op_reads(const infr_op_desc &op, uint32_t id) {
         return true;
     }
     return false;
+}
+
+// A Linear of one row that the one-row GEMV can run.
+bool row_linear(const infr_cuda_plan &p, size_t j) {
+    if (j >= p.ops.size()) return false;
+    const infr_op_desc &o = p.ops[j];
+    return o.tag == INFR_OP_LINEAR && o.u[0] == 1 && o.u[2] > 0 && o.u[1] <= 0x7fffffffu && o.u[2] <= 0x7fffff00u && o.t[0] != o.t[2] &&
+           gemv_row_takes((int)p.tensors[o.t[1]].dtype, (int)o.u[1]);
+}
+// The number of ops from i on that are one-row Linears one launch can take together (below two: none).
+uint32_t row_run(const infr_cuda_plan &p, uint32_t i, bool *same_row) {
+    if (!row_linear(p, i)) return 0;
+    const infr_op_desc &a = p.ops[i];
+    auto fmt = [&](size_t j) { return p.tensors[p.ops[j].t[1]].dtype; };
+    uint32_t n = 1;
+    for (; n < (uint32_t)kGemvRowMats && row_linear(p, i + n) && fmt(i + n) == fmt(i) && p.ops[i + n].u[1] == a.u[1]; n++) {
+        const infr_op_desc &l = p.ops[i + n];
+        bool ok = true;
+        for (uint32_t k = i; ok && k < i + n; k++) ok = l.t[0] != p.ops[k].t[2] && l.t[2] != p.ops[k].t[2] && l.t[2] != p.ops[k].t[0];
+        if (!ok) break;
+    }
+    uint32_t same = 1;
+    while (same < n && p.ops[i + same].t[0] == a.t[0]) same++;
+    *same_row = same == n && n <= 3;
+    return n == 2 && *same_row ? 0 : n;  // (two on one row: kLinearPair)
 }
 
 }  // namespace
@@ -207,7 +233,11 @@ Status CudaBackend::compile(const infr_graph_desc &g, infr_cuda_plan **out) {
                 n.t[2] != a.t[1])
                 st = PlanStep{PlanStep::kAddRmsNorm, i, 2};
         }
-        if (a.tag == INFR_OP_LINEAR && i + 1 < g.n_ops) {
+        bool same_row = false;
+        const uint32_t run = row_run(*plan, i, &same_row);
+        if (run >= 2) {
+            st = PlanStep{same_row ? PlanStep::kRow : PlanStep::kRows, i, run};
+        } else if (a.tag == INFR_OP_LINEAR && i + 1 < g.n_ops) {
             // two Linears of one weight format reading the same rows (q and k, gate and up): quantised once
             const infr_op_desc &n = g.ops[i + 1];
             if (n.tag == INFR_OP_LINEAR && n.t[0] == a.t[0] && n.u[0] == a.u[0] && n.u[1] == a.u[1] &&
@@ -363,58 +393,8 @@ Status CudaBackend::execute_steps(infr_cuda_plan *plan, infr_cuda_buf *const *bi
     } while (0)
     auto f32p = [](const DevSpan &s) { return reinterpret_cast<float *>(s.ptr); };
 
-    for (const PlanStep &st : plan->steps) {
-        const infr_op_desc &op = plan->ops[st.op0];
+    auto run_single = [&](const infr_op_desc &op) -> Status {
         Status s;
-        if (st.kind == PlanStep::kAddRmsNorm) {
-            const infr_op_desc &nm = plan->ops[st.op0 + 1];
-            const uint32_t rows = nm.u[0], dim = nm.u[1];
-            const size_t nb = (size_t)rows * dim * 4;
-            DevSpan a, b, sum, w, dst;
-            INFR_RESOLVE(op.t[0], nb, "Add a", &a);
-            INFR_RESOLVE(op.t[1], nb, "Add b", &b);
-            INFR_RESOLVE(op.t[2], nb, "Add dst", &sum);
-            INFR_RESOLVE(nm.t[1], (size_t)dim * 4, "RmsNorm weight", &w);
-            INFR_RESOLVE(nm.t[2], nb, "RmsNorm dst", &dst);
-            s = rms_norm(f32p(a), f32p(b), f32p(sum), f32p(w), f32p(dst), rows, dim, nm.f[0]);
-            if (!s.ok()) return s;
-            continue;
-        }
-        if (st.kind == PlanStep::kLinearPair) {
-            const infr_op_desc &o2 = plan->ops[st.op0 + 1];
-            const uint32_t m = op.u[0], in_f = op.u[1];
-            const int wdt = (int)plan->tensors[op.t[1]].dtype;
-            const size_t bpr = (size_t)(in_f / block_elems(wdt)) * block_bytes(wdt);
-            const size_t r1 = op.u[3] / in_f, r2 = o2.u[3] / in_f;
-            DevSpan x, w1, w2, y1, y2;
-            INFR_RESOLVE(op.t[0], (size_t)m * in_f * 4, "Linear x", &x);
-            INFR_RESOLVE(op.t[1], (r1 + op.u[2]) * bpr, "Linear weight", &w1);
-            INFR_RESOLVE(o2.t[1], (r2 + o2.u[2]) * bpr, "Linear weight", &w2);
-            INFR_RESOLVE(op.t[2], (size_t)m * op.u[2] * 4, "Linear dst", &y1);
-            INFR_RESOLVE(o2.t[2], (size_t)m * o2.u[2] * 4, "Linear dst", &y2);
-            s = linear_pair(wdt, w1.ptr + r1 * bpr, f32p(y1), op.u[2], w2.ptr + r2 * bpr, f32p(y2), o2.u[2], f32p(x), m, in_f,
-                            reference_ ? INFR_ACT_F32 : INFR_ACT_INT8);
-            if (!s.ok()) return s;
-            continue;
-        }
-        if (st.kind == PlanStep::kRopeWriteKv) {
-            const infr_op_desc &rq = plan->ops[st.op0 + 1], &wk = plan->ops[st.op0 + 2], &wv = plan->ops[st.op0 + 3];
-            const uint32_t rows = op.u[0], nkv = op.u[1], hd = op.u[2], nh = rq.u[1], pos = wk.u[2];
-            DevSpan k, q, v, p, kc, vc;
-            INFR_RESOLVE(op.t[0], (size_t)rows * nkv * hd * 4, "Rope x (k)", &k);
-            INFR_RESOLVE(rq.t[0], (size_t)rows * nh * hd * 4, "Rope x (q)", &q);
-            INFR_RESOLVE(wv.t[0], (size_t)rows * nkv * hd * 4, "WriteKv src (v)", &v);
-            INFR_RESOLVE(op.t[1], (size_t)rows * 4, "Rope positions", &p);
-            const size_t cache_need = ((size_t)pos + rows) * nkv * hd * 2;
-            INFR_RESOLVE(wk.t[1], cache_need, "WriteKv cache (k)", &kc);
-            INFR_RESOLVE(wv.t[1], cache_need, "WriteKv cache (v)", &vc);
-            infr_attn_desc d{};
-            d.rows = rows, d.pos = pos, d.n_head = nh, d.n_kv = nkv, d.head_dim = hd, d.scale = 0.f, d.n_seq = 1, d.seq_stride = 0;
-            s = rope_write_kv(d, op.f[0], op.u[5] != 0, f32p(q), f32p(k), f32p(v), reinterpret_cast<const int32_t *>(p.ptr), kc.ptr, vc.ptr,
-                              (int)pos);
-            if (!s.ok()) return s;
-            continue;
-        }
         switch (op.tag) {
         case INFR_OP_LINEAR: {
             const uint32_t m = op.u[0], in_f = op.u[1], out_f = op.u[2], w_off = op.u[3];
@@ -524,8 +504,84 @@ Status CudaBackend::execute_steps(infr_cuda_plan *plan, infr_cuda_buf *const *bi
             s = cuda_status(cudaMemcpyAsync(dst.ptr + dof * 4, src.ptr + so * 4, nel * 4, cudaMemcpyDeviceToDevice, stream_), "Copy");
             break;
         }
-        default: return Status::Err(INFR_E_UNSUPPORTED, pfmt("execute: op %u tag %u", st.op0, op.tag));
+        default: return Status::Err(INFR_E_UNSUPPORTED, pfmt("execute: op %u tag %u", (uint32_t)(&op - plan->ops.data()), op.tag));
         }
+        return s;
+    };
+
+    for (const PlanStep &st : plan->steps) {
+        const infr_op_desc &op = plan->ops[st.op0];
+        Status s;
+        if (st.kind == PlanStep::kAddRmsNorm) {
+            const infr_op_desc &nm = plan->ops[st.op0 + 1];
+            const uint32_t rows = nm.u[0], dim = nm.u[1];
+            const size_t nb = (size_t)rows * dim * 4;
+            DevSpan a, b, sum, w, dst;
+            INFR_RESOLVE(op.t[0], nb, "Add a", &a);
+            INFR_RESOLVE(op.t[1], nb, "Add b", &b);
+            INFR_RESOLVE(op.t[2], nb, "Add dst", &sum);
+            INFR_RESOLVE(nm.t[1], (size_t)dim * 4, "RmsNorm weight", &w);
+            INFR_RESOLVE(nm.t[2], nb, "RmsNorm dst", &dst);
+            s = rms_norm(f32p(a), f32p(b), f32p(sum), f32p(w), f32p(dst), rows, dim, nm.f[0]);
+            if (!s.ok()) return s;
+            continue;
+        }
+        if (st.kind == PlanStep::kLinearPair) {
+            const infr_op_desc &o2 = plan->ops[st.op0 + 1];
+            const uint32_t m = op.u[0], in_f = op.u[1];
+            const int wdt = (int)plan->tensors[op.t[1]].dtype;
+            const size_t bpr = (size_t)(in_f / block_elems(wdt)) * block_bytes(wdt);
+            const size_t r1 = op.u[3] / in_f, r2 = o2.u[3] / in_f;
+            DevSpan x, w1, w2, y1, y2;
+            INFR_RESOLVE(op.t[0], (size_t)m * in_f * 4, "Linear x", &x);
+            INFR_RESOLVE(op.t[1], (r1 + op.u[2]) * bpr, "Linear weight", &w1);
+            INFR_RESOLVE(o2.t[1], (r2 + o2.u[2]) * bpr, "Linear weight", &w2);
+            INFR_RESOLVE(op.t[2], (size_t)m * op.u[2] * 4, "Linear dst", &y1);
+            INFR_RESOLVE(o2.t[2], (size_t)m * o2.u[2] * 4, "Linear dst", &y2);
+            s = linear_pair(wdt, w1.ptr + r1 * bpr, f32p(y1), op.u[2], w2.ptr + r2 * bpr, f32p(y2), o2.u[2], f32p(x), m, in_f,
+                            reference_ ? INFR_ACT_F32 : INFR_ACT_INT8);
+            if (!s.ok()) return s;
+            continue;
+        }
+        if (st.kind == PlanStep::kRopeWriteKv) {
+            const infr_op_desc &rq = plan->ops[st.op0 + 1], &wk = plan->ops[st.op0 + 2], &wv = plan->ops[st.op0 + 3];
+            const uint32_t rows = op.u[0], nkv = op.u[1], hd = op.u[2], nh = rq.u[1], pos = wk.u[2];
+            DevSpan k, q, v, p, kc, vc;
+            INFR_RESOLVE(op.t[0], (size_t)rows * nkv * hd * 4, "Rope x (k)", &k);
+            INFR_RESOLVE(rq.t[0], (size_t)rows * nh * hd * 4, "Rope x (q)", &q);
+            INFR_RESOLVE(wv.t[0], (size_t)rows * nkv * hd * 4, "WriteKv src (v)", &v);
+            INFR_RESOLVE(op.t[1], (size_t)rows * 4, "Rope positions", &p);
+            const size_t cache_need = ((size_t)pos + rows) * nkv * hd * 2;
+            INFR_RESOLVE(wk.t[1], cache_need, "WriteKv cache (k)", &kc);
+            INFR_RESOLVE(wv.t[1], cache_need, "WriteKv cache (v)", &vc);
+            infr_attn_desc d{};
+            d.rows = rows, d.pos = pos, d.n_head = nh, d.n_kv = nkv, d.head_dim = hd, d.scale = 0.f, d.n_seq = 1, d.seq_stride = 0;
+            s = rope_write_kv(d, op.f[0], op.u[5] != 0, f32p(q), f32p(k), f32p(v), reinterpret_cast<const int32_t *>(p.ptr), kc.ptr, vc.ptr,
+                              (int)pos);
+            if (!s.ok()) return s;
+            continue;
+        }
+        if (st.kind == PlanStep::kRow || st.kind == PlanStep::kRows) {
+            GemvRowMat mats[kGemvRowMats];
+            GemvRow d{(int)plan->tensors[op.t[1]].dtype, (int)op.u[1], mats, (int)st.n_ops};
+            const size_t in_b = (size_t)op.u[1] * 4, bpr = (size_t)(op.u[1] / block_elems(d.dtype)) * block_bytes(d.dtype);
+            for (uint32_t k = 0; k < st.n_ops; k++) {
+                const infr_op_desc &l = plan->ops[st.op0 + k];
+                const size_t r0 = l.u[3] / l.u[1];
+                DevSpan x, w, y;
+                INFR_RESOLVE(l.t[0], in_b, "Linear x", &x);
+                INFR_RESOLVE(l.t[1], (r0 + l.u[2]) * bpr, "Linear weight", &w);
+                INFR_RESOLVE(l.t[2], (size_t)l.u[2] * 4, "Linear dst", &y);
+                mats[k] = GemvRowMat{w.ptr + r0 * bpr, f32p(y), (int)l.u[2], st.kind == PlanStep::kRows ? f32p(x) : nullptr};
+                if (st.kind == PlanStep::kRow) d.x = f32p(x);
+            }
+            bool taken = false;
+            s = linear_row(d, &taken);
+            for (uint32_t k = 0; s.ok() && !taken && k < st.n_ops; k++) s = run_single(plan->ops[st.op0 + k]);
+            if (!s.ok()) return s;
+            continue;
+        }
+        s = run_single(op);
         if (!s.ok()) return s;
     }
 #undef INFR_RESOLVE

@@ -85,3 +85,59 @@ def test_row_infinite_scales(be, oracle, dt):
     np.testing.assert_array_equal(np.isnan(got), np.isnan(want))
     np.testing.assert_array_equal(got[~np.isfinite(want)], want[~np.isfinite(want)])
     assert fx.rel_l2(got[np.isfinite(want)], want[np.isfinite(want)]) < 2e-6
+
+
+@pytest.mark.parametrize("dt,in_f", [(Q4K, 2048), (Q4K, 4352), (Q6K, 4096), (Q2_0, 1024)])
+def test_plan_of_independent_rows(be, dt, in_f):
+    """Neighbouring one-row Linears that do not depend on each other are one launch per 24, with the bits of single calls; one whose row is
+    another's result, or whose result lies in another's buffer, is not grouped with it."""
+    count, n = 30, [16 + 37 * (i % 5) for i in range(30)]
+    ws = [be.from_numpy(synth.weight(dt, n[i], in_f, seed=i)) for i in range(count)]
+    xs = [be.from_numpy(synth.normal(100 + i, (1, in_f))) for i in range(count)]
+    want = []
+    for i in range(count):
+        y = be.alloc(n[i] * 4)
+        be.linear(dt, ws[i], xs[i], y, 1, in_f, n[i])
+        want.append(be.download(y, np.uint32))
+
+    def run(shared):
+        g, bind, outs = infr_b200.Graph(), {}, []
+        out = be.alloc(n[0] * 4)
+        for i in range(count):
+            a, w, c = g.input(in_f), g.weight(n[i] * in_f, dt), g.output(n[i])
+            g.linear(a, w, c, 1, in_f, n[i])
+            outs.append(out if shared and i in (0, 5) else be.alloc(n[i] * 4))
+            bind.update({a: xs[i], w: ws[i], c: outs[i]})
+        n0 = be.launch_count()
+        be.execute(be.compile(g), bind)
+        return be.launch_count() - n0, [be.download(o, np.uint32) for o in outs]
+
+    launches, got = run(False)
+    assert launches == 2
+    for a, b in zip(got, want):
+        np.testing.assert_array_equal(a, b)
+    launches, got = run(True)  # handles 0 and 5 bound to one buffer (same height): in order, the later one stays
+    assert launches > 2
+    for i, (a, b) in enumerate(zip(got, want)):
+        np.testing.assert_array_equal(a, want[5] if i == 0 else b)
+
+
+@pytest.mark.parametrize("dt,in_f", [(Q4K, 1024), (Q6K, 2048), (Q2_0, 1536)])
+def test_plan_of_three_on_one_row(be, dt, in_f):
+    """q, k and v of a model in one format: one launch, the bits of single calls."""
+    n = (300, 64, 17)
+    xb, ws = be.from_numpy(synth.normal(1, (1, in_f))), [be.from_numpy(synth.weight(dt, k, in_f, seed=k)) for k in n]
+    g, outs, want = infr_b200.Graph(), [be.alloc(k * 4) for k in n], []
+    a, bind = g.input(in_f), {}
+    for k, w, o in zip(n, ws, outs):
+        wh, oh = g.weight(k * in_f, dt), g.output(k)
+        g.linear(a, wh, oh, 1, in_f, k)
+        bind.update({wh: w, oh: o})
+        y = be.alloc(k * 4)
+        be.linear(dt, w, xb, y, 1, in_f, k)
+        want.append(be.download(y, np.uint32))
+    n0 = be.launch_count()
+    be.execute(be.compile(g), {a: xb, **bind})
+    assert be.launch_count() - n0 == 1
+    for o, y in zip(outs, want):
+        np.testing.assert_array_equal(be.download(o, np.uint32), y)
