@@ -12,14 +12,17 @@
 //
 // The warps of a CTA split K; a warp's units (Q4_K 256 elements, Q6_K and Q2_0 512) come by tiled TMA, 16 rows a box, through a ring of its
 // own.  (More slots a warp: the warps drift apart, neighbouring 144-byte pieces of a weight row are fetched at different times, and
-// 4096 -> 128256 takes 55 us with three slots and 68 with four instead of 49 with two.  One more warp that fetches for all: 4096 -> 4096
-// 3.1 us, but 4096 -> 14336 7.8 and Q6_K 10.8.)
-// Partial sums meet in shared memory every kPartTiles tiles, in a fixed order (the result does not depend on timing).
+// 4096 -> 128256 takes 55 us with three slots and 68 with four instead of 49 with two.)
+// Q4_K and Q6_K: every block's term meets the others in shared memory, a few tiles at a time, and the terms of a row are added in the order
+// that row_group says: that of the kernels for two rows and more, had they one.  (A sum in another order differs in a last bit here and
+// there, and 32 layers that code their activations in 8 bits carry that on to 0.01 .. 0.03 of a model's result.)  Q2_0: the warps' sums meet,
+// in a fixed order.
 // All waits are bounded; an expired one records a status word for the host.
 // Measured (us a call in a chain of calls on cold weights; before = the columns-are-rows kernels, or the byte-dot kernel for Q2_0; codes / f32
-// rows): Q4_K 4096 -> 4096 3.5 / 4.4 -> 3.3 / 3.5, 4096 -> 14336 7.5 / 9.4 -> 7.3 / 7.7, 14336 -> 4096 8.5 / 11.5 -> 7.9 / 9.7;  Q6_K
-// 4096 -> 4096 5.3 / 6.8 -> 4.2 / 4.3, 4096 -> 14336 13.1 / 15.1 -> 9.9 / 10.4, 4096 -> 128256 79 -> 65;  Q2_0 4096 -> 4096 4.5 / 5.6 -> 3.5 / 3.9,
-// 14336 -> 4096 8.4 / 10.4 -> 6.8 / 8.2, 4096 -> 128256 54 -> 39.
+// rows): Q4_K 4096 -> 4096 3.5 / 4.4 -> 3.6 / 3.9, 4096 -> 14336 7.5 / 9.4 -> 7.8 / 8.0, 14336 -> 4096 8.5 / 11.5 -> 8.0 / 9.9;  Q6_K
+// 4096 -> 4096 5.3 / 6.8 -> 4.5 / 4.5, 4096 -> 14336 13.1 / 15.1 -> 10.1 / 10.1, 4096 -> 128256 79 -> 65;  Q2_0 4096 -> 4096 4.5 / 5.6 -> 3.6 / 4.1,
+// 14336 -> 4096 8.4 / 10.4 -> 6.9 / 8.4, 4096 -> 128256 54 -> 38.  Between other launches (the decode step of an 8B model) the Q4_K shapes gain
+// more: their CTAs leave room for the launch before.  Lost: long Q4_K rows on few tiles, 5632 -> 2048 3.4 -> 3.7.
 // What bounds it: small matrices the chain from one launch to the next (1 us) and one round trip to L2 for the activations (0.3 us);
 // large ones memory (4096 -> 128256 at 0.92 of the measured copy rate, Q6_K 1.0); Q2_0 the integer pipe (64 masks a unit, half rate).
 #include <cuda.h>
@@ -35,24 +38,25 @@ namespace {
 
 constexpr int kRowTile = 16;
 constexpr int kRowSlots = 3;   // ring slots of a warp, at most
-constexpr int kPartTiles = 4;  // tiles whose partial sums wait for one barrier
 constexpr uint32_t kRowSpin = 1u << 22;
 
+// kPart: tiles whose sums wait for one barrier; kTerm: floats of a block's term (Q4_K: d * sum - dmin * min sum, times the row's scale when
+// it is added; Q6_K: both factors).
 // kUnit elements of a row are one box of 16 rows x kPitch bytes.  A Q6_K unit (two blocks, 420 bytes) starts on a multiple of 4: its box
 // starts at the 16-byte boundary below.  Pitches of 36 and 108 words put the eight rows of a read on distinct banks.
 template <int DT>
 struct RowFmt;
 template <>
 struct RowFmt<DT_Q4K> {
-    static constexpr int kUnit = 256, kPitch = 144, kActBytes = 256 + 32, kWarps = 16;
+    static constexpr int kUnit = 256, kPitch = 144, kActBytes = 256 + 32, kWarps = 16, kPart = 4, kTerm = 1;
 };
 template <>
 struct RowFmt<DT_Q6K> {
-    static constexpr int kUnit = 512, kPitch = 432, kActBytes = 512 + 64 + 16, kWarps = 8;
+    static constexpr int kUnit = 512, kPitch = 432, kActBytes = 512 + 64 + 16, kWarps = 8, kPart = 2, kTerm = 2;
 };
 template <>
 struct RowFmt<DT_Q2_0> {
-    static constexpr int kUnit = 512, kPitch = 144, kActBytes = 512 + 128, kWarps = 16;
+    static constexpr int kUnit = 512, kPitch = 144, kActBytes = 512 + 128, kWarps = 16, kPart = 4, kTerm = 1;
 };
 
 __device__ __forceinline__ uint32_t rs32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -266,8 +270,8 @@ __device__ __forceinline__ int quad_sum(const int (&v)[2], int t) {
     return s + __shfl_xor_sync(0xffffffffu, s, 2);
 }
 
-// ---- one unit of 16 rows: adds to the lane's sum of row g (t even) or g + 8 (t odd).  A block's integer sum is complete before it is
-// converted and scaled, so every block contributes the CPU's value. ----
+// ---- one unit of 16 rows: the block's term in row g (t even) or g + 8 (t odd).  A block's integer sum is complete before it is converted
+// and scaled, so every block contributes the CPU's value. ----
 // Q4_K: columns 2p, 2p + 1 = sub-blocks of the low and the high nibbles of run p.  Of the bytes of a run only the low nibbles are masked out:
 //   masked bytes x (codes of 2p in column 2p, NEGATED codes of 2p + 1 in column 2p + 1)  +  whole bytes x (codes of 2p + 1 in column 2p + 1)
 // leaves 16 x the high nibbles' sum in column 2p + 1.  (The integer pipe has half rate: its instructions are what a unit costs, a mask per
@@ -285,7 +289,7 @@ __device__ __forceinline__ void select_q4k(const RowAct<DT_Q4K> &r, int g, RowB4
         b.lo[p][0] = on ? n0 : 0u, b.lo[p][1] = on ? n1 : 0u, b.hi[p][0] = on ? m0 : 0u, b.hi[p][1] = on ? m1 : 0u;
     }
 }
-__device__ __forceinline__ void unit_q4k(const uint8_t *sl, int lane, const RowAct<DT_Q4K> &r, const RowB4 &b, float &acc) {
+__device__ __forceinline__ float unit_q4k(const uint8_t *sl, int lane, const RowAct<DT_Q4K> &r, const RowB4 &b) {
     const int g = lane >> 2, t = lane & 3;
     const uint32_t at = rs32(sl) + ((lane & 7) + (lane & 8)) * 144 + 16 + (lane >> 4) * 16;
     int d0[4], d1[4];
@@ -307,7 +311,7 @@ __device__ __forceinline__ void unit_q4k(const uint8_t *sl, int lane, const RowA
         sm[i] = dp2a_hi_su(r.bs, k4);
     }
     const uint32_t dd = (t & 1) ? h[1].x : h[0].x;
-    acc += r.d * (h2f(dd) * (float)quad_sum(sd, t) - h2f(dd >> 16) * (float)quad_sum(sm, t));
+    return __fmaf_rn(h2f(dd), (float)quad_sum(sd, t), -__fmul_rn(h2f(dd >> 16), (float)quad_sum(sm, t)));
 }
 
 // word at byte offset `off` (a multiple of 4) of a block that starts at p; ODD: p is 2 bytes past a word boundary
@@ -319,7 +323,7 @@ __device__ __forceinline__ uint32_t word6(const uint8_t *p, int off) {
 }
 // p0, p1: the block in rows g and g + 8
 template <bool ODD>
-__device__ __forceinline__ void block_q6k(const uint8_t *p0, const uint8_t *p1, int lane, const uint32_t (&code)[2], const uint32_t (&bs)[2], float d, float &acc) {
+__device__ __forceinline__ float2 block_q6k(const uint8_t *p0, const uint8_t *p1, int lane, const uint32_t (&code)[2], const uint32_t (&bs)[2], float d) {
     const int g = lane >> 2, t = lane & 3;
     int pr[2][4];  // [n]: column s = sub-block 8n + s
 #pragma unroll
@@ -349,7 +353,7 @@ __device__ __forceinline__ void block_q6k(const uint8_t *p0, const uint8_t *p1, 
         isum[i] = sext8(sc, 0) * pr[0][2 * i] + sext8(sc, 1) * pr[0][2 * i + 1] + sext8(sc, 2) * pr[1][2 * i] + sext8(sc, 3) * pr[1][2 * i + 1] -
                   32 * dp2a_ss(bs[0], bs[1], sc);
     }
-    acc = fmaf(h2f(lds16(((t & 1) ? p1 : p0) + 208)) * d, (float)quad_sum(isum, t), acc);
+    return make_float2(__fmul_rn(h2f(lds16(((t & 1) ? p1 : p0) + 208)), d), (float)quad_sum(isum, t));
 }
 
 // Half a Q2_0 unit (4 blocks of 64): lane t has block t of rows g, g + 8; the sums of its groups 2t, 2t + 1 end up in its own columns.
@@ -395,6 +399,7 @@ struct RowMats {
     float *y[NM];
     int out_f[NM];
     int tile_end[NM];                       // tiles of matrices 0..i
+    int group[NM];                          // Q4_K, Q6_K: blocks added before their sum is added to the others'
     const float *x[NM > kSameRow ? NM : 1];
 };
 struct RowGeom {
@@ -413,7 +418,11 @@ __global__ void __launch_bounds__(RowFmt<DT>::kWarps * 32, 2)
     extern __shared__ __align__(128) uint8_t smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3, kw = blockDim.x >> 5, S = geo.slots;
     uint8_t *acts = smem + (size_t)S * kw * kBox;                                                                       // [units][kActBytes]
-    float *parts = reinterpret_cast<float *>(acts + (ONE && DT != DT_Q2_0 ? 0 : (size_t)geo.units * F::kActBytes));  // [kw][kPartTiles * 16]
+    // sums that wait for a barrier, twice: Q2_0 [warp][kPart * 16], else [block][kPart * 16 + 4] terms, and the blocks' activation scales behind them
+    constexpr int kCols = F::kPart * kRowTile, kStride = DT == DT_Q2_0 ? kCols : (kCols + 4) * F::kTerm, kBlocks = DT == DT_Q6K ? 2 : 1;
+    float *parts = reinterpret_cast<float *>(acts + (ONE && DT != DT_Q2_0 ? 0 : (size_t)geo.units * F::kActBytes));
+    const int buf = (DT == DT_Q2_0 ? kw : geo.units * kBlocks) * kStride;  // of two buffers
+    [[maybe_unused]] float *s_scale = parts + 2 * buf;
     __shared__ __align__(8) uint64_t s_bars[F::kWarps * kRowSlots];
     __shared__ __align__(16) uint32_t s_zero[8];
     __shared__ int s_dead;
@@ -503,25 +512,36 @@ __global__ void __launch_bounds__(RowFmt<DT>::kWarps * 32, 2)
             __syncwarp();
         }
         if constexpr (DT == DT_Q4K && ONE) select_q4k(act, g, b4);
+        if constexpr (DT == DT_Q4K) {
+            if (ONE) {
+                if (lane == 0) s_scale[u0] = act.d;
+            } else {
+                for (int u = lane; u < n_units; u += 32) s_scale[u0 + u] = reinterpret_cast<const float *>(acts + (size_t)u * F::kActBytes + 256)[1];
+            }
+        }
     };
     take_row();
 
     // ---- tiles ----
     int slot = 0;
     uint32_t ph = 0;
-    float *part0 = parts + warp * kPartTiles * kRowTile + g + 8 * t;
-    for (int b0 = 0; b0 < n_tiles; b0 += kPartTiles) {
-        const int nb = min(kPartTiles, n_tiles - b0);
-        for (int k = 0; k < nb; k++) {
-            if (NM > kSameRow && t_begin + b0 + k == c_end) {
+    int batch = 0;
+    for (int b0 = 0, nb; b0 < n_tiles; b0 += nb) {
+        float *sums = parts + (size_t)(batch & 1) * buf;
+        nb = min(F::kPart, n_tiles - b0);
+        if (NM > kSameRow) {  // a batch is of one row
+            if (t_begin + b0 == c_end) {
                 c_mat++;
                 c_end = mats.tile_end[c_mat];
                 x = mats.x[c_mat];
-                __syncwarp();
+                __syncthreads();  // the scales of the last row are read
                 take_row();
             }
-            float acc = 0.f;                               // of row g (t even) or g + 8 (t odd)
+            nb = min(nb, c_end - (t_begin + b0));
+        }
+        for (int k = 0; k < nb; k++) {
             [[maybe_unused]] float share[2] = {0.f, 0.f};  // Q2_0: this lane's shares of rows g, g + 8
+            float *out0 = sums + (DT == DT_Q2_0 ? warp : u0 * kBlocks) * kStride + (k * kRowTile + g + 8 * t) * F::kTerm;  // lanes t = 0, 1
             for (int u = 0; u < (ONE ? 1 : n_units); u++) {
                 if (!row_try(bar0 + 8 * slot, ph) && !row_wait_slow(bar0 + 8 * slot, ph, &s_dead)) {
                     // the launch's results are invalid: no more fetches, and those in flight land before the block gives its shared memory back
@@ -537,12 +557,17 @@ __global__ void __launch_bounds__(RowFmt<DT>::kWarps * 32, 2)
                         act.get(acts + (size_t)u * F::kActBytes, lane);
                         select_q4k(act, g, b4);
                     }
-                    unit_q4k(sl, lane, act, b4, acc);
+                    const float x4 = unit_q4k(sl, lane, act, b4);
+                    if (t < 2) out0[u * kStride] = x4;
                 } else if constexpr (DT == DT_Q6K) {
                     if (!ONE) act.get(acts + (size_t)u * F::kActBytes, lane);
                     const uint8_t *p0 = sl + g * F::kPitch + 4 * ((u0 + u) & 3), *p1 = p0 + 8 * F::kPitch;
-                    block_q6k<false>(p0, p1, lane, act.c[0], act.bs[0], act.d[0], acc);
-                    block_q6k<true>(p0 + 210, p1 + 210, lane, act.c[1], act.bs[1], act.d[1], acc);
+                    const float2 x0 = block_q6k<false>(p0, p1, lane, act.c[0], act.bs[0], act.d[0]);
+                    const float2 x1 = block_q6k<true>(p0 + 210, p1 + 210, lane, act.c[1], act.bs[1], act.d[1]);
+                    if (t < 2) {
+                        *reinterpret_cast<float2 *>(out0 + 2 * u * kStride) = x0;
+                        *reinterpret_cast<float2 *>(out0 + (2 * u + 1) * kStride) = x1;
+                    }
                 } else {
                     const uint8_t *rec = acts + (size_t)u * F::kActBytes;
                     const uint32_t mis = 2 * (t & 1);
@@ -561,45 +586,83 @@ __global__ void __launch_bounds__(RowFmt<DT>::kWarps * 32, 2)
                 if (++slot == S) slot = 0, ph ^= 1u;
             }
             if constexpr (DT == DT_Q2_0) {
-                acc = ((t & 1) ? share[1] : share[0]) + __shfl_xor_sync(0xffffffffu, (t & 1) ? share[0] : share[1], 1);
+                float acc = ((t & 1) ? share[1] : share[0]) + __shfl_xor_sync(0xffffffffu, (t & 1) ? share[0] : share[1], 1);
                 acc += __shfl_xor_sync(0xffffffffu, acc, 2);
+                if (t < 2) *out0 = acc;
             }
-            if (t < 2) part0[k * kRowTile] = acc;
         }
-        // a CTA has 32 threads or more, a batch 64 results
-        float *out[2];
-        int at[2] = {-1, -1};  // row of its matrix, -1: none
-#pragma unroll
-        for (int q = 0; q < 2; q++) {
-            const int i = threadIdx.x + q * blockDim.x;
-            if (i >= nb * kRowTile) break;
+        __syncthreads();
+        auto store = [&](int i, float v) {
             int T = t_begin + b0 + i / kRowTile, mi = 0;
             if (NM > 1) {
                 while (T >= mats.tile_end[mi]) mi++;
                 if (mi) T -= mats.tile_end[mi - 1];
             }
             const int row = T * kRowTile + i % kRowTile;
-            if (row >= mats.out_f[mi]) continue;
-            at[q] = row;
-            out[q] = mats.y[mi] + row;
-        }
-        __syncthreads();
+            if (row < mats.out_f[mi]) {
+                if constexpr (PUSH)
+                    push_store(push, s_epoch, (size_t)row, v);
+                else
+                    mats.y[mi][row] = v;
+            }
+        };
+        auto add_term = [&](const float *col, int b, float acc) {
+            if (DT == DT_Q4K) return __fmaf_rn(s_scale[b], col[b * kStride], acc);
+            const float2 x2 = *reinterpret_cast<const float2 *>(col + b * kStride);
+            return __fmaf_rn(x2.x, x2.y, acc);
+        };
+        const int blocks = geo.units * kBlocks;
+        if constexpr (!ONE && DT != DT_Q2_0) {
+            // Long rows: eight threads a result, each adds groups of blocks in order, and the groups are added in order (14336 -> 4096: 8.0 us,
+            // with one thread a result 8.8).  A warp's four results are of one tile.
+            for (int i = threadIdx.x >> 3; i < nb * kRowTile; i += blockDim.x >> 3) {
+                int mi = 0;
+                if (NM > 1)
+                    while (t_begin + b0 + i / kRowTile >= mats.tile_end[mi]) mi++;
+                const int gs = mats.group[mi], q = threadIdx.x & 7;
+                const float *col = sums + i * F::kTerm;
+                float part[2] = {0.f, 0.f}, v = 0.f;  // groups q and q + 8: at most 16
 #pragma unroll
-        for (int q = 0; q < 2; q++) {
-            const int i = threadIdx.x + q * blockDim.x;
-            if (at[q] < 0) continue;
-            float v4[4] = {0.f, 0.f, 0.f, 0.f};  // (four chains: less latency, and fewer roundings of a growing sum)
-            for (int w = 0; w < kw; w += 4)
+                for (int h = 0; h < 2; h++)
+                    for (int b = (q + 8 * h) * gs; b < min(blocks, (q + 8 * h + 1) * gs); b++) part[h] = add_term(col, b, part[h]);
 #pragma unroll
-                for (int j = 0; j < 4; j++)
-                    if (w + j < kw) v4[j] += parts[(w + j) * kPartTiles * kRowTile + i];
-            const float v = (v4[0] + v4[1]) + (v4[2] + v4[3]);
-            if constexpr (PUSH)
-                push_store(push, s_epoch, (size_t)at[q], v);
-            else
-                *out[q] = v;
+                for (int h = 0; h < 2; h++)
+                    if (h == 0 || blocks > 8 * gs)
+#pragma unroll
+                        for (int gr = 0; gr < 8; gr++) v += __shfl_sync(0xffffffffu, part[h], gr, 8);
+                if (q == 0) store(i, v);
+            }
+        } else {
+            // A thread a result, on two warps that change from batch to batch; the others go on (two buffers of sums).
+            for (int i = (int)threadIdx.x - batch * kCols % (int)blockDim.x; i < nb * kRowTile; i += blockDim.x) {
+                if (i < 0) i += blockDim.x;
+                if (i >= nb * kRowTile) break;
+                const float *col = sums + i * F::kTerm;
+                float v = 0.f;
+                if constexpr (DT == DT_Q2_0) {
+                    float v4[4] = {0.f, 0.f, 0.f, 0.f};  // (four chains: less latency, and fewer roundings of a growing sum)
+                    for (int w = 0; w < kw; w += 4)
+#pragma unroll
+                        for (int j = 0; j < 4; j++)
+                            if (w + j < kw) v4[j] += col[(w + j) * kStride];
+                    v = (v4[0] + v4[1]) + (v4[2] + v4[3]);
+                } else {
+                    int mi = 0;
+                    if (NM > 1)
+                        while (t_begin + b0 + i / kRowTile >= mats.tile_end[mi]) mi++;
+                    const int gs = mats.group[mi];
+                    float acc = 0.f;
+                    int left = gs;
+#pragma unroll 4
+                    for (int b = 0; b < blocks; b++) {
+                        acc = add_term(col, b, acc);
+                        if (--left == 0 || b == blocks - 1) v += acc, acc = 0.f, left = gs;
+                    }
+                }
+                store(i, v);
+            }
         }
-        if (b0 + kPartTiles < n_tiles) __syncthreads();
+        batch++;
     }
 }
 
@@ -648,7 +711,9 @@ template <int DT, int NM, bool FUSED, bool ONE, bool PUSH>
 cudaError_t launch_row(const RowMats<NM> &mats, const Q8Dev &a, const float *x, RowGeom geo, int kw, const DeviceInfo &dev, uint32_t *status, cudaStream_t st,
                        const typename PushParam<PUSH>::type &push) {
     using F = RowFmt<DT>;
-    const size_t fixed = (ONE && DT != DT_Q2_0 ? 0 : (size_t)geo.units * F::kActBytes) + (size_t)kw * kPartTiles * kRowTile * 4;
+    const size_t cols = F::kPart * kRowTile, blocks = (size_t)geo.units * (DT == DT_Q6K ? 2 : 1);
+    const size_t fixed = (ONE && DT != DT_Q2_0 ? 0 : (size_t)geo.units * F::kActBytes) +
+                         (DT == DT_Q2_0 ? 2 * (size_t)kw * cols : 2 * blocks * (cols + 4) * F::kTerm + (DT == DT_Q4K ? blocks : 0)) * 4;
     const size_t per_slot = (size_t)kw * kRowTile * F::kPitch;
     // Several CTAs a SM where rows are short and each has a tile: more warps at work, but each CTA reads (or quantises) the row for itself.
     // (us with one CTA a SM / as many as have a tile: Q4_K 2048 -> 5632 3.0 / 2.5, Q6_K 4096 -> 14336 10.0 / 9.5; Q2_0 4096 -> 4096 with two
@@ -685,6 +750,25 @@ cudaError_t launch_row(const RowMats<NM> &mats, const Q8Dev &a, const float *x, 
     return cudaLaunchKernelEx(&cfg, kernel, mats, a, x, geo, status, push);
 }
 
+// Blocks of a row that are added before their sum is added to the others': the K split over 4, 8 or 16 warps that the kernels for two rows and
+// more (gemv_mma.cu, gemv_mma_q6.cu) choose by the number of 16-row tiles and by what fits beside `nb` blocks of one staged row, so that a
+// result keeps the bits it has there.
+int row_group(int dt, int nb, int tiles, const DeviceInfo &dev) {
+    const size_t top = (size_t)dev.max_smem_optin;
+    auto need = [&](int kw, int units) {  // shared memory with `units` ring slots of a block a warp
+        return (size_t)nb * (dt == DT_Q4K ? 368 : 384) + (size_t)kw * 1056 + 64 + (size_t)units * kw * kRowTile * (dt == DT_Q4K ? 144 : 224);
+    };
+    auto two = [&](int kw) { return need(kw, dt == DT_Q4K && (nb + kw - 1) / kw > 1 ? 4 : 2); };
+    const int kw0 = tiles > 2 * dev.sm_count ? 4 : tiles > dev.sm_count ? 8 : 16;
+    int kw = kw0;
+    if (dt == DT_Q6K && kw == 4 && need(4, 3) > top / 4 - 2048) kw = 8;
+    while (kw < 16 && two(kw) > top / (16 / kw) - 2048) kw *= 2;
+    while (kw > 4 && kw > nb) kw /= 2;
+    while (kw > 4 && two(kw) > top - 1024) kw /= 2;
+    if (dt == DT_Q4K && kw == 16 && kw0 < 16 && nb >= 8 && need(8, 2) <= top / 2 - 2048) kw = 8;
+    return (nb + kw - 1) / kw;
+}
+
 template <int DT, int NM>
 cudaError_t launch_row_dt(const GemvRow &d, const DeviceInfo &dev, uint32_t *status, cudaStream_t st, const GemvPush *push) {
     using F = RowFmt<DT>;
@@ -702,6 +786,12 @@ cudaError_t launch_row_dt(const GemvRow &d, const DeviceInfo &dev, uint32_t *sta
         if constexpr (NM > kSameRow) mats.x[i] = d.mats[i].x;
     }
     for (int i = d.n; i < NM; i++) mats.tile_end[i] = geo.tiles;
+    if constexpr (DT != DT_Q2_0) {
+        auto tiles = [&](int i) { return (d.mats[i].out_f + kRowTile - 1) / kRowTile; };
+        // (two Q4_K matrices on one row are split as one)
+        for (int i = 0; i < d.n; i++)
+            mats.group[i] = row_group(DT, d.in_f / 256, DT == DT_Q4K && NM <= kSameRow && d.n > 1 && i < 2 ? tiles(0) + tiles(1) : tiles(i), dev);
+    }
     const Q8Dev none{nullptr, nullptr, nullptr, nullptr, 0};
     const bool one = geo.upw == 1 && DT != DT_Q2_0;
 #define INFR_ROW(FUSED_, PUSH_, A_, P_)                                                                                         \
