@@ -199,21 +199,18 @@ constexpr int kAttnThreads = 256;  // eight warps: 16 keys each in the score pha
 // every global request is a whole 128-byte line; all copies of the CTA are in flight together and none occupies a
 // register.
 //
-// Both products run on the warp-level matrix unit in tf32 WITHOUT giving up f32 operands: an f16 cache value is exact
-// in tf32 (10 mantissa bits), and the f32 operand (q, then the softmax weights p) is split into two tf32 pieces,
-// hi = the top 11 significant bits, mid = the next 11 of the remainder, which sit in two neighbouring columns of the
-// instruction's N dimension and are added afterwards; what is dropped is below 2^-22 of the operand, the size of the
-// rounding of an f32 accumulation itself.  Products are exact, sums are f32.  This takes the instruction count of a tile
-// from ~7100 (scalar FMAs on converted halves, which cost more issue slots than the tile's bytes cost HBM time) to
-// ~2800.
-// Phase 1: warp w scores keys 16w..16w+15 against the G query heads that share the KV head: A = the keys (ldmatrix,
-// halves -> f32), B = the q pieces, K = head_dim in steps of 8.  Phase 2: one warp per head turns the tile's scores into
-// exp(s - m), their sum, and the two tf32 pieces of each weight.  Phase 3: warp w owns output dims 16 (w mod HD/16):
+// Both products run on the warp-level matrix unit in f16 WITHOUT giving up f32 operands: the cache values are f16, and the f32 operand (q,
+// then the softmax weights p) is split into two f16 pieces, hi = its top 11 significant bits, mid = the next 11 of the remainder times 2^11,
+// which sit in two neighbouring columns of the instruction's N dimension and are added afterwards; what is dropped is below 2^-22 of the
+// operand, the size of the rounding of an f32 accumulation itself.  A power of two per head brings the largest |q| to 2^14 .. 2^15, weights
+// (at most 1) are multiplied by 2^15: an element down to 2^-26 of the largest keeps all these bits, one below that an error of 2^-49 of it.
+// Products are exact, sums are f32.  (The same split in tf32 pieces, with the same bits, had to widen every half of the tile to 32 bits first: a batch of 32 sequences at 4097 keys 113 -> 95 us a layer.)
+// Phase 1: warp w scores keys 16w..16w+15 against the G query heads that share the KV head: A = the keys (ldmatrix),
+// B = the q pieces, K = head_dim in steps of 8.  Phase 2: one warp per head turns the tile's scores into
+// exp(s - m), their sum, and the two pieces of each weight.  Phase 3: warp w owns output dims 16 (w mod HD/16):
 // A = the values transposed (ldmatrix.trans), B = the weight pieces, K = the keys in steps of 8; with head_dim 64 the
 // two halves of the keys go to two warps and meet in shared memory (over the key tile, dead by then).  The tile's
 // (m, l, o) goes to the workspace for the merge kernel.
-// The K index of the instruction is only a summation index: slot t takes element 2t of a group of 8 and slot t + 4
-// element 2t + 1, which is how ldmatrix hands out halves in pairs.
 template <int HD>
 struct AttnSmem {
     static constexpr int kKeyStride = HD * 2 + 16;  // bytes; 16 past a multiple of 128: the 8 rows of an ldmatrix hit distinct banks
@@ -254,26 +251,82 @@ __device__ __forceinline__ void ldsm4_trans(uint32_t (&r)[4], const void *row) {
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
                  : "r"((uint32_t)__cvta_generic_to_shared(row)));
 }
-// D += A(16x8, tf32) * B(8x8, tf32), f32 accumulate
-__device__ __forceinline__ void mma_tf32(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-    asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+// D += A(16x8, f16) * B(8x8, f16), f32 accumulate.  (Eight products a step: the bits of the tf32 instruction on the same values.  The step of
+// sixteen rounds differently, and 32 layers carry a last bit on to 0.04 of the result.)
+__device__ __forceinline__ void mma_f16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t b) {
+    asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%0,%1,%2,%3};"
                  : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+                 : "r"(a0), "r"(a1), "r"(b));
 }
-// the two halves of a word as f32 bit patterns (exact, and representable in tf32)
-__device__ __forceinline__ void half2_bits(uint32_t w, uint32_t &lo, uint32_t &hi) {
-    const float2 f = __half22float2(*reinterpret_cast<const __half2 *>(&w));
-    lo = __float_as_uint(f.x);
-    hi = __float_as_uint(f.y);
+// f16 pieces of two f32 values: hi = the top 11 significant bits, mid = the top 11 of what is left, times 2^11
+__device__ __forceinline__ void f16_pieces(float x, float y, uint32_t &hi, uint32_t &mid) {
+    const __half hx = __float2half_rz(x), hy = __float2half_rz(y);
+    const __half2 h = __halves2half2(hx, hy), m = __halves2half2(__float2half_rz((x - __half2float(hx)) * 2048.0f), __float2half_rz((y - __half2float(hy)) * 2048.0f));
+    hi = *reinterpret_cast<const uint32_t *>(&h);
+    mid = *reinterpret_cast<const uint32_t *>(&m);
 }
-// tf32 pieces of an f32 value: piece 0 = its top 11 significant bits, piece 1 = the top 11 of what is left
-__device__ __forceinline__ uint32_t tf32_piece(float v, int piece) {
-    const uint32_t hi = __float_as_uint(v) & 0xFFFFE000u;
-    return piece == 0 ? hi : (__float_as_uint(v - __uint_as_float(hi)) & 0xFFFFE000u);
+constexpr float kMid = 1.0f / 2048.0f;
+// The pieces of one head's query by a warp: columns 2 * pair, 2 * pair + 1 of s_q (rows of QS halves); returns what a sum of products is
+// to be multiplied by.
+template <int HD, int QS>
+__device__ __forceinline__ float split_query(const float *qrow, __half *s_q, int pair, int lane, bool valid) {
+    constexpr int N = HD / 64;
+    float2 v[N];
+    float am = 0.f;
+#pragma unroll
+    for (int i = 0; i < N; i++) {
+        v[i] = valid ? *reinterpret_cast<const float2 *>(qrow + i * 64 + lane * 2) : make_float2(0.f, 0.f);
+        am = fmaxf(am, fmaxf(fabsf(v[i].x), fabsf(v[i].y)));
+    }
+    am = warp_max(am);
+    const int e = (int)(__float_as_uint(am) >> 23);
+    const float f = __uint_as_float((uint32_t)min(268 - max(e, 1), 254) << 23);  // am * f is in [2^14, 2^15)
+#pragma unroll
+    for (int i = 0; i < N; i++) {
+        uint32_t hi, mid;
+        f16_pieces(v[i].x * f, v[i].y * f, hi, mid);
+        *reinterpret_cast<uint32_t *>(s_q + (2 * pair) * QS + i * 64 + lane * 2) = hi;
+        *reinterpret_cast<uint32_t *>(s_q + (2 * pair + 1) * QS + i * 64 + lane * 2) = mid;
+    }
+    return 1.0f / f;
+}
+// Scores of one head (f32, 128 keys, `keys` of them valid) -> the pieces of exp(s - m) in columns 2 * pair, 2 * pair + 1 of s_p, m and l.
+template <int PS>
+__device__ __forceinline__ void softmax_tile(const float *s_sc, __half *s_p, int pair, int lane, int keys, float factor, float *ml) {
+    float v[4], m = -INFINITY;
+#pragma unroll
+    for (int e = 0; e < 4; e++) {
+        v[e] = lane + 32 * e < keys ? s_sc[lane + 32 * e] * factor : -INFINITY;
+        m = fmaxf(m, v[e]);
+    }
+    m = warp_max(m);
+    float l = 0.f;
+#pragma unroll
+    for (int e = 0; e < 4; e++) {
+        v[e] = keys > 0 ? expf(v[e] - m) : 0.f;
+        l += v[e];
+    }
+    l = warp_sum(l);
+#pragma unroll
+    for (int e = 0; e < 4; e++) {
+        const float w = v[e] * 32768.0f;
+        const __half hi = __float2half_rz(w);
+        s_p[(2 * pair) * PS + lane + 32 * e] = hi;
+        s_p[(2 * pair + 1) * PS + lane + 32 * e] = __float2half_rz((w - __half2float(hi)) * 2048.0f);
+    }
+    if (lane == 0) ml[0] = m, ml[1] = l;
+}
+constexpr float kWeight = 1.0f / 32768.0f;
+// The B words of one lane: column g8 of a group of eight, elements 2 t4, 2 t4 + 1 and 2 t4 + 8, 2 t4 + 9 from `k0` on
+template <int S>
+__device__ __forceinline__ void b_words(const __half *cols, int col, int k0, int t4, uint32_t &b0, uint32_t &b1) {
+    const __half *p = cols + col * S + k0 + 2 * t4;
+    b0 = *reinterpret_cast<const uint32_t *>(p);
+    b1 = *reinterpret_cast<const uint32_t *>(p + 8);
 }
 
 constexpr int kAttnChunkPairs = 16;   // (query row, head) pairs of a chunk's tile
-constexpr int kAttnChunkStride = 136;  // floats between pairs of 128 values: four pairs read 8 words each from distinct banks
+constexpr int kAttnPad = 8;  // halves behind a column of 64 or 128: the eight columns of a read start four banks apart
 
 template <int HD, int G, bool BULK>
 __global__ void __launch_bounds__(kAttnThreads) attn_split_kernel(const float *q, const __half *k_cache,
@@ -290,8 +343,11 @@ __global__ void __launch_bounds__(kAttnThreads) attn_split_kernel(const float *q
     extern __shared__ __align__(16) uint8_t dyn_smem[];
     uint8_t *s_k = dyn_smem, *s_v = dyn_smem + kAttnTile * L::kKeyStride;
     float(*s_o)[G][HD] = reinterpret_cast<float(*)[G][HD]>(dyn_smem);  // KP x G x HD floats over the key tile (KP > 1 only)
-    __shared__ __align__(16) float s_q[G * HD];
-    __shared__ __align__(16) float s_pp[2][G][kAttnTile];  // [0]: scores, then the hi pieces of exp(s - m); [1]: the mid pieces
+    constexpr int QS = HD + kAttnPad, PS = kAttnTile + kAttnPad;
+    __shared__ __align__(16) __half s_q[NT * 8 * QS];  // columns past 2 G are never stored
+    __shared__ __align__(16) __half s_p[NT * 8 * PS];
+    __shared__ __align__(16) float s_sc[G][kAttnTile];
+    __shared__ float s_f[G];
     __shared__ float s_ml[G][2];
     __shared__ __align__(8) uint64_t s_bar[2];
     static_assert(KP * G * HD * 4 <= kAttnTile * L::kKeyStride, "the partial outputs reuse the key tile");
@@ -366,8 +422,10 @@ __global__ void __launch_bounds__(kAttnThreads) attn_split_kernel(const float *q
             *reinterpret_cast<uint4 *>(s_v + key * L::kValStride + c * 16) = make_uint4(0, 0, 0, 0);
         }
     }
-    const float *qrow = q + ((size_t)qr * n_head + (size_t)kvh * G) * HD;
-    for (int i = tid; i < G * HD; i += kAttnThreads) s_q[i] = qrow[i];
+    for (int g = warp; g < NT * 4; g += kAttnThreads / 32) {
+        const float f = split_query<HD, QS>(q + ((size_t)qr * n_head + (size_t)kvh * G + g) * HD, s_q, g, lane, g < G);
+        if (lane == 0 && g < G) s_f[g] = f * scale;
+    }
     // the keys have landed; q is staged, the zeroed rows are in place.  (BULK: a bounded wait; if it runs out, the CTA
     // records it and leaves after the wait for the values has had its own limit, so that no copy can land in shared
     // memory that is no longer this CTA's.)
@@ -389,25 +447,16 @@ __global__ void __launch_bounds__(kAttnThreads) attn_split_kernel(const float *q
         for (int nt = 0; nt < NT; nt++) acc[nt][0] = acc[nt][1] = acc[nt][2] = acc[nt][3] = 0.f;
         // ldmatrix rows: matrices 0 / 1 = keys 0..7 / 8..15 at dims d0.., matrices 2 / 3 = the same keys at dims d0 + 8..
         const uint8_t *arow = s_k + (size_t)(16 * warp + (lane & 7) + ((lane >> 3) & 1) * 8) * L::kKeyStride + (lane >> 4) * 16;
-#pragma unroll 4
+#pragma unroll
         for (int j = 0; j < HD / 16; j++) {
             uint32_t r[4];
             ldsm4(r, arow + j * 32);
-            uint32_t a[2][4];  // [dim group of 8][a0..a3]
-            half2_bits(r[0], a[0][0], a[0][2]);  // keys g8:     (slot t4, slot t4 + 4) = dims 2 t4, 2 t4 + 1
-            half2_bits(r[1], a[0][1], a[0][3]);  // keys g8 + 8
-            half2_bits(r[2], a[1][0], a[1][2]);
-            half2_bits(r[3], a[1][1], a[1][3]);
 #pragma unroll
             for (int nt = 0; nt < NT; nt++) {
-                const int c = nt * 8 + g8, head = c >> 1, piece = c & 1;  // this lane's B column
-                float2 q0 = make_float2(0.f, 0.f), q1 = q0;
-                if (head < G) {
-                    q0 = *reinterpret_cast<const float2 *>(s_q + head * HD + j * 16 + 2 * t4);
-                    q1 = *reinterpret_cast<const float2 *>(s_q + head * HD + j * 16 + 8 + 2 * t4);
-                }
-                mma_tf32(acc[nt], a[0][0], a[0][1], a[0][2], a[0][3], tf32_piece(q0.x, piece), tf32_piece(q0.y, piece));
-                mma_tf32(acc[nt], a[1][0], a[1][1], a[1][2], a[1][3], tf32_piece(q1.x, piece), tf32_piece(q1.y, piece));
+                uint32_t b0, b1;
+                b_words<QS>(s_q, nt * 8 + g8, j * 16, t4, b0, b1);
+                mma_f16(acc[nt], r[0], r[1], b0);
+                mma_f16(acc[nt], r[2], r[3], b1);
             }
         }
         // columns 2 t4, 2 t4 + 1 of group nt = the two pieces of head 4 nt + t4; rows g8 and g8 + 8 of the warp's keys
@@ -415,8 +464,8 @@ __global__ void __launch_bounds__(kAttnThreads) attn_split_kernel(const float *q
         for (int nt = 0; nt < NT; nt++) {
             const int head = nt * 4 + t4;
             if (head < G) {
-                s_pp[0][head][16 * warp + g8] = acc[nt][0] + acc[nt][1];
-                s_pp[0][head][16 * warp + g8 + 8] = acc[nt][2] + acc[nt][3];
+                s_sc[head][16 * warp + g8] = fmaf(acc[nt][1], kMid, acc[nt][0]);
+                s_sc[head][16 * warp + g8 + 8] = fmaf(acc[nt][3], kMid, acc[nt][2]);
             }
         }
     }
@@ -432,26 +481,7 @@ __global__ void __launch_bounds__(kAttnThreads) attn_split_kernel(const float *q
         __syncthreads();
     }
     // ---- phase 2
-    for (int g = warp; g < G; g += kAttnThreads / 32) {
-        float v[4], m = -INFINITY;
-#pragma unroll
-        for (int e = 0; e < 4; e++) {
-            const int key = lane + 32 * e;
-            v[e] = key < tile_keys ? s_pp[0][g][key] * scale : -INFINITY;
-            m = fmaxf(m, v[e]);
-        }
-        m = warp_max(m);  // finite: the tile holds at least one valid key
-        float l = 0.f;
-#pragma unroll
-        for (int e = 0; e < 4; e++) {
-            const float p = expf(v[e] - m);
-            s_pp[0][g][lane + 32 * e] = __uint_as_float(tf32_piece(p, 0));
-            s_pp[1][g][lane + 32 * e] = __uint_as_float(tf32_piece(p, 1));
-            l += p;
-        }
-        l = warp_sum(l);
-        if (lane == 0) s_ml[g][0] = m, s_ml[g][1] = l;
-    }
+    for (int g = warp; g < G; g += kAttnThreads / 32) softmax_tile<PS>(s_sc[g], s_p, g, lane, tile_keys, s_f[g], s_ml[g]);
     __syncthreads();
     // ---- phase 3: output dims 16 dg .. + 15 over this warp's share of the keys
     {
@@ -462,33 +492,23 @@ __global__ void __launch_bounds__(kAttnThreads) attn_split_kernel(const float *q
         for (int nt = 0; nt < NT; nt++) acc[nt][0] = acc[nt][1] = acc[nt][2] = acc[nt][3] = 0.f;
         // ldmatrix.trans rows: matrices 0 / 1 = keys 0..7 at dims 0..7 / 8..15 of the group, matrices 2 / 3 = keys 8..15
         const uint8_t *vrow = s_v + (size_t)(kp * KEYS + (lane & 7) + (lane >> 4) * 8) * L::kValStride + (size_t)(16 * dg + ((lane >> 3) & 1) * 8) * 2;
-#pragma unroll 4
+#pragma unroll
         for (int s16 = 0; s16 < KEYS / 16; s16++) {
             uint32_t r[4];
             ldsm4_trans(r, vrow + (size_t)s16 * 16 * L::kValStride);
-            uint32_t a[2][4];  // [key group of 8][a0..a3]
-            half2_bits(r[0], a[0][0], a[0][2]);  // dims g8:     (slot t4, slot t4 + 4) = keys 2 t4, 2 t4 + 1
-            half2_bits(r[1], a[0][1], a[0][3]);  // dims g8 + 8
-            half2_bits(r[2], a[1][0], a[1][2]);
-            half2_bits(r[3], a[1][1], a[1][3]);
-            const int k0 = kp * KEYS + s16 * 16 + 2 * t4;
 #pragma unroll
             for (int nt = 0; nt < NT; nt++) {
-                const int c = nt * 8 + g8, head = c >> 1, piece = c & 1;
-                float2 p0 = make_float2(0.f, 0.f), p1 = p0;
-                if (head < G) {
-                    p0 = *reinterpret_cast<const float2 *>(&s_pp[piece][head][k0]);
-                    p1 = *reinterpret_cast<const float2 *>(&s_pp[piece][head][k0 + 8]);
-                }
-                mma_tf32(acc[nt], a[0][0], a[0][1], a[0][2], a[0][3], __float_as_uint(p0.x), __float_as_uint(p0.y));
-                mma_tf32(acc[nt], a[1][0], a[1][1], a[1][2], a[1][3], __float_as_uint(p1.x), __float_as_uint(p1.y));
+                uint32_t b0, b1;
+                b_words<PS>(s_p, nt * 8 + g8, kp * KEYS + s16 * 16, t4, b0, b1);
+                mma_f16(acc[nt], r[0], r[1], b0);
+                mma_f16(acc[nt], r[2], r[3], b1);
             }
         }
 #pragma unroll
         for (int nt = 0; nt < NT; nt++) {
             const int head = nt * 4 + t4;
             if (head < G) {
-                const float o0 = acc[nt][0] + acc[nt][1], o1 = acc[nt][2] + acc[nt][3];  // dims 16 dg + g8, + 8
+                const float o0 = fmaf(acc[nt][1], kMid, acc[nt][0]) * kWeight, o1 = fmaf(acc[nt][3], kMid, acc[nt][2]) * kWeight;  // dims 16 dg + g8, + 8
                 if (KP == 1) {
                     float *po = part_o + (out_idx + (size_t)head * n_splits) * HD + 16 * dg + g8;
                     po[0] = o0;
@@ -517,12 +537,12 @@ __global__ void __launch_bounds__(kAttnThreads) attn_split_kernel(const float *q
 }
 
 // The same tile for 16 / G consecutive query rows of one sequence (a prompt chunk), head_dim 128: 16 (row, head) pairs are 32
-// columns of the matrix instruction, so a key or value fragment is loaded and widened once for all of them; the arithmetic of a
-// column, and so every bit, is that of attn_split_kernel.  A tile that ends inside the rows' causal edge multiplies the values
-// row by row, last row first: each row sees one key fewer, and that key's values are zeroed, so that the matrix unit multiplies 0
-// (not a later token's infinity) by its weight 0.
-// Measured (113 rows at position 384, 32 heads / 8): 51 -> 45 us a layer; one CTA per row was bound by its 64 KB tile and its
-// three barriers per row.
+// columns of the matrix instruction, so a key or value fragment is loaded once for all of them; the arithmetic of a
+// column, and so every bit, is that of attn_split_kernel.  Where a tile ends inside the rows' causal edge and a value there is infinite or
+// NaN, the values are multiplied row by row, last row first: each row sees one key fewer, and that key's values are zeroed, so that the
+// matrix unit multiplies 0 (not a later token's infinity) by its weight 0.
+// Measured (us a call with the merge, 113 rows at position 384, 32 heads / 8): a CTA per row 60, tf32 pieces and the edge always row by row
+// 56, now 40; 128 rows at 2048, 32 / 4, 171 -> 116; 128 rows at 1024, 8 / 8, 50 -> 26.
 template <int G>
 __global__ void __launch_bounds__(kAttnThreads) attn_chunk_kernel(const float *q, const __half *k_cache,
                                                                   const __half *v_cache, float *__restrict__ part_o,
@@ -530,13 +550,16 @@ __global__ void __launch_bounds__(kAttnThreads) attn_chunk_kernel(const float *q
                                                                   int n_splits, size_t seq_stride, uint32_t *__restrict__ status,
                                                                   const int32_t *seq_pos, const int32_t *block_table,
                                                                   int table_stride, int n_pages) {
-    constexpr int HD = 128, P = kAttnChunkPairs, SP = kAttnChunkStride, R = P / G, CPR = HD * 2 / 16, NT = 2 * P / 8, NT1 = (2 * G + 7) / 8;
+    constexpr int HD = 128, P = kAttnChunkPairs, S = HD + kAttnPad, R = P / G, CPR = HD * 2 / 16, NT = 2 * P / 8, NT1 = (2 * G + 7) / 8;
+    static_assert(kAttnTile == HD, "one stride for queries and weights");
     using L = AttnSmem<HD>;
     static_assert(kAttnThreads / 32 == HD / 16, "a warp owns 16 output dims");
     extern __shared__ __align__(16) uint8_t dyn_smem[];
     uint8_t *s_k = dyn_smem, *s_v = dyn_smem + kAttnTile * L::kKeyStride;
-    float *s_q = reinterpret_cast<float *>(dyn_smem + L::kBytes);                                  // [P][SP]
-    float(*s_pp)[P][SP] = reinterpret_cast<float(*)[P][SP]>(s_q + P * SP);                         // [2][P][SP]
+    __half *s_q = reinterpret_cast<__half *>(dyn_smem + L::kBytes);        // [2 P][S]: the queries' pieces
+    __half *s_p = s_q + 2 * P * S;                                         // [2 P][S]: the weights' pieces
+    float(*s_sc)[kAttnTile] = reinterpret_cast<float(*)[kAttnTile]>(s_p + 2 * P * S);  // [P][128]
+    __shared__ float s_f[P];
     __shared__ float s_ml[P][2];
     __shared__ __align__(8) uint64_t s_bar[2];
     const int row_blocks = (rows + R - 1) / R;
@@ -583,9 +606,10 @@ __global__ void __launch_bounds__(kAttnThreads) attn_chunk_kernel(const float *q
             for (int c = 0; c < CPR; c++) *reinterpret_cast<uint4 *>(dst + c * 16) = make_uint4(0, 0, 0, 0);
         }
     }
-    for (int i = tid; i < P * HD; i += kAttnThreads) {
-        const int pair = i / HD, r = pair / G;
-        s_q[pair * SP + i % HD] = r < nr ? q[(((size_t)seq * rows + ti0 + r) * n_head + (size_t)kvh * G + pair % G) * HD + i % HD] : 0.f;
+    for (int pair = warp; pair < P; pair += kAttnThreads / 32) {
+        const int r = pair / G;
+        const float f = split_query<HD, S>(q + (((size_t)seq * rows + ti0 + r) * n_head + (size_t)kvh * G + pair % G) * HD, s_q, pair, lane, r < nr);
+        if (lane == 0) s_f[pair] = f * scale;
     }
     // (bounded waits; a CTA that gives up leaves after both copies have had their limit)
     const bool k_ok = attn_wait(&s_bar[0]);
@@ -600,28 +624,22 @@ __global__ void __launch_bounds__(kAttnThreads) attn_chunk_kernel(const float *q
 #pragma unroll
         for (int nt = 0; nt < NT; nt++) acc[nt][0] = acc[nt][1] = acc[nt][2] = acc[nt][3] = 0.f;
         const uint8_t *arow = s_k + (size_t)(16 * warp + (lane & 7) + ((lane >> 3) & 1) * 8) * L::kKeyStride + (lane >> 4) * 16;
-#pragma unroll 2
+#pragma unroll
         for (int j = 0; j < HD / 16; j++) {
             uint32_t r[4];
             ldsm4(r, arow + j * 32);
-            uint32_t a[2][4];
-            half2_bits(r[0], a[0][0], a[0][2]);
-            half2_bits(r[1], a[0][1], a[0][3]);
-            half2_bits(r[2], a[1][0], a[1][2]);
-            half2_bits(r[3], a[1][1], a[1][3]);
 #pragma unroll
             for (int nt = 0; nt < NT; nt++) {
-                const int c = nt * 8 + g8, pair = c >> 1, piece = c & 1;
-                const float2 q0 = *reinterpret_cast<const float2 *>(s_q + pair * SP + j * 16 + 2 * t4);
-                const float2 q1 = *reinterpret_cast<const float2 *>(s_q + pair * SP + j * 16 + 8 + 2 * t4);
-                mma_tf32(acc[nt], a[0][0], a[0][1], a[0][2], a[0][3], tf32_piece(q0.x, piece), tf32_piece(q0.y, piece));
-                mma_tf32(acc[nt], a[1][0], a[1][1], a[1][2], a[1][3], tf32_piece(q1.x, piece), tf32_piece(q1.y, piece));
+                uint32_t b0, b1;
+                b_words<S>(s_q, nt * 8 + g8, j * 16, t4, b0, b1);
+                mma_f16(acc[nt], r[0], r[1], b0);
+                mma_f16(acc[nt], r[2], r[3], b1);
             }
         }
 #pragma unroll
         for (int nt = 0; nt < NT; nt++) {
-            s_pp[0][nt * 4 + t4][16 * warp + g8] = acc[nt][0] + acc[nt][1];
-            s_pp[0][nt * 4 + t4][16 * warp + g8 + 8] = acc[nt][2] + acc[nt][3];
+            s_sc[nt * 4 + t4][16 * warp + g8] = fmaf(acc[nt][1], kMid, acc[nt][0]);
+            s_sc[nt * 4 + t4][16 * warp + g8 + 8] = fmaf(acc[nt][3], kMid, acc[nt][2]);
         }
     }
     const bool v_ok = attn_wait(&s_bar[1]);
@@ -630,28 +648,17 @@ __global__ void __launch_bounds__(kAttnThreads) attn_chunk_kernel(const float *q
         return;
     }
     // ---- phase 2
-    for (int p = warp; p < P; p += kAttnThreads / 32) {
-        const int keys = p / G < nr ? min(kAttnTile, base + p / G) : 0;
-        float v[4], m = -INFINITY;
-#pragma unroll
-        for (int e = 0; e < 4; e++) {
-            const int key = lane + 32 * e;
-            v[e] = key < keys ? s_pp[0][p][key] * scale : -INFINITY;
-            m = fmaxf(m, v[e]);
+    for (int p = warp; p < P; p += kAttnThreads / 32)
+        softmax_tile<S>(s_sc[p], s_p, p, lane, p / G < nr ? min(kAttnTile, base + p / G) : 0, s_f[p], s_ml[p]);
+    // The rows see different numbers of keys where the tile ends inside their causal edge: a key that one of them does not see has weight 0
+    // there, which must not meet an infinity of a later token.
+    bool apart = false;
+    if (base < kAttnTile)
+        for (int i = tid; i < (min(base + nr - 1, kAttnTile) - max(base, 0)) * HD / 2; i += kAttnThreads) {
+            const uint32_t w = *reinterpret_cast<const uint32_t *>(s_v + (max(base, 0) + i / (HD / 2)) * L::kValStride + i % (HD / 2) * 4);
+            apart = apart || (w & 0x7C00u) == 0x7C00u || (w & 0x7C000000u) == 0x7C000000u;
         }
-        m = warp_max(m);
-        float l = 0.f;
-#pragma unroll
-        for (int e = 0; e < 4; e++) {
-            const float w = keys > 0 ? expf(v[e] - m) : 0.f;
-            s_pp[0][p][lane + 32 * e] = __uint_as_float(tf32_piece(w, 0));
-            s_pp[1][p][lane + 32 * e] = __uint_as_float(tf32_piece(w, 1));
-            l += w;
-        }
-        l = warp_sum(l);
-        if (lane == 0) s_ml[p][0] = m, s_ml[p][1] = l;
-    }
-    __syncthreads();
+    apart = __syncthreads_or(apart);
     // ---- phase 3: output dims 16 warp .. + 15
     const uint8_t *vrow = s_v + (size_t)((lane & 7) + (lane >> 4) * 8) * L::kValStride + (size_t)(16 * warp + ((lane >> 3) & 1) * 8) * 2;
     // NTC groups of four pairs from pair p0 on; pairs at or past p1 are computed for nothing and not stored
@@ -660,23 +667,16 @@ __global__ void __launch_bounds__(kAttnThreads) attn_chunk_kernel(const float *q
         float acc[NTC][4];
 #pragma unroll
         for (int nt = 0; nt < NTC; nt++) acc[nt][0] = acc[nt][1] = acc[nt][2] = acc[nt][3] = 0.f;
-#pragma unroll 2
+#pragma unroll
         for (int s16 = 0; s16 < kAttnTile / 16; s16++) {
             uint32_t r[4];
             ldsm4_trans(r, vrow + (size_t)s16 * 16 * L::kValStride);
-            uint32_t a[2][4];
-            half2_bits(r[0], a[0][0], a[0][2]);
-            half2_bits(r[1], a[0][1], a[0][3]);
-            half2_bits(r[2], a[1][0], a[1][2]);
-            half2_bits(r[3], a[1][1], a[1][3]);
-            const int k0 = s16 * 16 + 2 * t4;
 #pragma unroll
             for (int nt = 0; nt < NTC; nt++) {
-                const int c = nt * 8 + g8, pair = min(p0 + (c >> 1), P - 1), piece = c & 1;
-                const float2 w0 = *reinterpret_cast<const float2 *>(&s_pp[piece][pair][k0]);
-                const float2 w1 = *reinterpret_cast<const float2 *>(&s_pp[piece][pair][k0 + 8]);
-                mma_tf32(acc[nt], a[0][0], a[0][1], a[0][2], a[0][3], __float_as_uint(w0.x), __float_as_uint(w0.y));
-                mma_tf32(acc[nt], a[1][0], a[1][1], a[1][2], a[1][3], __float_as_uint(w1.x), __float_as_uint(w1.y));
+                uint32_t b0, b1;
+                b_words<S>(s_p, min(2 * p0 + nt * 8 + g8, 2 * P - 1), s16 * 16, t4, b0, b1);
+                mma_f16(acc[nt], r[0], r[1], b0);
+                mma_f16(acc[nt], r[2], r[3], b1);
             }
         }
 #pragma unroll
@@ -684,13 +684,13 @@ __global__ void __launch_bounds__(kAttnThreads) attn_chunk_kernel(const float *q
             const int pair = p0 + nt * 4 + t4;
             if (pair < p1) {
                 float *po = part_o + out_of(pair) * HD + 16 * warp + g8;
-                po[0] = acc[nt][0] + acc[nt][1];
-                po[8] = acc[nt][2] + acc[nt][3];
+                po[0] = fmaf(acc[nt][1], kMid, acc[nt][0]) * kWeight;
+                po[8] = fmaf(acc[nt][3], kMid, acc[nt][2]) * kWeight;
             }
         }
     };
-    if (base >= kAttnTile) {
-        values(std::integral_constant<int, NT>{}, 0, nr * G);  // every row sees the whole tile
+    if (!apart) {
+        values(std::integral_constant<int, NT>{}, 0, nr * G);
     } else {
 #pragma unroll 1
         for (int r = nr - 1; r >= 0 && base + r > 0; r--) {
@@ -808,7 +808,6 @@ __global__ void __launch_bounds__(256) argmax_stage2_kernel(const float *cand_v,
 // per-32 and per-16 code sums (crates/infr-cpu/src/quant.rs:27-58).  Same operations in the same order as
 // quantize_q8_kernel<256>, so a producer that ends with this emits the bits the separate quantiser would.
 __device__ __forceinline__ float q8_amax4(float4 v) { return fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))); }
-__device__ __forceinline__ int q8_code(float v, float id) { return q8_round_code(v, id); }
 __device__ __forceinline__ void quantize_block256(const float4 v[2], int lane, size_t row, int k, int chunk, int8_t *__restrict__ qs,
                                                   float *__restrict__ d, int32_t *__restrict__ sums, int32_t *__restrict__ sums16) {
     float m = fmaxf(q8_amax4(v[0]), q8_amax4(v[1]));
@@ -819,13 +818,12 @@ __device__ __forceinline__ void quantize_block256(const float4 v[2], int lane, s
 #pragma unroll
     for (int h = 0; h < 2; h++) {
         const int e = chunk * 256 + h * 128 + lane * 4;
-        const int q0 = q8_code(v[h].x, id), q1 = q8_code(v[h].y, id), q2 = q8_code(v[h].z, id), q3 = q8_code(v[h].w, id);
-        int sm = q0 + q1 + q2 + q3;
+        const uint32_t packed = q8_codes4(v[h], id);
+        int sm = q8_sum4(packed);
         sm += __shfl_xor_sync(0xffffffffu, sm, 1);
         sm += __shfl_xor_sync(0xffffffffu, sm, 2);
         const int s16 = sm;
         sm += __shfl_xor_sync(0xffffffffu, sm, 4);
-        const uint32_t packed = (uint32_t)(q0 & 0xff) | ((uint32_t)(q1 & 0xff) << 8) | ((uint32_t)(q2 & 0xff) << 16) | ((uint32_t)(q3 & 0xff) << 24);
         *reinterpret_cast<uint32_t *>(qs + row * k + e) = packed;
         if (sums16 && (lane & 3) == 0) sums16[row * (k / 16) + e / 16] = s16;
         if ((lane & 7) == 0) sums[row * (k / 32) + e / 32] = sm;
@@ -848,7 +846,6 @@ __global__ void __launch_bounds__(1024) rms_norm_q8_kernel(const float *a, const
                                                            float eps, float *__restrict__ dst, int8_t *__restrict__ qs, float *__restrict__ d,
                                                            int32_t *__restrict__ sums, int32_t *__restrict__ sums16) {
     __shared__ float s_part[32];
-    __shared__ float s_scale;
     pdl_go();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5, chunks = dim / 256;
     const bool in_regs = chunks <= nw;
@@ -879,13 +876,7 @@ __global__ void __launch_bounds__(1024) rms_norm_q8_kernel(const float *a, const
     ss = warp_sum(ss);
     if (lane == 0) s_part[warp] = ss;
     __syncthreads();
-    if (warp == 0) {
-        float t = lane < nw ? s_part[lane] : 0.f;
-        t = warp_sum(t);
-        if (lane == 0) s_scale = 1.0f / sqrtf(t / (float)dim + eps);
-    }
-    __syncthreads();
-    const float s = s_scale;
+    const float s = 1.0f / sqrtf(warp_sum(lane < nw ? s_part[lane] : 0.f) / (float)dim + eps);  // (every warp for itself: no second barrier)
     const float *src = (ADD ? sum_dst : a) + base;  // re-read by the warp that wrote it
     for (int chunk = warp; chunk < chunks; chunk += nw) {
         float4 v[2];
@@ -920,7 +911,6 @@ __global__ void __launch_bounds__(1024) rms_norm_q8_pull_kernel(const float *a, 
                                                                 int8_t *__restrict__ qs, float *__restrict__ d, int32_t *__restrict__ sums,
                                                                 int32_t *__restrict__ sums16, PullArgs pull) {
     __shared__ float s_part[32];
-    __shared__ float s_scale;
     pdl_go();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5, chunks = dim / 256;
     const bool in_regs = chunks <= nw;
@@ -969,13 +959,7 @@ __global__ void __launch_bounds__(1024) rms_norm_q8_pull_kernel(const float *a, 
     ss = warp_sum(ss);
     if (lane == 0) s_part[warp] = ss;
     __syncthreads();
-    if (warp == 0) {
-        float t = lane < nw ? s_part[lane] : 0.f;
-        t = warp_sum(t);
-        if (lane == 0) s_scale = 1.0f / sqrtf(t / (float)dim + eps);
-    }
-    __syncthreads();
-    const float s = s_scale;
+    const float s = 1.0f / sqrtf(warp_sum(lane < nw ? s_part[lane] : 0.f) / (float)dim + eps);
     for (int chunk = warp; chunk < chunks; chunk += nw) {
         float4 v[2];
 #pragma unroll
@@ -1028,7 +1012,9 @@ __global__ void __launch_bounds__(256) gated_silu_q8_kernel(const float *gate, c
 // sums meet in shared memory and warp 0 normalises and quantises.
 // With Q8 false the same sums are stored as f32 instead, so the two forms agree bit for bit.
 constexpr int kCombineMaxSplits = 512;
-template <bool Q8>
+// AHEAD (few rows): a warp's first tiles are on their way while the weights are formed, one round trip to L2 where the loads came one after
+// the other (one row, 33 tiles: 5.2 -> 4.1 us; 32 rows, whose registers it costs: 8.2 -> 10).
+template <bool Q8, bool AHEAD>
 __global__ void __launch_bounds__(256) attn_combine_wide_kernel(const float *part_o, const float *part_ml, int n_head,
                                                                 int head_dim, int n_splits, float *__restrict__ dst, int8_t *__restrict__ qs,
                                                                 float *__restrict__ d, int32_t *__restrict__ sums, int32_t *__restrict__ sums16) {
@@ -1041,19 +1027,32 @@ __global__ void __launch_bounds__(256) attn_combine_wide_kernel(const float *par
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, k = n_head * head_dim, cpr = k / 256;
     const int row = blockIdx.x / cpr, chunk = blockIdx.x % cpr;
     const int heads = 256 / head_dim, head0 = chunk * heads;
+    constexpr int kAhead = AHEAD ? 4 : 0;
+    float4 p[2][kAhead + 1];
+    const float *po[2];
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        const int e = h * 128 + lane * 4;
+        po[h] = part_o + ((size_t)row * n_head + head0 + e / head_dim) * n_splits * head_dim + e % head_dim;
+#pragma unroll
+        for (int j = 0; j < kAhead; j++)
+            if (warp + 8 * j < n_splits) p[h][j] = *reinterpret_cast<const float4 *>(po[h] + (size_t)(warp + 8 * j) * head_dim);
+    }
     if (warp < heads) {
-        const float *ml = part_ml + ((size_t)row * n_head + head0 + warp) * n_splits * 2;
-        float m = -INFINITY;
-        for (int s = lane; s < n_splits; s += 32) m = fmaxf(m, ml[2 * s]);
+        const float2 *ml = reinterpret_cast<const float2 *>(part_ml) + ((size_t)row * n_head + head0 + warp) * n_splits;
+        const float2 none = make_float2(-INFINITY, 0.f);
+        const float2 ml0 = lane < n_splits ? ml[lane] : none, ml1 = lane + 32 < n_splits ? ml[lane + 32] : none;
+        float m = fmaxf(ml0.x, ml1.x);
+        for (int s = lane + 64; s < n_splits; s += 32) m = fmaxf(m, ml[s].x);
         m = warp_max(m);
         float l = 0.f;
         int n = 0;
         for (int s = lane; s < n_splits; s += 32) {
-            const float ls = ml[2 * s + 1];
-            if (ls == 0.f) break;  // past the row's causal end, as all tiles after it (a tile with keys has l >= 1, or NaN)
-            const float wgt = expf(ml[2 * s] - m);
+            const float2 v = s < 32 ? ml0 : s < 64 ? ml1 : ml[s];
+            if (v.y == 0.f) break;  // past the row's causal end, as all tiles after it (a tile with keys has l >= 1, or NaN)
+            const float wgt = expf(v.x - m);
             s_w[warp][s] = wgt;
-            l += wgt * ls;
+            l += wgt * v.y;
             n = s + 1;
         }
         l = warp_sum(l);
@@ -1063,17 +1062,18 @@ __global__ void __launch_bounds__(256) attn_combine_wide_kernel(const float *par
     __syncthreads();
 #pragma unroll
     for (int h = 0; h < 2; h++) {
-        const int e = h * 128 + lane * 4, hh = e / head_dim, dim0 = e % head_dim;
-        const float *po = part_o + ((size_t)row * n_head + head0 + hh) * n_splits * head_dim + dim0;
+        const int e = h * 128 + lane * 4, hh = e / head_dim;
         float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+        auto add = [&](float wgt, float4 v) {
+            acc.x = fmaf(wgt, v.x, acc.x), acc.y = fmaf(wgt, v.y, acc.y), acc.z = fmaf(wgt, v.z, acc.z), acc.w = fmaf(wgt, v.w, acc.w);
+        };
         // (nobody writes the sums of the tiles past the causal end: what an earlier op left there may read as NaN)
         const int n = s_n[hh];
+#pragma unroll
+        for (int j = 0; j < kAhead; j++)
+            if (warp + 8 * j < n) add(s_w[hh][warp + 8 * j], p[h][j]);
 #pragma unroll 4
-        for (int s = warp; s < n; s += 8) {
-            const float wgt = s_w[hh][s];
-            const float4 p = *reinterpret_cast<const float4 *>(po + (size_t)s * head_dim);
-            acc.x = fmaf(wgt, p.x, acc.x), acc.y = fmaf(wgt, p.y, acc.y), acc.z = fmaf(wgt, p.z, acc.z), acc.w = fmaf(wgt, p.w, acc.w);
-        }
+        for (int s = warp + 8 * kAhead; s < n; s += 8) add(s_w[hh][s], *reinterpret_cast<const float4 *>(po[h] + (size_t)s * head_dim));
         *reinterpret_cast<float4 *>(&s_acc[warp][e]) = acc;
     }
     __syncthreads();
@@ -1188,7 +1188,7 @@ template <int G>
 static cudaError_t launch_attn_chunk(cudaStream_t st, const float *q, const __half *kc, const __half *vc, float *po, float *pml, int n_seq, int rows,
                                      int n_head, int n_kv, int pos, float scale, int n_splits, size_t seq_stride, uint32_t *status,
                                      const int32_t *seq_pos, const int32_t *block_table, int table_stride, int n_pages) {
-    constexpr int R = kAttnChunkPairs / G, bytes = AttnSmem<128>::kBytes + 3 * kAttnChunkPairs * kAttnChunkStride * 4;
+    constexpr int R = kAttnChunkPairs / G, bytes = AttnSmem<128>::kBytes + 4 * kAttnChunkPairs * (128 + kAttnPad) * 2 + kAttnChunkPairs * kAttnTile * 4;
     cudaError_t e = cudaFuncSetAttribute(attn_chunk_kernel<G>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     if (e != cudaSuccess) return e;
     return launch_pdl(attn_chunk_kernel<G>, dim3(n_splits, n_kv, n_seq * ((rows + R - 1) / R)), dim3(kAttnThreads), (size_t)bytes, st, q, kc, vc, po, pml,
@@ -1234,13 +1234,15 @@ cudaError_t launch_attention(const float *q, const void *k_cache, const void *v_
         return cudaErrorInvalidValue;
 #undef INFR_CHUNK
     if (e != cudaSuccess) return e;
+    const unsigned merge_ctas = (unsigned)(q_rows * (n_head * head_dim / 256));
+    const bool few = merge_ctas <= 2 * sms;
     if (qs) {  // the merged rows go straight to int8 (n_head * head_dim must be whole 256-element blocks)
         if ((n_head * head_dim) % 256 || n_splits > kCombineMaxSplits) return cudaErrorInvalidValue;
-        return launch_pdl(attn_combine_wide_kernel<true>, dim3((unsigned)(q_rows * (n_head * head_dim / 256))), dim3(256), 0, st, (const float *)po,
+        return launch_pdl(few ? attn_combine_wide_kernel<true, true> : attn_combine_wide_kernel<true, false>, dim3(merge_ctas), dim3(256), 0, st, (const float *)po,
                           (const float *)pml, n_head, head_dim, n_splits, (float *)nullptr, qs, d, sums, sums16);
     }
     if ((n_head * head_dim) % 256 == 0 && n_splits <= kCombineMaxSplits)
-        return launch_pdl(attn_combine_wide_kernel<false>, dim3((unsigned)(q_rows * (n_head * head_dim / 256))), dim3(256), 0, st, (const float *)po,
+        return launch_pdl(few ? attn_combine_wide_kernel<false, true> : attn_combine_wide_kernel<false, false>, dim3(merge_ctas), dim3(256), 0, st, (const float *)po,
                           (const float *)pml, n_head, head_dim, n_splits, dst, (int8_t *)nullptr, (float *)nullptr, (int32_t *)nullptr,
                           (int32_t *)nullptr);
     return launch_pdl(attn_combine_kernel, dim3(q_rows * n_head), dim3(head_dim), 0, st, (const float *)po, (const float *)pml, dst, head_dim, n_splits);

@@ -99,12 +99,9 @@ __global__ void __launch_bounds__(256) gemm_q2_prep_kernel(const float *x, int m
     if (e0 >= in_f) return;
     const float d = am / 127.0f;
     const float id = d > 0.0f ? 1.0f / d : 0.0f;
-    int q[8];
-#pragma unroll
-    for (int i = 0; i < 8; i++) q[i] = q8_round_code(v[i], id);
     const int tile = T / (8 * nt), tt = T % (8 * nt), n = tt >> 3, g = tt & 7, b = e0 >> 6, h = (lane >> 2) & 1, t = lane & 3;
     uint8_t *rec = act + ((size_t)tile * nb + b) * record_bytes(nt);
-    *reinterpret_cast<uint2 *>(rec + n * 512 + (g * 4 + t) * 16 + h * 8) = make_uint2(q8_pack4(q[0], q[2], q[4], q[6]), q8_pack4(q[1], q[3], q[5], q[7]));
+    *reinterpret_cast<uint2 *>(rec + n * 512 + (g * 4 + t) * 16 + h * 8) = make_uint2(q8_codes4(make_float4(v[0], v[2], v[4], v[6]), id), q8_codes4(make_float4(v[1], v[3], v[5], v[7]), id));
     if (t == 0) *reinterpret_cast<float *>(rec + nt * 512 + n * 64 + (g >> 1) * 16 + h * 8 + (g & 1) * 4) = d;
 }
 

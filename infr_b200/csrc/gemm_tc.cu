@@ -340,11 +340,8 @@ __global__ void __launch_bounds__(256) gemm_tc_prep_kernel(const float *x, Q8Dev
         for (int o = 1; o < 32; o <<= 1) am = fmaxf(am, __shfl_xor_sync(0xffffffffu, am, o));
         d = am / 127.0f;
         const float id = d > 0.0f ? 1.0f / d : 0.0f;
-        int q[8];
-#pragma unroll
-        for (int i = 0; i < 8; i++) q[i] = q8_round_code(v[i], id);
-        w0 = q8_pack4(q[0], q[1], q[2], q[3]);
-        w1 = q8_pack4(q[4], q[5], q[6], q[7]);
+        w0 = q8_codes4(make_float4(v[0], v[1], v[2], v[3]), id);
+        w1 = q8_codes4(make_float4(v[4], v[5], v[6], v[7]), id);
     } else if (row >= 0) {
         const uint2 c = *reinterpret_cast<const uint2 *>(a.qs + (size_t)row * in_f + (size_t)b * 256 + lane * 8);
         w0 = c.x, w1 = c.y;

@@ -144,17 +144,8 @@ __device__ __forceinline__ void quant_items(const float4 (&pa)[4], const float4 
     int sum[NK];
 #pragma unroll
     for (int k = 0; k < NK; k++) {
-        const float vv[8] = {pa[K0 + k].x, pa[K0 + k].y, pa[K0 + k].z, pa[K0 + k].w, pb[K0 + k].x, pb[K0 + k].y, pb[K0 + k].z, pb[K0 + k].w};
-        int q[8];
-        if (id[k] <= 3.0e38f) {  // (warp-uniform) the usual case: a finite scale, no clamp needed
-#pragma unroll
-            for (int e = 0; e < 8; e++) q[e] = q8_round_code_inrange(vv[e], id[k]);
-        } else {
-#pragma unroll
-            for (int e = 0; e < 8; e++) q[e] = q8_round_code(vv[e], id[k]);
-        }
-        pk[k].x = q8_pack4(q[0], q[1], q[2], q[3]);
-        pk[k].y = q8_pack4(q[4], q[5], q[6], q[7]);
+        pk[k].x = q8_codes4(pa[K0 + k], id[k]);
+        pk[k].y = q8_codes4(pb[K0 + k], id[k]);
         sum[k] = q8_sum4(pk[k].x) + q8_sum4(pk[k].y);
     }
 #pragma unroll

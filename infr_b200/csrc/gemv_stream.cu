@@ -344,7 +344,7 @@ __global__ void __launch_bounds__(kStreamThreads, (M <= 2 ? 2 : 1))
                 int sum = 0;
 #pragma unroll
                 for (int k = 0; k < 4; k++) {
-                    w[k] = q8_pack4(q8_round_code(f[p][k].x, id), q8_round_code(f[p][k].y, id), q8_round_code(f[p][k].z, id), q8_round_code(f[p][k].w, id));
+                    w[k] = q8_codes4(f[p][k], id);
                     sum += q8_sum4(w[k]);
                 }
                 sum += __shfl_xor_sync(0xffffffffu, sum, 1);

@@ -316,15 +316,8 @@ __global__ void __launch_bounds__(256) moe_swiglu_quant_kernel(const float *gate
     for (int o = 16; o > 0; o >>= 1) am = fmaxf(am, __shfl_xor_sync(0xffffffffu, am, o));
     const float dd = am / 127.0f;
     const float id = dd > 0.0f ? 1.0f / dd : 0.0f;
-    int q[8], sum = 0;
-#pragma unroll
-    for (int i = 0; i < 8; i++) {
-        q[i] = q8_round_code(v[i], id);
-        sum += q[i];
-    }
-    uint2 pk;
-    pk.x = (uint32_t)(q[0] & 0xff) | ((uint32_t)(q[1] & 0xff) << 8) | ((uint32_t)(q[2] & 0xff) << 16) | ((uint32_t)(q[3] & 0xff) << 24);
-    pk.y = (uint32_t)(q[4] & 0xff) | ((uint32_t)(q[5] & 0xff) << 8) | ((uint32_t)(q[6] & 0xff) << 16) | ((uint32_t)(q[7] & 0xff) << 24);
+    const uint2 pk = make_uint2(q8_codes4(make_float4(v[0], v[1], v[2], v[3]), id), q8_codes4(make_float4(v[4], v[5], v[6], v[7]), id));
+    int sum = q8_sum4(pk.x) + q8_sum4(pk.y);
     *reinterpret_cast<uint2 *>(qs + base) = pk;
     sum += __shfl_xor_sync(0xffffffffu, sum, 1);
     if (sums16 && (lane & 1) == 0) sums16[((size_t)p * nbk + b) * 16 + (lane >> 1)] = sum;  // Q6_K banks: sums per 16 codes

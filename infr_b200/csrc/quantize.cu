@@ -23,8 +23,6 @@ __device__ __forceinline__ float amax4(float4 v) {
     return fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w)));
 }
 
-__device__ __forceinline__ int q1(float v, float id) { return q8_round_code(v, id); }
-
 template <int GRAN>
 __global__ void __launch_bounds__(256) quantize_q8_kernel(const float *x, int rows, int k,
                                                           int8_t *__restrict__ qs, float *__restrict__ d,
@@ -67,15 +65,13 @@ __global__ void __launch_bounds__(256) quantize_q8_kernel(const float *x, int ro
 #pragma unroll
     for (int h = 0; h < 2; h++) {
         const float id = dd[h] > 0.0f ? 1.0f / dd[h] : 0.0f;
-        const int q0 = q1(v[h].x, id), q1_ = q1(v[h].y, id), q2 = q1(v[h].z, id), q3 = q1(v[h].w, id);
-        int s = q0 + q1_ + q2 + q3;
+        const uint32_t packed = q8_codes4(v[h], id);
+        int s = q8_sum4(packed);
         s += __shfl_xor_sync(0xffffffffu, s, 1);
         s += __shfl_xor_sync(0xffffffffu, s, 2);
         const int s16 = s;
         s += __shfl_xor_sync(0xffffffffu, s, 4);
         if (!ok[h]) continue;
-        const uint32_t packed = (uint32_t)(q0 & 0xff) | ((uint32_t)(q1_ & 0xff) << 8) |
-                                ((uint32_t)(q2 & 0xff) << 16) | ((uint32_t)(q3 & 0xff) << 24);
         *reinterpret_cast<uint32_t *>(qs + (size_t)row * k + e[h]) = packed;
         if (sums16 && (lane & 3) == 0) sums16[(size_t)row * (k / 16) + e[h] / 16] = s16;
         if ((lane & 7) == 0) {
