@@ -2,6 +2,7 @@
 #include "backend.h"
 
 #include <algorithm>
+#include <cmath>
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
@@ -805,6 +806,19 @@ Status CudaBackend::moe_ffn_f32(const MoeArgs &a) {
     return Status::Ok();
 }
 
+// 8-row items to expect of an expert that each of `rows` rows picks with probability p: the sum over k of P(more than 8 k rows).
+static double expected_items(double p, int rows) {
+    double pmf = std::pow(1.0 - p, rows);
+    if (p >= 1.0 || pmf < 1e-30) return (p * rows + 3.5) / 8;  // an item of every expert is half full on average
+    double below = 0, sum = 0;
+    for (int c = 0; c <= rows; c++) {  // P(c rows) from P(c - 1 rows)
+        below += pmf;
+        if (c % 8 == 0) sum += below < 1.0 ? 1.0 - below : 0.0;
+        pmf *= p / (1.0 - p) * (rows - c) / (c + 1);
+    }
+    return sum;
+}
+
 Status CudaBackend::moe_ffn(const MoeArgs &a) {
     auto bank_ok = [](int dt) { return dt == DT_Q4K || dt == DT_Q6K; };
     if (!bank_ok(a.gate_dt) || !bank_ok(a.up_dt) || !bank_ok(a.down_dt))
@@ -891,10 +905,13 @@ Status CudaBackend::moe_ffn(const MoeArgs &a) {
     INFR_STEP(launch_quantize_q8(a.x, (int)rows, (int)ne, 256, xq, xd, xs, xs16, nullptr, nullptr, stream_), "moe quantize x");
     Q8Dev xa{xq, xd, xs, xs16, 256};
     // one expert bank against the routed rows, 8-row items on the warp matrix unit (Q6_K rows too long for its tiles: byte-dot kernel)
-    auto bank_gemm = [&](int dt, const uint8_t *bank, const Q8Dev &acts, float *out, uint32_t k, uint32_t o, const int32_t *rows_of) {
+    const int items = (int)((double)a.n_local * expected_items((double)nu / (double)nx, (int)rows) + 0.5);
+    auto bank_gemm = [&](int dt, const uint8_t *bank, const Q8Dev &acts, float *out, uint32_t k, uint32_t o, const int32_t *rows_of, const uint8_t *bank2 = nullptr,
+                         float *out2 = nullptr) {
         if (dt == DT_Q4K)
-            return launch_grouped_q4k_mma(bank, (int)a.n_local, acts, out, (int)k, (int)o, ie, ip, ic, ni, rows_of, (int)max_items, dev_, status_dev_, stream_);
-        const cudaError_t e = launch_grouped_q6_mma(bank, acts, out, (int)k, (int)o, ie, ip, ic, ni, rows_of, (int)max_items, dev_, status_dev_, stream_);
+            return launch_grouped_q4k_mma(bank, bank2, (int)a.n_local, acts, out, out2, (int)k, (int)o, ie, ip, ic, ni, rows_of, (int)max_items, items, dev_, status_dev_,
+                                          stream_);
+        const cudaError_t e = launch_grouped_q6_mma(bank, acts, out, (int)k, (int)o, ie, ip, ic, ni, rows_of, (int)max_items, items, dev_, status_dev_, stream_);
         if (e != cudaErrorInvalidValue) return e;
         cudaGetLastError();
         return launch_grouped_q6k(bank, acts, out, (int)k, (int)o, ie, ip, ic, ni, rows_of, (int)max_items, dev_, stream_);
@@ -919,8 +936,12 @@ Status CudaBackend::moe_ffn(const MoeArgs &a) {
         return Status::Ok();
     }
     // stage B: gate and up expert GEMMs, rows gathered per pair
-    INFR_STEP(bank_gemm(a.gate_dt, a.gate, xa, g, (uint32_t)ne, (uint32_t)nff, prow), "moe gate");
-    INFR_STEP(bank_gemm(a.up_dt, a.up, xa, u, (uint32_t)ne, (uint32_t)nff, prow), "moe up");
+    if (a.gate_dt == DT_Q4K && a.up_dt == DT_Q4K) {
+        INFR_STEP(bank_gemm(DT_Q4K, a.gate, xa, g, (uint32_t)ne, (uint32_t)nff, prow, a.up, u), "moe gate, up");
+    } else {
+        INFR_STEP(bank_gemm(a.gate_dt, a.gate, xa, g, (uint32_t)ne, (uint32_t)nff, prow), "moe gate");
+        INFR_STEP(bank_gemm(a.up_dt, a.up, xa, u, (uint32_t)ne, (uint32_t)nff, prow), "moe up");
+    }
     // stage C: SwiGLU and re-quantisation per pair
     INFR_STEP(launch_moe_swiglu_quant(g, u, (int)n_pairs, (int)nff, aq, ad, as, as16, nullptr, stream_), "moe swiglu");
     Q8Dev aa{aq, ad, as, as16, 256};

@@ -1,6 +1,7 @@
 // Device helpers shared by the GEMV kernels: vector loads, the unsigned x signed byte dot product,
 // Q4_K scale unpacking, and the shared-memory staging of quantised activations.
 #pragma once
+#include <cmath>
 #include <cuda_fp16.h>
 
 #include "kernels.h"
@@ -133,6 +134,20 @@ __device__ __forceinline__ void stage_q8(const Q8Dev &a, int m, int M, int in_f,
     }
 }
 
+
+// CTAs an item of a grouped launch: `items` expected, `slots` CTAs fit the device, `tiles` of the item go to `lanes` groups of warps of a CTA.
+// A CTA costs its tiles and what it takes before the first of them (staging the item's rows: about five tiles' time), and waves of CTAs come one
+// after the other.  How many items there are is only known on the device, so a wave is taken to be full a fiftieth before it is.
+inline int grouped_ctas(int items, int slots, int tiles, int lanes) {
+    int best = 1;
+    double best_cost = 0;
+    const int most = (tiles + lanes - 1) / lanes;
+    for (int g = 1; g <= most && g <= 64; g++) {
+        const double waves = std::ceil((double)items * g / slots + 0.02), cost = waves * ((tiles + g * lanes - 1) / (g * lanes) + 5);
+        if (g == 1 || cost < best_cost) best = g, best_cost = cost;
+    }
+    return best;
+}
 
 }  // namespace
 }  // namespace infr

@@ -172,28 +172,29 @@ __device__ __forceinline__ void quant_items(const float4 (&pa)[4], const float4 
 //   bsplit : 16 B at (n*nb + b)*16: bytes 0..7 = low 6 bits of bsum_s, bytes 8..15 = bsum_s >> 6
 //   d8     : float [b][8 tokens], zero for absent tokens (a lane's two result columns are neighbours)
 // KW = warps per CTA (they split K), SB = super-blocks per ring slot per row.
-template <int M, bool FUSED, int KW, int SB, bool PUSH>
-__global__ void __launch_bounds__(KW * 32, 16 / KW)
+// TG: groups of KW warps that take the CTA's tiles in turn.
+template <int M, bool FUSED, int KW, int SB, bool PUSH, int TG = 1>
+__global__ void __launch_bounds__(KW * TG * 32, 16 / (KW * TG))
     gemv_q4k_mma_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ MmaSecond sec, Q8Dev a,
                         const float *x, float *__restrict__ y, int m, int in_f, int out_f, MmaGeom geo, MmaGroup grp,
                         uint32_t *__restrict__ status, const __grid_constant__ typename PushParam<PUSH>::type push) {
-    constexpr int kW = KW, kThreadsMma = KW * 32, kStepBlocks = SB, kSlotBytes = kTileRows * SB * 144;
+    constexpr int kW = KW, kThreadsMma = KW * TG * 32, kStepBlocks = SB, kSlotBytes = kTileRows * SB * 144;
     extern __shared__ __align__(128) uint8_t smem[];
     const int nb = geo.nb, S = geo.slots;
-    uint8_t *rings = smem;                                         // [kW][S][kSlotBytes]
-    uint8_t *s_codes = smem + (size_t)kW * S * kSlotBytes;         // [M][nb][256]
+    uint8_t *rings = smem;                                         // [kW * TG][S][kSlotBytes]
+    uint8_t *s_codes = smem + (size_t)kW * TG * S * kSlotBytes;    // [M][nb][256]
     uint8_t *s_bsplit = s_codes + (size_t)M * nb * kStagedBytes;   // [M][nb][16]
     float *s_d8 = reinterpret_cast<float *>(s_bsplit + (size_t)M * nb * 16);  // [nb][8]
-    float *s_part = s_d8 + (size_t)nb * 8;                         // [2][kW][16][8]
-    uint64_t *bars = reinterpret_cast<uint64_t *>(s_part + 2 * kW * 128);  // [kW][kMaxSlotsMma]
+    float *s_part = s_d8 + (size_t)nb * 8;                         // [TG][2][kW][16][8]
+    uint64_t *bars = reinterpret_cast<uint64_t *>(s_part + 2 * kW * TG * 128);  // [kW * TG][kMaxSlotsMma]
     __shared__ int s_bad;
     __shared__ uint32_t s_epoch;  // push mode: exchanges completed before this launch
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, kwarp = TG == 1 ? warp : warp % kW, tg = TG == 1 ? 0 : warp / kW;
     const int g = lane >> 2, t = lane & 3;
     if (threadIdx.x == 0) {
         s_bad = 0;
-        for (int i = 0; i < kW * kMaxSlotsMma; i++) bar_init(s_u32(bars + i), 1);
+        for (int i = 0; i < kW * TG * kMaxSlotsMma; i++) bar_init(s_u32(bars + i), 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
@@ -213,9 +214,9 @@ __global__ void __launch_bounds__(KW * 32, 16 / KW)
     const int total_tiles = tiles1 + (sec.out_f + kTileRows - 1) / kTileRows;
     const int G = gridDim.x, base = total_tiles / G, rem = total_tiles % G;
     const int t_begin = blockIdx.x * base + (blockIdx.x < rem ? blockIdx.x : rem);
-    const int n_tiles = base + (blockIdx.x < rem ? 1 : 0);
+    const int n_tiles = (base + (blockIdx.x < rem ? 1 : 0) - tg + TG - 1) / TG;  // of this warp's group: tg, tg + TG, ...
     // this warp's K range
-    const int kb0 = warp * geo.bpw;
+    const int kb0 = kwarp * geo.bpw;
     const int kb1 = min(nb, kb0 + geo.bpw);
     const int my_blocks = max(0, kb1 - kb0);
     const int steps_per_tile = (my_blocks + kStepBlocks - 1) / kStepBlocks;
@@ -237,11 +238,11 @@ __global__ void __launch_bounds__(KW * 32, 16 / KW)
             // order this warp's earlier reads of the slot before the engine overwrites it
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             bar_expect_tx(bar, (uint32_t)kSlotBytes);
-            const int T = t_begin + i_tile;
+            const int T = t_begin + tg + i_tile * TG;
             if (T < tiles1)
                 tma_load_2d_hint(s_u32(ring + (size_t)slot * kSlotBytes), &tmap, blk0 * 36, row_base + T * kTileRows, bar, l2_policy);
             else
-                tma_load_2d_hint(s_u32(ring + (size_t)slot * kSlotBytes), &sec.map, blk0 * 36, (T - tiles1) * kTileRows, bar, l2_policy);
+                tma_load_2d_hint(s_u32(ring + (size_t)slot * kSlotBytes), &sec.map, blk0 * 36, row_base + (T - tiles1) * kTileRows, bar, l2_policy);
         }
         __syncwarp();
         j_issue++;
@@ -419,19 +420,23 @@ __global__ void __launch_bounds__(KW * 32, 16 / KW)
             }
         }
         // partial sums of this warp's K range: [row 0..15][token 0..7]
-        float *part = s_part + ((size_t)(tile & 1) * kW + warp) * 128;
+        float *part = s_part + ((size_t)(tg * 2 + (tile & 1)) * kW + kwarp) * 128;
         part[g * 8 + 2 * t] = accf[0];
         part[g * 8 + 2 * t + 1] = accf[1];
         part[(g + 8) * 8 + 2 * t] = accf[2];
         part[(g + 8) * 8 + 2 * t + 1] = accf[3];
-        __syncthreads();
-        if (threadIdx.x < kTileRows * 8) {  // 16 rows x 8 token columns; CTAs have at least 128 threads
-            const int r = threadIdx.x >> 3, n = threadIdx.x & 7;
-            const int T = t_begin + tile;
+        if (TG == 1)
+            __syncthreads();
+        else
+            asm volatile("bar.sync %0, %1;" ::"r"(1 + tg), "n"(KW * 32) : "memory");
+        const int tid = threadIdx.x - tg * kW * 32;
+        if (tid < kTileRows * 8) {  // 16 rows x 8 token columns; groups have at least 128 threads
+            const int r = tid >> 3, n = tid & 7;
+            const int T = t_begin + tg + tile * TG;
             const bool second = T >= tiles1;
             const int row = (second ? T - tiles1 : T) * kTileRows + r, of = second ? sec.out_f : out_f;
             if (n < m && row < of) {
-                const float *pp = s_part + (size_t)(tile & 1) * kW * 128 + r * 8 + n;
+                const float *pp = s_part + (size_t)(tg * 2 + (tile & 1)) * kW * 128 + r * 8 + n;
                 float v = 0.f;
 #pragma unroll
                 for (int w = 0; w < kW; w++) v += pp[w * 128];
@@ -459,22 +464,22 @@ EncodeTiledFn encode_tiled() {
     return fn;
 }
 
-template <int M, bool FUSED, int KW, int SB>
+template <int M, bool FUSED, int KW, int SB, int TG = 1>
 cudaError_t launch_mma_cfg(const uint8_t *w, const Q8Dev &a, const float *x, float *y, int m, int in_f, int out_f,
                            const DeviceInfo &dev, uint32_t *status, cudaStream_t st, const MmaGroup &grp = MmaGroup{},
                            int n_experts = 1, int max_items = 1, const uint8_t *w2 = nullptr, float *y2 = nullptr, int out_f2 = 0,
-                           const GemvPush *push = nullptr) {
+                           const GemvPush *push = nullptr, int items = 1) {
     constexpr int kSlotBytes = kTileRows * SB * 144;
     MmaGeom geo;
     geo.nb = in_f / 256;
     geo.bpw = (geo.nb + KW - 1) / KW;
     const size_t acts = (size_t)M * geo.nb * (kStagedBytes + 16) + (size_t)geo.nb * 32;
     geo.act_bytes = (int)acts;
-    const size_t fixed = acts + (size_t)2 * KW * 128 * 4 + (size_t)KW * kMaxSlotsMma * 8 + 64;
-    const size_t per_slot = (size_t)KW * kSlotBytes;
+    const size_t fixed = acts + (size_t)2 * KW * TG * 128 * 4 + (size_t)KW * TG * kMaxSlotsMma * 8 + 64;
+    const size_t per_slot = (size_t)KW * TG * kSlotBytes;
     if (fixed + 2 * per_slot > (size_t)dev.max_smem_optin - 1024) return cudaErrorInvalidValue;
     // resident CTAs per SM: 16 math warps in total, each warp with at least two ring slots
-    int per_sm = 16 / KW;
+    int per_sm = 16 / (KW * TG);
     while (per_sm > 1 && fixed + 2 * per_slot > (size_t)dev.max_smem_optin / per_sm - 2048) per_sm /= 2;
     const size_t budget = (size_t)dev.max_smem_optin / per_sm - (per_sm > 1 ? 2048 : 1024);
     int slots = (int)((budget - fixed) / per_slot);
@@ -506,25 +511,23 @@ cudaError_t launch_mma_cfg(const uint8_t *w, const Q8Dev &a, const float *x, flo
     };
     if (!encode(&tmap, w, (cuuint64_t)out_f * (cuuint64_t)n_experts)) return cudaErrorInvalidValue;
     if (out_f2 > 0) {
-        if (!encode(&sec.map, w2, (cuuint64_t)out_f2)) return cudaErrorInvalidValue;
+        if (!encode(&sec.map, w2, (cuuint64_t)out_f2 * (cuuint64_t)n_experts)) return cudaErrorInvalidValue;
         sec.y = y2;
         sec.out_f = out_f2;
     }
     // the pushing form exists for pre-quantised rows only
-    auto kernel = gemv_q4k_mma_kernel<M, FUSED, KW, SB, false>;
+    auto kernel = gemv_q4k_mma_kernel<M, FUSED, KW, SB, false, TG>;
     auto kernel_push = gemv_q4k_mma_kernel<M, false, KW, SB, true>;
-    if (push && FUSED) return cudaErrorInvalidValue;
+    if (push && (FUSED || TG > 1)) return cudaErrorInvalidValue;
     cudaError_t e = push ? cudaFuncSetAttribute(kernel_push, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)
                          : cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};
     if (grp.item_expert) {
-        // many small (expert, 8-row) items: a few CTAs per item, the SMs fill up across items
-        const int tiles = (out_f + kTileRows - 1) / kTileRows;
-        grid = tiles < 4 ? tiles : 4;
+        grid = grouped_ctas(items < 1 ? 1 : items, dev.sm_count * per_sm, all_tiles, TG);
     }
     cfg.gridDim = dim3((unsigned)grid, (unsigned)max_items);
-    cfg.blockDim = dim3(KW * 32);
+    cfg.blockDim = dim3(KW * TG * 32);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
@@ -592,17 +595,24 @@ cudaError_t launch_mma(const uint8_t *w, const Q8Dev &a, const float *x, float *
 
 }  // namespace
 
-cudaError_t launch_grouped_q4k_mma(const uint8_t *bank, int n_experts, const Q8Dev &a, float *y, int in_f, int out_f,
+cudaError_t launch_grouped_q4k_mma(const uint8_t *bank, const uint8_t *bank2, int n_experts, const Q8Dev &a, float *y, float *y2, int in_f, int out_f,
                                    const int *item_expert, const int *item_p0, const int *item_cnt, const int *n_items,
-                                   const int *pair_row, int max_items, const DeviceInfo &dev, uint32_t *status,
+                                   const int *pair_row, int max_items, int items, const DeviceInfo &dev, uint32_t *status,
                                    cudaStream_t st) {
     if (in_f % 256 || max_items < 1) return cudaErrorInvalidValue;
     MmaGroup grp{item_expert, item_p0, item_cnt, n_items, pair_row};
-    const int nb = in_f / 256;
-    // four warps per 16-row tile: an item has few tiles and few K blocks, so the per-tile barrier and
-    // reduction are shared by two blocks per warp where the rows are long enough
-    if ((nb + 3) / 4 == 1) return launch_mma_cfg<8, false, 4, 1>(bank, a, nullptr, y, 8, in_f, out_f, dev, status, st, grp, n_experts, max_items);
-    return launch_mma_cfg<8, false, 4, 2>(bank, a, nullptr, y, 8, in_f, out_f, dev, status, st, grp, n_experts, max_items);
+    const int nb = in_f / 256, out2 = bank2 ? out_f : 0;
+    // Four warps per 16-row tile: an item has few tiles and few K blocks, so the per-tile barrier and reduction are shared by two blocks per
+    // warp where the rows are long enough; two such groups a CTA, because eight staged rows leave room for two CTAs on an SM.
+    // (Gate and up of 216 pairs over 128 experts, 2048 -> 768: 50 us; two launches of four CTAs of four warps an item, 1.4 waves of them, 76.
+    // Layers of 2..150 rows over 8..128 experts: 1.0 to 3.9 times as fast, most where few items left three quarters of the device idle.)
+    if ((nb + 3) / 4 == 1)
+        return launch_mma_cfg<8, false, 4, 1, 2>(bank, a, nullptr, y, 8, in_f, out_f, dev, status, st, grp, n_experts, max_items, bank2, y2, out2, nullptr, items);
+    const cudaError_t e =
+        launch_mma_cfg<8, false, 4, 2, 2>(bank, a, nullptr, y, 8, in_f, out_f, dev, status, st, grp, n_experts, max_items, bank2, y2, out2, nullptr, items);
+    if (e != cudaErrorInvalidValue) return e;
+    cudaGetLastError();  // rows so long that two groups' rings do not fit beside them
+    return launch_mma_cfg<8, false, 4, 2>(bank, a, nullptr, y, 8, in_f, out_f, dev, status, st, grp, n_experts, max_items, bank2, y2, out2, nullptr, items);
 }
 
 // Two Q4_K matrices with the same in_f against the same rows, one launch: pre-quantised rows (a), or f32 rows (x, a null)

@@ -558,7 +558,7 @@ cudaError_t launch_gemv_q6_mma(const uint8_t *w, const Q8Dev &a, float *y, int m
 // The grouped form.  cudaErrorInvalidValue when the shape does not qualify (heights that are not whole tiles, rows so long that two
 // tiles a warp do not fit, an unaligned bank): the caller takes the direct-load byte-dot kernel.
 cudaError_t launch_grouped_q6_mma(const uint8_t *bank, const Q8Dev &a, float *y, int in_f, int out_f, const int *item_expert, const int *item_p0,
-                                  const int *item_cnt, const int *n_items, const int *pair_row, int max_items, const DeviceInfo &dev, uint32_t *status,
+                                  const int *item_cnt, const int *n_items, const int *pair_row, int max_items, int items, const DeviceInfo &dev, uint32_t *status,
                                   cudaStream_t st) {
     if (in_f < 256 || in_f % 256 || out_f < 16 || out_f % 16 || max_items < 1 || max_items > 65535 || !a.sums16 || a.gran != 256 || (uintptr_t)bank % 16)
         return cudaErrorInvalidValue;
@@ -570,8 +570,9 @@ cudaError_t launch_grouped_q6_mma(const uint8_t *bank, const Q8Dev &a, float *y,
     if (need(kw) > (size_t)dev.max_smem_optin - 1024) return cudaErrorInvalidValue;
     cudaError_t e = cudaFuncSetAttribute(gemv_q6_mma_grouped_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)need(kw));
     if (e != cudaSuccess) return e;
-    int gx = out_f / 16 / (8 * kw);  // about eight tiles a warp
-    gx = gx < 1 ? 1 : (gx > 16 ? 16 : gx);
+    // (Whole layers with this bank as down, before: a CTA for eight tiles of each warp, 1 to 16 an item.  8 experts of 4096 -> 2048, 18 pairs:
+    // 113 us, 183 before; 128 experts of 2048 -> 768, 216 pairs: 122, 151; 512 pairs: 130, 162.)
+    const int gx = grouped_ctas(items < 1 ? 1 : items, dev.sm_count * (need(kw) > (size_t)dev.max_smem_optin / 2 - 2048 ? 1 : 2), out_f / 16, kw);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)gx, (unsigned)max_items);
     cfg.blockDim = dim3((unsigned)kw * 32);

@@ -158,14 +158,15 @@ cudaError_t launch_gemm_tc_grouped(int slab, const uint8_t *bank, int n_experts,
 // Grouped Q4_K GEMM over a bank of n_experts matrices [out_f, in_f] stored back to back: work item i
 // multiplies up to 8 quantised activation rows (pairs item_p0[i]..+item_cnt[i], gathered through
 // pair_row when non-null) with expert item_expert[i]; y is [n_pairs, out_f].
-cudaError_t launch_grouped_q4k_mma(const uint8_t *bank, int n_experts, const Q8Dev &a, float *y, int in_f, int out_f,
+// bank2 / y2: a second bank of that shape against the same rows in the same launch (gate and up), or null.  items: how many are expected.
+cudaError_t launch_grouped_q4k_mma(const uint8_t *bank, const uint8_t *bank2, int n_experts, const Q8Dev &a, float *y, float *y2, int in_f, int out_f,
                                    const int *item_expert, const int *item_p0, const int *item_cnt, const int *n_items,
-                                   const int *pair_row, int max_items, const DeviceInfo &dev, uint32_t *status,
+                                   const int *pair_row, int max_items, int items, const DeviceInfo &dev, uint32_t *status,
                                    cudaStream_t st);
 // The same grouped product for a Q6_K bank of whole 16-row tiles (rows of any length) on the matrix unit; `a` needs the sums per 16.
 // cudaErrorInvalidValue = shape not taken (launch_grouped_q6k takes it).
 cudaError_t launch_grouped_q6_mma(const uint8_t *bank, const Q8Dev &a, float *y, int in_f, int out_f, const int *item_expert, const int *item_p0,
-                                  const int *item_cnt, const int *n_items, const int *pair_row, int max_items, const DeviceInfo &dev, uint32_t *status,
+                                  const int *item_cnt, const int *n_items, const int *pair_row, int max_items, int items, const DeviceInfo &dev, uint32_t *status,
                                   cudaStream_t st);
 // The same grouped product for a Q6_K bank (direct-load byte-dot kernel, any row length); `a` needs the sums per 16.
 cudaError_t launch_grouped_q6k(const uint8_t *bank, const Q8Dev &a, float *y, int in_f, int out_f, const int *item_expert, const int *item_p0,
