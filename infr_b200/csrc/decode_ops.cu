@@ -16,6 +16,7 @@
 
 #include "pdl.cuh"
 #include "q8_code.cuh"
+#include "row_norm.cuh"
 
 namespace infr {
 namespace {
@@ -732,7 +733,7 @@ __global__ void __launch_bounds__(256) gated_silu_kernel(const float *gate, cons
     pdl_wait();
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
         const float g = gate[i];
-        dst[i] = g / (1.0f + expf(-g)) * up[i];
+        dst[i] = silu_mul(g, up[i]);
     }
 }
 
@@ -831,71 +832,21 @@ __device__ __forceinline__ void quantize_block256(const float4 v[2], int lane, s
     if (lane == 0) d[row * (k / 256) + chunk] = dd;
 }
 
-// Sum of squares of four values with every product and sum rounded on its own (no fused multiply-add): two kernels
-// that share this get the same bits whatever the compiler does around it, and it is how the CPU forms the sum.
-__device__ __forceinline__ float sumsq4(const float4 v) {
-    return __fadd_rn(__fadd_rn(__fadd_rn(__fmul_rn(v.x, v.x), __fmul_rn(v.y, v.y)), __fmul_rn(v.z, v.z)), __fmul_rn(v.w, v.w));
-}
-
-// RMSNorm (optionally of a + b, written to sum_dst) whose output goes straight to int8; dim % 256 == 0.
-// Warp c owns the 256-element blocks c, c + warps, ...; with one block per warp (dim <= 256 * warps, the launcher's
-// choice up to dim 8192) the row stays in registers between the sum of squares and the scaling.
-// With Q8 false the scaled row is stored as f32 to dst instead: the same arithmetic, so both forms agree bit for bit.
+// RMSNorm (rms_norm_row) whose output goes straight to int8.  With Q8 false the scaled row is stored as f32 to dst instead.
 template <bool ADD, bool Q8>
 __global__ void __launch_bounds__(1024) rms_norm_q8_kernel(const float *a, const float *b, float *sum_dst, const float *__restrict__ w, int dim,
                                                            float eps, float *__restrict__ dst, int8_t *__restrict__ qs, float *__restrict__ d,
                                                            int32_t *__restrict__ sums, int32_t *__restrict__ sums16) {
     __shared__ float s_part[32];
-    pdl_go();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5, chunks = dim / 256;
-    const bool in_regs = chunks <= nw;
-    // the norm weights do not depend on the previous kernel: fetch them before waiting for it
-    float4 g[2];
-    if (in_regs && warp < chunks) {
-#pragma unroll
-        for (int h = 0; h < 2; h++) g[h] = *reinterpret_cast<const float4 *>(w + warp * 256 + h * 128 + lane * 4);
-    }
-    pdl_wait();
-    const size_t base = (size_t)blockIdx.x * dim;
-    float4 x[2];
-    float ss = 0.f;
-    for (int chunk = warp; chunk < chunks; chunk += nw) {
-#pragma unroll
-        for (int h = 0; h < 2; h++) {
-            const int e = chunk * 256 + h * 128 + lane * 4;
-            float4 v = *reinterpret_cast<const float4 *>(a + base + e);
-            if (ADD) {
-                const float4 u = *reinterpret_cast<const float4 *>(b + base + e);
-                v.x += u.x, v.y += u.y, v.z += u.z, v.w += u.w;
-                *reinterpret_cast<float4 *>(sum_dst + base + e) = v;
-            }
-            ss = __fadd_rn(ss, sumsq4(v));
-            x[h] = v;
-        }
-    }
-    ss = warp_sum(ss);
-    if (lane == 0) s_part[warp] = ss;
-    __syncthreads();
-    const float s = 1.0f / sqrtf(warp_sum(lane < nw ? s_part[lane] : 0.f) / (float)dim + eps);  // (every warp for itself: no second barrier)
-    const float *src = (ADD ? sum_dst : a) + base;  // re-read by the warp that wrote it
-    for (int chunk = warp; chunk < chunks; chunk += nw) {
-        float4 v[2];
-#pragma unroll
-        for (int h = 0; h < 2; h++) {
-            const int e = chunk * 256 + h * 128 + lane * 4;
-            if (!in_regs) {
-                x[h] = *reinterpret_cast<const float4 *>(src + e);
-                g[h] = *reinterpret_cast<const float4 *>(w + e);
-            }
-            v[h] = make_float4(x[h].x * s * g[h].x, x[h].y * s * g[h].y, x[h].z * s * g[h].z, x[h].w * s * g[h].w);
-        }
+    const int lane = threadIdx.x & 31;
+    rms_norm_row<ADD>(a, b, sum_dst, w, dim, eps, blockIdx.x, s_part, [&](int chunk, const float4 (&v)[2]) {
         if (Q8) {
             quantize_block256(v, lane, blockIdx.x, dim, chunk, qs, d, sums, sums16);
         } else {
 #pragma unroll
-            for (int h = 0; h < 2; h++) *reinterpret_cast<float4 *>(dst + base + chunk * 256 + h * 128 + lane * 4) = v[h];
+            for (int h = 0; h < 2; h++) *reinterpret_cast<float4 *>(dst + (size_t)blockIdx.x * dim + chunk * 256 + h * 128 + lane * 4) = v[h];
         }
-    }
+    });
 }
 
 // The consumer of a pushed row-parallel GEMV (GemvPush): row = a + sum over ranks of the partial results that the
@@ -1000,8 +951,7 @@ __global__ void __launch_bounds__(256) gated_silu_q8_kernel(const float *gate, c
     for (int h = 0; h < 2; h++) {
         const size_t e = (size_t)row * nff + chunk * 256 + h * 128 + lane * 4;
         const float4 g = *reinterpret_cast<const float4 *>(gate + e), u = *reinterpret_cast<const float4 *>(up + e);
-        v[h] = make_float4(g.x / (1.0f + expf(-g.x)) * u.x, g.y / (1.0f + expf(-g.y)) * u.y, g.z / (1.0f + expf(-g.z)) * u.z,
-                           g.w / (1.0f + expf(-g.w)) * u.w);
+        v[h] = make_float4(silu_mul(g.x, u.x), silu_mul(g.y, u.y), silu_mul(g.z, u.z), silu_mul(g.w, u.w));
     }
     quantize_block256(v, lane, (size_t)row, nff, chunk, qs, d, sums, sums16);
 }
@@ -1097,6 +1047,82 @@ __global__ void __launch_bounds__(256) attn_combine_wide_kernel(const float *par
 #pragma unroll
             for (int h = 0; h < 2; h++) *reinterpret_cast<float4 *>(dst + (size_t)row * k + chunk * 256 + h * 128 + lane * 4) = v[h];
         }
+    }
+}
+
+// The same merge for at most NT key tiles: a warp for 256 outputs.  All its loads are on their way at once, nothing is shared and no warp waits for
+// another, where the kernel above makes two round trips and two barriers for a tile or two a warp.  The sums keep its order: tiles w, w + 8 into
+// partial sum w, the eight of them in turn.  (113 rows of 32 heads, 4 tiles: 1808 CTAs of 8 warps 9.1 us, 452 of 4 warps 3.2; a token of 32 heads at 1000: the step 2250 us, 2190.)
+constexpr int kMergeWarps = 4;
+template <bool Q8, int HEADS, int NT>
+__global__ void __launch_bounds__(kMergeWarps * 32) attn_combine_few_kernel(const float *part_o, const float *part_ml, int n_head, int n_splits, int n_blocks,
+                                                                            float *__restrict__ dst, int8_t *__restrict__ qs, float *__restrict__ d,
+                                                                            int32_t *__restrict__ sums, int32_t *__restrict__ sums16) {
+    constexpr int HD = 256 / HEADS;
+    pdl_go();
+    pdl_wait();
+    const int lane = threadIdx.x & 31, wg = blockIdx.x * kMergeWarps + (threadIdx.x >> 5), k = n_head * HD, cpr = k / 256;
+    if (wg >= n_blocks) return;
+    const int row = wg / cpr, chunk = wg % cpr, head0 = chunk * HEADS;
+    const size_t first = (size_t)row * n_head + head0;
+    float2 ml[HEADS];
+#pragma unroll
+    for (int h = 0; h < HEADS; h++)
+        ml[h] = lane < n_splits ? reinterpret_cast<const float2 *>(part_ml)[(first + h) * n_splits + lane] : make_float2(-INFINITY, 0.f);
+    float4 p[2][NT];
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        const int e = h * 128 + lane * 4;
+        const float *po = part_o + (first + e / HD) * n_splits * HD + e % HD;
+#pragma unroll
+        for (int s = 0; s < NT; s++)
+            if (s < n_splits) p[h][s] = *reinterpret_cast<const float4 *>(po + (size_t)s * HD);
+    }
+    float wgt[HEADS], l[HEADS];
+    int n[HEADS];
+#pragma unroll
+    for (int h = 0; h < HEADS; h++) {
+        const float m = warp_max(ml[h].x);
+        const bool has = ml[h].y != 0.f;  // not past the row's causal end (a tile with keys has l >= 1, or NaN)
+        wgt[h] = has ? expf(ml[h].x - m) : 0.f;
+        l[h] = warp_sum(has ? fmaf(wgt[h], ml[h].y, 0.f) : 0.f);
+        n[h] = __reduce_max_sync(0xffffffffu, has ? lane + 1 : 0);
+    }
+    float4 v[2];
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        const int hh = (h * 128 + lane * 4) / HD;
+        float lh = l[0];
+        int nh = n[0];
+#pragma unroll
+        for (int j = 1; j < HEADS; j++)
+            if (hh == j) lh = l[j], nh = n[j];
+        float4 acc[8];
+#pragma unroll
+        for (int s = 0; s < NT; s++) {
+            float w = 0.f;
+#pragma unroll
+            for (int j = 0; j < HEADS; j++) {
+                const float wj = __shfl_sync(0xffffffffu, wgt[j], s);
+                if (hh == j) w = wj;
+            }
+            float4 &t = acc[s & 7];
+            if (s < 8) t = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (s < nh) {  // (nobody writes the sums of the tiles past the causal end)
+                const float4 u = p[h][s];
+                t.x = fmaf(w, u.x, t.x), t.y = fmaf(w, u.y, t.y), t.z = fmaf(w, u.z, t.z), t.w = fmaf(w, u.w, t.w);
+            }
+        }
+        float4 t = acc[0];
+#pragma unroll
+        for (int w = 1; w < 8; w++) t.x += acc[w].x, t.y += acc[w].y, t.z += acc[w].z, t.w += acc[w].w;
+        v[h] = make_float4(t.x / lh, t.y / lh, t.z / lh, t.w / lh);
+    }
+    if (Q8) {
+        quantize_block256(v, lane, (size_t)row, k, chunk, qs, d, sums, sums16);
+    } else {
+#pragma unroll
+        for (int h = 0; h < 2; h++) *reinterpret_cast<float4 *>(dst + (size_t)row * k + chunk * 256 + h * 128 + lane * 4) = v[h];
     }
 }
 
@@ -1236,15 +1262,23 @@ cudaError_t launch_attention(const float *q, const void *k_cache, const void *v_
     if (e != cudaSuccess) return e;
     const unsigned merge_ctas = (unsigned)(q_rows * (n_head * head_dim / 256));
     const bool few = merge_ctas <= 2 * sms;
-    if (qs) {  // the merged rows go straight to int8 (n_head * head_dim must be whole 256-element blocks)
-        if ((n_head * head_dim) % 256 || n_splits > kCombineMaxSplits) return cudaErrorInvalidValue;
-        return launch_pdl(few ? attn_combine_wide_kernel<true, true> : attn_combine_wide_kernel<true, false>, dim3(merge_ctas), dim3(256), 0, st, (const float *)po,
-                          (const float *)pml, n_head, head_dim, n_splits, (float *)nullptr, qs, d, sums, sums16);
+    if (qs && ((n_head * head_dim) % 256 || n_splits > kCombineMaxSplits)) return cudaErrorInvalidValue;  // merged rows straight to int8: whole 256-element blocks
+    if (qs || ((n_head * head_dim) % 256 == 0 && n_splits <= kCombineMaxSplits)) {
+        if (n_splits <= 16) {
+            auto go = [&](auto kernel) {
+                return launch_pdl(kernel, dim3((merge_ctas + kMergeWarps - 1) / kMergeWarps), dim3(kMergeWarps * 32), 0, st, (const float *)po, (const float *)pml, n_head,
+                                  n_splits, (int)merge_ctas, qs ? nullptr : dst, qs, d, sums, sums16);
+            };
+            if (head_dim == 128)
+                return n_splits <= 8 ? go(qs ? attn_combine_few_kernel<true, 2, 8> : attn_combine_few_kernel<false, 2, 8>)
+                                     : go(qs ? attn_combine_few_kernel<true, 2, 16> : attn_combine_few_kernel<false, 2, 16>);
+            return n_splits <= 8 ? go(qs ? attn_combine_few_kernel<true, 4, 8> : attn_combine_few_kernel<false, 4, 8>)
+                                 : go(qs ? attn_combine_few_kernel<true, 4, 16> : attn_combine_few_kernel<false, 4, 16>);
+        }
+        auto kernel = qs ? (few ? attn_combine_wide_kernel<true, true> : attn_combine_wide_kernel<true, false>)
+                         : (few ? attn_combine_wide_kernel<false, true> : attn_combine_wide_kernel<false, false>);
+        return launch_pdl(kernel, dim3(merge_ctas), dim3(256), 0, st, (const float *)po, (const float *)pml, n_head, head_dim, n_splits, qs ? nullptr : dst, qs, d, sums, sums16);
     }
-    if ((n_head * head_dim) % 256 == 0 && n_splits <= kCombineMaxSplits)
-        return launch_pdl(few ? attn_combine_wide_kernel<false, true> : attn_combine_wide_kernel<false, false>, dim3(merge_ctas), dim3(256), 0, st, (const float *)po,
-                          (const float *)pml, n_head, head_dim, n_splits, dst, (int8_t *)nullptr, (float *)nullptr, (int32_t *)nullptr,
-                          (int32_t *)nullptr);
     return launch_pdl(attn_combine_kernel, dim3(q_rows * n_head), dim3(head_dim), 0, st, (const float *)po, (const float *)pml, dst, head_dim, n_splits);
 }
 
