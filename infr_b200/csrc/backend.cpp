@@ -471,12 +471,13 @@ size_t CudaBackend::tc_scratch_bytes(int dtype, uint32_t m, uint32_t in_f, uint3
 // One weight, or two against the same rows in one launch.  The context scratch holds the operand layout of the rows and the
 // K-split partial results behind it.
 Status CudaBackend::tc_linear(int dtype, const uint8_t *w, float *y, uint32_t out_f, const uint8_t *w2, float *y2, uint32_t out_f2, const float *x,
-                              const Q8Dev *a, uint32_t m, uint32_t in_f) {
+                              const Q8Dev *a, uint32_t m, uint32_t in_f, const RowSource *src) {
     const size_t rec = align_up(gemm_tc_record_bytes(dtype, (int)m, (int)in_f), 256);
     const size_t part = gemm_tc_partial_bytes(dtype, (int)m, (int)in_f, (int)out_f, (int)out_f2, dev_);
     Status s = ensure_scratch(tc_scratch_bytes(dtype, m, in_f, out_f, out_f2));
     if (!s.ok()) return s;
-    s = cuda_status(launch_gemm_tc_prep(dtype, x, a, scratch(), (int)m, (int)in_f, stream_), "gemm_tc layout");
+    s = cuda_status(src ? launch_gemm_tc_prep(dtype, *src, scratch(), (int)m, (int)in_f, stream_) : launch_gemm_tc_prep(dtype, x, a, scratch(), (int)m, (int)in_f, stream_),
+                    "gemm_tc layout");
     if (!s.ok()) return s;
     s = cuda_status(launch_gemm_tc(dtype, w, scratch(), y, part ? reinterpret_cast<float *>(scratch() + rec) : nullptr, (int)m, (int)in_f, (int)out_f, dev_,
                                    status_dev_, stream_, w2, y2, (int)out_f2),
@@ -503,6 +504,26 @@ Status CudaBackend::q2_linear(const uint8_t *w, float *y, uint32_t out_f, const 
                     "gemm_q2");
     if (s.ok()) launches_ += 2 + (part ? 1 : 0);
     return s;
+}
+
+bool CudaBackend::tc_rows(int dtype, uint32_t m, uint32_t in_f, uint64_t out_f) const {
+    if (reference_ || (dtype != DT_Q4K && dtype != DT_Q6K) || m == 0 || out_f == 0) return false;
+    const bool wide = wide_applies(dtype, m, in_f, out_f, INFR_ACT_INT8);
+    if (wide ? !tc_wins(dtype, m, in_f, out_f) : !tc_applies(dtype, m, in_f, out_f, INFR_ACT_INT8)) return false;
+    return !(dtype == DT_Q4K && mmq_impl_ == 1);
+}
+
+Status CudaBackend::linear_from(const RowSource &src, int dtype, const uint8_t *w1, float *y1, uint32_t out_f1, const uint8_t *w2, float *y2, uint32_t out_f2, uint32_t m,
+                                uint32_t in_f, bool *taken) {
+    *taken = false;
+    const size_t n = (size_t)m * in_f;
+    if (!tc_rows(dtype, m, in_f, (uint64_t)out_f1 + out_f2) || !out_f1 || (w2 && !out_f2)) return Status::Ok();
+    if (((uintptr_t)src.a | (uintptr_t)src.b | (uintptr_t)src.sum | (uintptr_t)src.norm_w | (uintptr_t)src.dst) % 16) return Status::Ok();
+    auto apart = [&](const float *p) { return !p || p == src.dst || !overlap(p, n, src.dst, n); };
+    if (!apart(src.a) || !apart(src.b) || !apart(src.sum)) return Status::Ok();
+    *taken = true;
+    cudaSetDevice(device_);
+    return tc_linear(dtype, w1, y1, out_f1, w2, y2, out_f2, nullptr, nullptr, m, in_f, &src);
 }
 
 // Two weights of one format against the same f32 rows (q and k, gate and up): the rows are quantised once.

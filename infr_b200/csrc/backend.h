@@ -114,6 +114,10 @@ public:
     // One-row Linears in one launch (gemv_row.cu).  *taken false: nothing was launched (the kernel does not take the call, spans overlap, or
     // the options ask for another kernel) and the caller runs the ops one by one.
     Status linear_row(const GemvRow &d, bool *taken);
+    // A Linear (w2 != null: two of one format) on rows that src forms, where the tensor-memory GEMM takes it: the rows are formed, stored and
+    // laid out in one launch; results are those of the two ops.  *taken false: nothing was launched, the caller runs the ops one by one.
+    Status linear_from(const RowSource &src, int dtype, const uint8_t *w1, float *y1, uint32_t out_f1, const uint8_t *w2, float *y2, uint32_t out_f2, uint32_t m,
+                       uint32_t in_f, bool *taken);
     // Op::MoeFfn (crates/infr-cpu/src/lib.rs:2264-2984), qwen3moe configuration.  Optional debug outputs:
     // sel_ids [rows,n_used] i32, sel_w [rows,n_used] f32, logits [rows,n_expert] f32 (null = not wanted).
     struct MoeArgs {
@@ -224,9 +228,10 @@ private:
     // Larger Q4_K and Q6_K batches through the tensor-memory GEMM, from f32 rows (x) or quantised ones (a).
     bool tc_applies(int dtype, uint32_t m, uint32_t in_f, uint64_t out_f, int act) const;
     bool tc_wins(int dtype, uint32_t m, uint32_t in_f, uint64_t out_f) const;
+    bool tc_rows(int dtype, uint32_t m, uint32_t in_f, uint64_t out_f) const;  // whether a Linear of that many f32 rows goes there
     size_t tc_scratch_bytes(int dtype, uint32_t m, uint32_t in_f, uint32_t out_f1, uint32_t out_f2 = 0) const;
     Status tc_linear(int dtype, const uint8_t *w, float *y, uint32_t out_f, const uint8_t *w2, float *y2, uint32_t out_f2, const float *x, const Q8Dev *a,
-                     uint32_t m, uint32_t in_f);
+                     uint32_t m, uint32_t in_f, const RowSource *src = nullptr);
     // Device blocks behind the Internal handles of compiled plans; a freed plan's blocks are reused by the next
     // compile (the reference rebuilds its graph every step, so compile must not cost an allocation each time).
     struct PoolBlock {

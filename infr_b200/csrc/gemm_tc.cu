@@ -43,6 +43,7 @@
 #include "gemv_common.cuh"
 #include "pdl.cuh"
 #include "q8_code.cuh"
+#include "row_norm.cuh"
 
 namespace infr {
 namespace {
@@ -374,6 +375,87 @@ __global__ void __launch_bounds__(256) gemm_tc_prep_kernel(const float *x, Q8Dev
     } else {
         if (lane == 0) reinterpret_cast<float *>(ex)[t] = d;
     }
+}
+
+// The same layout and quantiser for a block that a warp holds as lane l = elements 4l..4l+3 (v[0]) and 128+4l.. (v[1]): what the kernels
+// below end with, so that a row which a norm or a gated activation has just formed needs no launch (and no read) of its own.
+template <int FMT>
+__device__ __forceinline__ void store_operand(const float4 (&v)[2], int T, int b, int nb, int tn, uint8_t *__restrict__ units, uint8_t *__restrict__ extra) {
+    using C64 = Cfg<FMT, 64>;
+    constexpr int UPS = C64::kUnits, UB = C64::kUnitBytes / 64, EB = C64::kExtra / 64, PL = FMT == F_Q4 ? 16 : 8;
+    const int lane = threadIdx.x & 31, tt = T / tn, t = T - tt * tn;
+    float am = 0.f;
+#pragma unroll
+    for (int h = 0; h < 2; h++) am = fmaxf(fmaxf(am, fmaxf(fabsf(v[h].x), fabsf(v[h].y))), fmaxf(fabsf(v[h].z), fabsf(v[h].w)));
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) am = fmaxf(am, __shfl_xor_sync(0xffffffffu, am, o));
+    const float d = am / 127.0f, id = d > 0.0f ? 1.0f / d : 0.0f;
+    auto pair16 = [](uint32_t two) { return h2add(__byte_perm(two, 0x64646464u, 0x4140), dup(H_N1152)); };
+    const size_t rec = (size_t)tt * nb + b;
+    uint8_t *ex = extra + rec * EB * tn;
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        const uint32_t codes = q8_codes4(v[h], id), e = codes ^ 0x80808080u;
+        const int p = h * 16 + (lane >> 1), unit = p / PL, pl = p % PL;  // 8 elements a plane: two lanes fill its 16 bytes
+        *reinterpret_cast<uint2 *>(units + ((rec * UPS + unit) * UB + (size_t)pl * 16) * tn + (size_t)t * 16 + (lane & 1) * 8) =
+            make_uint2(pair16(__byte_perm(e, 0, 0x0020)), pair16(__byte_perm(e, 0, 0x0031)));
+        if (FMT == F_Q4) {
+            int sum = q8_sum4(codes);
+#pragma unroll
+            for (int o = 1; o < 8; o <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+            if ((lane & 7) == 0) {
+                __half *hl = reinterpret_cast<__half *>(ex + (size_t)t * 16) + h * 4 + (lane >> 3);
+                hl[0] = __int2half_rn((sum >> 6) * 64);
+                hl[(size_t)tn * 8] = __int2half_rn(sum & 63);
+            }
+        }
+    }
+    if (lane == 0) reinterpret_cast<float *>(ex + (FMT == F_Q4 ? (size_t)tn * 32 : 0))[t] = d;
+}
+
+// RMSNorm (of a + b with ADD) and the layout in one launch: CTA = token slot; the scaled row also goes to dst.
+template <int FMT, bool ADD>
+__global__ void __launch_bounds__(1024) gemm_tc_norm_prep_kernel(const float *a, const float *b, float *sum_dst, const float *__restrict__ w, float *__restrict__ dst,
+                                                                 float eps, int m, int tn, int in_f, uint8_t *__restrict__ units, uint8_t *__restrict__ extra) {
+    __shared__ float s_part[32];
+    const int lane = threadIdx.x & 31, T = blockIdx.x, nb = in_f >> 8;
+    if (T >= m) {  // a slot past the last token: zeros
+        pdl_go();
+        pdl_wait();
+        const float4 zero[2] = {make_float4(0.f, 0.f, 0.f, 0.f), make_float4(0.f, 0.f, 0.f, 0.f)};
+        for (int c = threadIdx.x >> 5; c < nb; c += blockDim.x >> 5) store_operand<FMT>(zero, T, c, nb, tn, units, extra);
+        return;
+    }
+    rms_norm_row<ADD>(a, b, sum_dst, w, in_f, eps, T, s_part, [&](int c, const float4 (&v)[2]) {
+#pragma unroll
+        for (int h = 0; h < 2; h++) *reinterpret_cast<float4 *>(dst + (size_t)T * in_f + c * 256 + h * 128 + lane * 4) = v[h];
+        store_operand<FMT>(v, T, c, nb, tn, units, extra);
+    });
+}
+
+// silu(gate) * up and the layout in one launch: a warp per (token slot, block); the rows also go to dst (which may be gate or up).
+template <int FMT>
+__global__ void __launch_bounds__(256) gemm_tc_silu_prep_kernel(const float *gate, const float *up, float *dst, int m, int tn, int in_f, uint8_t *__restrict__ units,
+                                                                uint8_t *__restrict__ extra, int n_tok) {
+    pdl_go();
+    pdl_wait();
+    const int lane = threadIdx.x & 31, nb = in_f >> 8;
+    const long long wg = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (wg >= (long long)n_tok * nb) return;
+    const int T = (int)(wg / nb), b = (int)(wg % nb);
+    float4 v[2] = {make_float4(0.f, 0.f, 0.f, 0.f), make_float4(0.f, 0.f, 0.f, 0.f)};
+    if (T < m) {
+        const size_t e = (size_t)T * in_f + (size_t)b * 256 + lane * 4;
+        float4 g[2], u[2];
+#pragma unroll
+        for (int h = 0; h < 2; h++) g[h] = *reinterpret_cast<const float4 *>(gate + e + h * 128), u[h] = *reinterpret_cast<const float4 *>(up + e + h * 128);
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            v[h] = make_float4(silu_mul(g[h].x, u[h].x), silu_mul(g[h].y, u[h].y), silu_mul(g[h].z, u[h].z), silu_mul(g[h].w, u[h].w));
+            *reinterpret_cast<float4 *>(dst + e + h * 128) = v[h];
+        }
+    }
+    store_operand<FMT>(v, T, b, nb, tn, units, extra);
 }
 
 template <int FMT, int TN>
@@ -986,6 +1068,21 @@ cudaError_t launch_gemm_tc_prep(int dtype, const float *x, const Q8Dev *a, void 
     const int f = fmt_of(dtype), tn = tile_of_batch(m), n = (m + tn - 1) / tn * tn;
     uint8_t *u = static_cast<uint8_t *>(records), *e = u + units_bytes(n, in_f);
     return x ? launch_prep<true>(f, x, Q8Dev{}, m, tn, in_f, u, e, n, TcGroup{}, st) : launch_prep<false>(f, nullptr, *a, m, tn, in_f, u, e, n, TcGroup{}, st);
+}
+
+// The same from what forms the rows (RowSource).
+cudaError_t launch_gemm_tc_prep(int dtype, const RowSource &src, void *records, int m, int in_f, cudaStream_t st) {
+    if (m < 1 || !gemm_tc_takes(dtype, in_f)) return cudaErrorInvalidValue;
+    const int f = fmt_of(dtype), tn = tile_of_batch(m), n = (m + tn - 1) / tn * tn, nb = in_f / 256;
+    uint8_t *u = static_cast<uint8_t *>(records), *e = u + units_bytes(n, in_f);
+    if (!src.norm_w) {
+        auto kernel = f == F_Q4 ? gemm_tc_silu_prep_kernel<F_Q4> : gemm_tc_silu_prep_kernel<F_Q6>;
+        return launch_pdl(kernel, dim3((unsigned)(((size_t)n * nb + 7) / 8)), dim3(256), 0, st, src.a, src.b, src.dst, m, tn, in_f, u, e, n);
+    }
+    const int threads = nb > 32 ? 1024 : nb * 32;
+    auto kernel = f == F_Q4 ? (src.b ? gemm_tc_norm_prep_kernel<F_Q4, true> : gemm_tc_norm_prep_kernel<F_Q4, false>)
+                            : (src.b ? gemm_tc_norm_prep_kernel<F_Q6, true> : gemm_tc_norm_prep_kernel<F_Q6, false>);
+    return launch_pdl(kernel, dim3((unsigned)n), dim3((unsigned)threads), 0, st, src.a, src.b, src.sum, src.norm_w, src.dst, src.eps, m, tn, in_f, u, e);
 }
 
 cudaError_t launch_gemm_tc(int dtype, const uint8_t *w, const void *records, float *c, float *partials, int m, int in_f, int out_f, const DeviceInfo &dev,

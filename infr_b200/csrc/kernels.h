@@ -137,6 +137,16 @@ bool gemm_tc_takes(int dtype, int in_f);
 size_t gemm_tc_record_bytes(int dtype, int m, int in_f);
 size_t gemm_tc_partial_bytes(int dtype, int m, int in_f, int out_f1, int out_f2, const DeviceInfo &dev);
 cudaError_t launch_gemm_tc_prep(int dtype, const float *x, const Q8Dev *a, void *records, int m, int in_f, cudaStream_t st);
+// What forms the f32 rows that a Linear reads, for a layout launch that does both: RMSNorm of a (b != null: of a + b, written to sum) with
+// weights norm_w, or, norm_w == null, silu(a) * b.  The rows also go to dst.  Every pointer 16-byte aligned; dst, a and b equal or apart.
+struct RowSource {
+    const float *a, *b;
+    float *sum;
+    const float *norm_w;
+    float *dst;
+    float eps;
+};
+cudaError_t launch_gemm_tc_prep(int dtype, const RowSource &src, void *records, int m, int in_f, cudaStream_t st);
 cudaError_t launch_gemm_tc(int dtype, const uint8_t *w, const void *records, float *c, float *partials, int m, int in_f, int out_f, const DeviceInfo &dev,
                            uint32_t *status, cudaStream_t st, const uint8_t *w2 = nullptr, float *c2 = nullptr, int out_f2 = 0);
 // Batched GEMM for Q2_0 (gemm_q2.cu), more than 8 rows of any length: prep quantises the f32 rows and lays them out in `records`

@@ -8,6 +8,7 @@
 //                                        (runner.rs:3824-3838 emits exactly this pair between the two halves of a layer)
 //   Linear, Linear (same rows, same format) -> rows quantised once, one launch for a decode batch of Q4_K
 //                                        (runner.rs:3476-3523 q/k/v, :3882-3933 gate/up)
+//   RmsNorm or GatedAct (or the first pair), then Linear(s) that the tensor-memory GEMM takes -> the rows are formed and laid out for it in one launch
 //   one-row Linears of one format and length that do not depend on each other -> up to 24 in a launch (three on the same row)
 //   Rope(k), Rope(q), WriteKv, WriteKv -> q rotated in place, k rotated and v cast straight into the f16 caches
 //                                        (runner.rs:3611-3656), when the rotated k has no other reader
@@ -509,9 +510,32 @@ Status CudaBackend::execute_steps(infr_cuda_plan *plan, infr_cuda_buf *const *bi
         return s;
     };
 
-    for (const PlanStep &st : plan->steps) {
+    // The rows that src forms go to tensor `id`; where the next step is a Linear or a pair of them that reads these rows and that the
+    // tensor-memory GEMM takes, both steps run here (*fed).
+    auto feed = [&](size_t next, uint32_t id, uint32_t rows, uint32_t dim, const RowSource &src, bool *fed) -> Status {
+        *fed = false;
+        if (next >= plan->steps.size()) return Status::Ok();
+        const PlanStep &ns = plan->steps[next];
+        const infr_op_desc &l = plan->ops[ns.op0];
+        if ((ns.kind != PlanStep::kSingle && ns.kind != PlanStep::kLinearPair) || l.tag != INFR_OP_LINEAR) return Status::Ok();
+        const bool pair = ns.kind == PlanStep::kLinearPair;
+        const infr_op_desc &l2 = plan->ops[pair ? ns.op0 + 1 : ns.op0];
+        const int wdt = (int)plan->tensors[l.t[1]].dtype;
+        if (l.t[0] != id || l.u[0] != rows || l.u[1] != dim || !tc_rows(wdt, rows, dim, (uint64_t)l.u[2] + (pair ? l2.u[2] : 0))) return Status::Ok();
+        const size_t bpr = (size_t)(dim / block_elems(wdt)) * block_bytes(wdt), r1 = l.u[3] / dim, r2 = l2.u[3] / dim;
+        DevSpan w1, w2, y1, y2;
+        INFR_RESOLVE(l.t[1], (r1 + l.u[2]) * bpr, "Linear weight", &w1);
+        INFR_RESOLVE(l2.t[1], (r2 + l2.u[2]) * bpr, "Linear weight", &w2);
+        INFR_RESOLVE(l.t[2], (size_t)rows * l.u[2] * 4, "Linear dst", &y1);
+        INFR_RESOLVE(l2.t[2], (size_t)rows * l2.u[2] * 4, "Linear dst", &y2);
+        return linear_from(src, wdt, w1.ptr + r1 * bpr, f32p(y1), l.u[2], pair ? w2.ptr + r2 * bpr : nullptr, pair ? f32p(y2) : nullptr, pair ? l2.u[2] : 0, rows, dim, fed);
+    };
+
+    for (size_t i = 0; i < plan->steps.size(); i++) {
+        const PlanStep &st = plan->steps[i];
         const infr_op_desc &op = plan->ops[st.op0];
         Status s;
+        bool fed = false;
         if (st.kind == PlanStep::kAddRmsNorm) {
             const infr_op_desc &nm = plan->ops[st.op0 + 1];
             const uint32_t rows = nm.u[0], dim = nm.u[1];
@@ -522,7 +546,9 @@ Status CudaBackend::execute_steps(infr_cuda_plan *plan, infr_cuda_buf *const *bi
             INFR_RESOLVE(op.t[2], nb, "Add dst", &sum);
             INFR_RESOLVE(nm.t[1], (size_t)dim * 4, "RmsNorm weight", &w);
             INFR_RESOLVE(nm.t[2], nb, "RmsNorm dst", &dst);
-            s = rms_norm(f32p(a), f32p(b), f32p(sum), f32p(w), f32p(dst), rows, dim, nm.f[0]);
+            s = feed(i + 1, nm.t[2], rows, dim, RowSource{f32p(a), f32p(b), f32p(sum), f32p(w), f32p(dst), nm.f[0]}, &fed);
+            if (fed) i++;
+            if (s.ok() && !fed) s = rms_norm(f32p(a), f32p(b), f32p(sum), f32p(w), f32p(dst), rows, dim, nm.f[0]);
             if (!s.ok()) return s;
             continue;
         }
@@ -581,7 +607,23 @@ Status CudaBackend::execute_steps(infr_cuda_plan *plan, infr_cuda_buf *const *bi
             if (!s.ok()) return s;
             continue;
         }
-        s = run_single(op);
+        if (op.tag == INFR_OP_RMS_NORM) {
+            const size_t nb = (size_t)op.u[0] * op.u[1] * 4;
+            DevSpan x, w, dst;
+            INFR_RESOLVE(op.t[0], nb, "RmsNorm x", &x);
+            INFR_RESOLVE(op.t[1], (size_t)op.u[1] * 4, "RmsNorm weight", &w);
+            INFR_RESOLVE(op.t[2], nb, "RmsNorm dst", &dst);
+            s = feed(i + 1, op.t[2], op.u[0], op.u[1], RowSource{f32p(x), nullptr, nullptr, f32p(w), f32p(dst), op.f[0]}, &fed);
+        } else if (op.tag == INFR_OP_GATED_ACT) {
+            const size_t nb = (size_t)op.u[0] * op.u[1] * 4;
+            DevSpan gt, up, dst;
+            INFR_RESOLVE(op.t[0], nb, "GatedAct gate", &gt);
+            INFR_RESOLVE(op.t[1], nb, "GatedAct up", &up);
+            INFR_RESOLVE(op.t[2], nb, "GatedAct dst", &dst);
+            s = feed(i + 1, op.t[2], op.u[0], op.u[1], RowSource{f32p(gt), f32p(up), nullptr, nullptr, f32p(dst), 0.f}, &fed);
+        }
+        if (fed) i++;
+        if (s.ok() && !fed) s = run_single(op);
         if (!s.ok()) return s;
     }
 #undef INFR_RESOLVE
