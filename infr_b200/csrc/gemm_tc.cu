@@ -29,7 +29,11 @@
 // Measured (B200, us, whole calls over rotated cold weights, back to back, so that a call's layout launch overlaps the call before; before
 // = a warp issuing under `lane == 0`, stages held until the epilogue, whole waves only):  Q4_K 4096 -> 14336, 512 rows 113 -> 82 (a call
 // that waits for the one before it: 112 -> 89), 113 rows 35 -> 30, 1024 rows 192 -> 153;  14336 -> 4096, 1024 rows 194 -> 175;  Q6_K
-// 14336 -> 4096, 113 rows 57 -> 53, 512 rows 183 -> 177.  Some Q6_K shapes lost: 33..64 rows of 4096 -> 14336 49 -> 52.
+// 14336 -> 4096, 113 rows 57 -> 53, 512 rows 183 -> 177.
+// Q6_K's unpacking was the longest part of a job (3900 of 5860 cycles of an unpack warp, clock64).  Nibble and high bits meet in one LOP3 before
+// the bytes part (5 integer instructions for 4 weights, 7 before), the offset is inside the multiply-add, rows are read in 8-byte words from
+// a pitch of 240 bytes (no conflicts, one level of selects less) and the two teams' slots are multiplied in turn.  Cold weights, us, before:
+// 4096 -> 14336, 33..64 rows 42, 53; 113 rows 52, 57; 512 rows 154, 165;  14336 -> 4096, 64 rows 42, 52; 113 rows 51, 55; 1000 rows 296, 318.
 // What bounds it: issue slots and waits.  At 128 tokens a Q4_K job takes ~2550 cycles, its MMAs
 // 1150 (tensor pipe 45 % busy); the warps issue 6670 instructions a job, 0.66 a cycle and scheduler.
 // Every wait is bounded: on expiry the role raises a CTA flag and a status word, every role leaves its loop, copies in
@@ -62,7 +66,7 @@ struct Cfg {
     // of 64 tokens and one half is drained while the other is multiplied.
     static constexpr int kJobBuf = FMT == F_Q6 && TN == 128 ? 1 : 2;
     static constexpr int kPass = 3 - kJobBuf;
-    static constexpr int kRowBytes = FMT == F_Q6 ? 224 : 144;
+    static constexpr int kRowBytes = FMT == F_Q6 ? 240 : 144;
     static constexpr int kRaw = kTM * kRowBytes;
     static constexpr int kUnitBytes = (FMT == F_Q4 ? 256 : 128) * TN;
     static constexpr int kExtra = FMT == F_Q4 ? 36 * TN : 4 * TN;    // per job: token scales, Q4_K also the split block sums
@@ -203,13 +207,19 @@ __device__ __forceinline__ uint32_t h2add(uint32_t a, uint32_t b) {
 }
 __device__ __forceinline__ constexpr uint32_t dup(uint32_t h) { return h | (h << 16); }
 // f16 bit patterns of the small constants used below (integers and powers of two)
-constexpr uint32_t H_1024 = 0x6400, H_N1024 = 0xE400, H_N1152 = 0xE480, H_64 = 0x5400, H_N72 = 0xD480, H_N8192 = 0xF000, H_1_16 = 0x2C00, H_1_4 = 0x3400, H_1_64 = 0x2400,
-                   H_1 = 0x3C00, H_N1032 = 0xE408, H_N1056 = 0xE420, H_N1536 = 0xE600;
+constexpr uint32_t H_1024 = 0x6400, H_N1024 = 0xE400, H_N1152 = 0xE480, H_64 = 0x5400, H_N72 = 0xD480, H_N8192 = 0xF000, H_1_4 = 0x3400, H_1_64 = 0x2400,
+                   H_1 = 0x3C00, H_N1032 = 0xE408, H_N1056 = 0xE420;
 
 // (a & m) | c in one instruction: with m and c in registers.  As constants they would be two immediates, which one LOP3 cannot take.
 __device__ __forceinline__ uint32_t and_or(uint32_t a, uint32_t m, uint32_t c) {
     uint32_t r;
     asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(r) : "r"(a), "r"(m), "r"(c));
+    return r;
+}
+// the low nibbles of a's bytes under the high nibbles of b's
+__device__ __forceinline__ uint32_t low_nibbles(uint32_t a, uint32_t b) {
+    uint32_t r;
+    asm("lop3.b32 %0, %1, %2, 0x0F0F0F0F, 0xE4;" : "=r"(r) : "r"(a), "r"(b));
     return r;
 }
 __device__ __forceinline__ uint32_t in_reg(uint32_t v) {
@@ -233,44 +243,44 @@ __device__ __forceinline__ void unpack_q4(const uint32_t *w, uint32_t s0, uint32
     }
 }
 
-// Q6_K: 32 elements (part = 0..3 of a half block): low nibbles from ql[8 words], two high bits from qh[8 words], scales of
-// the two 16-element sub-blocks (low byte each).  o[0..15] = sl * (q - 32), o[16..31] = sh * (q - 32) with sc = 16 sh + sl,
-// 0 <= sl < 16, -8 <= sh < 8, the same element order as above.  k = the f16 of 1024 twice (in_reg)
+// Q6_K: 32 elements (part = 0..3 of a half block): low or high nibbles from ql[8 words], two high bits from qh[8 words], scales
+// sc = 16 sh + sl of the two 16-element sub-blocks: bytes 2 (part & 1), + 1 of lw (sl, 0 <= sl < 16) and hw (sh + 8, -8 <= sh < 8).
+// o[0..15] = sl * (q - 32), o[16..31] = sh * (q - 32), the same element order as above.  m = 0x003F003F, k = the f16 of 1024 twice (in_reg)
 template <int PART>
-__device__ __forceinline__ void unpack_q6(const uint32_t *ql, const uint32_t *qh, uint32_t sc0, uint32_t sc1, uint32_t k, uint32_t (&o)[32]) {
-    constexpr bool HI = PART >= 2;
-    // the nibbles stay where they are, so q is built at bit 0 (parts 0, 1) or bit 4 (parts 2, 3), below the f16 of 1024
-    const uint32_t lm = in_reg(HI ? 0x00F000F0u : 0x000F000Fu), hm = in_reg(HI ? 0x03000300u : 0x00300030u);
-    constexpr uint32_t off = HI ? H_N1536 : H_N1056;         // -(1024 + 16 * 32), -(1024 + 32)
-    constexpr int up = PART & 1 ? 2 : 4;                     // the high bits' way to their place (bytes 1 and 3: 8 less)
-    const uint32_t sc[2] = {sc0, sc1};
+__device__ __forceinline__ void unpack_q6(const uint32_t *ql, const uint32_t *qh, uint32_t lw, uint32_t hw, uint32_t m, uint32_t k, uint32_t (&o)[32]) {
 #pragma unroll
     for (int g = 0; g < 2; g++) {
-        uint32_t sl = h2add(dup(H_1024) | (sc[g] & 0xFu) * 0x10001u, dup(H_N1024));
-        uint32_t sh = h2add(dup(H_1024) | (((sc[g] >> 4) & 0xFu) ^ 8u) * 0x10001u, dup(H_N1032));
-        if (HI) sl = h2mul(sl, dup(H_1_16)), sh = h2mul(sh, dup(H_1_16));
+        constexpr uint32_t sel0 = 0x4040u + (PART & 1) * 0x0202u;  // the scale's byte below the high byte of the f16 of 1024, twice
+        const uint32_t sl = h2add(__byte_perm(lw, 0x64646464u, sel0 + g * 0x0101u), dup(H_N1024));
+        const uint32_t sh = h2add(__byte_perm(hw, 0x64646464u, sel0 + g * 0x0101u), dup(H_N1032));
+        const uint32_t cl = h2mul(sl, dup(H_N1056)), ch = h2mul(sh, dup(H_N1056));  // (1024 + q) * s - 1056 * s: 33 * s has nine bits, one rounding, exact
 #pragma unroll
         for (int i = 4 * g; i < 4 * g + 4; i++) {
-            const uint32_t v = ql[i], u = v >> 8, y = qh[i] << up, z = qh[i] >> (8 - up);
-            const uint32_t a = h2add(and_or(v, lm, and_or(y, hm, k)), dup(off)), b = h2add(and_or(u, lm, and_or(z, hm, k)), dup(off));
-            o[2 * i] = h2mul(a, sl);
-            o[2 * i + 1] = h2mul(b, sl);
-            o[16 + 2 * i] = h2mul(a, sh);
-            o[17 + 2 * i] = h2mul(b, sh);
+            const uint32_t v = PART >= 2 ? ql[i] >> 4 : ql[i];
+            const uint32_t y = PART == 0 ? qh[i] << 4 : PART == 1 ? qh[i] << 2 : PART == 2 ? qh[i] : qh[i] >> 2;
+            const uint32_t q = low_nibbles(v, y), e = and_or(q, m, k), f = and_or(q >> 8, m, k);
+            o[2 * i] = h2fma(e, sl, cl);
+            o[2 * i + 1] = h2fma(f, sl, cl);
+            o[16 + 2 * i] = h2fma(e, sh, ch);
+            o[17 + 2 * i] = h2fma(f, sh, ch);
         }
     }
 }
 
-// words v[] starting `ow` words and `sh` / 8 bytes (sh = 0 or 16) into an aligned run
-template <int NIN, int NOUT>
-__device__ __forceinline__ void realign(uint32_t (&v)[NIN], int ow, uint32_t sh, uint32_t (&o)[NOUT]) {
-    static_assert(NIN >= NOUT + 4, "");
+// N words from byte p + rem on, p 8-byte aligned, rem = 0, 2, 4 or 6
+template <int N>
+__device__ __forceinline__ void load_words(const uint8_t *p, int rem, uint32_t (&o)[N]) {
+    static_assert(N % 2 == 0, "");
+    uint32_t v[N + 2];
 #pragma unroll
-    for (int i = 0; i < NOUT + 3; i++) v[i] = (ow & 1) ? v[i + 1] : v[i];
+    for (int i = 0; i < N + 2; i += 2) {
+        const uint2 w = *reinterpret_cast<const uint2 *>(p + 4 * i);
+        v[i] = w.x, v[i + 1] = w.y;
+    }
 #pragma unroll
-    for (int i = 0; i < NOUT + 1; i++) v[i] = (ow & 2) ? v[i + 2] : v[i];
+    for (int i = 0; i < N + 1; i++) v[i] = (rem & 4) ? v[i + 1] : v[i];
 #pragma unroll
-    for (int i = 0; i < NOUT; i++) o[i] = __funnelshift_r(v[i], v[i + 1], sh);
+    for (int i = 0; i < N; i++) o[i] = __funnelshift_r(v[i], v[i + 1], (uint32_t)(rem & 2) * 8);
 }
 
 struct TcMat {
@@ -630,7 +640,8 @@ __global__ void __launch_bounds__(Cfg<FMT, TN>::kWarps * 32, Cfg<FMT, TN>::kCtas
                             if (pass > 0) tc_fence_after();
                         }
 #pragma unroll
-                        for (int u = 0; u < K::kUnits; u++) {
+                        for (int uu = 0; uu < K::kUnits; uu++) {
+                            const int u = K::kUnits == 4 ? (uu >> 1) + (uu & 1) * 2 : uu;  // the teams' slots in turn: both get theirs back early
                             if (pass == 0 && !(ok = wait_bar(bar(K::B_BFULL + q + u), qp, dead))) break;
                             const uint64_t bd = bd0 + (uint64_t)((q + u) * (uint32_t)(K::kUnitBytes / 16) + pass * (TN / K::kPass));
                             constexpr int kTeamUnits = K::kUnits / 2;
@@ -648,7 +659,7 @@ __global__ void __launch_bounds__(Cfg<FMT, TN>::kWarps * 32, Cfg<FMT, TN>::kCtas
                                     // Q6_K: the sl and the sh operands of a slot meet the same 32 activations
                                     const int pl = FMT == F_Q6 ? h * 4 + (k & 1) * 2 : h * 8 + k * 2;
                                     const uint32_t dst = td + (uint32_t)((K::kAcc == 2 ? (k >> 1) * TN : 0) + pass * (TN / K::kPass));
-                                    const uint32_t keep = (uint32_t)(u > 0 || h > 0 || (K::kAcc == 2 ? (k & 1) : k > 0));
+                                    const uint32_t keep = (uint32_t)(uu > 0 || h > 0 || (K::kAcc == 2 ? (k & 1) : k > 0));
                                     mma_ta(dst, ta + (uint32_t)(k * 8), bd + (uint64_t)(pl * TN), idesc, keep);
                                 }
                                 if (pass == K::kPass - 1) mma_commit(bar(K::B_AFREE + sl));
@@ -745,7 +756,7 @@ __global__ void __launch_bounds__(Cfg<FMT, TN>::kWarps * 32, Cfg<FMT, TN>::kCtas
         const int n = n_items();
         const int quarter = warp & 3, team = warp >> 2, row = quarter * 32 + lane;
         const uint32_t tl = tmem + ((uint32_t)(quarter * 32) << 16) + K::kColA;
-        const uint32_t km = in_reg(0x00F000F0u), kc = in_reg(FMT == F_Q4 ? dup(H_64) : dup(H_1024));
+        const uint32_t km = in_reg(FMT == F_Q4 ? 0x00F000F0u : 0x003F003Fu), kc = in_reg(FMT == F_Q4 ? dup(H_64) : dup(H_1024));
         int js = 0;
         bool ok = true;
         // the team's slot of its use-th operand run: its previous MMAs are complete, it is filled, it is announced
@@ -784,43 +795,22 @@ __global__ void __launch_bounds__(Cfg<FMT, TN>::kWarps * 32, Cfg<FMT, TN>::kCtas
                     if (!(ok = put(js * 2 + 1, o))) break;
                 } else {
                     // half block `team`: the low and then the high nibbles of its 64 bytes
-                    const int off = (b * 210) & 15, ow = off >> 2;
-                    const uint32_t sh = (off & 2) * 8;
-                    uint32_t ql[16], qh[8], scw[2];
-                    {
-                        uint32_t v[20];
-#pragma unroll
-                        for (int k = 0; k < 5; k++) {
-                            const uint4 q = bv[4 * team + k];
-                            v[4 * k] = q.x, v[4 * k + 1] = q.y, v[4 * k + 2] = q.z, v[4 * k + 3] = q.w;
-                        }
-                        realign(v, ow, sh, ql);
-                    }
-                    {
-                        uint32_t v[12];
-#pragma unroll
-                        for (int k = 0; k < 3; k++) {
-                            const uint4 q = bv[8 + 2 * team + k];
-                            v[4 * k] = q.x, v[4 * k + 1] = q.y, v[4 * k + 2] = q.z, v[4 * k + 3] = q.w;
-                        }
-                        realign(v, ow, sh, qh);
-                    }
-                    {
-                        // scales [192 + off, +16)
-                        const uint4 p = bv[12], q = bv[13];
-                        uint32_t v[8] = {p.x, p.y, p.z, p.w, q.x, q.y, q.z, q.w}, u[4];
-                        realign(v, ow, sh, u);
-                        scw[0] = team ? u[2] : u[0];
-                        scw[1] = team ? u[3] : u[1];
-                    }
+                    const int off = (b * 210) & 15, rem = off & 7;
+                    const uint8_t *p = blk + (off & 8);
+                    uint32_t ql[16], qh[8], sc[2];
+                    load_words(p + 64 * team, rem, ql);
+                    load_words(p + 128 + 32 * team, rem, qh);
+                    load_words(p + 192 + 8 * team, rem, sc);
                     given_back();
-                    unpack_q6<0>(ql, qh, scw[0], scw[0] >> 8, kc, o);
+                    const uint32_t l0 = sc[0] & 0x0F0F0F0Fu, l1 = sc[1] & 0x0F0F0F0Fu;
+                    const uint32_t h0 = ((sc[0] >> 4) & 0x0F0F0F0Fu) ^ 0x08080808u, h1 = ((sc[1] >> 4) & 0x0F0F0F0Fu) ^ 0x08080808u;
+                    unpack_q6<0>(ql, qh, l0, h0, km, kc, o);
                     if (!(ok = put(js * 4, o))) break;
-                    unpack_q6<1>(ql + 8, qh, scw[0] >> 16, scw[0] >> 24, kc, o);
+                    unpack_q6<1>(ql + 8, qh, l0, h0, km, kc, o);
                     if (!(ok = put(js * 4 + 1, o))) break;
-                    unpack_q6<2>(ql, qh, scw[1], scw[1] >> 8, kc, o);
+                    unpack_q6<2>(ql, qh, l1, h1, km, kc, o);
                     if (!(ok = put(js * 4 + 2, o))) break;
-                    unpack_q6<3>(ql + 8, qh, scw[1] >> 16, scw[1] >> 24, kc, o);
+                    unpack_q6<3>(ql + 8, qh, l1, h1, km, kc, o);
                     if (!(ok = put(js * 4 + 3, o))) break;
                 }
             }
@@ -962,7 +952,7 @@ bool weight_map(int fmt, const uint8_t *w, size_t rows, int in_f, CUtensorMap *m
     const cuuint32_t one2[2] = {1, 1};
     if (fmt == F_Q6) {
         const cuuint64_t nb = (cuuint64_t)in_f / 256, gdim[2] = {nb * 105, (cuuint64_t)rows}, gstr[1] = {nb * 210};
-        const cuuint32_t box[2] = {112, kTM};
+        const cuuint32_t box[2] = {Cfg<F_Q6, 128>::kRowBytes / 2, kTM};
         return enc(map, CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, const_cast<uint8_t *>(w), gdim, gstr, box, one2, CU_TENSOR_MAP_INTERLEAVE_NONE,
                    CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
     }
