@@ -33,7 +33,7 @@
 // Q6_K's unpacking was the longest part of a job (3900 of 5860 cycles of an unpack warp, clock64).  Nibble and high bits meet in one LOP3 before
 // the bytes part (5 integer instructions for 4 weights, 7 before), the offset is inside the multiply-add, rows are read in 8-byte words from
 // a pitch of 240 bytes (no conflicts, one level of selects less) and the two teams' slots are multiplied in turn.  Cold weights, us, before:
-// 4096 -> 14336, 33..64 rows 42, 53; 113 rows 52, 57; 512 rows 154, 165;  14336 -> 4096, 64 rows 42, 52; 113 rows 51, 55; 1000 rows 296, 318.
+// 4096 -> 14336, 33..64 rows 42, 53; 113 rows 52, 57;  14336 -> 4096, 64 rows 42, 52; 113 rows 51, 55; 1000 rows 296, 318 (and one pass, kJobBuf, after that).
 // What bounds it: issue slots and waits.  At 128 tokens a Q4_K job takes ~2550 cycles, its MMAs
 // 1150 (tensor pipe 45 % busy); the warps issue 6670 instructions a job, 0.66 a cycle and scheduler.
 // Every wait is bounded: on expiry the role raises a CTA flag and a status word, every role leaves its loop, copies in
@@ -62,10 +62,11 @@ struct Cfg {
     static constexpr int kUse = FMT == F_Q4 ? 2 : 4;                 // slots that a team fills per job
     static constexpr int kUnpack = 8;
     static constexpr int kAcc = FMT == F_Q4 ? 1 : 2;                 // accumulators per job
-    // Jobs that have accumulators at a time.  Q6_K, 128 tokens: tensor memory holds those of one, so a job is multiplied in two passes
-    // of 64 tokens and one half is drained while the other is multiplied.
+    // Jobs that have accumulators at a time.  Q6_K, 128 tokens: tensor memory holds those of one.  The operands of the next job are unpacked
+    // while they are drained, so the drain costs nothing.  (Two passes of 64 tokens, one half drained while the other was multiplied, kept
+    // every operand slot until the second pass: 14336 -> 4096, 113 rows 50.6 us, in one pass 46.9;
+    // 1000 rows 296, 254.)
     static constexpr int kJobBuf = FMT == F_Q6 && TN == 128 ? 1 : 2;
-    static constexpr int kPass = 3 - kJobBuf;
     static constexpr int kRowBytes = FMT == F_Q6 ? 240 : 144;
     static constexpr int kRaw = kTM * kRowBytes;
     static constexpr int kUnitBytes = (FMT == F_Q4 ? 256 : 128) * TN;
@@ -493,7 +494,7 @@ __global__ void __launch_bounds__(Cfg<FMT, TN>::kWarps * 32, Cfg<FMT, TN>::kCtas
             if (i >= K::B_SFREE && i < K::B_XFULL) cnt = K::kUnpack + 1;
             if (i >= K::B_XFREE && i < K::B_BFULL) cnt = K::kEpi;
             if (i >= K::B_AFULL && i < K::B_AFREE) cnt = 4;
-            if (i >= K::B_ACCFREE && i <= K::B_MFREE) cnt = K::kEpi / K::kPass;
+            if (i >= K::B_ACCFREE && i <= K::B_MFREE) cnt = K::kEpi;
             asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(su32(&bars[i])), "r"(cnt));
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -617,7 +618,7 @@ __global__ void __launch_bounds__(Cfg<FMT, TN>::kWarps * 32, Cfg<FMT, TN>::kCtas
         // ------------------------------------------------------------------ MMA issuer: one thread, all of the loop
         pdl_wait();
         if (elect_one()) {
-            const uint32_t idesc = (1u << 4) | ((uint32_t)(TN / K::kPass >> 3) << 17) | ((uint32_t)(kTM >> 4) << 24);
+            const uint32_t idesc = (1u << 4) | ((uint32_t)(TN >> 3) << 17) | ((uint32_t)(kTM >> 4) << 24);
             const uint64_t bd0 = mk_desc(su32(bring), TN * 16);
             const int n = n_items();
             int j = 0;               // jobs of this CTA, over all tiles
@@ -628,50 +629,34 @@ __global__ void __launch_bounds__(Cfg<FMT, TN>::kWarps * 32, Cfg<FMT, TN>::kCtas
                 for (int b = t.b0; b < t.b1; b++, j++) {
                     const int s = j & 1;
                     const uint32_t jp = (uint32_t)(j >> 1) & 1u;
-                    const uint32_t td = tmem + (uint32_t)((K::kJobBuf == 2 ? s : 0) * K::kAcc * TN);
+                    const int sa = K::kJobBuf == 2 ? s : 0;  // its accumulators
+                    const uint32_t td = tmem + (uint32_t)(sa * K::kAcc * TN);
+                    // the job that had them before
+                    if (j >= K::kJobBuf && !(ok = wait_bar(bar(K::B_ACCFREE + sa), K::kJobBuf == 2 ? jp ^ 1u : (uint32_t)(j - 1) & 1u, dead))) break;
 #pragma unroll
-                    for (int pass = 0; pass < K::kPass; pass++) {
-                        // the job that had these accumulators before
-                        if (K::kPass == 1) {
-                            if (j >= 2 && !(ok = wait_bar(bar(K::B_ACCFREE + s), jp ^ 1u, dead))) break;
-                        } else {
-                            if (j >= 1 && !(ok = wait_bar(bar(K::B_ACCFREE + pass), (uint32_t)(j - 1) & 1u, dead))) break;
-                            // its reads come before this pass's multiplications (pass 0: the fence behind the operands' wait)
-                            if (pass > 0) tc_fence_after();
-                        }
+                    for (int uu = 0; uu < K::kUnits; uu++) {
+                        const int u = K::kUnits == 4 ? (uu >> 1) + (uu & 1) * 2 : uu;  // the teams' slots in turn: both get theirs back early
+                        if (!(ok = wait_bar(bar(K::B_BFULL + q + u), qp, dead))) break;
+                        const uint64_t bd = bd0 + (uint64_t)((q + u) * (uint32_t)(K::kUnitBytes / 16));
+                        constexpr int kTeamUnits = K::kUnits / 2;
+                        const int team = u / kTeamUnits;
 #pragma unroll
-                        for (int uu = 0; uu < K::kUnits; uu++) {
-                            const int u = K::kUnits == 4 ? (uu >> 1) + (uu & 1) * 2 : uu;  // the teams' slots in turn: both get theirs back early
-                            if (pass == 0 && !(ok = wait_bar(bar(K::B_BFULL + q + u), qp, dead))) break;
-                            const uint64_t bd = bd0 + (uint64_t)((q + u) * (uint32_t)(K::kUnitBytes / 16) + pass * (TN / K::kPass));
-                            constexpr int kTeamUnits = K::kUnits / 2;
-                            const int team = u / kTeamUnits;
+                        for (int h = 0; h < 2; h++) {
+                            const int use = j * K::kUse + (u % kTeamUnits) * 2 + h, sl = team * K::kSlots + use % K::kSlots;
+                            if (!(ok = wait_bar(bar(K::B_AFULL + sl), (uint32_t)(use / K::kSlots) & 1u, dead))) break;
+                            tc_fence_after();
+                            const uint32_t ta = tmem + K::kColA + (uint32_t)(sl * 32);
 #pragma unroll
-                            for (int h = 0; h < 2; h++) {
-                                const int use = j * K::kUse + (u % kTeamUnits) * 2 + h, sl = team * K::kSlots + use % K::kSlots;
-                                if (pass == 0) {
-                                    if (!(ok = wait_bar(bar(K::B_AFULL + sl), (uint32_t)(use / K::kSlots) & 1u, dead))) break;
-                                    tc_fence_after();
-                                }
-                                const uint32_t ta = tmem + K::kColA + (uint32_t)(sl * 32);
-#pragma unroll
-                                for (int k = 0; k < 4; k++) {
-                                    // Q6_K: the sl and the sh operands of a slot meet the same 32 activations
-                                    const int pl = FMT == F_Q6 ? h * 4 + (k & 1) * 2 : h * 8 + k * 2;
-                                    const uint32_t dst = td + (uint32_t)((K::kAcc == 2 ? (k >> 1) * TN : 0) + pass * (TN / K::kPass));
-                                    const uint32_t keep = (uint32_t)(uu > 0 || h > 0 || (K::kAcc == 2 ? (k & 1) : k > 0));
-                                    mma_ta(dst, ta + (uint32_t)(k * 8), bd + (uint64_t)(pl * TN), idesc, keep);
-                                }
-                                if (pass == K::kPass - 1) mma_commit(bar(K::B_AFREE + sl));
+                            for (int k = 0; k < 4; k++) {
+                                // Q6_K: the sl and the sh operands of a slot meet the same 32 activations
+                                const int pl = FMT == F_Q6 ? h * 4 + (k & 1) * 2 : h * 8 + k * 2;
+                                const uint32_t keep = (uint32_t)(uu > 0 || h > 0 || (K::kAcc == 2 ? (k & 1) : k > 0));
+                                mma_ta(td + (uint32_t)(K::kAcc == 2 ? (k >> 1) * TN : 0), ta + (uint32_t)(k * 8), bd + (uint64_t)(pl * TN), idesc, keep);
                             }
-                            if (!ok) break;
-                            if (pass == K::kPass - 1) mma_commit(bar(K::B_BFREE + q + u));
+                            mma_commit(bar(K::B_AFREE + sl));
                         }
                         if (!ok) break;
-                        if (pass < K::kPass - 1) {
-                            if (!(ok = wait_bar(bar(K::B_HEAD + s), jp, dead))) break;
-                            mma_commit(bar(K::B_ACCRDY + pass));
-                        }
+                        mma_commit(bar(K::B_BFREE + q + u));
                     }
                     q += K::kUnits;
                     if (q == K::kNB) q = 0, qp ^= 1;
@@ -685,7 +670,7 @@ __global__ void __launch_bounds__(Cfg<FMT, TN>::kWarps * 32, Cfg<FMT, TN>::kCtas
                         tc_fence_after();
                         mma_sa(tmem + K::kColM + (uint32_t)(K::kMBuf == 2 ? s * TN : 0), mk_desc(su32(amin + s * 4 * kTM * 16), kTM * 16), xd, idesc, 0u);
                     }
-                    mma_commit(bar(K::B_ACCRDY + (K::kPass == 1 ? s : 1)));
+                    mma_commit(bar(K::B_ACCRDY + sa));
                 }
             }
             if (!ok) fail(6u);
@@ -719,12 +704,12 @@ __global__ void __launch_bounds__(Cfg<FMT, TN>::kWarps * 32, Cfg<FMT, TN>::kCtas
                 }
                 __syncwarp();
                 if (lane == 0) bar_arrive(bar(K::B_SFREE + ls));
-                // The job before last (two passes: the last job, whose barrier is the next to complete) has been multiplied, so its
+                // The job before last (one accumulator: the last job, whose barrier is the next to complete) has been multiplied, so its
                 // operands are read, and the jobs before it are folded: the rings' places are free.
-                if (K::kPass == 1) {
+                if (K::kJobBuf == 2) {
                     if (js >= 2 && !(ok = wait_warp(bar(K::B_ACCRDY + s), (uint32_t)(((js >> 1) - 1) & 1), dead))) break;
                 } else {
-                    if (js >= 1 && !(ok = wait_warp(bar(K::B_ACCRDY + 1), (uint32_t)((js - 1) & 1), dead))) break;
+                    if (js >= 1 && !(ok = wait_warp(bar(K::B_ACCRDY), (uint32_t)((js - 1) & 1), dead))) break;
                 }
 #pragma unroll
                 for (int k = 0; k < 4; k++) {
@@ -831,10 +816,9 @@ __global__ void __launch_bounds__(Cfg<FMT, TN>::kWarps * 32, Cfg<FMT, TN>::kCtas
             for (int k = 0; k < K::kCols / 2; k++) acc[k] = 0ull;
 #pragma unroll 1
             for (int b = t.b0; b < t.b1; b++, j++) {
-                // its accumulators: those of the job's parity, or of its half of the tokens
-                const int x = j % K::kNX, s = K::kPass == 1 ? j & 1 : col0 / (TN / 2), sa = K::kPass == 1 ? s : 0;
+                const int x = j % K::kNX, s = K::kJobBuf == 2 ? j & 1 : 0;
                 if (!(ok = wait_warp(bar(K::B_XFULL + x), (uint32_t)((j / K::kNX) & 1), dead) &&
-                           wait_warp(bar(K::B_ACCRDY + s), (uint32_t)((K::kPass == 1 ? j >> 1 : j) & 1), dead)))
+                           wait_warp(bar(K::B_ACCRDY + s), (uint32_t)((K::kJobBuf == 2 ? j >> 1 : j) & 1), dead)))
                     break;
                 tc_fence_after();
                 const float *d8 = reinterpret_cast<const float *>(ext0 + x * K::kExtra + (FMT == F_Q4 ? 32 * TN : 0)) + col0;
@@ -843,9 +827,9 @@ __global__ void __launch_bounds__(Cfg<FMT, TN>::kWarps * 32, Cfg<FMT, TN>::kCtas
 #pragma unroll
                 for (int c = 0; c < K::kCols; c += K::kChunk) {
                     uint32_t sd[K::kChunk], sm[K::kChunk];
-                    tld(tlane + (uint32_t)(sa * K::kAcc * TN + c), sd);
+                    tld(tlane + (uint32_t)(s * K::kAcc * TN + c), sd);
                     if (FMT == F_Q4) tld(tlane + K::kColM + (uint32_t)((K::kMBuf == 2 ? s * TN : 0) + c), sm);
-                    if (K::kAcc == 2) tld(tlane + (uint32_t)(sa * K::kAcc * TN + TN + c), sm);
+                    if (K::kAcc == 2) tld(tlane + (uint32_t)(s * K::kAcc * TN + TN + c), sm);
                     tld_wait();
 #pragma unroll
                     for (int k4 = 0; k4 < K::kChunk / 4; k4++) {
