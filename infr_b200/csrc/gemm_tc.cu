@@ -67,6 +67,9 @@ struct Cfg {
     // every operand slot until the second pass: 14336 -> 4096, 113 rows 50.6 us, in one pass 46.9;
     // 1000 rows 296, 254.)
     static constexpr int kJobBuf = FMT == F_Q6 && TN == 128 ? 1 : 2;
+    // Tensor memory that only one job has (Q4_K: the minima's sums) goes back as early as can be: Q4_K 4096 -> 14336, 113 rows 31.3 -> 30.9 us, 512
+    // rows 84.1 -> 82.6.  With two jobs' worth the fold is off the path: at 64 rows it cost 2 %.
+    static constexpr bool kEarly = TN == 128;
     static constexpr int kRowBytes = FMT == F_Q6 ? 240 : 144;
     static constexpr int kRaw = kTM * kRowBytes;
     static constexpr int kUnitBytes = (FMT == F_Q4 ? 256 : 128) * TN;
@@ -824,6 +827,14 @@ __global__ void __launch_bounds__(Cfg<FMT, TN>::kWarps * 32, Cfg<FMT, TN>::kCtas
                 const float *d8 = reinterpret_cast<const float *>(ext0 + x * K::kExtra + (FMT == F_Q4 ? 32 * TN : 0)) + col0;
                 const uint32_t hd = dring[(j % K::kRing) * kTM + row];
                 const u64 dw = f2_dup(h2f(hd)), nm = f2_dup(FMT == F_Q4 ? -h2f(hd >> 16) : 16.f);
+                auto give_back = [&]() {
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) {
+                        if (K::kMBuf == 1) bar_arrive(bar(K::B_MFREE));  // before ACCFREE: an issuer that saw that one is one phase behind at most
+                        bar_arrive(bar(K::B_ACCFREE + s));
+                    }
+                };
 #pragma unroll
                 for (int c = 0; c < K::kCols; c += K::kChunk) {
                     uint32_t sd[K::kChunk], sm[K::kChunk];
@@ -831,6 +842,8 @@ __global__ void __launch_bounds__(Cfg<FMT, TN>::kWarps * 32, Cfg<FMT, TN>::kCtas
                     if (FMT == F_Q4) tld(tlane + K::kColM + (uint32_t)((K::kMBuf == 2 ? s * TN : 0) + c), sm);
                     if (K::kAcc == 2) tld(tlane + (uint32_t)(s * K::kAcc * TN + TN + c), sm);
                     tld_wait();
+                    // all of the job is in registers: its accumulators go back before the last chunk is folded
+                    if (K::kEarly && c + K::kChunk == K::kCols) give_back();
 #pragma unroll
                     for (int k4 = 0; k4 < K::kChunk / 4; k4++) {
                         const ulonglong2 dv = *reinterpret_cast<const ulonglong2 *>(d8 + c + 4 * k4);
@@ -845,13 +858,9 @@ __global__ void __launch_bounds__(Cfg<FMT, TN>::kWarps * 32, Cfg<FMT, TN>::kCtas
                         }
                     }
                 }
-                tc_fence_before();
+                if (!K::kEarly) give_back();
                 __syncwarp();
-                if (lane == 0) {
-                    if (K::kMBuf == 1) bar_arrive(bar(K::B_MFREE));  // before ACCFREE: an issuer that saw that one is one phase behind at most
-                    bar_arrive(bar(K::B_ACCFREE + s));
-                    bar_arrive(bar(K::B_XFREE + x));
-                }
+                if (lane == 0) bar_arrive(bar(K::B_XFREE + x));
             }
             if (!ok) break;
             auto val = [&](int k) { return __uint_as_float((uint32_t)(acc[k / 2] >> (32 * (k & 1)))); };
