@@ -864,7 +864,8 @@ Status CudaBackend::moe_ffn(const MoeArgs &a) {
     // Experts that see a few dozen rows each run on the tensor-memory GEMM in grouped form (one slab of 32 or 64 of an expert's
     // rows per token tile: the expert's weights are unpacked once per slab); with only a handful of rows per expert the 8-row
     // grouped GEMV does less padded work.  An expert's load is that of the whole layer, also on a rank that holds some experts.
-    // Measured, us a layer (items / slabs of 32 / of 64), by pairs per expert:
+    // Measured, us a layer (items / slabs of 32 / of 64), by pairs per expert; taken when gate and up, and SwiGLU and layout, were launches of their
+    // own (since then both sides gained: 128 experts, 9 pairs, items 224 -> 183; 16 pairs, slabs 236 -> 221; 16 experts of 4096 -> 256, 32 pairs, 97 -> 75):
     //   128 experts, 2048 -> 768   8: 232 / 259 / 296, 12: 266 / 259 / 296, 24: 388 / 292 / 323, 32: 500 / 365 / 337
     //   32 experts, 4096 -> 1792   8: 243 / 274 / 293, 16: 424 / 268 / 300, 32: 444 / 350 / 314, 64: 841 / 524 / 415
     //   60 experts, 2048 -> 1536   26: 348 / 243 / 254, 34: 447 / 313 / 266
@@ -940,19 +941,13 @@ Status CudaBackend::moe_ffn(const MoeArgs &a) {
     if (grouped_gemm) {
         // stage B: both banks read the same gathered activation planes (laid out once); stage C; stage D on the
         // re-quantised pairs; stage E
-        auto layout = [&](const Q8Dev &acts, uint8_t *rec, uint32_t k, const int32_t *rows_of) {
-            return launch_gemm_tc_grouped_prep(slab, acts, rec, (int)k, ie, ip, ic, ni, rows_of, (int)max_slabs, stream_);
+        auto gemm = [&](const uint8_t *bank, const uint8_t *bank2, const uint8_t *rec, float *out, float *out2, uint32_t k, uint32_t o) {
+            return launch_gemm_tc_grouped(slab, bank, bank2, (int)a.n_local, rec, out, out2, (int)k, (int)o, ie, ip, ic, ni, (int)max_slabs, dev_, status_dev_, stream_);
         };
-        auto gemm = [&](const uint8_t *bank, const uint8_t *rec, float *out, uint32_t k, uint32_t o) {
-            return launch_gemm_tc_grouped(slab, bank, (int)a.n_local, rec, out, (int)k, (int)o, ie, ip, ic, ni, (int)max_slabs, dev_, status_dev_, stream_);
-        };
-        INFR_STEP(layout(xa, b + o_px, (uint32_t)ne, prow), "moe layout x");
-        INFR_STEP(gemm(a.gate, b + o_px, g, (uint32_t)ne, (uint32_t)nff), "moe gate (grouped gemm)");
-        INFR_STEP(gemm(a.up, b + o_px, u, (uint32_t)ne, (uint32_t)nff), "moe up (grouped gemm)");
-        INFR_STEP(launch_moe_swiglu_quant(g, u, (int)n_pairs, (int)nff, aq, ad, as, nullptr, nullptr, stream_), "moe swiglu");
-        Q8Dev aa{aq, ad, as, nullptr, 256};
-        INFR_STEP(layout(aa, b + o_pa, (uint32_t)nff, nullptr), "moe layout act");
-        INFR_STEP(gemm(a.down, b + o_pa, y, (uint32_t)nff, (uint32_t)ne), "moe down (grouped gemm)");
+        INFR_STEP(launch_gemm_tc_grouped_prep(slab, xa, b + o_px, (int)ne, ie, ip, ic, ni, prow, (int)max_slabs, stream_), "moe layout x");
+        INFR_STEP(gemm(a.gate, a.up, b + o_px, g, u, (uint32_t)ne, (uint32_t)nff), "moe gate, up (grouped gemm)");
+        INFR_STEP(launch_gemm_tc_grouped_silu_prep(slab, g, u, b + o_pa, (int)nff, ie, ip, ic, ni, (int)max_slabs, stream_), "moe swiglu, layout");
+        INFR_STEP(gemm(a.down, nullptr, b + o_pa, y, nullptr, (uint32_t)nff, (uint32_t)ne), "moe down (grouped gemm)");
         INFR_STEP(launch_moe_combine(y, pslot, w, (int)rows, (int)nu, (int)ne, a.dst, stream_), "moe combine");
         return Status::Ok();
     }

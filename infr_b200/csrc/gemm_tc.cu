@@ -447,26 +447,33 @@ __global__ void __launch_bounds__(1024) gemm_tc_norm_prep_kernel(const float *a,
     });
 }
 
-// silu(gate) * up and the layout in one launch: a warp per (token slot, block); the rows also go to dst (which may be gate or up).
+// silu(gate) * up and the layout in one launch: a warp per (token slot, block); the rows also go to dst (null: nowhere; it may be gate or up).
+// Grouped: a slot's row is its routed pair.
 template <int FMT>
 __global__ void __launch_bounds__(256) gemm_tc_silu_prep_kernel(const float *gate, const float *up, float *dst, int m, int tn, int in_f, uint8_t *__restrict__ units,
-                                                                uint8_t *__restrict__ extra, int n_tok) {
+                                                                uint8_t *__restrict__ extra, int n_tok, TcGroup grp) {
     pdl_go();
     pdl_wait();
     const int lane = threadIdx.x & 31, nb = in_f >> 8;
     const long long wg = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (wg >= (long long)n_tok * nb) return;
     const int T = (int)(wg / nb), b = (int)(wg % nb);
+    long long row = T < m ? T : -1;
+    if (grp.slab_expert) {
+        const int tt = T / tn, t = T - tt * tn;
+        if (tt >= *grp.n_slabs) return;
+        row = t < grp.slab_cnt[tt] ? grp.slab_p0[tt] + t : -1;
+    }
     float4 v[2] = {make_float4(0.f, 0.f, 0.f, 0.f), make_float4(0.f, 0.f, 0.f, 0.f)};
-    if (T < m) {
-        const size_t e = (size_t)T * in_f + (size_t)b * 256 + lane * 4;
+    if (row >= 0) {
+        const size_t e = (size_t)row * in_f + (size_t)b * 256 + lane * 4;
         float4 g[2], u[2];
 #pragma unroll
         for (int h = 0; h < 2; h++) g[h] = *reinterpret_cast<const float4 *>(gate + e + h * 128), u[h] = *reinterpret_cast<const float4 *>(up + e + h * 128);
 #pragma unroll
         for (int h = 0; h < 2; h++) {
             v[h] = make_float4(silu_mul(g[h].x, u[h].x), silu_mul(g[h].y, u[h].y), silu_mul(g[h].z, u[h].z), silu_mul(g[h].w, u[h].w));
-            *reinterpret_cast<float4 *>(dst + e + h * 128) = v[h];
+            if (dst) *reinterpret_cast<float4 *>(dst + e + h * 128) = v[h];
         }
     }
     store_operand<FMT>(v, T, b, nb, tn, units, extra);
@@ -1060,7 +1067,7 @@ cudaError_t launch_gemm_tc_prep(int dtype, const RowSource &src, void *records, 
     uint8_t *u = static_cast<uint8_t *>(records), *e = u + units_bytes(n, in_f);
     if (!src.norm_w) {
         auto kernel = f == F_Q4 ? gemm_tc_silu_prep_kernel<F_Q4> : gemm_tc_silu_prep_kernel<F_Q6>;
-        return launch_pdl(kernel, dim3((unsigned)(((size_t)n * nb + 7) / 8)), dim3(256), 0, st, src.a, src.b, src.dst, m, tn, in_f, u, e, n);
+        return launch_pdl(kernel, dim3((unsigned)(((size_t)n * nb + 7) / 8)), dim3(256), 0, st, src.a, src.b, src.dst, m, tn, in_f, u, e, n, TcGroup{});
     }
     const int threads = nb > 32 ? 1024 : nb * 32;
     auto kernel = f == F_Q4 ? (src.b ? gemm_tc_norm_prep_kernel<F_Q4, true> : gemm_tc_norm_prep_kernel<F_Q4, false>)
@@ -1102,18 +1109,27 @@ cudaError_t launch_gemm_tc_grouped_prep(int slab, const Q8Dev &a, void *records,
     uint8_t *u = static_cast<uint8_t *>(records), *e = u + units_bytes(n, in_f);
     return launch_prep<false>(F_Q4, nullptr, a, n, slab, in_f, u, e, n, TcGroup{slab_expert, slab_p0, slab_cnt, n_slabs, pair_row}, st);
 }
-cudaError_t launch_gemm_tc_grouped(int slab, const uint8_t *bank, int n_experts, const void *records, float *y, int in_f, int out_f,
+cudaError_t launch_gemm_tc_grouped_silu_prep(int slab, const float *gate, const float *up, void *records, int in_f, const int *slab_expert, const int *slab_p0,
+                                             const int *slab_cnt, const int *n_slabs, int max_slabs, cudaStream_t st) {
+    if (!gemm_tc_takes(DT_Q4K, in_f) || max_slabs < 1) return cudaErrorInvalidValue;
+    const int n = max_slabs * slab;
+    uint8_t *u = static_cast<uint8_t *>(records), *e = u + units_bytes(n, in_f);
+    return launch_pdl(gemm_tc_silu_prep_kernel<F_Q4>, dim3((unsigned)(((size_t)n * (in_f / 256) + 7) / 8)), dim3(256), 0, st, gate, up, (float *)nullptr, n, slab, in_f, u, e, n,
+                      TcGroup{slab_expert, slab_p0, slab_cnt, n_slabs, nullptr});
+}
+cudaError_t launch_gemm_tc_grouped(int slab, const uint8_t *bank, const uint8_t *bank2, int n_experts, const void *records, float *y, float *y2, int in_f, int out_f,
                                    const int *slab_expert, const int *slab_p0, const int *slab_cnt, const int *n_slabs, int max_slabs,
                                    const DeviceInfo &dev, uint32_t *status, cudaStream_t st) {
     if (!gemm_tc_takes(DT_Q4K, in_f) || out_f < 1 || max_slabs < 1 || n_experts < 1 || (slab != 32 && slab != 64)) return cudaErrorInvalidValue;
     const int n = max_slabs * slab;
     const uint8_t *u = static_cast<const uint8_t *>(records), *e = u + units_bytes(n, in_f);
-    CUtensorMap mw;
-    if (!weight_map(F_Q4, bank, (size_t)n_experts * out_f, in_f, &mw)) return cudaErrorInvalidValue;
+    CUtensorMap mw, mw2;
+    if (!weight_map(F_Q4, bank, (size_t)n_experts * out_f, in_f, &mw) || !weight_map(F_Q4, bank2 ? bank2 : bank, (size_t)n_experts * out_f, in_f, &mw2))
+        return cudaErrorInvalidValue;
     TcGroup g{slab_expert, slab_p0, slab_cnt, n_slabs, nullptr};
-    TcMat m1{y, out_f}, m2{nullptr, 0};
-    const int tiles = ((out_f + kTM - 1) / kTM) * max_slabs, cap = ctas_of(F_Q4, slab, dev), grid = tiles < cap ? tiles : cap;
-    return launch_tn<F_Q4>(slab, mw, mw, u, e, m1, m2, n, in_f, status, g, TcSplit{1 << 30, 1, nullptr}, grid, st);
+    TcMat m1{y, out_f}, m2{y2, bank2 ? out_f : 0};
+    const int tiles = ((out_f + kTM - 1) / kTM) * (bank2 ? 2 : 1) * max_slabs, cap = ctas_of(F_Q4, slab, dev), grid = tiles < cap ? tiles : cap;
+    return launch_tn<F_Q4>(slab, mw, mw2, u, e, m1, m2, n, in_f, status, g, TcSplit{1 << 30, 1, nullptr}, grid, st);
 }
 
 }  // namespace infr

@@ -162,7 +162,11 @@ cudaError_t launch_gemm_q2(const uint8_t *w, const void *records, float *c, floa
 size_t gemm_tc_grouped_record_bytes(int slab, int max_slabs, int in_f);
 cudaError_t launch_gemm_tc_grouped_prep(int slab, const Q8Dev &a, void *records, int in_f, const int *slab_expert, const int *slab_p0,
                                         const int *slab_cnt, const int *n_slabs, const int *pair_row, int max_slabs, cudaStream_t st);
-cudaError_t launch_gemm_tc_grouped(int slab, const uint8_t *bank, int n_experts, const void *records, float *y, int in_f, int out_f,
+// The layout of silu(gate) * up, rows = pairs.
+cudaError_t launch_gemm_tc_grouped_silu_prep(int slab, const float *gate, const float *up, void *records, int in_f, const int *slab_expert, const int *slab_p0,
+                                             const int *slab_cnt, const int *n_slabs, int max_slabs, cudaStream_t st);
+// bank2 / y2: a second bank of that shape against the same rows in the same launch (gate and up), or null.
+cudaError_t launch_gemm_tc_grouped(int slab, const uint8_t *bank, const uint8_t *bank2, int n_experts, const void *records, float *y, float *y2, int in_f, int out_f,
                                    const int *slab_expert, const int *slab_p0, const int *slab_cnt, const int *n_slabs, int max_slabs,
                                    const DeviceInfo &dev, uint32_t *status, cudaStream_t st);
 // Grouped Q4_K GEMM over a bank of n_experts matrices [out_f, in_f] stored back to back: work item i
