@@ -1238,15 +1238,17 @@ cudaError_t launch_attention(const float *q, const void *k_cache, const void *v_
     // more than two waves of CTAs (three fit an SM): the per-tile instruction count decides, else the first byte's latency
     const bool bulk = (size_t)n_splits * n_kv * q_rows > (size_t)6 * (sm_count > 0 ? sm_count : 148);
     const int g = n_head / n_kv;
-    // Rows of a prompt chunk share a tile where that fills it (more than three rows of it, or 7/8 of its 16 (row, head) pairs)
-    // and leaves enough CTAs: a shared tile takes longer, above all at the causal edge, which is multiplied row by row.  Measured,
-    // a tile per row / shared (us, attention and merge): 32 heads / 8: 113 rows at 384 60 / 49, 33 rows at 100 14 / 18 (144 CTAs),
-    // 2 rows of 16 sequences at 1500 (half a tile) 52 / 61; 8 / 8: 64 rows at 0 13 / 28 (32 CTAs), at 1500 75 / 34 (416), 2 rows of
-    // 16 sequences at 4000 (an eighth) 105 / 126; 32 / 32: 16 rows at 100 14 / 28 (64); 32 / 4: 3 rows of 4 at 1500 (3/4) 22 / 24.
+    // Rows of a prompt chunk share a tile where a tile per row takes more than about a wave of CTAs (three fit an SM; two of the shared form, which
+    // take 1 us longer) and the shared tile has more than two rows, is nearly full or leaves a single wave.  live: the tiles with keys, each
+    // row for itself.  Measured, a tile per row / shared (us, attention and merge), 240 shapes; the rule takes the slower side in none by more than 1 us:
+    // 32 heads / 8: 113 rows at 384 40 / 28, 33 at 100 9 / 11 (live 304), 2 at 4000 12.8 / 11.6, 8 at 1500 14.0 / 11.1;  8 / 8: 33 at 0 8.1 / 9.3,
+    // 64 at 384 24 / 10;  32 / 32: 64 at 0 23 / 10, 2 at 1500 13.3 / 15.5 (384 shared CTAs);  2 rows of 16 sequences at 1500: 8 / 8 37 / 42, 32 / 4 28 / 24.
     const int rpt = kAttnChunkPairs / (g < 1 ? 1 : g), row_blocks = rpt ? (rows + rpt - 1) / rpt : 0;  // rows of a tile
     const size_t sms = (size_t)(sm_count > 0 ? sm_count : 148);
-    const bool chunk = head_dim == 128 && rows > 1 && (g == 1 || g == 2 || g == 4 || g == 8) && (rows > 3 * row_blocks || 8 * rows >= 7 * rpt * row_blocks) &&
-                       2 * (size_t)n_splits * n_kv * n_seq * row_blocks >= 3 * sms && (size_t)n_splits * n_kv * q_rows > 3 * sms;
+    auto tiles_to = [](size_t n) { return n / kAttnTile * (n / kAttnTile + 1) / 2 * kAttnTile + n % kAttnTile * (n / kAttnTile + 1); };  // of rows with 1..n keys
+    const size_t live = (tiles_to(max_keys) - tiles_to(pos)) * n_kv * n_seq, shared = (size_t)n_splits * n_kv * n_seq * row_blocks;
+    const bool chunk = head_dim == 128 && rows > 1 && (g == 1 || g == 2 || g == 4 || g == 8) && 2 * live > 5 * sms &&
+                       (rows > 2 * row_blocks || 8 * rows >= 7 * rpt * row_blocks || shared <= 2 * sms);
 #define INFR_CHUNK(G_) launch_attn_chunk<G_>(st, q, kc, vc, po, pml, n_seq, rows, n_head, n_kv, pos, scale, n_splits, seq_stride, status, seq_pos, block_table, table_stride, n_pages)
     if (chunk)
         e = g == 1 ? INFR_CHUNK(1) : g == 2 ? INFR_CHUNK(2) : g == 4 ? INFR_CHUNK(4) : INFR_CHUNK(8);
