@@ -864,18 +864,19 @@ Status CudaBackend::moe_ffn(const MoeArgs &a) {
     // Experts that see a few dozen rows each run on the tensor-memory GEMM in grouped form (one slab of 32 or 64 of an expert's
     // rows per token tile: the expert's weights are unpacked once per slab); with only a handful of rows per expert the 8-row
     // grouped GEMV does less padded work.  An expert's load is that of the whole layer, also on a rank that holds some experts.
-    // Measured, us a layer (items / slabs of 32 / of 64), by pairs per expert; taken when gate and up, and SwiGLU and layout, were launches of their
-    // own (since then both sides gained: 128 experts, 9 pairs, items 224 -> 183; 16 pairs, slabs 236 -> 221; 16 experts of 4096 -> 256, 32 pairs, 97 -> 75):
-    //   128 experts, 2048 -> 768   8: 232 / 259 / 296, 12: 266 / 259 / 296, 24: 388 / 292 / 323, 32: 500 / 365 / 337
-    //   32 experts, 4096 -> 1792   8: 243 / 274 / 293, 16: 424 / 268 / 300, 32: 444 / 350 / 314, 64: 841 / 524 / 415
-    //   60 experts, 2048 -> 1536   26: 348 / 243 / 254, 34: 447 / 313 / 266
-    // Where a slab per expert is at most a wave of tiles, so that a tile has an SM to itself either way, 64 rows cost no more:
-    //   8 experts, 4096 -> 2048    8: 242 / 147 / 130, 32: 268 / 169 / 136, 128: 494 / 292 / 260
-    //   16 experts, 2048 -> 1024   8: 117 / 90 / 83, 32: 129 / 110 / 89;  1024 -> 256   8: 51 / 57 / 52, 16: 59 / 59 / 53
+    // Measured, us a layer (items / slabs of 32 / of 64), by pairs per expert:
+    //   128 experts, 2048 -> 768   9: 181 / 214 / 245, 13: 211 / 219 / 253, 16: 258 / 224 / 257, 28: 390 / 286 / 281, 40: 503 / 395 / 306
+    //   60 experts, 2048 -> 1536   11: 164 / 189 / 202, 13: 186 / 190 / 204, 16: 194 / 190 / 207, 28: 328 / 230 / 223
+    //   32 experts, 1024 -> 1024   13: 70 / 73 / 78, 16: 81 / 74 / 78, 28: 102 / 77 / 82, 32: 103 / 92 / 81
+    //   16 experts, 2048 -> 1024   9: 62 / 75 / 79, 13: 68 / 76 / 79, 16: 73 / 77 / 80, 24: 86 / 77 / 81, 28: 96 / 90 / 82
+    //   8 experts, 4096 -> 2048    9: 75 / 90 / 97, 13: 90 / 93 / 98, 16: 96 / 92 / 98, 24: 136 / 108 / 115, 28: 153 / 125 / 115
+    //   64 experts, 1024 -> 256    9: 62 / 62 / 67, 13: 64 / 63 / 69, 16: 80 / 65 / 70, 28: 91 / 74 / 76
+    // and with more weights than those, where the GEMM's launches count less:
+    //   32 experts, 4096 -> 1792   7: 147 / 194 / 221, 9: 206 / 215 / 242, 11: 235 / 211 / 241, 24: 341 / 222 / 251, 32: 411 / 284 / 257
     // (a layer with a Q6_K bank takes 8-row items throughout: the GEMM's copies want rows of whole 2048-element chunks)
-    const bool one_wave = (size_t)a.n_local * ((nff + 127) / 128) <= (size_t)dev_.sm_count;
-    const bool grouped_gemm = !any_q6 && (mmq_impl_ == 2 || (mmq_impl_ == 0 && 2 * n_pairs >= (size_t)(one_wave ? 16 : 21) * nx));
-    const int slab = one_wave || n_pairs >= 28 * nx ? 64 : 32;
+    const bool large = a.n_local * ne * nff >= ((size_t)212 << 20);
+    const bool grouped_gemm = !any_q6 && (mmq_impl_ == 2 || (mmq_impl_ == 0 && 2 * n_pairs >= (size_t)(large ? 21 : 28) * nx));
+    const int slab = n_pairs >= 28 * nx ? 64 : 32;
     const size_t max_slabs = n_pairs / slab + a.n_local + 1;
     // scratch carve-up (all 256-byte aligned)
     size_t off = 0;

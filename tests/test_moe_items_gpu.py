@@ -1,5 +1,6 @@
 """Expert banks as 8-row items at the edges of their launch: few items (many CTAs each), more items than the device holds at once,
-one K block, rows so long that a CTA holds one group of warps only.
+one K block, rows so long that a CTA holds one group of warps only; and the rows per expert at which slabs of the tensor-memory GEMM
+take over.
 
 The integer products are exact, so a result differs from the CPU path's by the order of f32 additions alone: 1e-3 relative L2, as for
 the other expert-bank tests."""
@@ -20,6 +21,11 @@ pytestmark = pytest.mark.gpu
     (2, 256, 2, 2, 256, infr_b200.Q6K),      # one K block, one tile for some groups of warps and none for others
     (9, 512, 8, 8, 1280, infr_b200.Q6K),     # every row on every expert: items of eight rows and of one
     (40, 256, 200, 6, 256, Q4K),             # more items than SMs
+    (27, 512, 4, 2, 512, Q4K),               # 13.5 pairs an expert: items of every size
+    (28, 512, 4, 2, 512, Q4K),               # 14: slabs of 32 rows
+    (55, 512, 4, 2, 512, Q4K),               # 27.5: the last of them
+    (56, 512, 4, 2, 512, Q4K),               # 28: slabs of 64 rows
+    (150, 256, 3, 2, 1280, Q4K),             # 100: two of them
     (2, 14336, 2, 1, 256, Q4K),              # 56 blocks a row: no room for two groups' rings
 ])
 def test_items_at_the_edges(backend, oracle, rows, ne, n_expert, n_used, nff, down_dt):
