@@ -1028,7 +1028,7 @@ def run_b200(args):
                      # dram__bytes_read.sum + dram__bytes_write.sum of this kernel at this shape from the committed
                      # ncu capture (profiles/gemv_q4k_mma_4096x4096_m1.md): 9 467 136 + 0 bytes per launch
                      "traffic": 9467136, "peak_source": f"{peak_src} HBM copy bandwidth",
-                     "kernel": "gemv_q4k_mma_kernel (m=1, pre-quantised activations)", "kernel_us": ms_kern * 1e3 / (steps * ROT),
+                     "kernel": "gemv_row_kernel (m=1, pre-quantised activations)", "kernel_us": ms_kern * 1e3 / (steps * ROT),
                      "alg_bytes_per_launch": C1_BYTES},
         "e2e": {"value": total_bytes * e2e_steps / e2e_s / 1e9, "unit": "GB/s",
                 "h2d_bytes_per_step": ROT * IN_F * 4, "d2h_bytes_per_step": ROT * OUT_F * 4,
