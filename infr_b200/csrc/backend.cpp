@@ -834,7 +834,8 @@ static double expected_items(double p, int rows) {
     double below = 0, sum = 0;
     for (int c = 0; c <= rows; c++) {  // P(c rows) from P(c - 1 rows)
         below += pmf;
-        if (c % 8 == 0) sum += below < 1.0 ? 1.0 - below : 0.0;
+        if (1.0 - below < 1e-9) break;
+        if (c % 8 == 0) sum += 1.0 - below;
         pmf *= p / (1.0 - p) * (rows - c) / (c + 1);
     }
     return sum;
