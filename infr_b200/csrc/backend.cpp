@@ -342,9 +342,9 @@ Status CudaBackend::linear(int dtype, const uint8_t *w, const float *x, float *y
     // Kernels that read the f32 rows in every CTA need a result apart from them: in place the rows are quantised first.
     const bool in_place = overlap(x, (size_t)m * in_f, y, (size_t)m * out_f);
     // One Q2_0 row: quantised inside the GEMV, unless it is so long that every CTA's own quantising costs more than a launch.  Quantiser and
-    // GEMV / one launch (us, cold weights): 4096 -> 4096 6.9 / 5.8, 4096 -> 128256 57 / 56, 14336 -> 4096 11.2 / 10.9, 14336 -> 32768
-    // 43.3 / 42.7, 20480 -> 4096 14.3 / 15.0, 28672 -> 8192 27.0 / 29.1, 65536 -> 256 18.7 / 20.6.  (A pair saves two launches: always.)
-    if (dtype == DT_Q2_0 && m == 1 && in_f <= 16384 && act == INFR_ACT_INT8 && gemv_impl_ == 0 && !in_place) {
+    // GEMV / one launch (us, cold weights): 8192 -> 8192 8.5 / 9.2, 14336 -> 4096 9.6 / 9.5, -> 8192 12.6 / 14.6, 16384 -> 4096 10.2 / 9.8,
+    // 20480 -> 4096 13.0 / 12.6, 53248 -> 4096 24 / 32, 65536 -> 2048 19 / 21.  (A pair saves two launches: always.)
+    if (dtype == DT_Q2_0 && m == 1 && (in_f <= 4096 || (in_f <= 28672 && out_f <= 32u * (uint32_t)dev_.sm_count)) && act == INFR_ACT_INT8 && gemv_impl_ == 0 && !in_place) {
         const cudaError_t e = launch_gemv_q2_row(w, y, (int)out_f, nullptr, nullptr, 0, x, (int)in_f, dev_, status_dev_, stream_);
         if (e == cudaSuccess) launches_++;
         if (e != cudaErrorInvalidValue) return cuda_status(e, "gemv_q2");

@@ -15,13 +15,13 @@
 // 4096 -> 128256 takes 55 us with three slots and 68 with four instead of 49 with two.)
 // Q4_K and Q6_K: every block's term meets the others in shared memory, a few tiles at a time, and the terms of a row are added in the order
 // that row_group says: that of the kernels for two rows and more, had they one.  (A sum in another order differs in a last bit here and
-// there, and 32 layers that code their activations in 8 bits carry that on to 0.01 .. 0.03 of a model's result.)  Q2_0: the warps' sums meet,
-// in a fixed order.
+// there, and 32 layers that code their activations in 8 bits carry that on to 0.01 .. 0.03 of a model's result.)  Q2_0: chains of blocks in the
+// order of the byte-dot kernel, for the same reason (kQ2Chains).
 // All waits are bounded; an expired one records a status word for the host.
 // Measured (us a call in a chain of calls on cold weights; before = the columns-are-rows kernels, or the byte-dot kernel for Q2_0; codes / f32
 // rows): Q4_K 4096 -> 4096 3.5 / 4.4 -> 3.6 / 3.9, 4096 -> 14336 7.5 / 9.4 -> 7.8 / 8.0, 14336 -> 4096 8.5 / 11.5 -> 8.0 / 9.9;  Q6_K
-// 4096 -> 4096 5.3 / 6.8 -> 4.5 / 4.5, 4096 -> 14336 13.1 / 15.1 -> 10.1 / 10.1, 4096 -> 128256 79 -> 65;  Q2_0 4096 -> 4096 4.5 / 5.6 -> 3.6 / 4.1,
-// 14336 -> 4096 8.4 / 10.4 -> 6.9 / 8.4, 4096 -> 128256 54 -> 38.  Between other launches (the decode step of an 8B model) the Q4_K shapes gain
+// 4096 -> 4096 5.3 / 6.8 -> 4.5 / 4.5, 4096 -> 14336 13.1 / 15.1 -> 10.1 / 10.1, 4096 -> 128256 79 -> 65;  Q2_0 4096 -> 4096 4.5 / 5.6 -> 3.1 / 4.0,
+// 14336 -> 4096 8.4 / 10.4 -> 7.0 / 9.6, 4096 -> 128256 54 -> 33.  Between other launches (the decode step of an 8B model) the Q4_K shapes gain
 // more: their CTAs leave room for the launch before.  Lost: long Q4_K rows on few tiles, 5632 -> 2048 3.4 -> 3.7.
 // What bounds it: small matrices the chain from one launch to the next (1 us) and one round trip to L2 for the activations (0.3 us);
 // large ones memory (4096 -> 128256 at 0.92 of the measured copy rate, Q6_K 1.0); Q2_0 the integer pipe (64 masks a unit, half rate).
@@ -56,8 +56,22 @@ struct RowFmt<DT_Q6K> {
 };
 template <>
 struct RowFmt<DT_Q2_0> {
-    static constexpr int kUnit = 512, kPitch = 144, kActBytes = 512 + 128, kWarps = 16, kPart = 4, kTerm = 1;
+    static constexpr int kUnit = 512, kPitch = 144, kActBytes = 512 + 128, kWarps = 16, kPart = 1, kTerm = 2;
 };
+// Q2_0: a result is the sum of 32 chains (block b of the row is added to chain b mod 32, in order) along a fixed tree, the order of the byte-dot
+// kernel (gemv_stream.cu), whose bits a model keeps.  A unit's eight blocks belong to eight chains, those of unit u to eight of class u mod 4.
+// Short rows: four warps, each takes the units of a class and its lanes keep the chains; long rows, which four warps are too few for: up to 16,
+// every block's integer sums and scale meet in shared memory and a warp a row adds them.
+constexpr int kQ2ChainWarps = 4;
+constexpr int kQ2Stride = 24, kQ2Chains = 8 * kQ2Stride;  // floats between a tile's chains of one class (16 rows, padded: no bank conflicts)
+constexpr int kQ2Part = 2;                               // tiles whose chains wait for one barrier
+template <int DT>
+constexpr int kRowPad = DT == DT_Q2_0 ? 2 : 4;  // columns between the blocks' terms (Q2_0: writes and reads both two words a bank)
+// how a kernel's warps share a row: chains of Q2_0 (ONE) or not
+template <int DT, bool ONE>
+constexpr bool kChains = DT == DT_Q2_0 && ONE;
+template <int DT, bool ONE>
+constexpr int kRowWarps = kChains<DT, ONE> ? kQ2ChainWarps : RowFmt<DT>::kWarps;
 
 __device__ __forceinline__ uint32_t rs32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ bool row_try(uint32_t bar, uint32_t parity) {
@@ -221,16 +235,17 @@ __device__ __forceinline__ void load_act(RowAct<DT_Q6K> &r, const Q8Dev &a, cons
 // Q2_0: groups of 32 elements with a scale each, always in shared memory: group G's codes at 32 G as words [field f][word i] = elements
 // 16i + f, 16i + 4 + f, 16i + 8 + f, 16i + 12 + f (the order in which a code word yields its fields), then per (half, t) the scales of
 // groups 2t, 2t + 1 of the half and the negated sums of their codes.
+__device__ __forceinline__ void load_q2(float4 (&v)[4], const float *x, int unit, int lane) {
+#pragma unroll
+    for (int k = 0; k < 4; k++) v[k] = *reinterpret_cast<const float4 *>(x + (size_t)unit * 512 + lane * 16 + k * 4);
+}
 template <bool FUSED>
-__device__ __forceinline__ void put_act_q2(uint8_t *p, const Q8Dev &a, const float *x, int unit, int lane) {
+__device__ __forceinline__ void put_act_q2(uint8_t *p, const Q8Dev &a, const float4 (&v)[4], int unit, int lane) {
     uint32_t w[4];
     float d;
     int sum;
     const int grp = lane >> 1, i = lane & 1;
     if (FUSED) {
-        float4 v[4];
-#pragma unroll
-        for (int k = 0; k < 4; k++) v[k] = *reinterpret_cast<const float4 *>(x + (size_t)unit * 512 + lane * 16 + k * 4);
         float am = 0.f;
 #pragma unroll
         for (int k = 0; k < 4; k++) am = fmaxf(am, fmaxf(fmaxf(fabsf(v[k].x), fabsf(v[k].y)), fmaxf(fabsf(v[k].z), fabsf(v[k].w))));
@@ -357,10 +372,10 @@ __device__ __forceinline__ float2 block_q6k(const uint8_t *p0, const uint8_t *p1
 }
 
 // Half a Q2_0 unit (4 blocks of 64): lane t has block t of rows g, g + 8; the sums of its groups 2t, 2t + 1 end up in its own columns.
+// dw: the block's scales in the two rows, s: 64 x the groups' sums.
 // codes: this lane's groups for h = 0, 1 (zeros where another lane's column is meant), sc: scales and negated sums of groups 2t, 2t + 1.
-__device__ __forceinline__ void half_q2(const uint8_t *p0, const uint8_t *p1, uint32_t mis, const uint4 *c0, const uint4 *c1, uint4 sc, float (&acc)[2]) {
+__device__ __forceinline__ void half_q2(const uint8_t *p0, const uint8_t *p1, uint32_t mis, const uint4 *c0, const uint4 *c1, uint4 sc, float (&dw)[2], int (&s)[2][2]) {
     uint32_t c[2][4];
-    float dw[2];
     const uint32_t sh = 16u + 8u * mis;  // 16, or 32 (= take the upper word)
 #pragma unroll
     for (int i = 0; i < 2; i++) {
@@ -383,12 +398,13 @@ __device__ __forceinline__ void half_q2(const uint8_t *p0, const uint8_t *p1, ui
         }
     }
 #pragma unroll
-    for (int i = 0; i < 2; i++) {
-        int s[2];
+    for (int i = 0; i < 2; i++)
 #pragma unroll
-        for (int k = 0; k < 2; k++) s[k] = ((d[0][2 * i + k] * 4 + d[1][2 * i + k]) * 4 + d[2][2 * i + k]) * 4 + d[3][2 * i + k];  // 64 x the group's sum
-        acc[i] += fmaf(dw[i] * 0.015625f * __uint_as_float(sc.y), (float)s[1], dw[i] * 0.015625f * __uint_as_float(sc.x) * (float)s[0]);
-    }
+        for (int k = 0; k < 2; k++) s[i][k] = ((d[0][2 * i + k] * 4 + d[1][2 * i + k]) * 4 + d[2][2 * i + k]) * 4 + d[3][2 * i + k];
+}
+// A block's two groups added to a chain: products of the scales, then one multiply-add each with the group's sum.
+__device__ __forceinline__ float chain_q2(float chain, float dw, float sc0, float sc1, float sum0, float sum1) {
+    return __fmaf_rn(__fmul_rn(dw, sc1), sum1, __fmaf_rn(__fmul_rn(dw, sc0), sum0, chain));
 }
 
 // Matrices with one in_f in one launch: their 16-row tiles follow each other in the CTAs' tile ranges.  NM > kSameRow: with a row each.
@@ -408,9 +424,9 @@ struct RowGeom {
     int tiles;
 };
 
-// ONE: a warp has one unit, its activations stay in registers.
+// ONE: a warp has one unit, its activations stay in registers; Q2_0: chains in registers (kChains).
 template <int DT, int NM, bool FUSED, bool ONE, bool PUSH>
-__global__ void __launch_bounds__(RowFmt<DT>::kWarps * 32, 2)
+__global__ void __launch_bounds__(kRowWarps<DT, ONE> * 32, kChains<DT, ONE> ? 4 : 2)
     gemv_row_kernel(const __grid_constant__ RowMats<NM> mats, const Q8Dev a, const float *x, RowGeom geo, uint32_t *status,
                     const __grid_constant__ typename PushParam<PUSH>::type push) {
     using F = RowFmt<DT>;
@@ -418,12 +434,13 @@ __global__ void __launch_bounds__(RowFmt<DT>::kWarps * 32, 2)
     extern __shared__ __align__(128) uint8_t smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3, kw = blockDim.x >> 5, S = geo.slots;
     uint8_t *acts = smem + (size_t)S * kw * kBox;                                                                       // [units][kActBytes]
-    // sums that wait for a barrier, twice: Q2_0 [warp][kPart * 16], else [block][kPart * 16 + 4] terms, and the blocks' activation scales behind them
-    constexpr int kCols = F::kPart * kRowTile, kStride = DT == DT_Q2_0 ? kCols : (kCols + 4) * F::kTerm, kBlocks = DT == DT_Q6K ? 2 : 1;
+    // sums that wait for a barrier, twice: chains [tile][warp][kQ2Chains], else terms [block][kPart * 16 + a pad], and the blocks' activation scales behind them
+    constexpr int kPart = kChains<DT, ONE> ? kQ2Part : F::kPart, kCols = kPart * kRowTile, kStride = (kCols + kRowPad<DT>) * F::kTerm;
+    constexpr int kBlocks = DT == DT_Q2_0 ? 8 : DT == DT_Q6K ? 2 : 1;
     float *parts = reinterpret_cast<float *>(acts + (ONE && DT != DT_Q2_0 ? 0 : (size_t)geo.units * F::kActBytes));
-    const int buf = (DT == DT_Q2_0 ? kw : geo.units * kBlocks) * kStride;  // of two buffers
+    const int buf = kChains<DT, ONE> ? kPart * kw * kQ2Chains : geo.units * kBlocks * kStride;  // of two buffers
     [[maybe_unused]] float *s_scale = parts + 2 * buf;
-    __shared__ __align__(8) uint64_t s_bars[F::kWarps * kRowSlots];
+    __shared__ __align__(8) uint64_t s_bars[kRowWarps<DT, ONE> * kRowSlots];
     __shared__ __align__(16) uint32_t s_zero[8];
     __shared__ int s_dead;
     __shared__ uint32_t s_epoch;  // push mode: exchanges completed before this launch
@@ -441,7 +458,11 @@ __global__ void __launch_bounds__(RowFmt<DT>::kWarps * 32, 2)
     const int G = gridDim.x, base = geo.tiles / G, rem = geo.tiles % G;
     const int t_begin = blockIdx.x * base + (blockIdx.x < rem ? blockIdx.x : rem);
     const int n_tiles = base + (blockIdx.x < rem ? 1 : 0);
-    const int u0 = warp * geo.upw, n_units = ONE ? 1 : min(geo.upw, geo.units - u0);
+    // this warp's units: u0, u0 + kStep, ...
+    constexpr int kStep = kChains<DT, ONE> ? 4 : 1;
+    constexpr bool kOneUnit = ONE && DT != DT_Q2_0;
+    const int u0 = kChains<DT, ONE> ? warp : warp * geo.upw;
+    const int n_units = kOneUnit ? 1 : kChains<DT, ONE> ? (geo.units - warp + 3) / 4 : min(geo.upw, geo.units - u0);
     uint64_t policy;  // weights are read once a launch: they do not push what every CTA reads out of L2
     asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(policy));
 
@@ -458,7 +479,7 @@ __global__ void __launch_bounds__(RowFmt<DT>::kWarps * 32, 2)
     auto issue = [&](int slot) {
         if (i_left == 0) return;
         if (lane == 0) {
-            const int unit = u0 + i_unit, col = DT == DT_Q6K ? ((unit * 420) & ~15) >> 1 : unit * 36;  // 16-bit / 32-bit elements of the map
+            const int unit = u0 + i_unit * kStep, col = DT == DT_Q6K ? ((unit * 420) & ~15) >> 1 : unit * 36;  // 16-bit / 32-bit elements of the map
             const uint32_t bar = bar0 + 8 * slot;
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // earlier reads of the slot come first
             asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(kBox) : "memory");
@@ -468,7 +489,7 @@ __global__ void __launch_bounds__(RowFmt<DT>::kWarps * 32, 2)
                          : "memory");
         }
         i_left--;
-        if (ONE || ++i_unit == n_units) {
+        if (kOneUnit || ++i_unit == n_units) {
             i_unit = 0;
             i_row += kRowTile;
             if (NM > 1 && i_mat < NM - 1 && i_row >= mats.out_f[i_mat]) i_row = 0, i_mat++;
@@ -477,6 +498,7 @@ __global__ void __launch_bounds__(RowFmt<DT>::kWarps * 32, 2)
     for (int s = 0; s < S; s++) issue(s);
 
     // ---- activations (from the launch before) ----
+    [[maybe_unused]] const uint8_t *acts0 = acts;
     acts += (size_t)u0 * F::kActBytes;
     asm volatile("griddepcontrol.wait;" ::: "memory");
     if constexpr (PUSH) {
@@ -492,7 +514,21 @@ __global__ void __launch_bounds__(RowFmt<DT>::kWarps * 32, 2)
     [[maybe_unused]] RowB4 b4;
     auto take_row = [&]() {
         if constexpr (DT == DT_Q2_0) {
-            for (int u = 0; u < n_units; u++) put_act_q2<FUSED>(acts + (size_t)u * F::kActBytes, a, x, u0 + u, lane);
+            auto put = [&](int u, const float4 (&v)[4]) { put_act_q2<FUSED>(acts + (size_t)u * kStep * F::kActBytes, a, v, u0 + u * kStep, lane); };
+            float4 v0[4], v1[4];
+            if (FUSED && ONE) {
+                for (int u = 0; u < n_units; u += 2) {  // two units' loads in flight together
+                    load_q2(v0, x, u0 + u * kStep, lane);
+                    if (u + 1 < n_units) load_q2(v1, x, u0 + (u + 1) * kStep, lane);
+                    put(u, v0);
+                    if (u + 1 < n_units) put(u + 1, v1);
+                }
+            } else {
+                for (int u = 0; u < n_units; u++) {
+                    if (FUSED) load_q2(v0, x, u0 + u * kStep, lane);
+                    put(u, v0);
+                }
+            }
             __syncwarp();
         } else if constexpr (ONE) {
             load_act<FUSED>(act, a, x, u0, lane);
@@ -528,7 +564,7 @@ __global__ void __launch_bounds__(RowFmt<DT>::kWarps * 32, 2)
     int batch = 0;
     for (int b0 = 0, nb; b0 < n_tiles; b0 += nb) {
         float *sums = parts + (size_t)(batch & 1) * buf;
-        nb = min(F::kPart, n_tiles - b0);
+        nb = min(kPart, n_tiles - b0);
         if (NM > kSameRow) {  // a batch is of one row
             if (t_begin + b0 == c_end) {
                 c_mat++;
@@ -540,9 +576,9 @@ __global__ void __launch_bounds__(RowFmt<DT>::kWarps * 32, 2)
             nb = min(nb, c_end - (t_begin + b0));
         }
         for (int k = 0; k < nb; k++) {
-            [[maybe_unused]] float share[2] = {0.f, 0.f};  // Q2_0: this lane's shares of rows g, g + 8
-            float *out0 = sums + (DT == DT_Q2_0 ? warp : u0 * kBlocks) * kStride + (k * kRowTile + g + 8 * t) * F::kTerm;  // lanes t = 0, 1
-            for (int u = 0; u < (ONE ? 1 : n_units); u++) {
+            [[maybe_unused]] float chain[2][2] = {{0.f, 0.f}, {0.f, 0.f}};                                    // Q2_0: [half][row g, g + 8]
+            [[maybe_unused]] float *out0 = sums + u0 * kBlocks * kStride + (k * kRowTile + g + 8 * t) * F::kTerm;  // lanes t = 0, 1
+            for (int u = 0; u < (kOneUnit ? 1 : n_units); u++) {
                 if (!row_try(bar0 + 8 * slot, ph) && !row_wait_slow(bar0 + 8 * slot, ph, &s_dead)) {
                     // the launch's results are invalid: no more fetches, and those in flight land before the block gives its shared memory back
                     // (bounded; what is read from here on is in bounds)
@@ -569,26 +605,38 @@ __global__ void __launch_bounds__(RowFmt<DT>::kWarps * 32, 2)
                         *reinterpret_cast<float2 *>(out0 + (2 * u + 1) * kStride) = x1;
                     }
                 } else {
-                    const uint8_t *rec = acts + (size_t)u * F::kActBytes;
+                    const uint8_t *rec = acts + (size_t)u * kStep * F::kActBytes;
                     const uint32_t mis = 2 * (t & 1);
                     const bool mine = t == (g >> 1);
                     const uint4 *zero = reinterpret_cast<const uint4 *>(s_zero);
 #pragma unroll
                     for (int H = 0; H < 2; H++) {
+                        float dw[2];
+                        int s2[2][2];
                         const uint8_t *p0 = sl + g * 144 + H * 72 + 18 * t - mis;
                         const uint4 *cg = reinterpret_cast<const uint4 *>(rec + (8 * H + g) * 32);
-                        half_q2(p0, p0 + 8 * 144, mis, mine && !(g & 1) ? cg : zero, mine && (g & 1) ? cg : zero,
-                                *reinterpret_cast<const uint4 *>(rec + 512 + (4 * H + t) * 16), share);
+                        const uint4 sc = *reinterpret_cast<const uint4 *>(rec + 512 + (4 * H + t) * 16);
+                        half_q2(p0, p0 + 8 * 144, mis, mine && !(g & 1) ? cg : zero, mine && (g & 1) ? cg : zero, sc, dw, s2);
+                        if (ONE) {
+#pragma unroll
+                            for (int i = 0; i < 2; i++)
+                                chain[H][i] = chain_q2(chain[H][i], dw[i], __uint_as_float(sc.x), __uint_as_float(sc.y), (float)s2[i][0] * 0.015625f, (float)s2[i][1] * 0.015625f);
+                        } else {  // (a sum has 14 bits)
+                            float *o = sums + ((u0 + u) * 8 + 4 * H + t) * kStride + g * F::kTerm;
+#pragma unroll
+                            for (int i = 0; i < 2; i++)
+                                *reinterpret_cast<float2 *>(o + i * 8 * F::kTerm) = make_float2(dw[i], __uint_as_float(pack16(s2[i][0] >> 6, s2[i][1] >> 6)));
+                        }
                     }
                 }
                 __syncwarp();
                 issue(slot);
                 if (++slot == S) slot = 0, ph ^= 1u;
             }
-            if constexpr (DT == DT_Q2_0) {
-                float acc = ((t & 1) ? share[1] : share[0]) + __shfl_xor_sync(0xffffffffu, (t & 1) ? share[0] : share[1], 1);
-                acc += __shfl_xor_sync(0xffffffffu, acc, 2);
-                if (t < 2) *out0 = acc;
+            if constexpr (kChains<DT, ONE>) {
+                float *p = sums + (k * kw + warp) * kQ2Chains + t * kQ2Stride + g;
+                p[0] = chain[0][0], p[8] = chain[0][1];
+                p[4 * kQ2Stride] = chain[1][0], p[4 * kQ2Stride + 8] = chain[1][1];
             }
         }
         __syncthreads();
@@ -612,7 +660,33 @@ __global__ void __launch_bounds__(RowFmt<DT>::kWarps * 32, 2)
             return __fmaf_rn(x2.x, x2.y, acc);
         };
         const int blocks = geo.units * kBlocks;
-        if constexpr (!ONE && DT != DT_Q2_0) {
+        if constexpr (DT == DT_Q2_0 && !ONE) {
+            // a warp a result, a lane a chain
+            for (int i = warp; i < kRowTile; i += kw) {
+                float v = 0.f;
+#pragma unroll 4
+                for (int b = lane; b < blocks; b += 32) {
+                    const float2 x2 = *reinterpret_cast<const float2 *>(sums + b * kStride + i * F::kTerm);
+                    const float2 sc = *reinterpret_cast<const float2 *>(acts0 + (b >> 3) * F::kActBytes + 512 + (b & 7) * 16);
+                    const uint32_t s2 = __float_as_uint(x2.y);
+                    v = chain_q2(v, x2.x, sc.x, sc.y, (float)(int)(short)(s2 & 0xFFFFu), (float)((int)s2 >> 16));
+                }
+                v = warp_sum(v);
+                if (lane == 0) store(i, v);
+            }
+        } else if constexpr (DT == DT_Q2_0) {
+            // eight threads a result: chains j, j + 8, j + 16, j + 24 (one of each class), then across the threads
+            for (int i = threadIdx.x >> 3; i < nb * kRowTile; i += blockDim.x >> 3) {
+                const float *p = sums + i / kRowTile * kw * kQ2Chains + (threadIdx.x & 7) * kQ2Stride + i % kRowTile;
+                float v[4];
+#pragma unroll
+                for (int c = 0; c < 4; c++) v[c] = c < kw ? p[c * kQ2Chains] : 0.f;
+                float s = (v[0] + v[2]) + (v[1] + v[3]);
+#pragma unroll
+                for (int o = 4; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+                if ((threadIdx.x & 7) == 0) store(i, s);
+            }
+        } else if constexpr (!ONE) {
             // Long rows: eight threads a result, each adds groups of blocks in order, and the groups are added in order (14336 -> 4096: 8.0 us,
             // with one thread a result 8.8).  A warp's four results are of one tile.
             for (int i = threadIdx.x >> 3; i < nb * kRowTile; i += blockDim.x >> 3) {
@@ -638,26 +712,16 @@ __global__ void __launch_bounds__(RowFmt<DT>::kWarps * 32, 2)
                 if (i < 0) i += blockDim.x;
                 if (i >= nb * kRowTile) break;
                 const float *col = sums + i * F::kTerm;
-                float v = 0.f;
-                if constexpr (DT == DT_Q2_0) {
-                    float v4[4] = {0.f, 0.f, 0.f, 0.f};  // (four chains: less latency, and fewer roundings of a growing sum)
-                    for (int w = 0; w < kw; w += 4)
-#pragma unroll
-                        for (int j = 0; j < 4; j++)
-                            if (w + j < kw) v4[j] += col[(w + j) * kStride];
-                    v = (v4[0] + v4[1]) + (v4[2] + v4[3]);
-                } else {
-                    int mi = 0;
-                    if (NM > 1)
-                        while (t_begin + b0 + i / kRowTile >= mats.tile_end[mi]) mi++;
-                    const int gs = mats.group[mi];
-                    float acc = 0.f;
-                    int left = gs;
+                int mi = 0;
+                if (NM > 1)
+                    while (t_begin + b0 + i / kRowTile >= mats.tile_end[mi]) mi++;
+                const int gs = mats.group[mi];
+                float v = 0.f, acc = 0.f;
+                int left = gs;
 #pragma unroll 4
-                    for (int b = 0; b < blocks; b++) {
-                        acc = add_term(col, b, acc);
-                        if (--left == 0 || b == blocks - 1) v += acc, acc = 0.f, left = gs;
-                    }
+                for (int b = 0; b < blocks; b++) {
+                    acc = add_term(col, b, acc);
+                    if (--left == 0 || b == blocks - 1) v += acc, acc = 0.f, left = gs;
                 }
                 store(i, v);
             }
@@ -711,15 +775,18 @@ template <int DT, int NM, bool FUSED, bool ONE, bool PUSH>
 cudaError_t launch_row(const RowMats<NM> &mats, const Q8Dev &a, const float *x, RowGeom geo, int kw, const DeviceInfo &dev, uint32_t *status, cudaStream_t st,
                        const typename PushParam<PUSH>::type &push) {
     using F = RowFmt<DT>;
-    const size_t cols = F::kPart * kRowTile, blocks = (size_t)geo.units * (DT == DT_Q6K ? 2 : 1);
+    const size_t cols = F::kPart * kRowTile, blocks = (size_t)geo.units * (DT == DT_Q2_0 ? 8 : DT == DT_Q6K ? 2 : 1);
     const size_t fixed = (ONE && DT != DT_Q2_0 ? 0 : (size_t)geo.units * F::kActBytes) +
-                         (DT == DT_Q2_0 ? 2 * (size_t)kw * cols : 2 * blocks * (cols + 4) * F::kTerm + (DT == DT_Q4K ? blocks : 0)) * 4;
+                         (kChains<DT, ONE> ? 2 * (size_t)kQ2Part * kw * kQ2Chains : 2 * blocks * (cols + kRowPad<DT>) * F::kTerm + (DT == DT_Q4K ? blocks : 0)) * 4;
     const size_t per_slot = (size_t)kw * kRowTile * F::kPitch;
     // Several CTAs a SM where rows are short and each has a tile: more warps at work, but each CTA reads (or quantises) the row for itself.
-    // (us with one CTA a SM / as many as have a tile: Q4_K 2048 -> 5632 3.0 / 2.5, Q6_K 4096 -> 14336 10.0 / 9.5; Q2_0 4096 -> 4096 with two
-    // CTAs for 1.7 tiles a SM 3.7 / 4.1.)
+    // (us with one CTA a SM / as many as have a tile: Q4_K 2048 -> 5632 3.0 / 2.5.  Chains of Q2_0 also where only some SMs have two tiles, four
+    // warps are few: codes 4096 -> 4096 3.7 / 3.1, 14336 -> 4096 9.4 / 7.0, 3072 -> 8192 4.3 / 3.6.)
     int per_sm = F::kWarps / kw;
-    if (per_sm > geo.tiles / dev.sm_count) per_sm = geo.tiles < dev.sm_count ? 1 : geo.tiles / dev.sm_count;
+    int want = geo.tiles / dev.sm_count;
+    if (kChains<DT, ONE> && geo.tiles % dev.sm_count) want++;
+    if (per_sm > want) per_sm = want < 1 ? 1 : want;
+    while (per_sm > 1 && (fixed + 2 * per_slot + 1024) * per_sm > (size_t)dev.max_smem_optin + 1024) per_sm--;
     const int grid = geo.tiles < dev.sm_count * per_sm ? geo.tiles : dev.sm_count * per_sm;
     // Two slots, no more than a warp has units; three for long Q4_K rows, whose warps fetch neighbouring units (14336 -> 4096 8.8 / 8.1 us;
     // 4096 -> 128256, where they fetch tiles far apart, 50 / 56).
@@ -773,8 +840,6 @@ template <int DT, int NM>
 cudaError_t launch_row_dt(const GemvRow &d, const DeviceInfo &dev, uint32_t *status, cudaStream_t st, const GemvPush *push) {
     using F = RowFmt<DT>;
     RowGeom geo{d.in_f / F::kUnit, 0, 0, 0};
-    geo.upw = (geo.units + F::kWarps - 1) / F::kWarps;
-    const int kw = (geo.units + geo.upw - 1) / geo.upw;
     RowMats<NM> mats;
     memset(&mats, 0, sizeof mats);
     for (int i = 0; i < d.n; i++) {
@@ -786,6 +851,10 @@ cudaError_t launch_row_dt(const GemvRow &d, const DeviceInfo &dev, uint32_t *sta
         if constexpr (NM > kSameRow) mats.x[i] = d.mats[i].x;
     }
     for (int i = d.n; i < NM; i++) mats.tile_end[i] = geo.tiles;
+    auto split = [&](int warps) {
+        geo.upw = (geo.units + warps - 1) / warps;
+        return (geo.units + geo.upw - 1) / geo.upw;
+    };
     if constexpr (DT != DT_Q2_0) {
         auto tiles = [&](int i) { return (d.mats[i].out_f + kRowTile - 1) / kRowTile; };
         // (two Q4_K matrices on one row are split as one)
@@ -793,12 +862,24 @@ cudaError_t launch_row_dt(const GemvRow &d, const DeviceInfo &dev, uint32_t *sta
             mats.group[i] = row_group(DT, d.in_f / 256, DT == DT_Q4K && NM <= kSameRow && d.n > 1 && i < 2 ? tiles(0) + tiles(1) : tiles(i), dev);
     }
     const Q8Dev none{nullptr, nullptr, nullptr, nullptr, 0};
-    const bool one = geo.upw == 1 && DT != DT_Q2_0;
-#define INFR_ROW(FUSED_, PUSH_, A_, P_)                                                                                         \
-    do {                                                                                                                      \
-        if constexpr (DT != DT_Q2_0)                                                                                          \
-            if (one) return launch_row<DT, NM, FUSED_, true, PUSH_>(mats, A_, d.x, geo, kw, dev, status, st, P_);               \
-        return launch_row<DT, NM, FUSED_, false, PUSH_>(mats, A_, d.x, geo, kw, dev, status, st, P_);                           \
+    const int kw = split(F::kWarps);
+    bool one = geo.upw == 1;
+    if constexpr (DT == DT_Q2_0) {
+        // Chains in four warps a CTA; long rows whose CTAs have a tile or so each: more warps a row, the blocks' sums in shared memory (us a call,
+        // chains / sums: codes 14336 -> 1024 5.7 / 4.4, -> 4096 7.0 / 8.2, f32 rows 14336 -> 1024 9.0 / 5.8, -> 4096 10.6 / 9.5, -> 8192 14.6 / 15.5;
+        // 4096 -> 1024 3.2 / 3.0, -> 4096 4.1 / 4.8).
+        one = geo.units <= 8 || geo.tiles > (d.codes ? 1 : 2) * dev.sm_count;
+    }
+#define INFR_ROW(FUSED_, PUSH_, A_, P_)                                                                                              \
+    do {                                                                                                                             \
+        if (!one) {                                                                                                                  \
+            const cudaError_t e = launch_row<DT, NM, FUSED_, false, PUSH_>(mats, A_, d.x, geo, kw, dev, status, st, P_);             \
+            if (DT != DT_Q2_0 || e != cudaErrorInvalidValue || geo.tiles <= dev.sm_count) return e;                                  \
+            cudaGetLastError(); /* the row's blocks leave no room */                                                                 \
+        }                                                                                                                            \
+        const int w = DT == DT_Q2_0 ? (geo.units < kQ2ChainWarps ? geo.units : kQ2ChainWarps) : kw;                                   \
+        if (DT == DT_Q2_0) geo.upw = (geo.units + w - 1) / w;                                                                        \
+        return launch_row<DT, NM, FUSED_, true, PUSH_>(mats, A_, d.x, geo, w, dev, status, st, P_);                                  \
     } while (0)
     if constexpr (NM > kSameRow) {
         INFR_ROW(true, false, none, NoPush{});
