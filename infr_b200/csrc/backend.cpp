@@ -554,7 +554,7 @@ Status CudaBackend::linear_pair(int dtype, const uint8_t *w1, float *y1, uint32_
         const size_t nx = (size_t)m * in_f, n1 = (size_t)m * out_f1, n2 = (size_t)m * out_f2;
         const bool apart = !overlap(x, nx, y1, n1) && !overlap(x, nx, y2, n2) && !overlap(y1, n1, y2, n2);
         if (m == 1 && gemv_impl_ == 0 && apart && gemv_row_takes(dtype, (int)in_f)) {
-            const GemvRowMat mats[2] = {{w1, y1, (int)out_f1}, {w2, y2, (int)out_f2}};
+            const GemvRowMat mats[2] = {{w1, y1, (int)out_f1, nullptr, (int)out_f2}, {w2, y2, (int)out_f2, nullptr, (int)out_f1}};
             const cudaError_t e = launch_gemv_row(GemvRow{dtype, (int)in_f, mats, 2, nullptr, x}, dev_, status_dev_, stream_);
             if (e == cudaSuccess) launches_++;
             if (e != cudaErrorInvalidValue) return cuda_status(e, "linear_pair");
@@ -662,7 +662,7 @@ Status CudaBackend::gemv_q8_pair(int dtype, const uint8_t *w1, float *y1, uint32
     }
     if (m == 1 && gemv_impl_ == 0 && out_f1 && out_f2 && a.gran == act_gran(dtype) && gemv_row_takes(dtype, (int)in_f) && !overlap(y1, out_f1, y2, out_f2)) {
         cudaSetDevice(device_);
-        const GemvRowMat mats[2] = {{w1, y1, (int)out_f1}, {w2, y2, (int)out_f2}};
+        const GemvRowMat mats[2] = {{w1, y1, (int)out_f1, nullptr, (int)out_f2}, {w2, y2, (int)out_f2, nullptr, (int)out_f1}};
         const cudaError_t e = launch_gemv_row(GemvRow{dtype, (int)in_f, mats, 2, &a}, dev_, status_dev_, stream_);
         if (e == cudaSuccess) launches_++;
         if (e != cudaErrorInvalidValue) return cuda_status(e, "gemv_q8_pair");

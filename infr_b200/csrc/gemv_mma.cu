@@ -621,7 +621,7 @@ cudaError_t launch_gemv_q4k_mma_pair(const uint8_t *w1, float *y1, int out_f1, c
                                      const float *x, int m, int in_f, const DeviceInfo &dev, uint32_t *status, cudaStream_t st) {
     if (m < 1 || m > 8 || in_f % 256 || out_f1 < 1 || out_f2 < 1) return cudaErrorInvalidValue;
     if (m == 1) {
-        const GemvRowMat mats[2] = {{w1, y1, out_f1}, {w2, y2, out_f2}};
+        const GemvRowMat mats[2] = {{w1, y1, out_f1, nullptr, out_f2}, {w2, y2, out_f2, nullptr, out_f1}};
         return launch_gemv_row(GemvRow{DT_Q4K, in_f, mats, 2, a, x}, dev, status, st);
     }
     if (a) return launch_mma<false>(w1, *a, nullptr, y1, m, in_f, out_f1, dev, status, st, w2, y2, out_f2);

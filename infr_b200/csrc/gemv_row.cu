@@ -856,10 +856,9 @@ cudaError_t launch_row_dt(const GemvRow &d, const DeviceInfo &dev, uint32_t *sta
         return (geo.units + geo.upw - 1) / geo.upw;
     };
     if constexpr (DT != DT_Q2_0) {
-        auto tiles = [&](int i) { return (d.mats[i].out_f + kRowTile - 1) / kRowTile; };
-        // (two Q4_K matrices on one row are split as one)
+        auto tiles = [](int rows) { return (rows + kRowTile - 1) / kRowTile; };
         for (int i = 0; i < d.n; i++)
-            mats.group[i] = row_group(DT, d.in_f / 256, DT == DT_Q4K && NM <= kSameRow && d.n > 1 && i < 2 ? tiles(0) + tiles(1) : tiles(i), dev);
+            mats.group[i] = row_group(DT, d.in_f / 256, DT == DT_Q4K ? tiles(d.mats[i].out_f) + tiles(d.mats[i].with) : tiles(d.mats[i].out_f), dev);
     }
     const Q8Dev none{nullptr, nullptr, nullptr, nullptr, 0};
     const int kw = split(F::kWarps);

@@ -97,6 +97,7 @@ struct GemvRowMat {
     float *y;
     int out_f;
     const float *x = nullptr;
+    int with = 0;  // Q4_K: rows of the matrix whose K split it shares (a pair on one row is split as one matrix: the bits of a pair call)
 };
 struct GemvRow {
     int dtype, in_f;

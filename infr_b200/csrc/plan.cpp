@@ -98,7 +98,15 @@ bool row_linear(const infr_cuda_plan &p, size_t j) {
     return o.tag == INFR_OP_LINEAR && o.u[0] == 1 && o.u[2] > 0 && o.u[1] <= 0x7fffffffu && o.u[2] <= 0x7fffff00u && o.t[0] != o.t[2] &&
            gemv_row_takes((int)p.tensors[o.t[1]].dtype, (int)o.u[1]);
 }
-// The number of ops from i on that are one-row Linears one launch can take together (below two: none).
+// Two neighbouring Linears of one weight format reading the same rows (q and k, gate and up).
+bool linear_pair_at(const infr_cuda_plan &p, size_t i) {
+    if (i + 1 >= p.ops.size()) return false;
+    const infr_op_desc &a = p.ops[i], &n = p.ops[i + 1];
+    return a.tag == INFR_OP_LINEAR && n.tag == INFR_OP_LINEAR && n.t[0] == a.t[0] && n.u[0] == a.u[0] && n.u[1] == a.u[1] &&
+           p.tensors[n.t[1]].dtype == p.tensors[a.t[1]].dtype && n.t[2] != a.t[2] && a.t[2] != a.t[0] && n.t[2] != a.t[0];
+}
+// The number of ops from i on that are one-row Linears one launch can take together (below two: none).  Pairs among them, taken greedily, are
+// split as pairs, so the last op stays outside where it makes a pair with the one behind it.
 uint32_t row_run(const infr_cuda_plan &p, uint32_t i, bool *same_row) {
     if (!row_linear(p, i)) return 0;
     const infr_op_desc &a = p.ops[i];
@@ -110,6 +118,10 @@ uint32_t row_run(const infr_cuda_plan &p, uint32_t i, bool *same_row) {
         for (uint32_t k = i; ok && k < i + n; k++) ok = l.t[0] != p.ops[k].t[2] && l.t[2] != p.ops[k].t[2] && l.t[2] != p.ops[k].t[0];
         if (!ok) break;
     }
+    uint32_t lone = i;  // the first op behind the pairs and lone ops before it
+    while (lone + 1 < i + n) lone += linear_pair_at(p, lone) ? 2 : 1;
+    if (lone + 1 == i + n && linear_pair_at(p, lone)) n--;
+    if (n < 2) return 0;
     uint32_t same = 1;
     while (same < n && p.ops[i + same].t[0] == a.t[0]) same++;
     *same_row = same == n && n <= 3;
@@ -238,12 +250,8 @@ Status CudaBackend::compile(const infr_graph_desc &g, infr_cuda_plan **out) {
         const uint32_t run = row_run(*plan, i, &same_row);
         if (run >= 2) {
             st = PlanStep{same_row ? PlanStep::kRow : PlanStep::kRows, i, run};
-        } else if (a.tag == INFR_OP_LINEAR && i + 1 < g.n_ops) {
-            // two Linears of one weight format reading the same rows (q and k, gate and up): quantised once
-            const infr_op_desc &n = g.ops[i + 1];
-            if (n.tag == INFR_OP_LINEAR && n.t[0] == a.t[0] && n.u[0] == a.u[0] && n.u[1] == a.u[1] &&
-                plan->tensors[n.t[1]].dtype == plan->tensors[a.t[1]].dtype && n.t[2] != a.t[2] && a.t[2] != a.t[0] && n.t[2] != a.t[0])
-                st = PlanStep{PlanStep::kLinearPair, i, 2};
+        } else if (linear_pair_at(*plan, i)) {
+            st = PlanStep{PlanStep::kLinearPair, i, 2};  // quantised once
         }
         if (a.tag == INFR_OP_ROPE && i + 3 < g.n_ops) {
             const infr_op_desc &rq = g.ops[i + 1], &wk = g.ops[i + 2], &wv = g.ops[i + 3];
@@ -510,6 +518,21 @@ Status CudaBackend::execute_steps(infr_cuda_plan *plan, infr_cuda_buf *const *bi
         return s;
     };
 
+    auto run_pair = [&](const infr_op_desc &op, const infr_op_desc &o2) -> Status {
+        const uint32_t m = op.u[0], in_f = op.u[1];
+        const int wdt = (int)plan->tensors[op.t[1]].dtype;
+        const size_t bpr = (size_t)(in_f / block_elems(wdt)) * block_bytes(wdt);
+        const size_t r1 = op.u[3] / in_f, r2 = o2.u[3] / in_f;
+        DevSpan x, w1, w2, y1, y2;
+        INFR_RESOLVE(op.t[0], (size_t)m * in_f * 4, "Linear x", &x);
+        INFR_RESOLVE(op.t[1], (r1 + op.u[2]) * bpr, "Linear weight", &w1);
+        INFR_RESOLVE(o2.t[1], (r2 + o2.u[2]) * bpr, "Linear weight", &w2);
+        INFR_RESOLVE(op.t[2], (size_t)m * op.u[2] * 4, "Linear dst", &y1);
+        INFR_RESOLVE(o2.t[2], (size_t)m * o2.u[2] * 4, "Linear dst", &y2);
+        return linear_pair(wdt, w1.ptr + r1 * bpr, f32p(y1), op.u[2], w2.ptr + r2 * bpr, f32p(y2), o2.u[2], f32p(x), m, in_f,
+                           reference_ ? INFR_ACT_F32 : INFR_ACT_INT8);
+    };
+
     // The rows that src forms go to tensor `id`; where the next step is a Linear or a pair of them that reads these rows and that the
     // tensor-memory GEMM takes, both steps run here (*fed).
     auto feed = [&](size_t next, uint32_t id, uint32_t rows, uint32_t dim, const RowSource &src, bool *fed) -> Status {
@@ -553,19 +576,7 @@ Status CudaBackend::execute_steps(infr_cuda_plan *plan, infr_cuda_buf *const *bi
             continue;
         }
         if (st.kind == PlanStep::kLinearPair) {
-            const infr_op_desc &o2 = plan->ops[st.op0 + 1];
-            const uint32_t m = op.u[0], in_f = op.u[1];
-            const int wdt = (int)plan->tensors[op.t[1]].dtype;
-            const size_t bpr = (size_t)(in_f / block_elems(wdt)) * block_bytes(wdt);
-            const size_t r1 = op.u[3] / in_f, r2 = o2.u[3] / in_f;
-            DevSpan x, w1, w2, y1, y2;
-            INFR_RESOLVE(op.t[0], (size_t)m * in_f * 4, "Linear x", &x);
-            INFR_RESOLVE(op.t[1], (r1 + op.u[2]) * bpr, "Linear weight", &w1);
-            INFR_RESOLVE(o2.t[1], (r2 + o2.u[2]) * bpr, "Linear weight", &w2);
-            INFR_RESOLVE(op.t[2], (size_t)m * op.u[2] * 4, "Linear dst", &y1);
-            INFR_RESOLVE(o2.t[2], (size_t)m * o2.u[2] * 4, "Linear dst", &y2);
-            s = linear_pair(wdt, w1.ptr + r1 * bpr, f32p(y1), op.u[2], w2.ptr + r2 * bpr, f32p(y2), o2.u[2], f32p(x), m, in_f,
-                            reference_ ? INFR_ACT_F32 : INFR_ACT_INT8);
+            s = run_pair(op, plan->ops[st.op0 + 1]);
             if (!s.ok()) return s;
             continue;
         }
@@ -601,9 +612,15 @@ Status CudaBackend::execute_steps(infr_cuda_plan *plan, infr_cuda_buf *const *bi
                 mats[k] = GemvRowMat{w.ptr + r0 * bpr, f32p(y), (int)l.u[2], st.kind == PlanStep::kRows ? f32p(x) : nullptr};
                 if (st.kind == PlanStep::kRow) d.x = f32p(x);
             }
+            auto pair_at = [&](uint32_t k) { return k + 1 < st.n_ops && linear_pair_at(*plan, st.op0 + k); };
+            for (uint32_t k = 0; k < st.n_ops; k++)
+                if (pair_at(k)) mats[k].with = mats[k + 1].out_f, mats[k + 1].with = mats[k].out_f, k++;
             bool taken = false;
             s = linear_row(d, &taken);
-            for (uint32_t k = 0; s.ok() && !taken && k < st.n_ops; k++) s = run_single(plan->ops[st.op0 + k]);
+            for (uint32_t k = 0; s.ok() && !taken && k < st.n_ops; k++) {
+                const infr_op_desc &l = plan->ops[st.op0 + k];
+                s = pair_at(k) ? run_pair(l, plan->ops[st.op0 + ++k]) : run_single(l);
+            }
             if (!s.ok()) return s;
             continue;
         }
