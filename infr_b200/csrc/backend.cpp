@@ -350,8 +350,8 @@ Status CudaBackend::linear(int dtype, const uint8_t *w, const float *x, float *y
         if (e != cudaErrorInvalidValue) return cuda_status(e, "gemv_q2");
         cudaGetLastError();
     }
-    // One Q6_K row: quantised inside the GEMV.
-    if (dtype == DT_Q6K && m == 1 && act == INFR_ACT_INT8 && gemv_impl_ == 0 && !in_place && gemv_row_takes(dtype, (int)in_f)) {
+    // One Q6_K row: the same.
+    if (dtype == DT_Q6K && m == 1 && in_f <= 36864 && act == INFR_ACT_INT8 && gemv_impl_ == 0 && !in_place && gemv_row_takes(dtype, (int)in_f)) {
         const GemvRowMat mat{w, y, (int)out_f};
         const cudaError_t e = launch_gemv_row(GemvRow{dtype, (int)in_f, &mat, 1, nullptr, x}, dev_, status_dev_, stream_);
         if (e == cudaSuccess) launches_++;
@@ -553,7 +553,7 @@ Status CudaBackend::linear_pair(int dtype, const uint8_t *w1, float *y1, uint32_
         // (in place: quantise first; results that overlap each other: one launch each, in order)
         const size_t nx = (size_t)m * in_f, n1 = (size_t)m * out_f1, n2 = (size_t)m * out_f2;
         const bool apart = !overlap(x, nx, y1, n1) && !overlap(x, nx, y2, n2) && !overlap(y1, n1, y2, n2);
-        if (m == 1 && gemv_impl_ == 0 && apart && gemv_row_takes(dtype, (int)in_f)) {
+        if (m == 1 && gemv_impl_ == 0 && apart && dtype == DT_Q6K && in_f <= 36864 && gemv_row_takes(dtype, (int)in_f)) {
             const GemvRowMat mats[2] = {{w1, y1, (int)out_f1, nullptr, (int)out_f2}, {w2, y2, (int)out_f2, nullptr, (int)out_f1}};
             const cudaError_t e = launch_gemv_row(GemvRow{dtype, (int)in_f, mats, 2, nullptr, x}, dev_, status_dev_, stream_);
             if (e == cudaSuccess) launches_++;
@@ -660,7 +660,8 @@ Status CudaBackend::gemv_q8_pair(int dtype, const uint8_t *w1, float *y1, uint32
         if (s.ok()) launches_++;
         return s;
     }
-    if (m == 1 && gemv_impl_ == 0 && out_f1 && out_f2 && a.gran == act_gran(dtype) && gemv_row_takes(dtype, (int)in_f) && !overlap(y1, out_f1, y2, out_f2)) {
+    if (m == 1 && gemv_impl_ == 0 && out_f1 && out_f2 && a.gran == act_gran(dtype) && gemv_row_takes(dtype, (int)in_f) && (dtype != DT_Q6K || in_f <= 36864) &&
+        !overlap(y1, out_f1, y2, out_f2)) {
         cudaSetDevice(device_);
         const GemvRowMat mats[2] = {{w1, y1, (int)out_f1, nullptr, (int)out_f2}, {w2, y2, (int)out_f2, nullptr, (int)out_f1}};
         const cudaError_t e = launch_gemv_row(GemvRow{dtype, (int)in_f, mats, 2, &a}, dev_, status_dev_, stream_);

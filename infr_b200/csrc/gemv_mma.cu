@@ -1,4 +1,4 @@
-// Q4_K GEMV of small batches (2 <= m <= 8; one row: gemv_row.cu) on the warp-level int8 matrix unit.
+// Q4_K GEMV of small batches (m <= 8; one row mostly in gemv_row.cu: row_first) on the warp-level int8 matrix unit.
 //
 // y[m,out_f] = x[m,in_f] * W^T with the production infr-cpu arithmetic
 // (crates/infr-cpu/src/kernels.rs:151-184): per 256-element super-block
@@ -290,6 +290,36 @@ __global__ void __launch_bounds__(KW * TG * 32, 16 / (KW * TG))
             }
         }
     } else {
+        if (M == 1) {
+            // One row.  Every global load of a thread is issued before its first shared-memory store (the compiler
+            // may not move a load of a generic pointer across such a store), so the staging costs one round trip to
+            // L2 instead of one per loop.
+            const int units = in_f / 8;
+            const int tid = threadIdx.x;
+            const int sum0 = tid < nb * 8 ? a.sums[tid] : 0;
+            const float d0 = tid < nb ? a.d[tid] : 0.f;
+            for (int u0 = tid; u0 < units; u0 += 4 * kThreadsMma) {
+                uint2 v[4];
+#pragma unroll
+                for (int k = 0; k < 4; k++) {
+                    const int u = u0 + k * kThreadsMma;
+                    v[k] = make_uint2(0, 0);
+                    if (u < units) v[k] = *reinterpret_cast<const uint2 *>(a.qs + (size_t)u * 8);
+                }
+#pragma unroll
+                for (int k = 0; k < 4; k++) {
+                    const int u = u0 + k * kThreadsMma;
+                    const int b = u >> 5, uu = u & 31, s = uu >> 2, tt = uu & 3;
+                    if (u < units) *reinterpret_cast<uint2 *>(s_codes + (size_t)b * kStagedBytes + tt * kLaneBytes + s * 8) = v[k];
+                }
+            }
+            for (int r = tid; r < nb * 8; r += kThreadsMma) {
+                const int b = r >> 3, s = r & 7, sum = r == tid ? sum0 : a.sums[r];
+                s_bsplit[(size_t)b * 16 + s] = (uint8_t)(sum & 63);
+                s_bsplit[(size_t)b * 16 + 8 + s] = (uint8_t)(int8_t)(sum >> 6);
+            }
+            for (int b = tid; b < nb; b += kThreadsMma) s_d8[b * 8] = b == tid ? d0 : a.d[b];
+        } else {
         // activation row of column n: the item's n-th pair (gathered through pair_row when given)
         __shared__ uint32_t s_row[8];
         if (threadIdx.x < 8) s_row[threadIdx.x] = threadIdx.x < m ? (uint32_t)(grp.pair_row ? grp.pair_row[p0 + threadIdx.x] : p0 + threadIdx.x) : 0u;
@@ -321,6 +351,7 @@ __global__ void __launch_bounds__(KW * TG * 32, 16 / (KW * TG))
         for (int i = threadIdx.x; i < M * nb; i += kThreadsMma) {
             const int n = i / nb, b = i - n * nb;
             s_d8[b * 8 + n] = n < m ? a.d[(size_t)s_row[n] * nb + b] : 0.f;
+        }
         }
     }
     __syncthreads();
@@ -389,10 +420,12 @@ __global__ void __launch_bounds__(KW * TG * 32, 16 / (KW * TG))
                         sdh[0] += sa_hi * dhi[0];
                         sdl[2] += sb_lo * dlo[2];
                         sdh[2] += sb_hi * dhi[2];
-                        sdl[1] += sa_lo * dlo[1];
-                        sdh[1] += sa_hi * dhi[1];
-                        sdl[3] += sb_lo * dlo[3];
-                        sdh[3] += sb_hi * dhi[3];
+                        if (M > 1) {
+                            sdl[1] += sa_lo * dlo[1];
+                            sdh[1] += sa_hi * dhi[1];
+                            sdl[3] += sb_lo * dlo[3];
+                            sdh[3] += sb_hi * dhi[3];
+                        }
                     }
                     int sd[4];
 #pragma unroll
@@ -407,9 +440,11 @@ __global__ void __launch_bounds__(KW * TG * 32, 16 / (KW * TG))
                     const float e0 = e01.x;
                     accf[0] += e0 * (d0 * (float)sd[0] - dm0 * (float)(sml[0] + 64 * smh[0]));
                     accf[2] += e0 * (d1 * (float)sd[2] - dm1 * (float)(sml[2] + 64 * smh[2]));
-                    const float e1 = e01.y;
-                    accf[1] += e1 * (d0 * (float)sd[1] - dm0 * (float)(sml[1] + 64 * smh[1]));
-                    accf[3] += e1 * (d1 * (float)sd[3] - dm1 * (float)(sml[3] + 64 * smh[3]));
+                    if (M > 1) {
+                        const float e1 = e01.y;
+                        accf[1] += e1 * (d0 * (float)sd[1] - dm0 * (float)(sml[1] + 64 * smh[1]));
+                        accf[3] += e1 * (d1 * (float)sd[3] - dm1 * (float)(sml[3] + 64 * smh[3]));
+                    }
                 }
             }
             __syncwarp();
@@ -588,7 +623,8 @@ template <bool FUSED>
 cudaError_t launch_mma(const uint8_t *w, const Q8Dev &a, const float *x, float *y, int m, int in_f, int out_f,
                        const DeviceInfo &dev, uint32_t *status, cudaStream_t st, const uint8_t *w2 = nullptr, float *y2 = nullptr,
                        int out_f2 = 0, const GemvPush *push = nullptr) {
-    if (m <= 2) return launch_mma_m<2, FUSED>(w, a, x, y, m, in_f, out_f, dev, status, st, w2, y2, out_f2, push);
+    if (m == 1) return launch_mma_m<1, FUSED>(w, a, x, y, m, in_f, out_f, dev, status, st, w2, y2, out_f2, push);
+    if (m == 2) return launch_mma_m<2, FUSED>(w, a, x, y, m, in_f, out_f, dev, status, st, w2, y2, out_f2, push);
     if (m <= 4) return launch_mma_m<4, FUSED>(w, a, x, y, m, in_f, out_f, dev, status, st, w2, y2, out_f2, push);
     return launch_mma_m<8, FUSED>(w, a, x, y, m, in_f, out_f, dev, status, st, w2, y2, out_f2, push);
 }
@@ -615,30 +651,37 @@ cudaError_t launch_grouped_q4k_mma(const uint8_t *bank, const uint8_t *bank2, in
     return launch_mma_cfg<8, false, 4, 2>(bank, a, nullptr, y, 8, in_f, out_f, dev, status, st, grp, n_experts, max_items, bank2, y2, out2, nullptr, items);
 }
 
-// Two Q4_K matrices with the same in_f against the same rows, one launch: pre-quantised rows (a), or f32 rows (x, a null)
+// One row: whether gemv_row.cu comes first, or this kernel (the same bits).  A long row's terms leave that kernel's warps one ring slot (from 153
+// blocks on) and then no room at all (232).  us a call of f32 rows / codes, gemv_row: 40960 -> 1024 18 / 13, 57344 -> 8192 72 / 65; this kernel:
+// 14 / 9.5, 62 / 54.
+static bool row_first(int in_f, int rows, bool codes, const DeviceInfo &dev) { return in_f <= 38912; }
+
+// Two Q4_K matrices with the same in_f against the same rows, one launch (w2 null: one): pre-quantised rows (a), or f32 rows (x, a null)
 // quantised inside the kernel.
+static cudaError_t launch_q4k(const uint8_t *w1, float *y1, int out_f1, const uint8_t *w2, float *y2, int out_f2, const Q8Dev *a, const float *x, int m, int in_f,
+                              const DeviceInfo &dev, uint32_t *status, cudaStream_t st, const GemvPush *push) {
+    if (m == 1 && !a && (uintptr_t)x % 16) return cudaErrorInvalidValue;
+    if (m == 1 && row_first(in_f, out_f1 + out_f2, a, dev)) {
+        const GemvRowMat mats[2] = {{w1, y1, out_f1, nullptr, out_f2}, {w2, y2, out_f2, nullptr, out_f1}};
+        const cudaError_t e = launch_gemv_row(GemvRow{DT_Q4K, in_f, mats, w2 ? 2 : 1, a, x}, dev, status, st, push);
+        if (e != cudaErrorInvalidValue) return e;
+        cudaGetLastError();
+    }
+    if (a) return launch_mma<false>(w1, *a, nullptr, y1, m, in_f, out_f1, dev, status, st, w2, y2, out_f2, push);
+    Q8Dev none{nullptr, nullptr, nullptr, nullptr, 256};
+    return launch_mma<true>(w1, none, x, y1, m, in_f, out_f1, dev, status, st, w2, y2, out_f2, push);
+}
+
 cudaError_t launch_gemv_q4k_mma_pair(const uint8_t *w1, float *y1, int out_f1, const uint8_t *w2, float *y2, int out_f2, const Q8Dev *a,
                                      const float *x, int m, int in_f, const DeviceInfo &dev, uint32_t *status, cudaStream_t st) {
     if (m < 1 || m > 8 || in_f % 256 || out_f1 < 1 || out_f2 < 1) return cudaErrorInvalidValue;
-    if (m == 1) {
-        const GemvRowMat mats[2] = {{w1, y1, out_f1, nullptr, out_f2}, {w2, y2, out_f2, nullptr, out_f1}};
-        return launch_gemv_row(GemvRow{DT_Q4K, in_f, mats, 2, a, x}, dev, status, st);
-    }
-    if (a) return launch_mma<false>(w1, *a, nullptr, y1, m, in_f, out_f1, dev, status, st, w2, y2, out_f2);
-    Q8Dev none{nullptr, nullptr, nullptr, nullptr, 256};
-    return launch_mma<true>(w1, none, x, y1, m, in_f, out_f1, dev, status, st, w2, y2, out_f2);
+    return launch_q4k(w1, y1, out_f1, w2, y2, out_f2, a, x, m, in_f, dev, status, st, nullptr);
 }
 
 cudaError_t launch_gemv_q4k_mma(const uint8_t *w, const Q8Dev *a, const float *x, float *y, int m, int in_f, int out_f,
                                 const DeviceInfo &dev, uint32_t *status, cudaStream_t st, const GemvPush *push) {
     if (m < 1 || m > 8 || in_f % 256) return cudaErrorInvalidValue;
-    if (m == 1) {
-        const GemvRowMat mat{w, y, out_f};
-        return launch_gemv_row(GemvRow{DT_Q4K, in_f, &mat, 1, a, x}, dev, status, st, push);
-    }
-    if (a) return launch_mma<false>(w, *a, nullptr, y, m, in_f, out_f, dev, status, st, nullptr, nullptr, 0, push);
-    Q8Dev none{nullptr, nullptr, nullptr, nullptr, 256};
-    return launch_mma<true>(w, none, x, y, m, in_f, out_f, dev, status, st, nullptr, nullptr, 0, push);
+    return launch_q4k(w, y, out_f, nullptr, nullptr, 0, a, x, m, in_f, dev, status, st, push);
 }
 
 }  // namespace infr

@@ -1,5 +1,5 @@
 // Q6_K (256 elements / 210 bytes: ql[128] low nibbles, qh[64] high 2 bits, 16 int8 sub-block scales, f16 d;
-// w = d * sc_s * (q - 32)) GEMV of small batches (2 <= m <= 8; one row: gemv_row.cu) on the warp-level int8 matrix unit, for
+// w = d * sc_s * (q - 32)) GEMV of small batches (m <= 8; one row of up to 36864: gemv_row.cu) on the warp-level int8 matrix unit, for
 // rows whose byte length is a multiple of 16 (8 | blocks per row), the stride rule of a TMA tensor map.
 //
 // Arithmetic of vec_dot_q6k (vec_dot_q6k_scalar, crates/infr-cpu/src/kernels.rs:487-526): per block
@@ -72,7 +72,7 @@ struct Q6Geom {
     int slots;  // ring slots per warp
 };
 
-template <bool ODD>
+template <int M, bool ODD>
 __device__ __forceinline__ void block_q6(const uint8_t *p0, const uint8_t *p1, const uint8_t *st, const float *s_d8b, int t, int n0,
                                          float (&accf)[4]) {
     // the lane's 16 activation words of the block (one per sub-block) and its words of the split sums
@@ -118,8 +118,10 @@ __device__ __forceinline__ void block_q6(const uint8_t *p0, const uint8_t *p1, c
                 const int s0 = sbyte(sc0[s >> 2], s & 3), s1 = sbyte(sc1[s >> 2], s & 3);
                 isum[0] += s0 * pr[0];
                 isum[2] += s1 * pr[2];
-                isum[1] += s0 * pr[1];
-                isum[3] += s1 * pr[3];
+                if (M > 1) {
+                    isum[1] += s0 * pr[1];
+                    isum[3] += s1 * pr[3];
+                }
             }
         }
     }
@@ -134,8 +136,10 @@ __device__ __forceinline__ void block_q6(const uint8_t *p0, const uint8_t *p1, c
     const float2 e = *reinterpret_cast<const float2 *>(s_d8b + n0);  // zero for absent tokens
     accf[0] = fmaf(d0 * e.x, (float)(isum[0] - 32 * (cl[0] + 64 * ch[0])), accf[0]);
     accf[2] = fmaf(d1 * e.x, (float)(isum[2] - 32 * (cl[2] + 64 * ch[2])), accf[2]);
-    accf[1] = fmaf(d0 * e.y, (float)(isum[1] - 32 * (cl[1] + 64 * ch[1])), accf[1]);
-    accf[3] = fmaf(d1 * e.y, (float)(isum[3] - 32 * (cl[3] + 64 * ch[3])), accf[3]);
+    if (M > 1) {
+        accf[1] = fmaf(d0 * e.y, (float)(isum[1] - 32 * (cl[1] + 64 * ch[1])), accf[1]);
+        accf[3] = fmaf(d1 * e.y, (float)(isum[3] - 32 * (cl[3] + 64 * ch[3])), accf[3]);
+    }
 }
 
 // Shared memory: rings [KW][slots][16 x 224 B]; staged activations per token n and block b: 352 B at
@@ -210,13 +214,13 @@ __global__ void __launch_bounds__(KW * 32, 16 / KW)
             uint4 v[4];
 #pragma unroll
             for (int k = 0; k < 4; k++) {
-                const int i = i0 + k * KW * 32, n = i / units, u = i - n * units;
+                const int i = i0 + k * KW * 32, n = M == 1 ? 0 : i / units, u = i - n * units;
                 v[k] = make_uint4(0, 0, 0, 0);
                 if (i < total && n < m) v[k] = *reinterpret_cast<const uint4 *>(a.qs + (size_t)n * in_f + (size_t)u * 16);
             }
 #pragma unroll
             for (int k = 0; k < 4; k++) {
-                const int i = i0 + k * KW * 32, n = i / units, u = i - n * units;
+                const int i = i0 + k * KW * 32, n = M == 1 ? 0 : i / units, u = i - n * units;
                 if (i < total) {
                     uint8_t *dst = s_act + (size_t)(n * nb + (u >> 4)) * kStagedBlock + (u & 15) * 4;
                     *reinterpret_cast<uint32_t *>(dst) = v[k].x;
@@ -259,9 +263,9 @@ __global__ void __launch_bounds__(KW * 32, 16 / KW)
                 const uint8_t *p0 = ring + (size_t)slot * kSlotBytes6 + (size_t)g * kPitch + off, *p1 = p0 + 8 * kPitch;
                 const uint8_t *st = s_act + (size_t)(gt * nb + b) * kStagedBlock;
                 if (b & 1)
-                    block_q6<true>(p0, p1, st, s_d8 + b * 8, t, n0, accf);
+                    block_q6<M, true>(p0, p1, st, s_d8 + b * 8, t, n0, accf);
                 else
-                    block_q6<false>(p0, p1, st, s_d8 + b * 8, t, n0, accf);
+                    block_q6<M, false>(p0, p1, st, s_d8 + b * 8, t, n0, accf);
             }
             __syncwarp();
             issue(slot);
@@ -547,8 +551,15 @@ cudaError_t launch_gemv_q6_mma(const uint8_t *w, const Q8Dev &a, float *y, int m
                                uint32_t *status, cudaStream_t st, const GemvPush *push) {
     if (m < 1 || m > 8 || in_f % 2048 || a.gran != 256 || !a.sums16) return cudaErrorInvalidValue;
     if (m == 1) {
-        const GemvRowMat mat{w, y, out_f};
-        return launch_gemv_row(GemvRow{DT_Q6K, in_f, &mat, 1, &a}, dev, status, st, push);
+        // gemv_row.cu (the same bits), unless the terms of a row's blocks leave too little room beside them (us a call of codes, gemv_row / this
+        // kernel: 34816 -> 4096 24 / 29, 40960 -> 1024 18.7 / 16.9, 53248 -> 4096 56 / 41, where gemv_row declines and the byte-dot kernel ran)
+        if (in_f <= 36864) {
+            const GemvRowMat mat{w, y, out_f};
+            const cudaError_t e = launch_gemv_row(GemvRow{DT_Q6K, in_f, &mat, 1, &a}, dev, status, st, push);
+            if (e != cudaErrorInvalidValue) return e;
+            cudaGetLastError();
+        }
+        return launch_m6<1>(w, a, y, m, in_f, out_f, dev, status, st, push);
     }
     if (m == 2) return launch_m6<2>(w, a, y, m, in_f, out_f, dev, status, st, push);
     if (m <= 4) return launch_m6<4>(w, a, y, m, in_f, out_f, dev, status, st, push);
