@@ -651,10 +651,18 @@ cudaError_t launch_grouped_q4k_mma(const uint8_t *bank, const uint8_t *bank2, in
     return launch_mma_cfg<8, false, 4, 2>(bank, a, nullptr, y, 8, in_f, out_f, dev, status, st, grp, n_experts, max_items, bank2, y2, out2, nullptr, items);
 }
 
-// One row: whether gemv_row.cu comes first, or this kernel (the same bits).  A long row's terms leave that kernel's warps one ring slot (from 153
-// blocks on) and then no room at all (232).  us a call of f32 rows / codes, gemv_row: 40960 -> 1024 18 / 13, 57344 -> 8192 72 / 65; this kernel:
-// 14 / 9.5, 62 / 54.
-static bool row_first(int in_f, int rows, bool codes, const DeviceInfo &dev) { return in_f <= 38912; }
+// One row: whether gemv_row.cu comes first, or this kernel (the same bits).  A row of more than 16 blocks costs that kernel a second pass over its
+// terms; above 152 they leave its warps one ring slot, and from 232 on they do not fit.  us a call, gemv_row / this kernel:
+//   f32 rows  5632 -> 2048 4.5 / 4.1, 8192 -> 2048 5.4 / 4.8, 14336 -> 1024 7.0 / 6.4, but with more than a tile an SM 5632 -> 4096 5.6 / 5.7,
+//             14336 -> 4096 10.3 / 11.4, 28672 -> 8192 29 / 34;  40960 -> 1024 18 / 14, 57344 -> 8192 72 / 62
+//   codes     8192 -> 2048 4.5 / 3.8, 12288 -> 4096 8.0 / 7.5, 14336 -> 8192 14.5 / 13.8, 20480 -> 4096 11.1 / 10.7, 28672 -> 8192 26 / 28,
+//             34816 -> 4096 17 / 18;  53248 -> 4096 32 / 27.  A decoded token of a model 8192 wide (4 layers): 590 / 577.
+// (4096 -> 4096 codes in a chain of their own 3.6 / 3.5, but between the other launches of a decoded token gemv_row leaves more room: 1871 / 1994.)
+static bool row_first(int in_f, int rows, bool codes, const DeviceInfo &dev) {
+    if (in_f <= 4096) return true;
+    if (in_f > 38912) return false;
+    return codes ? in_f > 24576 : rows > kTileRows * dev.sm_count;
+}
 
 // Two Q4_K matrices with the same in_f against the same rows, one launch (w2 null: one): pre-quantised rows (a), or f32 rows (x, a null)
 // quantised inside the kernel.
