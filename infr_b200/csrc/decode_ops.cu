@@ -204,8 +204,9 @@ constexpr int kAttnThreads = 256;  // eight warps: 16 keys each in the score pha
 // then the softmax weights p) is split into two f16 pieces, hi = its top 11 significant bits, mid = the next 11 of the remainder times 2^11,
 // which sit in two neighbouring columns of the instruction's N dimension and are added afterwards; what is dropped is below 2^-22 of the
 // operand, the size of the rounding of an f32 accumulation itself.  A power of two per head brings the largest |q| to 2^14 .. 2^15, weights
-// (at most 1) are multiplied by 2^15: an element down to 2^-26 of the largest keeps all these bits, one below that an error of 2^-49 of it.
-// Products are exact, sums are f32.  (The same split in tf32 pieces, with the same bits, had to widen every half of the tile to 32 bits first: a batch of 32 sequences at 4097 keys 113 -> 95 us a layer.)
+// (at most 1) are multiplied by 2^15: an element down to 2^-26 of the largest keeps all these bits.  A tile with an element below that (f16 ends
+// there) is multiplied in tf32 pieces, which have the exponents of f32 (tile_tf32): every element keeps its bits, whatever the others are.
+// Products are exact, sums are f32.  (The same split in tf32 pieces, with the same bits, has to widen every half of the tile to 32 bits first: a batch of 32 sequences at 4097 keys 113 -> 95 us a layer.)
 // Phase 1: warp w scores keys 16w..16w+15 against the G query heads that share the KV head: A = the keys (ldmatrix),
 // B = the q pieces, K = head_dim in steps of 8.  Phase 2: one warp per head turns the tile's scores into
 // exp(s - m), their sum, and the two pieces of each weight.  Phase 3: warp w owns output dims 16 (w mod HD/16):
@@ -267,17 +268,20 @@ __device__ __forceinline__ void f16_pieces(float x, float y, uint32_t &hi, uint3
     mid = *reinterpret_cast<const uint32_t *>(&m);
 }
 constexpr float kMid = 1.0f / 2048.0f;
+// The f16 pieces of a scaled element that is not zero lose bits below 2^-12: its last bit is below 2^-35 then, the last bit of the second piece.
+constexpr float kShort = 1.0f / 4096.0f;
 // The pieces of one head's query by a warp: columns 2 * pair, 2 * pair + 1 of s_q (rows of QS halves); returns what a sum of products is
-// to be multiplied by.
+// to be multiplied by.  small: set where an element of this lane loses bits (or is zero: cheaper to ask, and rare).
 template <int HD, int QS>
-__device__ __forceinline__ float split_query(const float *qrow, __half *s_q, int pair, int lane, bool valid) {
+__device__ __forceinline__ float split_query(const float *qrow, __half *s_q, int pair, int lane, bool valid, bool &small) {
     constexpr int N = HD / 64;
     float2 v[N];
-    float am = 0.f;
+    float am = 0.f, least = INFINITY;
 #pragma unroll
     for (int i = 0; i < N; i++) {
         v[i] = valid ? *reinterpret_cast<const float2 *>(qrow + i * 64 + lane * 2) : make_float2(0.f, 0.f);
         am = fmaxf(am, fmaxf(fabsf(v[i].x), fabsf(v[i].y)));
+        least = fminf(least, fminf(fabsf(v[i].x), fabsf(v[i].y)));
     }
     am = warp_max(am);
     const int e = (int)(__float_as_uint(am) >> 23);
@@ -289,15 +293,15 @@ __device__ __forceinline__ float split_query(const float *qrow, __half *s_q, int
         *reinterpret_cast<uint32_t *>(s_q + (2 * pair) * QS + i * 64 + lane * 2) = hi;
         *reinterpret_cast<uint32_t *>(s_q + (2 * pair + 1) * QS + i * 64 + lane * 2) = mid;
     }
+    small = small || (valid && least * f < kShort);
     return 1.0f / f;
 }
-// Scores of one head (f32, 128 keys, `keys` of them valid) -> the pieces of exp(s - m) in columns 2 * pair, 2 * pair + 1 of s_p, m and l.
-template <int PS>
-__device__ __forceinline__ void softmax_tile(const float *s_sc, __half *s_p, int pair, int lane, int keys, float factor, float *ml) {
-    float v[4], m = -INFINITY;
+// Scores of one head (f32, 128 keys, `keys` of them valid) -> this lane's four of exp(s - m), and m and l in ml.
+__device__ __forceinline__ void tile_weights(const float *s_sc, int lane, int keys, float factor, float *ml, float (&v)[4]) {
+    float m = -INFINITY;
 #pragma unroll
     for (int e = 0; e < 4; e++) {
-        v[e] = lane + 32 * e < keys ? s_sc[lane + 32 * e] * factor : -INFINITY;
+        v[e] = lane + 32 * e < keys ? __fmul_rn(s_sc[lane + 32 * e], factor) : -INFINITY;
         m = fmaxf(m, v[e]);
     }
     m = warp_max(m);
@@ -308,14 +312,23 @@ __device__ __forceinline__ void softmax_tile(const float *s_sc, __half *s_p, int
         l += v[e];
     }
     l = warp_sum(l);
+    if (lane == 0) ml[0] = m, ml[1] = l;
+}
+// The weights' pieces in columns 2 * pair, 2 * pair + 1 of s_p.  Returns whether a weight of this lane loses bits.
+template <int PS>
+__device__ __forceinline__ bool softmax_tile(const float *s_sc, __half *s_p, int pair, int lane, int keys, float factor, float *ml) {
+    float v[4];
+    tile_weights(s_sc, lane, keys, factor, ml, v);
+    uint32_t least = 0xFFFFFFFFu;  // of the bits - 1: zero becomes the largest number
 #pragma unroll
     for (int e = 0; e < 4; e++) {
         const float w = v[e] * 32768.0f;
+        least = min(least, __float_as_uint(v[e]) - 1u);
         const __half hi = __float2half_rz(w);
         s_p[(2 * pair) * PS + lane + 32 * e] = hi;
         s_p[(2 * pair + 1) * PS + lane + 32 * e] = __float2half_rz((w - __half2float(hi)) * 2048.0f);
     }
-    if (lane == 0) ml[0] = m, ml[1] = l;
+    return least < __float_as_uint(kShort / 32768.0f) - 1u;
 }
 constexpr float kWeight = 1.0f / 32768.0f;
 // The B words of one lane: column g8 of a group of eight, elements 2 t4, 2 t4 + 1 and 2 t4 + 8, 2 t4 + 9 from `k0` on
@@ -324,6 +337,118 @@ __device__ __forceinline__ void b_words(const __half *cols, int col, int k0, int
     const __half *p = cols + col * S + k0 + 2 * t4;
     b0 = *reinterpret_cast<const uint32_t *>(p);
     b1 = *reinterpret_cast<const uint32_t *>(p + 8);
+}
+
+// D += A(16x8, tf32) * B(8x8, tf32), f32 accumulate
+__device__ __forceinline__ void mma_tf32(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+// tf32 pieces of an f32 value: piece 0 = its top 11 significant bits, piece 1 = the top 11 of what is left
+__device__ __forceinline__ uint32_t tf32_piece(float v, int piece) {
+    const uint32_t hi = __float_as_uint(v) & 0xFFFFE000u;
+    return piece == 0 ? hi : (__float_as_uint(v - __uint_as_float(hi)) & 0xFFFFE000u);
+}
+// Two 16x8 tf32 fragments from the four matrices of an ldmatrix of halves.  The K index of the instruction is only a summation index: slot t takes
+// element 2t of a group of 8 and slot t + 4 element 2t + 1, which is how ldmatrix hands out halves in pairs.
+__device__ __forceinline__ void widen(const uint32_t (&r)[4], uint32_t (&a)[2][4]) {
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const float2 f = __half22float2(*reinterpret_cast<const __half2 *>(&r[i]));
+        a[i >> 1][i & 1] = __float_as_uint(f.x);
+        a[i >> 1][2 + (i & 1)] = __float_as_uint(f.y);
+    }
+}
+// NT groups of four pairs from p0 on (at or past p_end: as the one before it) in one pass over the 16 x 16 fragments that `frag` loads: the pairs'
+// f32 operands are at row(pair) + 16 step; sums(pair, v0, v1) gets rows g8 and g8 + 8.
+template <int NT, int STEPS, class Frag, class Row, class Sums>
+__device__ __forceinline__ void pairs_tf32(int p0, int p_end, const Frag &frag, const Row &row, const Sums &sums) {
+    const int lane = threadIdx.x & 31, g8 = lane >> 2, t4 = lane & 3, piece = g8 & 1;
+    float acc[NT][4];
+    const float *b[NT];
+#pragma unroll
+    for (int nt = 0; nt < NT; nt++) {
+        acc[nt][0] = acc[nt][1] = acc[nt][2] = acc[nt][3] = 0.f;
+        b[nt] = row(min(p0 + nt * 4 + (g8 >> 1), p_end - 1)) + 2 * t4;
+    }
+#pragma unroll 4
+    for (int j = 0; j < STEPS; j++) {
+        uint32_t r[4], a[2][4];
+        frag(r, j);
+        widen(r, a);
+#pragma unroll
+        for (int nt = 0; nt < NT; nt++) {
+            const float2 x = *reinterpret_cast<const float2 *>(b[nt] + j * 16), y = *reinterpret_cast<const float2 *>(b[nt] + j * 16 + 8);
+            mma_tf32(acc[nt], a[0], tf32_piece(x.x, piece), tf32_piece(x.y, piece));
+            mma_tf32(acc[nt], a[1], tf32_piece(y.x, piece), tf32_piece(y.y, piece));
+        }
+    }
+#pragma unroll
+    for (int nt = 0; nt < NT; nt++)
+        if (p0 + nt * 4 + t4 < p_end) sums(p0 + nt * 4 + t4, acc[nt][0] + acc[nt][1], acc[nt][2] + acc[nt][3]);
+}
+// A landed tile for the `pairs` (row, head) pairs of rows 0 .. pairs / G - 1, both products in tf32 pieces: the bits of the f16 form where that one
+// loses none.  Row r sees keys0 + r keys of the tile; sc: [pair][kAttnTile], the scores, to be multiplied by f[pair]; rescore: an element of a query
+// loses bits too, so the scores come again from q.  q, part_o, part_ml: of row 0 and head 0 of the group.
+// A function of its own behind which the kernels return (few tiles need it), its arguments in registers: as a structure they lie in local memory, which
+// has little L1 beside that much shared memory (1 us a tile).  Where every tile takes it: 32 sequences at 4097 keys, 32 heads / 8, 103 -> 121 us.
+template <int HD, int G, int P>
+__device__ __noinline__ void tile_tf32(uint8_t *s_k, uint8_t *s_v, float *sc, const float *f, float (*ml)[2], const float *q, float *part_o, float *part_ml, int n_head,
+                                       int n_splits, int pairs, int keys0, float scale, bool rescore) {
+    using L = AttnSmem<HD>;
+    constexpr int DG = HD / 16, KP = (kAttnThreads / 32) / DG, KEYS = kAttnTile / KP, NT = (P + 3) / 4, NT1 = (G + 3) / 4;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g8 = lane >> 2;
+    auto out_of = [&](int pair) { return ((size_t)(pair / G) * n_head + pair % G) * n_splits; };
+    if (rescore) {  // scores of keys 16 warp .. 16 warp + 15
+        const uint8_t *arow = s_k + (size_t)(16 * warp + (lane & 7) + ((lane >> 3) & 1) * 8) * L::kKeyStride + (lane >> 4) * 16;
+        pairs_tf32<NT, HD / 16>(
+            0, pairs, [&](uint32_t(&r)[4], int j) { ldsm4(r, arow + j * 32); }, [&](int p) { return q + ((size_t)(p / G) * n_head + p % G) * HD; },
+            [&](int p, float v0, float v1) { sc[p * kAttnTile + 16 * warp + g8] = v0, sc[p * kAttnTile + 16 * warp + g8 + 8] = v1; });
+        __syncthreads();
+    }
+    for (int p = warp; p < pairs; p += kAttnThreads / 32) {  // the weights in the scores' place
+        float v[4];
+        tile_weights(sc + p * kAttnTile, lane, min(kAttnTile, keys0 + p / G), rescore ? scale : f[p], ml[p], v);
+#pragma unroll
+        for (int e = 0; e < 4; e++) sc[p * kAttnTile + lane + 32 * e] = v[e];
+    }
+    __syncthreads();
+    if (tid < pairs) part_ml[out_of(tid) * 2] = ml[tid][0], part_ml[out_of(tid) * 2 + 1] = ml[tid][1];
+    // output dims 16 dg .. + 15 over this warp's share of the keys; a row at a time, last row first, where the rows see different keys: 0 must not
+    // meet an infinity of a later token
+    const int dg = warp % DG, kp = warp / DG, nr = pairs / G;
+    const uint8_t *vrow = s_v + (size_t)(kp * KEYS + (lane & 7) + (lane >> 4) * 8) * L::kValStride + (size_t)(16 * dg + ((lane >> 3) & 1) * 8) * 2;
+    float *s_o = reinterpret_cast<float *>(s_k);  // KP > 1: [KP][G][HD], the key tile is dead
+    auto values = [&](auto ntc, int first, int end) {
+        pairs_tf32<decltype(ntc)::value, KEYS / 16>(
+            first, end, [&](uint32_t(&r)[4], int j) { ldsm4_trans(r, vrow + (size_t)j * 16 * L::kValStride); }, [&](int p) { return sc + p * kAttnTile + kp * KEYS; },
+            [&](int p, float v0, float v1) {
+                float *o = (KP == 1 ? part_o + out_of(p) * HD : s_o + (kp * G + p) * HD) + 16 * dg + g8;
+                o[0] = v0, o[8] = v1;
+            });
+    };
+    if (P == G || keys0 >= kAttnTile) {
+        values(std::integral_constant<int, NT>{}, 0, pairs);
+    } else {
+        for (int r = nr - 1; r >= 0 && keys0 + r > 0; r--) {
+            if (r != nr - 1) {
+                __syncthreads();  // the row after this one has been multiplied
+                if (keys0 + r < kAttnTile && tid < HD / 8) *reinterpret_cast<uint4 *>(s_v + (keys0 + r) * L::kValStride + tid * 16) = make_uint4(0, 0, 0, 0);
+                __syncthreads();
+            }
+            values(std::integral_constant<int, NT1>{}, r * G, r * G + G);
+        }
+    }
+    if (KP > 1) {
+        __syncthreads();
+        for (int i = tid; i < G * HD; i += kAttnThreads) {
+            float t = s_o[i];
+#pragma unroll
+            for (int w = 1; w < KP; w++) t += s_o[w * G * HD + i];
+            part_o[out_of(i / HD) * HD + i % HD] = t;
+        }
+    }
 }
 
 constexpr int kAttnChunkPairs = 16;   // (query row, head) pairs of a chunk's tile
@@ -351,12 +476,14 @@ __global__ void __launch_bounds__(kAttnThreads) attn_split_kernel(const float *q
     __shared__ float s_f[G];
     __shared__ float s_ml[G][2];
     __shared__ __align__(8) uint64_t s_bar[2];
+    __shared__ int s_short[2];  // a weight, an element of a query loses bits
     static_assert(KP * G * HD * 4 <= kAttnTile * L::kKeyStride, "the partial outputs reuse the key tile");
     static_assert(KP >= 1 && KP * DG == kAttnThreads / 32, "head_dim 64 or 128");
     const int split = blockIdx.x, kvh = blockIdx.y, qr = blockIdx.z;
     const int seq = qr / rows, ti = qr % rows;
     const int key0 = split * kAttnTile;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g8 = lane >> 2, t4 = lane & 3;
+    if (tid < 2) s_short[tid] = 0;
     pdl_go();
     pdl_wait();
     // sequences at positions of their own (seq_pos, written by an earlier kernel or the host): `pos` is their maximum
@@ -423,8 +550,10 @@ __global__ void __launch_bounds__(kAttnThreads) attn_split_kernel(const float *q
             *reinterpret_cast<uint4 *>(s_v + key * L::kValStride + c * 16) = make_uint4(0, 0, 0, 0);
         }
     }
+    const float *qrow = q + ((size_t)qr * n_head + (size_t)kvh * G) * HD;
+    bool small = false;
     for (int g = warp; g < NT * 4; g += kAttnThreads / 32) {
-        const float f = split_query<HD, QS>(q + ((size_t)qr * n_head + (size_t)kvh * G + g) * HD, s_q, g, lane, g < G);
+        const float f = split_query<HD, QS>(qrow + (size_t)g * HD, s_q, g, lane, g < G, small);
         if (lane == 0 && g < G) s_f[g] = f * scale;
     }
     // the keys have landed; q is staged, the zeroed rows are in place.  (BULK: a bounded wait; if it runs out, the CTA
@@ -482,8 +611,16 @@ __global__ void __launch_bounds__(kAttnThreads) attn_split_kernel(const float *q
         __syncthreads();
     }
     // ---- phase 2
-    for (int g = warp; g < G; g += kAttnThreads / 32) softmax_tile<PS>(s_sc[g], s_p, g, lane, tile_keys, s_f[g], s_ml[g]);
+    if (small) s_short[1] = 1;
+    small = false;
+    for (int g = warp; g < G; g += kAttnThreads / 32) small = softmax_tile<PS>(s_sc[g], s_p, g, lane, tile_keys, s_f[g], s_ml[g]) || small;
+    if (small) s_short[0] = 1;
     __syncthreads();
+    if (s_short[0] || s_short[1]) {
+        tile_tf32<HD, G, G>(
+            s_k, s_v, s_sc[0], s_f, s_ml, qrow, part_o + out_idx * HD, part_ml + out_idx * 2, n_head, n_splits, G, tile_keys, scale, s_short[1] != 0);
+        return;
+    }
     // ---- phase 3: output dims 16 dg .. + 15 over this warp's share of the keys
     {
         const int dg = warp % DG, kp = warp / DG;
@@ -563,6 +700,7 @@ __global__ void __launch_bounds__(kAttnThreads) attn_chunk_kernel(const float *q
     __shared__ float s_f[P];
     __shared__ float s_ml[P][2];
     __shared__ __align__(8) uint64_t s_bar[2];
+    __shared__ int s_short[2];  // a weight, an element of a query loses bits
     const int row_blocks = (rows + R - 1) / R;
     const int split = blockIdx.x, kvh = blockIdx.y, seq = blockIdx.z / row_blocks, ti0 = (blockIdx.z % row_blocks) * R, nr = min(R, rows - ti0);
     const int key0 = split * kAttnTile;
@@ -584,6 +722,7 @@ __global__ void __launch_bounds__(kAttnThreads) attn_chunk_kernel(const float *q
     const __half *kbase = k_cache + (size_t)kvh * HD + tile_off;
     const __half *vbase = v_cache + (size_t)kvh * HD + tile_off;
     if (tid == 0) {
+        s_short[0] = s_short[1] = 0;
 #pragma unroll
         for (int i = 0; i < 2; i++) {
             const uint32_t b = (uint32_t)__cvta_generic_to_shared(&s_bar[i]);
@@ -607,9 +746,11 @@ __global__ void __launch_bounds__(kAttnThreads) attn_chunk_kernel(const float *q
             for (int c = 0; c < CPR; c++) *reinterpret_cast<uint4 *>(dst + c * 16) = make_uint4(0, 0, 0, 0);
         }
     }
+    const float *qrow = q + (((size_t)seq * rows + ti0) * n_head + (size_t)kvh * G) * HD;
+    bool small = false;
     for (int pair = warp; pair < P; pair += kAttnThreads / 32) {
         const int r = pair / G;
-        const float f = split_query<HD, S>(q + (((size_t)seq * rows + ti0 + r) * n_head + (size_t)kvh * G + pair % G) * HD, s_q, pair, lane, r < nr);
+        const float f = split_query<HD, S>(qrow + ((size_t)r * n_head + pair % G) * HD, s_q, pair, lane, r < nr, small);
         if (lane == 0) s_f[pair] = f * scale;
     }
     // (bounded waits; a CTA that gives up leaves after both copies have had their limit)
@@ -649,8 +790,11 @@ __global__ void __launch_bounds__(kAttnThreads) attn_chunk_kernel(const float *q
         return;
     }
     // ---- phase 2
+    if (small) s_short[1] = 1;
+    small = false;
     for (int p = warp; p < P; p += kAttnThreads / 32)
-        softmax_tile<S>(s_sc[p], s_p, p, lane, p / G < nr ? min(kAttnTile, base + p / G) : 0, s_f[p], s_ml[p]);
+        small = softmax_tile<S>(s_sc[p], s_p, p, lane, p / G < nr ? min(kAttnTile, base + p / G) : 0, s_f[p], s_ml[p]) || small;
+    if (small) s_short[0] = 1;
     // The rows see different numbers of keys where the tile ends inside their causal edge: a key that one of them does not see has weight 0
     // there, which must not meet an infinity of a later token.
     bool apart = false;
@@ -660,6 +804,11 @@ __global__ void __launch_bounds__(kAttnThreads) attn_chunk_kernel(const float *q
             apart = apart || (w & 0x7C00u) == 0x7C00u || (w & 0x7C000000u) == 0x7C000000u;
         }
     apart = __syncthreads_or(apart);
+    if (s_short[0] || s_short[1]) {
+        tile_tf32<HD, G, P>(
+            s_k, s_v, s_sc[0], s_f, s_ml, qrow, part_o + out_of(0) * HD, part_ml + out_of(0) * 2, n_head, n_splits, nr * G, base, scale, s_short[1] != 0);
+        return;
+    }
     // ---- phase 3: output dims 16 warp .. + 15
     const uint8_t *vrow = s_v + (size_t)((lane & 7) + (lane >> 4) * 8) * L::kValStride + (size_t)(16 * warp + ((lane >> 3) & 1) * 8) * 2;
     // NTC groups of four pairs from pair p0 on; pairs at or past p1 are computed for nothing and not stored
