@@ -877,7 +877,8 @@ Status CudaBackend::moe_ffn(const MoeArgs &a) {
     //   32 experts, 4096 -> 1792   7: 147 / 194 / 221, 9: 206 / 215 / 242, 11: 235 / 211 / 241, 24: 341 / 222 / 251, 32: 411 / 284 / 257
     // (a layer with a Q6_K bank takes 8-row items throughout: the GEMM's copies want rows of whole 2048-element chunks)
     const bool large = a.n_local * ne * nff >= ((size_t)212 << 20);
-    const bool grouped_gemm = !any_q6 && (mmq_impl_ == 2 || (mmq_impl_ == 0 && 2 * n_pairs >= (size_t)(large ? 21 : 28) * nx));
+    const bool long_rows = !grouped_q4k_takes((int)(ne > nff ? ne : nff), dev_);  // no room for an item's rows
+    const bool grouped_gemm = !any_q6 && (mmq_impl_ == 2 || (mmq_impl_ == 0 && (long_rows || 2 * n_pairs >= (size_t)(large ? 21 : 28) * nx)));
     const int slab = n_pairs >= 28 * nx ? 64 : 32;
     const size_t max_slabs = n_pairs / slab + a.n_local + 1;
     // scratch carve-up (all 256-byte aligned)

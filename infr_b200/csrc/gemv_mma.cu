@@ -95,7 +95,6 @@ struct MmaGeom {
     int nb;         // super-blocks per row
     int bpw;        // super-blocks per warp (K split)
     int slots;      // ring slots per warp
-    int act_bytes;  // staged activation bytes
 };
 
 // Grouped (mixture-of-experts) mode: blockIdx.y walks a device-built list of work items, each up to 8
@@ -499,6 +498,11 @@ EncodeTiledFn encode_tiled() {
     return fn;
 }
 
+// shared memory of a CTA beside its ring
+size_t mma_fixed_bytes(int M, int nb, int warps) {
+    return (size_t)M * nb * (kStagedBytes + 16) + (size_t)nb * 32 + (size_t)2 * warps * 128 * 4 + (size_t)warps * kMaxSlotsMma * 8 + 64;
+}
+
 template <int M, bool FUSED, int KW, int SB, int TG = 1>
 cudaError_t launch_mma_cfg(const uint8_t *w, const Q8Dev &a, const float *x, float *y, int m, int in_f, int out_f,
                            const DeviceInfo &dev, uint32_t *status, cudaStream_t st, const MmaGroup &grp = MmaGroup{},
@@ -508,9 +512,7 @@ cudaError_t launch_mma_cfg(const uint8_t *w, const Q8Dev &a, const float *x, flo
     MmaGeom geo;
     geo.nb = in_f / 256;
     geo.bpw = (geo.nb + KW - 1) / KW;
-    const size_t acts = (size_t)M * geo.nb * (kStagedBytes + 16) + (size_t)geo.nb * 32;
-    geo.act_bytes = (int)acts;
-    const size_t fixed = acts + (size_t)2 * KW * TG * 128 * 4 + (size_t)KW * TG * kMaxSlotsMma * 8 + 64;
+    const size_t fixed = mma_fixed_bytes(M, geo.nb, KW * TG);
     const size_t per_slot = (size_t)KW * TG * kSlotBytes;
     if (fixed + 2 * per_slot > (size_t)dev.max_smem_optin - 1024) return cudaErrorInvalidValue;
     // resident CTAs per SM: 16 math warps in total, each warp with at least two ring slots
@@ -630,6 +632,12 @@ cudaError_t launch_mma(const uint8_t *w, const Q8Dev &a, const float *x, float *
 }
 
 }  // namespace
+
+// Whether eight rows of that length can be staged beside the smallest ring.
+bool grouped_q4k_takes(int in_f, const DeviceInfo &dev) {
+    const int nb = in_f / 256, sb = nb <= 4 ? 1 : 2;
+    return mma_fixed_bytes(8, nb, 4) + (size_t)2 * 4 * kTileRows * sb * 144 <= (size_t)dev.max_smem_optin - 1024;
+}
 
 cudaError_t launch_grouped_q4k_mma(const uint8_t *bank, const uint8_t *bank2, int n_experts, const Q8Dev &a, float *y, float *y2, int in_f, int out_f,
                                    const int *item_expert, const int *item_p0, const int *item_cnt, const int *n_items,

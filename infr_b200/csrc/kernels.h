@@ -174,6 +174,8 @@ cudaError_t launch_gemm_tc_grouped(int slab, const uint8_t *bank, const uint8_t 
 // multiplies up to 8 quantised activation rows (pairs item_p0[i]..+item_cnt[i], gathered through
 // pair_row when non-null) with expert item_expert[i]; y is [n_pairs, out_f].
 // bank2 / y2: a second bank of that shape against the same rows in the same launch (gate and up), or null.  items: how many are expected.
+// grouped_q4k_takes: row lengths that fit (others: cudaErrorInvalidValue).
+bool grouped_q4k_takes(int in_f, const DeviceInfo &dev);
 cudaError_t launch_grouped_q4k_mma(const uint8_t *bank, const uint8_t *bank2, int n_experts, const Q8Dev &a, float *y, float *y2, int in_f, int out_f,
                                    const int *item_expert, const int *item_p0, const int *item_cnt, const int *n_items,
                                    const int *pair_row, int max_items, int items, const DeviceInfo &dev, uint32_t *status,
