@@ -873,10 +873,15 @@ Status CudaBackend::moe_ffn(const MoeArgs &a) {
     //   16 experts, 2048 -> 1024   9: 62 / 75 / 79, 13: 68 / 76 / 79, 16: 73 / 77 / 80, 24: 86 / 77 / 81, 28: 96 / 90 / 82
     //   8 experts, 4096 -> 2048    9: 75 / 90 / 97, 13: 90 / 93 / 98, 16: 96 / 92 / 98, 24: 136 / 108 / 115, 28: 153 / 125 / 115
     //   64 experts, 1024 -> 256    9: 62 / 62 / 67, 13: 64 / 63 / 69, 16: 80 / 65 / 70, 28: 91 / 74 / 76
-    // and with more weights than those, where the GEMM's launches count less:
-    //   32 experts, 4096 -> 1792   7: 147 / 194 / 221, 9: 206 / 215 / 242, 11: 235 / 211 / 241, 24: 341 / 222 / 251, 32: 411 / 284 / 257
+    // Items lose their lead earlier, from 11 rows an expert on, where rows are long and the weights many (items / slabs of 32, M = 2^20 weights a bank):
+    //   32 experts, 3072 -> 1536 (144 M)  10: 161 / 173, 11: 183 / 172;  4096 -> 1536 (192 M)  10: 194 / 211, 11: 223 / 210;  128 experts (768 M)  10: 563 /
+    //   601, 12: 709 / 607;  8 experts, 4096 -> 7168 (224 M)  9: 180 / 192, 11: 209 / 192;  64 experts, 2048 -> 5632 (704 M)  11: 511 / 529, 12: 581 / 525
+    // and not with shorter rows or fewer weights:
+    //   64 experts, 2048 -> 1792 (224 M)  11: 182 / 225, 14: 205 / 223;  128 experts, 2048 -> 1024 (256 M)  11: 255 / 268, 14: 257 / 272;  16 experts,
+    //   4096 -> 2048 (128 M)  11: 121 / 142, 14: 141 / 143, 15: 169 / 142;  3072 -> 2048 (96 M)  14: 120 / 128
     // (a layer with a Q6_K bank takes 8-row items throughout: the GEMM's copies want rows of whole 2048-element chunks)
-    const bool large = a.n_local * ne * nff >= ((size_t)212 << 20);
+    const size_t bank_weights = a.n_local * ne * nff;
+    const bool large = (ne >= 3072 && bank_weights > ((size_t)128 << 20)) || bank_weights >= ((size_t)512 << 20);
     const bool long_rows = !grouped_q4k_takes((int)(ne > nff ? ne : nff), dev_);  // no room for an item's rows
     const bool grouped_gemm = !any_q6 && (mmq_impl_ == 2 || (mmq_impl_ == 0 && (long_rows || 2 * n_pairs >= (size_t)(large ? 21 : 28) * nx)));
     const int slab = n_pairs >= 28 * nx ? 64 : 32;
