@@ -679,8 +679,8 @@ __global__ void __launch_bounds__(kAttnThreads) attn_split_kernel(const float *q
 // column, and so every bit, is that of attn_split_kernel.  Where a tile ends inside the rows' causal edge and a value there is infinite or
 // NaN, the values are multiplied row by row, last row first: each row sees one key fewer, and that key's values are zeroed, so that the
 // matrix unit multiplies 0 (not a later token's infinity) by its weight 0.
-// Measured (us a call with the merge, 113 rows at position 384, 32 heads / 8): a CTA per row 60, tf32 pieces and the edge always row by row
-// 56, now 40; 128 rows at 2048, 32 / 4, 171 -> 116; 128 rows at 1024, 8 / 8, 50 -> 26.
+// Measured (us a call with the merge, 113 rows at position 384, 32 heads / 8): in tf32 pieces with the edge always row by row and eight warps a merged
+// block 46, now 29 (all eight steps of a product unrolled 31.5).
 template <int G>
 __global__ void __launch_bounds__(kAttnThreads) attn_chunk_kernel(const float *q, const __half *k_cache,
                                                                   const __half *v_cache, float *__restrict__ part_o,
@@ -766,7 +766,7 @@ __global__ void __launch_bounds__(kAttnThreads) attn_chunk_kernel(const float *q
 #pragma unroll
         for (int nt = 0; nt < NT; nt++) acc[nt][0] = acc[nt][1] = acc[nt][2] = acc[nt][3] = 0.f;
         const uint8_t *arow = s_k + (size_t)(16 * warp + (lane & 7) + ((lane >> 3) & 1) * 8) * L::kKeyStride + (lane >> 4) * 16;
-#pragma unroll
+#pragma unroll 2
         for (int j = 0; j < HD / 16; j++) {
             uint32_t r[4];
             ldsm4(r, arow + j * 32);
@@ -817,7 +817,7 @@ __global__ void __launch_bounds__(kAttnThreads) attn_chunk_kernel(const float *q
         float acc[NTC][4];
 #pragma unroll
         for (int nt = 0; nt < NTC; nt++) acc[nt][0] = acc[nt][1] = acc[nt][2] = acc[nt][3] = 0.f;
-#pragma unroll
+#pragma unroll 2
         for (int s16 = 0; s16 < kAttnTile / 16; s16++) {
             uint32_t r[4];
             ldsm4_trans(r, vrow + (size_t)s16 * 16 * L::kValStride);
