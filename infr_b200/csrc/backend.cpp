@@ -509,8 +509,7 @@ Status CudaBackend::q2_linear(const uint8_t *w, float *y, uint32_t out_f, const 
 bool CudaBackend::tc_rows(int dtype, uint32_t m, uint32_t in_f, uint64_t out_f) const {
     if (reference_ || (dtype != DT_Q4K && dtype != DT_Q6K) || m == 0 || out_f == 0) return false;
     const bool wide = wide_applies(dtype, m, in_f, out_f, INFR_ACT_INT8);
-    if (wide ? !tc_wins(dtype, m, in_f, out_f) : !tc_applies(dtype, m, in_f, out_f, INFR_ACT_INT8)) return false;
-    return !(dtype == DT_Q4K && mmq_impl_ == 1);
+    return wide ? tc_wins(dtype, m, in_f, out_f) : tc_applies(dtype, m, in_f, out_f, INFR_ACT_INT8);
 }
 
 Status CudaBackend::linear_from(const RowSource &src, int dtype, const uint8_t *w1, float *y1, uint32_t out_f1, const uint8_t *w2, float *y2, uint32_t out_f2, uint32_t m,
@@ -899,7 +898,8 @@ Status CudaBackend::moe_ffn(const MoeArgs &a) {
     const size_t o_xq = take(rows * ne), o_xd = take(rows * (ne / 256) * 4), o_xs = take(rows * (ne / 32) * 4);
     const size_t o_xs16 = any_q6 ? take(rows * (ne / 16) * 4) : 0, o_as16 = any_q6 ? take(n_pairs * (nff / 16) * 4) : 0;
     const size_t o_g = take(n_pairs * nff * 4), o_u = take(n_pairs * nff * 4);
-    const size_t o_aq = take(n_pairs * nff), o_ad = take(n_pairs * (nff / 256) * 4), o_as = take(n_pairs * (nff / 32) * 4);
+    auto items_only = [&](size_t bytes) { return grouped_gemm ? 0 : take(bytes); };
+    const size_t o_aq = items_only(n_pairs * nff), o_ad = items_only(n_pairs * (nff / 256) * 4), o_as = items_only(n_pairs * (nff / 32) * 4);
     const size_t o_y = take(n_pairs * ne * 4);
     const size_t o_px = grouped_gemm ? take(gemm_tc_grouped_record_bytes(slab, (int)max_slabs, (int)ne)) : 0;
     const size_t o_pa = grouped_gemm ? take(gemm_tc_grouped_record_bytes(slab, (int)max_slabs, (int)nff)) : 0;
