@@ -1025,9 +1025,8 @@ def run_b200(args):
                                    f"in mmq_sharded / tp_decode_step / ep_moe)") if world > 1 else "1 GPU",
                    "fraction_of_8TBs": value / world / 8000.0},
         "roofline": {"bound": "hbm", "achieved": kern_gbs, "peak": hbm_peak, "unit": "GB/s", "frac": kern_gbs / hbm_peak,
-                     # dram__bytes_read.sum + dram__bytes_write.sum of this kernel at this shape from the committed
-                     # ncu capture (profiles/gemv_q4k_mma_4096x4096_m1.md): 9 467 136 + 0 bytes per launch
-                     "traffic": 9467136, "peak_source": f"{peak_src} HBM copy bandwidth",
+                     # dram__bytes_read.sum + dram__bytes_write.sum of this kernel at this shape, under ncu: 9 460 992 + 0 bytes a launch
+                     "traffic": 9460992, "peak_source": f"{peak_src} HBM copy bandwidth",
                      "kernel": "gemv_row_kernel (m=1, pre-quantised activations)", "kernel_us": ms_kern * 1e3 / (steps * ROT),
                      "alg_bytes_per_launch": C1_BYTES},
         "e2e": {"value": total_bytes * e2e_steps / e2e_s / 1e9, "unit": "GB/s",

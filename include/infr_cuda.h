@@ -262,8 +262,9 @@ INFR_API int32_t infr_cuda_gemv_q8(infr_cuda_ctx *ctx, int32_t dtype, const infr
                                    const infr_cuda_buf *qs, const infr_cuda_buf *d, const infr_cuda_buf *sums,
                                    const infr_cuda_buf *sums16, infr_cuda_buf *y, uint32_t m, uint32_t in_f,
                                    uint32_t out_f);
-/* Two weights of one format against the same quantised rows (infr_cuda_gemv_q8 twice; for at most 24 rows the same bits,
- * above equal up to the order of f32 sums, see infr_cuda_linear_pair): q and k, or gate and up, of a decode step.  The reference gets the same effect from `w_off` slices of one fused weight
+/* Two weights of one format against the same quantised rows: q and k, or gate and up, of a decode step.  Results as from
+ * infr_cuda_gemv_q8 twice, with the same bits where infr_cuda_linear_pair says so of two infr_cuda_linear calls (Q2_0: up to 8 rows,
+ * all that this call takes).  The reference gets the same effect from `w_off` slices of one fused weight
  * (crates/infr-llama/src/seam/runner.rs:3445-3461, :3842-3879); here the two weights may live anywhere, and Q4_K
  * pairs run as ONE launch (a decode step pays a fixed few microseconds per dependent launch). */
 INFR_API int32_t infr_cuda_gemv_q8_pair(infr_cuda_ctx *ctx, int32_t dtype, const infr_cuda_buf *w1, uint64_t w_off1, infr_cuda_buf *y1,

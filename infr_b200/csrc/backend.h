@@ -108,7 +108,8 @@ public:
     Status linear(int dtype, const uint8_t *w, const float *x, float *y, uint32_t m, uint32_t in_f,
                   uint32_t out_f, int act);
     // Two Linears of one weight format on the same rows (q and k, gate and up): the rows are quantised once, and laid
-    // out once for the tensor-memory GEMM; results are those of two `linear` calls.
+    // out once for the tensor-memory GEMM.  Results are those of two `linear` calls, but for the K split that the heights choose together (Q4_K up
+    // to 8 rows, the GEMMs): last bits.
     Status linear_pair(int dtype, const uint8_t *w1, float *y1, uint32_t out_f1, const uint8_t *w2, float *y2, uint32_t out_f2, const float *x,
                        uint32_t m, uint32_t in_f, int act);
     // One-row Linears in one launch (gemv_row.cu).  *taken false: nothing was launched (the kernel does not take the call, spans overlap, or

@@ -67,8 +67,9 @@ struct Cfg {
     // every operand slot until the second pass: 14336 -> 4096, 113 rows 50.6 us, in one pass 46.9;
     // 1000 rows 296, 254.)
     static constexpr int kJobBuf = FMT == F_Q6 && TN == 128 ? 1 : 2;
-    // Tensor memory that only one job has (Q4_K: the minima's sums) goes back as early as can be: Q4_K 4096 -> 14336, 113 rows 31.3 -> 30.9 us, 512
-    // rows 84.1 -> 82.6.  With two jobs' worth the fold is off the path: at 64 rows it cost 2 %.
+    // Tensor memory that only one job has (Q4_K: the minima's sums) goes back as early as can be: Q4_K in a chain, 4096 -> 14336, 113 rows 28.8 ->
+    // 28.5 us, 512 rows 80.0 -> 79.3, 14336 -> 4096, 1000 rows 171 -> 168; a call that waits for the one before it gains nothing (512 rows 90).
+    // With two jobs' worth the fold is off the path: at 64 rows it cost 2 %.
     static constexpr bool kEarly = TN == 128;
     static constexpr int kRowBytes = FMT == F_Q6 ? 240 : 144;
     static constexpr int kRaw = kTM * kRowBytes;

@@ -22,7 +22,8 @@
 // rows): Q4_K 4096 -> 4096 3.5 / 4.4 -> 3.6 / 3.9, 4096 -> 14336 7.5 / 9.4 -> 7.8 / 8.0, 14336 -> 4096 8.5 / 11.5 -> 8.0 / 9.9;  Q6_K
 // 4096 -> 4096 5.3 / 6.8 -> 4.5 / 4.5, 4096 -> 14336 13.1 / 15.1 -> 10.1 / 10.1, 4096 -> 128256 79 -> 65;  Q2_0 4096 -> 4096 4.5 / 5.6 -> 3.1 / 4.0,
 // 14336 -> 4096 8.4 / 10.4 -> 7.0 / 9.6, 4096 -> 128256 54 -> 33.  Between other launches (the decode step of an 8B model) the Q4_K shapes gain
-// more: their CTAs leave room for the launch before.  Lost: long Q4_K rows on few tiles, 5632 -> 2048 3.4 -> 3.7.
+// more: their CTAs leave room for the launch before.  Long rows of few tiles, codes of more than 16 blocks and rows whose terms leave no room are
+// faster there still and go there (row_first in gemv_mma.cu, the lines in launch_gemv_q6_mma and CudaBackend::linear).
 // What bounds it: small matrices the chain from one launch to the next (1 us) and one round trip to L2 for the activations (0.3 us);
 // large ones memory (4096 -> 128256 at 0.92 of the measured copy rate, Q6_K 1.0); Q2_0 the integer pipe (64 masks a unit, half rate).
 #include <cuda.h>
@@ -707,7 +708,7 @@ __global__ void __launch_bounds__(kRowWarps<DT, ONE> * 32, kChains<DT, ONE> ? 4 
                 if (q == 0) store(i, v);
             }
         } else {
-            // A thread a result, on two warps that change from batch to batch; the others go on (two buffers of sums).
+            // A thread a result, on two warps (Q6_K: one) that change from batch to batch; the others go on (two buffers of sums).
             for (int i = (int)threadIdx.x - batch * kCols % (int)blockDim.x; i < nb * kRowTile; i += blockDim.x) {
                 if (i < 0) i += blockDim.x;
                 if (i >= nb * kRowTile) break;

@@ -1,5 +1,6 @@
 """One row against Q4_K, Q6_K and Q2_0 weights (the GEMV whose matrix-instruction columns are sub-blocks): f32 rows and quantised rows,
-one matrix and two, the same bits in every form, and the CPU restatement's values.
+one matrix and two, the same bits in every form (the heights are such that the K split of a Q4_K pair, which both heights choose, is that
+of two calls), and the CPU restatement's values.
 
 Sizes: rows of one K unit, of as many units as a CTA has warps (16 x 256, 8 x 512, 16 x 512), of one unit more, of several per warp with the
 last warp short; heights of part of a 16-row tile, one tile and its neighbours, and more tiles than CTAs (several flushes of partial sums)."""
