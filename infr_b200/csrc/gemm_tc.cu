@@ -5,7 +5,8 @@
 // while they stay below 2^24, their f32 sums are integers.  The operands are chosen so that every partial sum of a block does:
 //   Q4_K  (q - 8) * sc    <= 8 * 63 = 504        one multiply per weight; an int8 form needs two (q * (sc & 7), q * (sc >> 3)).  A block's
 //                                                 sum stays below 504 * 127 * 256 < 2^24 (q * sc: 3.1e7); the last instruction of a block
-//                                                 adds 8 * sum_s sc_s * bsum_s (K = 16, as below): one rounding, where |sum| > 2^24
+//                                                 adds 8 * sum_s sc_s * bsum_s (K = 16, as below): one rounding, where |sum| > 2^24.
+//                                                 (All of it times 2^-14, which the row scale takes back: unpack_q4.)
 //   Q4_K  m_s, 64h + l    the block minimum: sum_s m_s * bsum_s as ONE K = 16 instruction (8 sub-blocks x {64h, l})
 //   Q6_K  sl * (q - 32), sh * (q - 32)            sc = 16 sh + sl, one accumulator each (a block's |L| <= 15 * 32 * 127 * 256 and |H|
 //                                                 <= 8 * 32 * 127 * 256 stay below 2^24; sums of sc * (q - 32) reach 1.3e8); sum = 16 H + L
@@ -17,9 +18,9 @@
 //               = 64 operand values, each published by itself; two teams (four warps = 128 rows) fill the two halves of a block
 //   kEpi warps  epilogue: tensor-memory lane quarter x column part; folds a job's sums into running f32 registers
 //   1 warp      block headers: row scales for the epilogue; Q4_K: minima and scales as operands of the two K = 16 instructions
-//   2 producers raw rows by tiled TMA (zero-filled past the matrix); activation operands by plain bulk copies (laid out
-//               per token tile by gemm_tc_prep_kernel, so that a unit's operand is one contiguous run)
-//   1 issuer    one elected thread that runs the whole loop.  (A warp that runs the loop and issues under `lane == 0` spends 54
+//   1 producer  raw rows by tiled TMA (zero-filled past the matrix); a job's activation operands by two plain bulk copies (laid out
+//               per token tile by gemm_tc_prep_kernel, so that they are contiguous)
+//   2 issuers   in turn a job; one elected thread that runs the whole loop.  (A warp that runs the loop and issues under `lane == 0` spends 54
 //               cycles on each tcgen05.mma, under an elect around a batch 20, a lone thread 8: clock64 around 8 instructions.)
 // A raw stage is given back when it has been unpacked; what the epilogue needs of a block (row and token scales) has rings of its
 // own, so that the weights' ring covers the memory's latency and not the whole pipeline's.
@@ -34,8 +35,15 @@
 // the bytes part (5 integer instructions for 4 weights, 7 before), the offset is inside the multiply-add, rows are read in 8-byte words from
 // a pitch of 240 bytes (no conflicts, one level of selects less) and the two teams' slots are multiplied in turn.  Cold weights, us, before:
 // 4096 -> 14336, 33..64 rows 42, 53; 113 rows 52, 57;  14336 -> 4096, 64 rows 42, 52; 113 rows 51, 55; 1000 rows 296, 318 (and one pass, kJobBuf, after that).
-// What bounds it: issue slots and waits.  At 128 tokens a Q4_K job takes ~2550 cycles, its MMAs
-// 1150 (tensor pipe 45 % busy); the warps issue 6670 instructions a job, 0.66 a cycle and scheduler.
+// What bounds it: every role is a chain of dependent instructions and of barriers that cost its warp 100 to 200 cycles each, seen or not; a
+// barrier between two roles is therefore as dear as what it guards.  Hence one barrier for a job's activation operands, none for giving them
+// back where the accumulators' says as much, one epilogue warp that waits for the others (they stand at a named barrier), two issuers (one was
+// busy for 2400 cycles of a job's 2550), and as few instructions as can be for a weight.  Before / after, us, cold weights, back to back: Q4_K
+// 4096 -> 28672, 32 rows 34.2 / 31.1, 113 rows 50.8 / 47.2; 4096 -> 14336, 512 rows 81 / 75; Q6_K 14336 -> 4096, 512 rows 148 / 137.
+// At 128 tokens a Q4_K job takes ~2050 cycles, its MMAs 1150; the warps issue 6540 instructions (10060 before, most of them polls).
+// Tried: 16 unpack and 8 epilogue warps (4 % slower), waits as tight loops in PTX (30 to 100 % slower: they poll more often), sleeping
+// between polls (1 to 15 % slower), the issuer's loop not unrolled (17 % slower), a look at all of a job's barriers at once (no gain), a chunk's
+// tensor-memory load during the fold of the one before it (spills).
 // Every wait is bounded: on expiry the role raises a CTA flag and a status word, every role leaves its loop, copies in
 // flight are drained and the tensor memory is freed.
 #include <cuda.h>
@@ -87,7 +95,7 @@ struct Cfg {
     static constexpr int kEpi = TN == 32 ? 4 : (TN == 128 ? 16 : 8);
     static constexpr int kCols = TN / (kEpi / 4);                    // output columns of an epilogue thread
     static constexpr int kChunk = TN == 64 && FMT == F_Q4 ? 16 : 8;  // columns per tensor-memory load (registers)
-    static constexpr int W_HEAD = kUnpack + kEpi, W_RAW = W_HEAD + 1, W_ACT = W_HEAD + 2, W_MMA = W_HEAD + 3, kWarps = W_HEAD + 4;
+    static constexpr int W_HEAD = kUnpack + kEpi, W_LOAD = W_HEAD + 1, W_MMA = W_HEAD + 2, kWarps = W_HEAD + 4;
     static constexpr int kCtas = TN == 32 && FMT != F_Q6 ? 2 : 1;
     // tensor-memory columns: accumulators of two jobs (one where there is no room), block-minimum sums of two jobs (one where there is no room), operands
     static constexpr int kMBuf = FMT == F_Q4 ? (TN == 128 ? 1 : 2) : 0;
@@ -96,9 +104,11 @@ struct Cfg {
     static constexpr uint32_t kCols0 = kColA + 2 * kSlots * 32;
     static constexpr uint32_t kTmem = kCols0 <= 256 ? 256 : 512;
     // barriers
-    static constexpr int B_SFULL = 0, B_SFREE = B_SFULL + kStages, B_XFULL = B_SFREE + kStages, B_XFREE = B_XFULL + kNX, B_BFULL = B_XFREE + kNX,
-                         B_BFREE = B_BFULL + kNB, B_AFULL = B_BFREE + kNB, B_AFREE = B_AFULL + 2 * kSlots, B_HEAD = B_AFREE + 2 * kSlots,
-                         B_ACCRDY = B_HEAD + 2, B_ACCFREE = B_ACCRDY + 2, B_MFREE = B_ACCFREE + 2, B_DRAIN = B_MFREE + 1, B_COUNT = B_DRAIN + 1;
+    static constexpr int kJB = kNB / kUnits;                         // jobs whose activation operands fit
+    static constexpr bool kOwnB = !(kJobBuf == 2 && kJB == 2);       // else B_ACCRDY says that a job's activation operands have been read
+    static constexpr int B_SFULL = 0, B_SFREE = B_SFULL + kStages, B_XFULL = B_SFREE + kStages, B_XFREE = B_XFULL + kNX,
+                         B_BFREE = B_XFREE + kNX, B_AFULL = B_BFREE + kJB, B_AFREE = B_AFULL + 4 * kUse, B_HEAD = B_AFREE + 2 * kSlots,
+                         B_ACCRDY = B_HEAD + 2, B_ACCFREE = B_ACCRDY + 2, B_MFREE = B_ACCFREE + 2, B_DRAIN = B_MFREE + 1, B_COUNT = B_DRAIN + 2;
     static_assert(kCols0 <= 512 && (kCtas == 1 || kCols0 <= 256), "tensor memory");
     static_assert(kSmem <= (kCtas == 2 ? 111 : 226) * 1024, "shared memory");
     static_assert(kWarps <= 32 && kNB % kUnits == 0, "");
@@ -181,6 +191,17 @@ __device__ __forceinline__ bool wait_warp(uint32_t bar, uint32_t parity, volatil
     return __all_sync(0xffffffffu, wait_bar(bar, parity, dead));
 }
 
+// Named barrier 1 of N threads; true where `ok` is true in all of them.
+template <int N>
+__device__ __forceinline__ bool bar_and(bool ok) {
+    uint32_t r;
+    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 q, %1, 0;\n\tbarrier.cta.red.and.aligned.pred p, 1, %2, q;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                 : "=r"(r)
+                 : "r"((uint32_t)ok), "n"(N)
+                 : "memory");
+    return r != 0;
+}
+
 __device__ __forceinline__ void tma2(uint32_t dst, const CUtensorMap *map, int x, int y, uint32_t bar) {
     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
                  "l"(map), "r"(x), "r"(y), "r"(bar)
@@ -212,8 +233,8 @@ __device__ __forceinline__ uint32_t h2add(uint32_t a, uint32_t b) {
 }
 __device__ __forceinline__ constexpr uint32_t dup(uint32_t h) { return h | (h << 16); }
 // f16 bit patterns of the small constants used below (integers and powers of two)
-constexpr uint32_t H_1024 = 0x6400, H_N1024 = 0xE400, H_N1152 = 0xE480, H_64 = 0x5400, H_N72 = 0xD480, H_N8192 = 0xF000, H_1_4 = 0x3400, H_1_64 = 0x2400,
-                   H_1 = 0x3C00, H_N1032 = 0xE408, H_N1056 = 0xE420;
+constexpr uint32_t H_1024 = 0x6400, H_N1024 = 0xE400, H_N1152 = 0xE480, H_64 = 0x5400, H_N1032 = 0xE408, H_N1056 = 0xE420, H_2M14 = 0x0400,
+                   H_N2M11 = 0x9000, H_NHALF = 0xB800;
 
 // (a & m) | c in one instruction: with m and c in registers.  As constants they would be two immediates, which one LOP3 cannot take.
 __device__ __forceinline__ uint32_t and_or(uint32_t a, uint32_t m, uint32_t c) {
@@ -232,19 +253,21 @@ __device__ __forceinline__ uint32_t in_reg(uint32_t v) {
     return v;
 }
 
-// Q4_K: 64 elements = two sub-blocks in 8 words, scales s0 (low nibbles) and s1 (high nibbles); value = (q - 8) * scale.
+// Q4_K: 64 elements = two sub-blocks in 8 words, scales s0 (low nibbles) and s1 (high nibbles); value = (q - 8) * scale * 2^-14.
 // Operand values leave in the order (0, 2, 1, 3) of every four elements; gemm_tc_prep_kernel lays the activations out the same way.
-// m = 0x00F000F0, k = the f16 of 64 twice (in_reg)
-__device__ __forceinline__ void unpack_q4(const uint32_t *w, uint32_t s0, uint32_t s1, uint32_t m, uint32_t k, uint32_t (&o)[32]) {
-    const uint32_t a0 = h2add(dup(H_1024) | s0 * 0x10001u, dup(H_N1024)), a1 = h2add(dup(H_1024) | s1 * 0x10001u, dup(H_N1024));
-    const uint32_t c0 = h2mul(a0, dup(H_N72)), c1 = h2mul(a1, dup(H_N72));  // (64 + q) * sc - 72 * sc: one rounding, exact
+// A nibble alone in a 16-bit half IS an f16: q * 2^-24 (subnormal) at bit 0, q * 2^-20 at bit 4.  With the scale times 2^10 and 2^6 one
+// fused multiply-add gives q * sc * 2^-14 - 8 * sc * 2^-14, exact and not below the smallest normal: 9 instructions for 8 weights.  (A
+// nibble under the f16 of 64, moved to bit 4, took 11: 4096 -> 28672 at 32 rows 33.0 -> 31.0 us, 512 rows of 4096 -> 14336 78.8 -> 76.7.)
+__device__ __forceinline__ void unpack_q4(const uint32_t *w, uint32_t s0, uint32_t s1, uint32_t (&o)[32]) {
+    const uint32_t t0 = h2add(dup(H_1024) | s0 * 0x10001u, dup(H_N1024)), t1 = h2add(dup(H_1024) | s1 * 0x10001u, dup(H_N1024));
+    const uint32_t a0 = h2mul(t0, dup(H_1024)), a1 = h2mul(t1, dup(H_64)), c0 = h2mul(t0, dup(H_N2M11)), c1 = h2mul(t1, dup(H_N2M11));
 #pragma unroll
     for (int i = 0; i < 8; i++) {
-        const uint32_t v = w[i];  // a nibble at bit 4 under the f16 of 64 is 64 + q
-        o[2 * i] = h2fma(and_or(v << 4, m, k), a0, c0);
-        o[2 * i + 1] = h2fma(and_or(v >> 4, m, k), a0, c0);
-        o[16 + 2 * i] = h2fma(and_or(v, m, k), a1, c1);
-        o[17 + 2 * i] = h2fma(and_or(v >> 8, m, k), a1, c1);
+        const uint32_t v = w[i], x = v >> 8;
+        o[2 * i] = h2fma(v & 0x000F000Fu, a0, c0);
+        o[2 * i + 1] = h2fma(x & 0x000F000Fu, a0, c0);
+        o[16 + 2 * i] = h2fma(v & 0x00F000F0u, a1, c1);
+        o[17 + 2 * i] = h2fma(x & 0x00F000F0u, a1, c1);
     }
 }
 
@@ -503,8 +526,8 @@ __global__ void __launch_bounds__(Cfg<FMT, TN>::kWarps * 32, Cfg<FMT, TN>::kCtas
         for (int i = 0; i < K::B_COUNT; i++) {
             int cnt = 1;
             if (i >= K::B_SFREE && i < K::B_XFULL) cnt = K::kUnpack + 1;
-            if (i >= K::B_XFREE && i < K::B_BFULL) cnt = K::kEpi;
-            if (i >= K::B_AFULL && i < K::B_AFREE) cnt = 4;
+            if (i >= K::B_XFREE && i < K::B_BFREE) cnt = K::kEpi;
+            if (i >= K::B_AFULL && i < K::B_AFREE) cnt = 4;  // [job's parity][team][use]: a barrier belongs to one issuer, who sees all of its phases
             if (i >= K::B_ACCFREE && i <= K::B_MFREE) cnt = K::kEpi;
             asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(su32(&bars[i])), "r"(cnt));
         }
@@ -550,144 +573,140 @@ __global__ void __launch_bounds__(Cfg<FMT, TN>::kWarps * 32, Cfg<FMT, TN>::kCtas
         *dead = 1;
     };
 
-    if (warp == K::W_RAW) {
-        // ------------------------------------------------------------------ weights
-        // they do not depend on the kernels before this one: the first stages are fetched before the wait
-        int pre = 0;
-        if (lane == 0 && !grp.slab_expert && (int)blockIdx.x < n_items()) {
-            const Tile t = tile_of(blockIdx.x);
-            const bool second = t.rt >= rt1;
-            for (; pre < K::kStages && t.b0 + pre < t.b1; pre++) {
-                expect_tx(bar(K::B_SFULL + pre), K::kRaw);
-                tma2(su32(raw0 + pre * K::kRaw), second ? &map_w2 : &map_w, stage_x(t.b0 + pre), (second ? t.rt - rt1 : t.rt) * kTM,
-                     bar(K::B_SFULL + pre));
-            }
+    if (warp == K::W_LOAD) {
+        // ------------------------------------------------------------------ weights, activation operands
+        struct Jobs {  // the jobs of this CTA, one after the other
+            int i, b;
+            Tile t;
+        };
+        int n = 0;
+        auto first = [&](Jobs &c) {
+            c.i = blockIdx.x;
+            if (c.i < n) c.t = tile_of(c.i), c.b = c.t.b0;
+        };
+        auto next = [&](Jobs &c) {
+            if (++c.b == c.t.b1 && (c.i += gridDim.x) < n) c.t = tile_of(c.i), c.b = c.t.b0;
+        };
+        Jobs cw{};
+        int jw = 0;
+        auto load_w = [&]() {  // the next job's weights
+            const int s = jw % K::kStages;
+            const bool second = cw.t.rt >= rt1;
+            const int row0 = (grp.slab_expert ? grp.slab_expert[cw.t.tt] * m1.out_f : 0) + (second ? cw.t.rt - rt1 : cw.t.rt) * kTM;
+            expect_tx(bar(K::B_SFULL + s), K::kRaw);
+            tma2(su32(raw0 + s * K::kRaw), second ? &map_w2 : &map_w, stage_x(cw.b), row0, bar(K::B_SFULL + s));
+            jw++;
+            next(cw);
+        };
+        // weights do not depend on the kernels before this one: the first stages are fetched before the wait
+        if (lane == 0 && !grp.slab_expert) {
+            n = n_items();
+            first(cw);
+            while (jw < K::kStages && cw.i < n) load_w();
         }
         __syncwarp();
         pdl_wait();
         if (lane == 0) {
-            const int n = n_items();
+            if (grp.slab_expert) {
+                n = n_items();
+                first(cw);
+                while (jw < K::kStages && cw.i < n) load_w();
+            }
+            Jobs ca;
+            first(ca);
             int js = 0;
             bool ok = true;
-            for (int i = blockIdx.x; i < n && ok; i += gridDim.x) {
-                const Tile t = tile_of(i);
-                const bool second = t.rt >= rt1;
-                const CUtensorMap *mp = second ? &map_w2 : &map_w;
-                const int row0 = (grp.slab_expert ? grp.slab_expert[t.tt] * m1.out_f : 0) + (second ? t.rt - rt1 : t.rt) * kTM;
-                for (int b = t.b0; b < t.b1; b++, js++) {
-                    if (js < pre) continue;
-                    const int s = js % K::kStages;
-                    if (js >= K::kStages && !(ok = wait_bar(bar(K::B_SFREE + s), (uint32_t)((js / K::kStages - 1) & 1), dead))) break;
-                    expect_tx(bar(K::B_SFULL + s), K::kRaw);
-                    tma2(su32(raw0 + s * K::kRaw), mp, stage_x(b), row0, bar(K::B_SFULL + s));
+            for (; ca.i < n; js++, next(ca)) {
+                const int x = js % K::kNX;
+                const size_t rec = (size_t)ca.t.tt * nst + ca.b;
+                if (js >= K::kNX && !(ok = wait_bar(bar(K::B_XFREE + x), (uint32_t)((js / K::kNX - 1) & 1), dead))) break;
+                if (js >= K::kJB) {  // the operands of the job that had the place before have been read
+                    const int p = js - K::kJB;
+                    if (!(ok = K::kOwnB ? wait_bar(bar(K::B_BFREE + js % K::kJB), (uint32_t)(p / K::kJB) & 1u, dead)
+                                        : wait_bar(bar(K::B_ACCRDY + (p & 1)), (uint32_t)(p >> 1) & 1u, dead)))
+                        break;
+                }
+                expect_tx(bar(K::B_XFULL + x), K::kExtra + K::kUnits * K::kUnitBytes);
+                bulk(su32(bring + (js % K::kJB) * K::kUnits * K::kUnitBytes), units + rec * K::kUnits * K::kUnitBytes, K::kUnits * K::kUnitBytes, bar(K::B_XFULL + x));
+                bulk(su32(ext0 + x * K::kExtra), extra + rec * K::kExtra, K::kExtra, bar(K::B_XFULL + x));
+                // the job before is unpacked by the time that the one before that has been multiplied
+                if (js >= 1 && cw.i < n) {
+                    if (!(ok = wait_bar(bar(K::B_SFREE + (js - 1) % K::kStages), (uint32_t)((js - 1) / K::kStages) & 1u, dead))) {
+                        js++;
+                        break;
+                    }
+                    load_w();
                 }
             }
             if (!ok) fail(5u);
             if (*dead) {
                 // copies in flight land before the CTA's shared memory is released
-                const int end = js > pre ? js : pre;
-                for (int k = end > K::kStages ? end - K::kStages : 0; k < end; k++)
+                for (int k = jw > K::kStages ? jw - K::kStages : 0; k < jw; k++)
                     for (uint32_t i = 0; i < (1u << 14) && !try_bar(bar(K::B_SFULL + k % K::kStages), (uint32_t)((k / K::kStages) & 1)); i++) {
                     }
-            }
-        }
-    } else if (warp == K::W_ACT) {
-        // ------------------------------------------------------------------ activation operands
-        pdl_wait();
-        if (lane == 0) {
-            const int n = n_items();
-            int js = 0, ju = 0;
-            bool ok = true;
-            for (int i = blockIdx.x; i < n && ok; i += gridDim.x) {
-                const Tile t = tile_of(i);
-                for (int b = t.b0; b < t.b1 && ok; b++) {
-                    const int x = js % K::kNX;
-                    const size_t rec = (size_t)t.tt * nst + b;
-                    if (js >= K::kNX && !(ok = wait_bar(bar(K::B_XFREE + x), (uint32_t)((js / K::kNX - 1) & 1), dead))) break;
-                    expect_tx(bar(K::B_XFULL + x), K::kExtra);
-                    bulk(su32(ext0 + x * K::kExtra), extra + rec * K::kExtra, K::kExtra, bar(K::B_XFULL + x));
-                    js++;
-                    for (int u = 0; u < K::kUnits; u++, ju++) {
-                        const int q = ju % K::kNB;
-                        if (ju >= K::kNB && !(ok = wait_bar(bar(K::B_BFREE + q), (uint32_t)((ju / K::kNB - 1) & 1), dead))) break;
-                        expect_tx(bar(K::B_BFULL + q), K::kUnitBytes);
-                        bulk(su32(bring + q * K::kUnitBytes), units + (rec * K::kUnits + u) * K::kUnitBytes, K::kUnitBytes, bar(K::B_BFULL + q));
-                    }
-                }
-            }
-            if (!ok) fail(5u);
-            if (*dead) {
                 for (int k = js > K::kNX ? js - K::kNX : 0; k < js; k++)
                     for (uint32_t i = 0; i < (1u << 14) && !try_bar(bar(K::B_XFULL + k % K::kNX), (uint32_t)((k / K::kNX) & 1)); i++) {
                     }
-                for (int k = ju > K::kNB ? ju - K::kNB : 0; k < ju; k++)
-                    for (uint32_t i = 0; i < (1u << 14) && !try_bar(bar(K::B_BFULL + k % K::kNB), (uint32_t)((k / K::kNB) & 1)); i++) {
-                    }
             }
         }
-    } else if (warp == K::W_MMA) {
-        // ------------------------------------------------------------------ MMA issuer: one thread, all of the loop
+    } else if (warp >= K::W_MMA) {
+        // ------------------------------------------------------------------ MMA issuers, in turn a job: one thread, all of the loop
+        const int me = warp - K::W_MMA;
         pdl_wait();
         if (elect_one()) {
             const uint32_t idesc = (1u << 4) | ((uint32_t)(TN >> 3) << 17) | ((uint32_t)(kTM >> 4) << 24);
             const uint64_t bd0 = mk_desc(su32(bring), TN * 16);
             const int n = n_items();
             int j = 0;               // jobs of this CTA, over all tiles
-            uint32_t q = 0, qp = 0;  // activation ring: next unit's place and phase
             bool ok = true;
             for (int i = blockIdx.x; i < n && ok; i += gridDim.x) {
                 const Tile t = tile_of(i);
                 for (int b = t.b0; b < t.b1; b++, j++) {
                     const int s = j & 1;
+                    if (s != me) continue;
                     const uint32_t jp = (uint32_t)(j >> 1) & 1u;
                     const int sa = K::kJobBuf == 2 ? s : 0;  // its accumulators
+                    const uint32_t q = (uint32_t)(j % K::kJB);  // its place in the activation ring
                     const uint32_t td = tmem + (uint32_t)(sa * K::kAcc * TN);
-                    // the job that had them before
-                    if (j >= K::kJobBuf && !(ok = wait_bar(bar(K::B_ACCFREE + sa), K::kJobBuf == 2 ? jp ^ 1u : (uint32_t)(j - 1) & 1u, dead))) break;
+                    // what the header warp has seen: its own operands, and the accumulators given back by the job that had them before
+                    if (!(ok = wait_bar(bar(K::B_HEAD + s), jp, dead))) break;
+                    if (!(ok = wait_bar(bar(K::B_XFULL + j % K::kNX), (uint32_t)(j / K::kNX) & 1u, dead))) break;
 #pragma unroll
-                    for (int uu = 0; uu < K::kUnits; uu++) {
-                        const int u = K::kUnits == 4 ? (uu >> 1) + (uu & 1) * 2 : uu;  // the teams' slots in turn: both get theirs back early
-                        if (!(ok = wait_bar(bar(K::B_BFULL + q + u), qp, dead))) break;
-                        const uint64_t bd = bd0 + (uint64_t)((q + u) * (uint32_t)(K::kUnitBytes / 16));
-                        constexpr int kTeamUnits = K::kUnits / 2;
-                        const int team = u / kTeamUnits;
+                    for (int st = 0; st < 2 * K::kUnits; st++) {
+                        // (Q6_K: the teams' slots in turn, both get theirs back early)
+                        const int k8 = K::kUnits == 4 ? (st >> 2) * 2 + ((st >> 1) & 1) * 4 + (st & 1) : st;
+                        const int u = k8 >> 1, h = k8 & 1, team = k8 / K::kUse;
+                        const uint64_t bd = bd0 + (uint64_t)((q * K::kUnits + u) * (uint32_t)(K::kUnitBytes / 16));
+                        const int sl = team * K::kSlots + (j * K::kUse + k8 % K::kUse) % K::kSlots;
+                        if (!(ok = wait_bar(bar(K::B_AFULL + (s * 2 + team) * K::kUse + k8 % K::kUse), jp, dead))) break;
+                        tc_fence_after();
+                        const uint32_t ta = tmem + K::kColA + (uint32_t)(sl * 32);
 #pragma unroll
-                        for (int h = 0; h < 2; h++) {
-                            const int use = j * K::kUse + (u % kTeamUnits) * 2 + h, sl = team * K::kSlots + use % K::kSlots;
-                            if (!(ok = wait_bar(bar(K::B_AFULL + sl), (uint32_t)(use / K::kSlots) & 1u, dead))) break;
-                            tc_fence_after();
-                            const uint32_t ta = tmem + K::kColA + (uint32_t)(sl * 32);
-#pragma unroll
-                            for (int k = 0; k < 4; k++) {
-                                // Q6_K: the sl and the sh operands of a slot meet the same 32 activations
-                                const int pl = FMT == F_Q6 ? h * 4 + (k & 1) * 2 : h * 8 + k * 2;
-                                const uint32_t keep = (uint32_t)(uu > 0 || h > 0 || (K::kAcc == 2 ? (k & 1) : k > 0));
-                                mma_ta(td + (uint32_t)(K::kAcc == 2 ? (k >> 1) * TN : 0), ta + (uint32_t)(k * 8), bd + (uint64_t)(pl * TN), idesc, keep);
-                            }
-                            mma_commit(bar(K::B_AFREE + sl));
+                        for (int k = 0; k < 4; k++) {
+                            // Q6_K: the sl and the sh operands of a slot meet the same 32 activations
+                            const int pl = FMT == F_Q6 ? h * 4 + (k & 1) * 2 : h * 8 + k * 2;
+                            const uint32_t keep = (uint32_t)(st > 0 || (K::kAcc == 2 ? (k & 1) : k > 0));
+                            mma_ta(td + (uint32_t)(K::kAcc == 2 ? (k >> 1) * TN : 0), ta + (uint32_t)(k * 8), bd + (uint64_t)(pl * TN), idesc, keep);
                         }
-                        if (!ok) break;
-                        mma_commit(bar(K::B_BFREE + q + u));
+                        mma_commit(bar(K::B_AFREE + sl));
                     }
-                    q += K::kUnits;
-                    if (q == K::kNB) q = 0, qp ^= 1;
-                    if (!ok || !(ok = wait_bar(bar(K::B_HEAD + s), jp, dead))) break;
+                    if (!ok) break;
                     if (FMT == F_Q4) {
-                        const int x = j % K::kNX;
-                        if (!(ok = wait_bar(bar(K::B_XFULL + x), (uint32_t)(j / K::kNX) & 1u, dead))) break;
-                        const uint64_t xd = mk_desc(su32(ext0 + x * K::kExtra), TN * 16);
+                        const uint64_t xd = mk_desc(su32(ext0 + (j % K::kNX) * K::kExtra), TN * 16);
                         mma_sa(td, mk_desc(su32(amin + (s * 4 + 2) * kTM * 16), kTM * 16), xd, idesc, 1u);
+                        // (the other issuer's job; the one before that is folded, or B_HEAD would not be here)
                         if (K::kMBuf == 1 && j >= 1 && !(ok = wait_bar(bar(K::B_MFREE), (uint32_t)((j - 1) & 1), dead))) break;
                         tc_fence_after();
                         mma_sa(tmem + K::kColM + (uint32_t)(K::kMBuf == 2 ? s * TN : 0), mk_desc(su32(amin + s * 4 * kTM * 16), kTM * 16), xd, idesc, 0u);
                     }
+                    if (K::kOwnB) mma_commit(bar(K::B_BFREE + q));
                     mma_commit(bar(K::B_ACCRDY + sa));
                 }
             }
             if (!ok) fail(6u);
             // every issued MMA has completed before the tensor memory is freed
-            mma_commit(bar(K::B_DRAIN));
-            for (uint32_t i = 0; i < (1u << 20) && !try_bar(bar(K::B_DRAIN), 0u); i++) {
+            mma_commit(bar(K::B_DRAIN + me));
+            for (uint32_t i = 0; i < (1u << 20) && !try_bar(bar(K::B_DRAIN + me), 0u); i++) {
             }
         }
         __syncwarp();
@@ -715,12 +734,12 @@ __global__ void __launch_bounds__(Cfg<FMT, TN>::kWarps * 32, Cfg<FMT, TN>::kCtas
                 }
                 __syncwarp();
                 if (lane == 0) bar_arrive(bar(K::B_SFREE + ls));
-                // The job before last (one accumulator: the last job, whose barrier is the next to complete) has been multiplied, so its
-                // operands are read, and the jobs before it are folded: the rings' places are free.
+                // The job before last (one accumulator: the last job) has been multiplied and its accumulators are given back: the rings'
+                // places are free, and the issuer, who waits for this warp, need not wait for them.
                 if (K::kJobBuf == 2) {
-                    if (js >= 2 && !(ok = wait_warp(bar(K::B_ACCRDY + s), (uint32_t)(((js >> 1) - 1) & 1), dead))) break;
+                    if (js >= 2 && !(ok = wait_warp(bar(K::B_ACCFREE + s), (uint32_t)(((js >> 1) - 1) & 1), dead))) break;
                 } else {
-                    if (js >= 1 && !(ok = wait_warp(bar(K::B_ACCRDY), (uint32_t)((js - 1) & 1), dead))) break;
+                    if (js >= 1 && !(ok = wait_warp(bar(K::B_ACCFREE), (uint32_t)((js - 1) & 1), dead))) break;
                 }
 #pragma unroll
                 for (int k = 0; k < 4; k++) {
@@ -730,7 +749,7 @@ __global__ void __launch_bounds__(Cfg<FMT, TN>::kWarps * 32, Cfg<FMT, TN>::kCtas
                         const uint32_t n0 = h.z & 0x3F3F3F3Fu, n1 = ((h.w >> 4) & 0x0F0F0F0Fu) | ((h.z >> 2) & 0x30303030u);
                         const uint32_t c0 = h.y & 0x3F3F3F3Fu, c1 = (h.w & 0x0F0F0F0Fu) | ((h.y >> 2) & 0x30303030u);
                         auto two = [](uint32_t v, uint32_t sel) { return h2add(__byte_perm(v, 0x64646464u, sel), dup(H_N1024)); };
-                        auto two8 = [](uint32_t v, uint32_t sel) { return h2add(__byte_perm(v, 0x70707070u, sel), dup(H_N8192)); };  // 8 v
+                        auto two8 = [](uint32_t v, uint32_t sel) { return h2fma(__byte_perm(v, 0x70707070u, sel), dup(H_2M14), dup(H_NHALF)); };  // 8 v * 2^-14
                         const uint4 p = make_uint4(two(n0, 0x4140), two(n0, 0x4342), two(n1, 0x4140), two(n1, 0x4342));
                         const uint4 e = make_uint4(two8(c0, 0x4140), two8(c0, 0x4342), two8(c1, 0x4140), two8(c1, 0x4342));
                         uint4 *mp = reinterpret_cast<uint4 *>(amin + s * 4 * kTM * 16) + k * 32 + lane;
@@ -752,7 +771,7 @@ __global__ void __launch_bounds__(Cfg<FMT, TN>::kWarps * 32, Cfg<FMT, TN>::kCtas
         const int n = n_items();
         const int quarter = warp & 3, team = warp >> 2, row = quarter * 32 + lane;
         const uint32_t tl = tmem + ((uint32_t)(quarter * 32) << 16) + K::kColA;
-        const uint32_t km = in_reg(FMT == F_Q4 ? 0x00F000F0u : 0x003F003Fu), kc = in_reg(FMT == F_Q4 ? dup(H_64) : dup(H_1024));
+        const uint32_t km = in_reg(0x003F003Fu), kc = in_reg(dup(H_1024));  // (Q6_K)
         int js = 0;
         bool ok = true;
         // the team's slot of its use-th operand run: its previous MMAs are complete, it is filled, it is announced
@@ -764,7 +783,7 @@ __global__ void __launch_bounds__(Cfg<FMT, TN>::kWarps * 32, Cfg<FMT, TN>::kCtas
             tst_wait();
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) bar_arrive(bar(K::B_AFULL + sl));
+            if (lane == 0) bar_arrive(bar(K::B_AFULL + ((use / K::kUse & 1) * 2 + team) * K::kUse + use % K::kUse));
             return true;
         };
         for (int i = blockIdx.x; i < n && ok; i += gridDim.x) {
@@ -785,9 +804,9 @@ __global__ void __launch_bounds__(Cfg<FMT, TN>::kWarps * 32, Cfg<FMT, TN>::kCtas
                     const uint32_t w[16] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w, q2.x, q2.y, q2.z, q2.w, q3.x, q3.y, q3.z, q3.w};
                     const uint32_t sc = team ? (hdr.w & 0x0F0F0F0Fu) | ((hdr.y >> 2) & 0x30303030u) : hdr.y & 0x3F3F3F3Fu;
                     given_back();
-                    unpack_q4(w, sc & 0xFFu, (sc >> 8) & 0xFFu, km, kc, o);
+                    unpack_q4(w, sc & 0xFFu, (sc >> 8) & 0xFFu, o);
                     if (!(ok = put(js * 2, o))) break;
-                    unpack_q4(w + 8, (sc >> 16) & 0xFFu, sc >> 24, km, kc, o);
+                    unpack_q4(w + 8, (sc >> 16) & 0xFFu, sc >> 24, o);
                     if (!(ok = put(js * 2 + 1, o))) break;
                 } else {
                     // half block `team`: the low and then the high nibbles of its 64 bytes
@@ -828,13 +847,16 @@ __global__ void __launch_bounds__(Cfg<FMT, TN>::kWarps * 32, Cfg<FMT, TN>::kCtas
 #pragma unroll 1
             for (int b = t.b0; b < t.b1; b++, j++) {
                 const int x = j % K::kNX, s = K::kJobBuf == 2 ? j & 1 : 0;
-                if (!(ok = wait_warp(bar(K::B_XFULL + x), (uint32_t)((j / K::kNX) & 1), dead) &&
-                           wait_warp(bar(K::B_ACCRDY + s), (uint32_t)((K::kJobBuf == 2 ? j >> 1 : j) & 1), dead)))
-                    break;
+                // one warp waits (sixteen of them took 1500 instructions a job to look, Q6_K at 512 rows 148 -> 141 us), the others stand at the barrier
+                if (warp == K::kUnpack)
+                    ok = wait_bar(bar(K::B_XFULL + x), (uint32_t)((j / K::kNX) & 1), dead) &&
+                         wait_bar(bar(K::B_ACCRDY + s), (uint32_t)((K::kJobBuf == 2 ? j >> 1 : j) & 1), dead);
+                __syncwarp();
+                if (!(ok = bar_and<K::kEpi * 32>(ok))) break;
                 tc_fence_after();
                 const float *d8 = reinterpret_cast<const float *>(ext0 + x * K::kExtra + (FMT == F_Q4 ? 32 * TN : 0)) + col0;
                 const uint32_t hd = dring[(j % K::kRing) * kTM + row];
-                const u64 dw = f2_dup(h2f(hd)), nm = f2_dup(FMT == F_Q4 ? -h2f(hd >> 16) : 16.f);
+                const u64 dw = f2_dup(FMT == F_Q4 ? h2f(hd) * 16384.f : h2f(hd)), nm = f2_dup(FMT == F_Q4 ? -h2f(hd >> 16) : 16.f);
                 auto give_back = [&]() {
                     tc_fence_before();
                     __syncwarp();
