@@ -1,6 +1,7 @@
 // Device helpers shared by the GEMV kernels: vector loads, the unsigned x signed byte dot product,
 // Q4_K scale unpacking, and the shared-memory staging of quantised activations.
 #pragma once
+#include <algorithm>
 #include <cmath>
 #include <cuda_fp16.h>
 
@@ -135,17 +136,38 @@ __device__ __forceinline__ void stage_q8(const Q8Dev &a, int m, int M, int in_f,
 }
 
 
-// CTAs an item of a grouped launch: `items` expected, `slots` CTAs fit the device, `tiles` of the item go to `lanes` groups of warps of a CTA.
-// A CTA costs its tiles and what it takes before the first of them (staging the item's rows: about five tiles' time), and waves of CTAs come one
-// after the other.  How many items there are is only known on the device, so a wave is taken to be full a fiftieth before it is.
-inline int grouped_ctas(int items, int slots, int tiles, int lanes) {
-    int best = 1;
+// The tiles of this CTA of a grouped launch, counted over all items.
+struct GroupedShare {
+    int t0, n;
+};
+__device__ __forceinline__ GroupedShare grouped_share(int n_items, int tiles, bool per_item) {
+    if (per_item && (int)blockIdx.y >= n_items) return {0, 0};
+    const int all = per_item ? tiles : n_items * tiles, G = gridDim.x, base = all / G, rem = all - base * G, i = blockIdx.x;
+    return {(per_item ? (int)blockIdx.y * tiles : 0) + i * base + min(i, rem), base + (i < rem ? 1 : 0)};
+}
+
+// How the CTAs of a grouped launch share the work: `items` expected, `slots` CTAs fit the device, an item has `tiles`, `lanes` groups of warps of a CTA
+// take one each a round.  per_item: x CTAs an item; otherwise x CTAs share the tiles of all items evenly, one item after the other, which leaves no
+// place idle where an item is a large part of a CTA's share.  A CTA costs its rounds and `stage` of them before the first (staging the item's rows),
+// and again for every item that its share goes on to; waves of CTAs come one after the other.  How many items there are is only known on the
+// device, so a wave is taken to be full a fiftieth before it is.
+// Measured, us a launch, CTAs an item / even shares (128 experts, top-8): gate and up, 2048 -> 2 x 768: 27 rows 49.6 / 41.4, 100 rows 69 / 57, 256 rows
+// 120 / 102; 2048 -> 2 x 256: 33 rows 21.2 / 21.0, 100 rows 34 / 26, 512 rows 68 / 70; 8 experts, 4096 -> 2 x 2048: 5 rows 32.6 / 36.3.  Q6_K down, 768 ->
+// 2048: 27 rows 43.8 / 37.7, 256 rows 103 / 92; 2048 -> 1024, 64 experts, 64 rows 74 / 66; 256 -> 2048: 100 rows 26 / 40, 256 rows 43 / 72 (rows of one
+// block: staging an item costs more than its tiles).
+struct GroupedGrid {
+    int x;
+    bool per_item;
+};
+inline GroupedGrid grouped_grid(int items, int slots, int tiles, int lanes, double stage, bool may_share) {
+    GroupedGrid best{1, true};
     double best_cost = 0;
     const int most = (tiles + lanes - 1) / lanes;
     for (int g = 1; g <= most && g <= 64; g++) {
-        const double waves = std::ceil((double)items * g / slots + 0.02), cost = waves * ((tiles + g * lanes - 1) / (g * lanes) + 5);
-        if (g == 1 || cost < best_cost) best = g, best_cost = cost;
+        const double waves = std::ceil((double)items * g / slots + 0.02), cost = waves * ((tiles + g * lanes - 1) / (g * lanes) + stage);
+        if (g == 1 || cost < best_cost) best.x = g, best_cost = cost;
     }
+    if (may_share && std::ceil((double)items * tiles / slots / lanes) + stage * (1 + std::ceil((double)items / slots)) < best_cost) best = {slots, false};
     return best;
 }
 

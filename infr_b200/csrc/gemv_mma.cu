@@ -31,6 +31,7 @@
 // stops consuming (the block still reaches its barriers, results of the launch are invalid).
 #include <cuda.h>
 
+#include <algorithm>
 #include <cstring>
 
 #include "gemv_common.cuh"
@@ -172,7 +173,9 @@ __device__ __forceinline__ void quant_items(const float4 (&pa)[4], const float4 
 //   d8     : float [b][8 tokens], zero for absent tokens (a lane's two result columns are neighbours)
 // KW = warps per CTA (they split K), SB = super-blocks per ring slot per row.
 // TG: groups of KW warps that take the CTA's tiles in turn.
-template <int M, bool FUSED, int KW, int SB, bool PUSH, int TG = 1>
+// SHARE: expert-grouped with even shares (GroupedGrid): a CTA's tiles can span items, whose rows are staged one item after the other.  (Its state takes
+// 15 registers more, so a form of its own: beside the other form of grouped launches the next kernel can become resident earlier.)
+template <int M, bool FUSED, int KW, int SB, bool PUSH, int TG = 1, bool SHARE = false>
 __global__ void __launch_bounds__(KW * TG * 32, 16 / (KW * TG))
     gemv_q4k_mma_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ MmaSecond sec, Q8Dev a,
                         const float *x, float *__restrict__ y, int m, int in_f, int out_f, MmaGeom geo, MmaGroup grp,
@@ -199,7 +202,7 @@ __global__ void __launch_bounds__(KW * TG * 32, 16 / (KW * TG))
     __syncthreads();
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     int row_base = 0, p0 = 0;  // grouped mode: first row of the expert in the bank, first pair of the item
-    if (grp.item_expert) {
+    if (!SHARE && grp.item_expert) {
         asm volatile("griddepcontrol.wait;" ::: "memory");  // the work list comes from the previous kernels
         const int item = blockIdx.y;
         if (item >= *grp.n_items) return;
@@ -211,9 +214,18 @@ __global__ void __launch_bounds__(KW * TG * 32, 16 / (KW * TG))
     // balanced contiguous range of 16-row tiles of this CTA (only the matrix's last tile can be partial)
     const int tiles1 = (out_f + kTileRows - 1) / kTileRows;  // tiles of the first matrix; the second's follow
     const int total_tiles = tiles1 + (sec.out_f + kTileRows - 1) / kTileRows;
-    const int G = gridDim.x, base = total_tiles / G, rem = total_tiles % G;
-    const int t_begin = blockIdx.x * base + (blockIdx.x < rem ? blockIdx.x : rem);
-    const int n_tiles = (base + (blockIdx.x < rem ? 1 : 0) - tg + TG - 1) / TG;  // of this warp's group: tg, tg + TG, ...
+    int t_begin, cta_tiles;
+    if (SHARE) {
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        const GroupedShare share = grouped_share(*grp.n_items, total_tiles, false);
+        t_begin = share.t0, cta_tiles = share.n;
+        if (cta_tiles <= 0) return;
+    } else {
+        const int G = gridDim.x, base = total_tiles / G, rem = total_tiles % G;
+        t_begin = blockIdx.x * base + (blockIdx.x < rem ? blockIdx.x : rem);
+        cta_tiles = base + (blockIdx.x < rem ? 1 : 0);
+    }
+    const int n_tiles = (cta_tiles - tg + TG - 1) / TG;  // of this warp's group: tg, tg + TG, ...
     // this warp's K range
     const int kb0 = kwarp * geo.bpw;
     const int kb1 = min(nb, kb0 + geo.bpw);
@@ -228,7 +240,15 @@ __global__ void __launch_bounds__(KW * TG * 32, 16 / (KW * TG))
     uint64_t l2_policy;
     asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(l2_policy));
     // ---- issue side: one elected lane fetches the 16-row x K-step box of the slot ----
-    int j_issue = 0, i_tile = 0, i_step = 0;
+    int j_issue = 0, i_step = 0, i_T = t_begin + tg;
+    int i_item = 0;  // the item of tile i_T
+    if (SHARE) {
+        i_item = t_begin / total_tiles;
+        p0 = grp.item_p0[i_item], m = grp.item_cnt[i_item];  // (on their way while the weights are asked for)
+        i_T -= i_item * total_tiles;
+        while (i_T >= total_tiles && n_jobs > 0) i_T -= total_tiles, i_item++;
+        row_base = grp.item_expert[i_item] * out_f;
+    }
     auto issue = [&](int slot) {
         if (j_issue >= n_jobs) return;
         if (lane == 0) {
@@ -237,7 +257,7 @@ __global__ void __launch_bounds__(KW * TG * 32, 16 / (KW * TG))
             // order this warp's earlier reads of the slot before the engine overwrites it
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             bar_expect_tx(bar, (uint32_t)kSlotBytes);
-            const int T = t_begin + tg + i_tile * TG;
+            const int T = i_T;
             if (T < tiles1)
                 tma_load_2d_hint(s_u32(ring + (size_t)slot * kSlotBytes), &tmap, blk0 * 36, row_base + T * kTileRows, bar, l2_policy);
             else
@@ -247,7 +267,11 @@ __global__ void __launch_bounds__(KW * TG * 32, 16 / (KW * TG))
         j_issue++;
         if (++i_step == steps_per_tile) {
             i_step = 0;
-            i_tile++;
+            i_T += TG;
+            if (SHARE && i_T >= total_tiles && j_issue < n_jobs) {
+                while (i_T >= total_tiles) i_T -= total_tiles, i_item++;
+                row_base = grp.item_expert[i_item] * out_f;
+            }
         }
     };
     for (int s = 0; s < S; s++) issue(s);
@@ -256,6 +280,21 @@ __global__ void __launch_bounds__(KW * TG * 32, 16 / (KW * TG))
     asm volatile("griddepcontrol.wait;" ::: "memory");
     if constexpr (PUSH) {
         if (threadIdx.x == 0) s_epoch = *reinterpret_cast<const volatile uint32_t *>(push.ctrl);  // read by all after the barrier below
+    }
+    const int gt = g < M ? g : 0;  // token whose codes this lane feeds as its B column
+    int slot = 0, tile = 0;
+    uint32_t phase = 0;
+    bool dead = false;
+    for (int item = SHARE ? t_begin / total_tiles : 0;; item++) {  // even shares: the items of this CTA, otherwise once (body not indented)
+    int seg_end = 0, tid = threadIdx.x;
+    if (SHARE) asm volatile("" : "+r"(tid));  // (what the staging derives from it is not kept in registers from one item to the next)
+    if (SHARE) {
+        if (item * total_tiles >= t_begin + cta_tiles) break;
+        seg_end = (item + 1) * total_tiles;
+        if (item * total_tiles > t_begin) {
+            __syncthreads();  // everybody is through with the rows of the item before
+            p0 = grp.item_p0[item], m = grp.item_cnt[item];
+        }
     }
     if (M < 8)  // scale columns of tokens the template does not stage
         for (int i = threadIdx.x; i < nb * 8; i += kThreadsMma)
@@ -321,12 +360,12 @@ __global__ void __launch_bounds__(KW * TG * 32, 16 / (KW * TG))
         } else {
         // activation row of column n: the item's n-th pair (gathered through pair_row when given)
         __shared__ uint32_t s_row[8];
-        if (threadIdx.x < 8) s_row[threadIdx.x] = threadIdx.x < m ? (uint32_t)(grp.pair_row ? grp.pair_row[p0 + threadIdx.x] : p0 + threadIdx.x) : 0u;
+        if (tid < 8) s_row[tid] = tid < m ? (uint32_t)(grp.pair_row ? grp.pair_row[p0 + tid] : p0 + tid) : 0u;
         __syncthreads();
         // eight independent 8-byte loads in flight per thread: the copy is latency-bound, not bandwidth-bound
         // (flattened over tokens and units: with one token's few hundred units per pass most of the loads would be masked)
         const int units = in_f / 8, total = M * units;
-        for (int i0 = threadIdx.x; i0 < total; i0 += 8 * kThreadsMma) {
+        for (int i0 = tid; i0 < total; i0 += 8 * kThreadsMma) {
             uint2 v[8];
 #pragma unroll
             for (int k = 0; k < 8; k++) {
@@ -341,13 +380,13 @@ __global__ void __launch_bounds__(KW * TG * 32, 16 / (KW * TG))
                 if (i < total) *reinterpret_cast<uint2 *>(s_codes + (size_t)(n * nb + b) * kStagedBytes + tt * kLaneBytes + s * 8) = v[k];
             }
         }
-        for (int i = threadIdx.x; i < M * nb * 8; i += kThreadsMma) {
+        for (int i = tid; i < M * nb * 8; i += kThreadsMma) {
             const int n = i / (nb * 8), r = i - n * nb * 8, b = r >> 3, s = r & 7;
             const int sum = n < m ? a.sums[(size_t)s_row[n] * nb * 8 + r] : 0;
             s_bsplit[(size_t)(n * nb + b) * 16 + s] = (uint8_t)(sum & 63);
             s_bsplit[(size_t)(n * nb + b) * 16 + 8 + s] = (uint8_t)(int8_t)(sum >> 6);
         }
-        for (int i = threadIdx.x; i < M * nb; i += kThreadsMma) {
+        for (int i = tid; i < M * nb; i += kThreadsMma) {
             const int n = i / nb, b = i - n * nb;
             s_d8[b * 8 + n] = n < m ? a.d[(size_t)s_row[n] * nb + b] : 0.f;
         }
@@ -356,13 +395,9 @@ __global__ void __launch_bounds__(KW * TG * 32, 16 / (KW * TG))
     __syncthreads();
 
     // ---- consume ----
-    const int gt = g < M ? g : 0;  // token whose codes this lane feeds as its B column
-    int slot = 0, jc = 0;
-    uint32_t phase = 0;
-    bool dead = false;
-    for (int tile = 0; tile < n_tiles; tile++) {
+    for (; tile < n_tiles && (!SHARE || t_begin + tg + tile * TG < seg_end); tile++) {
         float accf[4] = {0.f, 0.f, 0.f, 0.f};
-        for (int step = 0; step < steps_per_tile; step++, jc++) {
+        for (int step = 0; step < steps_per_tile; step++) {
             if (!dead && !bar_wait(s_u32(wbar + slot), phase)) {
                 dead = true;
                 if (lane == 0) {
@@ -463,10 +498,10 @@ __global__ void __launch_bounds__(KW * TG * 32, 16 / (KW * TG))
             __syncthreads();
         else
             asm volatile("bar.sync %0, %1;" ::"r"(1 + tg), "n"(KW * 32) : "memory");
-        const int tid = threadIdx.x - tg * kW * 32;
-        if (tid < kTileRows * 8) {  // 16 rows x 8 token columns; groups have at least 128 threads
-            const int r = tid >> 3, n = tid & 7;
-            const int T = t_begin + tg + tile * TG;
+        const int gid = threadIdx.x - tg * kW * 32;
+        if (gid < kTileRows * 8) {  // 16 rows x 8 token columns; groups have at least 128 threads
+            const int r = gid >> 3, n = gid & 7;
+            const int T = t_begin + tg + tile * TG - (SHARE ? item * total_tiles : 0);
             const bool second = T >= tiles1;
             const int row = (second ? T - tiles1 : T) * kTileRows + r, of = second ? sec.out_f : out_f;
             if (n < m && row < of) {
@@ -480,6 +515,8 @@ __global__ void __launch_bounds__(KW * TG * 32, 16 / (KW * TG))
                     (second ? sec.y : y)[(size_t)(p0 + n) * of + row] = v;
             }
         }
+    }
+    if (!SHARE) break;
     }
 }
 
@@ -503,7 +540,7 @@ size_t mma_fixed_bytes(int M, int nb, int warps) {
     return (size_t)M * nb * (kStagedBytes + 16) + (size_t)nb * 32 + (size_t)2 * warps * 128 * 4 + (size_t)warps * kMaxSlotsMma * 8 + 64;
 }
 
-template <int M, bool FUSED, int KW, int SB, int TG = 1>
+template <int M, bool FUSED, int KW, int SB, int TG = 1, bool SHARE = false>
 cudaError_t launch_mma_cfg(const uint8_t *w, const Q8Dev &a, const float *x, float *y, int m, int in_f, int out_f,
                            const DeviceInfo &dev, uint32_t *status, cudaStream_t st, const MmaGroup &grp = MmaGroup{},
                            int n_experts = 1, int max_items = 1, const uint8_t *w2 = nullptr, float *y2 = nullptr, int out_f2 = 0,
@@ -533,6 +570,9 @@ cudaError_t launch_mma_cfg(const uint8_t *w, const Q8Dev &a, const float *x, flo
     }
     geo.slots = slots;
     const size_t smem = fixed + (size_t)slots * per_slot;
+    if constexpr (!SHARE && M == 8 && !FUSED && KW == 4)
+        if (grp.item_expert && !grouped_grid(items < 1 ? 1 : items, dev.sm_count * per_sm, all_tiles, TG, 3.0, true).per_item)
+            return launch_mma_cfg<M, FUSED, KW, SB, TG, true>(w, a, x, y, m, in_f, out_f, dev, status, st, grp, n_experts, max_items, w2, y2, out_f2, push, items);
     EncodeTiledFn enc = encode_tiled();
     if (!enc) return cudaErrorNotSupported;
     CUtensorMap tmap;
@@ -553,17 +593,18 @@ cudaError_t launch_mma_cfg(const uint8_t *w, const Q8Dev &a, const float *x, flo
         sec.out_f = out_f2;
     }
     // the pushing form exists for pre-quantised rows only
-    auto kernel = gemv_q4k_mma_kernel<M, FUSED, KW, SB, false, TG>;
+    auto kernel = gemv_q4k_mma_kernel<M, FUSED, KW, SB, false, TG, SHARE>;
     auto kernel_push = gemv_q4k_mma_kernel<M, false, KW, SB, true>;
-    if (push && (FUSED || TG > 1)) return cudaErrorInvalidValue;
+    if (push && (FUSED || TG > 1 || SHARE)) return cudaErrorInvalidValue;
     cudaError_t e = push ? cudaFuncSetAttribute(kernel_push, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)
                          : cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};
-    if (grp.item_expert) {
-        grid = grouped_ctas(items < 1 ? 1 : items, dev.sm_count * per_sm, all_tiles, TG);
-    }
-    cfg.gridDim = dim3((unsigned)grid, (unsigned)max_items);
+    if (SHARE)
+        grid = dev.sm_count * per_sm;
+    else if (grp.item_expert)
+        grid = grouped_grid(items < 1 ? 1 : items, dev.sm_count * per_sm, all_tiles, TG, 3.0, false).x;
+    cfg.gridDim = dim3((unsigned)grid, SHARE ? 1u : (unsigned)max_items);
     cfg.blockDim = dim3(KW * TG * 32);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;

@@ -19,6 +19,7 @@
 // reduction, programmatic dependent launch, bounded waits) is the scheme of the Q4_K kernel in gemv_mma.cu.
 #include <cuda.h>
 
+#include <algorithm>
 #include <cstring>
 
 #include "gemv_common.cuh"
@@ -300,13 +301,15 @@ __global__ void __launch_bounds__(KW * 32, 16 / KW)
 // ---- Expert-grouped form (mixture of experts): blockIdx.y walks the device-built list of work items, each up to 8 routed pairs of one
 // expert; the bank holds the experts' [out_f, in_f] matrices back to back; pair p reads activation row pair_row[p] (or p) and writes
 // y row p.  Rows of any length: 16 of them are one contiguous run of 16 * (in_f / 256) * 210 bytes, a multiple of 16, so a tile is ONE
-// plain bulk copy.  A warp owns whole tiles (all of K, two in flight) and stores its sums itself: no barrier between the warps of a CTA
+// plain bulk copy.  A warp owns whole tiles (all of K) and stores its sums itself: no barrier between the warps of a CTA
 // after the staging of the activations.  A lane's rows start on any even address: its words are put together from two aligned loads
 // and a shift by 0 or 16 bits.
-// What bounds it: the chain of loads and instructions around 18 matrix instructions a block with
-// two warps a scheduler (0.46 instructions a cycle), and items of unequal size; shared memory is 44 % busy.  The weights of 105 experts
-// of 2048 x 768 are 135 MB = 21 us.  Measured there (27 rows, top-8 of 128): 51 us; the byte-dot kernel, whose lanes load 2 bytes at a
-// time, 196.
+// What bounds it: the chain of loads and instructions around 18 matrix instructions a block, and shared memory (44 % busy with two warps a
+// scheduler).  Long rows left room for few warps while each had two tiles in shared memory (two a CTA at 1024 elements, 0.46 instructions a cycle
+// and scheduler): the CTA's warps share the tiles now, one each and a few on their way, and an even share of all items' tiles leaves no SM
+// waiting (GroupedGrid).  128 experts of 2048 x 768, 27 rows (135 MB = 21 us): 44.5 -> 37.2 us; 64 experts of 1024 x 2048, 64 rows 113 -> 66;
+// layers of 8 experts 4096 -> 2048, 512 rows 893 -> 591.  (The byte-dot kernel, whose lanes load 2 bytes at a time, took 196 on the first.)
+constexpr int kGroupedWarps6 = 8;  // at most, of a CTA (16 at 64 registers: 18 pairs of 8 experts 1024 -> 1024 11.4 us, 8.6)
 __device__ __forceinline__ void block_q6_any(const uint8_t *p0, const uint8_t *p1, uint32_t sh, const uint8_t *st, const float *s_d8b, int t, int n0,
                                              float (&accf)[4]) {
     // p0, p1: the word boundary at or below the block; sh: 0, or 16 where the block starts two bytes past it
@@ -360,104 +363,132 @@ __device__ __forceinline__ void block_q6_any(const uint8_t *p0, const uint8_t *p
     accf[3] = fmaf(d1 * e.y, (float)(isum[3] - 32 * (cl[3] + 64 * ch[3])), accf[3]);
 }
 
-// Shared memory: tiles [warps][2][16 rows]; staged activations [8][nb][352] and scales [nb][8] as in the kernel above; barriers [warps][2].
-__global__ void __launch_bounds__(256) gemv_q6_mma_grouped_kernel(const uint8_t *__restrict__ bank, Q8Dev a, float *__restrict__ y, int in_f, int out_f,
-                                                                  const int *item_expert, const int *item_p0,
+// Shared memory: tiles [slots][16 rows]; staged activations [8][nb][352] and scales [nb][8] as in the kernel above; barriers [slots]; the tile that
+// a slot holds or waits for [slots].  The CTA's i-th tile goes to warp i mod kw and to slot i mod slots, which the warp that has read the tile before it
+// there fills again: slots beyond one a warp are what is on its way.
+__global__ void __launch_bounds__(32 * kGroupedWarps6, 2) gemv_q6_mma_grouped_kernel(const uint8_t *__restrict__ bank, Q8Dev a, float *__restrict__ y, int in_f, int out_f,
+                                                                  int slots, bool per_item, const int *item_expert, const int *item_p0,
                                                                   const int *item_cnt, const int *n_items,
                                                                   const int *pair_row, uint32_t *__restrict__ status) {
     extern __shared__ __align__(128) uint8_t smem[];
     const int nb = in_f >> 8, row_bytes = nb * 210, tile_bytes = kRows6 * row_bytes, kw = blockDim.x >> 5;
-    uint8_t *s_act = smem + (size_t)kw * 2 * tile_bytes;
+    uint8_t *s_act = smem + (size_t)slots * tile_bytes;
     float *s_d8 = reinterpret_cast<float *>(s_act + (size_t)8 * nb * kStagedBlock);
     uint64_t *bars = reinterpret_cast<uint64_t *>(s_d8 + nb * 8);
+    volatile int *s_tile = reinterpret_cast<volatile int *>(bars + slots);
     __shared__ int s_row[8];
+    __shared__ volatile int s_dead;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
     if (threadIdx.x == 0) {
-        for (int i = 0; i < kw * 2; i++) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(sm6(bars + i)) : "memory");
+        s_dead = 0;
+        for (int i = 0; i < slots; i++) {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(sm6(bars + i)) : "memory");
+            s_tile[i] = -1;
+        }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");  // the work list comes from the kernels before
-    const int item = blockIdx.y;
-    if (item >= *n_items) return;
-    const int p0 = item_p0[item], m = item_cnt[item];
-    const uint8_t *W = bank + (size_t)item_expert[item] * out_f * row_bytes;
-    // this CTA's tiles; a warp takes every kw-th of them
-    const int tiles = out_f / kRows6, t0 = (int)((long long)blockIdx.x * tiles / gridDim.x), t1 = (int)((long long)(blockIdx.x + 1) * tiles / gridDim.x);
-    uint8_t *ring = smem + (size_t)warp * 2 * tile_bytes;
-    auto issue = [&](int slot, int tile) {
-        if (lane == 0 && tile < t1) {
-            const uint32_t bar = sm6(bars + warp * 2 + slot);
+    const int tiles = out_f / kRows6;
+    const GroupedShare share = grouped_share(*n_items, tiles, per_item);
+    const int t0 = share.t0, n_tiles = share.n;
+    if (n_tiles <= 0) return;
+    const int item0 = t0 / tiles, first_p0 = item_p0[item0], first_m = item_cnt[item0], first_e = item_expert[item0];  // (on their way while the weights are asked for)
+    // A warp takes tiles warp, warp + kw, ...; what it has read is followed in its slot by the tile `slots` further on, which is some warp's.
+    int ask_item = item0, ask_tile = t0 - item0 * tiles + warp;  // the tile that it asks for next, as one of its item
+    auto issue = [&](int i, int slot) {  // that tile is the CTA's i-th
+        if (i < n_tiles && lane == 0 && !s_dead) {
+            while (ask_tile >= tiles) ask_tile -= tiles, ask_item++;
+            const uint32_t bar = sm6(bars + slot);
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // earlier reads of the slot come first
             asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(tile_bytes) : "memory");
-            asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(sm6(ring + (size_t)slot * tile_bytes)),
-                         "l"(W + (size_t)tile * tile_bytes), "r"(tile_bytes), "r"(bar)
+            asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(sm6(smem + (size_t)slot * tile_bytes)),
+                         "l"(bank + ((size_t)(ask_item == item0 ? first_e : item_expert[ask_item]) * tiles + ask_tile) * tile_bytes), "r"(tile_bytes), "r"(bar)
                          : "memory");
+            s_tile[slot] = i;
         }
+        ask_tile += kw;
         __syncwarp();
     };
-    issue(0, t0 + warp);
-    issue(1, t0 + warp + kw);
-    if (threadIdx.x < 8) s_row[threadIdx.x] = (int)threadIdx.x < m ? (pair_row ? pair_row[p0 + threadIdx.x] : p0 + (int)threadIdx.x) : 0;
-    __syncthreads();
-    {
-        const int units = in_f / 16, total = 8 * units;
-        for (int i0 = threadIdx.x; i0 < total; i0 += 4 * blockDim.x) {
-            uint4 v[4];
+    // Landed?  (Bounded.  Not before the slot is this tile's: a parity cannot tell "not yet issued" from "landed".)
+    auto landed = [&](int i, int slot, uint32_t phase, bool once) {
+        uint32_t k = 0;
+        for (const uint32_t most = once ? 1u : 1u << 22; s_tile[slot] != i; k++)
+            if (k >= most) return false;
+        return wait_parity6(sm6(bars + slot), phase);
+    };
+    for (int i = warp; i < slots; i += kw) issue(i, i);
+    ask_item = item0, ask_tile = t0 - item0 * tiles + warp + slots;
+    int i = warp, slot = warp;
+    uint32_t phase = 0;
+    const int n0 = 2 * t;
+    bool dead = false;
+    for (int item = item0; item * tiles < t0 + n_tiles; item++) {
+        const int p0 = item == item0 ? first_p0 : item_p0[item], m = item == item0 ? first_m : item_cnt[item], lo = max(item * tiles - t0, 0), hi = min((item + 1) * tiles - t0, n_tiles);
+        if (lo > 0) __syncthreads();  // everybody is through with the rows of the item before
+        if (threadIdx.x < 8) s_row[threadIdx.x] = (int)threadIdx.x < m ? (pair_row ? pair_row[p0 + threadIdx.x] : p0 + (int)threadIdx.x) : 0;
+        __syncthreads();
+        {
+            const int units = in_f / 16, total = 8 * units;
+            for (int i0 = threadIdx.x; i0 < total; i0 += 4 * blockDim.x) {
+                uint4 v[4];
 #pragma unroll
-            for (int k = 0; k < 4; k++) {
-                const int i = i0 + k * blockDim.x, n = i / units, u = i - n * units;
-                v[k] = make_uint4(0, 0, 0, 0);
-                if (i < total && n < m) v[k] = *reinterpret_cast<const uint4 *>(a.qs + (size_t)s_row[n] * in_f + (size_t)u * 16);
-            }
+                for (int k = 0; k < 4; k++) {
+                    const int i = i0 + k * blockDim.x, n = i / units, u = i - n * units;
+                    v[k] = make_uint4(0, 0, 0, 0);
+                    if (i < total && n < m) v[k] = *reinterpret_cast<const uint4 *>(a.qs + (size_t)s_row[n] * in_f + (size_t)u * 16);
+                }
 #pragma unroll
-            for (int k = 0; k < 4; k++) {
-                const int i = i0 + k * blockDim.x, n = i / units, u = i - n * units;
-                if (i < total) {
-                    uint8_t *dst = s_act + (size_t)(n * nb + (u >> 4)) * kStagedBlock + (u & 15) * 4;
-                    *reinterpret_cast<uint32_t *>(dst) = v[k].x;
-                    *reinterpret_cast<uint32_t *>(dst + kLane6) = v[k].y;
-                    *reinterpret_cast<uint32_t *>(dst + 2 * kLane6) = v[k].z;
-                    *reinterpret_cast<uint32_t *>(dst + 3 * kLane6) = v[k].w;
+                for (int k = 0; k < 4; k++) {
+                    const int i = i0 + k * blockDim.x, n = i / units, u = i - n * units;
+                    if (i < total) {
+                        uint8_t *dst = s_act + (size_t)(n * nb + (u >> 4)) * kStagedBlock + (u & 15) * 4;
+                        *reinterpret_cast<uint32_t *>(dst) = v[k].x;
+                        *reinterpret_cast<uint32_t *>(dst + kLane6) = v[k].y;
+                        *reinterpret_cast<uint32_t *>(dst + 2 * kLane6) = v[k].z;
+                        *reinterpret_cast<uint32_t *>(dst + 3 * kLane6) = v[k].w;
+                    }
                 }
             }
+            for (int i = threadIdx.x; i < 8 * nb * 16; i += blockDim.x) {
+                const int n = i / (nb * 16), r = i - n * nb * 16, b = r >> 4, s = r & 15;
+                const int bs = n < m ? a.sums16[(size_t)s_row[n] * nb * 16 + r] : 0;
+                uint8_t *sp = s_act + (size_t)(n * nb + b) * kStagedBlock + 4 * kLane6;
+                sp[s] = (uint8_t)(bs & 63);
+                sp[16 + s] = (uint8_t)(int8_t)(bs >> 6);
+            }
+            for (int i = threadIdx.x; i < nb * 8; i += blockDim.x) {
+                const int b = i >> 3, n = i & 7;
+                s_d8[i] = n < m ? a.d[(size_t)s_row[n] * nb + b] : 0.f;
+            }
         }
-        for (int i = threadIdx.x; i < 8 * nb * 16; i += blockDim.x) {
-            const int n = i / (nb * 16), r = i - n * nb * 16, b = r >> 4, s = r & 15;
-            const int bs = n < m ? a.sums16[(size_t)s_row[n] * nb * 16 + r] : 0;
-            uint8_t *sp = s_act + (size_t)(n * nb + b) * kStagedBlock + 4 * kLane6;
-            sp[s] = (uint8_t)(bs & 63);
-            sp[16 + s] = (uint8_t)(int8_t)(bs >> 6);
+        __syncthreads();
+        for (; i < hi; i += kw) {
+            const bool ok = __all_sync(0xffffffffu, landed(i, slot, phase, dead));
+            if (!ok && !dead) {  // from here on only what is on its way is waited for
+                dead = true;
+                if (lane == 0) s_dead = 1, atomicExch(status, 3u);
+            }
+            const uint8_t *tile = smem + (size_t)slot * tile_bytes;
+            const int here = slot;
+            slot += kw;
+            if (slot >= slots) slot -= slots, phase ^= 1u;
+            if (dead) continue;
+            float accf[4] = {0.f, 0.f, 0.f, 0.f};
+            const uint8_t *r0 = tile + (size_t)g * row_bytes, *st = s_act + (size_t)g * nb * kStagedBlock;
+#pragma unroll 1
+            for (int b = 0; b < nb; b++) {
+                const uint8_t *p = r0 + b * 210;
+                const uint32_t mis = sm6(p) & 2u;  // (eight rows on: the same)
+                block_q6_any(p - mis, p - mis + 8 * row_bytes, mis * 8, st + (size_t)b * kStagedBlock, s_d8 + b * 8, t, n0, accf);
+            }
+            __syncwarp();
+            issue(i + slots, here);
+            float *yr = y + (size_t)(p0 + n0) * out_f + (t0 + i - item * tiles) * kRows6 + g;
+            if (n0 < m) yr[0] = accf[0], yr[8] = accf[2];
+            if (n0 + 1 < m) yr[out_f] = accf[1], yr[out_f + 8] = accf[3];
         }
-        for (int i = threadIdx.x; i < nb * 8; i += blockDim.x) {
-            const int b = i >> 3, n = i & 7;
-            s_d8[i] = n < m ? a.d[(size_t)s_row[n] * nb + b] : 0.f;
-        }
-    }
-    __syncthreads();
-    const int n0 = 2 * t;
-    int k = 0;
-    for (int tile = t0 + warp; tile < t1; tile += kw, k++) {
-        const int slot = k & 1;
-        if (!wait_parity6(sm6(bars + warp * 2 + slot), (uint32_t)(k >> 1) & 1u)) {
-            if (lane == 0) atomicExch(status, 3u);
-            // the other slot's copy gets its own limit before the warp leaves
-            if (tile + kw < t1) wait_parity6(sm6(bars + warp * 2 + (slot ^ 1)), (uint32_t)((k + 1) >> 1) & 1u);
-            return;
-        }
-        float accf[4] = {0.f, 0.f, 0.f, 0.f};
-        const uint8_t *r0 = ring + (size_t)slot * tile_bytes + (size_t)g * row_bytes, *st = s_act + (size_t)g * nb * kStagedBlock;
-        for (int b = 0; b < nb; b++) {
-            const uint8_t *p = r0 + b * 210;
-            const uint32_t mis = sm6(p) & 2u;  // (eight rows on: the same)
-            block_q6_any(p - mis, p - mis + 8 * row_bytes, mis * 8, st + (size_t)b * kStagedBlock, s_d8 + b * 8, t, n0, accf);
-        }
-        __syncwarp();
-        issue(slot, tile + 2 * kw);
-        float *yr = y + (size_t)(p0 + n0) * out_f + tile * kRows6 + g;
-        if (n0 < m) yr[0] = accf[0], yr[8] = accf[2];
-        if (n0 + 1 < m) yr[out_f] = accf[1], yr[out_f + 8] = accf[3];
     }
 }
 
@@ -574,27 +605,34 @@ cudaError_t launch_grouped_q6_mma(const uint8_t *bank, const Q8Dev &a, float *y,
     if (in_f < 256 || in_f % 256 || out_f < 16 || out_f % 16 || max_items < 1 || max_items > 65535 || !a.sums16 || a.gran != 256 || (uintptr_t)bank % 16)
         return cudaErrorInvalidValue;
     const size_t nb = in_f / 256;
-    auto need = [&](int kw) { return (size_t)kw * 2 * kRows6 * nb * 210 + 8 * nb * kStagedBlock + nb * 32 + (size_t)kw * 16 + 16; };
-    // as many warps as leave room for two CTAs on an SM, or at least for one
-    int kw = 8;
-    while (kw > 2 && need(kw) > (size_t)dev.max_smem_optin / 2 - 2048) kw /= 2;
-    if (need(kw) > (size_t)dev.max_smem_optin - 1024) return cudaErrorInvalidValue;
-    cudaError_t e = cudaFuncSetAttribute(gemv_q6_mma_grouped_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)need(kw));
+    const size_t tile = (size_t)kRows6 * nb * 210, rest = 8 * nb * kStagedBlock + nb * 32 + 16;
+    // Two CTAs an SM, or one, whichever has more warps: a slot a warp and two (or a fifth of them) for what is on its way.
+    auto slots_of = [&](int ctas) {
+        const size_t budget = (size_t)dev.max_smem_optin / ctas - (ctas > 1 ? 2048 : 1024);
+        return budget < rest ? 0 : (int)((budget - rest) / (tile + 12));
+    };
+    auto warps_of = [&](int n) { return n < 2 ? 0 : std::min(kGroupedWarps6, n - std::max(n > 4 ? 2 : 1, n / 5)); };
+    const int s2 = slots_of(2), s1 = slots_of(1), ctas = 2 * warps_of(s2) >= warps_of(s1) ? 2 : 1;
+    int kw = warps_of(ctas == 2 ? s2 : s1);
+    const long long all = (long long)(items < 1 ? 1 : items) * (out_f / kRows6);
+    while (nb >= 3 && kw > 2 && all < (long long)kw * dev.sm_count) kw--;  // few large tiles: on all SMs rather than on all warps of some
+    const int slots = std::min(ctas == 2 ? s2 : s1, 2 * kw);
+    if (std::max(s1, s2) < 4) return cudaErrorInvalidValue;
+    const size_t smem = slots * (tile + 12) + rest;
+    cudaError_t e = cudaFuncSetAttribute(gemv_q6_mma_grouped_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    // (Whole layers with this bank as down, before: a CTA for eight tiles of each warp, 1 to 16 an item.  8 experts of 4096 -> 2048, 18 pairs:
-    // 113 us, 183 before; 128 experts of 2048 -> 768, 216 pairs: 122, 151; 512 pairs: 130, 162.)
-    const int gx = grouped_ctas(items < 1 ? 1 : items, dev.sm_count * (need(kw) > (size_t)dev.max_smem_optin / 2 - 2048 ? 1 : 2), out_f / 16, kw);
+    const GroupedGrid grid = grouped_grid(items < 1 ? 1 : items, dev.sm_count * ctas, out_f / kRows6, kw, nb >= 3 ? 1.5 : 5.0, nb >= 3);
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)gx, (unsigned)max_items);
+    cfg.gridDim = dim3((unsigned)grid.x, grid.per_item ? (unsigned)max_items : 1u);
     cfg.blockDim = dim3((unsigned)kw * 32);
-    cfg.dynamicSmemBytes = need(kw);
+    cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, gemv_q6_mma_grouped_kernel, bank, a, y, in_f, out_f, item_expert, item_p0, item_cnt, n_items, pair_row, status);
+    return cudaLaunchKernelEx(&cfg, gemv_q6_mma_grouped_kernel, bank, a, y, in_f, out_f, slots, grid.per_item, item_expert, item_p0, item_cnt, n_items, pair_row, status);
 }
 
 }  // namespace infr
