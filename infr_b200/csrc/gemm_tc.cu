@@ -337,12 +337,14 @@ struct TcGroup {
 
 namespace {
 
-// Activations -> operand layout.  One warp per (token slot, 256 elements), lane l owns elements [8l, 8l + 8).
+// Activations -> operand layout.  One warp per (token slot, 256 elements), or PER times 256, lane l owns elements [8l, 8l + 8) of them.
 //   units:  [token tile][block][unit][plane][TN][16 B]  f16 codes, 8 per 16 bytes, in the order the unpack warps emit
 //   extra:  [token tile][block]{Q4_K: [2][TN][8] f16 of 64h and l of the 32-element sums; scales [TN] f32}
 // F32: quantises f32 rows (quantize_q8, crates/infr-cpu/src/quant.rs:27-58: the operations of quantize.cu in the same order);
-// otherwise re-lays rows that are already quantised.  Slots past the last token are zero.
-template <int FMT, bool F32>
+// otherwise re-lays rows that are already quantised.  Slots past the last token are zero (grouped: as they were).
+// PER > 1 (grouped): a slot's place in the work list is four dependent reads, and with a warp a block there are five waves of warps behind them
+// (a layer of 256 rows over 128 experts, 2048 -> 768: 190.4 us one block a warp, 189.3; 200 rows over 16, 2048 -> 1024: 79.2, 76.6).
+template <int FMT, bool F32, int PER>
 __global__ void __launch_bounds__(256) gemm_tc_prep_kernel(const float *x, Q8Dev a, int m, int tn, int in_f, uint8_t *__restrict__ units,
                                                            uint8_t *__restrict__ extra, int n_tok, TcGroup grp) {
     pdl_go();
@@ -351,67 +353,81 @@ __global__ void __launch_bounds__(256) gemm_tc_prep_kernel(const float *x, Q8Dev
     constexpr int UPS = C64::kUnits, UB = C64::kUnitBytes / 64, EB = C64::kExtra / 64;  // (per token: the same for every tile)
     const int lane = threadIdx.x & 31, nb = in_f >> 8;
     const long long wg = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (wg >= (long long)n_tok * nb) return;
-    const int T = (int)(wg / nb), b = (int)(wg % nb), tt = T / tn, t = T - tt * tn;
+    const int per = (nb + PER - 1) / PER;  // warps of a slot
+    if (wg >= (long long)n_tok * per) return;
+    const int T = (int)(wg / per), b0 = (int)(wg % per) * PER, tt = T / tn, t = T - tt * tn;
     long long row = T < m ? T : -1;
     if (grp.slab_expert) {
         if (tt >= *grp.n_slabs) return;
-        row = -1;
-        if (t < grp.slab_cnt[tt]) {
-            const int pair = grp.slab_p0[tt] + t;
-            row = grp.pair_row ? grp.pair_row[pair] : pair;
-        }
+        if (t >= grp.slab_cnt[tt]) return;  // (what a slot without a pair holds meets sums that are not stored: half the slots at 16 pairs an expert)
+        const int pair = grp.slab_p0[tt] + t;
+        row = grp.pair_row ? grp.pair_row[pair] : pair;
     }
-    uint32_t w0 = 0, w1 = 0;  // eight codes
-    float d = 0.f;
-    int sum = 0;
-    if (F32) {
-        float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-        if (row >= 0) {
+    float v[PER][8];
+    uint2 c[PER];
+#pragma unroll
+    for (int k = 0; k < PER; k++) {
+        const int b = b0 + k;
+        c[k] = make_uint2(0, 0);
+#pragma unroll
+        for (int i = 0; i < 8; i++) v[k][i] = 0.f;
+        if (row < 0 || b >= nb) continue;
+        if (F32) {
             const float4 *xp = reinterpret_cast<const float4 *>(x + (size_t)row * in_f + (size_t)b * 256) + lane * 2;
             const float4 p = xp[0], q = xp[1];
-            v[0] = p.x, v[1] = p.y, v[2] = p.z, v[3] = p.w, v[4] = q.x, v[5] = q.y, v[6] = q.z, v[7] = q.w;
+            v[k][0] = p.x, v[k][1] = p.y, v[k][2] = p.z, v[k][3] = p.w, v[k][4] = q.x, v[k][5] = q.y, v[k][6] = q.z, v[k][7] = q.w;
+        } else {
+            c[k] = *reinterpret_cast<const uint2 *>(a.qs + (size_t)row * in_f + (size_t)b * 256 + lane * 8);
         }
-        float am = 0.f;
-#pragma unroll
-        for (int i = 0; i < 8; i++) am = fmaxf(am, fabsf(v[i]));
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) am = fmaxf(am, __shfl_xor_sync(0xffffffffu, am, o));
-        d = am / 127.0f;
-        const float id = d > 0.0f ? 1.0f / d : 0.0f;
-        w0 = q8_codes4(make_float4(v[0], v[1], v[2], v[3]), id);
-        w1 = q8_codes4(make_float4(v[4], v[5], v[6], v[7]), id);
-    } else if (row >= 0) {
-        const uint2 c = *reinterpret_cast<const uint2 *>(a.qs + (size_t)row * in_f + (size_t)b * 256 + lane * 8);
-        w0 = c.x, w1 = c.y;
-        d = a.d[(size_t)row * nb + b];
     }
-    if (FMT == F_Q4) {
-        sum = q8_sum4(w0) + q8_sum4(w1);
-        sum += __shfl_xor_sync(0xffffffffu, sum, 1);
-        sum += __shfl_xor_sync(0xffffffffu, sum, 2);
-    }
-    // byte -> f16: 1024 + (code + 128) - 1152
-    auto pair16 = [](uint32_t two) { return h2add(__byte_perm(two, 0x64646464u, 0x4140), dup(H_N1152)); };
-    const uint32_t e0 = w0 ^ 0x80808080u, e1 = w1 ^ 0x80808080u;
-    const uint4 o = make_uint4(pair16(__byte_perm(e0, 0, 0x0020)), pair16(__byte_perm(e0, 0, 0x0031)), pair16(__byte_perm(e1, 0, 0x0020)),
-                               pair16(__byte_perm(e1, 0, 0x0031)));
-    constexpr int PL = FMT == F_Q4 ? 16 : 8;  // planes per unit
-    const int unit = lane / PL, pl = lane % PL;
-    const size_t rec = (size_t)tt * nb + b;
-    *reinterpret_cast<uint4 *>(units + ((rec * UPS + unit) * UB + (size_t)pl * 16) * tn + (size_t)t * 16) = o;
-    uint8_t *ex = extra + rec * EB * tn;
-    if (FMT == F_Q4) {
-        const int h = sum >> 6, l = sum & 63;
-        uint32_t v = (uint32_t)__half_as_ushort(__int2half_rn(h * 64)) | ((uint32_t)__half_as_ushort(__int2half_rn(l)) << 16);
-        const uint32_t nx = __shfl_down_sync(0xffffffffu, v, 4);
-        if ((lane & 7) == 0) {
-            *reinterpret_cast<uint32_t *>(ex + (size_t)t * 16 + (lane >> 3) * 4) = __byte_perm(v, nx, 0x5410);
-            *reinterpret_cast<uint32_t *>(ex + (size_t)tn * 16 + (size_t)t * 16 + (lane >> 3) * 4) = __byte_perm(v, nx, 0x7632);
+#pragma unroll
+    for (int k = 0; k < PER; k++) {
+        const int b = b0 + k;
+        if (b >= nb) break;
+        uint32_t w0 = 0, w1 = 0;  // eight codes
+        float d = 0.f;
+        int sum = 0;
+        if (F32) {
+            float am = 0.f;
+#pragma unroll
+            for (int i = 0; i < 8; i++) am = fmaxf(am, fabsf(v[k][i]));
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) am = fmaxf(am, __shfl_xor_sync(0xffffffffu, am, o));
+            d = am / 127.0f;
+            const float id = d > 0.0f ? 1.0f / d : 0.0f;
+            w0 = q8_codes4(make_float4(v[k][0], v[k][1], v[k][2], v[k][3]), id);
+            w1 = q8_codes4(make_float4(v[k][4], v[k][5], v[k][6], v[k][7]), id);
+        } else if (row >= 0) {
+            w0 = c[k].x, w1 = c[k].y;
+            d = a.d[(size_t)row * nb + b];
         }
-        if (lane == 0) reinterpret_cast<float *>(ex + (size_t)tn * 32)[t] = d;
-    } else {
-        if (lane == 0) reinterpret_cast<float *>(ex)[t] = d;
+        if (FMT == F_Q4) {
+            sum = q8_sum4(w0) + q8_sum4(w1);
+            sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+            sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+        }
+        // byte -> f16: 1024 + (code + 128) - 1152
+        auto pair16 = [](uint32_t two) { return h2add(__byte_perm(two, 0x64646464u, 0x4140), dup(H_N1152)); };
+        const uint32_t e0 = w0 ^ 0x80808080u, e1 = w1 ^ 0x80808080u;
+        const uint4 o = make_uint4(pair16(__byte_perm(e0, 0, 0x0020)), pair16(__byte_perm(e0, 0, 0x0031)), pair16(__byte_perm(e1, 0, 0x0020)),
+                                   pair16(__byte_perm(e1, 0, 0x0031)));
+        constexpr int PL = FMT == F_Q4 ? 16 : 8;  // planes per unit
+        const int unit = lane / PL, pl = lane % PL;
+        const size_t rec = (size_t)tt * nb + b;
+        *reinterpret_cast<uint4 *>(units + ((rec * UPS + unit) * UB + (size_t)pl * 16) * tn + (size_t)t * 16) = o;
+        uint8_t *ex = extra + rec * EB * tn;
+        if (FMT == F_Q4) {
+            const int h = sum >> 6, l = sum & 63;
+            uint32_t v = (uint32_t)__half_as_ushort(__int2half_rn(h * 64)) | ((uint32_t)__half_as_ushort(__int2half_rn(l)) << 16);
+            const uint32_t nx = __shfl_down_sync(0xffffffffu, v, 4);
+            if ((lane & 7) == 0) {
+                *reinterpret_cast<uint32_t *>(ex + (size_t)t * 16 + (lane >> 3) * 4) = __byte_perm(v, nx, 0x5410);
+                *reinterpret_cast<uint32_t *>(ex + (size_t)tn * 16 + (size_t)t * 16 + (lane >> 3) * 4) = __byte_perm(v, nx, 0x7632);
+            }
+            if (lane == 0) reinterpret_cast<float *>(ex + (size_t)tn * 32)[t] = d;
+        } else {
+            if (lane == 0) reinterpret_cast<float *>(ex)[t] = d;
+        }
     }
 }
 
@@ -486,7 +502,8 @@ __global__ void __launch_bounds__(256) gemm_tc_silu_prep_kernel(const float *gat
     if (grp.slab_expert) {
         const int tt = T / tn, t = T - tt * tn;
         if (tt >= *grp.n_slabs) return;
-        row = t < grp.slab_cnt[tt] ? grp.slab_p0[tt] + t : -1;
+        if (t >= grp.slab_cnt[tt]) return;  // (as above)
+        row = grp.slab_p0[tt] + t;
     }
     float4 v[2] = {make_float4(0.f, 0.f, 0.f, 0.f), make_float4(0.f, 0.f, 0.f, 0.f)};
     if (row >= 0) {
@@ -1003,12 +1020,15 @@ cudaError_t launch_tn(int tn, const CUtensorMap &mw, const CUtensorMap &mw2, con
     return launch_fmt<FMT, 128>(mw, mw2, units, extra, m1, m2, m, in_f, status, grp, split, grid, st);
 }
 
+constexpr int kGroupedPer = 2;  // blocks of a warp, grouped
 template <bool F32>
 cudaError_t launch_prep(int fmt, const float *x, const Q8Dev &a, int m, int tn, int in_f, uint8_t *units, uint8_t *extra, int n_tok, const TcGroup &grp,
                         cudaStream_t st) {
-    const dim3 grid((unsigned)(((size_t)n_tok * (in_f / 256) + 7) / 8)), block(256);
-    if (fmt == F_Q4) return launch_pdl(gemm_tc_prep_kernel<F_Q4, F32>, grid, block, 0, st, x, a, m, tn, in_f, units, extra, n_tok, grp);
-    return launch_pdl(gemm_tc_prep_kernel<F_Q6, F32>, grid, block, 0, st, x, a, m, tn, in_f, units, extra, n_tok, grp);
+    const int nb = in_f / 256, per = grp.slab_expert ? (nb + kGroupedPer - 1) / kGroupedPer : nb;
+    const dim3 grid((unsigned)(((size_t)n_tok * per + 7) / 8)), block(256);
+    if (grp.slab_expert) return launch_pdl(gemm_tc_prep_kernel<F_Q4, F32, kGroupedPer>, grid, block, 0, st, x, a, m, tn, in_f, units, extra, n_tok, grp);
+    if (fmt == F_Q4) return launch_pdl(gemm_tc_prep_kernel<F_Q4, F32, 1>, grid, block, 0, st, x, a, m, tn, in_f, units, extra, n_tok, grp);
+    return launch_pdl(gemm_tc_prep_kernel<F_Q6, F32, 1>, grid, block, 0, st, x, a, m, tn, in_f, units, extra, n_tok, grp);
 }
 
 int ctas_of(int fmt, int tn, const DeviceInfo &dev) { return dev.sm_count * (tn == 32 && fmt != F_Q6 ? 2 : 1); }
@@ -1125,12 +1145,14 @@ size_t gemm_tc_grouped_record_bytes(int slab, int max_slabs, int in_f) {
     const int n = max_slabs * slab;
     return units_bytes(n, in_f) + extra_bytes(F_Q4, n, in_f);
 }
-cudaError_t launch_gemm_tc_grouped_prep(int slab, const Q8Dev &a, void *records, int in_f, const int *slab_expert, const int *slab_p0,
+cudaError_t launch_gemm_tc_grouped_prep(int slab, const float *x, const Q8Dev *a, void *records, int in_f, const int *slab_expert, const int *slab_p0,
                                         const int *slab_cnt, const int *n_slabs, const int *pair_row, int max_slabs, cudaStream_t st) {
     if (!gemm_tc_takes(DT_Q4K, in_f) || max_slabs < 1) return cudaErrorInvalidValue;
     const int n = max_slabs * slab;
     uint8_t *u = static_cast<uint8_t *>(records), *e = u + units_bytes(n, in_f);
-    return launch_prep<false>(F_Q4, nullptr, a, n, slab, in_f, u, e, n, TcGroup{slab_expert, slab_p0, slab_cnt, n_slabs, pair_row}, st);
+    if (x && (uintptr_t)x % 16) return cudaErrorInvalidValue;
+    const TcGroup g{slab_expert, slab_p0, slab_cnt, n_slabs, pair_row};
+    return x ? launch_prep<true>(F_Q4, x, Q8Dev{}, n, slab, in_f, u, e, n, g, st) : launch_prep<false>(F_Q4, nullptr, *a, n, slab, in_f, u, e, n, g, st);
 }
 cudaError_t launch_gemm_tc_grouped_silu_prep(int slab, const float *gate, const float *up, void *records, int in_f, const int *slab_expert, const int *slab_p0,
                                              const int *slab_cnt, const int *n_slabs, int max_slabs, cudaStream_t st) {

@@ -161,7 +161,7 @@ cudaError_t launch_gemm_q2(const uint8_t *w, const void *records, float *c, floa
 // The same over a bank of Q4_K expert matrices, one slab of up to `slab` (32, 64) routed rows of an expert per token tile; `a`
 // quantised rows, gathered through pair_row when it is non-null.
 size_t gemm_tc_grouped_record_bytes(int slab, int max_slabs, int in_f);
-cudaError_t launch_gemm_tc_grouped_prep(int slab, const Q8Dev &a, void *records, int in_f, const int *slab_expert, const int *slab_p0,
+cudaError_t launch_gemm_tc_grouped_prep(int slab, const float *x, const Q8Dev *a, void *records, int in_f, const int *slab_expert, const int *slab_p0,
                                         const int *slab_cnt, const int *n_slabs, const int *pair_row, int max_slabs, cudaStream_t st);
 // The layout of silu(gate) * up, rows = pairs.
 cudaError_t launch_gemm_tc_grouped_silu_prep(int slab, const float *gate, const float *up, void *records, int in_f, const int *slab_expert, const int *slab_p0,
@@ -190,7 +190,7 @@ cudaError_t launch_grouped_q6k(const uint8_t *bank, const Q8Dev &a, float *y, in
                                const int *item_cnt, const int *n_items, const int *pair_row, int max_items, const DeviceInfo &dev,
                                cudaStream_t st);
 cudaError_t launch_moe_router(const float *router, const float *x, float *logits, int rows, int ne, int n_expert,
-                              const DeviceInfo &dev, cudaStream_t st);
+                              const DeviceInfo &dev, uint32_t *status, cudaStream_t st);
 cudaError_t launch_moe_route(const float *logits, int rows, int n_expert, int n_used, float scale, int norm_w,
                              int32_t *sel_ids, float *sel_w, cudaStream_t st);
 cudaError_t launch_moe_bucket(const int32_t *sel_ids, int rows, int n_used, int n_expert, int e_lo, int n_local, int item_rows,
@@ -205,6 +205,7 @@ cudaError_t launch_moe_combine(const float *y_pairs, const int32_t *pair_of_slot
 // (act: n_used * nff floats); down and the weighted sum.  moe_row_takes false: the shape takes the general launches.
 bool moe_row_takes(int ne, int nff, int n_expert, int n_used, const float *x, const float *router, const uint8_t *gate, const uint8_t *up, const uint8_t *down);
 size_t moe_router_row_smem(int ne);  // of a CTA: four experts, four rows
+cudaError_t launch_moe_route_rows(const float *logits, int rows, int n_expert, int n_used, float scale, int norm_w, int32_t *sel_ids, float *sel_w, cudaStream_t st);
 cudaError_t launch_moe_router_row(const float *router, const float *x, float *logits, int rows, int ne, int n_expert, cudaStream_t st);
 cudaError_t launch_moe_gate_up_row(const float *logits, const float *x, const uint8_t *gate, const uint8_t *up, float *act, int32_t *sel_ids, float *sel_w, int ne,
                                    int nff, int n_expert, int n_used, float scale, int norm_w, const DeviceInfo &dev, cudaStream_t st);

@@ -20,81 +20,92 @@
 namespace infr {
 
 // logits[r, e] = dot(router[e, :], x[r, :]).  Eight lanes per dot product replay the eight accumulators of the CPU
-// `dot` (lane j takes elements j, 8 + j, ... in order, the lanes are then summed in order, the tail is added by fused
-// multiply-adds).  A block of four warps computes 8 rows x 16 experts; a group of eight lanes holds 4 rows x 2 experts of it: six
-// shared-memory reads feed eight multiply-adds.  Columns are staged 512 at a time by 16-byte cp.async, double-buffered; the row pitch
-// (516 words) puts the four groups of a warp on disjoint banks.
-// What bounds it: one warp a scheduler, whose chain of reads and multiply-adds nothing hides (24 reads a column of eight and block).
-// Measured (128 experts x 2048, 256 rows): 18.5 us; 256 columns at a time through registers, 2 x 2 a group: 19.7.
-constexpr int kRtRows = 8, kRtExperts = 16, kRtK = 512, kRtPitch = kRtK + 4, kRtBuf = (kRtRows + kRtExperts) * kRtPitch;
+// `dot` (lane j takes elements j, 8 + j, ... in order, the lanes are then summed in order; rows are whole groups of eight).  A lane has 4 rows x 4 experts, a warp 4 x 16, a block of four warps 16 x 16.  Columns come 512 at a time, a bulk copy a row (the copy engine
+// takes a row in 45 cycles, however short), into a ring of three; the row pitch (520 words) puts the four groups of a warp on disjoint banks.
+// What bounds it: shared memory delivers 128 bytes a cycle to registers however many lanes share an address, so that the work per value read counts: 8
+// reads feed 16 multiply-adds (128 experts x 2048, 256 rows: 7100 cycles), where 6 fed 8.  Behind that one warp a scheduler.
+// Measured there: 13.6 us (the first copies land after 3.3, 16000 cycles are reads and multiply-adds), 18.7 before; 512 rows of 4096: 46, 66.  (Columns
+// 256 at a time 18.7; a row and two experts a thread by 16-byte reads and packed multiply-adds 21.7.)
+constexpr int kRtRows = 16, kRtExperts = 16, kRtK = 512, kRtPitch = kRtK + 8, kRtBuf = (kRtRows + kRtExperts) * kRtPitch, kRtRing = 3;
 __global__ void __launch_bounds__(128) moe_router_kernel(const float *__restrict__ router, const float *x,
-                                                         float *__restrict__ logits, int rows, int ne, int n_expert) {
-    pdl_go();
-    pdl_wait();
-    extern __shared__ __align__(16) float s_rt[];  // [2][8 rows, 16 router rows][kRtPitch]
+                                                         float *__restrict__ logits, int rows, int ne, int n_expert, uint32_t *__restrict__ status) {
+    extern __shared__ __align__(16) float s_rt[];  // [kRtRing][16 rows, 16 router rows][kRtPitch]
+    __shared__ uint64_t bars[kRtRing];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, grp = lane >> 3, j = lane & 7;
     const int r0 = blockIdx.x * kRtRows, e0 = blockIdx.y * kRtExperts;
-    const int rl = (warp >> 1) * 4, el = (warp & 1) * 8 + grp * 2;  // the group's first row and expert
-    const int kend = ne / 8 * 8;  // whole groups of eight columns; the rest is the tail
-    const bool vec = (ne & 3) == 0 && (((uintptr_t)x | (uintptr_t)router) & 15) == 0;
-    auto fetch = [&](int k0) {
-        float *dst = s_rt + ((k0 / kRtK) & 1) * kRtBuf;
-        for (int i = threadIdx.x; i < (kRtRows + kRtExperts) * (kRtK / 4); i += 128) {
-            const int r = i / (kRtK / 4), k = (i % (kRtK / 4)) * 4;
-            const bool is_w = r >= kRtRows;
-            const int gr = is_w ? e0 + r - kRtRows : r0 + r;
-            if (gr >= (is_w ? n_expert : rows) || k0 + k >= kend) continue;  // (never read, or multiplied into a sum that is not stored)
-            const float *src = (is_w ? router : x) + (size_t)gr * ne + k0 + k;
-            float *d = dst + r * kRtPitch + k;
-            if (vec) {
-                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(d)), "l"(src) : "memory");
-            } else {
-                for (int q = 0; q < 4; q++)
-                    if (k0 + k + q < kend) d[q] = src[q];
-            }
-        }
-        asm volatile("cp.async.commit_group;" ::: "memory");
+    const int rl = warp * 4;  // the warp's first row; its group has experts grp, grp + 4, ...
+    const int n_chunks = (ne + kRtK - 1) / kRtK;
+    auto su32 = [](const void *p) { return (uint32_t)__cvta_generic_to_shared(p); };
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < kRtRing; i++) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(su32(&bars[i])) : "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncthreads();
+    pdl_go();
+    pdl_wait();
+    // columns c * kRtK .. of the block's rows and router rows (rows past the last are not read: what is there goes into sums that are not stored)
+    auto source = [&](int i) { return i < kRtRows ? (r0 + i < rows ? x + (size_t)(r0 + i) * ne : nullptr) : (e0 + i - kRtRows < n_expert ? router + (size_t)(e0 + i - kRtRows) * ne : nullptr); };
+    auto fetch = [&](int c) {  // (warp 0: a row a lane)
+        const float *src = source(lane);
+        const uint32_t bytes = (uint32_t)min(kRtK, ne - c * kRtK) * 4, bar = su32(&bars[c % kRtRing]), n = __popc(__ballot_sync(0xffffffffu, src != nullptr));
+        if (lane == 0) asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(n * bytes) : "memory");
+        __syncwarp();
+        if (src)
+            asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                             su32(s_rt + (c % kRtRing) * kRtBuf + lane * kRtPitch)),
+                         "l"(src + c * kRtK), "r"(bytes), "r"(bar)
+                         : "memory");
     };
-    float acc[4][2];
-#pragma unroll
-    for (int a = 0; a < 4; a++) acc[a][0] = acc[a][1] = 0.f;
-    fetch(0);
-    for (int k0 = 0; k0 < kend; k0 += kRtK) {
-        if (k0 + kRtK < kend) {
-            fetch(k0 + kRtK);
-            asm volatile("cp.async.wait_group 1;" ::: "memory");
-        } else {
-            asm volatile("cp.async.wait_group 0;" ::: "memory");
+    auto landed = [&](int c) {
+        for (uint32_t i = 0; i < (1u << 22); i++) {
+            uint32_t ok;
+            asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                         : "=r"(ok)
+                         : "r"(su32(&bars[c % kRtRing])), "r"((uint32_t)(c / kRtRing) & 1u)
+                         : "memory");
+            if (ok) return true;
         }
-        __syncthreads();
-        const float *b = s_rt + ((k0 / kRtK) & 1) * kRtBuf + j, *xa = b + rl * kRtPitch, *wa = b + (kRtRows + el) * kRtPitch;
-        const int kc = min(kRtK, kend - k0);
+        return false;
+    };
+    if (warp == 0)
+        for (int c = 0; c < kRtRing && c < n_chunks; c++) fetch(c);
+    float acc[4][4];
+#pragma unroll
+    for (int a = 0; a < 16; a++) (&acc[0][0])[a] = 0.f;
+    for (int c0 = 0; c0 < n_chunks; c0++) {
+        const int kc = min(kRtK, ne - c0 * kRtK);
+        const float *buf = s_rt + (c0 % kRtRing) * kRtBuf;
+        if (!__syncthreads_and(landed(c0))) {  // give up; the copies in flight get their own limit
+            if (threadIdx.x == 0) atomicExch(status, 14u);
+            for (int c = c0 + 1; c < c0 - 1 + kRtRing && c < n_chunks; c++) landed(c);
+            return;
+        }
+        if (warp == 0 && c0 >= 1 && c0 - 1 + kRtRing < n_chunks) {  // everybody has finished with the columns before these
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            fetch(c0 - 1 + kRtRing);
+        }
+        const float *xa = buf + rl * kRtPitch + j, *wa = buf + (kRtRows + grp) * kRtPitch + j;
 #pragma unroll 8
         for (int c = 0; c < kc; c += 8) {
-            const float w0 = wa[c], w1 = wa[kRtPitch + c];
+            float v[4], w[4];
 #pragma unroll
-            for (int a = 0; a < 4; a++) {
-                const float v = xa[a * kRtPitch + c];
-                acc[a][0] = fmaf(w0, v, acc[a][0]);
-                acc[a][1] = fmaf(w1, v, acc[a][1]);
-            }
+            for (int a = 0; a < 4; a++) v[a] = xa[a * kRtPitch + c], w[a] = wa[4 * a * kRtPitch + c];
+#pragma unroll
+            for (int a = 0; a < 4; a++)
+#pragma unroll
+                for (int b = 0; b < 4; b++) acc[a][b] = fmaf(w[b], v[a], acc[a][b]);
         }
-        __syncthreads();  // everybody has finished with these columns
     }
 #pragma unroll
     for (int a = 0; a < 4; a++)
 #pragma unroll
-        for (int b = 0; b < 2; b++) {
-            // s = ((((acc0 + acc1) + acc2) + ...) + acc7), then the FMA tail
+        for (int b = 0; b < 4; b++) {
+            // s = ((((acc0 + acc1) + acc2) + ...) + acc7)
             float sum = 0.f;
 #pragma unroll
             for (int k = 0; k < 8; k++) sum = __fadd_rn(sum, __shfl_sync(0xffffffffu, acc[a][b], grp * 8 + k));
-            const int r = r0 + rl + a, e = e0 + el + b;
-            if (r < rows && e < n_expert) {
-                const float *w = router + (size_t)e * ne, *xr = x + (size_t)r * ne;
-                for (int i = kend; i < ne; i++) sum = fmaf(w[i], xr[i], sum);
-                if (j == 0) logits[(size_t)r * n_expert + e] = sum;
-            }
+            const int r = r0 + rl + a, e = e0 + grp + 4 * b;
+            if (j == ((a * 4 + b) & 7) && r < rows && e < n_expert) logits[(size_t)r * n_expert + e] = sum;
         }
 }
 
@@ -345,10 +356,10 @@ __global__ void __launch_bounds__(256) moe_combine_kernel(const float *y_pairs, 
 }
 
 cudaError_t launch_moe_router(const float *router, const float *x, float *logits, int rows, int ne, int n_expert,
-                              const DeviceInfo &dev, cudaStream_t st) {
+                              const DeviceInfo &dev, uint32_t *status, cudaStream_t st) {
     if (rows < 1 || n_expert < 1) return cudaErrorInvalidValue;
     const dim3 grid((unsigned)((rows + kRtRows - 1) / kRtRows), (unsigned)((n_expert + kRtExperts - 1) / kRtExperts));
-    if (grid.y > 65535) return cudaErrorInvalidValue;
+    if (grid.y > 65535 || ne % 8 || (((uintptr_t)x | (uintptr_t)router) & 15)) return cudaErrorInvalidValue;
     // A few rows: a warp an expert and four rows, all columns staged at once, as long as its CTAs are four waves at most.  Measured, tiles /
     // rows (us a layer; waves): 27 rows, 128 experts x 2048 15 / 7.4 (the router alone); 64 rows, 64 experts x 2048 (0.6) 85 / 71,
     // 128 x 4096 (3.5) 155 / 145, 512 x 1024 (2.3) 72 / 77, 256 x 4096 (6.9) 163 / 175; 48 rows, 192 x 6144 (3.9) 205 / 195, 256 x 6144
@@ -360,15 +371,16 @@ cudaError_t launch_moe_router(const float *router, const float *x, float *logits
         if (e != cudaErrorInvalidValue) return e;
         cudaGetLastError();
     }
-    const size_t smem = (size_t)2 * kRtBuf * 4;
+    const size_t smem = (size_t)kRtRing * kRtBuf * 4;
     cudaError_t e = cudaFuncSetAttribute(moe_router_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    return launch_pdl(moe_router_kernel, grid, dim3(128), smem, st, router, x, logits, rows, ne, n_expert);
+    return launch_pdl(moe_router_kernel, grid, dim3(128), smem, st, router, x, logits, rows, ne, n_expert, status);
 }
 
 cudaError_t launch_moe_route(const float *logits, int rows, int n_expert, int n_used, float scale, int norm_w,
                              int32_t *sel_ids, float *sel_w, cudaStream_t st) {
     if (n_expert > 1024 || n_used > 32 || n_used > n_expert) return cudaErrorInvalidValue;
+    if (n_expert <= 256) return launch_moe_route_rows(logits, rows, n_expert, n_used, scale, norm_w, sel_ids, sel_w, st);
     const int warps = 4;
     return launch_pdl(moe_route_kernel, dim3((unsigned)((rows + warps - 1) / warps)), dim3(warps * 32), (size_t)warps * n_expert * 4, st, logits, rows,
                       n_expert, n_used, scale, norm_w, sel_ids, sel_w);

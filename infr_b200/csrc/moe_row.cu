@@ -132,6 +132,23 @@ __device__ __forceinline__ void moe_route_row(const float *logits, float *p, int
     weight = norm_w ? __fmul_rn(__fdiv_rn(myw, wsum), scale) : __fmul_rn(myw, scale);
 }
 
+// ---- routing of many rows: one warp each.  (128 experts, 8 of them, 256 rows: 4.2 us; probabilities in shared memory and shuffles for every round
+// of the choice, as moe_route_kernel has them for more than 256 experts, 6.4.)
+constexpr int kRouteWarps = 4;
+template <int EPL>
+__global__ void __launch_bounds__(kRouteWarps * 32) moe_route_rows_kernel(const float *logits, int rows, int n_expert, int n_used, float scale, int norm_w,
+                                                                          int32_t *__restrict__ sel_ids, float *__restrict__ sel_w) {
+    __shared__ __align__(16) float s_p[kRouteWarps][32 * EPL];
+    pdl_go();
+    pdl_wait();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, r = blockIdx.x * kRouteWarps + warp;
+    if (r >= rows) return;
+    int id;
+    float w;
+    moe_route_row<EPL>(logits + (size_t)r * n_expert, s_p[warp], n_expert, n_used, scale, norm_w, lane, id, w);
+    if (lane < n_used) sel_ids[(size_t)r * n_used + lane] = id, sel_w[(size_t)r * n_used + lane] = w;
+}
+
 // Activations of a 256-element block as the lanes consume them: four lanes, lane t the sub-blocks 2t and 2t + 1; 16-byte unit
 // u * 4 + t holds elements 2u, 2u + 1 of both: (lo, hi, lo, hi).  Blocks are 64 bytes more than their kilobyte apart: the two blocks of
 // eight lanes' 16-byte reads lie on different banks.
@@ -333,6 +350,13 @@ cudaError_t launch_moe_router_row(const float *router, const float *x, float *lo
     if (e != cudaSuccess) return e;
     const dim3 grid((unsigned)((n_expert + kRtWarps - 1) / kRtWarps), (unsigned)((rows + kRtRowsCta - 1) / kRtRowsCta));
     return launch_pdl(moe_router_row_kernel, grid, dim3(kRtWarps * 32), smem, st, router, x, logits, rows, ne, n_expert);
+}
+// cudaErrorInvalidValue: more experts than a warp's registers take here.
+cudaError_t launch_moe_route_rows(const float *logits, int rows, int n_expert, int n_used, float scale, int norm_w, int32_t *sel_ids, float *sel_w, cudaStream_t st) {
+    if (n_expert > 256) return cudaErrorInvalidValue;
+    auto kernel = n_expert <= 32 ? moe_route_rows_kernel<1> : n_expert <= 64 ? moe_route_rows_kernel<2> : n_expert <= 128 ? moe_route_rows_kernel<4> : moe_route_rows_kernel<8>;
+    return launch_pdl(kernel, dim3((unsigned)((rows + kRouteWarps - 1) / kRouteWarps)), dim3(kRouteWarps * 32), 0, st, logits, rows, n_expert, n_used, scale, norm_w,
+                      sel_ids, sel_w);
 }
 cudaError_t launch_moe_gate_up_row(const float *logits, const float *x, const uint8_t *gate, const uint8_t *up, float *act, int32_t *sel_ids, float *sel_w, int ne,
                                    int nff, int n_expert, int n_used, float scale, int norm_w, const DeviceInfo &dev, cudaStream_t st) {
