@@ -6,11 +6,12 @@
 // All of them are HBM- or latency-bound elementwise / reduction kernels; every kernel waits for its producer
 // with `griddepcontrol.wait` before its first read, so a chain of them can overlap launch with the tail of
 // the previous kernel.
-#include <type_traits>
+#include <cuda.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <type_traits>
 
 #include "kernels.h"
 
@@ -196,9 +197,7 @@ constexpr int kAttnTile = 128;     // keys per CTA
 constexpr int kAttnThreads = 256;  // eight warps: 16 keys each in the score phase, 16 output dims each in the value phase
 
 // CTA = (key tile, KV head, query row).  The tile's 128 key rows and 128 value rows (head_dim halves each) are
-// copied into shared memory with 16-byte cp.async, consecutive threads taking consecutive 16-byte pieces of a row, so
-// every global request is a whole 128-byte line; all copies of the CTA are in flight together and none occupies a
-// register.
+// copied into shared memory, all copies of the CTA in flight together and none in a register.
 //
 // Both products run on the warp-level matrix unit in f16 WITHOUT giving up f32 operands: the cache values are f16, and the f32 operand (q,
 // then the softmax weights p) is split into two f16 pieces, hi = its top 11 significant bits, mid = the next 11 of the remainder times 2^11,
@@ -213,12 +212,78 @@ constexpr int kAttnThreads = 256;  // eight warps: 16 keys each in the score pha
 // A = the values transposed (ldmatrix.trans), B = the weight pieces, K = the keys in steps of 8; with head_dim 64 the
 // two halves of the keys go to two warps and meet in shared memory (over the key tile, dead by then).  The tile's
 // (m, l, o) goes to the workspace for the merge kernel.
+// A tile's keys or values in shared memory: kAttnTile rows of HD halves.  frag: the 16-byte piece 2 j + hi (hi = 0, 1) of a row;
+// that of the row 8 n rows on is 8 n kStride bytes on.  Either way the eight rows
+// of an ldmatrix lie in distinct banks.
 template <int HD>
-struct AttnSmem {
-    static constexpr int kKeyStride = HD * 2 + 16;  // bytes; 16 past a multiple of 128: the 8 rows of an ldmatrix hit distinct banks
-    static constexpr int kValStride = HD * 2 + 16;
-    static constexpr int kBytes = kAttnTile * (kKeyStride + kValStride);
+struct PaddedTile {  // rows 16 bytes past a multiple of 128
+    static constexpr int kStride = HD * 2 + 16, kBytes = kAttnTile * kStride, kAlign = 16;
+    static __device__ __forceinline__ uint8_t *frag(uint8_t *tile, int row, int hi, int j) { return tile + row * kStride + hi * 16 + j * 32; }
 };
+template <int HD>
+struct BoxedTile {  // as tensor copies of rows x 64 halves with the 128-byte swizzle leave it, the first 64 dims first
+    static constexpr int kStride = 128, kBytes = kAttnTile * HD * 2, kAlign = 1024;
+    static __device__ __forceinline__ uint8_t *frag(uint8_t *tile, int row, int hi, int j) {
+        return tile + row * 128 + (j >> 2) * (kAttnTile * 128) + ((((hi ^ row) & 7) << 4) ^ ((j & 3) << 5));
+    }
+};
+constexpr int kBoxRows = 16;
+__device__ __forceinline__ int boxed_rows(int keys) { return (keys + kBoxRows - 1) / kBoxRows * kBoxRows; }
+// dynamic shared memory from a multiple of the tile's alignment on
+template <class T>
+__device__ __forceinline__ uint8_t *align_tile(uint8_t *p) {
+    return p + (-(uint32_t)__cvta_generic_to_shared(p) & (T::kAlign - 1));
+}
+template <class T>
+constexpr int kTileBytes = 2 * T::kBytes + T::kAlign - 16;
+// Maps of the caches (rows of n_kv * HD halves), keys and values, in boxes of a whole tile's rows and of kBoxRows.
+struct AttnMaps {
+    CUtensorMap whole[2], part[2];
+};
+struct NoMaps {};
+// By one thread; by the whole CTA with the maps
+template <int HD>
+__device__ __forceinline__ void init_bars(uint64_t *s_bar) {
+#pragma unroll
+    for (int i = 0; i < 2; i++)
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"((uint32_t)__cvta_generic_to_shared(s_bar + i)), "n"(HD / 64) : "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+}
+template <int HD>
+__device__ __forceinline__ void init_bars(uint64_t *s_bar, const AttnMaps &maps) {
+    if (threadIdx.x % 32 == 0 && threadIdx.x < 128) asm volatile("prefetch.tensormap [%0];" ::"l"(maps.whole + threadIdx.x / 32) : "memory");
+    if (threadIdx.x == 0) init_bars<HD>(s_bar);
+}
+// Warps 0 .. HD / 32 - 1 fetch a tile, from row `row0` of a sequence's caches on: warp w the dims 64 (w / 2) .. + 63 of the keys (even) or values, in one copy; of a tile of
+// fewer than 128 keys the boxes with keys.  What bounds a batch's attention is how many bytes an SM has on their way, three tiles at most: the time a tile takes to
+// ask for its bytes counts in full.  32 sequences at 4097 keys, us a call with the merge: a bulk copy for every row (a warp issues those of its lanes one
+// after the other) 102.6; 16 boxes a warp 98; this 91.8 (skeleton without arithmetic: 89).  head_dim 64, 16 heads / 16: 130 -> 90.
+template <int HD>
+__device__ __forceinline__ void fetch_tile(const AttnMaps &maps, uint8_t *s_k, uint8_t *s_v, uint64_t *s_bar, int kvh, int row0, int seq, int keys) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, which = warp & 1, half = warp >> 1;
+    if (half >= HD / 64) return;
+    const uint32_t b = (uint32_t)__cvta_generic_to_shared(s_bar + which), to = (uint32_t)__cvta_generic_to_shared(which ? s_v : s_k) + half * (kAttnTile * 128);
+    if (lane == 0)
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(b), "r"((uint32_t)(boxed_rows(keys) * 128)) : "memory");
+    __syncwarp();
+    auto copy = [&](const CUtensorMap *map, int first) {
+        asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(to + first * 128), "l"(map),
+                     "r"(kvh * HD + half * 64), "r"(row0 + first), "r"(seq), "r"(b)
+                     : "memory");
+    };
+    if (keys == kAttnTile) {
+        if (lane == 0) copy(maps.whole + which, 0);
+    } else if (lane * kBoxRows < keys) {
+        copy(maps.part + which, lane * kBoxRows);
+    }
+}
+// Rows r0 .. r1 - 1 of the values, past the end of a tile: the matrix unit is to multiply 0 (not stale bits) by the weight 0.  Those of a box that
+// is fetched once it has landed, the others at once.  (Scores past the end are not looked at.)
+template <class T, int HD>
+__device__ __forceinline__ void zero_rows(uint8_t *s_v, int r0, int r1) {
+    for (int i = threadIdx.x; i < (r1 - r0) * (HD / 8); i += kAttnThreads)
+        *reinterpret_cast<uint4 *>(T::frag(s_v, r0 + i / (HD / 8), i & 1, i % (HD / 8) >> 1)) = make_uint4(0, 0, 0, 0);
+}
 
 __device__ __forceinline__ void cp_async16(void *smem, const void *gmem) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(smem)), "l"(gmem) : "memory");
@@ -393,17 +458,16 @@ __device__ __forceinline__ void pairs_tf32(int p0, int p_end, const Frag &frag, 
 // loses bits too, so the scores come again from q.  q, part_o, part_ml: of row 0 and head 0 of the group.
 // A function of its own behind which the kernels return (few tiles need it), its arguments in registers: as a structure they lie in local memory, which
 // has little L1 beside that much shared memory (1 us a tile).  Where every tile takes it: 32 sequences at 4097 keys, 32 heads / 8, 103 -> 121 us.
-template <int HD, int G, int P>
+template <class T, int HD, int G, int P>
 __device__ __noinline__ void tile_tf32(uint8_t *s_k, uint8_t *s_v, float *sc, const float *f, float (*ml)[2], const float *q, float *part_o, float *part_ml, int n_head,
                                        int n_splits, int pairs, int keys0, float scale, bool rescore) {
-    using L = AttnSmem<HD>;
     constexpr int DG = HD / 16, KP = (kAttnThreads / 32) / DG, KEYS = kAttnTile / KP, NT = (P + 3) / 4, NT1 = (G + 3) / 4;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g8 = lane >> 2;
     auto out_of = [&](int pair) { return ((size_t)(pair / G) * n_head + pair % G) * n_splits; };
     if (rescore) {  // scores of keys 16 warp .. 16 warp + 15
-        const uint8_t *arow = s_k + (size_t)(16 * warp + (lane & 7) + ((lane >> 3) & 1) * 8) * L::kKeyStride + (lane >> 4) * 16;
+        const int arow = 16 * warp + (lane & 7) + ((lane >> 3) & 1) * 8;
         pairs_tf32<NT, HD / 16>(
-            0, pairs, [&](uint32_t(&r)[4], int j) { ldsm4(r, arow + j * 32); }, [&](int p) { return q + ((size_t)(p / G) * n_head + p % G) * HD; },
+            0, pairs, [&](uint32_t(&r)[4], int j) { ldsm4(r, T::frag(s_k, arow, lane >> 4, j)); }, [&](int p) { return q + ((size_t)(p / G) * n_head + p % G) * HD; },
             [&](int p, float v0, float v1) { sc[p * kAttnTile + 16 * warp + g8] = v0, sc[p * kAttnTile + 16 * warp + g8 + 8] = v1; });
         __syncthreads();
     }
@@ -418,11 +482,11 @@ __device__ __noinline__ void tile_tf32(uint8_t *s_k, uint8_t *s_v, float *sc, co
     // output dims 16 dg .. + 15 over this warp's share of the keys; a row at a time, last row first, where the rows see different keys: 0 must not
     // meet an infinity of a later token
     const int dg = warp % DG, kp = warp / DG, nr = pairs / G;
-    const uint8_t *vrow = s_v + (size_t)(kp * KEYS + (lane & 7) + (lane >> 4) * 8) * L::kValStride + (size_t)(16 * dg + ((lane >> 3) & 1) * 8) * 2;
+    const uint8_t *vrow = T::frag(s_v, kp * KEYS + (lane & 7) + (lane >> 4) * 8, (lane >> 3) & 1, dg);
     float *s_o = reinterpret_cast<float *>(s_k);  // KP > 1: [KP][G][HD], the key tile is dead
     auto values = [&](auto ntc, int first, int end) {
         pairs_tf32<decltype(ntc)::value, KEYS / 16>(
-            first, end, [&](uint32_t(&r)[4], int j) { ldsm4_trans(r, vrow + (size_t)j * 16 * L::kValStride); }, [&](int p) { return sc + p * kAttnTile + kp * KEYS; },
+            first, end, [&](uint32_t(&r)[4], int j) { ldsm4_trans(r, vrow + j * 16 * T::kStride); }, [&](int p) { return sc + p * kAttnTile + kp * KEYS; },
             [&](int p, float v0, float v1) {
                 float *o = (KP == 1 ? part_o + out_of(p) * HD : s_o + (kp * G + p) * HD) + 16 * dg + g8;
                 o[0] = v0, o[8] = v1;
@@ -434,7 +498,7 @@ __device__ __noinline__ void tile_tf32(uint8_t *s_k, uint8_t *s_v, float *sc, co
         for (int r = nr - 1; r >= 0 && keys0 + r > 0; r--) {
             if (r != nr - 1) {
                 __syncthreads();  // the row after this one has been multiplied
-                if (keys0 + r < kAttnTile && tid < HD / 8) *reinterpret_cast<uint4 *>(s_v + (keys0 + r) * L::kValStride + tid * 16) = make_uint4(0, 0, 0, 0);
+                if (keys0 + r < kAttnTile && tid < HD / 8) *reinterpret_cast<uint4 *>(T::frag(s_v, keys0 + r, tid & 1, tid >> 1)) = make_uint4(0, 0, 0, 0);
                 __syncthreads();
             }
             values(std::integral_constant<int, NT1>{}, r * G, r * G + G);
@@ -454,21 +518,21 @@ __device__ __noinline__ void tile_tf32(uint8_t *s_k, uint8_t *s_v, float *sc, co
 constexpr int kAttnChunkPairs = 16;   // (query row, head) pairs of a chunk's tile
 constexpr int kAttnPad = 8;  // halves behind a column of 64 or 128: the eight columns of a read start four banks apart
 
-template <int HD, int G, bool BULK>
+template <int HD, int G, bool BOXED>
 __global__ void __launch_bounds__(kAttnThreads) attn_split_kernel(const float *q, const __half *k_cache,
                                                                const __half *v_cache, float *__restrict__ part_o,
                                                                float *__restrict__ part_ml, int rows, int n_head, int n_kv, int pos,
                                                                float scale, int n_splits, size_t seq_stride, uint32_t *__restrict__ status,
                                                                const int32_t *seq_pos, const int32_t *block_table,
-                                                               int table_stride, int n_pages) {
+                                                               int table_stride, int n_pages, const __grid_constant__ std::conditional_t<BOXED, AttnMaps, NoMaps> maps) {
     constexpr int CPR = HD * 2 / 16;           // 16-byte pieces per row
     constexpr int NT = (2 * G + 7) / 8;        // 8-column groups of the instruction: column c = head c / 2, piece c % 2
     constexpr int DG = HD / 16;                // 16-dim output groups
     constexpr int KP = (kAttnThreads / 32) / DG;  // warps per output group: they split the keys (1 for head_dim 128, 2 for 64)
-    using L = AttnSmem<HD>;
+    using T = std::conditional_t<BOXED, BoxedTile<HD>, PaddedTile<HD>>;
     extern __shared__ __align__(16) uint8_t dyn_smem[];
-    uint8_t *s_k = dyn_smem, *s_v = dyn_smem + kAttnTile * L::kKeyStride;
-    float(*s_o)[G][HD] = reinterpret_cast<float(*)[G][HD]>(dyn_smem);  // KP x G x HD floats over the key tile (KP > 1 only)
+    uint8_t *s_k = align_tile<T>(dyn_smem), *s_v = s_k + T::kBytes;
+    float(*s_o)[G][HD] = reinterpret_cast<float(*)[G][HD]>(s_k);  // KP x G x HD floats over the key tile (KP > 1 only)
     constexpr int QS = HD + kAttnPad, PS = kAttnTile + kAttnPad;
     __shared__ __align__(16) __half s_q[NT * 8 * QS];  // columns past 2 G are never stored
     __shared__ __align__(16) __half s_p[NT * 8 * PS];
@@ -477,13 +541,17 @@ __global__ void __launch_bounds__(kAttnThreads) attn_split_kernel(const float *q
     __shared__ float s_ml[G][2];
     __shared__ __align__(8) uint64_t s_bar[2];
     __shared__ int s_short[2];  // a weight, an element of a query loses bits
-    static_assert(KP * G * HD * 4 <= kAttnTile * L::kKeyStride, "the partial outputs reuse the key tile");
+    static_assert(KP * G * HD * 4 <= T::kBytes, "the partial outputs reuse the key tile");
     static_assert(KP >= 1 && KP * DG == kAttnThreads / 32, "head_dim 64 or 128");
     const int split = blockIdx.x, kvh = blockIdx.y, qr = blockIdx.z;
     const int seq = qr / rows, ti = qr % rows;
     const int key0 = split * kAttnTile;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g8 = lane >> 2, t4 = lane & 3;
     if (tid < 2) s_short[tid] = 0;
+    if constexpr (BOXED) {
+        init_bars<HD>(s_bar, maps);
+        __syncthreads();
+    }
     pdl_go();
     pdl_wait();
     // sequences at positions of their own (seq_pos, written by an earlier kernel or the host): `pos` is their maximum
@@ -496,70 +564,40 @@ __global__ void __launch_bounds__(kAttnThreads) attn_split_kernel(const float *q
         }
         return;
     }
+    // contiguous caches: the sequence's own rows; paged: the tile is one page of the pool (a page holds a tile's 128 rows)
     const size_t kv_row = (size_t)n_kv * HD;
-    // contiguous caches: the sequence's own; paged: the tile is one page of the pool (a page holds a tile's 128 rows)
-    const size_t tile_off = block_table ? (size_t)min(max(block_table[(size_t)seq * table_stride + split], 0), n_pages - 1) * kAttnTile * kv_row
-                                        : (size_t)seq * seq_stride + (size_t)key0 * kv_row;
-    const __half *kbase = k_cache + (size_t)kvh * HD + tile_off;
-    const __half *vbase = v_cache + (size_t)kvh * HD + tile_off;
+    const int page = block_table ? min(max(block_table[(size_t)seq * table_stride + split], 0), n_pages - 1) : 0;
     const int tile_keys = min(kAttnTile, n_keys - key0);
-    // Two ways to fetch the tile.  BULK (many CTAs per SM over the launch: a batch of sequences): one bulk copy per row
-    // (head_dim halves, contiguous in the cache) into the padded tile, thread r < 128 the key row r, thread 128 + r the
-    // value row r, so a tile costs each warp two instructions instead of 32 cp.async with their address arithmetic (a
-    // third of the kernel's instructions); keys and values complete on separate barriers.  Otherwise (a single wave of
+    // Two ways to fetch the tile.  BOXED (more than two waves of CTAs: a batch of sequences): tensor copies of 64 dims, so that
+    // a tile costs its warps next to nothing; keys and values complete on separate barriers.  Otherwise (a single wave of
     // CTAs, where the latency of the first byte is what counts): 16-byte cp.async, consecutive threads taking consecutive
-    // pieces of a row.  Rows past the end of a partial tile are zeroed, so that the matrix unit multiplies 0 (not stale
-    // bits) by the weight 0.
-    if (BULK) {
-        if (tid == 0) {
-#pragma unroll
-            for (int i = 0; i < 2; i++) {
-                const uint32_t b = (uint32_t)__cvta_generic_to_shared(&s_bar[i]);
-                asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(b) : "memory");
-                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(b), "r"((uint32_t)(tile_keys * HD * 2)) : "memory");
-            }
-            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        }
-        __syncthreads();  // the barriers are armed before any copy can complete
-        const int which = tid >> 7, r = tid & (kAttnTile - 1);  // 0: key row r, 1: value row r
-        uint8_t *dst = (which ? s_v + r * L::kValStride : s_k + r * L::kKeyStride);
-        if (r < tile_keys) {
-            const __half *src = (which ? vbase : kbase) + (size_t)r * kv_row;
-            asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                             (uint32_t)__cvta_generic_to_shared(dst)),
-                         "l"(src), "r"((uint32_t)(HD * 2)), "r"((uint32_t)__cvta_generic_to_shared(&s_bar[which]))
-                         : "memory");
-        } else {
-#pragma unroll
-            for (int c = 0; c < CPR; c++) *reinterpret_cast<uint4 *>(dst + c * 16) = make_uint4(0, 0, 0, 0);
-        }
+    // pieces of a row.
+    if constexpr (BOXED) {
+        fetch_tile<HD>(maps, s_k, s_v, s_bar, kvh, block_table ? page * kAttnTile : key0, block_table ? 0 : seq, tile_keys);
     } else {
+        const size_t tile_off = (size_t)kvh * HD + (block_table ? (size_t)page * kAttnTile * kv_row : (size_t)seq * seq_stride + (size_t)key0 * kv_row);
         for (int i = tid; i < tile_keys * CPR; i += kAttnThreads) {
             const int key = i / CPR, c = i % CPR;
-            cp_async16(s_k + key * L::kKeyStride + c * 16, kbase + (size_t)key * kv_row + c * 8);
+            cp_async16(s_k + key * T::kStride + c * 16, k_cache + tile_off + (size_t)key * kv_row + c * 8);
         }
         cp_async_commit();
         for (int i = tid; i < tile_keys * CPR; i += kAttnThreads) {
             const int key = i / CPR, c = i % CPR;
-            cp_async16(s_v + key * L::kValStride + c * 16, vbase + (size_t)key * kv_row + c * 8);
+            cp_async16(s_v + key * T::kStride + c * 16, v_cache + tile_off + (size_t)key * kv_row + c * 8);
         }
         cp_async_commit();
-        for (int i = tid; i < (kAttnTile - tile_keys) * CPR; i += kAttnThreads) {
-            const int key = tile_keys + i / CPR, c = i % CPR;
-            *reinterpret_cast<uint4 *>(s_k + key * L::kKeyStride + c * 16) = make_uint4(0, 0, 0, 0);
-            *reinterpret_cast<uint4 *>(s_v + key * L::kValStride + c * 16) = make_uint4(0, 0, 0, 0);
-        }
     }
+    zero_rows<T, HD>(s_v, BOXED ? boxed_rows(tile_keys) : tile_keys, kAttnTile);
     const float *qrow = q + ((size_t)qr * n_head + (size_t)kvh * G) * HD;
     bool small = false;
     for (int g = warp; g < NT * 4; g += kAttnThreads / 32) {
         const float f = split_query<HD, QS>(qrow + (size_t)g * HD, s_q, g, lane, g < G, small);
         if (lane == 0 && g < G) s_f[g] = f * scale;
     }
-    // the keys have landed; q is staged, the zeroed rows are in place.  (BULK: a bounded wait; if it runs out, the CTA
+    // the keys have landed; q is staged.  (BOXED: a bounded wait; if it runs out, the CTA
     // records it and leaves after the wait for the values has had its own limit, so that no copy can land in shared
     // memory that is no longer this CTA's.)
-    if (BULK) {
+    if (BOXED) {
         const bool k_ok = attn_wait(&s_bar[0]);
         if (!__syncthreads_and(k_ok)) {
             attn_wait(&s_bar[1]);
@@ -576,11 +614,11 @@ __global__ void __launch_bounds__(kAttnThreads) attn_split_kernel(const float *q
 #pragma unroll
         for (int nt = 0; nt < NT; nt++) acc[nt][0] = acc[nt][1] = acc[nt][2] = acc[nt][3] = 0.f;
         // ldmatrix rows: matrices 0 / 1 = keys 0..7 / 8..15 at dims d0.., matrices 2 / 3 = the same keys at dims d0 + 8..
-        const uint8_t *arow = s_k + (size_t)(16 * warp + (lane & 7) + ((lane >> 3) & 1) * 8) * L::kKeyStride + (lane >> 4) * 16;
+        const int arow = 16 * warp + (lane & 7) + ((lane >> 3) & 1) * 8;
 #pragma unroll
         for (int j = 0; j < HD / 16; j++) {
             uint32_t r[4];
-            ldsm4(r, arow + j * 32);
+            ldsm4(r, T::frag(s_k, arow, lane >> 4, j));
 #pragma unroll
             for (int nt = 0; nt < NT; nt++) {
                 uint32_t b0, b1;
@@ -600,7 +638,7 @@ __global__ void __launch_bounds__(kAttnThreads) attn_split_kernel(const float *q
         }
     }
     // the values have landed; scores complete, key tile no longer read
-    if (BULK) {
+    if (BOXED) {
         const bool v_ok = attn_wait(&s_bar[1]);
         if (!__syncthreads_and(v_ok)) {
             if (tid == 0) atomicExch(status, 12u);
@@ -611,13 +649,14 @@ __global__ void __launch_bounds__(kAttnThreads) attn_split_kernel(const float *q
         __syncthreads();
     }
     // ---- phase 2
+    if (BOXED) zero_rows<T, HD>(s_v, tile_keys, boxed_rows(tile_keys));
     if (small) s_short[1] = 1;
     small = false;
     for (int g = warp; g < G; g += kAttnThreads / 32) small = softmax_tile<PS>(s_sc[g], s_p, g, lane, tile_keys, s_f[g], s_ml[g]) || small;
     if (small) s_short[0] = 1;
     __syncthreads();
     if (s_short[0] || s_short[1]) {
-        tile_tf32<HD, G, G>(
+        tile_tf32<T, HD, G, G>(
             s_k, s_v, s_sc[0], s_f, s_ml, qrow, part_o + out_idx * HD, part_ml + out_idx * 2, n_head, n_splits, G, tile_keys, scale, s_short[1] != 0);
         return;
     }
@@ -629,11 +668,11 @@ __global__ void __launch_bounds__(kAttnThreads) attn_split_kernel(const float *q
 #pragma unroll
         for (int nt = 0; nt < NT; nt++) acc[nt][0] = acc[nt][1] = acc[nt][2] = acc[nt][3] = 0.f;
         // ldmatrix.trans rows: matrices 0 / 1 = keys 0..7 at dims 0..7 / 8..15 of the group, matrices 2 / 3 = keys 8..15
-        const uint8_t *vrow = s_v + (size_t)(kp * KEYS + (lane & 7) + (lane >> 4) * 8) * L::kValStride + (size_t)(16 * dg + ((lane >> 3) & 1) * 8) * 2;
+        const uint8_t *vrow = T::frag(s_v, kp * KEYS + (lane & 7) + (lane >> 4) * 8, (lane >> 3) & 1, dg);
 #pragma unroll
         for (int s16 = 0; s16 < KEYS / 16; s16++) {
             uint32_t r[4];
-            ldsm4_trans(r, vrow + (size_t)s16 * 16 * L::kValStride);
+            ldsm4_trans(r, vrow + s16 * 16 * T::kStride);
 #pragma unroll
             for (int nt = 0; nt < NT; nt++) {
                 uint32_t b0, b1;
@@ -681,20 +720,20 @@ __global__ void __launch_bounds__(kAttnThreads) attn_split_kernel(const float *q
 // matrix unit multiplies 0 (not a later token's infinity) by its weight 0.
 // Measured (us a call with the merge, 113 rows at position 384, 32 heads / 8): in tf32 pieces with the edge always row by row and eight warps a merged
 // block 46, now 29 (all eight steps of a product unrolled 31.5).
-template <int G>
+template <int G, bool BOXED>
 __global__ void __launch_bounds__(kAttnThreads) attn_chunk_kernel(const float *q, const __half *k_cache,
                                                                   const __half *v_cache, float *__restrict__ part_o,
                                                                   float *__restrict__ part_ml, int rows, int n_head, int n_kv, int pos, float scale,
                                                                   int n_splits, size_t seq_stride, uint32_t *__restrict__ status,
                                                                   const int32_t *seq_pos, const int32_t *block_table,
-                                                                  int table_stride, int n_pages) {
+                                                                  int table_stride, int n_pages, const __grid_constant__ std::conditional_t<BOXED, AttnMaps, NoMaps> maps) {
     constexpr int HD = 128, P = kAttnChunkPairs, S = HD + kAttnPad, R = P / G, CPR = HD * 2 / 16, NT = 2 * P / 8, NT1 = (2 * G + 7) / 8;
     static_assert(kAttnTile == HD, "one stride for queries and weights");
-    using L = AttnSmem<HD>;
+    using T = std::conditional_t<BOXED, BoxedTile<HD>, PaddedTile<HD>>;
     static_assert(kAttnThreads / 32 == HD / 16, "a warp owns 16 output dims");
     extern __shared__ __align__(16) uint8_t dyn_smem[];
-    uint8_t *s_k = dyn_smem, *s_v = dyn_smem + kAttnTile * L::kKeyStride;
-    __half *s_q = reinterpret_cast<__half *>(dyn_smem + L::kBytes);        // [2 P][S]: the queries' pieces
+    uint8_t *s_k = align_tile<T>(dyn_smem), *s_v = s_k + T::kBytes;
+    __half *s_q = reinterpret_cast<__half *>(s_v + T::kBytes);        // [2 P][S]: the queries' pieces
     __half *s_p = s_q + 2 * P * S;                                         // [2 P][S]: the weights' pieces
     float(*s_sc)[kAttnTile] = reinterpret_cast<float(*)[kAttnTile]>(s_p + 2 * P * S);  // [P][128]
     __shared__ float s_f[P];
@@ -705,6 +744,12 @@ __global__ void __launch_bounds__(kAttnThreads) attn_chunk_kernel(const float *q
     const int split = blockIdx.x, kvh = blockIdx.y, seq = blockIdx.z / row_blocks, ti0 = (blockIdx.z % row_blocks) * R, nr = min(R, rows - ti0);
     const int key0 = split * kAttnTile;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g8 = lane >> 2, t4 = lane & 3;
+    if (tid < 2) s_short[tid] = 0;
+    if constexpr (BOXED)
+        init_bars<HD>(s_bar, maps);
+    else if (tid == 0)
+        init_bars<64>(s_bar);
+    __syncthreads();
     pdl_go();
     pdl_wait();
     const int base = (seq_pos ? max(0, min(seq_pos[seq], pos)) : pos) + ti0 + 1 - key0;  // keys of this tile that row r sees: base + r
@@ -716,36 +761,24 @@ __global__ void __launch_bounds__(kAttnThreads) attn_chunk_kernel(const float *q
         if (tid < nr * G) part_ml[out_of(tid) * 2] = -INFINITY, part_ml[out_of(tid) * 2 + 1] = 0.f;
         return;
     }
+    const int page = block_table ? min(max(block_table[(size_t)seq * table_stride + split], 0), n_pages - 1) : 0;
     const size_t kv_row = (size_t)n_kv * HD;
-    const size_t tile_off = block_table ? (size_t)min(max(block_table[(size_t)seq * table_stride + split], 0), n_pages - 1) * kAttnTile * kv_row
-                                        : (size_t)seq * seq_stride + (size_t)key0 * kv_row;
-    const __half *kbase = k_cache + (size_t)kvh * HD + tile_off;
-    const __half *vbase = v_cache + (size_t)kvh * HD + tile_off;
-    if (tid == 0) {
-        s_short[0] = s_short[1] = 0;
-#pragma unroll
-        for (int i = 0; i < 2; i++) {
-            const uint32_t b = (uint32_t)__cvta_generic_to_shared(&s_bar[i]);
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(b) : "memory");
-            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(b), "r"((uint32_t)(tile_keys * HD * 2)) : "memory");
-        }
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    __syncthreads();  // the barriers are armed before any copy can complete
-    {
-        const int which = tid >> 7, r = tid & (kAttnTile - 1);  // 0: key row r, 1: value row r
-        uint8_t *dst = (which ? s_v + r * L::kValStride : s_k + r * L::kKeyStride);
+    if constexpr (BOXED) {
+        fetch_tile<HD>(maps, s_k, s_v, s_bar, kvh, block_table ? page * kAttnTile : key0, block_table ? 0 : seq, tile_keys);
+    } else {  // a bulk copy for a row: thread r < 128 the key row r, thread 128 + r the value row r
+        const int which = tid >> 7, r = tid & (kAttnTile - 1);
+        const uint32_t b = (uint32_t)__cvta_generic_to_shared(s_bar + which);
+        if (r == 0) asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(b), "r"((uint32_t)(tile_keys * HD * 2)) : "memory");
+        __syncthreads();  // the barriers are armed before any copy can complete
         if (r < tile_keys) {
-            const __half *src = (which ? vbase : kbase) + (size_t)r * kv_row;
+            const __half *src = (which ? v_cache : k_cache) + (size_t)kvh * HD + (block_table ? (size_t)page * kAttnTile * kv_row : (size_t)seq * seq_stride + (size_t)key0 * kv_row) + (size_t)r * kv_row;
             asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                             (uint32_t)__cvta_generic_to_shared(dst)),
-                         "l"(src), "r"((uint32_t)(HD * 2)), "r"((uint32_t)__cvta_generic_to_shared(&s_bar[which]))
+                             (uint32_t)__cvta_generic_to_shared(T::frag(which ? s_v : s_k, r, 0, 0))),
+                         "l"(src), "r"((uint32_t)(HD * 2)), "r"(b)
                          : "memory");
-        } else {
-#pragma unroll
-            for (int c = 0; c < CPR; c++) *reinterpret_cast<uint4 *>(dst + c * 16) = make_uint4(0, 0, 0, 0);
         }
     }
+    zero_rows<T, HD>(s_v, BOXED ? boxed_rows(tile_keys) : tile_keys, kAttnTile);
     const float *qrow = q + (((size_t)seq * rows + ti0) * n_head + (size_t)kvh * G) * HD;
     bool small = false;
     for (int pair = warp; pair < P; pair += kAttnThreads / 32) {
@@ -765,11 +798,11 @@ __global__ void __launch_bounds__(kAttnThreads) attn_chunk_kernel(const float *q
         float acc[NT][4];
 #pragma unroll
         for (int nt = 0; nt < NT; nt++) acc[nt][0] = acc[nt][1] = acc[nt][2] = acc[nt][3] = 0.f;
-        const uint8_t *arow = s_k + (size_t)(16 * warp + (lane & 7) + ((lane >> 3) & 1) * 8) * L::kKeyStride + (lane >> 4) * 16;
+        const int arow = 16 * warp + (lane & 7) + ((lane >> 3) & 1) * 8;
 #pragma unroll 2
         for (int j = 0; j < HD / 16; j++) {
             uint32_t r[4];
-            ldsm4(r, arow + j * 32);
+            ldsm4(r, T::frag(s_k, arow, lane >> 4, j));
 #pragma unroll
             for (int nt = 0; nt < NT; nt++) {
                 uint32_t b0, b1;
@@ -790,6 +823,7 @@ __global__ void __launch_bounds__(kAttnThreads) attn_chunk_kernel(const float *q
         return;
     }
     // ---- phase 2
+    if (BOXED) zero_rows<T, HD>(s_v, tile_keys, boxed_rows(tile_keys));
     if (small) s_short[1] = 1;
     small = false;
     for (int p = warp; p < P; p += kAttnThreads / 32)
@@ -800,17 +834,18 @@ __global__ void __launch_bounds__(kAttnThreads) attn_chunk_kernel(const float *q
     bool apart = false;
     if (base < kAttnTile)
         for (int i = tid; i < (min(base + nr - 1, kAttnTile) - max(base, 0)) * HD / 2; i += kAttnThreads) {
-            const uint32_t w = *reinterpret_cast<const uint32_t *>(s_v + (max(base, 0) + i / (HD / 2)) * L::kValStride + i % (HD / 2) * 4);
+            const int c = i % (HD / 2) >> 2;  // of four words
+            const uint32_t w = *reinterpret_cast<const uint32_t *>(T::frag(s_v, max(base, 0) + i / (HD / 2), c & 1, c >> 1) + (i & 3) * 4);
             apart = apart || (w & 0x7C00u) == 0x7C00u || (w & 0x7C000000u) == 0x7C000000u;
         }
     apart = __syncthreads_or(apart);
     if (s_short[0] || s_short[1]) {
-        tile_tf32<HD, G, P>(
+        tile_tf32<T, HD, G, P>(
             s_k, s_v, s_sc[0], s_f, s_ml, qrow, part_o + out_of(0) * HD, part_ml + out_of(0) * 2, n_head, n_splits, nr * G, base, scale, s_short[1] != 0);
         return;
     }
     // ---- phase 3: output dims 16 warp .. + 15
-    const uint8_t *vrow = s_v + (size_t)((lane & 7) + (lane >> 4) * 8) * L::kValStride + (size_t)(16 * warp + ((lane >> 3) & 1) * 8) * 2;
+    const uint8_t *vrow = T::frag(s_v, (lane & 7) + (lane >> 4) * 8, (lane >> 3) & 1, warp);
     // NTC groups of four pairs from pair p0 on; pairs at or past p1 are computed for nothing and not stored
     auto values = [&](auto ntc, int p0, int p1) {
         constexpr int NTC = decltype(ntc)::value;
@@ -820,7 +855,7 @@ __global__ void __launch_bounds__(kAttnThreads) attn_chunk_kernel(const float *q
 #pragma unroll 2
         for (int s16 = 0; s16 < kAttnTile / 16; s16++) {
             uint32_t r[4];
-            ldsm4_trans(r, vrow + (size_t)s16 * 16 * L::kValStride);
+            ldsm4_trans(r, vrow + s16 * 16 * T::kStride);
 #pragma unroll
             for (int nt = 0; nt < NTC; nt++) {
                 uint32_t b0, b1;
@@ -846,7 +881,7 @@ __global__ void __launch_bounds__(kAttnThreads) attn_chunk_kernel(const float *q
         for (int r = nr - 1; r >= 0 && base + r > 0; r--) {
             if (r != nr - 1) {
                 __syncthreads();  // the row after this one has been multiplied
-                if (base + r < kAttnTile && tid < CPR) *reinterpret_cast<uint4 *>(s_v + (base + r) * L::kValStride + tid * 16) = make_uint4(0, 0, 0, 0);
+                if (base + r < kAttnTile && tid < CPR) *reinterpret_cast<uint4 *>(T::frag(s_v, base + r, tid & 1, tid >> 1)) = make_uint4(0, 0, 0, 0);
                 __syncthreads();
             }
             values(std::integral_constant<int, NT1>{}, r * G, r * G + G);
@@ -1329,45 +1364,75 @@ size_t attention_workspace_bytes(int q_rows, int n_head, int head_dim, int max_k
     return (size_t)q_rows * n_head * n_splits * ((size_t)head_dim + 2) * sizeof(float);
 }
 
+typedef CUresult (*EncodeAttnFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *, const cuuint32_t *,
+                                 const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+static EncodeAttnFn attn_encode() {
+    static EncodeAttnFn fn = [] {
+        void *p = nullptr;
+        cudaDriverEntryPointQueryResult r;
+        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &r) != cudaSuccess) p = nullptr;
+        return reinterpret_cast<EncodeAttnFn>(p);
+    }();
+    return fn;
+}
+// Maps of the caches of n_seq sequences, `seq_stride` halves apart, with `n_rows` rows of `row` halves each
+static bool attn_maps(const void *k, const void *v, size_t n_rows, int n_seq, size_t row, size_t seq_stride, AttnMaps *maps) {
+    EncodeAttnFn enc = attn_encode();
+    if (!enc) return false;
+    const cuuint64_t dim[3] = {(cuuint64_t)row, (cuuint64_t)n_rows, (cuuint64_t)n_seq}, stride[2] = {(cuuint64_t)row * 2, (cuuint64_t)(n_seq > 1 ? seq_stride : n_rows * row) * 2};
+    const cuuint32_t one[3] = {1, 1, 1};
+    auto make = [&](CUtensorMap *map, const void *base, int box_rows) {
+        const cuuint32_t box[3] = {64, (cuuint32_t)box_rows, 1};
+        return enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<void *>(base), dim, stride, box, one, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                   CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+    };
+    return make(&maps->whole[0], k, kAttnTile) && make(&maps->whole[1], v, kAttnTile) && make(&maps->part[0], k, kBoxRows) && make(&maps->part[1], v, kBoxRows);
+}
+
 template <int HD, int G>
 static cudaError_t launch_attn_one(dim3 grid, cudaStream_t st, const float *q, const __half *kc, const __half *vc, float *po, float *pml, int rows,
-                                   int n_head, int n_kv, int pos, float scale, int n_splits, size_t seq_stride, uint32_t *status, bool bulk,
-                                   const int32_t *seq_pos, const int32_t *block_table, int table_stride, int n_pages) {
+                                   int n_head, int n_kv, int pos, float scale, int n_splits, size_t seq_stride, uint32_t *status, bool boxed,
+                                   const int32_t *seq_pos, const int32_t *block_table, int table_stride, int n_pages, const AttnMaps &maps) {
     // the tile needs more than the default 48 KB of dynamic shared memory; the attribute is per device, so it is set
     // on every launch (cheap, allocates nothing) rather than remembered per process
-    auto kernel = bulk ? attn_split_kernel<HD, G, true> : attn_split_kernel<HD, G, false>;
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, AttnSmem<HD>::kBytes);
-    if (e != cudaSuccess) return e;
-    return launch_pdl(kernel, grid, dim3(kAttnThreads), (size_t)AttnSmem<HD>::kBytes, st, q, kc, vc, po, pml, rows, n_head, n_kv, pos, scale, n_splits,
-                      seq_stride, status, seq_pos, block_table, table_stride, n_pages);
+    auto go = [&](auto kernel, int bytes, const auto &m) {
+        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+        if (e != cudaSuccess) return e;
+        return launch_pdl(kernel, grid, dim3(kAttnThreads), (size_t)bytes, st, q, kc, vc, po, pml, rows, n_head, n_kv, pos, scale, n_splits, seq_stride, status, seq_pos,
+                          block_table, table_stride, n_pages, m);
+    };
+    return boxed ? go(attn_split_kernel<HD, G, true>, kTileBytes<BoxedTile<HD>>, maps) : go(attn_split_kernel<HD, G, false>, kTileBytes<PaddedTile<HD>>, NoMaps{});
 }
 
 template <int HD>
 static cudaError_t launch_attn_hd(int group, dim3 grid, cudaStream_t st, const float *q, const __half *kc, const __half *vc, float *po, float *pml,
-                                  int rows, int n_head, int n_kv, int pos, float scale, int n_splits, size_t seq_stride, uint32_t *status, bool bulk,
-                                  const int32_t *seq_pos, const int32_t *block_table, int table_stride, int n_pages) {
+                                  int rows, int n_head, int n_kv, int pos, float scale, int n_splits, size_t seq_stride, uint32_t *status, bool boxed,
+                                  const int32_t *seq_pos, const int32_t *block_table, int table_stride, int n_pages, const AttnMaps &maps) {
     switch (group) {
-        case 1: return launch_attn_one<HD, 1>(grid, st, q, kc, vc, po, pml, rows, n_head, n_kv, pos, scale, n_splits, seq_stride, status, bulk, seq_pos, block_table,
-                                                  table_stride, n_pages);
-        case 2: return launch_attn_one<HD, 2>(grid, st, q, kc, vc, po, pml, rows, n_head, n_kv, pos, scale, n_splits, seq_stride, status, bulk, seq_pos, block_table,
-                                                  table_stride, n_pages);
-        case 4: return launch_attn_one<HD, 4>(grid, st, q, kc, vc, po, pml, rows, n_head, n_kv, pos, scale, n_splits, seq_stride, status, bulk, seq_pos, block_table,
-                                                  table_stride, n_pages);
-        case 8: return launch_attn_one<HD, 8>(grid, st, q, kc, vc, po, pml, rows, n_head, n_kv, pos, scale, n_splits, seq_stride, status, bulk, seq_pos, block_table,
-                                                  table_stride, n_pages);
+        case 1: return launch_attn_one<HD, 1>(grid, st, q, kc, vc, po, pml, rows, n_head, n_kv, pos, scale, n_splits, seq_stride, status, boxed, seq_pos, block_table,
+                                                  table_stride, n_pages, maps);
+        case 2: return launch_attn_one<HD, 2>(grid, st, q, kc, vc, po, pml, rows, n_head, n_kv, pos, scale, n_splits, seq_stride, status, boxed, seq_pos, block_table,
+                                                  table_stride, n_pages, maps);
+        case 4: return launch_attn_one<HD, 4>(grid, st, q, kc, vc, po, pml, rows, n_head, n_kv, pos, scale, n_splits, seq_stride, status, boxed, seq_pos, block_table,
+                                                  table_stride, n_pages, maps);
+        case 8: return launch_attn_one<HD, 8>(grid, st, q, kc, vc, po, pml, rows, n_head, n_kv, pos, scale, n_splits, seq_stride, status, boxed, seq_pos, block_table,
+                                                  table_stride, n_pages, maps);
         default: return cudaErrorInvalidValue;
     }
 }
 
 template <int G>
 static cudaError_t launch_attn_chunk(cudaStream_t st, const float *q, const __half *kc, const __half *vc, float *po, float *pml, int n_seq, int rows,
-                                     int n_head, int n_kv, int pos, float scale, int n_splits, size_t seq_stride, uint32_t *status,
-                                     const int32_t *seq_pos, const int32_t *block_table, int table_stride, int n_pages) {
-    constexpr int R = kAttnChunkPairs / G, bytes = AttnSmem<128>::kBytes + 4 * kAttnChunkPairs * (128 + kAttnPad) * 2 + kAttnChunkPairs * kAttnTile * 4;
-    cudaError_t e = cudaFuncSetAttribute(attn_chunk_kernel<G>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    if (e != cudaSuccess) return e;
-    return launch_pdl(attn_chunk_kernel<G>, dim3(n_splits, n_kv, n_seq * ((rows + R - 1) / R)), dim3(kAttnThreads), (size_t)bytes, st, q, kc, vc, po, pml,
-                      rows, n_head, n_kv, pos, scale, n_splits, seq_stride, status, seq_pos, block_table, table_stride, n_pages);
+                                     int n_head, int n_kv, int pos, float scale, int n_splits, size_t seq_stride, uint32_t *status, bool boxed,
+                                     const int32_t *seq_pos, const int32_t *block_table, int table_stride, int n_pages, const AttnMaps &maps) {
+    constexpr int R = kAttnChunkPairs / G, more = 4 * kAttnChunkPairs * (128 + kAttnPad) * 2 + kAttnChunkPairs * kAttnTile * 4;
+    auto go = [&](auto kernel, int bytes, const auto &m) {
+        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+        if (e != cudaSuccess) return e;
+        return launch_pdl(kernel, dim3(n_splits, n_kv, n_seq * ((rows + R - 1) / R)), dim3(kAttnThreads), (size_t)bytes, st, q, kc, vc, po, pml, rows, n_head, n_kv, pos, scale,
+                          n_splits, seq_stride, status, seq_pos, block_table, table_stride, n_pages, m);
+    };
+    return boxed ? go(attn_chunk_kernel<G, true>, kTileBytes<BoxedTile<128>> + more, maps) : go(attn_chunk_kernel<G, false>, kTileBytes<PaddedTile<128>> + more, NoMaps{});
 }
 
 cudaError_t launch_attention(const float *q, const void *k_cache, const void *v_cache, float *dst, void *workspace, int n_seq, int rows, int n_head,
@@ -1376,7 +1441,7 @@ cudaError_t launch_attention(const float *q, const void *k_cache, const void *v_
     if (n_seq <= 0 || rows <= 0 || n_head <= 0 || n_kv <= 0 || n_head % n_kv || pos < 0) return cudaErrorInvalidValue;
     const int max_keys = pos + rows, n_splits = (max_keys + kAttnTile - 1) / kAttnTile, q_rows = n_seq * rows;
     if (n_kv > 65535 || q_rows > 65535) return cudaErrorInvalidValue;
-    // the tiles are fetched with 16-byte-granular bulk copies of whole rows
+    // the tiles are fetched in 16-byte pieces
     if (((uintptr_t)k_cache | (uintptr_t)v_cache) % 16 || seq_stride % 8 || ((size_t)n_kv * head_dim) % 8) return cudaErrorInvalidValue;
     if (block_table && (n_pages < 1 || table_stride < n_splits)) return cudaErrorInvalidValue;
     float *po = static_cast<float *>(workspace);
@@ -1384,8 +1449,6 @@ cudaError_t launch_attention(const float *q, const void *k_cache, const void *v_
     const dim3 grid(n_splits, n_kv, q_rows);
     const __half *kc = static_cast<const __half *>(k_cache), *vc = static_cast<const __half *>(v_cache);
     cudaError_t e;
-    // more than two waves of CTAs (three fit an SM): the per-tile instruction count decides, else the first byte's latency
-    const bool bulk = (size_t)n_splits * n_kv * q_rows > (size_t)6 * (sm_count > 0 ? sm_count : 148);
     const int g = n_head / n_kv;
     // Rows of a prompt chunk share a tile where a tile per row takes more than about a wave of CTAs (three fit an SM; two of the shared form, which
     // take 1 us longer) and the shared tile has more than two rows, is nearly full or leaves a single wave.  live: the tiles with keys, each
@@ -1398,15 +1461,23 @@ cudaError_t launch_attention(const float *q, const void *k_cache, const void *v_
     const size_t live = (tiles_to(max_keys) - tiles_to(pos)) * n_kv * n_seq, shared = (size_t)n_splits * n_kv * n_seq * row_blocks;
     const bool chunk = head_dim == 128 && rows > 1 && (g == 1 || g == 2 || g == 4 || g == 8) && 2 * live > 5 * sms &&
                        (rows > 2 * row_blocks || 8 * rows >= 7 * rpt * row_blocks || shared <= 2 * sms);
-#define INFR_CHUNK(G_) launch_attn_chunk<G_>(st, q, kc, vc, po, pml, n_seq, rows, n_head, n_kv, pos, scale, n_splits, seq_stride, status, seq_pos, block_table, table_stride, n_pages)
+    // Tensor copies where the tiles are more than two waves of CTAs (three fit an SM, two of the shared form).  Before that the latency of the first byte
+    // counts, which is 0.5 to 1 us longer with them: shared tiles, bulk copies of rows / tensor copies, us a call: 32 heads / 8, 64 rows at 128 (256 tiles) 12.1 / 13.1;
+    // 8 / 8, 20 rows at 640 (96) 16.0 / 17.2, 300 at 0 (264) 18.3 / 19.2, 64 at 1500 (400) 18.2 / 16.3, 128 at 3000 45 / 42; 32 / 8, 113 at 384 (928) 29.4 / 27.4,
+    // 128 at 3000 153 / 142.
+    const size_t kv_row = (size_t)n_kv * head_dim;
+    AttnMaps maps;
+    const bool boxed = (chunk ? live / rows * row_blocks > 2 * sms : (size_t)n_splits * n_kv * q_rows > 6 * sms) && (head_dim == 128 || head_dim == 64) &&
+                       attn_maps(k_cache, v_cache, block_table ? (size_t)n_pages * kAttnTile : (size_t)max_keys, block_table ? 1 : n_seq, kv_row, seq_stride, &maps);
+#define INFR_CHUNK(G_) launch_attn_chunk<G_>(st, q, kc, vc, po, pml, n_seq, rows, n_head, n_kv, pos, scale, n_splits, seq_stride, status, boxed, seq_pos, block_table, table_stride, n_pages, maps)
     if (chunk)
         e = g == 1 ? INFR_CHUNK(1) : g == 2 ? INFR_CHUNK(2) : g == 4 ? INFR_CHUNK(4) : INFR_CHUNK(8);
     else if (head_dim == 128)
-        e = launch_attn_hd<128>(g, grid, st, q, kc, vc, po, pml, rows, n_head, n_kv, pos, scale, n_splits, seq_stride, status, bulk, seq_pos, block_table, table_stride,
-                                n_pages);
+        e = launch_attn_hd<128>(g, grid, st, q, kc, vc, po, pml, rows, n_head, n_kv, pos, scale, n_splits, seq_stride, status, boxed, seq_pos, block_table, table_stride,
+                                n_pages, maps);
     else if (head_dim == 64)
-        e = launch_attn_hd<64>(g, grid, st, q, kc, vc, po, pml, rows, n_head, n_kv, pos, scale, n_splits, seq_stride, status, bulk, seq_pos, block_table, table_stride,
-                               n_pages);
+        e = launch_attn_hd<64>(g, grid, st, q, kc, vc, po, pml, rows, n_head, n_kv, pos, scale, n_splits, seq_stride, status, boxed, seq_pos, block_table, table_stride,
+                               n_pages, maps);
     else
         return cudaErrorInvalidValue;
 #undef INFR_CHUNK
