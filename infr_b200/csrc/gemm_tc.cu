@@ -40,7 +40,8 @@
 // back where the accumulators' says as much, one epilogue warp that waits for the others (they stand at a named barrier), two issuers (one was
 // busy for 2400 cycles of a job's 2550), and as few instructions as can be for a weight.  Before / after, us, cold weights, back to back: Q4_K
 // 4096 -> 28672, 32 rows 34.2 / 31.1, 113 rows 50.8 / 47.2; 4096 -> 14336, 512 rows 81 / 75; Q6_K 14336 -> 4096, 512 rows 148 / 137.
-// At 128 tokens a Q4_K job takes ~2050 cycles, its MMAs 1150; the warps issue 6540 instructions (10060 before, most of them polls).
+// At 128 tokens a Q4_K job takes ~2320 cycles (2550), its MMAs 1150; the warps issue 5980 instructions (6670).  Q6_K calls with a few jobs a CTA are 0.9 us
+// slower for it (4096 -> 4096, 113 rows 20.6 / 21.5), of a cause that neither the place of the waits nor the size of the first copies is.
 // Tried: 16 unpack and 8 epilogue warps (4 % slower), waits as tight loops in PTX (30 to 100 % slower: they poll more often), sleeping
 // between polls (1 to 15 % slower), the issuer's loop not unrolled (17 % slower), a look at all of a job's barriers at once (no gain), a chunk's
 // tensor-memory load during the fold of the one before it (spills).
