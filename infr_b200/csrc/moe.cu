@@ -75,9 +75,9 @@ __global__ void __launch_bounds__(128) moe_router_kernel(const float *__restrict
     for (int c0 = 0; c0 < n_chunks; c0++) {
         const int kc = min(kRtK, ne - c0 * kRtK);
         const float *buf = s_rt + (c0 % kRtRing) * kRtBuf;
-        if (!__syncthreads_and(landed(c0))) {  // give up; the copies in flight get their own limit
+        if (!__syncthreads_and(landed(c0))) {  // give up; the copies in flight get their own limit (chunk 1 is the first whose landing asks for another)
             if (threadIdx.x == 0) atomicExch(status, 14u);
-            for (int c = c0 + 1; c < c0 - 1 + kRtRing && c < n_chunks; c++) landed(c);
+            for (int c = c0 + 1; c < kRtRing + (c0 > 1 ? c0 - 1 : 0) && c < n_chunks; c++) landed(c);
             return;
         }
         if (warp == 0 && c0 >= 1 && c0 - 1 + kRtRing < n_chunks) {  // everybody has finished with the columns before these
