@@ -98,6 +98,11 @@ struct Cfg {
     static constexpr int kChunk = TN == 64 && FMT == F_Q4 ? 16 : 8;  // columns per tensor-memory load (registers)
     static constexpr int W_HEAD = kUnpack + kEpi, W_LOAD = W_HEAD + 1, W_MMA = W_HEAD + 2, kWarps = W_HEAD + 4;
     static constexpr int kCtas = TN == 32 && FMT != F_Q6 ? 2 : 1;
+    // The waits' loops as a function of their own.  Every role is at another place of the code, and with a loop at each wait Q6_K's warps lack an
+    // instruction to issue more often (1.5 warps an issue slot, 1.4 this way): 1 us of a call with a few jobs a CTA.  us a call, loops at the
+    // waits / one function: Q6_K 4096 -> 4096, 113 rows 21.2 / 20.35, 2048 -> 2048, 300 rows 19.6 / 18.5, 4096 -> 28672, 64 rows 71.6 / 65.9; Q4_K, whose
+    // unpacking is shorter: 4096 -> 14336, 113 rows 27.6 / 28.4, 512 rows 75 / 77, 4096 -> 4096, 64 rows 13.5 / 13.7.
+    static constexpr bool kFarWaits = FMT == F_Q6;
     // tensor-memory columns: accumulators of two jobs (one where there is no room), block-minimum sums of two jobs (one where there is no room), operands
     static constexpr int kMBuf = FMT == F_Q4 ? (TN == 128 ? 1 : 2) : 0;
     static constexpr uint32_t kColM = kJobBuf * kAcc * TN;
@@ -179,17 +184,23 @@ __device__ __forceinline__ bool try_bar(uint32_t bar, uint32_t parity) {
 }
 // Bounded wait; gives up early when another role has raised the CTA flag.  A role waits on a barrier by parity only where it
 // has seen every earlier phase and the next completion depends on the waiter having passed, so it is never two phases off.
-__device__ __forceinline__ bool wait_bar(uint32_t bar, uint32_t parity, volatile int *dead) {
-    if (try_bar(bar, parity)) return true;
+__device__ __forceinline__ bool poll_bar(uint32_t bar, uint32_t parity, volatile int *dead) {
     for (uint32_t i = 1; i < kSpin; i++) {
         if (try_bar(bar, parity)) return true;
         if ((i & 1023u) == 0 && *dead) return false;
     }
     return false;
 }
+__device__ __noinline__ bool poll_bar_far(uint32_t bar, uint32_t parity, volatile int *dead) { return poll_bar(bar, parity, dead); }
+template <class K>
+__device__ __forceinline__ bool wait_bar(uint32_t bar, uint32_t parity, volatile int *dead) {
+    if (try_bar(bar, parity)) return true;
+    return K::kFarWaits ? poll_bar_far(bar, parity, dead) : poll_bar(bar, parity, dead);
+}
 // All lanes of a converged warp wait together: the result is one for the warp.
+template <class K>
 __device__ __forceinline__ bool wait_warp(uint32_t bar, uint32_t parity, volatile int *dead) {
-    return __all_sync(0xffffffffu, wait_bar(bar, parity, dead));
+    return __all_sync(0xffffffffu, wait_bar<K>(bar, parity, dead));
 }
 
 // Named barrier 1 of N threads; true where `ok` is true in all of them.
@@ -637,11 +648,11 @@ __global__ void __launch_bounds__(Cfg<FMT, TN>::kWarps * 32, Cfg<FMT, TN>::kCtas
             for (; ca.i < n; js++, next(ca)) {
                 const int x = js % K::kNX;
                 const size_t rec = (size_t)ca.t.tt * nst + ca.b;
-                if (js >= K::kNX && !(ok = wait_bar(bar(K::B_XFREE + x), (uint32_t)((js / K::kNX - 1) & 1), dead))) break;
+                if (js >= K::kNX && !(ok = wait_bar<K>(bar(K::B_XFREE + x), (uint32_t)((js / K::kNX - 1) & 1), dead))) break;
                 if (js >= K::kJB) {  // the operands of the job that had the place before have been read
                     const int p = js - K::kJB;
-                    if (!(ok = K::kOwnB ? wait_bar(bar(K::B_BFREE + js % K::kJB), (uint32_t)(p / K::kJB) & 1u, dead)
-                                        : wait_bar(bar(K::B_ACCRDY + (p & 1)), (uint32_t)(p >> 1) & 1u, dead)))
+                    if (!(ok = K::kOwnB ? wait_bar<K>(bar(K::B_BFREE + js % K::kJB), (uint32_t)(p / K::kJB) & 1u, dead)
+                                        : wait_bar<K>(bar(K::B_ACCRDY + (p & 1)), (uint32_t)(p >> 1) & 1u, dead)))
                         break;
                 }
                 expect_tx(bar(K::B_XFULL + x), K::kExtra + K::kUnits * K::kUnitBytes);
@@ -649,7 +660,7 @@ __global__ void __launch_bounds__(Cfg<FMT, TN>::kWarps * 32, Cfg<FMT, TN>::kCtas
                 bulk(su32(ext0 + x * K::kExtra), extra + rec * K::kExtra, K::kExtra, bar(K::B_XFULL + x));
                 // the job before is unpacked by the time that the one before that has been multiplied
                 if (js >= 1 && cw.i < n) {
-                    if (!(ok = wait_bar(bar(K::B_SFREE + (js - 1) % K::kStages), (uint32_t)((js - 1) / K::kStages) & 1u, dead))) {
+                    if (!(ok = wait_bar<K>(bar(K::B_SFREE + (js - 1) % K::kStages), (uint32_t)((js - 1) / K::kStages) & 1u, dead))) {
                         js++;
                         break;
                     }
@@ -687,8 +698,8 @@ __global__ void __launch_bounds__(Cfg<FMT, TN>::kWarps * 32, Cfg<FMT, TN>::kCtas
                     const uint32_t q = (uint32_t)(j % K::kJB);  // its place in the activation ring
                     const uint32_t td = tmem + (uint32_t)(sa * K::kAcc * TN);
                     // what the header warp has seen: its own operands, and the accumulators given back by the job that had them before
-                    if (!(ok = wait_bar(bar(K::B_HEAD + s), jp, dead))) break;
-                    if (!(ok = wait_bar(bar(K::B_XFULL + j % K::kNX), (uint32_t)(j / K::kNX) & 1u, dead))) break;
+                    if (!(ok = wait_bar<K>(bar(K::B_HEAD + s), jp, dead))) break;
+                    if (!(ok = wait_bar<K>(bar(K::B_XFULL + j % K::kNX), (uint32_t)(j / K::kNX) & 1u, dead))) break;
 #pragma unroll
                     for (int st = 0; st < 2 * K::kUnits; st++) {
                         // (Q6_K: the teams' slots in turn, both get theirs back early)
@@ -696,7 +707,7 @@ __global__ void __launch_bounds__(Cfg<FMT, TN>::kWarps * 32, Cfg<FMT, TN>::kCtas
                         const int u = k8 >> 1, h = k8 & 1, team = k8 / K::kUse;
                         const uint64_t bd = bd0 + (uint64_t)((q * K::kUnits + u) * (uint32_t)(K::kUnitBytes / 16));
                         const int sl = team * K::kSlots + (j * K::kUse + k8 % K::kUse) % K::kSlots;
-                        if (!(ok = wait_bar(bar(K::B_AFULL + (s * 2 + team) * K::kUse + k8 % K::kUse), jp, dead))) break;
+                        if (!(ok = wait_bar<K>(bar(K::B_AFULL + (s * 2 + team) * K::kUse + k8 % K::kUse), jp, dead))) break;
                         tc_fence_after();
                         const uint32_t ta = tmem + K::kColA + (uint32_t)(sl * 32);
 #pragma unroll
@@ -713,7 +724,7 @@ __global__ void __launch_bounds__(Cfg<FMT, TN>::kWarps * 32, Cfg<FMT, TN>::kCtas
                         const uint64_t xd = mk_desc(su32(ext0 + (j % K::kNX) * K::kExtra), TN * 16);
                         mma_sa(td, mk_desc(su32(amin + (s * 4 + 2) * kTM * 16), kTM * 16), xd, idesc, 1u);
                         // (the other issuer's job; the one before that is folded, or B_HEAD would not be here)
-                        if (K::kMBuf == 1 && j >= 1 && !(ok = wait_bar(bar(K::B_MFREE), (uint32_t)((j - 1) & 1), dead))) break;
+                        if (K::kMBuf == 1 && j >= 1 && !(ok = wait_bar<K>(bar(K::B_MFREE), (uint32_t)((j - 1) & 1), dead))) break;
                         tc_fence_after();
                         mma_sa(tmem + K::kColM + (uint32_t)(K::kMBuf == 2 ? s * TN : 0), mk_desc(su32(amin + s * 4 * kTM * 16), kTM * 16), xd, idesc, 0u);
                     }
@@ -738,7 +749,7 @@ __global__ void __launch_bounds__(Cfg<FMT, TN>::kWarps * 32, Cfg<FMT, TN>::kCtas
             const Tile t = tile_of(i);
             for (int b = t.b0; b < t.b1; b++, js++) {
                 const int ls = js % K::kStages, s = js & 1;
-                if (!(ok = wait_warp(bar(K::B_SFULL + ls), (uint32_t)((js / K::kStages) & 1), dead))) break;
+                if (!(ok = wait_warp<K>(bar(K::B_SFULL + ls), (uint32_t)((js / K::kStages) & 1), dead))) break;
                 const uint8_t *blk = raw0 + ls * K::kRaw;
                 uint4 hdr[4];
                 uint32_t dh[4];
@@ -755,9 +766,9 @@ __global__ void __launch_bounds__(Cfg<FMT, TN>::kWarps * 32, Cfg<FMT, TN>::kCtas
                 // The job before last (one accumulator: the last job) has been multiplied and its accumulators are given back: the rings'
                 // places are free, and the issuer, who waits for this warp, need not wait for them.
                 if (K::kJobBuf == 2) {
-                    if (js >= 2 && !(ok = wait_warp(bar(K::B_ACCFREE + s), (uint32_t)(((js >> 1) - 1) & 1), dead))) break;
+                    if (js >= 2 && !(ok = wait_warp<K>(bar(K::B_ACCFREE + s), (uint32_t)(((js >> 1) - 1) & 1), dead))) break;
                 } else {
-                    if (js >= 1 && !(ok = wait_warp(bar(K::B_ACCFREE), (uint32_t)((js - 1) & 1), dead))) break;
+                    if (js >= 1 && !(ok = wait_warp<K>(bar(K::B_ACCFREE), (uint32_t)((js - 1) & 1), dead))) break;
                 }
 #pragma unroll
                 for (int k = 0; k < 4; k++) {
@@ -795,7 +806,7 @@ __global__ void __launch_bounds__(Cfg<FMT, TN>::kWarps * 32, Cfg<FMT, TN>::kCtas
         // the team's slot of its use-th operand run: its previous MMAs are complete, it is filled, it is announced
         auto put = [&](int use, const uint32_t (&o)[32]) {
             const int sl = team * K::kSlots + use % K::kSlots, ph = use / K::kSlots;
-            if (ph >= 1 && !wait_warp(bar(K::B_AFREE + sl), (uint32_t)((ph - 1) & 1), dead)) return false;
+            if (ph >= 1 && !wait_warp<K>(bar(K::B_AFREE + sl), (uint32_t)((ph - 1) & 1), dead)) return false;
             tc_fence_after();
             tst32(tl + (uint32_t)(sl * 32), o);
             tst_wait();
@@ -808,7 +819,7 @@ __global__ void __launch_bounds__(Cfg<FMT, TN>::kWarps * 32, Cfg<FMT, TN>::kCtas
             const Tile t = tile_of(i);
             for (int b = t.b0; b < t.b1; b++, js++) {
                 const int ls = js % K::kStages;
-                if (!(ok = wait_warp(bar(K::B_SFULL + ls), (uint32_t)((js / K::kStages) & 1), dead))) break;
+                if (!(ok = wait_warp<K>(bar(K::B_SFULL + ls), (uint32_t)((js / K::kStages) & 1), dead))) break;
                 const uint8_t *blk = raw0 + ls * K::kRaw + (size_t)row * K::kRowBytes;
                 const uint4 *bv = reinterpret_cast<const uint4 *>(blk);
                 uint32_t o[32];
@@ -867,8 +878,8 @@ __global__ void __launch_bounds__(Cfg<FMT, TN>::kWarps * 32, Cfg<FMT, TN>::kCtas
                 const int x = j % K::kNX, s = K::kJobBuf == 2 ? j & 1 : 0;
                 // one warp waits (sixteen of them took 1500 instructions a job to look, Q6_K at 512 rows 148 -> 141 us), the others stand at the barrier
                 if (warp == K::kUnpack)
-                    ok = wait_bar(bar(K::B_XFULL + x), (uint32_t)((j / K::kNX) & 1), dead) &&
-                         wait_bar(bar(K::B_ACCRDY + s), (uint32_t)((K::kJobBuf == 2 ? j >> 1 : j) & 1), dead);
+                    ok = wait_bar<K>(bar(K::B_XFULL + x), (uint32_t)((j / K::kNX) & 1), dead) &&
+                         wait_bar<K>(bar(K::B_ACCRDY + s), (uint32_t)((K::kJobBuf == 2 ? j >> 1 : j) & 1), dead);
                 __syncwarp();
                 if (!(ok = bar_and<K::kEpi * 32>(ok))) break;
                 tc_fence_after();
