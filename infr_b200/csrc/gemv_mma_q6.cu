@@ -412,10 +412,9 @@ __global__ void __launch_bounds__(32 * kGroupedWarps6, 2) gemv_q6_mma_grouped_ke
         __syncwarp();
     };
     // Landed?  (Bounded.  Not before the slot is this tile's: a parity cannot tell "not yet issued" from "landed".)
-    auto landed = [&](int i, int slot, uint32_t phase, bool once) {
-        uint32_t k = 0;
-        for (const uint32_t most = once ? 1u : 1u << 22; s_tile[slot] != i; k++)
-            if (k >= most) return false;
+    auto landed = [&](int i, int slot, uint32_t phase) {
+        for (uint32_t k = 0; s_tile[slot] != i; k++)
+            if (k >= 1u << 22) return false;
         return wait_parity6(sm6(bars + slot), phase);
     };
     for (int i = warp; i < slots; i += kw) issue(i, i);
@@ -465,8 +464,7 @@ __global__ void __launch_bounds__(32 * kGroupedWarps6, 2) gemv_q6_mma_grouped_ke
         }
         __syncthreads();
         for (; i < hi; i += kw) {
-            const bool ok = __all_sync(0xffffffffu, landed(i, slot, phase, dead));
-            if (!ok && !dead) {  // from here on only what is on its way is waited for
+            if (!dead && !__all_sync(0xffffffffu, landed(i, slot, phase))) {  // from here on nothing is asked for
                 dead = true;
                 if (lane == 0) s_dead = 1, atomicExch(status, 3u);
             }
@@ -490,6 +488,11 @@ __global__ void __launch_bounds__(32 * kGroupedWarps6, 2) gemv_q6_mma_grouped_ke
             if (n0 + 1 < m) yr[out_f] = accf[1], yr[out_f + 8] = accf[3];
         }
     }
+    // Somebody gave up: what is on its way, the last tile of every slot, lands before the shared memory is another CTA's.  (Only here has the last
+    // of them been asked for: a warp that had not seen s_dead may have asked after the tile's own warp had looked.)
+    if (__syncthreads_or(dead))
+        for (int s = threadIdx.x; s < slots; s += blockDim.x)
+            if (s_tile[s] >= 0) wait_parity6(sm6(bars + s), (uint32_t)(s_tile[s] / slots) & 1u);
 }
 
 typedef CUresult (*EncQ6)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,

@@ -1,14 +1,28 @@
-"""A kernel that gives up waiting for a chunk of its ring (the MoE router) waits for every other copy that is on its way.  The bound of that loop is taken from the
-kernel's source, compiled for the host, and held against a replay of the copies: a ring of chunks at once, then one more for each that lands after the first."""
+"""Kernels that give up waiting for a copy wait for every other one that is on its way, so that none lands in shared memory that has gone to another block.  No
+wait runs out on a GPU here: the loops that do this are taken from the kernels' sources, compiled for the host and held against a replay of the copies."""
 import os
 import re
 import subprocess
 
 import infr_b200
 
-PROGRAM = r"""
+
+def _loop(source, pattern):
+    with open(os.path.join(os.path.dirname(infr_b200.__file__), "csrc", source)) as f:
+        return re.search(pattern, f.read(), re.S).group(1)
+
+
+def _run(tmp_path, program):
+    src, exe = tmp_path / "ring.cpp", tmp_path / "ring"
+    src.write_text(program)
+    subprocess.run(["g++", "-std=c++17", str(src), "-o", str(exe)], check=True)
+    return subprocess.run([str(exe)], check=True, capture_output=True, text=True).stdout
+
+
+ROUTER = r"""
 #include <cstdio>
 
+// a ring of chunks at once, then one more for each chunk that lands after the first
 int main() {
     int left = 0;
     for (int kRtRing = 2; kRtRing <= 5; kRtRing++)
@@ -24,11 +38,39 @@ int main() {
 }
 """
 
+ITEMS = r"""
+#include <cstdio>
+#include <cstdint>
 
-def test_no_copy_is_left_behind(tmp_path):
-    with open(os.path.join(os.path.dirname(infr_b200.__file__), "csrc", "moe.cu")) as f:
-        loop = re.search(r"atomicExch\(status, 14u\);\s*(for \(.*?landed\(c\);)", f.read(), re.S)
-    src, exe = tmp_path / "ring.cpp", tmp_path / "ring"
-    src.write_text(PROGRAM.replace("LOOP", loop.group(1)))
-    subprocess.run(["g++", "-std=c++17", str(src), "-o", str(exe)], check=True)
-    assert subprocess.run([str(exe)], check=True, capture_output=True, text=True).stdout == "0\n"
+// tile i in slot i % slots, asked for when tile i - slots has been read: a slot's last tile is any of its own
+int main() {
+    int left = 0;
+    for (int slots = 4; slots <= 16; slots++)
+        for (int n = 0; n <= 3 * slots; n++)
+            for (int threads = 32; threads <= 256; threads *= 2) {
+                int s_tile[16], waited[16], parity[16], bars[16];
+                for (int s = 0; s < slots; s++) s_tile[s] = -1, waited[s] = 0;
+                for (int i = 0; i < n; i++) s_tile[i % slots] = i;
+                auto sm6 = [&](int *b) { return (int)(b - bars); };
+                auto wait_parity6 = [&](int s, uint32_t p) { waited[s]++, parity[s] = (int)p; };
+                struct { int x; } blockDim{threads}, threadIdx{0};
+                for (; threadIdx.x < threads; threadIdx.x++) {
+                    LOOP
+                }
+                for (int s = 0; s < slots; s++) {
+                    int uses = 0;  // of the slot: its last copy completes phase uses - 1
+                    for (int i = s; i < n; i += slots) uses++;
+                    left += waited[s] != (uses > 0) || (uses && parity[s] != ((uses - 1) & 1));
+                }
+            }
+    std::printf("%d\n", left);
+}
+"""
+
+
+def test_router(tmp_path):
+    assert _run(tmp_path, ROUTER.replace("LOOP", _loop("moe.cu", r"atomicExch\(status, 14u\);\s*(for \(.*?landed\(c\);)"))) == "0\n"
+
+
+def test_expert_items_q6k(tmp_path):
+    assert _run(tmp_path, ITEMS.replace("LOOP", _loop("gemv_mma_q6.cu", r"if \(__syncthreads_or\(dead\)\)\s*(for \(.*?& 1u\);)"))) == "0\n"
