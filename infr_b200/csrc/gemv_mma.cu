@@ -240,6 +240,7 @@ __global__ void __launch_bounds__(KW * TG * 32, 16 / (KW * TG))
     uint64_t l2_policy;
     asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(l2_policy));
     // ---- issue side: one elected lane fetches the 16-row x K-step box of the slot ----
+    bool dead = false;
     int j_issue = 0, i_step = 0, i_T = t_begin + tg;
     int i_item = 0;  // the item of tile i_T
     if (SHARE) {
@@ -250,7 +251,7 @@ __global__ void __launch_bounds__(KW * TG * 32, 16 / (KW * TG))
         row_base = grp.item_expert[i_item] * out_f;
     }
     auto issue = [&](int slot) {
-        if (j_issue >= n_jobs) return;
+        if (j_issue >= n_jobs || dead) return;
         if (lane == 0) {
             const int blk0 = kb0 + i_step * kStepBlocks;
             const uint32_t bar = s_u32(wbar + slot);
@@ -284,7 +285,6 @@ __global__ void __launch_bounds__(KW * TG * 32, 16 / (KW * TG))
     const int gt = g < M ? g : 0;  // token whose codes this lane feeds as its B column
     int slot = 0, tile = 0;
     uint32_t phase = 0;
-    bool dead = false;
     for (int item = SHARE ? t_begin / total_tiles : 0;; item++) {  // even shares: the items of this CTA, otherwise once (body not indented)
     int seg_end = 0, tid = threadIdx.x;
     if (SHARE) asm volatile("" : "+r"(tid));  // (what the staging derives from it is not kept in registers from one item to the next)
@@ -518,6 +518,7 @@ __global__ void __launch_bounds__(KW * TG * 32, 16 / (KW * TG))
     }
     if (!SHARE) break;
     }
+    if (dead) drain_ring(wbar, S, j_issue);
 }
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,

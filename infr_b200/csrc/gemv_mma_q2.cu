@@ -95,8 +95,9 @@ __global__ void __launch_bounds__(KW * 32, 16 / KW)
     uint64_t *wbar = bars + warp * kMaxSlots;
 
     int j_issue = 0, i_tile = 0, i_ch = 0;
+    bool dead = false;
     auto issue = [&](int slot) {
-        if (j_issue >= n_jobs) return;
+        if (j_issue >= n_jobs || dead) return;
         if (lane == 0) {
             const uint32_t bar = sm32(wbar + slot);
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // earlier reads of the slot come first
@@ -154,7 +155,6 @@ __global__ void __launch_bounds__(KW * 32, 16 / KW)
     const int n0 = 2 * t, n1 = 2 * t + 1;    // tokens of this lane's result columns
     int slot = 0;
     uint32_t phase = 0;
-    bool dead = false;
     for (int tile = 0; tile < n_tiles; tile++) {
         float accf[4] = {0.f, 0.f, 0.f, 0.f};
         for (int ci = 0; ci < my_chunks; ci++) {
@@ -218,6 +218,7 @@ __global__ void __launch_bounds__(KW * 32, 16 / KW)
             }
         }
     }
+    if (dead) drain_ring(wbar, S, j_issue);
 }
 
 typedef CUresult (*EncQ2)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,

@@ -179,8 +179,9 @@ __global__ void __launch_bounds__(KW * 32, 16 / KW)
     uint64_t *wbar = bars + warp * kMaxSlots6;
 
     int j_issue = 0, i_tile = 0, i_b = 0;
+    bool dead = false;
     auto issue = [&](int slot) {
-        if (j_issue >= n_jobs) return;
+        if (j_issue >= n_jobs || dead) return;
         if (lane == 0) {
             const uint32_t bar = sm6(wbar + slot);
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // earlier reads of the slot come first
@@ -250,7 +251,6 @@ __global__ void __launch_bounds__(KW * 32, 16 / KW)
     const int n0 = 2 * t;          // first of this lane's two result columns
     int slot = 0;
     uint32_t phase = 0;
-    bool dead = false;
     for (int tile = 0; tile < n_tiles; tile++) {
         float accf[4] = {0.f, 0.f, 0.f, 0.f};
         for (int bi = 0; bi < my_blocks; bi++) {
@@ -296,6 +296,7 @@ __global__ void __launch_bounds__(KW * 32, 16 / KW)
             }
         }
     }
+    if (dead) drain_ring(wbar, S, j_issue);
 }
 
 // ---- Expert-grouped form (mixture of experts): blockIdx.y walks the device-built list of work items, each up to 8 routed pairs of one

@@ -299,8 +299,9 @@ __global__ void __launch_bounds__(kWWarps * 32, 1)
     uint64_t l2_policy;
     asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(l2_policy));
     int j_issue = 0;
+    bool dead = false;
     auto issue = [&](int slot) {
-        if (j_issue >= n_jobs) return;
+        if (j_issue >= n_jobs || dead) return;
         if (lane == 0) {
             const uint32_t bar = sw32(wbar + slot);
             // order this warp's earlier reads of the slot before the engine overwrites it
@@ -338,7 +339,6 @@ __global__ void __launch_bounds__(kWWarps * 32, 1)
     float *dst2 = sec.out + (size_t)blockIdx.y * (size_t)m * sec.out_f;
     int slot = 0;
     uint32_t phase = 0;
-    bool dead = false;
     for (int tile = 0; tile < n_tiles; tile++) {
         float accf[NT][4];
 #pragma unroll
@@ -384,6 +384,7 @@ __global__ void __launch_bounds__(kWWarps * 32, 1)
             }
         }
     }
+    if (dead) drain_ring(wbar, S, j_issue);
 }
 
 // y[i] = part[0][i] + part[1][i] + ... in chunk order (the same bits on every run).

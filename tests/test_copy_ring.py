@@ -4,6 +4,8 @@ import os
 import re
 import subprocess
 
+import pytest
+
 import infr_b200
 
 
@@ -74,3 +76,37 @@ def test_router(tmp_path):
 
 def test_expert_items_q6k(tmp_path):
     assert _run(tmp_path, ITEMS.replace("LOOP", _loop("gemv_mma_q6.cu", r"if \(__syncthreads_or\(dead\)\)\s*(for \(.*?& 1u\);)"))) == "0\n"
+
+
+WARP = r"""
+#include <cstdio>
+#include <cstdint>
+
+// a warp's ring: copy j in slot j % slots; when the wait for one runs out, it and those behind it are on their way, no more than there are slots
+int main() {
+    int left = 0;
+    for (int slots = 1; slots <= 12; slots++)
+        for (int asked = 0; asked <= 4 * slots; asked++) {
+            uint64_t bars[12];
+            int waited[12] = {}, uses[12] = {};
+            for (int j = 0; j < asked; j++) uses[j % slots]++;  // a slot's last copy completes phase uses - 1
+            auto __cvta_generic_to_shared = [&](uint64_t *b) { return (uint64_t)(b - bars); };
+            LOOP
+                left += waited[bar]++ || parity != ((uint32_t)(uses[bar] - 1) & 1u);
+            }
+            for (int s = 0; s < slots; s++) left += waited[s] != (uses[s] > 0);
+        }
+    std::printf("%d\n", left);
+}
+"""
+
+
+def test_ring_of_a_warp(tmp_path):
+    assert _run(tmp_path, WARP.replace("LOOP", _loop("gemv_common.cuh", r"drain_ring\(.*?\{\n(.*?)\n\s*for \(uint32_t i"))) == "0\n"
+
+
+@pytest.mark.parametrize("source", ["gemv_mma.cu", "gemv_mma_q2.cu", "gemv_mma_q6.cu", "gemv_wide.cu"])
+def test_rings_of_warps_are_drained(source):
+    # a warp that has given up asks for nothing more, and its kernel ends with the wait for what it had asked for
+    body = _loop(source, r"auto issue = \[&\]\(int slot\) \{(.*?\n\}\n)")
+    assert body.lstrip().startswith("if (j_issue >= n_jobs || dead) return;") and body.endswith("    if (dead) drain_ring(wbar, S, j_issue);\n}\n")
