@@ -154,9 +154,11 @@ __global__ void __launch_bounds__(kMathThreads + 32, 1)
                     if (j >= kStages && !mbar_wait_bounded(sm_u32(&bars[kStages + 2 + s]), (uint32_t)((j / kStages - 1) & 1))) {
                         atomicExch(status, 5u);
                         *(volatile int *)&s_dead = 1;
+                    }
+                    if (*(volatile int *)&s_dead) {  // the copies that are on their way land first
+                        drain_ring(bars, kStages, j);
                         return;
                     }
-                    if (*(volatile int *)&s_dead) return;
                     uint8_t *st = stage0 + (size_t)s * kStageBytes;
                     const uint32_t bar = sm_u32(&bars[s]);
                     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(kStageBytes) : "memory");

@@ -110,3 +110,7 @@ def test_rings_of_warps_are_drained(source):
     # a warp that has given up asks for nothing more, and its kernel ends with the wait for what it had asked for
     body = _loop(source, r"auto issue = \[&\]\(int slot\) \{(.*?\n\}\n)")
     assert body.lstrip().startswith("if (j_issue >= n_jobs || dead) return;") and body.endswith("    if (dead) drain_ring(wbar, S, j_issue);\n}\n")
+
+
+def test_gemm_producer_is_drained():
+    assert re.match(r"[^\n]*\n\s*drain_ring\(bars, kStages, j\);\s*return;", _loop("mmq.cu", r"(if \(\*\(volatile int \*\)&s_dead\) .*)"))
