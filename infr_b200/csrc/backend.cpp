@@ -851,6 +851,8 @@ Status CudaBackend::moe_ffn(const MoeArgs &a) {
     if (a.n_expert == 0 || a.n_expert > 1024 || a.n_used == 0 || a.n_used > 32 || a.n_used > a.n_expert)
         return Status::Err(INFR_E_INVALID, fmt("moe_ffn: n_expert=%u (<=1024), n_used=%u (<=32)", a.n_expert, a.n_used));
     if (a.rows == 0) return Status::Ok();
+    if (((uintptr_t)a.x | (uintptr_t)a.router_x | (uintptr_t)a.router) % 16)  // (rows go by 16-byte loads and bulk copies)
+        return Status::Err(INFR_E_INVALID, "moe_ffn: x, router_x and router must be 16-byte aligned");
     if (((size_t)a.rows * a.n_used + 31) / 32 * a.n_expert * 4 > (size_t)200 * 1024)
         return Status::Err(INFR_E_UNSUPPORTED, fmt("moe_ffn: %u rows x %u experts per row exceed what one call sorts (split the rows)", a.rows, a.n_used));
     if (a.rows < 2 || reference_) {
@@ -895,10 +897,10 @@ Status CudaBackend::moe_ffn(const MoeArgs &a) {
     const size_t o_logits = take(rows * nx * 4), o_ids = take(n_pairs * 4), o_w = take(n_pairs * 4);
     const size_t o_prow = take(n_pairs * 4), o_pslot = take(n_pairs * 4);
     const size_t o_ie = take(max_items * 4), o_ip = take(max_items * 4), o_ic = take(max_items * 4), o_ni = take(4);
-    const size_t o_xq = take(rows * ne), o_xd = take(rows * (ne / 256) * 4), o_xs = take(rows * (ne / 32) * 4);
+    auto items_only = [&](size_t bytes) { return grouped_gemm ? 0 : take(bytes); };  // (the GEMM's layouts quantise the rows)
+    const size_t o_xq = items_only(rows * ne), o_xd = items_only(rows * (ne / 256) * 4), o_xs = items_only(rows * (ne / 32) * 4);
     const size_t o_xs16 = any_q6 ? take(rows * (ne / 16) * 4) : 0, o_as16 = any_q6 ? take(n_pairs * (nff / 16) * 4) : 0;
     const size_t o_g = take(n_pairs * nff * 4), o_u = take(n_pairs * nff * 4);
-    auto items_only = [&](size_t bytes) { return grouped_gemm ? 0 : take(bytes); };
     const size_t o_aq = items_only(n_pairs * nff), o_ad = items_only(n_pairs * (nff / 256) * 4), o_as = items_only(n_pairs * (nff / 32) * 4);
     const size_t o_y = take(n_pairs * ne * 4);
     const size_t o_px = grouped_gemm ? take(gemm_tc_grouped_record_bytes(slab, (int)max_slabs, (int)ne)) : 0;
@@ -933,9 +935,8 @@ Status CudaBackend::moe_ffn(const MoeArgs &a) {
               "moe bucket");
     // stage A: every distinct row quantised once (lib.rs:2688-2718), or by each of its slots where they are laid out for the GEMM (the layout waits on
     // its stores, not on the quantiser, and a launch of 3 us is saved)
-    const bool quantise_slots = grouped_gemm && (uintptr_t)a.x % 16 == 0;
     int32_t *xs16 = any_q6 ? reinterpret_cast<int32_t *>(b + o_xs16) : nullptr, *as16 = any_q6 ? reinterpret_cast<int32_t *>(b + o_as16) : nullptr;
-    if (!quantise_slots) INFR_STEP(launch_quantize_q8(a.x, (int)rows, (int)ne, 256, xq, xd, xs, xs16, nullptr, nullptr, stream_), "moe quantize x");
+    if (!grouped_gemm) INFR_STEP(launch_quantize_q8(a.x, (int)rows, (int)ne, 256, xq, xd, xs, xs16, nullptr, nullptr, stream_), "moe quantize x");
     Q8Dev xa{xq, xd, xs, xs16, 256};
     // one expert bank against the routed rows, 8-row items on the warp matrix unit (Q6_K rows too long for its tiles: byte-dot kernel)
     const int items = (int)((double)a.n_local * expected_items((double)nu / (double)nx, (int)rows) + 0.5);
@@ -955,7 +956,7 @@ Status CudaBackend::moe_ffn(const MoeArgs &a) {
         auto gemm = [&](const uint8_t *bank, const uint8_t *bank2, const uint8_t *rec, float *out, float *out2, uint32_t k, uint32_t o) {
             return launch_gemm_tc_grouped(slab, bank, bank2, (int)a.n_local, rec, out, out2, (int)k, (int)o, ie, ip, ic, ni, (int)max_slabs, dev_, status_dev_, stream_);
         };
-        INFR_STEP(launch_gemm_tc_grouped_prep(slab, quantise_slots ? a.x : nullptr, &xa, b + o_px, (int)ne, ie, ip, ic, ni, prow, (int)max_slabs, stream_), "moe layout x");
+        INFR_STEP(launch_gemm_tc_grouped_prep(slab, a.x, b + o_px, (int)ne, ie, ip, ic, ni, prow, (int)max_slabs, stream_), "moe layout x");
         INFR_STEP(gemm(a.gate, a.up, b + o_px, g, u, (uint32_t)ne, (uint32_t)nff), "moe gate, up (grouped gemm)");
         INFR_STEP(launch_gemm_tc_grouped_silu_prep(slab, g, u, b + o_pa, (int)nff, ie, ip, ic, ni, (int)max_slabs, stream_), "moe swiglu, layout");
         INFR_STEP(gemm(a.down, nullptr, b + o_pa, y, nullptr, (uint32_t)nff, (uint32_t)ne), "moe down (grouped gemm)");

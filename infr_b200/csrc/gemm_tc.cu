@@ -344,7 +344,7 @@ struct TcGroup {
     const int *slab_p0;      // [n_slabs] first routed pair of the slab; output row = pair
     const int *slab_cnt;     // [n_slabs] pairs in the slab (1..TN)
     const int *n_slabs;      // device scalar
-    const int *pair_row;     // [n_pairs] activation row of each pair, or nullptr: pair p reads row p
+    const int *pair_row;     // [n_pairs] row of x of each pair (the layout of x)
 };
 
 namespace {
@@ -372,8 +372,7 @@ __global__ void __launch_bounds__(256) gemm_tc_prep_kernel(const float *x, Q8Dev
     if (grp.slab_expert) {
         if (tt >= *grp.n_slabs) return;
         if (t >= grp.slab_cnt[tt]) return;  // (what a slot without a pair holds meets sums that are not stored: half the slots at 16 pairs an expert)
-        const int pair = grp.slab_p0[tt] + t;
-        row = grp.pair_row ? grp.pair_row[pair] : pair;
+        row = grp.pair_row[grp.slab_p0[tt] + t];
     }
     float v[PER][8];
     uint2 c[PER];
@@ -1038,7 +1037,8 @@ cudaError_t launch_prep(int fmt, const float *x, const Q8Dev &a, int m, int tn, 
                         cudaStream_t st) {
     const int nb = in_f / 256, per = grp.slab_expert ? (nb + kGroupedPer - 1) / kGroupedPer : nb;
     const dim3 grid((unsigned)(((size_t)n_tok * per + 7) / 8)), block(256);
-    if (grp.slab_expert) return launch_pdl(gemm_tc_prep_kernel<F_Q4, F32, kGroupedPer>, grid, block, 0, st, x, a, m, tn, in_f, units, extra, n_tok, grp);
+    if constexpr (F32)
+        if (grp.slab_expert) return launch_pdl(gemm_tc_prep_kernel<F_Q4, F32, kGroupedPer>, grid, block, 0, st, x, a, m, tn, in_f, units, extra, n_tok, grp);
     if (fmt == F_Q4) return launch_pdl(gemm_tc_prep_kernel<F_Q4, F32, 1>, grid, block, 0, st, x, a, m, tn, in_f, units, extra, n_tok, grp);
     return launch_pdl(gemm_tc_prep_kernel<F_Q6, F32, 1>, grid, block, 0, st, x, a, m, tn, in_f, units, extra, n_tok, grp);
 }
@@ -1157,14 +1157,12 @@ size_t gemm_tc_grouped_record_bytes(int slab, int max_slabs, int in_f) {
     const int n = max_slabs * slab;
     return units_bytes(n, in_f) + extra_bytes(F_Q4, n, in_f);
 }
-cudaError_t launch_gemm_tc_grouped_prep(int slab, const float *x, const Q8Dev *a, void *records, int in_f, const int *slab_expert, const int *slab_p0,
+cudaError_t launch_gemm_tc_grouped_prep(int slab, const float *x, void *records, int in_f, const int *slab_expert, const int *slab_p0,
                                         const int *slab_cnt, const int *n_slabs, const int *pair_row, int max_slabs, cudaStream_t st) {
-    if (!gemm_tc_takes(DT_Q4K, in_f) || max_slabs < 1) return cudaErrorInvalidValue;
+    if (!gemm_tc_takes(DT_Q4K, in_f) || max_slabs < 1 || (uintptr_t)x % 16) return cudaErrorInvalidValue;
     const int n = max_slabs * slab;
     uint8_t *u = static_cast<uint8_t *>(records), *e = u + units_bytes(n, in_f);
-    if (x && (uintptr_t)x % 16) return cudaErrorInvalidValue;
-    const TcGroup g{slab_expert, slab_p0, slab_cnt, n_slabs, pair_row};
-    return x ? launch_prep<true>(F_Q4, x, Q8Dev{}, n, slab, in_f, u, e, n, g, st) : launch_prep<false>(F_Q4, nullptr, *a, n, slab, in_f, u, e, n, g, st);
+    return launch_prep<true>(F_Q4, x, Q8Dev{}, n, slab, in_f, u, e, n, TcGroup{slab_expert, slab_p0, slab_cnt, n_slabs, pair_row}, st);
 }
 cudaError_t launch_gemm_tc_grouped_silu_prep(int slab, const float *gate, const float *up, void *records, int in_f, const int *slab_expert, const int *slab_p0,
                                              const int *slab_cnt, const int *n_slabs, int max_slabs, cudaStream_t st) {

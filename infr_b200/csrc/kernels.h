@@ -158,10 +158,9 @@ size_t gemm_q2_partial_bytes(int m, int in_f, int out_f1, int out_f2, const Devi
 cudaError_t launch_gemm_q2_prep(const float *x, void *records, int m, int in_f, cudaStream_t st);
 cudaError_t launch_gemm_q2(const uint8_t *w, const void *records, float *c, float *partials, int m, int in_f, int out_f, const DeviceInfo &dev,
                            uint32_t *status, cudaStream_t st, const uint8_t *w2 = nullptr, float *c2 = nullptr, int out_f2 = 0);
-// The same over a bank of Q4_K expert matrices, one slab of up to `slab` (32, 64) routed rows of an expert per token tile; `a`
-// quantised rows, gathered through pair_row when it is non-null.
+// The same over a bank of Q4_K expert matrices, one slab of up to `slab` (32, 64) routed rows of an expert per token tile: pair p is row pair_row[p] of x.
 size_t gemm_tc_grouped_record_bytes(int slab, int max_slabs, int in_f);
-cudaError_t launch_gemm_tc_grouped_prep(int slab, const float *x, const Q8Dev *a, void *records, int in_f, const int *slab_expert, const int *slab_p0,
+cudaError_t launch_gemm_tc_grouped_prep(int slab, const float *x, void *records, int in_f, const int *slab_expert, const int *slab_p0,
                                         const int *slab_cnt, const int *n_slabs, const int *pair_row, int max_slabs, cudaStream_t st);
 // The layout of silu(gate) * up, rows = pairs.
 cudaError_t launch_gemm_tc_grouped_silu_prep(int slab, const float *gate, const float *up, void *records, int in_f, const int *slab_expert, const int *slab_p0,
