@@ -237,9 +237,9 @@ __device__ __forceinline__ uint8_t *align_tile(uint8_t *p) {
 }
 template <class T>
 constexpr int kTileBytes = 2 * T::kBytes + T::kAlign - 16;
-// Maps of the caches (rows of n_kv * HD halves), keys and values, in boxes of a whole tile's rows and of kBoxRows.
+// Maps of the caches (rows of n_kv * HD halves): keys and values in boxes of a whole tile's rows, the same in boxes of kBoxRows.
 struct AttnMaps {
-    CUtensorMap whole[2], part[2];
+    CUtensorMap map[4];
 };
 struct NoMaps {};
 // By one thread; by the whole CTA with the maps
@@ -252,7 +252,7 @@ __device__ __forceinline__ void init_bars(uint64_t *s_bar) {
 }
 template <int HD>
 __device__ __forceinline__ void init_bars(uint64_t *s_bar, const AttnMaps &maps) {
-    if (threadIdx.x % 32 == 0 && threadIdx.x < 128) asm volatile("prefetch.tensormap [%0];" ::"l"(maps.whole + threadIdx.x / 32) : "memory");
+    if (threadIdx.x % 32 == 0 && threadIdx.x < 128) asm volatile("prefetch.tensormap [%0];" ::"l"(maps.map + threadIdx.x / 32) : "memory");
     if (threadIdx.x == 0) init_bars<HD>(s_bar);
 }
 // Warps 0 .. HD / 32 - 1 fetch a tile, from row `row0` of a sequence's caches on: warp w the dims 64 (w / 2) .. + 63 of the keys (even) or values, in one copy; of a tile of
@@ -273,9 +273,9 @@ __device__ __forceinline__ void fetch_tile(const AttnMaps &maps, uint8_t *s_k, u
                      : "memory");
     };
     if (keys == kAttnTile) {
-        if (lane == 0) copy(maps.whole + which, 0);
+        if (lane == 0) copy(maps.map + which, 0);
     } else if (lane * kBoxRows < keys) {
-        copy(maps.part + which, lane * kBoxRows);
+        copy(maps.map + 2 + which, lane * kBoxRows);
     }
 }
 // Rows r0 .. r1 - 1 of the values, past the end of a tile: the matrix unit is to multiply 0 (not stale bits) by the weight 0.  Those of a box that
@@ -1401,7 +1401,7 @@ static bool attn_maps(const void *k, const void *v, size_t n_rows, int n_seq, si
         return enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<void *>(base), dim, stride, box, one, CU_TENSOR_MAP_INTERLEAVE_NONE,
                    CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
     };
-    return make(&maps->whole[0], k, kAttnTile) && make(&maps->whole[1], v, kAttnTile) && make(&maps->part[0], k, kBoxRows) && make(&maps->part[1], v, kBoxRows);
+    return make(&maps->map[0], k, kAttnTile) && make(&maps->map[1], v, kAttnTile) && make(&maps->map[2], k, kBoxRows) && make(&maps->map[3], v, kBoxRows);
 }
 
 template <int HD, int G>
