@@ -601,8 +601,8 @@ cudaError_t launch_gemv_q6_mma(const uint8_t *w, const Q8Dev &a, float *y, int m
     return launch_m6<8>(w, a, y, m, in_f, out_f, dev, status, st, push);
 }
 
-// The grouped form.  cudaErrorInvalidValue when the shape does not qualify (heights that are not whole tiles, rows so long that two
-// tiles a warp do not fit, an unaligned bank): the caller takes the direct-load byte-dot kernel.
+// The grouped form.  cudaErrorInvalidValue when the shape does not qualify (heights that are not whole tiles, rows so long that fewer than four
+// tiles fit beside eight staged rows, an unaligned bank): the caller takes the direct-load byte-dot kernel.
 cudaError_t launch_grouped_q6_mma(const uint8_t *bank, const Q8Dev &a, float *y, int in_f, int out_f, const int *item_expert, const int *item_p0,
                                   const int *item_cnt, const int *n_items, const int *pair_row, int max_items, int items, const DeviceInfo &dev, uint32_t *status,
                                   cudaStream_t st) {
@@ -616,12 +616,13 @@ cudaError_t launch_grouped_q6_mma(const uint8_t *bank, const Q8Dev &a, float *y,
         return budget < rest ? 0 : (int)((budget - rest) / (tile + 12));
     };
     auto warps_of = [&](int n) { return n < 2 ? 0 : std::min(kGroupedWarps6, n - std::max(n > 4 ? 2 : 1, n / 5)); };
-    const int s2 = slots_of(2), s1 = slots_of(1), ctas = 2 * warps_of(s2) >= warps_of(s1) ? 2 : 1;
+    const int s2 = slots_of(2), s1 = slots_of(1);
+    if (std::max(s1, s2) < 4) return cudaErrorInvalidValue;
+    const int ctas = 2 * warps_of(s2) >= warps_of(s1) ? 2 : 1;
     int kw = warps_of(ctas == 2 ? s2 : s1);
     const long long all = (long long)(items < 1 ? 1 : items) * (out_f / kRows6);
     while (nb >= 3 && kw > 2 && all < (long long)kw * dev.sm_count) kw--;  // few large tiles: on all SMs rather than on all warps of some
     const int slots = std::min(ctas == 2 ? s2 : s1, 2 * kw);
-    if (std::max(s1, s2) < 4) return cudaErrorInvalidValue;
     const size_t smem = slots * (tile + 12) + rest;
     cudaError_t e = cudaFuncSetAttribute(gemv_q6_mma_grouped_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
