@@ -189,13 +189,12 @@ __global__ void __launch_bounds__(KW * TG * 32, 16 / (KW * TG))
     float *s_d8 = reinterpret_cast<float *>(s_bsplit + (size_t)M * nb * 16);  // [nb][8]
     float *s_part = s_d8 + (size_t)nb * 8;                         // [TG][2][kW][16][8]
     uint64_t *bars = reinterpret_cast<uint64_t *>(s_part + 2 * kW * TG * 128);  // [kW * TG][kMaxSlotsMma]
-    __shared__ int s_bad;
+    __shared__ int s_asked[KW * TG];  // by a warp that has given up: its copies
     __shared__ uint32_t s_epoch;  // push mode: exchanges completed before this launch
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, kwarp = TG == 1 ? warp : warp % kW, tg = TG == 1 ? 0 : warp / kW;
     const int g = lane >> 2, t = lane & 3;
     if (threadIdx.x == 0) {
-        s_bad = 0;
         for (int i = 0; i < kW * TG * kMaxSlotsMma; i++) bar_init(s_u32(bars + i), 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -240,7 +239,6 @@ __global__ void __launch_bounds__(KW * TG * 32, 16 / (KW * TG))
     uint64_t l2_policy;
     asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(l2_policy));
     // ---- issue side: one elected lane fetches the 16-row x K-step box of the slot ----
-    bool dead = false;
     int j_issue = 0, i_step = 0, i_T = t_begin + tg;
     int i_item = 0;  // the item of tile i_T
     if (SHARE) {
@@ -251,7 +249,7 @@ __global__ void __launch_bounds__(KW * TG * 32, 16 / (KW * TG))
         row_base = grp.item_expert[i_item] * out_f;
     }
     auto issue = [&](int slot) {
-        if (j_issue >= n_jobs || dead) return;
+        if (j_issue >= n_jobs) return;
         if (lane == 0) {
             const int blk0 = kb0 + i_step * kStepBlocks;
             const uint32_t bar = s_u32(wbar + slot);
@@ -285,6 +283,7 @@ __global__ void __launch_bounds__(KW * TG * 32, 16 / (KW * TG))
     const int gt = g < M ? g : 0;  // token whose codes this lane feeds as its B column
     int slot = 0, tile = 0;
     uint32_t phase = 0;
+    bool dead = false;
     for (int item = SHARE ? t_begin / total_tiles : 0;; item++) {  // even shares: the items of this CTA, otherwise once (body not indented)
     int seg_end = 0, tid = threadIdx.x;
     if (SHARE) asm volatile("" : "+r"(tid));  // (what the staging derives from it is not kept in registers from one item to the next)
@@ -400,10 +399,8 @@ __global__ void __launch_bounds__(KW * TG * 32, 16 / (KW * TG))
         for (int step = 0; step < steps_per_tile; step++) {
             if (!dead && !bar_wait(s_u32(wbar + slot), phase)) {
                 dead = true;
-                if (lane == 0) {
-                    atomicExch(status, 3u);
-                    s_bad = 1;
-                }
+                s_asked[warp] = j_issue, j_issue = n_jobs;  // nothing more is asked for
+                if (lane == 0) atomicExch(status, 3u);
             }
             const int blk0 = kb0 + step * kStepBlocks;
             const int nblk = min(kStepBlocks, kb1 - blk0);
@@ -518,7 +515,7 @@ __global__ void __launch_bounds__(KW * TG * 32, 16 / (KW * TG))
     }
     if (!SHARE) break;
     }
-    if (dead) drain_ring(wbar, S, j_issue);
+    if (dead) drain_ring(wbar, S, s_asked[warp]);
 }
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,

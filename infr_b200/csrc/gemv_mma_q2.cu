@@ -65,6 +65,7 @@ template <int M, int KW>
 __global__ void __launch_bounds__(KW * 32, 16 / KW)
     gemv_q2_mma_kernel(const __grid_constant__ CUtensorMap tmap, Q8Dev a, float *__restrict__ y, int m, int in_f, int out_f,
                        Q2Geom geo, uint32_t *__restrict__ status) {
+    __shared__ int s_asked[KW];  // by a warp that has given up: its copies
     extern __shared__ __align__(128) uint8_t smem[];
     const int nch = geo.nch, S = geo.slots, ng = nch * kChunkGroups;
     uint8_t *rings = smem;
@@ -95,9 +96,8 @@ __global__ void __launch_bounds__(KW * 32, 16 / KW)
     uint64_t *wbar = bars + warp * kMaxSlots;
 
     int j_issue = 0, i_tile = 0, i_ch = 0;
-    bool dead = false;
     auto issue = [&](int slot) {
-        if (j_issue >= n_jobs || dead) return;
+        if (j_issue >= n_jobs) return;
         if (lane == 0) {
             const uint32_t bar = sm32(wbar + slot);
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // earlier reads of the slot come first
@@ -155,11 +155,13 @@ __global__ void __launch_bounds__(KW * 32, 16 / KW)
     const int n0 = 2 * t, n1 = 2 * t + 1;    // tokens of this lane's result columns
     int slot = 0;
     uint32_t phase = 0;
+    bool dead = false;
     for (int tile = 0; tile < n_tiles; tile++) {
         float accf[4] = {0.f, 0.f, 0.f, 0.f};
         for (int ci = 0; ci < my_chunks; ci++) {
             if (!dead && !wait_parity(sm32(wbar + slot), phase)) {
                 dead = true;
+                s_asked[warp] = j_issue, j_issue = n_jobs;  // nothing more is asked for
                 if (lane == 0) atomicExch(status, 3u);
             }
             if (!dead) {
@@ -218,7 +220,7 @@ __global__ void __launch_bounds__(KW * 32, 16 / KW)
             }
         }
     }
-    if (dead) drain_ring(wbar, S, j_issue);
+    if (dead) drain_ring(wbar, S, s_asked[warp]);
 }
 
 typedef CUresult (*EncQ2)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,

@@ -151,6 +151,7 @@ __global__ void __launch_bounds__(KW * 32, 16 / KW)
     gemv_q6_mma_kernel(const __grid_constant__ CUtensorMap tmap, Q8Dev a, float *__restrict__ y, int m, int in_f, int out_f,
                        Q6Geom geo, uint32_t *__restrict__ status, const __grid_constant__ typename PushParam<PUSH>::type push) {
     __shared__ uint32_t s_epoch;  // push mode: exchanges completed before this launch
+    __shared__ int s_asked[KW];  // by a warp that has given up: its copies
     extern __shared__ __align__(128) uint8_t smem[];
     const int nb = geo.nb, S = geo.slots;
     uint8_t *rings = smem;
@@ -179,9 +180,8 @@ __global__ void __launch_bounds__(KW * 32, 16 / KW)
     uint64_t *wbar = bars + warp * kMaxSlots6;
 
     int j_issue = 0, i_tile = 0, i_b = 0;
-    bool dead = false;
     auto issue = [&](int slot) {
-        if (j_issue >= n_jobs || dead) return;
+        if (j_issue >= n_jobs) return;
         if (lane == 0) {
             const uint32_t bar = sm6(wbar + slot);
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // earlier reads of the slot come first
@@ -251,11 +251,13 @@ __global__ void __launch_bounds__(KW * 32, 16 / KW)
     const int n0 = 2 * t;          // first of this lane's two result columns
     int slot = 0;
     uint32_t phase = 0;
+    bool dead = false;
     for (int tile = 0; tile < n_tiles; tile++) {
         float accf[4] = {0.f, 0.f, 0.f, 0.f};
         for (int bi = 0; bi < my_blocks; bi++) {
             if (!dead && !wait_parity6(sm6(wbar + slot), phase)) {
                 dead = true;
+                s_asked[warp] = j_issue, j_issue = n_jobs;  // nothing more is asked for
                 if (lane == 0) atomicExch(status, 3u);
             }
             if (!dead) {
@@ -296,7 +298,7 @@ __global__ void __launch_bounds__(KW * 32, 16 / KW)
             }
         }
     }
-    if (dead) drain_ring(wbar, S, j_issue);
+    if (dead) drain_ring(wbar, S, s_asked[warp]);
 }
 
 // ---- Expert-grouped form (mixture of experts): blockIdx.y walks the device-built list of work items, each up to 8 routed pairs of one

@@ -270,6 +270,7 @@ __global__ void __launch_bounds__(kWWarps * 32, 1)
                      const __grid_constant__ WideSecond sec) {
     constexpr int kPart = 8 * NT * kWPitch;  // floats of one warp's partial tile
     __shared__ uint32_t s_epoch;  // push mode (one K chunk only): exchanges completed before this launch
+    __shared__ int s_asked[kWWarps];  // by a warp that has given up: its copies
     extern __shared__ __align__(128) uint8_t smem[];
     const int S = slots;
     uint8_t *rings = smem;
@@ -299,9 +300,8 @@ __global__ void __launch_bounds__(kWWarps * 32, 1)
     uint64_t l2_policy;
     asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(l2_policy));
     int j_issue = 0;
-    bool dead = false;
     auto issue = [&](int slot) {
-        if (j_issue >= n_jobs || dead) return;
+        if (j_issue >= n_jobs) return;
         if (lane == 0) {
             const uint32_t bar = sw32(wbar + slot);
             // order this warp's earlier reads of the slot before the engine overwrites it
@@ -339,6 +339,7 @@ __global__ void __launch_bounds__(kWWarps * 32, 1)
     float *dst2 = sec.out + (size_t)blockIdx.y * (size_t)m * sec.out_f;
     int slot = 0;
     uint32_t phase = 0;
+    bool dead = false;
     for (int tile = 0; tile < n_tiles; tile++) {
         float accf[NT][4];
 #pragma unroll
@@ -346,6 +347,7 @@ __global__ void __launch_bounds__(kWWarps * 32, 1)
         if (active) {
             if (!dead && !wide_wait(sw32(wbar + slot), phase)) {
                 dead = true;
+                s_asked[warp] = j_issue, j_issue = n_jobs;  // nothing more is asked for
                 if (lane == 0) atomicExch(status, 3u);
             }
             if (!dead) F::template block<NT>(ring + (size_t)slot * F::kSlotBytes, b, g, t, bw, e, accf);
@@ -384,7 +386,7 @@ __global__ void __launch_bounds__(kWWarps * 32, 1)
             }
         }
     }
-    if (dead) drain_ring(wbar, S, j_issue);
+    if (dead) drain_ring(wbar, S, s_asked[warp]);
 }
 
 // y[i] = part[0][i] + part[1][i] + ... in chunk order (the same bits on every run).

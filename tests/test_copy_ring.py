@@ -109,7 +109,8 @@ def test_ring_of_a_warp(tmp_path):
 def test_rings_of_warps_are_drained(source):
     # a warp that has given up asks for nothing more, and its kernel ends with the wait for what it had asked for
     body = _loop(source, r"auto issue = \[&\]\(int slot\) \{(.*?\n\}\n)")
-    assert body.lstrip().startswith("if (j_issue >= n_jobs || dead) return;") and body.endswith("    if (dead) drain_ring(wbar, S, j_issue);\n}\n")
+    assert body.lstrip().startswith("if (j_issue >= n_jobs) return;") and body.endswith("    if (dead) drain_ring(wbar, S, s_asked[warp]);\n}\n")
+    assert "s_asked[warp] = j_issue, j_issue = n_jobs;" in _loop(source, r"if \(!dead && !\w+\(\w+\(wbar \+ slot\), phase\)\) \{(.*?)\n            \}\n")
 
 
 def test_gemm_producer_is_drained():
