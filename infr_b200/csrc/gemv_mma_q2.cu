@@ -65,7 +65,6 @@ template <int M, int KW>
 __global__ void __launch_bounds__(KW * 32, 16 / KW)
     gemv_q2_mma_kernel(const __grid_constant__ CUtensorMap tmap, Q8Dev a, float *__restrict__ y, int m, int in_f, int out_f,
                        Q2Geom geo, uint32_t *__restrict__ status) {
-    __shared__ int s_asked[KW];  // by a warp that has given up: its copies
     extern __shared__ __align__(128) uint8_t smem[];
     const int nch = geo.nch, S = geo.slots, ng = nch * kChunkGroups;
     uint8_t *rings = smem;
@@ -91,7 +90,7 @@ __global__ void __launch_bounds__(KW * 32, 16 / KW)
     const int r_begin = t_begin * kRows;
     const int c0 = warp * geo.cpw, c1 = min(nch, c0 + geo.cpw);
     const int my_chunks = max(0, c1 - c0);
-    const int n_jobs = n_tiles * my_chunks;
+    int n_jobs = n_tiles * my_chunks;
     uint8_t *ring = rings + (size_t)warp * S * kSlotBytes;
     uint64_t *wbar = bars + warp * kMaxSlots;
 
@@ -161,7 +160,7 @@ __global__ void __launch_bounds__(KW * 32, 16 / KW)
         for (int ci = 0; ci < my_chunks; ci++) {
             if (!dead && !wait_parity(sm32(wbar + slot), phase)) {
                 dead = true;
-                s_asked[warp] = j_issue, j_issue = n_jobs;  // nothing more is asked for
+                n_jobs = j_issue;  // nothing more is asked for
                 if (lane == 0) atomicExch(status, 3u);
             }
             if (!dead) {
@@ -220,7 +219,7 @@ __global__ void __launch_bounds__(KW * 32, 16 / KW)
             }
         }
     }
-    if (dead) drain_ring(wbar, S, s_asked[warp]);
+    if (dead) drain_ring(wbar, S, j_issue);
 }
 
 typedef CUresult (*EncQ2)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,

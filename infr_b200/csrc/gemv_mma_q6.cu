@@ -151,7 +151,6 @@ __global__ void __launch_bounds__(KW * 32, 16 / KW)
     gemv_q6_mma_kernel(const __grid_constant__ CUtensorMap tmap, Q8Dev a, float *__restrict__ y, int m, int in_f, int out_f,
                        Q6Geom geo, uint32_t *__restrict__ status, const __grid_constant__ typename PushParam<PUSH>::type push) {
     __shared__ uint32_t s_epoch;  // push mode: exchanges completed before this launch
-    __shared__ int s_asked[KW];  // by a warp that has given up: its copies
     extern __shared__ __align__(128) uint8_t smem[];
     const int nb = geo.nb, S = geo.slots;
     uint8_t *rings = smem;
@@ -175,7 +174,7 @@ __global__ void __launch_bounds__(KW * 32, 16 / KW)
     const int r_begin = t_begin * kRows6;
     const int b0 = warp * geo.bpw, b1 = min(nb, b0 + geo.bpw);
     const int my_blocks = max(0, b1 - b0);
-    const int n_jobs = n_tiles * my_blocks;
+    int n_jobs = n_tiles * my_blocks;
     uint8_t *ring = rings + (size_t)warp * S * kSlotBytes6;
     uint64_t *wbar = bars + warp * kMaxSlots6;
 
@@ -257,7 +256,7 @@ __global__ void __launch_bounds__(KW * 32, 16 / KW)
         for (int bi = 0; bi < my_blocks; bi++) {
             if (!dead && !wait_parity6(sm6(wbar + slot), phase)) {
                 dead = true;
-                s_asked[warp] = j_issue, j_issue = n_jobs;  // nothing more is asked for
+                n_jobs = j_issue;  // nothing more is asked for
                 if (lane == 0) atomicExch(status, 3u);
             }
             if (!dead) {
@@ -298,7 +297,7 @@ __global__ void __launch_bounds__(KW * 32, 16 / KW)
             }
         }
     }
-    if (dead) drain_ring(wbar, S, s_asked[warp]);
+    if (dead) drain_ring(wbar, S, j_issue);
 }
 
 // ---- Expert-grouped form (mixture of experts): blockIdx.y walks the device-built list of work items, each up to 8 routed pairs of one
@@ -491,10 +490,10 @@ __global__ void __launch_bounds__(32 * kGroupedWarps6, 2) gemv_q6_mma_grouped_ke
             if (n0 + 1 < m) yr[out_f] = accf[1], yr[out_f + 8] = accf[3];
         }
     }
-    // Somebody gave up: what is on its way, the last tile of every slot, lands before the shared memory is another CTA's.  (Only here has the last
-    // of them been asked for: a warp that had not seen s_dead may have asked after the tile's own warp had looked.)
-    if (__syncthreads_or(dead))
-        for (int s = threadIdx.x; s < slots; s += blockDim.x)
+    // Somebody gave up: what is on its way, the last tile of every slot, lands before the shared memory is another CTA's.  (A warp asks for a tile only while it does
+    // not see s_dead, and then either the warp that sets it finds that tile here or this warp does.)
+    if (s_dead)
+        for (int s = lane; s < slots; s += 32)
             if (s_tile[s] >= 0) wait_parity6(sm6(bars + s), (uint32_t)(s_tile[s] / slots) & 1u);
 }
 

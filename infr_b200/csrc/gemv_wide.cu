@@ -270,7 +270,6 @@ __global__ void __launch_bounds__(kWWarps * 32, 1)
                      const __grid_constant__ WideSecond sec) {
     constexpr int kPart = 8 * NT * kWPitch;  // floats of one warp's partial tile
     __shared__ uint32_t s_epoch;  // push mode (one K chunk only): exchanges completed before this launch
-    __shared__ int s_asked[kWWarps];  // by a warp that has given up: its copies
     extern __shared__ __align__(128) uint8_t smem[];
     const int S = slots;
     uint8_t *rings = smem;
@@ -293,7 +292,7 @@ __global__ void __launch_bounds__(kWWarps * 32, 1)
     const int n_tiles = base + (blockIdx.x < rem ? 1 : 0);
     const int b = blockIdx.y * kWWarps + warp;
     const bool active = b < nb;
-    const int n_jobs = active ? n_tiles : 0;
+    int n_jobs = active ? n_tiles : 0;
     uint8_t *ring = rings + (size_t)warp * S * F::kSlotBytes;
     uint64_t *wbar = bars + warp * kWSlots;
 
@@ -347,7 +346,7 @@ __global__ void __launch_bounds__(kWWarps * 32, 1)
         if (active) {
             if (!dead && !wide_wait(sw32(wbar + slot), phase)) {
                 dead = true;
-                s_asked[warp] = j_issue, j_issue = n_jobs;  // nothing more is asked for
+                n_jobs = j_issue;  // nothing more is asked for
                 if (lane == 0) atomicExch(status, 3u);
             }
             if (!dead) F::template block<NT>(ring + (size_t)slot * F::kSlotBytes, b, g, t, bw, e, accf);
@@ -386,7 +385,7 @@ __global__ void __launch_bounds__(kWWarps * 32, 1)
             }
         }
     }
-    if (dead) drain_ring(wbar, S, s_asked[warp]);
+    if (dead) drain_ring(wbar, S, j_issue);
 }
 
 // y[i] = part[0][i] + part[1][i] + ... in chunk order (the same bits on every run).
