@@ -1476,7 +1476,7 @@ cudaError_t launch_attention(const float *q, const void *k_cache, const void *v_
     const size_t live = (tiles_to(max_keys) - tiles_to(pos)) * n_kv * n_seq, shared = (size_t)n_splits * n_kv * n_seq * row_blocks;
     const bool chunk = head_dim == 128 && rows > 1 && (g == 1 || g == 2 || g == 4 || g == 8) && 2 * live > 5 * sms &&
                        (rows > 2 * row_blocks || 8 * rows >= 7 * rpt * row_blocks || shared <= 2 * sms);
-    // Tensor copies where the tiles are more than two waves of CTAs (three fit an SM, two of the shared form).  Before that the latency of the first byte
+    // Tensor copies where a tile for each row makes more than two waves of CTAs (three fit an SM), shared tiles more than one (two fit).  Before that the latency of the first byte
     // counts, which is 0.5 to 1 us longer with them: shared tiles, bulk copies of rows / tensor copies, us a call: 32 heads / 8, 64 rows at 128 (256 tiles) 12.1 / 13.1;
     // 8 / 8, 20 rows at 640 (96) 16.0 / 17.2, 300 at 0 (264) 18.3 / 19.2, 64 at 1500 (400) 18.2 / 16.3, 128 at 3000 45 / 42; 32 / 8, 113 at 384 (928) 29.4 / 27.4,
     // 128 at 3000 153 / 142.

@@ -27,21 +27,19 @@
 // TN = 32 (Q4_K) keeps to half an SM's shared and tensor memory, so that two CTAs hide each other's waits.
 // Tiles: whole waves of them are multiplied over all of K; the rest of them is split over K so that it fills the SMs too, and a
 // small kernel adds the parts in split order (deterministic).
-// Measured (B200, us, whole calls over rotated cold weights, back to back, so that a call's layout launch overlaps the call before; before
-// = a warp issuing under `lane == 0`, stages held until the epilogue, whole waves only):  Q4_K 4096 -> 14336, 512 rows 113 -> 82 (a call
-// that waits for the one before it: 112 -> 89), 113 rows 35 -> 30, 1024 rows 192 -> 153;  14336 -> 4096, 1024 rows 194 -> 175;  Q6_K
-// 14336 -> 4096, 113 rows 57 -> 53, 512 rows 183 -> 177.
-// Q6_K's unpacking was the longest part of a job (3900 of 5860 cycles of an unpack warp, clock64).  Nibble and high bits meet in one LOP3 before
-// the bytes part (5 integer instructions for 4 weights, 7 before), the offset is inside the multiply-add, rows are read in 8-byte words from
-// a pitch of 240 bytes (no conflicts, one level of selects less) and the two teams' slots are multiplied in turn.  Cold weights, us, before:
-// 4096 -> 14336, 33..64 rows 42, 53; 113 rows 52, 57;  14336 -> 4096, 64 rows 42, 52; 113 rows 51, 55; 1000 rows 296, 318 (and one pass, kJobBuf, after that).
 // What bounds it: every role is a chain of dependent instructions and of barriers that cost its warp 100 to 200 cycles each, seen or not; a
 // barrier between two roles is therefore as dear as what it guards.  Hence one barrier for a job's activation operands, none for giving them
 // back where the accumulators' says as much, one epilogue warp that waits for the others (they stand at a named barrier), two issuers (one was
-// busy for 2400 cycles of a job's 2550), and as few instructions as can be for a weight.  Before / after, us, cold weights, back to back: Q4_K
-// 4096 -> 28672, 32 rows 34.2 / 31.1, 113 rows 50.8 / 47.2; 4096 -> 14336, 512 rows 81 / 75; Q6_K 14336 -> 4096, 512 rows 148 / 137.
-// At 128 tokens a Q4_K job takes ~2320 cycles (2550), its MMAs 1150; the warps issue 5980 instructions (6670).  Q6_K calls with a few jobs a CTA are 0.9 us
-// slower for it (4096 -> 4096, 113 rows 20.6 / 21.5), of a cause that neither the place of the waits nor the size of the first copies is.
+// busy for 2400 cycles of a job's 2550), and as few instructions as can be for a weight.  Q6_K's unpacking is the longest part of a job: nibble and high bits
+// meet in one LOP3 before the bytes part, the offset is inside the multiply-add, rows are read in 8-byte words from a pitch of 240 bytes and
+// the two teams' slots are multiplied in turn.  At 128 tokens a Q4_K job takes ~2320 cycles, its MMAs 1150; the warps issue 5980 instructions.
+// Measured (B200, us, whole calls over rotated cold weights, back to back, so that a call's layout launch overlaps the call before):
+//   Q4_K  4096 -> 14336  113 rows 26.8, 512 rows 74 (a call that waits for the one before it 86), 1024 rows 136;  14336 -> 4096, 1024 rows 150;  4096 -> 28672, 32 rows 31.6
+//   Q6_K  14336 -> 4096  64 rows 37, 113 rows 43.1, 512 rows 136, 1000 rows 246;  4096 -> 14336  64 rows 37.8, 113 rows 45, 512 rows 125;  4096 -> 4096, 113 rows 20.2
+// What the steps gave: one elected thread that issues, stages given back when unpacked, only the last tiles split over K: Q4_K, 512 rows 113 -> 82;
+// the unpacking of Q6_K 4096 -> 14336, 64 rows 53 -> 42; Q6_K at 128 tokens in one pass (kJobBuf); fewer barriers, two issuers, nibbles as subnormals 82 -> 74 and
+// Q6_K 14336 -> 4096, 512 rows 148 -> 142; Q6_K's waits (kFarWaits, the issuer's for the accumulators) 142 -> 136, and calls with a few jobs a CTA, which
+// the step before had slowed down, 21.2 -> 20.2.
 // Tried: 16 unpack and 8 epilogue warps (4 % slower), waits as tight loops in PTX (30 to 100 % slower: they poll more often), sleeping
 // between polls (1 to 15 % slower), the issuer's loop not unrolled (17 % slower), a look at all of a job's barriers at once (no gain), a chunk's
 // tensor-memory load during the fold of the one before it (spills).

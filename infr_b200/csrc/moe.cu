@@ -23,7 +23,7 @@ namespace infr {
 // `dot` (lane j takes elements j, 8 + j, ... in order, the lanes are then summed in order; rows are whole groups of eight).  A lane has 4 rows x 4 experts, a warp 4 x 16, a block of four warps 16 x 16.  Columns come 512 at a time, a bulk copy a row (the copy engine
 // takes a row in 45 cycles, however short), into a ring of three; the row pitch (520 words) puts the four groups of a warp on disjoint banks.
 // What bounds it: shared memory delivers 128 bytes a cycle to registers however many lanes share an address, so that the work per value read counts: 8
-// reads feed 16 multiply-adds (128 experts x 2048, 256 rows: 7100 cycles), where 6 fed 8.  Behind that one warp a scheduler.
+// reads feed 16 multiply-adds (128 experts x 2048, 256 rows: 4 warps x 256 x 8 = 8192 cycles a block), where 6 fed 8.  Behind that one warp a scheduler.
 // Measured there: 13.6 us (the first copies land after 3.3, 16000 cycles are reads and multiply-adds), 18.7 before; 512 rows of 4096: 46, 66.  (Columns
 // 256 at a time 18.7; a row and two experts a thread by 16-byte reads and packed multiply-adds 21.7.)
 constexpr int kRtRows = 16, kRtExperts = 16, kRtK = 512, kRtPitch = kRtK + 8, kRtBuf = (kRtRows + kRtExperts) * kRtPitch, kRtRing = 3;
