@@ -12,7 +12,7 @@ KEYS = [1, 15, 16, 17, 31, 33, 112, 113, 127, 128, 129, 143, 144, 145, 255, 256]
 
 
 def _form(backend, call):
-    return [f"{name}<{args}>" for name, args, _ in launched(backend, call) if name in ("attn_chunk_kernel", "attn_split_kernel")]
+    return [f"{name}<{args}>" for name, args, _ in launched(backend, call, ("attn_chunk_kernel", "attn_split_kernel"))]
 
 
 @pytest.mark.parametrize("n_head,n_kv,hd,n_seq,rows,gap,form", [

@@ -34,7 +34,8 @@ def test_grids_and_bits(backend, rows, ne, n_expert, n_used, nff, even):
         rows_in = wrap(x[r0:r0 + n])
         backend.moe_ffn(rows_in, rows_in, *weights, wrap(dst[r0:r0 + n]), rows=n, ne=ne, n_expert=n_expert, n_used=n_used, n_ff_exp=nff, wdt=Q4K, down_dt=Q6K)
 
-    grids = {name: grid for name, _, grid in launched(backend, lambda: call(out, 0, rows))}
+    records = launched(backend, lambda: call(out, 0, rows), ("gemv_q4k_mma_kernel",), ("gemv_q6_mma_grouped_kernel",))
+    grids = {name: grid for name, _, grid in records}
     assert (grids["gemv_q4k_mma_kernel"][1] == 1, grids["gemv_q6_mma_grouped_kernel"][1] == 1) == even
     n = rows - (rows % 3 == 1)  # (a single row takes the f32 path)
     for r0 in range(0, n, 3):
